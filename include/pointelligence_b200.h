@@ -112,6 +112,27 @@ int pcx_mvmr(const void *d_weight, const void *d_feat, const int32_t *d_gather,
              int64_t n_out, int K, int G, int C, int M, int transpose,
              int dtype, int engine, void *d_ws, size_t ws_bytes, void *stream);
 
+/* pcx_mvmr with a bias (G*out_width elements of `dtype`, or NULL) added to every
+ * output row before the single rounding, and `flags` in place of `transpose`:
+ * bit 0 (PCX_MVMR_TRANSPOSE) is `transpose`, bit 1 (PCX_MVMR_REVERSE_TAPS) makes
+ * tap k of the rulebook use weight K-1-k -- the input gradient over a rulebook
+ * that is its own mirror image.  The bias replaces the `output + bias` pass of
+ * layers/conv.py:430-465. */
+#define PCX_MVMR_TRANSPOSE 1
+#define PCX_MVMR_REVERSE_TAPS 2
+int pcx_mvmr_bias(const void *d_weight, const void *d_feat,
+                  const int32_t *d_gather, const int32_t *d_scatter,
+                  const int64_t *d_seg_offs, const int32_t *d_tap_idx,
+                  const void *d_bias, void *d_out, int64_t T, int64_t n_feat,
+                  int64_t n_out, int K, int G, int C, int M, int flags,
+                  int dtype, int engine, void *d_ws, size_t ws_bytes,
+                  void *stream);
+
+/* out[c] = sum over r of x[r, c], fp32 sums, one rounding: the bias gradient. */
+size_t pcx_column_sums_workspace_bytes(int64_t N, int C);
+int pcx_column_sums(const void *d_x, void *d_out, int64_t N, int C, int dtype,
+                    void *d_ws, size_t ws_bytes, void *stream);
+
 /* ------------------------------------------------------------------------
  * Output-stationary MVMR: same result as pcx_mvmr (fp16 / bf16, one group,
  * tap-sorted triplets), computed from a "plan" of the rulebook.
@@ -164,6 +185,13 @@ int pcx_mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan,
                      int64_t n_out, int K, int C, int M, int transpose,
                      int dtype, int group_blocks, int64_t multi_buckets,
                      void *d_ws, size_t ws_bytes, void *stream);
+/* ... with a bias and `flags` in place of `transpose`, as pcx_mvmr_bias. */
+int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat,
+                          void *d_plan, size_t plan_bytes, const void *d_bias,
+                          void *d_out, int64_t T, int64_t n_feat, int64_t n_out,
+                          int K, int C, int M, int flags, int dtype,
+                          int group_blocks, int64_t multi_buckets, void *d_ws,
+                          size_t ws_bytes, void *stream);
 
 /* Launches one thread that waits on a barrier nothing arrives at: the bounded
  * wait gives up after limit_ns (at most 100 ms), sets bit 8 of the device

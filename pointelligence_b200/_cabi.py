@@ -47,6 +47,9 @@ SIGNATURES = {
     "pcx_profile_get": (c_int, [c_int, ctypes.POINTER(ctypes.c_char_p), ctypes.POINTER(ctypes.c_float)]),
     "pcx_mvmr_workspace_bytes": (c_size_t, [c_int64, c_int, c_int, c_int, c_int, c_int, c_int]),
     "pcx_mvmr": (c_int, [c_void_p] * 7 + [c_int64] * 3 + [c_int] * 7 + [c_void_p, c_size_t, c_void_p]),
+    "pcx_mvmr_bias": (c_int, [c_void_p] * 8 + [c_int64] * 3 + [c_int] * 7 + [c_void_p, c_size_t, c_void_p]),
+    "pcx_column_sums_workspace_bytes": (c_size_t, [c_int64, c_int]),
+    "pcx_column_sums": (c_int, [c_void_p] * 2 + [c_int64, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "pcx_mvmr_plan_group_blocks": (c_int, [c_int]),
     "pcx_mvmr_plan_bytes": (c_size_t, [c_int64, c_int64, c_int, c_int]),
     "pcx_mvmr_plan_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int, c_int]),
@@ -56,6 +59,8 @@ SIGNATURES = {
     "pcx_mvmr_planned_workspace_bytes": (c_size_t, [c_int64, c_int]),
     "pcx_mvmr_planned": (c_int, [c_void_p] * 3 + [c_size_t, c_void_p] + [c_int64] * 3 + [c_int] * 6
                          + [c_int64, c_void_p, c_size_t, c_void_p]),
+    "pcx_mvmr_planned_bias": (c_int, [c_void_p] * 3 + [c_size_t] + [c_void_p] * 2 + [c_int64] * 3 + [c_int] * 6
+                              + [c_int64, c_void_p, c_size_t, c_void_p]),
     "pcx_debug_wait_runs_out": (c_int, [ctypes.c_ulonglong, c_void_p]),
     "pcx_vvor_workspace_bytes": (c_size_t, [c_int64, c_int, c_int, c_int, c_int]),
     "pcx_vvor": (c_int, [c_void_p] * 7 + [c_int64] * 4 + [c_int] * 5 + [c_void_p, c_size_t, c_void_p]),
@@ -127,6 +132,27 @@ def lib():
             fn.argtypes = args
         _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The compiled host path (``csrc/host.cpp``) of the hot operators; raises if it has not been built."""
+    global _host
+    if _host is None:
+        lib()
+        try:
+            from .lib import _pcx_host
+        except ImportError as exc:
+            raise RuntimeError("pointelligence_b200/lib/_pcx_host.so is missing or does not load: build it with "
+                               f"`python -m pointelligence_b200.build` ({exc})") from exc
+        _pcx_host.set_hooks(_plan_hook, is_symmetric, _differentiable_backward)
+        from .sparse_engines._dispatch_override import current_engine
+
+        _pcx_host.set_engine(current_engine())
+        _host = _pcx_host
+    return _host
 
 
 def check(rc):
@@ -402,21 +428,8 @@ def mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks):
     """Build the plan of a tap-sorted rulebook: ``scatter`` indexes the rows that are summed
     into (n_out of them), ``gather`` the rows that are read."""
     require_cuda(scatter, gather, seg_offs)
-    scatter, gather = as_i32(scatter), as_i32(gather)
-    seg_offs = seg_offs.to(torch.int64).contiguous()
-    dev, T, n_out, K, G = scatter.device, scatter.numel(), int(n_out), int(K), int(group_blocks)
-    L = lib()
-    nbytes = L.pcx_mvmr_plan_bytes(T, n_out, K, G)
-    if nbytes == 0:
-        raise NotImplementedError(f"no output-stationary plan for T={T} n_out={n_out} K={K} group={G}")
-    with torch.cuda.device(dev):
-        buf = workspace(nbytes, dev)
-        ws = workspace(L.pcx_mvmr_plan_workspace_bytes(T, n_out, K, G), dev)
-        check(L.pcx_mvmr_plan_build(ptr(scatter), ptr(gather), ptr(seg_offs), T, K, n_out, G, ptr(buf), buf.numel(),
-                                    ptr(ws), ws.numel(), stream_ptr()))
-        multi = c_int64(0)
-        check(L.pcx_mvmr_plan_multi_buckets(ptr(buf), ctypes.byref(multi), stream_ptr()))
-    return MvmrPlan(buf, T, K, n_out, G, int(multi.value))
+    buf, multi = host().plan_build(scatter, gather, seg_offs, int(K), int(n_out), int(group_blocks))
+    return MvmrPlan(buf, scatter.numel(), int(K), int(n_out), int(group_blocks), multi)
 
 
 _PLAN_CACHE = {}
@@ -475,16 +488,8 @@ def mvmr_planned(weight, feat, plan, transpose):
     require_cuda(weight, feat)
     K, G, C, M = weight.shape
     assert G == 1 and K == plan.K and weight.dtype == feat.dtype, (weight.shape, plan.K, weight.dtype, feat.dtype)
-    weight, feat = weight.contiguous(), feat.contiguous()
-    inw, outw = (M, C) if transpose else (C, M)
-    out = torch.empty((plan.n_out, outw), dtype=feat.dtype, device=feat.device)
-    L = lib()
-    with torch.cuda.device(feat.device):
-        ws = workspace(L.pcx_mvmr_planned_workspace_bytes(plan.multi_buckets, inw), feat.device)
-        check(L.pcx_mvmr_planned(ptr(weight), ptr(feat), ptr(plan.buffer), plan.buffer.numel(), ptr(out), plan.T,
-                                 feat.shape[0], plan.n_out, K, C, M, int(bool(transpose)), dtype_code(feat.dtype),
-                                 plan.group_blocks, plan.multi_buckets, ptr(ws), ws.numel(), stream_ptr()))
-    return out
+    return host().planned(weight, feat, plan.buffer, plan.group_blocks, plan.multi_buckets, plan.T, plan.n_out,
+                          bool(transpose))
 
 
 def debug_wait_runs_out(limit_ns=1_000_000):
@@ -499,35 +504,27 @@ def mvmr(weight, feat, gather, scatter, seg_offs, tap_idx, n_out, transpose, eng
     automatic engine, wide rows and dense neighbourhoods take the output-stationary kernel
     (``ENGINE_PLANNED`` forces it), everything else the scatter engines of ``pcx_mvmr``.
     """
-    require_cuda(weight, feat, gather, scatter, seg_offs, tap_idx)
-    K, G, C, M = weight.shape
-    code = dtype_code(feat.dtype)
-    assert weight.dtype == feat.dtype, (weight.dtype, feat.dtype)
-    weight, feat = weight.contiguous(), feat.contiguous()
-    n_out = int(n_out)
-    if engine in (ENGINE_AUTO, ENGINE_PLANNED):
-        fits = planned_supported(weight, feat, gather, scatter, seg_offs, n_out, transpose)
-        if engine == ENGINE_PLANNED and not fits:
-            raise NotImplementedError("the output-stationary engine needs fp16/bf16 features, one group, tap-sorted "
-                                      "triplets, channel counts that are multiples of 16 and rows of at most 256 channels")
-        outw = C if transpose else M
-        if fits and (engine == ENGINE_PLANNED or _planned_pays(gather.numel(), n_out, outw, K)):
-            plan = cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, plan_group_blocks(outw))
-            return mvmr_planned(weight, feat, plan, transpose)
-        engine = ENGINE_AUTO
-    gather, scatter, tap_idx = as_i32(gather), as_i32(scatter), as_i32(tap_idx)
-    if seg_offs is not None:
-        seg_offs = seg_offs.to(torch.int64).contiguous()
-    outw = C if transpose else M
-    out = torch.empty((n_out, G * outw), dtype=feat.dtype, device=feat.device)
-    L = lib()
-    with torch.cuda.device(feat.device):
-        nbytes = L.pcx_mvmr_workspace_bytes(n_out, K, G, C, M, int(bool(transpose)), code)
-        ws = workspace(nbytes, feat.device)
-        check(L.pcx_mvmr(ptr(weight), ptr(feat), ptr(gather), ptr(scatter), ptr(seg_offs), ptr(tap_idx),
-                         ptr(out), gather.numel(), feat.shape[0], n_out, K, G, C, M,
-                         int(bool(transpose)), code, engine, ptr(ws), ws.numel(), stream_ptr()))
-    return out
+    return host().mvmr(weight, feat, gather, scatter, seg_offs, tap_idx, int(n_out), bool(transpose), int(engine))
+
+
+def _plan_hook(scatter, gather, seg_offs, K, n_out, outw, inw, forced):
+    """Asked by the host path for every pass the output-stationary kernel could take: the plan to run
+    (buffer, blocks per group, multi-triplet buckets) or None for the scatter engine."""
+    if not forced and not _planned_pays(gather.numel(), n_out, outw, K):
+        return None
+    plan = cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, plan_group_blocks(outw))
+    return plan.buffer, plan.group_blocks, plan.multi_buckets
+
+
+def _differentiable_backward(weight, feat, grad, i, j, seg_offs, n_out, n_in, K, cover_out, cover_in, want_w, want_x,
+                             want_b):
+    """Gradients of a convolution as differentiable operators (``create_graph=True``)."""
+    from .sparse_engines import tig
+
+    index = tig.TigIndex.from_flat(i, j, seg_offs, n_out, n_in, K, cover_out, cover_in)
+    gw = tig.tig_grad_weight(feat, grad, index, weight.shape).to(weight.dtype) if want_w else None
+    gf = tig.tig_grad_input(weight, grad, index).to(feat.dtype) if want_x else None
+    return gw, gf, (grad.sum(0) if want_b else None)
 
 
 def prepare_mvmr(weight, gather, scatter, seg_offs, n_out, transpose=False):
@@ -552,23 +549,7 @@ def vvor(a, a_idx, b, b_idx, seg_offs, o_idx, n_o, engine=ENGINE_AUTO):
 
     a (n_a, G, Ma); b (n_b, G, Cb); returns (n_o, G, Ma, Cb) in a.dtype.
     """
-    require_cuda(a, b, a_idx, b_idx, seg_offs, o_idx)
-    code = dtype_code(a.dtype)
-    assert a.dtype == b.dtype, (a.dtype, b.dtype)
-    a, b = a.contiguous(), b.contiguous()
-    G, Ma, Cb = a.shape[1], a.shape[2], b.shape[2]
-    a_idx, b_idx, o_idx = as_i32(a_idx), as_i32(b_idx), as_i32(o_idx)
-    if seg_offs is not None:
-        seg_offs = seg_offs.to(torch.int64).contiguous()
-    n_o = int(n_o)
-    out = torch.empty((n_o, G, Ma, Cb), dtype=a.dtype, device=a.device)
-    L = lib()
-    with torch.cuda.device(a.device):
-        ws = workspace(L.pcx_vvor_workspace_bytes(n_o, G, Ma, Cb, code), a.device)
-        check(L.pcx_vvor(ptr(a), ptr(a_idx), ptr(b), ptr(b_idx), ptr(seg_offs), ptr(o_idx), ptr(out),
-                         a_idx.numel(), a.shape[0], b.shape[0], n_o, G, Ma, Cb, code, engine,
-                         ptr(ws), ws.numel(), stream_ptr()))
-    return out
+    return host().vvor(a, a_idx, b, b_idx, seg_offs, o_idx, int(n_o), int(engine))
 
 
 def vvor_static_scratch(a, a_idx, b, b_idx, seg_offs, out):
@@ -667,45 +648,13 @@ def _f32_or_none(t):
 
 def ragged_layer_norm(x, lengths, weight, bias, residual, eps, relu):
     """Fused ``relu?(layer_norm_per_sample(x) * weight + bias (+ residual))``; returns ``(y, mean, rstd)``."""
-    require_cuda(x, lengths, weight, bias, residual)
-    x = x.contiguous()
-    lengths = lengths.to(torch.int64).contiguous()
-    weight, bias = _f32_or_none(weight), _f32_or_none(bias)
-    residual = None if residual is None else residual.to(x.dtype).contiguous()
-    N, C = x.shape
-    S = lengths.numel()
-    y = torch.empty_like(x)
-    mean = torch.empty(S, dtype=torch.float32, device=x.device)
-    rstd = torch.empty(S, dtype=torch.float32, device=x.device)
-    L = lib()
-    with torch.cuda.device(x.device):
-        ws = workspace(L.pcx_ragged_layer_norm_workspace_bytes(N, S), x.device)
-        check(L.pcx_ragged_layer_norm(ptr(x), ptr(lengths), ptr(weight), ptr(bias), ptr(residual), ptr(y), ptr(mean),
-                                      ptr(rstd), N, S, C, float(eps), int(bool(relu)), dtype_code(x.dtype), ptr(ws),
-                                      ws.numel(), stream_ptr()))
-    return y, mean, rstd
+    return host().layer_norm_forward(x, lengths, weight, bias, residual, float(eps), bool(relu))
 
 
 def ragged_layer_norm_backward(grad_y, x, y, lengths, weight, mean, rstd, relu, want_affine, want_residual):
     """Returns ``(grad_x, grad_weight|None, grad_bias|None, grad_residual|None)`` (affine gradients in fp32)."""
-    require_cuda(grad_y, x, lengths)
-    grad_y, x = grad_y.contiguous(), x.contiguous()
-    lengths = lengths.to(torch.int64).contiguous()
-    weight = _f32_or_none(weight)
-    N, C = x.shape
-    S = lengths.numel()
-    grad_x = torch.empty_like(x)
-    gw = torch.empty(C, dtype=torch.float32, device=x.device) if want_affine else None
-    gb = torch.empty(C, dtype=torch.float32, device=x.device) if want_affine else None
-    gres = torch.empty_like(x) if want_residual else None
-    L = lib()
-    with torch.cuda.device(x.device):
-        ws = workspace(L.pcx_ragged_layer_norm_workspace_bytes(N, S), x.device)
-        check(L.pcx_ragged_layer_norm_backward(ptr(grad_y), ptr(x), ptr(y), ptr(lengths), ptr(weight), ptr(mean),
-                                               ptr(rstd), ptr(grad_x), ptr(gw), ptr(gb), ptr(gres), N, S, C,
-                                               int(bool(relu)), dtype_code(x.dtype), ptr(ws), ws.numel(),
-                                               stream_ptr()))
-    return grad_x, gw, gb, gres
+    return host().layer_norm_backward(grad_y, x, y, lengths, weight, mean, rstd, bool(relu), bool(want_affine),
+                                      bool(want_residual))
 
 
 def ragged_group_norm(x, lengths, weight, bias, groups, eps):
@@ -857,66 +806,22 @@ def _radius_taps(points, queries, radius, ps, qs, distance_type, kernel_size, ke
     """Tap-segmented search through ``pcx_radius_taps_*``: the pairs are written into buffers sized
     from the density of earlier searches (exactly sized after a counted first call or when the
     estimate turns out too small) and returned as views of the first ``total`` entries."""
-    dev = points.device
-    P, Q = points.shape[0], queries.shape[0]
-    L = lib()
-    k3 = kernel_size ** 3
-    with torch.cuda.device(dev):
-        ws = workspace(L.pcx_radius_taps_workspace_bytes(P, Q, kernel_size), dev)
-        num_neighbors = torch.empty(Q, dtype=torch.int64, device=dev)
-        seg = torch.empty(k3 + 1, dtype=torch.int64, device=dev)
-        check(L.pcx_radius_taps_count(ptr(points), ptr(queries), ptr(ps), ptr(qs), P, Q, float(radius),
-                                      distance_type, kernel_size, float(kernel_grid_size), ptr(num_neighbors),
-                                      ptr(seg), ptr(ws), ws.numel(), stream_ptr()))
-        total = (c_int64 * 3)()
-        ratio_key = (kernel_size, distance_type, float(radius))
-        ratio = _TAPS_RATIO.get(ratio_key)
-        if ratio is None:
-            check(L.pcx_radius_taps_total(P, Q, kernel_size, total, ptr(ws), ws.numel(), stream_ptr()))
-            capacity = int(total[0])
-        else:
-            capacity = min(int(ratio * Q * 1.25) + 4096, 2 ** 31 - 1)
-        for attempt in range(2):
-            out_i = torch.empty(capacity, dtype=torch.int32, device=dev)
-            out_j = torch.empty(capacity, dtype=torch.int32, device=dev)
-            out_k = torch.empty(capacity, dtype=torch.int32, device=dev) if want_k else None
-            rc = L.pcx_radius_taps_fill(ptr(queries), ptr(ps), ptr(qs), P, Q, float(radius), distance_type,
-                                        kernel_size, float(kernel_grid_size), capacity, ptr(out_i), ptr(out_j),
-                                        ptr(out_k), total, ptr(ws), ws.numel(), stream_ptr())
-            if rc == PCX_E_CAPACITY and attempt == 0 and int(total[0]) > capacity:
-                capacity = int(total[0])   # the estimate was too small: exact size, fill pass only
-                continue
-            check(rc)
-            break
-        if total[2]:                 # the hand-over of the fill pass brought the status word along
-            raise_if_device_reported()
-        n = int(total[0])
-        if len(_TAPS_RATIO) > 256:
-            _TAPS_RATIO.clear()
-        _TAPS_RATIO[ratio_key] = max(ratio or 0.0, n / Q)
-        num_neighbors.pcx_queries_without_neighbor = int(total[1])   # spares the caller a pass over the counts
-    return out_i[:n], out_j[:n], (out_k[:n] if want_k else None), seg, num_neighbors
+    ratio_key = (kernel_size, distance_type, float(radius))
+    ratio = _TAPS_RATIO.get(ratio_key)
+    i, j, k, seg, num_neighbors, n, lonely, status = host().radius_taps(
+        points, queries, float(radius), ps, qs, distance_type, kernel_size, float(kernel_grid_size), want_k,
+        -1.0 if ratio is None else ratio)
+    if status:                 # the hand-over of the fill pass brought the status word along
+        raise_if_device_reported()
+    if len(_TAPS_RATIO) > 256:
+        _TAPS_RATIO.clear()
+    _TAPS_RATIO[ratio_key] = max(ratio or 0.0, n / queries.shape[0])
+    num_neighbors.pcx_queries_without_neighbor = lonely   # spares the caller a pass over the counts
+    return i, j, k, seg, num_neighbors
 
 
 @on_geometry_stream
 def grid_sample_center_nearest(points, cell, sample, return_mapping):
     """Returns ``(indices int64 (S,), points_f (S,3), sample_f int32 (S,)|None, mapping int64|None)``."""
     require_cuda(points, sample)
-    dev = points.device
-    points = points.contiguous()
-    smp = as_i32(sample)
-    N = points.shape[0]
-    L = lib()
-    with torch.cuda.device(dev):
-        ws = workspace(L.pcx_grid_sample_workspace_bytes(N), dev)
-        ncells = c_int64(0)
-        check(L.pcx_grid_sample_count(ptr(points), ptr(smp), N, float(cell), ctypes.byref(ncells), ptr(ws),
-                                      ws.numel(), stream_ptr()))
-        S = int(ncells.value)
-        indices = torch.empty(S, dtype=torch.int64, device=dev)
-        out_pts = torch.empty((S, 3), dtype=torch.float32, device=dev)
-        out_smp = torch.empty(S, dtype=torch.int32, device=dev) if smp is not None else None
-        mapping = torch.empty(N, dtype=torch.int64, device=dev) if return_mapping else None
-        check(L.pcx_grid_sample_select(ptr(points), ptr(smp), N, float(cell), S, ptr(indices), ptr(out_pts),
-                                       ptr(out_smp), ptr(mapping), ptr(ws), ws.numel(), stream_ptr()))
-    return indices, out_pts, out_smp, mapping
+    return host().grid_sample(points, float(cell), sample, bool(return_mapping))

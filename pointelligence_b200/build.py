@@ -19,8 +19,9 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "lib", "obj")
 LIB = os.path.join(HERE, "lib", "libpointelligence_b200.so")
+HOST = os.path.join(HERE, "lib", "_pcx_host.so")   # CPython module: host path of the hot operators over the C ABI
 SOURCES = ("status.cu", "geometry.cu", "sparse_generic.cu", "sparse_tc.cu", "sparse_api.cu",
-           "sparse_noalloc.cu", "segment_reduce.cu", "ragged_norm.cu", "mvmr_os.cu", "rnet.cu", "radius_taps.cu")
+           "sparse_noalloc.cu", "segment_reduce.cu", "ragged_norm.cu", "mvmr_os.cu", "rnet.cu", "radius_taps.cu", "columns.cu")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
          "-Xcompiler", "-fPIC", "-Xptxas", "-v"] + os.environ.get("PCX_NVCC_EXTRA", "").split()
@@ -39,9 +40,13 @@ def _stale(target, deps):
     return any(os.path.getmtime(d) > t for d in deps)
 
 
-def _compile(src):
+def _compile(src, force=False):
     obj = os.path.join(OBJ, src.replace(".cu", ".o"))
     log = obj + ".log"
+    headers = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh")]
+    headers.append(os.path.join(os.path.dirname(HERE), "include", "pointelligence_b200.h"))
+    if not force and not _stale(obj, [os.path.join(CSRC, src), *headers]):
+        return obj
     cmd = [NVCC, *FLAGS, "-c", os.path.join(CSRC, src), "-o", obj]
     r = subprocess.run(cmd, capture_output=True, text=True)
     with open(log, "w") as f:
@@ -51,13 +56,32 @@ def _compile(src):
     return obj
 
 
+def _build_host():
+    """The CPython module (csrc/host.cpp): plain C++ against PyTorch's headers, linked to the library."""
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")
+    includes = [f for d in cpp_extension.include_paths() + [sysconfig.get_paths()["include"], "/usr/local/cuda/include"]
+                for f in ("-isystem", d)]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_pcx_host",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *includes, os.path.join(CSRC, "host.cpp"),
+           "-o", HOST, "-L" + os.path.dirname(LIB), "-lpointelligence_b200", "-L" + torch_lib, "-ltorch", "-ltorch_cpu",
+           "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN", "-Wl,-rpath," + torch_lib]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("g++ failed for host.cpp:\n" + r.stderr[-4000:])
+
+
 def build(force=False, verbose=False):
     deps = _deps()
-    if not force and not _stale(LIB, deps):
+    if not force and not _stale(LIB, deps) and not _stale(HOST, deps):
         return LIB
     os.makedirs(OBJ, exist_ok=True)
     with ThreadPoolExecutor(max_workers=len(SOURCES)) as ex:
-        objs = list(ex.map(_compile, SOURCES))
+        objs = list(ex.map(lambda src: _compile(src, force), SOURCES))
     rpaths = ["/usr/local/cuda/lib64"]
     try:
         import nvidia.cuda_runtime  # the runtime PyTorch loads
@@ -71,6 +95,9 @@ def build(force=False, verbose=False):
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("link failed:\n" + r.stderr[-4000:])
+    if force or _stale(HOST, [os.path.join(CSRC, "host.cpp"), deps[-1]]):
+        _build_host()
+    os.utime(HOST)
     if verbose:
         print("built", LIB)
     return LIB

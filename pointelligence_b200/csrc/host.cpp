@@ -1,0 +1,508 @@
+// Host path of the hot operators: argument checks, output and workspace allocation, the C-ABI
+// calls and the autograd nodes of the convolution and the ragged layer norm, compiled.
+//
+// The kernels live behind the C ABI (include/pointelligence_b200.h).  What this file replaces is the
+// interpreter between a layer's forward() and those entry points: a training pass of one layer
+// through Python operators, Python autograd and ctypes marshalling cost 0.5-0.6 ms of host time on
+// B200 boxes (150 000 points, 64 channels: 0.54 ms per pass for 0.29 ms of kernels); small layers and
+// whole networks on small scenes were bound by it.  The policy that needs Python objects -- which
+// engine a rulebook takes, the plans remembered per rulebook -- stays in Python and is asked through
+// two hooks (set_hooks), once per convolution pass.
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/extension.h>
+
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+
+#include "../../include/pointelligence_b200.h"
+
+namespace py = pybind11;
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+
+namespace {
+
+// ------------------------------------------------------------------ helpers ----
+PyObject *g_plan_hook = nullptr;       // (scatter, gather, seg, K, n_out, out_width, in_width, forced) -> None | plan tuple
+PyObject *g_symmetric_hook = nullptr;  // (i, j) -> bool
+PyObject *g_double_backward = nullptr; // differentiable backward of the convolution (create_graph)
+
+[[noreturn]] void raise(PyObject *type, const std::string &msg) {
+    PyErr_SetString(type, msg.c_str());
+    throw py::error_already_set();
+}
+
+// C-ABI status -> the exception type the ctypes binding raises for it
+void check(int rc) {
+    if (rc == PCX_OK) return;
+    PyObject *type = PyExc_RuntimeError;
+    if (rc == PCX_E_ARG || rc == PCX_E_ALIGN) type = PyExc_ValueError;
+    else if (rc == PCX_E_DTYPE) type = PyExc_TypeError;
+    else if (rc == PCX_E_UNSUPPORTED) type = PyExc_NotImplementedError;
+    const std::string msg = std::string(pcx_last_error_string()) + " [pcx status " + std::to_string(rc) + "]";
+    py::gil_scoped_acquire gil;
+    raise(type, msg);
+}
+
+void require_cuda(const Tensor &t) {
+    if (t.defined() && !t.is_cuda()) {
+        py::gil_scoped_acquire gil;
+        raise(PyExc_RuntimeError, "pointelligence_b200 operators run on CUDA tensors only (no CPU fallback); got a tensor on " +
+                                      t.device().str());
+    }
+}
+void require_cuda(const OptTensor &t) {
+    if (t) require_cuda(*t);
+}
+
+int dtype_code(at::ScalarType t) {
+    switch (t) {
+        case at::kFloat: return PCX_F32;
+        case at::kHalf: return PCX_F16;
+        case at::kBFloat16: return PCX_BF16;
+        default: break;
+    }
+    py::gil_scoped_acquire gil;
+    raise(PyExc_TypeError, std::string("unsupported feature dtype torch.") + c10::toString(t) +
+                               "; expected float32, float16 or bfloat16");
+}
+
+Tensor as_i32(const Tensor &t) { return t.scalar_type() == at::kInt ? t.contiguous() : t.to(at::kInt).contiguous(); }
+Tensor as_i64(const Tensor &t) { return t.scalar_type() == at::kLong ? t.contiguous() : t.to(at::kLong).contiguous(); }
+
+Tensor workspace(size_t bytes, const Tensor &like) {
+    return at::empty({(int64_t)std::max<size_t>(bytes, 256)}, at::TensorOptions().dtype(at::kByte).device(like.device()));
+}
+void *stream() { return (void *)at::cuda::getCurrentCUDAStream().stream(); }
+void *ptr(const Tensor &t) { return t.defined() ? t.data_ptr() : nullptr; }
+template <typename T>
+T *ptr_as(const Tensor &t) { return t.defined() ? static_cast<T *>(t.data_ptr()) : nullptr; }
+
+// --------------------------------------------------------------------- MVMR ----
+// Plan of the output-stationary kernel as the hook returns it.
+struct Plan {
+    Tensor buffer;
+    int64_t group = 0, multi = 0;
+    bool valid = false;
+};
+
+Plan ask_plan(const Tensor &scatter, const Tensor &gather, const Tensor &seg, int64_t K, int64_t n_out, int64_t outw,
+              int64_t inw, bool forced) {
+    Plan plan;
+    py::gil_scoped_acquire gil;
+    py::object r = py::reinterpret_borrow<py::object>(g_plan_hook)(scatter, gather, seg, K, n_out, outw, inw, forced);
+    if (!r.is_none()) {
+        py::tuple t = py::cast<py::tuple>(r);
+        plan.buffer = py::cast<Tensor>(t[0]);
+        plan.group = py::cast<int64_t>(t[1]);
+        plan.multi = py::cast<int64_t>(t[2]);
+        plan.valid = true;
+    }
+    return plan;
+}
+
+// Shapes and types the output-stationary kernel takes (one group, 16-bit elements, widths in sixteens).
+bool plan_fits(at::ScalarType dtype, int64_t T, int64_t n_out, int64_t K, int64_t G, int64_t inw, int64_t outw, bool has_seg) {
+    if (G != 1 || !has_seg || (dtype != at::kHalf && dtype != at::kBFloat16) || n_out <= 0) return false;
+    if (inw % 16 || outw % 16 || outw > 256 || inw > 1024 || K > 512) return false;
+    const int64_t nblocks = (n_out + 127) / 128;
+    return T < (int64_t(1) << 31) && nblocks * K * 128 <= (int64_t(1) << 32);
+}
+
+constexpr int ENGINE_PLANNED = 3;
+
+Tensor mvmr_planned(const Tensor &weight, const Tensor &feat, const Plan &plan, int64_t T, int64_t n_out, int flags,
+                    const Tensor &bias) {
+    const int64_t K = weight.size(0), C = weight.size(2), M = weight.size(3);
+    const bool transpose = flags & 1;
+    const int64_t inw = transpose ? M : C, outw = transpose ? C : M;
+    Tensor out = at::empty({n_out, outw}, feat.options());
+    const size_t bytes = pcx_mvmr_planned_workspace_bytes(plan.multi, (int)inw);
+    Tensor ws = workspace(bytes, feat);
+    check(pcx_mvmr_planned_bias(ptr(weight), ptr(feat), ptr(plan.buffer), plan.buffer.numel(), ptr(bias), ptr(out), T, feat.size(0),
+                                n_out, (int)K, (int)C, (int)M, flags, dtype_code(feat.scalar_type()), (int)plan.group, plan.multi,
+                                ptr(ws), ws.numel(), stream()));
+    return out;
+}
+
+// out[scatter[t]] += feat[gather[t]] @ W[tap(t)] (+ bias).  flags: 1 = W transposed, 2 = taps of the weight
+// in reverse order.  Rows of the result are (G * out width) in feat's type.
+Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor &scatter_, const OptTensor &seg_,
+                 const OptTensor &tap_, int64_t n_out, int flags, int64_t engine, const Tensor &bias) {
+    require_cuda(weight), require_cuda(feat), require_cuda(gather_), require_cuda(scatter_);
+    require_cuda(seg_), require_cuda(tap_);
+    const int code = dtype_code(feat.scalar_type());
+    TORCH_CHECK(weight.scalar_type() == feat.scalar_type(), "weight and features differ in type");
+    weight = weight.contiguous(), feat = feat.contiguous();
+    const int64_t K = weight.size(0), G = weight.size(1), C = weight.size(2), M = weight.size(3);
+    const bool transpose = flags & 1;
+    const int64_t inw = transpose ? M : C, outw = transpose ? C : M, T = gather_.numel();
+    c10::cuda::CUDAGuard guard(feat.device());
+    if (engine == 0 || engine == ENGINE_PLANNED) {
+        const bool fits = plan_fits(feat.scalar_type(), T, n_out, K, G, inw, outw, seg_.has_value());
+        if (engine == ENGINE_PLANNED && !fits) {
+            py::gil_scoped_acquire gil;
+            raise(PyExc_NotImplementedError,
+                  "the output-stationary engine needs fp16/bf16 features, one group, tap-sorted triplets, channel counts "
+                  "that are multiples of 16 and rows of at most 256 channels");
+        }
+        if (fits && (K > 1 || engine == ENGINE_PLANNED)) {
+            const Plan plan = ask_plan(scatter_, gather_, *seg_, K, n_out, outw, inw, engine == ENGINE_PLANNED);
+            if (plan.valid) return mvmr_planned(weight, feat, plan, T, n_out, flags, bias);
+        }
+        engine = 0;
+    }
+    const Tensor gather = as_i32(gather_), scatter = as_i32(scatter_);
+    const Tensor tap = tap_ ? as_i32(*tap_) : Tensor(), seg = seg_ ? as_i64(*seg_) : Tensor();
+    Tensor out = at::empty({n_out, G * outw}, feat.options());
+    Tensor ws = workspace(pcx_mvmr_workspace_bytes(n_out, (int)K, (int)G, (int)C, (int)M, transpose, code), feat);
+    check(pcx_mvmr_bias(ptr(weight), ptr(feat), ptr_as<int32_t>(gather), ptr_as<int32_t>(scatter), ptr_as<int64_t>(seg),
+                        ptr_as<int32_t>(tap), ptr(bias), ptr(out), T, feat.size(0), n_out, (int)K, (int)G, (int)C, (int)M, flags,
+                        code, (int)engine, ptr(ws), ws.numel(), stream()));
+    return out;
+}
+
+Tensor mvmr(const Tensor &weight, const Tensor &feat, const Tensor &gather, const Tensor &scatter, const OptTensor &seg,
+            const OptTensor &tap, int64_t n_out, bool transpose, int64_t engine) {
+    return mvmr_impl(weight, feat, gather, scatter, seg, tap, n_out, transpose ? 1 : 0, engine, Tensor());
+}
+
+// --------------------------------------------------------------------- VVOR ----
+Tensor vvor(Tensor a, const Tensor &a_idx_, Tensor b, const Tensor &b_idx_, const OptTensor &seg_, const OptTensor &o_idx_,
+            int64_t n_o, int64_t engine) {
+    require_cuda(a), require_cuda(b), require_cuda(a_idx_), require_cuda(b_idx_), require_cuda(seg_), require_cuda(o_idx_);
+    const int code = dtype_code(a.scalar_type());
+    TORCH_CHECK(a.scalar_type() == b.scalar_type(), "operands differ in type");
+    a = a.contiguous(), b = b.contiguous();
+    const int64_t G = a.size(1), Ma = a.size(2), Cb = b.size(2);
+    c10::cuda::CUDAGuard guard(a.device());
+    const Tensor a_idx = as_i32(a_idx_), b_idx = as_i32(b_idx_), o_idx = o_idx_ ? as_i32(*o_idx_) : Tensor(),
+                 seg = seg_ ? as_i64(*seg_) : Tensor();
+    Tensor out = at::empty({n_o, G, Ma, Cb}, a.options());
+    Tensor ws = workspace(pcx_vvor_workspace_bytes(n_o, (int)G, (int)Ma, (int)Cb, code), a);
+    check(pcx_vvor(ptr(a), ptr_as<int32_t>(a_idx), ptr(b), ptr_as<int32_t>(b_idx), ptr_as<int64_t>(seg), ptr_as<int32_t>(o_idx),
+                   ptr(out), a_idx.numel(), a.size(0), b.size(0), n_o, (int)G, (int)Ma, (int)Cb, code, (int)engine, ptr(ws),
+                   ws.numel(), stream()));
+    return out;
+}
+
+Tensor column_sums(const Tensor &x_) {
+    const Tensor x = x_.contiguous();
+    c10::cuda::CUDAGuard guard(x.device());
+    const int64_t N = x.size(0), C = x.size(1);
+    Tensor out = at::empty({C}, x.options());
+    Tensor ws = workspace(pcx_column_sums_workspace_bytes(N, (int)C), x);
+    check(pcx_column_sums(ptr(x), ptr(out), N, (int)C, dtype_code(x.scalar_type()), ptr(ws), ws.numel(), stream()));
+    return out;
+}
+
+// ------------------------------------------------------- convolution (autograd) ----
+std::atomic<int> g_engine{0};   // engine of the current dispatch mode (0 automatic, 1 CUDA cores)
+
+constexpr int64_t FAN_IN_ONE = PCX_ENGINE_FLAG_FAN_IN_ONE;
+
+bool is_symmetric(const Tensor &i, const Tensor &j) {
+    py::gil_scoped_acquire gil;
+    return py::cast<bool>(py::reinterpret_borrow<py::object>(g_symmetric_hook)(i, j));
+}
+
+void match(Tensor &w, Tensor &x) {
+    if (w.scalar_type() == x.scalar_type()) return;
+    const auto t = c10::promoteTypes(w.scalar_type(), x.scalar_type());
+    w = w.to(t), x = x.to(t);
+}
+
+struct ConvSizes {
+    int64_t n_out, n_in, K;
+    bool cover_out, cover_in;
+};
+
+Tensor as4(const Tensor &w) { return w.dim() == 4 ? w : w.unsqueeze(1); }
+
+Tensor conv_forward(const Tensor &weight, const Tensor &feat, const Tensor &bias, const Tensor &i, const Tensor &j,
+                    const Tensor &seg, const ConvSizes &s) {
+    Tensor w = as4(weight), x = feat;
+    TORCH_CHECK(w.size(0) == s.K && x.dim() == 2 && x.size(1) == w.size(1) * w.size(2), "features ", x.sizes(),
+                " do not fit a weight ", weight.sizes(), " of ", s.K, " taps");
+    TORCH_CHECK(x.size(0) == s.n_in, "feat rows ", x.size(0), " != index.N_in ", s.n_in);
+    match(w, x);
+    int64_t engine = g_engine;
+    if (s.cover_out && i.numel() == s.n_out) engine |= FAN_IN_ONE;   // one triplet per output row: stored, not reduced
+    return mvmr_impl(w, x, j, i, seg, std::nullopt, s.n_out, 0, engine, bias).to(feat.scalar_type());
+}
+
+Tensor conv_grad_input(const Tensor &weight, const Tensor &grad, const Tensor &i, const Tensor &j, const Tensor &seg,
+                       const ConvSizes &s) {
+    Tensor w = as4(weight), g = grad;
+    match(w, g);
+    int64_t engine = g_engine;
+    // a self-search rulebook holds (j, i, K - 1 - k) with every (i, j, k): the input gradient is the forward
+    // schedule over the same rulebook (and the same plan) with the taps of the weight in reverse order
+    if (s.n_out == s.n_in && is_symmetric(i, j))
+        return mvmr_impl(w, g, j, i, seg, std::nullopt, s.n_in, 3, engine, Tensor()).to(grad.scalar_type());
+    if (s.cover_in && i.numel() == s.n_in) engine |= FAN_IN_ONE;
+    return mvmr_impl(w, g, i, j, seg, std::nullopt, s.n_in, 1, engine, Tensor()).to(grad.scalar_type());
+}
+
+Tensor conv_grad_weight(const Tensor &feat, const Tensor &grad, const Tensor &i, const Tensor &j, const Tensor &seg,
+                        at::IntArrayRef weight_shape, const ConvSizes &s) {
+    const int64_t G = weight_shape.size() == 4 ? weight_shape[1] : 1;
+    Tensor x = feat, g = grad;
+    match(x, g);
+    return vvor(x.view({x.size(0), G, -1}), j, g.view({g.size(0), G, -1}), i, seg, std::nullopt, s.K, g_engine)
+        .to(feat.scalar_type())
+        .view(weight_shape);
+}
+
+// out[i] += feat[j] @ W[k] (+ bias), with its three gradients; one node of the autograd graph.
+struct Conv : public torch::autograd::Function<Conv> {
+    static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &weight, const Tensor &feat, const OptTensor &bias,
+                          const Tensor &i, const Tensor &j, const Tensor &seg, int64_t n_out, int64_t n_in, int64_t K,
+                          bool cover_out, bool cover_in) {
+        ctx->save_for_backward({weight, feat, i, j, seg});
+        ctx->saved_data["sizes"] = std::vector<int64_t>{n_out, n_in, K, cover_out, cover_in, bias.has_value()};
+        return conv_forward(weight, feat, bias ? *bias : Tensor(), i, j, seg, {n_out, n_in, K, cover_out, cover_in});
+    }
+
+    static torch::autograd::variable_list backward(torch::autograd::AutogradContext *ctx, torch::autograd::variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &weight = saved[0], &feat = saved[1], &i = saved[2], &j = saved[3], &seg = saved[4];
+        const auto v = ctx->saved_data["sizes"].toIntVector();
+        const ConvSizes s{v[0], v[1], v[2], v[3] != 0, v[4] != 0};
+        torch::autograd::variable_list out(11);
+        if (!grads[0].defined()) return out;
+        const Tensor &go = grads[0];
+        const bool want_w = ctx->needs_input_grad(0), want_x = ctx->needs_input_grad(1), want_b = v[5] && ctx->needs_input_grad(2);
+        if (at::GradMode::is_enabled()) {   // create_graph: the gradients themselves have to be differentiable
+            py::gil_scoped_acquire gil;
+            py::tuple r = py::cast<py::tuple>(py::reinterpret_borrow<py::object>(g_double_backward)(
+                weight, feat, go, i, j, seg, s.n_out, s.n_in, s.K, s.cover_out, s.cover_in, want_w, want_x, want_b));
+            for (int q = 0; q < 3; ++q)
+                if (!r[q].is_none()) out[q] = py::cast<Tensor>(r[q]);
+            return out;
+        }
+        const Tensor g = go.contiguous();
+        c10::cuda::CUDAGuard guard(g.device());
+        if (want_b) out[2] = column_sums(g);
+        if (want_w) out[0] = conv_grad_weight(feat, g, i, j, seg, weight.sizes(), s).to(weight.scalar_type());
+        if (want_x) out[1] = conv_grad_input(weight, g, i, j, seg, s).to(feat.scalar_type());
+        return out;
+    }
+};
+
+Tensor conv(const Tensor &weight, const Tensor &feat, const OptTensor &bias, const Tensor &i, const Tensor &j, const Tensor &seg,
+            int64_t n_out, int64_t n_in, int64_t K, bool cover_out, bool cover_in) {
+    if (!at::GradMode::is_enabled() ||
+        !(weight.requires_grad() || feat.requires_grad() || (bias && bias->requires_grad())))
+        return conv_forward(weight, feat, bias ? *bias : Tensor(), i, j, seg, {n_out, n_in, K, cover_out, cover_in});
+    return Conv::apply(weight, feat, bias, i, j, seg, n_out, n_in, K, cover_out, cover_in);
+}
+
+// --------------------------------------------------- ragged layer norm (autograd) ----
+Tensor f32_or_none(const OptTensor &t) { return t ? t->detach().to(at::kFloat).contiguous() : Tensor(); }
+
+std::tuple<Tensor, Tensor, Tensor> layer_norm_forward(Tensor x, const Tensor &lengths_, const OptTensor &weight_,
+                                                      const OptTensor &bias_, const OptTensor &residual_, double eps, bool relu) {
+    require_cuda(x), require_cuda(lengths_), require_cuda(weight_), require_cuda(bias_), require_cuda(residual_);
+    const int code = dtype_code(x.scalar_type());
+    c10::cuda::CUDAGuard guard(x.device());
+    x = x.contiguous();
+    const Tensor lengths = as_i64(lengths_), weight = f32_or_none(weight_), bias = f32_or_none(bias_);
+    const Tensor residual = residual_ ? residual_->to(x.scalar_type()).contiguous() : Tensor();
+    const int64_t N = x.size(0), C = x.size(1), S = lengths.numel();
+    Tensor y = at::empty_like(x);
+    Tensor stats = at::empty({2, S}, x.options().dtype(at::kFloat));
+    Tensor mean = stats.select(0, 0), rstd = stats.select(0, 1);
+    Tensor ws = workspace(pcx_ragged_layer_norm_workspace_bytes(N, S), x);
+    check(pcx_ragged_layer_norm(ptr(x), ptr_as<int64_t>(lengths), ptr_as<float>(weight), ptr_as<float>(bias), ptr(residual), ptr(y),
+                                ptr_as<float>(mean), ptr_as<float>(rstd), N, S, (int)C, eps, relu, code, ptr(ws), ws.numel(),
+                                stream()));
+    return {y, mean, rstd};
+}
+
+std::tuple<Tensor, Tensor, Tensor, Tensor> layer_norm_backward(Tensor grad_y, Tensor x, const Tensor &y, const Tensor &lengths_,
+                                                               const OptTensor &weight_, const Tensor &mean, const Tensor &rstd,
+                                                               bool relu, bool want_affine, bool want_residual) {
+    require_cuda(grad_y), require_cuda(x), require_cuda(lengths_);
+    const int code = dtype_code(x.scalar_type());
+    c10::cuda::CUDAGuard guard(x.device());
+    grad_y = grad_y.contiguous(), x = x.contiguous();
+    const Tensor lengths = as_i64(lengths_), weight = f32_or_none(weight_);
+    const int64_t N = x.size(0), C = x.size(1), S = lengths.numel();
+    Tensor gx = at::empty_like(x), gw, gb, gres;
+    if (want_affine) {
+        gw = at::empty({C}, x.options().dtype(at::kFloat));
+        gb = at::empty({C}, x.options().dtype(at::kFloat));
+    }
+    if (want_residual) gres = at::empty_like(x);
+    Tensor ws = workspace(pcx_ragged_layer_norm_workspace_bytes(N, S), x);
+    check(pcx_ragged_layer_norm_backward(ptr(grad_y), ptr(x), ptr(y), ptr_as<int64_t>(lengths), ptr_as<float>(weight),
+                                         ptr_as<float>(mean), ptr_as<float>(rstd), ptr(gx), ptr_as<float>(gw), ptr_as<float>(gb),
+                                         ptr(gres), N, S, (int)C, relu, code, ptr(ws), ws.numel(), stream()));
+    return {gx, gw, gb, gres};
+}
+
+struct LayerNorm : public torch::autograd::Function<LayerNorm> {
+    static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &x, const Tensor &lengths, const OptTensor &weight,
+                          const OptTensor &bias, const OptTensor &residual, double eps, bool relu) {
+        auto [y, mean, rstd] = layer_norm_forward(x, lengths, weight, bias, residual, eps, relu);
+        ctx->save_for_backward({x, y, lengths, weight ? *weight : Tensor(), mean, rstd});
+        ctx->saved_data["relu"] = relu;
+        // edges of the node exist for the tensors that were given: remember where theirs are (-1: none)
+        const int64_t at_weight = weight ? 2 : -1, at_bias = bias ? 2 + (weight ? 1 : 0) : -1;
+        const int64_t at_residual = residual ? 2 + (weight ? 1 : 0) + (bias ? 1 : 0) : -1;
+        ctx->saved_data["edges"] = std::vector<int64_t>{at_weight, at_bias, at_residual};
+        ctx->saved_data["bias_type"] = (int64_t)(bias ? bias->scalar_type() : at::kFloat);
+        ctx->saved_data["residual_type"] = (int64_t)(residual ? residual->scalar_type() : x.scalar_type());
+        return y;
+    }
+
+    static torch::autograd::variable_list backward(torch::autograd::AutogradContext *ctx, torch::autograd::variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        torch::autograd::variable_list out(7);
+        if (!grads[0].defined()) return out;
+        // as the Python node did: once differentiable (its backward is opaque to autograd)
+        at::AutoGradMode no_graph(false);
+        const auto edges = ctx->saved_data["edges"].toIntVector();
+        const auto needs = [&](int q) { return edges[q] >= 0 && ctx->needs_input_grad((size_t)edges[q]); };
+        const bool affine = saved[3].defined() && (needs(0) || needs(1));
+        auto [gx, gw, gb, gres] =
+            layer_norm_backward(grads[0], saved[0], saved[1], saved[2], saved[3].defined() ? OptTensor(saved[3]) : std::nullopt,
+                                saved[4], saved[5], ctx->saved_data["relu"].toBool(), affine, needs(2));
+        out[0] = gx;
+        if (affine) {
+            out[2] = gw.to(saved[3].scalar_type());
+            if (edges[1] >= 0) out[3] = gb.to((at::ScalarType)ctx->saved_data["bias_type"].toInt());
+        }
+        if (gres.defined()) out[4] = gres.to((at::ScalarType)ctx->saved_data["residual_type"].toInt());
+        return out;
+    }
+};
+
+Tensor layer_norm(const Tensor &x, const Tensor &lengths, const OptTensor &weight, const OptTensor &bias,
+                  const OptTensor &residual, double eps, bool relu) {
+    const auto wants = [](const OptTensor &t) { return t && t->requires_grad(); };
+    if (!at::GradMode::is_enabled() || !(x.requires_grad() || wants(weight) || wants(bias) || wants(residual)))
+        return std::get<0>(layer_norm_forward(x, lengths, weight, bias, residual, eps, relu));
+    return LayerNorm::apply(x, lengths, weight, bias, residual, eps, relu);
+}
+
+// ----------------------------------------------------------------- geometry ----
+// Tap-segmented search: enqueue, fill into buffers sized from `ratio` (pairs per query of earlier searches
+// of this kind; negative: count first) and one hand-over.  Returns
+// (i, j, k | undefined, seg, num_neighbors, total, queries without neighbour, device status).
+std::tuple<Tensor, Tensor, OptTensor, Tensor, Tensor, int64_t, int64_t, int64_t> radius_taps(
+    const Tensor &points_, const Tensor &queries_, double radius, const OptTensor &ps_, const OptTensor &qs_, int64_t distance_type,
+    int64_t kernel_size, double grid, bool want_k, double ratio) {
+    require_cuda(points_), require_cuda(queries_), require_cuda(ps_), require_cuda(qs_);
+    c10::cuda::CUDAGuard guard(points_.device());
+    const Tensor points = points_.contiguous(), queries = queries_.contiguous();
+    const Tensor ps = ps_ ? as_i32(*ps_) : Tensor();
+    const Tensor qs = !qs_ ? Tensor() : (ps_ && qs_->is_same(*ps_)) ? ps : as_i32(*qs_);
+    const int64_t P = points.size(0), Q = queries.size(0), k3 = kernel_size * kernel_size * kernel_size;
+    const auto i32 = at::TensorOptions().dtype(at::kInt).device(points.device());
+    const auto i64 = i32.dtype(at::kLong);
+    Tensor ws = workspace(pcx_radius_taps_workspace_bytes(P, Q, (int)kernel_size), points);
+    Tensor num_neighbors = at::empty({Q}, i64), seg = at::empty({k3 + 1}, i64);
+    check(pcx_radius_taps_count(ptr_as<float>(points), ptr_as<float>(queries), ptr_as<int32_t>(ps), ptr_as<int32_t>(qs), P, Q, radius,
+                                (int)distance_type, (int)kernel_size, grid, ptr_as<int64_t>(num_neighbors), ptr_as<int64_t>(seg),
+                                ptr(ws), ws.numel(), stream()));
+    int64_t total[3] = {0, 0, 0}, capacity;
+    if (ratio < 0) {
+        check(pcx_radius_taps_total(P, Q, (int)kernel_size, total, ptr(ws), ws.numel(), stream()));
+        capacity = total[0];
+    } else {
+        capacity = std::min<int64_t>((int64_t)(ratio * (double)Q * 1.25) + 4096, ((int64_t)1 << 31) - 1);
+    }
+    Tensor i, j, k;
+    for (int attempt = 0; attempt < 2; ++attempt) {
+        i = at::empty({capacity}, i32), j = at::empty({capacity}, i32);
+        if (want_k) k = at::empty({capacity}, i32);
+        const int rc = pcx_radius_taps_fill(ptr_as<float>(queries), ptr_as<int32_t>(ps), ptr_as<int32_t>(qs), P, Q, radius,
+                                            (int)distance_type, (int)kernel_size, grid, capacity, ptr_as<int32_t>(i),
+                                            ptr_as<int32_t>(j), ptr_as<int32_t>(k), total, ptr(ws), ws.numel(), stream());
+        if (rc == PCX_E_CAPACITY && attempt == 0 && total[0] > capacity) {
+            capacity = total[0];   // the estimate was too small: exact size, fill pass only
+            continue;
+        }
+        check(rc);
+        break;
+    }
+    const int64_t n = total[0];
+    return {i.narrow(0, 0, n), j.narrow(0, 0, n), want_k ? OptTensor(k.narrow(0, 0, n)) : std::nullopt, seg, num_neighbors, n, total[1],
+            total[2]};
+}
+
+// (indices, points, sample | undefined, mapping | undefined) of the centre-nearest point of every occupied cell
+std::tuple<Tensor, Tensor, OptTensor, OptTensor> grid_sample(const Tensor &points_, double cell, const OptTensor &sample_,
+                                                             bool want_mapping) {
+    require_cuda(points_), require_cuda(sample_);
+    c10::cuda::CUDAGuard guard(points_.device());
+    const Tensor points = points_.contiguous(), sample = sample_ ? as_i32(*sample_) : Tensor();
+    const int64_t N = points.size(0);
+    const auto i64 = at::TensorOptions().dtype(at::kLong).device(points.device());
+    Tensor ws = workspace(pcx_grid_sample_workspace_bytes(N), points);
+    int64_t cells = 0;
+    check(pcx_grid_sample_count(ptr_as<float>(points), ptr_as<int32_t>(sample), N, cell, &cells, ptr(ws), ws.numel(), stream()));
+    Tensor indices = at::empty({cells}, i64), out = at::empty({cells, 3}, i64.dtype(at::kFloat));
+    Tensor out_sample = sample_ ? at::empty({cells}, i64.dtype(at::kInt)) : Tensor();
+    Tensor mapping = want_mapping ? at::empty({N}, i64) : Tensor();
+    check(pcx_grid_sample_select(ptr_as<float>(points), ptr_as<int32_t>(sample), N, cell, cells, ptr_as<int64_t>(indices),
+                                 ptr_as<float>(out), ptr_as<int32_t>(out_sample), ptr_as<int64_t>(mapping), ptr(ws), ws.numel(),
+                                 stream()));
+    return {indices, out, sample_ ? OptTensor(out_sample) : std::nullopt, want_mapping ? OptTensor(mapping) : std::nullopt};
+}
+
+// (plan buffer, number of buckets with several triplets)
+std::tuple<Tensor, int64_t> plan_build(const Tensor &scatter_, const Tensor &gather_, const Tensor &seg_, int64_t K, int64_t n_out,
+                                       int64_t group) {
+    require_cuda(scatter_), require_cuda(gather_), require_cuda(seg_);
+    c10::cuda::CUDAGuard guard(scatter_.device());
+    const Tensor scatter = as_i32(scatter_), gather = as_i32(gather_), seg = as_i64(seg_);
+    const int64_t T = scatter.numel();
+    const size_t bytes = pcx_mvmr_plan_bytes(T, n_out, (int)K, (int)group);
+    if (bytes == 0) {
+        py::gil_scoped_acquire gil;
+        raise(PyExc_NotImplementedError, "no output-stationary plan for T=" + std::to_string(T) + " n_out=" + std::to_string(n_out) +
+                                             " K=" + std::to_string(K) + " group=" + std::to_string(group));
+    }
+    Tensor buf = workspace(bytes, scatter), ws = workspace(pcx_mvmr_plan_workspace_bytes(T, n_out, (int)K, (int)group), scatter);
+    check(pcx_mvmr_plan_build(ptr_as<int32_t>(scatter), ptr_as<int32_t>(gather), ptr_as<int64_t>(seg), T, (int)K, n_out, (int)group,
+                              ptr(buf), buf.numel(), ptr(ws), ws.numel(), stream()));
+    int64_t multi = 0;
+    check(pcx_mvmr_plan_multi_buckets(ptr(buf), &multi, stream()));
+    return {buf, multi};
+}
+
+Tensor planned(const Tensor &weight, const Tensor &feat, const Tensor &buffer, int64_t group, int64_t multi, int64_t T, int64_t n_out,
+               bool transpose) {
+    require_cuda(weight), require_cuda(feat);
+    c10::cuda::CUDAGuard guard(feat.device());
+    Plan plan;
+    plan.buffer = buffer, plan.group = group, plan.multi = multi;
+    return mvmr_planned(weight.contiguous(), feat.contiguous(), plan, T, n_out, transpose ? 1 : 0, Tensor());
+}
+
+void set_hooks(py::object plan, py::object symmetric, py::object double_backward) {
+    g_plan_hook = plan.release().ptr();
+    g_symmetric_hook = symmetric.release().ptr();
+    g_double_backward = double_backward.release().ptr();
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_pcx_host, m) {
+    m.def("set_hooks", &set_hooks);
+    m.def("set_engine", [](int e) { g_engine = e; });
+    m.def("mvmr", &mvmr);
+    m.def("vvor", &vvor);
+    m.def("conv", &conv);
+    m.def("column_sums", &column_sums);
+    m.def("layer_norm", &layer_norm);
+    m.def("layer_norm_forward", &layer_norm_forward);
+    m.def("layer_norm_backward", &layer_norm_backward);
+    m.def("radius_taps", &radius_taps, py::call_guard<py::gil_scoped_release>());
+    m.def("grid_sample", &grid_sample, py::call_guard<py::gil_scoped_release>());
+    m.def("plan_build", &plan_build, py::call_guard<py::gil_scoped_release>());
+    m.def("planned", &planned);
+}

@@ -332,6 +332,8 @@ struct OsParams {
     const uint16_t *feat;
     uint16_t *out;
     const uint16_t *weight;
+    const uint16_t *bias;      // added before the rounding; null: none
+    int reverse;               // tap k uses weight K-1-k
     const int32_t *perm, *tile_offs, *group_order, *tile_rows;
     const uint16_t *scratch;   // sums of the multi-triplet buckets
     const uint2 *entries;
@@ -590,6 +592,13 @@ mvmr_os_kernel(const __grid_constant__ CUtensorMap tmap, const OsParams p) {
                         for (int c = 0; c < 16; ++c) acc[c] = 0.f;
                     }
                     if (row >= 0) {
+                        if (p.bias) {
+#pragma unroll
+                            for (int c = 0; c < 16; ++c) {
+                                const uint16_t b = __ldg(p.bias + cc * 16 + c);
+                                acc[c] += p.fmt ? __bfloat162float(__ushort_as_bfloat16(b)) : __half2float(__ushort_as_half(b));
+                            }
+                        }
                         uint4 *dst = reinterpret_cast<uint4 *>(p.out + (int64_t)row * p.outw + cc * 16);
                         uint4 o;
                         o.x = pack2(acc[0], acc[1], p.fmt), o.y = pack2(acc[2], acc[3], p.fmt);
@@ -662,7 +671,8 @@ mvmr_os_kernel(const __grid_constant__ CUtensorMap tmap, const OsParams p) {
             uint32_t wslot = w_n % (uint32_t)p.nw, wuse = w_n / (uint32_t)p.nw;
             bool ok_role = true;
             for (int wt = 0; wt < w_total && ok_role; ++wt) {
-                const int tap = s_wtask[wt] & 0xffff, q = s_wtask[wt] >> 16;
+                const int rb_tap = s_wtask[wt] & 0xffff, q = s_wtask[wt] >> 16;
+                const int tap = p.reverse ? p.K - 1 - rb_tap : rb_tap;
                 const uint32_t w_slot = w_base + wslot * p.w_slot_bytes, full = smem_u32(&s_w_full[wslot]);
                 STAT_T0(t_w);
                 ok_role = mbar_wait_abortable(smem_u32(&s_w_empty[wslot]), (wuse & 1u) ^ 1u, STATUS_BIT, p.status, abort_flag,
@@ -907,7 +917,15 @@ int pcx_mvmr_plan_multi_buckets(const void *d_plan, int64_t *h_count, void *stre
 
 int pcx_mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan, size_t plan_bytes, void *d_out, int64_t T,
                      int64_t n_feat, int64_t n_out, int K, int C, int M, int transpose, int dtype, int group_blocks,
-                     int64_t multi_buckets, void *d_ws, size_t ws_bytes, void *stream_) {
+                     int64_t multi_buckets, void *d_ws, size_t ws_bytes, void *stream) {
+    return pcx_mvmr_planned_bias(d_weight, d_feat, d_plan, plan_bytes, nullptr, d_out, T, n_feat, n_out, K, C, M,
+                                 transpose ? PCX_MVMR_TRANSPOSE : 0, dtype, group_blocks, multi_buckets, d_ws, ws_bytes, stream);
+}
+
+int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan, size_t plan_bytes, const void *d_bias, void *d_out,
+                          int64_t T, int64_t n_feat, int64_t n_out, int K, int C, int M, int flags, int dtype, int group_blocks,
+                          int64_t multi_buckets, void *d_ws, size_t ws_bytes, void *stream_) {
+    const int transpose = flags & PCX_MVMR_TRANSPOSE;
     cudaStream_t stream = (cudaStream_t)stream_;
     const int G = group_blocks;
     if (dtype != PCX_F16 && dtype != PCX_BF16) PCX_FAIL(PCX_E_DTYPE, "pcx_mvmr_planned: fp16 or bf16 only (dtype %d)", dtype);
@@ -933,6 +951,7 @@ int pcx_mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan, siz
     p.feat = (const uint16_t *)d_feat, p.out = (uint16_t *)d_out, p.weight = (const uint16_t *)d_weight;
     p.perm = pv.perm, p.tile_offs = pv.tile_offs, p.group_order = pv.group_order, p.entries = pv.entries, p.ctrl = pv.ctrl;
     p.tile_rows = pv.tile_rows, p.scratch = (const uint16_t *)d_ws;
+    p.bias = (const uint16_t *)d_bias, p.reverse = (flags & PCX_MVMR_REVERSE_TAPS) ? 1 : 0;
     p.status = status_word();
     if (!p.status) PCX_FAIL(PCX_E_LAUNCH, "pcx_mvmr_planned: no device status word");
     p.K = K, p.C = C, p.M = M, p.transpose = transpose ? 1 : 0, p.fmt = dtype == PCX_BF16 ? 1 : 0;

@@ -66,8 +66,17 @@ size_t pcx_mvmr_workspace_bytes(int64_t n_out, int K, int G, int C, int M, int t
 int pcx_mvmr(const void *d_weight, const void *d_feat, const int32_t *d_gather, const int32_t *d_scatter,
              const int64_t *d_seg_offs, const int32_t *d_tap_idx, void *d_out, int64_t T, int64_t n_feat,
              int64_t n_out, int K, int G, int C, int M, int transpose, int dtype, int engine, void *d_ws,
-             size_t ws_bytes, void *stream_) {
+             size_t ws_bytes, void *stream) {
+    return pcx_mvmr_bias(d_weight, d_feat, d_gather, d_scatter, d_seg_offs, d_tap_idx, nullptr, d_out, T, n_feat, n_out, K, G, C, M,
+                         transpose ? PCX_MVMR_TRANSPOSE : 0, dtype, engine, d_ws, ws_bytes, stream);
+}
+
+int pcx_mvmr_bias(const void *d_weight, const void *d_feat, const int32_t *d_gather, const int32_t *d_scatter,
+                  const int64_t *d_seg_offs, const int32_t *d_tap_idx, const void *d_bias, void *d_out, int64_t T, int64_t n_feat,
+                  int64_t n_out, int K, int G, int C, int M, int flags, int dtype, int engine, void *d_ws, size_t ws_bytes,
+                  void *stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
+    const int transpose = flags & PCX_MVMR_TRANSPOSE;
     if (T < 0 || n_feat < 0 || n_out < 0 || K <= 0 || G <= 0 || C <= 0 || M <= 0)
         PCX_FAIL(PCX_E_ARG, "pcx_mvmr: negative or zero size (T=%lld n_feat=%lld n_out=%lld K=%d G=%d C=%d M=%d)",
                  (long long)T, (long long)n_feat, (long long)n_out, K, G, C, M);
@@ -99,6 +108,7 @@ int pcx_mvmr(const void *d_weight, const void *d_feat, const int32_t *d_gather, 
     a.chunk_table = w.chunk_table;
     a.T = T, a.n_feat = n_feat, a.n_out = n_out;
     a.K = K, a.G = G, a.C = C, a.M = M, a.transpose = transpose ? 1 : 0, a.dtype = dtype;
+    a.bias = d_bias, a.reverse = (flags & PCX_MVMR_REVERSE_TAPS) ? 1 : 0;
     if (force_engine()) engine = force_engine();
     if (fan_in_one && T > 0 && engine != PCX_ENGINE_CUDA_CORE && mvmr_tensor_supported(a) && ((uintptr_t)d_out & 15) == 0) {
         // every output row has exactly one triplet: the tensor kernel stores the rounded rows
@@ -106,7 +116,7 @@ int pcx_mvmr(const void *d_weight, const void *d_feat, const int32_t *d_gather, 
         a.out_rows = d_out;
         return mvmr_tensor(a, stream);
     }
-    PCX_CUDA(cudaMemsetAsync(a.acc, 0, (size_t)out_elems * sizeof(float), stream));
+    if (int rc = clear_accumulator(a.acc, d_bias, n_out, G * outw, dtype, stream)) return rc;
     if (T > 0) {
         bool tensor_ok = mvmr_tensor_supported(a);
         if (engine == PCX_ENGINE_TENSOR && !tensor_ok)

@@ -73,7 +73,7 @@ template <typename T, bool TRANSPOSE>
 __global__ void __launch_bounds__(128) mvmr_sorted_kernel(
     const T *__restrict__ W, const T *__restrict__ feat, const int32_t *__restrict__ gather,
     const int32_t *__restrict__ scatter, const int64_t *__restrict__ seg, const int32_t *__restrict__ cum,
-    float *__restrict__ acc, int K, int G, int C, int M) {
+    float *__restrict__ acc, int K, int G, int C, int M, int reverse) {
     __shared__ float xs[GL][GK + 1];
     __shared__ float ws[GK][GN + 1];
     __shared__ int32_t s_gather[GL], s_scatter[GL];
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(128) mvmr_sorted_kernel(
         s_scatter[tid] = tid < rows ? scatter[t0 + tid] : 0;
     }
     __syncthreads();
-    const T *Wk = W + ((int64_t)tap * G + g) * C * M;
+    const T *Wk = W + ((int64_t)(reverse ? K - 1 - tap : tap) * G + g) * C * M;
     const int ty = tid >> 4, tx = tid & 15;
     float a[4][4] = {};
     for (int k0 = 0; k0 < inw; k0 += GK) {
@@ -143,12 +143,12 @@ template <typename T, bool TRANSPOSE>
 __global__ void mvmr_unsorted_kernel(const T *__restrict__ W, const T *__restrict__ feat,
                                      const int32_t *__restrict__ gather, const int32_t *__restrict__ scatter,
                                      const int32_t *__restrict__ tap_idx, float *__restrict__ acc,
-                                     int64_t Tn, int G, int C, int M) {
+                                     int64_t Tn, int K, int G, int C, int M, int reverse) {
     int64_t t = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= Tn) return;
     const int lane = threadIdx.x & 31;
     const int inw = TRANSPOSE ? M : C, outw = TRANSPOSE ? C : M;
-    const int64_t k = tap_idx[t], src = gather[t], dst = scatter[t];
+    const int64_t k = reverse ? K - 1 - tap_idx[t] : tap_idx[t], src = gather[t], dst = scatter[t];
     for (int g = 0; g < G; ++g) {
         const T *Wk = W + (k * G + g) * C * M;
         const T *x = feat + (src * G + g) * inw;
@@ -273,15 +273,15 @@ int mvmr_generic_t(const MvmrArgs &a, cudaStream_t stream) {
         int64_t upper = (a.T + GL - 1) / GL + a.K;
         dim3 grid((unsigned)upper, (unsigned)((outw + GN - 1) / GN), (unsigned)a.G);
         if (a.transpose)
-            mvmr_sorted_kernel<T, true><<<grid, 128, 0, stream>>>(W, feat, a.gather, a.scatter, a.seg_offs, a.chunk_table, a.acc, a.K, a.G, a.C, a.M);
+            mvmr_sorted_kernel<T, true><<<grid, 128, 0, stream>>>(W, feat, a.gather, a.scatter, a.seg_offs, a.chunk_table, a.acc, a.K, a.G, a.C, a.M, a.reverse);
         else
-            mvmr_sorted_kernel<T, false><<<grid, 128, 0, stream>>>(W, feat, a.gather, a.scatter, a.seg_offs, a.chunk_table, a.acc, a.K, a.G, a.C, a.M);
+            mvmr_sorted_kernel<T, false><<<grid, 128, 0, stream>>>(W, feat, a.gather, a.scatter, a.seg_offs, a.chunk_table, a.acc, a.K, a.G, a.C, a.M, a.reverse);
     } else {
         unsigned blocks = (unsigned)((a.T + 7) / 8);
         if (a.transpose)
-            mvmr_unsorted_kernel<T, true><<<blocks, 256, 0, stream>>>(W, feat, a.gather, a.scatter, a.tap_idx, a.acc, a.T, a.G, a.C, a.M);
+            mvmr_unsorted_kernel<T, true><<<blocks, 256, 0, stream>>>(W, feat, a.gather, a.scatter, a.tap_idx, a.acc, a.T, a.K, a.G, a.C, a.M, a.reverse);
         else
-            mvmr_unsorted_kernel<T, false><<<blocks, 256, 0, stream>>>(W, feat, a.gather, a.scatter, a.tap_idx, a.acc, a.T, a.G, a.C, a.M);
+            mvmr_unsorted_kernel<T, false><<<blocks, 256, 0, stream>>>(W, feat, a.gather, a.scatter, a.tap_idx, a.acc, a.T, a.K, a.G, a.C, a.M, a.reverse);
     }
     if (a.seg_offs) prof_end(stream);
     PCX_LAUNCH_CHECK();

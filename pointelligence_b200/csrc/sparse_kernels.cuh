@@ -15,7 +15,9 @@ struct MvmrArgs {
     void *out_rows;          // tensor engine, fan-in 1: the output itself, written row by row (acc unused)
     int32_t *chunk_table;    // (K+1) scratch of the CUDA-core engine
     int64_t T, n_feat, n_out;
+    const void *bias;        // (G*outw) of dtype or null; only the fan-in 1 stores read it, elsewhere acc starts as it
     int K, G, C, M, transpose, dtype;
+    int reverse;             // tap k uses weight K-1-k
 };
 
 struct VvorArgs {
@@ -35,6 +37,7 @@ __global__ void chunk_table_kernel(const int64_t *__restrict__ seg, int K, int L
 
 int mvmr_generic(const MvmrArgs &a, cudaStream_t stream);
 int vvor_generic(const VvorArgs &a, cudaStream_t stream);
+int clear_accumulator(float *acc, const void *bias, int64_t rows, int width, int dtype, cudaStream_t stream);
 int round_accumulator(const float *acc, void *out, int64_t n, int dtype, cudaStream_t stream);
 
 bool mvmr_tensor_supported(const MvmrArgs &a);

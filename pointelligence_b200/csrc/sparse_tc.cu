@@ -175,6 +175,10 @@ __device__ __forceinline__ uint32_t pack_pair(float a, float b, int fmt) {
     return *reinterpret_cast<uint32_t *>(&h);
 }
 
+__device__ __forceinline__ float unpack_one(uint16_t v, int fmt) {
+    return fmt ? __bfloat162float(__ushort_as_bfloat16(v)) : __half2float(__ushort_as_half(v));
+}
+
 struct MvmrTcParams {
     const uint16_t *weight;  // (K, C, M) as stored
     const uint16_t *feat;
@@ -182,6 +186,8 @@ struct MvmrTcParams {
     const int64_t *seg;
     float *acc;
     uint16_t *out;           // MODE 2: the output rows themselves (every row occurs in exactly one triplet)
+    const uint16_t *bias;    // MODE 2: added before the rounding (null: none); the other modes start from it
+    int reverse;             // tap k uses weight K-1-k
     int K, C, M, transpose, fmt, nbuf, slab;  // slab: columns parked per bulk reduction (32 or 64)
     int prow_log2;                            // a warp parks 2^prow_log2 rows at a time (8, 16 or 32)
     uint32_t park_bytes;                      // size of the parking area (the chunk table follows it)
@@ -250,7 +256,7 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
     bool alive = true;
 
     auto load_weight = [&](int tap) {
-        const uint16_t *w = p.weight + (int64_t)tap * p.C * p.M;
+        const uint16_t *w = p.weight + (int64_t)(p.reverse ? p.K - 1 - tap : tap) * p.C * p.M;
         const int cpr = p.M >> 3;
         for (int e = tid; e < p.C * cpr; e += 128) {
             int c = e / cpr, ch = e - c * cpr;
@@ -377,6 +383,10 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
 #pragma unroll
                     for (int q = 0; q < 4; ++q) {
                         if (col0 + 8 * q < outw) {
+                            if (p.bias) {
+#pragma unroll
+                                for (int e = 0; e < 8; ++e) v[8 * q + e] += unpack_one(p.bias[col0 + 8 * q + e], p.fmt);
+                            }
                             uint4 o;
                             o.x = pack_pair(v[8 * q], v[8 * q + 1], p.fmt), o.y = pack_pair(v[8 * q + 2], v[8 * q + 3], p.fmt);
                             o.z = pack_pair(v[8 * q + 4], v[8 * q + 5], p.fmt), o.w = pack_pair(v[8 * q + 6], v[8 * q + 7], p.fmt);
@@ -775,7 +785,7 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
     MvmrTcParams p;
     p.weight = (const uint16_t *)a.weight, p.feat = (const uint16_t *)a.feat;
     p.gather = a.gather, p.scatter = a.scatter, p.seg = a.seg_offs, p.acc = a.acc;
-    p.out = (uint16_t *)a.out_rows;
+    p.out = (uint16_t *)a.out_rows, p.bias = (const uint16_t *)a.bias, p.reverse = a.reverse;
     p.K = a.K, p.C = a.C, p.M = a.M, p.transpose = a.transpose, p.fmt = a.dtype == PCX_BF16 ? 1 : 0;
     p.ncols = pow2_cols((outw + 63) / 64 * 64);  // the epilogue reads blocks of up to 64 columns
     // Measured on B200: rows of exactly 64 floats leave fastest through one bulk reduction

@@ -116,7 +116,8 @@ class GeneralConv(Module):
                 output = (parts[0] + parts[1]).to(x3.dtype)
             else:
                 output = tig_mvmr(weight, x3.view(n_in, -1), idx,
-                                  input_precision=resolve_input_precision(x3.dtype))
+                                  input_precision=resolve_input_precision(x3.dtype), bias=bias)
+                bias = None
         else:
             output = sparse_matrix_vector_multiplication_reduction(weight, k, x3, j, i, n)
         output = output.reshape(-1, weight.shape[1] * weight.shape[3])

@@ -24,33 +24,6 @@ __all__ = ["RaggedNorm", "RaggedBatchNorm", "RaggedInstanceNorm", "RaggedLayerNo
            "fused_layer_norm", "fused_group_norm"]
 
 
-class _FusedLayerNorm(torch.autograd.Function):
-    """One autograd node over the library's fused kernels (``pcx_ragged_layer_norm`` and its
-    backward): statistics, affine, optional residual add and ReLU."""
-
-    @staticmethod
-    def forward(ctx, x, lengths, weight, bias, residual, eps, relu):
-        y, mean, rstd = _cabi.ragged_layer_norm(x, lengths, weight, bias, residual, eps, relu)
-        ctx.save_for_backward(x, y, lengths, weight, mean, rstd)
-        ctx.relu, ctx.has_residual = bool(relu), residual is not None
-        ctx.param_dtypes = (None if weight is None else weight.dtype, None if bias is None else bias.dtype)
-        ctx.residual_dtype = None if residual is None else residual.dtype
-        return y
-
-    @staticmethod
-    def backward(ctx, grad_y):
-        x, y, lengths, weight, mean, rstd = ctx.saved_tensors
-        want_affine = weight is not None and (ctx.needs_input_grad[2] or ctx.needs_input_grad[3])
-        want_res = ctx.has_residual and ctx.needs_input_grad[4]
-        gx, gw, gb, gres = _cabi.ragged_layer_norm_backward(grad_y, x, y, lengths, weight, mean, rstd, ctx.relu,
-                                                            want_affine, want_res)
-        if gw is not None:
-            gw, gb = gw.to(ctx.param_dtypes[0]), gb.to(ctx.param_dtypes[1])
-        if gres is not None:
-            gres = gres.to(ctx.residual_dtype)
-        return gx, None, gw, gb, gres, None, None
-
-
 class _FusedGroupNorm(torch.autograd.Function):
     """Group / instance norm over the library's kernels (``pcx_ragged_group_norm`` and its backward)."""
 
@@ -84,7 +57,7 @@ def fused_layer_norm(x, lengths, weight=None, bias=None, eps=1e-5, residual=None
 
     Same arithmetic as ``RaggedLayerNorm`` (layers/norm.py:59-83,118-130 of the reference) followed by
     the ``out += identity; relu(out)`` tail of its residual blocks (models/resnet.py:129-130)."""
-    return _FusedLayerNorm.apply(x, lengths, weight, bias, residual, eps, relu)
+    return _cabi.host().layer_norm(x, lengths, weight, bias, residual, float(eps), bool(relu))
 
 
 class RaggedNorm(nn.Module):

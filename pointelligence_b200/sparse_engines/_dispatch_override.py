@@ -44,6 +44,14 @@ def _normalize(mode):
 _state = {"mode": _normalize(os.environ.get("PNT_DISPATCH_MODE", "auto")), "precision": "default"}
 
 
+def _set_mode(mode):
+    _state["mode"] = mode
+    from .. import _cabi
+
+    if _cabi._host is not None:      # the compiled host path reads the engine of the mode on every pass
+        _cabi._host.set_engine(current_engine())
+
+
 def current_mode():
     return _state["mode"]
 
@@ -75,11 +83,11 @@ def dispatch_mode(mode):
             raise ValueError(f"dispatch mode {mode!r} was renamed to {_RENAMED[mode]!r}")
         raise ValueError(f"unknown dispatch mode: {mode!r}")
     prev = _state["mode"]
-    _state["mode"] = _normalize(mode)
+    _set_mode(_normalize(mode))
     try:
         yield
     finally:
-        _state["mode"] = prev
+        _set_mode(prev)
 
 
 @contextmanager

@@ -156,9 +156,30 @@ def _tig_backward(ctx, grad_out):
 _tig_mvmr_op.register_autograd(_tig_backward, setup_context=_tig_setup)
 
 
-def tig_mvmr(weight, feat, index, mode="auto", input_precision: Optional[str] = None):
+_PLAIN = (Tensor, torch.nn.Parameter)
+
+
+def _takes_host_path(*tensors):
+    """Whether a call goes straight to the compiled host path: eager mode on plain CUDA tensors.
+    Tracing (``torch.compile``) and tensor subclasses see the registered operator instead."""
+    if torch.compiler.is_compiling():
+        return False
+    for t in tensors:
+        if t is not None and (type(t) not in _PLAIN or not t.is_cuda):
+            return False
+    return True
+
+
+def tig_mvmr(weight, feat, index, mode="auto", input_precision: Optional[str] = None, bias: Optional[Tensor] = None):
     """Differentiable tap-sorted convolution: one autograd node, three kernel
-    families (forward MVMR, transposed MVMR, VVOR)."""
+    families (forward MVMR, transposed MVMR, VVOR).  A ``bias`` of the output's type is added
+    before the rows are rounded."""
+    if _takes_host_path(weight, feat, bias, index.flat_i, index.flat_j, index.flat_seg) and (
+            bias is None or bias.dtype == feat.dtype == weight.dtype):
+        return _cabi.host().conv(weight, feat, bias, index.flat_i, index.flat_j, index.flat_seg, index.N, index.N_in,
+                                 index.K, index.exact_cover_out, index.exact_cover_in)
+    if bias is not None:
+        return tig_mvmr(weight, feat, index, mode, input_precision) + bias
     if input_precision is None:
         input_precision = resolve_input_precision(feat.dtype)
     return _tig_mvmr_op(weight, feat, index.flat_i, index.flat_j, index.flat_seg, index.N, index.N_in,
