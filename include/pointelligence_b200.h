@@ -157,9 +157,8 @@ int pcx_column_sums(const void *d_x, void *d_out, int64_t N, int C, int dtype,
  *                 for an output row of out_width channels.  The same value
  *                 must be passed to both calls (a plan built for one value is
  *                 not valid for another).
- *   d_plan        caller-owned, 256-byte aligned, pcx_mvmr_plan_bytes();
- *                 pcx_mvmr_planned updates a work counter inside it, so two
- *                 launches that use the same plan must not overlap on the GPU
+ *   d_plan        caller-owned, 256-byte aligned, pcx_mvmr_plan_bytes(); not
+ *                 written after the build
  *   limits        K <= 512, channel counts multiples of 16, out_width <= 256,
  *                 T < 2^31, ceil(n_out / 128) * K * 128 <= 2^32
  * The feature rows of a (row, tap) bucket with several triplets are summed
@@ -185,7 +184,12 @@ int pcx_mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan,
                      int64_t n_out, int K, int C, int M, int transpose,
                      int dtype, int group_blocks, int64_t multi_buckets,
                      void *d_ws, size_t ws_bytes, void *stream);
-/* ... with a bias and `flags` in place of `transpose`, as pcx_mvmr_bias. */
+/* ... with a bias and `flags` in place of `transpose`, as pcx_mvmr_bias.  A
+ * workspace of pcx_mvmr_planned_scratch_bytes() lets a small rulebook be split
+ * over the whole chip (its fp32 sums go through the workspace); with less it
+ * runs on as many SMs as it has groups. */
+size_t pcx_mvmr_planned_scratch_bytes(int64_t multi_buckets, int in_width,
+                                      int64_t n_out, int out_width, int K);
 int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat,
                           void *d_plan, size_t plan_bytes, const void *d_bias,
                           void *d_out, int64_t T, int64_t n_feat, int64_t n_out,

@@ -59,6 +59,7 @@ SIGNATURES = {
     "pcx_mvmr_planned_workspace_bytes": (c_size_t, [c_int64, c_int]),
     "pcx_mvmr_planned": (c_int, [c_void_p] * 3 + [c_size_t, c_void_p] + [c_int64] * 3 + [c_int] * 6
                          + [c_int64, c_void_p, c_size_t, c_void_p]),
+    "pcx_mvmr_planned_scratch_bytes": (c_size_t, [c_int64, c_int, c_int64, c_int, c_int]),
     "pcx_mvmr_planned_bias": (c_int, [c_void_p] * 3 + [c_size_t] + [c_void_p] * 2 + [c_int64] * 3 + [c_int] * 6
                               + [c_int64, c_void_p, c_size_t, c_void_p]),
     "pcx_debug_wait_runs_out": (c_int, [ctypes.c_ulonglong, c_void_p]),

@@ -117,7 +117,7 @@ Tensor mvmr_planned(const Tensor &weight, const Tensor &feat, const Plan &plan, 
     const bool transpose = flags & 1;
     const int64_t inw = transpose ? M : C, outw = transpose ? C : M;
     Tensor out = at::empty({n_out, outw}, feat.options());
-    const size_t bytes = pcx_mvmr_planned_workspace_bytes(plan.multi, (int)inw);
+    const size_t bytes = pcx_mvmr_planned_scratch_bytes(plan.multi, (int)inw, n_out, (int)outw, (int)K);
     Tensor ws = workspace(bytes, feat);
     check(pcx_mvmr_planned_bias(ptr(weight), ptr(feat), ptr(plan.buffer), plan.buffer.numel(), ptr(bias), ptr(out), T, feat.size(0),
                                 n_out, (int)K, (int)C, (int)M, flags, dtype_code(feat.scalar_type()), (int)plan.group, plan.multi,

@@ -18,27 +18,27 @@
 //   entries  per triplet (slot | position in its bucket << 8, feature row), ordered by
 //            (block, tap, slot): the members of a bucket are consecutive
 //   buckets  (first entry, length) of every bucket with more than one triplet
-//   groups   G consecutive blocks share the weight tiles they stream; groups are handed out
-//            most expensive first (a ticket counter inside the plan)
+//   groups   two consecutive blocks share the weight slices they stream; most expensive first
+//   masks    the taps that touch a block: what the walk goes through, so no task lists are built
 //
 // Per call: a small kernel sums the rows of the multi-triplet buckets into the scratch (fp32 sum,
-// one rounding), then the main kernel (TMEM columns = G accumulators of out_width fp32 each):
+// one rounding), then one persistent CTA per SM works off its steps (unit, slice, tap):
 //
-//   producer warps   together, one (block, tap, 64-channel slice) A tile after the other: every
-//                    thread issues its 16-byte cp.async copies of the tile's source rows straight
-//                    into the 128-byte-swizzled slot (rows without a source are zero-filled by the
-//                    same instruction with a source size of 0); a tile is handed to the tensor
-//                    core two tiles later, when its copies have landed anyway, with one mbarrier
-//                    arrival per warp; the copies of several tiles are in flight at any time
-//   weight warp      streams the 64-channel slices of W[tap] through a small ring with TMA
-//                    (cp.async.bulk.tensor tile loads, 128-byte swizzle); one slice serves
-//                    all blocks of the group that use the tap
-//   MMA warp         one thread issues tcgen05.mma (M = 128 rows, N = out_width, K = 16 per
-//                    instruction) with accumulate = 1 from the block's second tile on;
-//                    tcgen05.commit releases the A slot, the weight slot and finally hands
-//                    the accumulators to the epilogue
-//   epilogue         the producer warps read TMEM (tcgen05.ld), round once and write each
-//                    output row with 16-byte stores
+//   walk warp        decides the steps and fetches the source rows of their two tiles into shared memory
+//                    eight steps early.  The tables come from DRAM: looked up one step ahead, every step
+//                    waited out most of that latency and a tile took 1500 - 1800 clocks
+//   copy teams       two teams fill the A tiles, a step each in turn: 16-byte cp.async copies of the
+//                    tiles' source rows straight into the 128-byte-swizzled slot (rows without a source
+//                    are zero-filled by the same instruction with a source size of 0).  A copy loop alone
+//                    moves a 16 KB tile of random rows in 230 - 290 clocks (a TMA row gather, measured: 2260)
+//   weight warp      the 64-channel slice of W[tap] for both blocks, by TMA into the same slot
+//   MMA warps        one per block: one wait per step, up to four tcgen05.mma (M = 128, N = out_width)
+//                    and one commit
+//   epilogue warps   read TMEM (tcgen05.ld), round once and write each output row; up to 128 channels
+//                    the accumulators are double-buffered, so the next group is built meanwhile
+//
+// Units are groups; where those do not fill the chip (small clouds, deep levels) their taps are split
+// over several CTAs, which leave fp32 sums that a last kernel adds in a fixed order.
 //
 // Every wait is bounded (one second) and abortable: a role that gives up raises a flag in the
 // status word and in shared memory, the other roles leave their waits, and the CTA frees its
@@ -58,19 +58,13 @@ using namespace tc;
 
 constexpr int ROWS = 128;             // output rows per block (the M of the MMA)
 constexpr int SLOT_BYTES = ROWS * 128;  // one A tile: 128 rows of a 64-channel slice
-constexpr int MAX_NPW = 8;            // producer warps
-constexpr int MAX_SLOTS = 12;         // A slots
-constexpr int MAX_NW = 4;             // weight slots
-constexpr int MAX_GROUP = 8;          // blocks per group
-constexpr int MAX_TAPS = 512;         // taps the shared-memory tables are sized for
-constexpr int SIGNAL_LAG = 2;          // a tile is handed to the tensor core once the copies of the two tiles after it are issued
-constexpr int ROW_PREFETCH = 1;        // tiles whose source rows a producer thread holds ahead of the one it issues (deeper did not pay: the copies, not this table, bound the producer)
-constexpr int ROW_PASSES = 8;         // rows a producer thread copies per tile, at most (128 rows / (4 warps * 4 row lanes))
+constexpr int GROUP_BLOCKS = 2;         // blocks of a group
+constexpr int MAX_TAPS = 512;           // taps of a plan
 constexpr unsigned STATUS_BIT = 4u;   // bit of the device status word this kernel raises
 constexpr unsigned PLAN_MAGIC = 0x70637832u;
 
 // control words at the head of a plan
-enum { CTRL_TICKET = 0, CTRL_DONE = 1, CTRL_MAGIC = 2, CTRL_GROUP = 3, CTRL_NMULTI = 4, CTRL_WORDS = 64 };
+enum { CTRL_MAGIC = 2, CTRL_GROUP = 3, CTRL_NMULTI = 4, CTRL_WORDS = 64 };
 
 struct PlanView {
     uint32_t *ctrl;        // CTRL_WORDS
@@ -80,6 +74,7 @@ struct PlanView {
     int32_t *group_order;  // ngroups
     int32_t *tile_rows;    // nblocks * K * ROWS: source row of (tile, slot): >= 0 feature row, -1 none, <= -2 scratch row -2 - x
     uint2 *buckets;        // T / 2 + 1: (first entry, length) of the buckets with several triplets
+    uint32_t *tap_masks;   // nblocks * ceil(K / 32): the taps that touch a block
     int64_t nblocks, ngroups;
 };
 
@@ -95,6 +90,7 @@ size_t carve_plan(void *base, int64_t T, int64_t n_out, int K, int G, PlanView *
     v.group_order = c.take<int32_t>((size_t)std::max<int64_t>(v.ngroups, 1));
     v.tile_rows = c.take<int32_t>((size_t)v.nblocks * K * ROWS);
     v.buckets = c.take<uint2>((size_t)(T / 2 + 1));
+    v.tap_masks = c.take<uint32_t>((size_t)v.nblocks * ((K + 31) / 32));
     if (out) *out = v;
     return c.off;
 }
@@ -314,431 +310,397 @@ void launch_bucket_sum(int64_t multi, int inw, const uint16_t *feat, const uint2
 #undef PCX_BS
 }
 
-// cost of a group = its non-empty tiles (each is one A tile to gather and multiply)
+// cost of a group = its non-empty tiles (each is one A tile to copy and multiply); the tap sets of its blocks
 __global__ void plan_cost_kernel(const int32_t *__restrict__ tile_offs, int64_t nblocks, int K, int G, int64_t ngroups,
-                                 uint32_t *cost, int32_t *gid) {
+                                 uint32_t *cost, int32_t *gid, uint32_t *tap_masks) {
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ngroups) return;
-    const int64_t t0 = g * G * K, t1 = min((g + 1) * (int64_t)G, nblocks) * K;
+    const int words = (K + 31) / 32;
     uint32_t c = 0;
-    for (int64_t x = t0; x < t1; ++x) c += tile_offs[x + 1] > tile_offs[x];
+    for (int64_t b = g * G; b < min((g + 1) * (int64_t)G, nblocks); ++b)
+        for (int w = 0; w < words; ++w) {
+            uint32_t m = 0;
+            for (int k = 32 * w; k < min(K, 32 * w + 32); ++k)
+                if (tile_offs[b * K + k + 1] > tile_offs[b * K + k]) m |= 1u << (k & 31);
+            tap_masks[b * words + w] = m;
+            c += (uint32_t)__popc(m);
+        }
     cost[g] = c;
     gid[g] = (int32_t)g;
 }
 
 // ------------------------------------------------------------------ kernel ----
+constexpr int EPI_WARPS = 4, TEAMS = 2, TEAM_WARPS = 8, COPY_WARPS = TEAMS * TEAM_WARPS;
+constexpr int COPY_WARP0 = EPI_WARPS, WALK_WARP = COPY_WARP0 + COPY_WARPS, WEIGHT_WARP = WALK_WARP + 1, MMA_WARP0 = WEIGHT_WARP + 1;
+constexpr int THREADS = (MMA_WARP0 + GROUP_BLOCKS) * 32;
+constexpr int MAX_SLOTS = 8;
+constexpr int AHEAD = 8;                              // steps the walk runs ahead (even: an entry always belongs to the same team)
+constexpr uint32_t ENTRY_BYTES = 2 * ROWS * 4;        // source rows of a step's two tiles
+// a step in one word: tap | slice << 9 | tiles that have the tap << 13 | first of its unit << 15 | end << 16
+constexpr uint32_t STEP_FIRST = 1u << 15, STEP_END = 1u << 16;
 
 struct OsParams {
-    const uint16_t *feat;
+    const uint16_t *feat, *bias;            // bias: added before the rounding; null: none
+    const uint16_t *scratch;                // sums of the multi-triplet buckets
     uint16_t *out;
-    const uint16_t *weight;
-    const uint16_t *bias;      // added before the rounding; null: none
-    int reverse;               // tap k uses weight K-1-k
-    const int32_t *perm, *tile_offs, *group_order, *tile_rows;
-    const uint16_t *scratch;   // sums of the multi-triplet buckets
-    const uint2 *entries;
-    uint32_t *ctrl;
+    float *partial;                         // nsplit > 1: [split][nblocks * ROWS][outw]
+    const int32_t *perm, *group_order, *tile_rows;
+    const uint32_t *tap_masks;
     unsigned int *status;
-    int K, C, M, transpose, fmt;
-    int inw, outw, nkb, G, ngroups, nblocks;
-    int npw, nslots, nw, use_tma;
-    int lag;   // 0: every thread's copies report to the slot's barrier themselves; SIGNAL_LAG: one arrival per warp, SIGNAL_LAG tiles later
-    uint32_t w_slot_bytes, w_box_rows, w_tx_bytes;
-    uint32_t ncols, col_stride;
+    int K, C, M, transpose, reverse, fmt;   // reverse: tap k uses weight K-1-k
+    int inw, outw, nkb, ngroups, nblocks, nsplit, mask_words;
+    int nslots, nacc;
+    uint32_t slot_bytes, w_box_rows, w_tx_bytes, ncols, col_stride;
     uint64_t wait_limit_ns;
 };
 
-__device__ __forceinline__ uint4 ldg_nc_v4(const void *p) {
-    uint4 v;
-    asm volatile("ld.global.nc.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ uint2 ldg_nc_v2(const void *p) {
-    uint2 v;
-    asm volatile("ld.global.nc.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ void sts_v4(uint32_t addr, uint4 v) {
-    asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
-}
 __device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
     uint4 v;
     asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
     return v;
 }
+__device__ __forceinline__ float bias_at(const uint16_t *b, int c, int fmt) {
+    const uint16_t v = __ldg(b + c);
+    return fmt ? __bfloat162float(__ushort_as_bfloat16(v)) : __half2float(__ushort_as_half(v));
+}
 
-// Optional cycle accounting per role (compile with -DPCX_OS_STATS): sums of clock64() spans are
-// added to the plan's spare control words 8.. and read back by the caller.
-#ifdef PCX_OS_STATS
-#define STAT_T0(name) const long long name = clock64()
-#define STAT_ADD(word, t0) do { if (lane == 0) atomicAdd(&p.ctrl[word], (uint32_t)((clock64() - (t0)) >> 4)); } while (0)
-#else
-#define STAT_T0(name)
-#define STAT_ADD(word, t0)
-#endif
+// Position `n` of a CTA in the list of units (groups, most expensive first, times their parts): rows of
+// the list run to and fro over the CTAs, so that the sums of their costs stay close without a shared
+// work counter.  -1 behind the end.
+__device__ __forceinline__ int unit_at(int n, int units) {
+    const int pos = n * (int)gridDim.x + ((n & 1) ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x);
+    return pos < units ? pos : -1;
+}
 
-// Task lists of a group, built in shared memory by the whole CTA before the roles start:
-//   A task   one (block, tap, 64-channel slice) tile: its entries [lo, hi) and
-//            meta = block | slice << 4 | first-of-slice << 8 | last-of-slice << 9 | tap << 16
-//   W task   one (tap, slice) weight tile: tap | slice << 16
-// Order (every role walks the same lists): taps ascending; per tap the slices of the
-// contraction; per slice the blocks of the group that use the tap.
-__device__ __forceinline__ int pieces_of(int inw, int q) { return min(8, (inw - q * 64) >> 3); }
+// The steps of a CTA: unit after unit, in a unit the 64-channel slices of the contraction, per slice the
+// taps that touch one of the group's two blocks.
+struct Walk {
+    const OsParams &p;
+    int n = -1, unit = 0, block0 = 0, q = 0, word = 0, tap = 0;
+    int tap_lo = 0, tap_hi = 0;     // taps of this part of the group
+    uint32_t m0 = 0, m1 = 0, left = 0;
+    uint32_t has = 0;               // of the current step: bit b = block b of the group has the tap
+    bool opened = false;            // no step of the unit yet
+    bool first = false;             // the current step is the first of its unit
+    __device__ __forceinline__ explicit Walk(const OsParams &params) : p(params) { q = params.nkb; }
 
-__global__ void __launch_bounds__(512, 1)
-mvmr_os_kernel(const __grid_constant__ CUtensorMap tmap, const OsParams p) {
+    __device__ __forceinline__ static uint32_t below(int w, int tap) {   // bits of mask word w that belong to taps < tap
+        const int n = min(max(tap - 32 * w, 0), 32);
+        return n >= 32 ? 0xffffffffu : (1u << n) - 1u;
+    }
+    __device__ __forceinline__ void load(int w) {
+        const uint32_t r = below(w, tap_hi) & ~below(w, tap_lo);
+        m0 = __ldg(p.tap_masks + (int64_t)block0 * p.mask_words + w) & r;
+        m1 = block0 + 1 < p.nblocks ? __ldg(p.tap_masks + (int64_t)(block0 + 1) * p.mask_words + w) & r : 0u;
+        left = m0 | m1;
+    }
+    __device__ __forceinline__ bool open(int at) {   // the unit at position `at`; false behind the end
+        unit = unit_at(at, p.ngroups * p.nsplit);
+        if (unit < 0) return false;
+        const int s = unit % p.nsplit;
+        block0 = __ldg(p.group_order + unit / p.nsplit) * GROUP_BLOCKS;
+        tap_lo = p.K * s / p.nsplit, tap_hi = p.K * (s + 1) / p.nsplit;
+        return true;
+    }
+    __device__ __forceinline__ bool next() {
+        for (;;) {
+            if (left) {
+                const int b = __ffs(left) - 1;
+                left &= left - 1;
+                tap = word * 32 + b;
+                has = ((m0 >> b) & 1u) | (((m1 >> b) & 1u) << 1);
+                first = opened, opened = false;
+                return true;
+            }
+            if (q < p.nkb && ++word < p.mask_words) {
+                load(word);
+            } else if (++q < p.nkb) {
+                word = 0;
+                if (p.mask_words > 1) load(0);
+                else left = m0 | m1;
+            } else {
+                if (!open(++n)) return false;
+                q = 0, word = 0, opened = true;
+                load(0);
+            }
+        }
+    }
+};
+
+struct Ring {
+    uint32_t slot = 0, turn = 0;   // slot, and how often the ring has gone round
+    __device__ __forceinline__ void next(int depth) {
+        if (++slot == (uint32_t)depth) slot = 0, ++turn;
+    }
+};
+
+__global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ OsParams p) {
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t s_a_full[MAX_SLOTS], s_a_empty[MAX_SLOTS], s_w_full[MAX_NW], s_w_empty[MAX_NW], s_d_full;
+    __shared__ uint64_t s_full[MAX_SLOTS], s_empty[MAX_SLOTS], s_acc_full[2], s_acc_empty[2], s_step_full[AHEAD], s_step_empty[AHEAD];
+    __shared__ uint32_t s_step[AHEAD];
     __shared__ uint32_t s_tmem;
-    __shared__ int s_group, s_ntiles, s_ntaps, s_abort;
+    __shared__ int s_abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t a_base = base, w_base = base + (uint32_t)p.nslots * SLOT_BYTES;
-    uint8_t *tab_raw = smem_raw + (w_base + (uint32_t)p.nw * p.w_slot_bytes - smem_u32(smem_raw));
-    // tables of the current group (16-byte aligned): A tasks, tile offsets, tile list, run ordinals, W tasks
-    int4 *s_task = reinterpret_cast<int4 *>(tab_raw);                       // G*K*nkb
-    int32_t *s_tab = reinterpret_cast<int32_t *>(s_task + p.G * p.K * p.nkb);  // G*K + 1
-    int32_t *s_list = s_tab + (p.G * p.K + 1);                                // G*K: tap << 8 | block, tap-major
-    int32_t *s_run = s_list + p.G * p.K;                                      // G*K: ordinal of the tile's tap among the group's taps
-    int32_t *s_wtask = s_run + p.G * p.K;                                     // K*nkb
+    // a slot: the A tiles of the group's two blocks, then the weight slice both use; behind the slots the
+    // source rows of the next steps
+    const uint32_t slot0 = (smem_u32(smem_raw) + 1023u) & ~1023u, rows0 = slot0 + (uint32_t)p.nslots * p.slot_bytes;
     volatile int *abort_flag = &s_abort;
+    auto wait = [&](const uint64_t &bar, uint32_t parity) {   // the verdict is the same in the whole warp
+        return __all_sync(0xffffffffu, mbar_wait_abortable(smem_u32(&bar), parity & 1u, STATUS_BIT, p.status, abort_flag, p.wait_limit_ns)) != 0;
+    };
 
     if (tid == 0) {
-        for (int s = 0; s < p.nslots; ++s) mbar_init(smem_u32(&s_a_full[s]), (uint32_t)p.npw * (p.lag ? 1u : 32u)), mbar_init(smem_u32(&s_a_empty[s]), 1);
-        for (int s = 0; s < p.nw; ++s) mbar_init(smem_u32(&s_w_full[s]), p.use_tma ? 1 : 32), mbar_init(smem_u32(&s_w_empty[s]), 1);
-        mbar_init(smem_u32(&s_d_full), 1);
+        for (int s = 0; s < p.nslots; ++s)   // a team's copies and the weight slice; both MMA warps
+            mbar_init(smem_u32(&s_full[s]), TEAM_WARPS * 32 + 1), mbar_init(smem_u32(&s_empty[s]), GROUP_BLOCKS);
+        for (int s = 0; s < 2; ++s) mbar_init(smem_u32(&s_acc_full[s]), GROUP_BLOCKS), mbar_init(smem_u32(&s_acc_empty[s]), EPI_WARPS);
+        for (int s = 0; s < AHEAD; ++s)   // the walk's copies and its word; a team, the MMA warps and the weight warp
+            mbar_init(smem_u32(&s_step_full[s]), 33), mbar_init(smem_u32(&s_step_empty[s]), TEAM_WARPS + GROUP_BLOCKS + 1);
         fence_mbar_init();
         s_abort = 0;
-        if (p.use_tma) tma_prefetch_desc(&tmap);
+        tma_prefetch_desc(&tmap);
     }
     if (warp == 0) tmem_alloc(smem_u32(&s_tmem), p.ncols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
-    const uint32_t idesc = instr_desc(p.fmt, ROWS, p.outw, 0, p.transpose ? 0 : 1);
 
-    // A tiles, weight tiles and accumulator hand-overs of the groups this CTA has finished (all
-    // roles count alike): tile n uses A slot n mod nslots for the (n / nslots)-th time, and so on
-    uint32_t a_n = 0, w_n = 0, d_n = 0;
-
-    for (;;) {
-        STAT_T0(t_group);
-        if (tid == 0) {
-            const uint32_t ticket = atomicAdd(&p.ctrl[CTRL_TICKET], 1u);
-            s_group = ticket < (uint32_t)p.ngroups ? p.group_order[ticket] : -1;
-        }
-        __syncthreads();
-        const int g = s_group;
-        if (g < 0 || s_abort) break;
-        const int b0 = g * p.G, nb = min(p.G, p.nblocks - b0);
-        for (int x = tid; x <= nb * p.K; x += blockDim.x) s_tab[x] = p.tile_offs[(int64_t)b0 * p.K + x];
-        __syncthreads();
-        if (warp == 0) {  // the non-empty (tap, block) pairs, tap-major, and the ordinal of each pair's tap
-            int count = 0;
-            for (int x0 = 0; x0 < nb * p.K; x0 += 32) {
-                const int x = x0 + lane;
-                int tap = 0, blk = 0;
-                bool has = false;
-                if (x < nb * p.K) {
-                    tap = x / nb, blk = x - tap * nb;
-                    has = s_tab[blk * p.K + tap + 1] > s_tab[blk * p.K + tap];
-                }
-                const unsigned m = __ballot_sync(0xffffffffu, has);
-                if (has) s_list[count + __popc(m & ((1u << lane) - 1u))] = (tap << 8) | blk;
-                count += __popc(m);
+    if (warp < EPI_WARPS) {
+        // -------------------------------------------------------------- epilogue ----
+        Walk w(p);
+        Ring acc;
+        for (int n = 0; w.open(n); ++n) {
+            uint32_t any0 = 0, any1 = 0;
+            for (int x = 0; x < p.mask_words; ++x) w.load(x), any0 |= w.m0, any1 |= w.m1;
+            if (any0 | any1) {
+                if (!wait(s_acc_full[acc.slot], acc.turn)) break;
+                tc_fence_after();
             }
-            __syncwarp();
-            int taps = 0;
-            for (int x0 = 0; x0 < count; x0 += 32) {
-                const int x = x0 + lane;
-                const bool head = x < count && (x == 0 || (s_list[x] >> 8) != (s_list[x - 1] >> 8));
-                const unsigned m = __ballot_sync(0xffffffffu, head);
-                if (x < count) s_run[x] = taps + __popc(m & (0xffffffffu >> (31 - lane))) - 1;
-                taps += __popc(m);
-            }
-            if (lane == 0) s_ntiles = count, s_ntaps = taps;
-        }
-        __syncthreads();
-        const int ntiles = s_ntiles, a_total = ntiles * p.nkb, w_total = s_ntaps * p.nkb;
-        for (int x = tid; x < ntiles; x += blockDim.x) {  // expand the tile list into the task lists
-            const int tap = s_list[x] >> 8, blk = s_list[x] & 255;
-            int r0 = x, r1 = x + 1;
-            while (r0 > 0 && (s_list[r0 - 1] >> 8) == tap) --r0;
-            while (r1 < ntiles && (s_list[r1] >> 8) == tap) ++r1;
-            const int lo = s_tab[blk * p.K + tap], hi = s_tab[blk * p.K + tap + 1];
-            for (int q = 0; q < p.nkb; ++q) {
-                const int meta = blk | (q << 4) | ((x == r0) << 8) | ((x + 1 == r1) << 9) | (tap << 16);
-                s_task[r0 * p.nkb + q * (r1 - r0) + (x - r0)] = make_int4(lo, hi, meta, 0);
-                if (x == r0) s_wtask[s_run[x] * p.nkb + q] = tap | (q << 16);
-            }
-        }
-        __syncthreads();
-
-        if (warp == 0) STAT_ADD(8, t_group);
-        STAT_T0(t_role);
-        if (warp < p.npw) {
-            // ---------------------------------------------------------- producer ----
-            // All producer threads fill every tile together: 8 threads per row (one 16-byte piece
-            // each), npw * 4 rows per pass.  The source rows of the next tile are fetched while
-            // the current one is issued.
-            const int piece = tid & 7, row_lane = tid >> 3, row_lanes = p.npw * 4, passes = ROWS / row_lanes;
-            // row_lanes is a multiple of 8, so the rows of a thread share their low three bits and
-            // with them the swizzled position of the thread's piece inside a row
-            const uint32_t lane_offset = (uint32_t)row_lane * 128 + (uint32_t)((piece ^ (row_lane & 7)) << 4);
-            const uint32_t pass_stride = (uint32_t)row_lanes * 128;
-            uint32_t slot = a_n % (uint32_t)p.nslots, use = a_n / (uint32_t)p.nslots;
-            uint32_t signal_slot = slot;   // slot of the oldest tile not handed over yet
-            bool ok_role = true;
-            // source rows of the next ROW_PREFETCH tiles: buffer u holds tile t with t mod ROW_PREFETCH == u
-            // (static indexing: the loop below is unrolled by ROW_PREFETCH, so no register is moved
-            // while its load is in flight)
-            int rows_q[ROW_PREFETCH][ROW_PASSES];
-            auto fetch_rows = [&](int task, int (&dst)[ROW_PASSES]) {
-#pragma unroll
-                for (int k = 0; k < ROW_PASSES; ++k) dst[k] = -1;
-                if (task >= a_total) return;
-                const int meta = s_task[task].z;
-                const int32_t *table = p.tile_rows + ((int64_t)(b0 + (meta & 15)) * p.K + (meta >> 16)) * ROWS + row_lane;
-#pragma unroll
-                for (int k = 0; k < ROW_PASSES; ++k)
-                    if (k < passes) dst[k] = __ldg(table + k * row_lanes);
-            };
-#pragma unroll
-            for (int u = 0; u < ROW_PREFETCH; ++u) fetch_rows(u, rows_q[u]);
-            for (int t0 = 0; t0 < a_total && ok_role; t0 += ROW_PREFETCH) {
-#pragma unroll
-              for (int u = 0; u < ROW_PREFETCH; ++u) {
-                const int t = t0 + u;
-                if (t >= a_total || !ok_role) break;
-                int rows_cur[ROW_PASSES];
-#pragma unroll
-                for (int k = 0; k < ROW_PASSES; ++k) rows_cur[k] = rows_q[u][k];
-                fetch_rows(t + ROW_PREFETCH, rows_q[u]);
-                const int q = (s_task[t].z >> 4) & 15;
-                const bool piece_ok = piece < pieces_of(p.inw, q);
-                const uint16_t *feat_col = p.feat + q * 64 + piece * 8, *sum_col = p.scratch + q * 64 + piece * 8;
-                const uint32_t dst0 = a_base + slot * SLOT_BYTES + lane_offset;
-                // the tensor core has finished reading this slot's previous tile
-                STAT_T0(t_w);
-                ok_role = mbar_wait_abortable(smem_u32(&s_a_empty[slot]), (use & 1u) ^ 1u, STATUS_BIT, p.status, abort_flag,
-                                              p.wait_limit_ns);
-                STAT_ADD(9, t_w);
-                if (!ok_role) break;
-                if (piece_ok) {
-#pragma unroll
-                    for (int k = 0; k < ROW_PASSES; ++k) {
-                        if (k < passes) {
-                            const int src_row = rows_cur[k];
-                            // a feature row, a row of bucket sums, or nothing (16 bytes of zeros: source size 0)
-                            const uint16_t *src = src_row >= 0 ? feat_col + (int64_t)src_row * p.inw
-                                                               : sum_col + (int64_t)(src_row == -1 ? 0 : -2 - src_row) * p.inw;
-                            cp_async16_zfill(dst0 + (uint32_t)k * pass_stride, src_row == -1 ? (const void *)feat_col : (const void *)src,
-                                             src_row == -1 ? 0u : 16u);
-                        }
-                    }
-                }
-                if (p.lag == 0) {
-                    cp_async_mbar_arrive(smem_u32(&s_a_full[slot]));   // fires once this thread's copies have landed
-                    if (++slot == (uint32_t)p.nslots) slot = 0, ++use;
-                    continue;
-                }
-                cp_async_commit();
-                // Hand over the tile issued SIGNAL_LAG tiles ago: its copies (a cp.async group of this
-                // thread) have landed once at most SIGNAL_LAG newer groups are pending.  One arrival
-                // per warp: an mbarrier takes arrivals one at a time, and one per thread and tile
-                // would cost more than the copies.
-                if (t >= SIGNAL_LAG) {
-                    cp_async_wait<SIGNAL_LAG>();
-                    fence_async_smem();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&s_a_full[signal_slot]));
-                    if (++signal_slot == (uint32_t)p.nslots) signal_slot = 0;
-                }
-                if (++slot == (uint32_t)p.nslots) slot = 0, ++use;
-              }
-            }
-            // the last tiles of the group
-            cp_async_wait<0>();
-            fence_async_smem();
-            __syncwarp();
-            for (int t = max(a_total - SIGNAL_LAG, 0); t < a_total && ok_role && p.lag; ++t) {
-                if (lane == 0) mbar_arrive(smem_u32(&s_a_full[signal_slot]));
-                if (++signal_slot == (uint32_t)p.nslots) signal_slot = 0;
-            }
-            ok_role = __all_sync(0xffffffffu, ok_role);
-            STAT_ADD(10, t_role);
-            STAT_T0(t_epi);
-            // ---------------------------------------------------------- epilogue ----
-            if (ok_role && a_total > 0) {
-                ok_role = mbar_wait_abortable(smem_u32(&s_d_full), d_n & 1u, STATUS_BIT, p.status, abort_flag, p.wait_limit_ns);
-                ok_role = __all_sync(0xffffffffu, ok_role);
-            }
-            STAT_ADD(11, t_epi);
-            tc_fence_after();
-            const int teams = p.npw >> 2;
-            if (ok_role && warp < teams * 4) {
-                const int quarter = warp & 3, team = warp >> 2;
-                const int chunks = p.outw >> 4;  // units of 16 columns
-                for (int u = team; u < nb * chunks; u += teams) {
-                    const int blk = u / chunks, cc = u - blk * chunks;
-                    const int32_t row = p.perm[(int64_t)(b0 + blk) * ROWS + quarter * 32 + lane];
-                    const bool blk_has = s_tab[(blk + 1) * p.K] > s_tab[blk * p.K];
-                    float acc[16];
-                    if (blk_has) {
-                        tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)blk * p.col_stride + (uint32_t)cc * 16, acc);
+            for (int b = 0; b < GROUP_BLOCKS && w.block0 + b < p.nblocks; ++b) {
+                const int64_t slot = (int64_t)(w.block0 + b) * ROWS + warp * 32 + lane;
+                const int32_t row = __ldg(p.perm + slot);
+                const bool has = (b ? any1 : any0) != 0u;
+                const uint32_t d = tmem + ((uint32_t)(warp * 32) << 16) + (acc.slot * 2 + (uint32_t)b) * p.col_stride;
+                for (int c0 = 0; c0 < p.outw; c0 += 16) {
+                    float v[16];
+                    if (has) {
+                        tmem_ld16(d + (uint32_t)c0, v);
                     } else {
 #pragma unroll
-                        for (int c = 0; c < 16; ++c) acc[c] = 0.f;
+                        for (int e = 0; e < 16; ++e) v[e] = 0.f;
                     }
                     if (row >= 0) {
-                        if (p.bias) {
+                        if (p.nsplit > 1) {
+                            float4 *dst = reinterpret_cast<float4 *>(
+                                p.partial + ((int64_t)(w.unit % p.nsplit) * p.nblocks * ROWS + slot) * p.outw + c0);
 #pragma unroll
-                            for (int c = 0; c < 16; ++c) {
-                                const uint16_t b = __ldg(p.bias + cc * 16 + c);
-                                acc[c] += p.fmt ? __bfloat162float(__ushort_as_bfloat16(b)) : __half2float(__ushort_as_half(b));
-                            }
-                        }
-                        uint4 *dst = reinterpret_cast<uint4 *>(p.out + (int64_t)row * p.outw + cc * 16);
-                        uint4 o;
-                        o.x = pack2(acc[0], acc[1], p.fmt), o.y = pack2(acc[2], acc[3], p.fmt);
-                        o.z = pack2(acc[4], acc[5], p.fmt), o.w = pack2(acc[6], acc[7], p.fmt);
-                        dst[0] = o;
-                        o.x = pack2(acc[8], acc[9], p.fmt), o.y = pack2(acc[10], acc[11], p.fmt);
-                        o.z = pack2(acc[12], acc[13], p.fmt), o.w = pack2(acc[14], acc[15], p.fmt);
-                        dst[1] = o;
-                    }
-                }
-            }
-            tc_fence_before();
-            STAT_ADD(12, t_epi);
-        } else if (warp == p.npw) {
-            // --------------------------------------------------------------- MMA ----
-            if (lane == 0) {
-                uint32_t slot = a_n % (uint32_t)p.nslots, use = a_n / (uint32_t)p.nslots;
-                uint32_t wslot = w_n % (uint32_t)p.nw, wuse = w_n / (uint32_t)p.nw;
-                uint32_t started = 0;
-                bool ok_role = true;
-                // descriptors of slot 0 / contraction step 0; the address field counts 16-byte units, so
-                // another slot or step is an addition to the low word
-                const uint64_t a_desc0 = smem_desc(a_base, 16, 1024);
-                const uint64_t b_desc0 = p.transpose ? smem_desc(w_base, 16, 1024) : smem_desc(w_base, p.w_box_rows * 128, 1024);
-                const uint32_t b_step = p.transpose ? 2u : 128u;  // 32 bytes along a K-major row / 16 contraction rows of 128 bytes
-                const uint32_t w_slot16 = p.w_slot_bytes >> 4;
-                for (int t = 0; t < a_total; ++t) {
-                    const int meta = s_task[t].z;
-                    const int blk = meta & 15, q = (meta >> 4) & 15;
-                    if (meta & 256) {  // first tile of a weight slice: the slice has landed
-                        STAT_T0(t_w);
-                        ok_role = mbar_wait_abortable(smem_u32(&s_w_full[wslot]), wuse & 1u, STATUS_BIT, p.status, abort_flag,
-                                                      p.wait_limit_ns);
-                        if (!ok_role) break;
-                        if (!p.use_tma) fence_async_smem();
-                        STAT_ADD(13, t_w);
-                    }
-                    STAT_T0(t_a);
-                    ok_role = mbar_wait_abortable(smem_u32(&s_a_full[slot]), use & 1u, STATUS_BIT, p.status, abort_flag,
-                                                  p.wait_limit_ns);
-                    if (!ok_role) break;
-                    STAT_ADD(14, t_a);
-                    fence_async_smem();   // the tile was written through the generic proxy, the tensor core reads through the async proxy
-                    tc_fence_after();
-                    const uint64_t ad = a_desc0 + (uint64_t)(slot * (SLOT_BYTES >> 4));
-                    const uint64_t bd = b_desc0 + (uint64_t)(wslot * w_slot16);
-                    const int ksteps = min(64, p.inw - q * 64) >> 4;
-                    const uint32_t d_addr = tmem + (uint32_t)blk * p.col_stride;
-                    const uint32_t first = (q > 0 || ((started >> blk) & 1u)) ? 1u : 0u;
-                    STAT_T0(t_m);
-                    tc_mma(d_addr, ad, bd, idesc, first);
-                    for (int s = 1; s < ksteps; ++s) tc_mma(d_addr, ad + (uint64_t)(2 * s), bd + (uint64_t)(b_step * s), idesc, 1u);
-                    STAT_ADD(18, t_m);
-                    started |= 1u << blk;
-                    STAT_T0(t_c);
-                    tc_commit(smem_u32(&s_a_empty[slot]));
-                    if (++slot == (uint32_t)p.nslots) slot = 0, ++use;
-                    if (meta & 512) {  // last tile of the weight slice: its slot is free once these MMAs are done
-                        tc_commit(smem_u32(&s_w_empty[wslot]));
-                        if (++wslot == (uint32_t)p.nw) wslot = 0, ++wuse;
-                    }
-                    STAT_ADD(19, t_c);
-                }
-                if (ok_role && a_total > 0) tc_commit(smem_u32(&s_d_full));
-                STAT_ADD(15, t_role);
-            }
-            __syncwarp();
-        } else {
-            // ------------------------------------------------------ weight loader ----
-            uint32_t wslot = w_n % (uint32_t)p.nw, wuse = w_n / (uint32_t)p.nw;
-            bool ok_role = true;
-            for (int wt = 0; wt < w_total && ok_role; ++wt) {
-                const int rb_tap = s_wtask[wt] & 0xffff, q = s_wtask[wt] >> 16;
-                const int tap = p.reverse ? p.K - 1 - rb_tap : rb_tap;
-                const uint32_t w_slot = w_base + wslot * p.w_slot_bytes, full = smem_u32(&s_w_full[wslot]);
-                STAT_T0(t_w);
-                ok_role = mbar_wait_abortable(smem_u32(&s_w_empty[wslot]), (wuse & 1u) ^ 1u, STATUS_BIT, p.status, abort_flag,
-                                              p.wait_limit_ns);
-                ok_role = __all_sync(0xffffffffu, ok_role);
-                STAT_ADD(16, t_w);
-                if (!ok_role) break;
-                if (p.use_tma) {
-                    if (lane == 0) {
-                        mbar_arrive_expect_tx(full, p.w_tx_bytes);
-                        if (p.transpose) {
-                            // contraction over m: the slice is the m-block q of all C rows of W[tap]
-                            tma_load_2d(w_slot, &tmap, q * 64, tap * p.C, full);
+                            for (int e = 0; e < 4; ++e) dst[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
                         } else {
-                            // contraction over c: rows [64q, 64q + box) of W[tap], one box per 64 output channels
-                            for (int mb = 0; mb * 64 < p.M; ++mb)
-                                tma_load_2d(w_slot + (uint32_t)mb * p.w_box_rows * 128, &tmap, mb * 64, tap * p.C + q * 64, full);
+                            if (p.bias) {
+#pragma unroll
+                                for (int e = 0; e < 16; ++e) v[e] += bias_at(p.bias, c0 + e, p.fmt);
+                            }
+                            uint4 *dst = reinterpret_cast<uint4 *>(p.out + (int64_t)row * p.outw + c0);
+#pragma unroll
+                            for (int e = 0; e < 2; ++e)
+                                dst[e] = make_uint4(pack2(v[8 * e], v[8 * e + 1], p.fmt), pack2(v[8 * e + 2], v[8 * e + 3], p.fmt),
+                                                    pack2(v[8 * e + 4], v[8 * e + 5], p.fmt), pack2(v[8 * e + 6], v[8 * e + 7], p.fmt));
                         }
                     }
-                } else {
-                    const uint16_t *w = p.weight + (int64_t)tap * p.C * p.M;
-                    if (p.transpose) {
-                        // rows c = 0..C-1, the 64 m-channels of block q (fewer in a last partial block)
-                        const int cpr = min(8, (p.M - q * 64) >> 3);
-                        for (int e = lane; e < p.C * cpr; e += 32) {
-                            const int c = e / cpr, ch = e - c * cpr;
-                            cp_async16(w_slot + (uint32_t)c * 128 + (uint32_t)((ch ^ (c & 7)) << 4),
-                                       w + (int64_t)c * p.M + q * 64 + ch * 8);
-                        }
-                    } else {
-                        // rows c = 64q .. 64q + rows - 1, all M channels in 64-channel blocks
-                        const int rows = min(64, p.C - q * 64), cpr = p.M >> 3;
-                        for (int e = lane; e < rows * cpr; e += 32) {
-                            const int c = e / cpr, ch = e - c * cpr;
-                            cp_async16(w_slot + (uint32_t)(ch >> 3) * p.w_box_rows * 128 + (uint32_t)c * 128 +
-                                           (uint32_t)(((ch & 7) ^ (c & 7)) << 4),
-                                       w + (int64_t)(q * 64 + c) * p.M + ch * 8);
-                        }
-                    }
-                    cp_async_mbar_arrive(full);
+                    __syncwarp();
                 }
-                if (++wslot == (uint32_t)p.nw) wslot = 0, ++wuse;
+            }
+            if (any0 | any1) {
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&s_acc_empty[acc.slot]));
+                acc.next(p.nacc);
             }
         }
-        if (warp == 0) STAT_ADD(17, t_group);
-        // counters advance identically in every role
-        a_n += (uint32_t)a_total;
-        w_n += (uint32_t)w_total;
-        d_n += a_total > 0 ? 1u : 0u;
-        __syncthreads();
-        if (s_abort) break;
+    } else if (warp < WALK_WARP) {
+        // ------------------------------------------------------------------ copies ----
+        // Two teams take the steps in turn: while one team's copies go through the load/store unit (230 clocks
+        // for a 16 KB tile) the other one waits for its slot and fetches its rows.  A warp owns 16 rows of
+        // either tile, eight lanes a row, a group of eight lanes four consecutive rows.
+        const int team = (warp - COPY_WARP0) / TEAM_WARPS, piece = lane & 7;
+        const int row0 = ((warp - COPY_WARP0) % TEAM_WARPS) * 16 + (lane >> 3) * 4;
+        uint32_t dst_off[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) dst_off[k] = (uint32_t)(row0 + k) * 128 + (uint32_t)((piece ^ ((row0 + k) & 7)) << 4);
+        Ring ring, step;
+        for (int n = 0;; n ^= 1) {   // (two teams)
+            if (n == team) {
+                if (!wait(s_step_full[step.slot], step.turn)) break;
+                const uint32_t word = *(volatile uint32_t *)&s_step[step.slot];
+                if (word & STEP_END) break;
+                const uint32_t at = rows0 + step.slot * ENTRY_BYTES + (uint32_t)row0 * 4;
+                const uint4 rows[2] = {lds_v4(at), lds_v4(at + ROWS * 4)};
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&s_step_empty[step.slot]));
+                const int slice = (int)(word >> 9) & 15;
+                const uint16_t *col = p.feat + slice * 64 + piece * 8, *sums = p.scratch + slice * 64 + piece * 8;
+                const bool piece_ok = piece * 8 < p.inw - slice * 64;
+                // the tensor core has finished with what was in the slot
+                if (!wait(s_empty[ring.slot], ring.turn ^ 1u)) break;
+                const uint32_t dst = slot0 + ring.slot * p.slot_bytes;
+                if (piece_ok) {
+#pragma unroll
+                    for (int t = 0; t < 2; ++t) {
+                        if (!((word >> (13 + t)) & 1u)) continue;
+                        const int32_t rr[4] = {(int32_t)rows[t].x, (int32_t)rows[t].y, (int32_t)rows[t].z, (int32_t)rows[t].w};
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) {
+                            // a feature row, a row of bucket sums, or nothing (zeros: source size 0)
+                            const uint32_t idx = (uint32_t)(rr[k] >= 0 ? rr[k] : rr[k] == -1 ? 0 : -2 - rr[k]);
+                            const uint16_t *src = (rr[k] < -1 ? sums : col) + (uint64_t)idx * (uint32_t)p.inw;
+                            cp_async16_zfill(dst + (uint32_t)t * SLOT_BYTES + dst_off[k], src, rr[k] == -1 ? 0u : 16u);
+                        }
+                    }
+                }
+                cp_async_mbar_arrive(smem_u32(&s_full[ring.slot]));   // fires once this thread's copies have landed
+            }
+            ring.next(p.nslots);
+            step.next(AHEAD);
+        }
+        cp_async_wait<0>();
+    } else if (warp == WALK_WARP) {
+        // -------------------------------------------------------------------- walk ----
+        // Decides the steps and brings the source rows of their tiles into shared memory, AHEAD steps early:
+        // the tables come from DRAM, once.
+        Walk w(p);
+        Ring step;
+        bool more = true;
+        for (int ends = 0; ends < TEAMS;) {   // an end mark for either team
+            if (!wait(s_step_empty[step.slot], step.turn ^ 1u)) break;
+            if (more) more = w.next();
+            const uint32_t entry = rows0 + step.slot * ENTRY_BYTES + (uint32_t)lane * 16, full = smem_u32(&s_step_full[step.slot]);
+            if (more) {
+                const int32_t *src = p.tile_rows + ((int64_t)w.block0 * p.K + w.tap) * ROWS + lane * 4;
+                if (w.has & 1u) cp_async16(entry, src);
+                if (w.has & 2u) cp_async16(entry + ROWS * 4, src + (int64_t)p.K * ROWS);
+            } else {
+                ++ends;
+            }
+            if (lane == 0) {
+                s_step[step.slot] = more ? (uint32_t)w.tap | ((uint32_t)w.q << 9) | (w.has << 13) | (w.first ? STEP_FIRST : 0u) : STEP_END;
+                mbar_arrive(full);
+            }
+            cp_async_mbar_arrive(full);
+            step.next(AHEAD);
+        }
+        cp_async_wait<0>();
+    } else if (warp == WEIGHT_WARP) {
+        // ---------------------------------------------------------------- weights ----
+        Ring ring, step;
+        for (;;) {
+            if (!wait(s_step_full[step.slot], step.turn)) break;
+            const uint32_t word = *(volatile uint32_t *)&s_step[step.slot];
+            if (word & STEP_END) break;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&s_step_empty[step.slot]));
+            const int tap_r = (int)(word & 511u), q = (int)(word >> 9) & 15, tap = p.reverse ? p.K - 1 - tap_r : tap_r;
+            if (!wait(s_empty[ring.slot], ring.turn ^ 1u)) break;
+            const uint32_t dst = slot0 + ring.slot * p.slot_bytes + 2 * SLOT_BYTES, full = smem_u32(&s_full[ring.slot]);
+            if (lane == 0) {
+                mbar_arrive_expect_tx(full, p.w_tx_bytes);
+                if (p.transpose) {   // contraction over m: the m-block q of all C rows of W[tap]
+                    tma_load_2d(dst, &tmap, q * 64, tap * p.C, full);
+                } else {             // contraction over c: rows [64q, 64q + box), one box per 64 output channels
+                    for (int mb = 0; mb * 64 < p.M; ++mb)
+                        tma_load_2d(dst + (uint32_t)mb * p.w_box_rows * 128, &tmap, mb * 64, tap * p.C + q * 64, full);
+                }
+            }
+            ring.next(p.nslots);
+            step.next(AHEAD);
+        }
+    } else {
+        // -------------------------------------------------------------------- MMA ----
+        // One warp per block of the group: the issue of a step (waits, descriptors, four tcgen05.mma, commit) is a
+        // serial chain of several hundred clocks, and with one warp for both tiles it bounded the kernel.
+        const int t = warp - MMA_WARP0;
+        const uint32_t idesc = instr_desc(p.fmt, ROWS, p.outw, 0, p.transpose ? 0 : 1);
+        // descriptors of slot 0 / contraction step 0; the address field counts 16-byte units, so another
+        // slot or step is an addition to the low word
+        const uint32_t w0 = slot0 + 2 * SLOT_BYTES;
+        const uint64_t a_desc0 = smem_desc(slot0 + (uint32_t)t * SLOT_BYTES, 16, 1024);
+        const uint64_t b_desc0 = p.transpose ? smem_desc(w0, 16, 1024) : smem_desc(w0, p.w_box_rows * 128, 1024);
+        const uint32_t b_step = p.transpose ? 2u : 128u;   // 32 bytes along a K-major row / 16 contraction rows of 128 bytes
+        Ring ring, acc, step;
+        uint32_t started = 0;
+        bool open = false, ok = true;
+        for (;;) {
+            ok = wait(s_step_full[step.slot], step.turn);
+            if (!ok) break;
+            const uint32_t word = *(volatile uint32_t *)&s_step[step.slot];
+            if (word & STEP_END) break;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&s_step_empty[step.slot]));
+            if (word & STEP_FIRST) {
+                if (open) {
+                    if (elect_one()) tc_commit(smem_u32(&s_acc_full[acc.slot]));
+                    acc.next(p.nacc);
+                }
+                ok = wait(s_acc_empty[acc.slot], acc.turn ^ 1u);
+                if (!ok) break;
+                open = true, started = 0;
+            }
+            ok = wait(s_full[ring.slot], ring.turn);
+            if (!ok) break;
+            if ((word >> (13 + t)) & 1u) {
+                fence_async_smem();   // the copies came through the generic proxy, the tensor core reads through the async proxy
+                tc_fence_after();
+                const uint64_t at = (uint64_t)(ring.slot * (p.slot_bytes >> 4));
+                const int ksteps = min(64, p.inw - (int)((word >> 9) & 15) * 64) >> 4;
+                const uint64_t ad = a_desc0 + at, bd = b_desc0 + at;
+                const uint32_t d = tmem + (acc.slot * 2 + (uint32_t)t) * p.col_stride;
+                if (elect_one()) {
+                    tc_mma(d, ad, bd, idesc, started);
+                    if (ksteps == 4) {
+                        tc_mma(d, ad + 2, bd + b_step, idesc, 1u);
+                        tc_mma(d, ad + 4, bd + 2 * b_step, idesc, 1u);
+                        tc_mma(d, ad + 6, bd + 3 * b_step, idesc, 1u);
+                    } else {
+                        for (int k = 1; k < ksteps; ++k) tc_mma(d, ad + (uint64_t)(2 * k), bd + (uint64_t)(b_step * k), idesc, 1u);
+                    }
+                    tc_commit(smem_u32(&s_empty[ring.slot]));
+                }
+                started = 1u;
+            } else if (lane == 0) {
+                mbar_arrive(smem_u32(&s_empty[ring.slot]));
+            }
+            __syncwarp();
+            ring.next(p.nslots);
+            step.next(AHEAD);
+        }
+        if (ok && open && elect_one()) tc_commit(smem_u32(&s_acc_full[acc.slot]));
+        __syncwarp();
     }
-
     tc_fence_before();
     __syncthreads();
     if (warp == 0) tmem_dealloc(tmem, p.ncols);
-    // the last CTA to finish re-arms the ticket counter for the next launch
-    if (tid == 0) {
-        __threadfence();
-        const uint32_t done = atomicAdd(&p.ctrl[CTRL_DONE], 1u);
-        if (done == gridDim.x - 1) {
-            p.ctrl[CTRL_TICKET] = 0u;
-            p.ctrl[CTRL_DONE] = 0u;
-            __threadfence();
-        }
+}
+
+// out[perm[slot]] = the parts of a split group added in order, plus the bias, rounded once
+__global__ void os_reduce_kernel(const float *__restrict__ partial, const int32_t *__restrict__ perm, const uint16_t *__restrict__ bias,
+                                 int64_t slots, int outw, int nsplit, int fmt, uint16_t *out) {
+    const int ppr = outw >> 3;
+    const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= slots * ppr) return;
+    const int64_t slot = x / ppr;
+    const int c = (int)(x - slot * ppr) * 8;
+    const int32_t row = perm[slot];
+    if (row < 0) return;
+    float v[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = bias ? bias_at(bias, c + e, fmt) : 0.f;
+#pragma unroll 4
+    for (int s = 0; s < nsplit; ++s) {
+        const float4 *src = reinterpret_cast<const float4 *>(partial + ((int64_t)s * slots + slot) * outw + c);
+        const float4 a = __ldcs(src), b = __ldcs(src + 1);
+        v[0] += a.x, v[1] += a.y, v[2] += a.z, v[3] += a.w, v[4] += b.x, v[5] += b.y, v[6] += b.z, v[7] += b.w;
     }
+    *reinterpret_cast<uint4 *>(out + (int64_t)row * outw + c) =
+        make_uint4(pack2(v[0], v[1], fmt), pack2(v[2], v[3], fmt), pack2(v[4], v[5], fmt), pack2(v[6], v[7], fmt));
 }
 
 // A single thread waits on an mbarrier that nothing arrives at: the bounded wait runs out,
@@ -794,9 +756,27 @@ uint64_t wait_limit() {
     return v;
 }
 
+// Parts the taps of a group are split into when the groups alone do not fill the chip: the count with the
+// smallest time, a part costing a tenth of a whole group more than its share (its fp32 sums go through
+// memory).  1000 points of 256 channels, 4 groups: 183 us on 4 CTAs, 28 us in 27 parts per group.
+int split_parts(int64_t ngroups, int K) {
+    const int sms = num_sms();
+    int best = 1;
+    double best_cost = 1e30;
+    for (int s = 1; s <= std::min(K, 64) && ngroups < 2 * sms; ++s) {
+        const double waves = (double)((ngroups * s + sms - 1) / sms), cost = waves * (1.0 / s + (s > 1 ? 0.1 : 0.0));
+        if (cost < best_cost * 0.999) best_cost = cost, best = s;
+    }
+    return best;
+}
+
+size_t partial_bytes(int64_t n_out, int outw, int parts) {
+    return parts > 1 ? (size_t)parts * ((n_out + ROWS - 1) / ROWS) * ROWS * outw * sizeof(float) : 0;
+}
+
 bool plan_sizes_ok(int64_t T, int64_t n_out, int K, int G) {
     if (T < 0 || T > INT32_MAX || n_out <= 0 || n_out > INT32_MAX || K <= 0 || K > MAX_TAPS) return false;
-    if (G < 1 || G > MAX_GROUP) return false;
+    if (G != GROUP_BLOCKS) return false;
     const int64_t nblocks = (n_out + ROWS - 1) / ROWS;
     return nblocks * K * ROWS <= ((int64_t)1 << 32) && nblocks * K < INT32_MAX;
 }
@@ -810,16 +790,9 @@ extern "C" {
 
 int pcx_mvmr_plan_group_blocks(int out_width) {
     if (out_width <= 0 || out_width > 256) return 0;
-    const int stride = (out_width + 31) / 32 * 32;
-    // Two blocks per group, measured best at every width: up to 128 channels two accumulators fit
-    // half of the tensor memory (two CTAs per SM), at 256 channels they fill it (one CTA per SM);
-    // larger groups share each weight tile among more blocks but balance worse.
-    int g = 2;
-    if (const char *e = getenv("PCX_OS_GROUP")) {
-        const int want = atoi(e);
-        if (want >= 1 && want <= MAX_GROUP && want * stride <= 512) g = want;
-    }
-    return g;
+    // Two: both accumulators of the widest rows (256 channels) fill the tensor memory, and every weight
+    // slice that is streamed serves 256 output rows.
+    return GROUP_BLOCKS;
 }
 
 size_t pcx_mvmr_plan_bytes(int64_t T, int64_t n_out, int K, int group_blocks) {
@@ -892,7 +865,7 @@ int pcx_mvmr_plan_build(const int32_t *d_scatter, const int32_t *d_gather, const
                                                            pv.ctrl);
         PCX_LAUNCH_CHECK();
     }
-    plan_cost_kernel<<<blocks(pv.ngroups), TPB, 0, stream>>>(pv.tile_offs, pv.nblocks, K, G, pv.ngroups, w.cost, w.gid);
+    plan_cost_kernel<<<blocks(pv.ngroups), TPB, 0, stream>>>(pv.tile_offs, pv.nblocks, K, G, pv.ngroups, w.cost, w.gid, pv.tap_masks);
     PCX_LAUNCH_CHECK();
     bytes = w.cub_bytes;
     PCX_CUDA(cub::DeviceRadixSort::SortPairsDescending(w.cub_tmp, bytes, w.cost, w.cost_sorted, w.gid, pv.group_order,
@@ -903,6 +876,12 @@ int pcx_mvmr_plan_build(const int32_t *d_scatter, const int32_t *d_gather, const
 size_t pcx_mvmr_planned_workspace_bytes(int64_t multi_buckets, int in_width) {
     if (multi_buckets < 0 || in_width <= 0) return 0;
     return align_up((size_t)std::max<int64_t>(multi_buckets, 1) * in_width * 2, 256);
+}
+
+size_t pcx_mvmr_planned_scratch_bytes(int64_t multi_buckets, int in_width, int64_t n_out, int out_width, int K) {
+    if (multi_buckets < 0 || in_width <= 0 || n_out <= 0 || out_width <= 0 || K <= 0) return 0;
+    const int64_t ngroups = (n_out + GROUP_BLOCKS * ROWS - 1) / (GROUP_BLOCKS * ROWS);
+    return pcx_mvmr_planned_workspace_bytes(multi_buckets, in_width) + partial_bytes(n_out, out_width, split_parts(ngroups, K));
 }
 
 int pcx_mvmr_plan_multi_buckets(const void *d_plan, int64_t *h_count, void *stream_) {
@@ -948,86 +927,55 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     if (plan_bytes < need_plan) PCX_FAIL(PCX_E_CAPACITY, "pcx_mvmr_planned: plan buffer %zu < %zu bytes", plan_bytes, need_plan);
 
     OsParams p = {};
-    p.feat = (const uint16_t *)d_feat, p.out = (uint16_t *)d_out, p.weight = (const uint16_t *)d_weight;
-    p.perm = pv.perm, p.tile_offs = pv.tile_offs, p.group_order = pv.group_order, p.entries = pv.entries, p.ctrl = pv.ctrl;
-    p.tile_rows = pv.tile_rows, p.scratch = (const uint16_t *)d_ws;
-    p.bias = (const uint16_t *)d_bias, p.reverse = (flags & PCX_MVMR_REVERSE_TAPS) ? 1 : 0;
+    p.feat = (const uint16_t *)d_feat, p.out = (uint16_t *)d_out, p.bias = (const uint16_t *)d_bias;
+    p.perm = pv.perm, p.group_order = pv.group_order, p.tile_rows = pv.tile_rows, p.tap_masks = pv.tap_masks;
+    p.scratch = (const uint16_t *)d_ws;
     p.status = status_word();
     if (!p.status) PCX_FAIL(PCX_E_LAUNCH, "pcx_mvmr_planned: no device status word");
     p.K = K, p.C = C, p.M = M, p.transpose = transpose ? 1 : 0, p.fmt = dtype == PCX_BF16 ? 1 : 0;
-    p.inw = inw, p.outw = outw, p.nkb = (inw + 63) / 64, p.G = G;
+    p.reverse = (flags & PCX_MVMR_REVERSE_TAPS) ? 1 : 0;
+    p.inw = inw, p.outw = outw, p.nkb = (inw + 63) / 64, p.mask_words = (K + 31) / 32;
     p.ngroups = (int)pv.ngroups, p.nblocks = (int)pv.nblocks;
     p.col_stride = (uint32_t)((outw + 31) / 32 * 32);
-    if ((uint32_t)G * p.col_stride > 512u)
-        PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_planned: %d blocks of %d columns exceed the 512 TMEM columns", G, (int)p.col_stride);
+    p.nacc = 4 * p.col_stride <= 512 ? 2 : 1;   // up to 128 channels the next group starts while the last one is written
     p.ncols = 32;
-    while (p.ncols < (uint32_t)G * p.col_stride) p.ncols <<= 1;
+    while (p.ncols < 2u * (uint32_t)p.nacc * p.col_stride) p.ncols <<= 1;
     p.w_box_rows = (uint32_t)(transpose ? C : std::min(64, C));
-    const uint32_t w_image = transpose ? (uint32_t)C * 128u : (uint32_t)((M + 63) / 64) * p.w_box_rows * 128u;
-    p.w_slot_bytes = (uint32_t)align_up(w_image, 1024);
-    p.w_tx_bytes = w_image;
+    p.w_tx_bytes = transpose ? (uint32_t)C * 128u : (uint32_t)((M + 63) / 64) * p.w_box_rows * 128u;
+    p.slot_bytes = 2 * SLOT_BYTES + (uint32_t)align_up(p.w_tx_bytes, 1024);
     p.wait_limit_ns = wait_limit();
-    p.use_tma = (M % 64 == 0) && encode_tiled() != nullptr;
-    if (const char *e = getenv("PCX_OS_WTMA")) p.use_tma = p.use_tma && atoi(e) != 0;
+    if (!encode_tiled()) PCX_FAIL(PCX_E_LAUNCH, "pcx_mvmr_planned: the driver offers no cuTensorMapEncodeTiled");
 
+    // widths that are not multiples of 64: the last box of a row ends in zero fill
     CUtensorMap tmap;
     memset(&tmap, 0, sizeof(tmap));
-    if (p.use_tma) {
-        const cuuint64_t gdim[2] = {(cuuint64_t)M, (cuuint64_t)K * (cuuint64_t)C};
-        const cuuint64_t gstride[1] = {(cuuint64_t)M * 2};
-        const cuuint32_t box[2] = {64u, p.w_box_rows};
-        const cuuint32_t estride[2] = {1u, 1u};
-        const CUresult r = encode_tiled()(&tmap, dtype == PCX_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                                          2, const_cast<void *>(d_weight), gdim, gstride, box, estride,
-                                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                          CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-        if (r != CUDA_SUCCESS) PCX_FAIL(PCX_E_LAUNCH, "pcx_mvmr_planned: cuTensorMapEncodeTiled failed (%d)", (int)r);
-    }
+    const cuuint64_t gdim[2] = {(cuuint64_t)M, (cuuint64_t)K * (cuuint64_t)C};
+    const cuuint64_t gstride[1] = {(cuuint64_t)M * 2};
+    const cuuint32_t box[2] = {64u, p.w_box_rows};
+    const cuuint32_t estride[2] = {1u, 1u};
+    const CUresult r = encode_tiled()(&tmap, dtype == PCX_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
+                                      const_cast<void *>(d_weight), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) PCX_FAIL(PCX_E_LAUNCH, "pcx_mvmr_planned: cuTensorMapEncodeTiled failed (%d)", (int)r);
 
-    // Two CTAs share an SM when their accumulators fit half of the tensor memory: while one
-    // writes its output rows or sets up its next group, the other keeps the tensor core and the
-    // gathers going, and two threads issue MMAs.  Shared memory per CTA: A slots, weight slots,
-    // the group's task tables.
-    int ctas = p.ncols <= 256 ? 2 : 1;
-    if (const char *e = getenv("PCX_OS_CTAS")) ctas = (atoi(e) == 1 || p.ncols > 256) ? 1 : 2;
-    const size_t nkb = (size_t)p.nkb;
-    const size_t table_fixed = align_up((size_t)G * K * nkb * 16 + ((size_t)G * K * 3 + 1 + (size_t)K * nkb) * 4, 16);
-    const size_t static_smem = 512;
-    int nslots = 0, nw = 0;
-    for (; ctas >= 1 && !nslots; --ctas) {
-        const size_t budget = (size_t)232448 / ctas - 1024 - static_smem - 1024;
-        for (int a = MAX_SLOTS; a >= SIGNAL_LAG + 2 && !nslots; --a)
-            for (int b = (ctas == 2 ? 3 : MAX_NW); b >= 2 && !nslots; --b)
-                if ((size_t)a * SLOT_BYTES + (size_t)b * p.w_slot_bytes + table_fixed <= budget) nslots = a, nw = b;
-        if (nslots) break;
-    }
-    if (!nslots) PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_planned: shared memory does not fit (K=%d C=%d M=%d group=%d)", K, C, M, G);
-    int npw = MAX_NPW;
-    if (const char *e = getenv("PCX_OS_WARPS")) {
-        const int want = atoi(e);
-        if (want == 4 || want == 8) npw = want;
-    }
-    if (const char *e = getenv("PCX_OS_SLOTS")) {
-        const int want = atoi(e);
-        if (want >= SIGNAL_LAG + 2 && want <= nslots) nslots = want;
-    }
-    if (const char *e = getenv("PCX_OS_WSLOTS")) {
-        const int want = atoi(e);
-        if (want >= 2 && want <= nw) nw = want;
-    }
-    p.npw = npw, p.nslots = nslots, p.nw = nw;
-    p.lag = 0;
-    if (const char *e = getenv("PCX_OS_LAG")) p.lag = atoi(e) ? SIGNAL_LAG : 0;
-    const size_t smem = 1024 + (size_t)nslots * SLOT_BYTES + (size_t)nw * p.w_slot_bytes + table_fixed;
+    // as many slots as fit: three of 64 KB at 256 output channels, five of 40 KB at 64
+    p.nslots = (int)std::min<size_t>(MAX_SLOTS, ((size_t)232448 - 1024 - 1024 - AHEAD * ENTRY_BYTES) / p.slot_bytes);
+    if (p.nslots < 2) PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_planned: shared memory does not fit (C=%d M=%d)", C, M);
+    // the fp32 sums of a split rulebook lie behind the bucket sums; a caller that made no room for them gets one part
+    const size_t sums_bytes = pcx_mvmr_planned_workspace_bytes(multi_buckets, inw);
+    p.nsplit = split_parts(pv.ngroups, K);
+    if (p.nsplit > 1 && (!d_ws || ws_bytes < sums_bytes + partial_bytes(n_out, outw, p.nsplit))) p.nsplit = 1;
+    p.partial = p.nsplit > 1 ? (float *)((char *)d_ws + sums_bytes) : nullptr;
+    const size_t smem = 1024 + (size_t)p.nslots * p.slot_bytes + AHEAD * ENTRY_BYTES;
     static int granted[64] = {};
     int dev = 0;
     PCX_CUDA(cudaGetDevice(&dev));
     if ((int)smem > granted[dev & 63]) {
         PCX_CUDA(cudaFuncSetAttribute(mvmr_os_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        PCX_CUDA(cudaFuncSetAttribute(mvmr_os_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
         granted[dev & 63] = (int)smem;
     }
-    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(pv.ngroups, (int64_t)ctas * num_sms()));
+    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(pv.ngroups * p.nsplit, num_sms()));
     if (multi_buckets > 0) {
         prof_begin("bucket_sum_kernel", stream);
         if (p.fmt) launch_bucket_sum<1>(multi_buckets, inw, p.feat, pv.entries, pv.buckets, pv.ctrl, (uint16_t *)d_ws, stream);
@@ -1036,9 +984,15 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
         PCX_LAUNCH_CHECK();
     }
     prof_begin(transpose ? "mvmr_os_kernel(dgrad)" : "mvmr_os_kernel(fwd)", stream);
-    mvmr_os_kernel<<<grid, (unsigned)(npw + 2) * 32, smem, stream>>>(tmap, p);
+    mvmr_os_kernel<<<grid, THREADS, smem, stream>>>(tmap, p);
     prof_end(stream);
     PCX_LAUNCH_CHECK();
+    if (p.nsplit > 1) {
+        const int64_t slots = pv.nblocks * ROWS;
+        os_reduce_kernel<<<(unsigned)((slots * (outw / 8) + 255) / 256), 256, 0, stream>>>(p.partial, p.perm, p.bias, slots, outw, p.nsplit,
+                                                                                           p.fmt, p.out);
+        PCX_LAUNCH_CHECK();
+    }
     return PCX_OK;
 }
 
