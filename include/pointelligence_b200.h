@@ -128,6 +128,12 @@ int pcx_mvmr_bias(const void *d_weight, const void *d_feat,
                   int dtype, int engine, void *d_ws, size_t ws_bytes,
                   void *stream);
 
+/* Copies `outer` matrices of 16-bit elements into a larger or smaller shape:
+ * rows and columns that the source lacks are zero, surplus ones are dropped.
+ * Pads channel counts to what the tensor engines take and crops their results. */
+int pcx_reshape16(const void *d_src, void *d_dst, int64_t outer, int rows_in,
+                  int cols_in, int rows_out, int cols_out, void *stream);
+
 /* out[c] = sum over r of x[r, c], fp32 sums, one rounding: the bias gradient. */
 size_t pcx_column_sums_workspace_bytes(int64_t N, int C);
 int pcx_column_sums(const void *d_x, void *d_out, int64_t N, int C, int dtype,
@@ -184,16 +190,19 @@ int pcx_mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan,
                      int64_t n_out, int K, int C, int M, int transpose,
                      int dtype, int group_blocks, int64_t multi_buckets,
                      void *d_ws, size_t ws_bytes, void *stream);
-/* ... with a bias and `flags` in place of `transpose`, as pcx_mvmr_bias.  A
+/* ... with a bias, `flags` in place of `transpose` and a grouped weight, as
+ * pcx_mvmr_bias; output rows of a group may be wider than 256 channels where
+ * ceil(width / 256) equal parts of a multiple of 16 channels make them up.  A
  * workspace of pcx_mvmr_planned_scratch_bytes() lets a small rulebook be split
  * over the whole chip (its fp32 sums go through the workspace); with less it
  * runs on as many SMs as it has groups. */
 size_t pcx_mvmr_planned_scratch_bytes(int64_t multi_buckets, int in_width,
-                                      int64_t n_out, int out_width, int K);
+                                      int64_t n_out, int out_width, int K,
+                                      int G);
 int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat,
                           void *d_plan, size_t plan_bytes, const void *d_bias,
                           void *d_out, int64_t T, int64_t n_feat, int64_t n_out,
-                          int K, int C, int M, int flags, int dtype,
+                          int K, int G, int C, int M, int flags, int dtype,
                           int group_blocks, int64_t multi_buckets, void *d_ws,
                           size_t ws_bytes, void *stream);
 

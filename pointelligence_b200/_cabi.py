@@ -48,6 +48,7 @@ SIGNATURES = {
     "pcx_mvmr_workspace_bytes": (c_size_t, [c_int64, c_int, c_int, c_int, c_int, c_int, c_int]),
     "pcx_mvmr": (c_int, [c_void_p] * 7 + [c_int64] * 3 + [c_int] * 7 + [c_void_p, c_size_t, c_void_p]),
     "pcx_mvmr_bias": (c_int, [c_void_p] * 8 + [c_int64] * 3 + [c_int] * 7 + [c_void_p, c_size_t, c_void_p]),
+    "pcx_reshape16": (c_int, [c_void_p] * 2 + [c_int64] + [c_int] * 4 + [c_void_p]),
     "pcx_column_sums_workspace_bytes": (c_size_t, [c_int64, c_int]),
     "pcx_column_sums": (c_int, [c_void_p] * 2 + [c_int64, c_int, c_int, c_void_p, c_size_t, c_void_p]),
     "pcx_mvmr_plan_group_blocks": (c_int, [c_int]),
@@ -59,8 +60,8 @@ SIGNATURES = {
     "pcx_mvmr_planned_workspace_bytes": (c_size_t, [c_int64, c_int]),
     "pcx_mvmr_planned": (c_int, [c_void_p] * 3 + [c_size_t, c_void_p] + [c_int64] * 3 + [c_int] * 6
                          + [c_int64, c_void_p, c_size_t, c_void_p]),
-    "pcx_mvmr_planned_scratch_bytes": (c_size_t, [c_int64, c_int, c_int64, c_int, c_int]),
-    "pcx_mvmr_planned_bias": (c_int, [c_void_p] * 3 + [c_size_t] + [c_void_p] * 2 + [c_int64] * 3 + [c_int] * 6
+    "pcx_mvmr_planned_scratch_bytes": (c_size_t, [c_int64, c_int, c_int64, c_int, c_int, c_int]),
+    "pcx_mvmr_planned_bias": (c_int, [c_void_p] * 3 + [c_size_t] + [c_void_p] * 2 + [c_int64] * 3 + [c_int] * 7
                               + [c_int64, c_void_p, c_size_t, c_void_p]),
     "pcx_debug_wait_runs_out": (c_int, [ctypes.c_ulonglong, c_void_p]),
     "pcx_vvor_workspace_bytes": (c_size_t, [c_int64, c_int, c_int, c_int, c_int]),
@@ -407,17 +408,23 @@ class MvmrPlan:
 
 def plan_group_blocks(out_width):
     """Blocks of 128 output rows that share the weight tiles they stream, for rows of ``out_width`` channels."""
-    return int(lib().pcx_mvmr_plan_group_blocks(int(out_width)))
+    return int(lib().pcx_mvmr_plan_group_blocks(min(int(out_width), 256)))
+
+
+def padded_width(width):
+    """Channels the tensor engines work on for a row of ``width``: parts of at most 256, multiples of 16."""
+    unit = 16 * ((width + 255) // 256)
+    return (width + unit - 1) // unit * unit
 
 
 def planned_supported(weight, feat, gather, scatter, seg_offs, n_out, transpose):
-    """Whether the output-stationary kernel takes this call (fp16 / bf16, one group, tap-sorted
-    int32 triplets, channel counts that are multiples of 16, output rows of at most 256 channels)."""
+    """Whether the output-stationary kernel takes this call (fp16 / bf16, tap-sorted int32 triplets;
+    channel counts are padded on the way)."""
     K, G, C, M = weight.shape
-    inw, outw = (M, C) if transpose else (C, M)
-    if G != 1 or seg_offs is None or feat.dtype not in (torch.float16, torch.bfloat16) or n_out <= 0:
+    inw, outw = (padded_width(M), padded_width(C)) if transpose else (padded_width(C), padded_width(M))
+    if seg_offs is None or feat.dtype not in (torch.float16, torch.bfloat16) or n_out <= 0:
         return False
-    if inw % 16 or outw % 16 or outw > 256 or inw > 1024 or K > 512:
+    if inw > 1024 or G * inw > 2048 or K > 512 or G * ((outw + 255) // 256) > 64:
         return False
     T = gather.numel()
     nblocks = (int(n_out) + 127) // 128
@@ -535,7 +542,7 @@ def prepare_mvmr(weight, gather, scatter, seg_offs, n_out, transpose=False):
     was prepared, False when the policy keeps the scatter engines (which need no preparation)."""
     K, G, C, M = weight.shape
     n_out = int(n_out)
-    outw = C if transpose else M
+    outw = padded_width(C if transpose else M)
     if not (gather is not None and gather.is_cuda and planned_supported(weight, weight, gather, scatter, seg_offs,
                                                                         n_out, transpose)):
         return False

@@ -132,6 +132,23 @@ int launch_fill(float *acc, const void *bias, int64_t rows, int width, cudaStrea
     return PCX_OK;
 }
 
+// dst[o][r][c] = src[o][r][c] where it exists, else zero, for 16-bit elements: rows and columns of a matrix
+// are added (padding to the tensor core's channel counts) or dropped.  V output columns per thread.
+template <int V>
+__global__ void reshape16_kernel(const uint16_t *__restrict__ src, uint16_t *__restrict__ dst, int64_t pieces, int r_in, int c_in, int r_out,
+                                 int c_out) {
+    const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (x >= pieces) return;
+    const int per_row = c_out / V;
+    const int64_t row = x / per_row, o = row / r_out;
+    const int c = (int)(x - row * per_row) * V, r = (int)(row - o * r_out);
+    uint16_t v[V];
+#pragma unroll
+    for (int e = 0; e < V; ++e) v[e] = r < r_in && c + e < c_in ? __ldg(src + (o * r_in + r) * c_in + c + e) : (uint16_t)0;
+    if (V == 8) *reinterpret_cast<uint4 *>(dst + row * c_out + c) = *reinterpret_cast<const uint4 *>(v);
+    else dst[row * c_out + c] = v[0];
+}
+
 }  // namespace
 
 // Every row of the accumulator starts as `bias` (zeros when null): the bias of a layer costs the store
@@ -154,6 +171,21 @@ int clear_accumulator(float *acc, const void *bias, int64_t rows, int width, int
 using namespace pcx;
 
 extern "C" {
+
+int pcx_reshape16(const void *d_src, void *d_dst, int64_t outer, int rows_in, int cols_in, int rows_out, int cols_out, void *stream_) {
+    cudaStream_t stream = (cudaStream_t)stream_;
+    if (outer < 0 || rows_in <= 0 || cols_in <= 0 || rows_out <= 0 || cols_out <= 0) PCX_FAIL(PCX_E_ARG, "pcx_reshape16: bad sizes");
+    if (outer == 0) return PCX_OK;
+    if (!d_src || !d_dst) PCX_FAIL(PCX_E_ARG, "pcx_reshape16: null pointer");
+    const bool wide = cols_out % 8 == 0 && (uintptr_t)d_dst % 16 == 0;
+    const int64_t pieces = outer * rows_out * (cols_out / (wide ? 8 : 1));
+    if ((pieces + 255) / 256 > INT32_MAX) PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_reshape16: too large");
+    const unsigned grid = (unsigned)((pieces + 255) / 256);
+    if (wide) reshape16_kernel<8><<<grid, 256, 0, stream>>>((const uint16_t *)d_src, (uint16_t *)d_dst, pieces, rows_in, cols_in, rows_out, cols_out);
+    else reshape16_kernel<1><<<grid, 256, 0, stream>>>((const uint16_t *)d_src, (uint16_t *)d_dst, pieces, rows_in, cols_in, rows_out, cols_out);
+    PCX_LAUNCH_CHECK();
+    return PCX_OK;
+}
 
 size_t pcx_column_sums_workspace_bytes(int64_t N, int C) {
     if (N < 0 || C <= 0) return 0;

@@ -101,10 +101,24 @@ Plan ask_plan(const Tensor &scatter, const Tensor &gather, const Tensor &seg, in
     return plan;
 }
 
-// Shapes and types the output-stationary kernel takes (one group, 16-bit elements, widths in sixteens).
+// Channels the tensor engines work on for a row of `width`: parts of at most 256 channels, multiples of 16.
+int64_t padded(int64_t width) {
+    const int64_t unit = 16 * ((width + 255) / 256);
+    return (width + unit - 1) / unit * unit;
+}
+bool is_half(at::ScalarType t) { return t == at::kHalf || t == at::kBFloat16; }
+
+// `outer` matrices (rows x cols) of 16-bit elements in another shape, zeros where the source has nothing
+Tensor reshape16(const Tensor &src, int64_t outer, int64_t rows, int64_t cols, int64_t rows_out, int64_t cols_out, at::IntArrayRef shape) {
+    Tensor dst = at::empty(shape, src.options());
+    check(pcx_reshape16(ptr(src), ptr(dst), outer, (int)rows, (int)cols, (int)rows_out, (int)cols_out, stream()));
+    return dst;
+}
+
+// Shapes and types the output-stationary kernel takes (16-bit elements, widths in sixteens).
 bool plan_fits(at::ScalarType dtype, int64_t T, int64_t n_out, int64_t K, int64_t G, int64_t inw, int64_t outw, bool has_seg) {
-    if (G != 1 || !has_seg || (dtype != at::kHalf && dtype != at::kBFloat16) || n_out <= 0) return false;
-    if (inw % 16 || outw % 16 || outw > 256 || inw > 1024 || K > 512) return false;
+    if (!has_seg || !is_half(dtype) || n_out <= 0) return false;
+    if (inw != padded(inw) || outw != padded(outw) || inw > 1024 || G * inw > 2048 || K > 512 || G * ((outw + 255) / 256) > 64) return false;
     const int64_t nblocks = (n_out + 127) / 128;
     return T < (int64_t(1) << 31) && nblocks * K * 128 <= (int64_t(1) << 32);
 }
@@ -113,14 +127,14 @@ constexpr int ENGINE_PLANNED = 3;
 
 Tensor mvmr_planned(const Tensor &weight, const Tensor &feat, const Plan &plan, int64_t T, int64_t n_out, int flags,
                     const Tensor &bias) {
-    const int64_t K = weight.size(0), C = weight.size(2), M = weight.size(3);
+    const int64_t K = weight.size(0), G = weight.size(1), C = weight.size(2), M = weight.size(3);
     const bool transpose = flags & 1;
     const int64_t inw = transpose ? M : C, outw = transpose ? C : M;
-    Tensor out = at::empty({n_out, outw}, feat.options());
-    const size_t bytes = pcx_mvmr_planned_scratch_bytes(plan.multi, (int)inw, n_out, (int)outw, (int)K);
+    Tensor out = at::empty({n_out, G * outw}, feat.options());
+    const size_t bytes = pcx_mvmr_planned_scratch_bytes(plan.multi, (int)inw, n_out, (int)outw, (int)K, (int)G);
     Tensor ws = workspace(bytes, feat);
     check(pcx_mvmr_planned_bias(ptr(weight), ptr(feat), ptr(plan.buffer), plan.buffer.numel(), ptr(bias), ptr(out), T, feat.size(0),
-                                n_out, (int)K, (int)C, (int)M, flags, dtype_code(feat.scalar_type()), (int)plan.group, plan.multi,
+                                n_out, (int)K, (int)G, (int)C, (int)M, flags, dtype_code(feat.scalar_type()), (int)plan.group, plan.multi,
                                 ptr(ws), ws.numel(), stream()));
     return out;
 }
@@ -138,6 +152,17 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
     const bool transpose = flags & 1;
     const int64_t inw = transpose ? M : C, outw = transpose ? C : M, T = gather_.numel();
     c10::cuda::CUDAGuard guard(feat.device());
+    if ((engine & 0xff) == 0 && is_half(feat.scalar_type()) && seg_ && T > 0 && n_out > 0 && K <= 1024 && G <= 64 &&
+        (C != padded(C) || M != padded(M))) {
+        // channel counts the tensor engines do not take (the 3 or 6 channels of an input, 20 classes): zero columns
+        // make them up; the CUDA-core engine needed 0.72 ms for a 6 -> 32 layer of 125 taps at 80 000 points
+        const int64_t Cp = padded(C), Mp = padded(M), inp = transpose ? Mp : Cp, outp = transpose ? Cp : Mp;
+        const Tensor w = reshape16(weight, K * G, C, M, Cp, Mp, {K, G, Cp, Mp});
+        const Tensor x = inp == inw ? feat : reshape16(feat, feat.size(0) * G, 1, inw, 1, inp, {feat.size(0), G * inp});
+        const Tensor b = !bias.defined() || outp == outw ? bias : reshape16(bias.contiguous(), G, 1, outw, 1, outp, {G * outp});
+        const Tensor y = mvmr_impl(w, x, gather_, scatter_, seg_, tap_, n_out, flags, engine, b);
+        return outp == outw ? y : reshape16(y, n_out * G, 1, outp, 1, outw, {n_out, G * outw});
+    }
     if (engine == 0 || engine == ENGINE_PLANNED) {
         const bool fits = plan_fits(feat.scalar_type(), T, n_out, K, G, inw, outw, seg_.has_value());
         if (engine == ENGINE_PLANNED && !fits) {
@@ -176,6 +201,13 @@ Tensor vvor(Tensor a, const Tensor &a_idx_, Tensor b, const Tensor &b_idx_, cons
     a = a.contiguous(), b = b.contiguous();
     const int64_t G = a.size(1), Ma = a.size(2), Cb = b.size(2);
     c10::cuda::CUDAGuard guard(a.device());
+    if (engine == 0 && is_half(a.scalar_type()) && seg_ && a_idx_.numel() > 0 && n_o <= 1024 && G <= 64 &&
+        (Ma != padded(Ma) || Cb != padded(Cb))) {
+        const int64_t Mp = padded(Ma), Cp = padded(Cb);
+        const Tensor ap = Mp == Ma ? a : reshape16(a, a.size(0) * G, 1, Ma, 1, Mp, {a.size(0), G, Mp});
+        const Tensor bp = Cp == Cb ? b : reshape16(b, b.size(0) * G, 1, Cb, 1, Cp, {b.size(0), G, Cp});
+        return reshape16(vvor(ap, a_idx_, bp, b_idx_, seg_, o_idx_, n_o, engine), n_o * G, Mp, Cp, Ma, Cb, {n_o, G, Ma, Cb});
+    }
     const Tensor a_idx = as_i32(a_idx_), b_idx = as_i32(b_idx_), o_idx = o_idx_ ? as_i32(*o_idx_) : Tensor(),
                  seg = seg_ ? as_i64(*seg_) : Tensor();
     Tensor out = at::empty({n_o, G, Ma, Cb}, a.options());

@@ -336,11 +336,11 @@ constexpr int THREADS = (MMA_WARP0 + GROUP_BLOCKS) * 32;
 constexpr int MAX_SLOTS = 8;
 constexpr int AHEAD = 8;                              // steps the walk runs ahead (even: an entry always belongs to the same team)
 constexpr uint32_t ENTRY_BYTES = 2 * ROWS * 4;        // source rows of a step's two tiles
-// a step in one word: tap | slice << 9 | tiles that have the tap << 13 | first of its unit << 15 | end << 16
+// a step's word: slice << 9 | tiles that have the tap << 13 | first of its unit << 15 | end << 16
 constexpr uint32_t STEP_FIRST = 1u << 15, STEP_END = 1u << 16;
 
 struct OsParams {
-    const uint16_t *feat, *bias;            // bias: added before the rounding; null: none
+    const uint16_t *feat, *bias;            // rows of in_pitch elements; bias: added before the rounding; null: none
     const uint16_t *scratch;                // sums of the multi-triplet buckets
     uint16_t *out;
     float *partial;                         // nsplit > 1: [split][nblocks * ROWS][outw]
@@ -348,7 +348,8 @@ struct OsParams {
     const uint32_t *tap_masks;
     unsigned int *status;
     int K, C, M, transpose, reverse, fmt;   // reverse: tap k uses weight K-1-k
-    int inw, outw, nkb, ngroups, nblocks, nsplit, mask_words;
+    int inw, outw, nkb, ngroups, nblocks, nsplit, mask_words;   // inw, outw: of a part
+    int nparts, out_parts, in_pitch, out_pitch;   // parts of an output row: groups of the weight, each in out_parts
     int nslots, nacc;
     uint32_t slot_bytes, w_box_rows, w_tx_bytes, ncols, col_stride;
     uint64_t wait_limit_ns;
@@ -372,11 +373,11 @@ __device__ __forceinline__ int unit_at(int n, int units) {
     return pos < units ? pos : -1;
 }
 
-// The steps of a CTA: unit after unit, in a unit the 64-channel slices of the contraction, per slice the
+// The steps of a CTA: unit (group, split, part of the output row) after unit, in a unit the 64-channel slices of the contraction, per slice the
 // taps that touch one of the group's two blocks.
 struct Walk {
     const OsParams &p;
-    int n = -1, unit = 0, block0 = 0, q = 0, word = 0, tap = 0;
+    int n = -1, split = 0, part = 0, block0 = 0, q = 0, word = 0, tap = 0;
     int tap_lo = 0, tap_hi = 0;     // taps of this part of the group
     uint32_t m0 = 0, m1 = 0, left = 0;
     uint32_t has = 0;               // of the current step: bit b = block b of the group has the tap
@@ -395,11 +396,12 @@ struct Walk {
         left = m0 | m1;
     }
     __device__ __forceinline__ bool open(int at) {   // the unit at position `at`; false behind the end
-        unit = unit_at(at, p.ngroups * p.nsplit);
+        int unit = unit_at(at, p.ngroups * p.nsplit * p.nparts);
         if (unit < 0) return false;
-        const int s = unit % p.nsplit;
-        block0 = __ldg(p.group_order + unit / p.nsplit) * GROUP_BLOCKS;
-        tap_lo = p.K * s / p.nsplit, tap_hi = p.K * (s + 1) / p.nsplit;
+        part = unit % p.nparts, unit /= p.nparts;
+        split = unit % p.nsplit, unit /= p.nsplit;
+        block0 = __ldg(p.group_order + unit) * GROUP_BLOCKS;
+        tap_lo = p.K * split / p.nsplit, tap_hi = p.K * (split + 1) / p.nsplit;
         return true;
     }
     __device__ __forceinline__ bool next() {
@@ -437,7 +439,7 @@ struct Ring {
 __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ OsParams p) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t s_full[MAX_SLOTS], s_empty[MAX_SLOTS], s_acc_full[2], s_acc_empty[2], s_step_full[AHEAD], s_step_empty[AHEAD];
-    __shared__ uint32_t s_step[AHEAD];
+    __shared__ uint4 s_step[AHEAD];   // the step's word, its first feature column, the corner of its weight slice
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -476,6 +478,7 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
                 if (!wait(s_acc_full[acc.slot], acc.turn)) break;
                 tc_fence_after();
             }
+            const int col0 = w.part * p.outw;
             for (int b = 0; b < GROUP_BLOCKS && w.block0 + b < p.nblocks; ++b) {
                 const int64_t slot = (int64_t)(w.block0 + b) * ROWS + warp * 32 + lane;
                 const int32_t row = __ldg(p.perm + slot);
@@ -492,15 +495,15 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
                     if (row >= 0) {
                         if (p.nsplit > 1) {
                             float4 *dst = reinterpret_cast<float4 *>(
-                                p.partial + ((int64_t)(w.unit % p.nsplit) * p.nblocks * ROWS + slot) * p.outw + c0);
+                                p.partial + ((int64_t)w.split * p.nblocks * ROWS + slot) * p.out_pitch + col0 + c0);
 #pragma unroll
                             for (int e = 0; e < 4; ++e) dst[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
                         } else {
                             if (p.bias) {
 #pragma unroll
-                                for (int e = 0; e < 16; ++e) v[e] += bias_at(p.bias, c0 + e, p.fmt);
+                                for (int e = 0; e < 16; ++e) v[e] += bias_at(p.bias, col0 + c0 + e, p.fmt);
                             }
-                            uint4 *dst = reinterpret_cast<uint4 *>(p.out + (int64_t)row * p.outw + c0);
+                            uint4 *dst = reinterpret_cast<uint4 *>(p.out + (int64_t)row * p.out_pitch + col0 + c0);
 #pragma unroll
                             for (int e = 0; e < 2; ++e)
                                 dst[e] = make_uint4(pack2(v[8 * e], v[8 * e + 1], p.fmt), pack2(v[8 * e + 2], v[8 * e + 3], p.fmt),
@@ -531,14 +534,15 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
         for (int n = 0;; n ^= 1) {   // (two teams)
             if (n == team) {
                 if (!wait(s_step_full[step.slot], step.turn)) break;
-                const uint32_t word = *(volatile uint32_t *)&s_step[step.slot];
+                const uint32_t word = *(volatile uint32_t *)&s_step[step.slot].x;
                 if (word & STEP_END) break;
                 const uint32_t at = rows0 + step.slot * ENTRY_BYTES + (uint32_t)row0 * 4;
                 const uint4 rows[2] = {lds_v4(at), lds_v4(at + ROWS * 4)};
+                const uint32_t column = *(volatile uint32_t *)&s_step[step.slot].y + (uint32_t)piece * 8;
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&s_step_empty[step.slot]));
                 const int slice = (int)(word >> 9) & 15;
-                const uint16_t *col = p.feat + slice * 64 + piece * 8, *sums = p.scratch + slice * 64 + piece * 8;
+                const uint16_t *col = p.feat + column, *sums = p.scratch + column;
                 const bool piece_ok = piece * 8 < p.inw - slice * 64;
                 // the tensor core has finished with what was in the slot
                 if (!wait(s_empty[ring.slot], ring.turn ^ 1u)) break;
@@ -552,7 +556,7 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
                         for (int k = 0; k < 4; ++k) {
                             // a feature row, a row of bucket sums, or nothing (zeros: source size 0)
                             const uint32_t idx = (uint32_t)(rr[k] >= 0 ? rr[k] : rr[k] == -1 ? 0 : -2 - rr[k]);
-                            const uint16_t *src = (rr[k] < -1 ? sums : col) + (uint64_t)idx * (uint32_t)p.inw;
+                            const uint16_t *src = (rr[k] < -1 ? sums : col) + (uint64_t)idx * (uint32_t)p.in_pitch;
                             cp_async16_zfill(dst + (uint32_t)t * SLOT_BYTES + dst_off[k], src, rr[k] == -1 ? 0u : 16u);
                         }
                     }
@@ -582,7 +586,17 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
                 ++ends;
             }
             if (lane == 0) {
-                s_step[step.slot] = more ? (uint32_t)w.tap | ((uint32_t)w.q << 9) | (w.has << 13) | (w.first ? STEP_FIRST : 0u) : STEP_END;
+                uint4 s = make_uint4(STEP_END, 0u, 0u, 0u);
+                if (more) {
+                    // feature columns of the part's group; corner (x, y) of the weight slice in the (taps * groups * C, M) matrix
+                    const int g = w.part / p.out_parts, o = (w.part - g * p.out_parts) * p.outw;
+                    const int groups = p.nparts / p.out_parts, tap = p.reverse ? p.K - 1 - w.tap : w.tap;
+                    s.x = (uint32_t)w.q << 9 | (w.has << 13) | (w.first ? STEP_FIRST : 0u);
+                    s.y = (uint32_t)(g * p.inw + w.q * 64);
+                    s.z = (uint32_t)(p.transpose ? w.q * 64 : o);
+                    s.w = (uint32_t)((tap * groups + g) * p.C + (p.transpose ? o : w.q * 64));
+                }
+                s_step[step.slot] = s;
                 mbar_arrive(full);
             }
             cp_async_mbar_arrive(full);
@@ -594,20 +608,20 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
         Ring ring, step;
         for (;;) {
             if (!wait(s_step_full[step.slot], step.turn)) break;
-            const uint32_t word = *(volatile uint32_t *)&s_step[step.slot];
+            const uint32_t word = *(volatile uint32_t *)&s_step[step.slot].x;
             if (word & STEP_END) break;
+            const int x = *(volatile int *)&s_step[step.slot].z, y = *(volatile int *)&s_step[step.slot].w;
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&s_step_empty[step.slot]));
-            const int tap_r = (int)(word & 511u), q = (int)(word >> 9) & 15, tap = p.reverse ? p.K - 1 - tap_r : tap_r;
             if (!wait(s_empty[ring.slot], ring.turn ^ 1u)) break;
             const uint32_t dst = slot0 + ring.slot * p.slot_bytes + 2 * SLOT_BYTES, full = smem_u32(&s_full[ring.slot]);
             if (lane == 0) {
                 mbar_arrive_expect_tx(full, p.w_tx_bytes);
-                if (p.transpose) {   // contraction over m: the m-block q of all C rows of W[tap]
-                    tma_load_2d(dst, &tmap, q * 64, tap * p.C, full);
-                } else {             // contraction over c: rows [64q, 64q + box), one box per 64 output channels
-                    for (int mb = 0; mb * 64 < p.M; ++mb)
-                        tma_load_2d(dst + (uint32_t)mb * p.w_box_rows * 128, &tmap, mb * 64, tap * p.C + q * 64, full);
+                if (p.transpose) {   // contraction over m: an m-block of the output channels' rows
+                    tma_load_2d(dst, &tmap, x, y, full);
+                } else {             // contraction over c: 64 rows, one box per 64 output channels
+                    for (int mb = 0; mb * 64 < p.outw; ++mb)
+                        tma_load_2d(dst + (uint32_t)mb * p.w_box_rows * 128, &tmap, x + mb * 64, y, full);
                 }
             }
             ring.next(p.nslots);
@@ -631,7 +645,7 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
         for (;;) {
             ok = wait(s_step_full[step.slot], step.turn);
             if (!ok) break;
-            const uint32_t word = *(volatile uint32_t *)&s_step[step.slot];
+            const uint32_t word = *(volatile uint32_t *)&s_step[step.slot].x;
             if (word & STEP_END) break;
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&s_step_empty[step.slot]));
@@ -759,19 +773,23 @@ uint64_t wait_limit() {
 // Parts the taps of a group are split into when the groups alone do not fill the chip: the count with the
 // smallest time, a part costing a tenth of a whole group more than its share (its fp32 sums go through
 // memory).  1000 points of 256 channels, 4 groups: 183 us on 4 CTAs, 28 us in 27 parts per group.
-int split_parts(int64_t ngroups, int K) {
+int split_parts(int64_t ngroups, int K, int nparts) {
     const int sms = num_sms();
     int best = 1;
     double best_cost = 1e30;
-    for (int s = 1; s <= std::min(K, 64) && ngroups < 2 * sms; ++s) {
-        const double waves = (double)((ngroups * s + sms - 1) / sms), cost = waves * (1.0 / s + (s > 1 ? 0.1 : 0.0));
+    for (int s = 1; s <= std::min(K, 64) && ngroups * nparts < 2 * sms; ++s) {
+        const double waves = (double)((ngroups * nparts * s + sms - 1) / sms), cost = waves * (1.0 / s + (s > 1 ? 0.1 : 0.0));
         if (cost < best_cost * 0.999) best_cost = cost, best = s;
     }
     return best;
 }
 
-size_t partial_bytes(int64_t n_out, int outw, int parts) {
-    return parts > 1 ? (size_t)parts * ((n_out + ROWS - 1) / ROWS) * ROWS * outw * sizeof(float) : 0;
+// Output rows wider than the tensor memory's two accumulators (256 channels), and those of a grouped
+// weight, are worked off in parts of the same width.
+int parts_of(int width) { return (width + 255) / 256; }
+
+size_t partial_bytes(int64_t n_out, int outw, int splits) {
+    return splits > 1 ? (size_t)splits * ((n_out + ROWS - 1) / ROWS) * ROWS * outw * sizeof(float) : 0;
 }
 
 bool plan_sizes_ok(int64_t T, int64_t n_out, int K, int G) {
@@ -789,7 +807,7 @@ using namespace pcx;
 extern "C" {
 
 int pcx_mvmr_plan_group_blocks(int out_width) {
-    if (out_width <= 0 || out_width > 256) return 0;
+    if (out_width <= 0 || out_width > 256) return 0;   // wider rows are worked off in parts of at most 256
     // Two: both accumulators of the widest rows (256 channels) fill the tensor memory, and every weight
     // slice that is streamed serves 256 output rows.
     return GROUP_BLOCKS;
@@ -878,10 +896,11 @@ size_t pcx_mvmr_planned_workspace_bytes(int64_t multi_buckets, int in_width) {
     return align_up((size_t)std::max<int64_t>(multi_buckets, 1) * in_width * 2, 256);
 }
 
-size_t pcx_mvmr_planned_scratch_bytes(int64_t multi_buckets, int in_width, int64_t n_out, int out_width, int K) {
-    if (multi_buckets < 0 || in_width <= 0 || n_out <= 0 || out_width <= 0 || K <= 0) return 0;
+size_t pcx_mvmr_planned_scratch_bytes(int64_t multi_buckets, int in_width, int64_t n_out, int out_width, int K, int G) {
+    if (multi_buckets < 0 || in_width <= 0 || n_out <= 0 || out_width <= 0 || K <= 0 || G <= 0) return 0;
     const int64_t ngroups = (n_out + GROUP_BLOCKS * ROWS - 1) / (GROUP_BLOCKS * ROWS);
-    return pcx_mvmr_planned_workspace_bytes(multi_buckets, in_width) + partial_bytes(n_out, out_width, split_parts(ngroups, K));
+    return pcx_mvmr_planned_workspace_bytes(multi_buckets, G * in_width) +
+           partial_bytes(n_out, G * out_width, split_parts(ngroups, K, G * parts_of(out_width)));
 }
 
 int pcx_mvmr_plan_multi_buckets(const void *d_plan, int64_t *h_count, void *stream_) {
@@ -897,31 +916,32 @@ int pcx_mvmr_plan_multi_buckets(const void *d_plan, int64_t *h_count, void *stre
 int pcx_mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan, size_t plan_bytes, void *d_out, int64_t T,
                      int64_t n_feat, int64_t n_out, int K, int C, int M, int transpose, int dtype, int group_blocks,
                      int64_t multi_buckets, void *d_ws, size_t ws_bytes, void *stream) {
-    return pcx_mvmr_planned_bias(d_weight, d_feat, d_plan, plan_bytes, nullptr, d_out, T, n_feat, n_out, K, C, M,
+    return pcx_mvmr_planned_bias(d_weight, d_feat, d_plan, plan_bytes, nullptr, d_out, T, n_feat, n_out, K, 1, C, M,
                                  transpose ? PCX_MVMR_TRANSPOSE : 0, dtype, group_blocks, multi_buckets, d_ws, ws_bytes, stream);
 }
 
 int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan, size_t plan_bytes, const void *d_bias, void *d_out,
-                          int64_t T, int64_t n_feat, int64_t n_out, int K, int C, int M, int flags, int dtype, int group_blocks,
-                          int64_t multi_buckets, void *d_ws, size_t ws_bytes, void *stream_) {
+                          int64_t T, int64_t n_feat, int64_t n_out, int K, int groups, int C, int M, int flags, int dtype,
+                          int group_blocks, int64_t multi_buckets, void *d_ws, size_t ws_bytes, void *stream_) {
     const int transpose = flags & PCX_MVMR_TRANSPOSE;
     cudaStream_t stream = (cudaStream_t)stream_;
     const int G = group_blocks;
     if (dtype != PCX_F16 && dtype != PCX_BF16) PCX_FAIL(PCX_E_DTYPE, "pcx_mvmr_planned: fp16 or bf16 only (dtype %d)", dtype);
-    if (C <= 0 || M <= 0 || n_feat < 0) PCX_FAIL(PCX_E_ARG, "pcx_mvmr_planned: bad sizes");
+    if (C <= 0 || M <= 0 || n_feat < 0 || groups <= 0) PCX_FAIL(PCX_E_ARG, "pcx_mvmr_planned: bad sizes");
     if (!plan_sizes_ok(T, n_out, K, G))
         PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_planned: sizes out of range (T=%lld n_out=%lld K=%d group=%d)", (long long)T,
                  (long long)n_out, K, G);
     const int inw = transpose ? M : C, outw = transpose ? C : M;
-    if (inw % 16 || outw % 16 || inw > 1024 || outw > 256)
-        PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_planned: channel counts must be multiples of 16, output width at most 256 (C=%d M=%d)", C, M);
+    const int out_parts = parts_of(outw), nparts = groups * out_parts;
+    if (inw % 16 || outw % (16 * out_parts) || inw > 1024 || groups * inw > 2048 || nparts > 64)
+        PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_planned: channel counts must be multiples of 16 and the parts of an output row equal (groups=%d C=%d M=%d)", groups, C, M);
     if (!d_weight || !d_plan || !d_out || (T > 0 && !d_feat)) PCX_FAIL(PCX_E_ARG, "pcx_mvmr_planned: null pointer");
     if ((uintptr_t)d_weight % 16 || (uintptr_t)d_feat % 16 || (uintptr_t)d_out % 16 || (uintptr_t)d_plan % 256 || (uintptr_t)d_ws % 256)
         PCX_FAIL(PCX_E_ALIGN, "pcx_mvmr_planned: weight, features and output must be 16-byte aligned, plan and workspace 256-byte aligned");
     if (multi_buckets < 0 || multi_buckets > T / 2) PCX_FAIL(PCX_E_ARG, "pcx_mvmr_planned: multi_buckets out of range");
-    if (multi_buckets > 0 && (!d_ws || ws_bytes < pcx_mvmr_planned_workspace_bytes(multi_buckets, transpose ? M : C)))
+    if (multi_buckets > 0 && (!d_ws || ws_bytes < pcx_mvmr_planned_workspace_bytes(multi_buckets, groups * inw)))
         PCX_FAIL(PCX_E_CAPACITY, "pcx_mvmr_planned: workspace %zu < %zu bytes", ws_bytes,
-                 pcx_mvmr_planned_workspace_bytes(multi_buckets, transpose ? M : C));
+                 pcx_mvmr_planned_workspace_bytes(multi_buckets, groups * inw));
     PlanView pv;
     const size_t need_plan = carve_plan(d_plan, T, n_out, K, G, &pv);
     if (plan_bytes < need_plan) PCX_FAIL(PCX_E_CAPACITY, "pcx_mvmr_planned: plan buffer %zu < %zu bytes", plan_bytes, need_plan);
@@ -934,14 +954,15 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     if (!p.status) PCX_FAIL(PCX_E_LAUNCH, "pcx_mvmr_planned: no device status word");
     p.K = K, p.C = C, p.M = M, p.transpose = transpose ? 1 : 0, p.fmt = dtype == PCX_BF16 ? 1 : 0;
     p.reverse = (flags & PCX_MVMR_REVERSE_TAPS) ? 1 : 0;
-    p.inw = inw, p.outw = outw, p.nkb = (inw + 63) / 64, p.mask_words = (K + 31) / 32;
+    p.nparts = nparts, p.out_parts = out_parts, p.in_pitch = groups * inw, p.out_pitch = groups * outw;
+    p.inw = inw, p.outw = outw / out_parts, p.nkb = (inw + 63) / 64, p.mask_words = (K + 31) / 32;
     p.ngroups = (int)pv.ngroups, p.nblocks = (int)pv.nblocks;
-    p.col_stride = (uint32_t)((outw + 31) / 32 * 32);
+    p.col_stride = (uint32_t)((p.outw + 31) / 32 * 32);
     p.nacc = 4 * p.col_stride <= 512 ? 2 : 1;   // up to 128 channels the next group starts while the last one is written
     p.ncols = 32;
     while (p.ncols < 2u * (uint32_t)p.nacc * p.col_stride) p.ncols <<= 1;
-    p.w_box_rows = (uint32_t)(transpose ? C : std::min(64, C));
-    p.w_tx_bytes = transpose ? (uint32_t)C * 128u : (uint32_t)((M + 63) / 64) * p.w_box_rows * 128u;
+    p.w_box_rows = (uint32_t)(transpose ? p.outw : std::min(64, C));
+    p.w_tx_bytes = (transpose ? 1u : (uint32_t)((p.outw + 63) / 64)) * p.w_box_rows * 128u;
     p.slot_bytes = 2 * SLOT_BYTES + (uint32_t)align_up(p.w_tx_bytes, 1024);
     p.wait_limit_ns = wait_limit();
     if (!encode_tiled()) PCX_FAIL(PCX_E_LAUNCH, "pcx_mvmr_planned: the driver offers no cuTensorMapEncodeTiled");
@@ -949,7 +970,7 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     // widths that are not multiples of 64: the last box of a row ends in zero fill
     CUtensorMap tmap;
     memset(&tmap, 0, sizeof(tmap));
-    const cuuint64_t gdim[2] = {(cuuint64_t)M, (cuuint64_t)K * (cuuint64_t)C};
+    const cuuint64_t gdim[2] = {(cuuint64_t)M, (cuuint64_t)K * (cuuint64_t)groups * (cuuint64_t)C};
     const cuuint64_t gstride[1] = {(cuuint64_t)M * 2};
     const cuuint32_t box[2] = {64u, p.w_box_rows};
     const cuuint32_t estride[2] = {1u, 1u};
@@ -963,9 +984,9 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     p.nslots = (int)std::min<size_t>(MAX_SLOTS, ((size_t)232448 - 1024 - 1024 - AHEAD * ENTRY_BYTES) / p.slot_bytes);
     if (p.nslots < 2) PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_planned: shared memory does not fit (C=%d M=%d)", C, M);
     // the fp32 sums of a split rulebook lie behind the bucket sums; a caller that made no room for them gets one part
-    const size_t sums_bytes = pcx_mvmr_planned_workspace_bytes(multi_buckets, inw);
-    p.nsplit = split_parts(pv.ngroups, K);
-    if (p.nsplit > 1 && (!d_ws || ws_bytes < sums_bytes + partial_bytes(n_out, outw, p.nsplit))) p.nsplit = 1;
+    const size_t sums_bytes = pcx_mvmr_planned_workspace_bytes(multi_buckets, p.in_pitch);
+    p.nsplit = split_parts(pv.ngroups, K, nparts);
+    if (p.nsplit > 1 && (!d_ws || ws_bytes < sums_bytes + partial_bytes(n_out, p.out_pitch, p.nsplit))) p.nsplit = 1;
     p.partial = p.nsplit > 1 ? (float *)((char *)d_ws + sums_bytes) : nullptr;
     const size_t smem = 1024 + (size_t)p.nslots * p.slot_bytes + AHEAD * ENTRY_BYTES;
     static int granted[64] = {};
@@ -975,11 +996,11 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
         PCX_CUDA(cudaFuncSetAttribute(mvmr_os_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         granted[dev & 63] = (int)smem;
     }
-    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(pv.ngroups * p.nsplit, num_sms()));
+    const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(pv.ngroups * p.nsplit * nparts, num_sms()));
     if (multi_buckets > 0) {
         prof_begin("bucket_sum_kernel", stream);
-        if (p.fmt) launch_bucket_sum<1>(multi_buckets, inw, p.feat, pv.entries, pv.buckets, pv.ctrl, (uint16_t *)d_ws, stream);
-        else launch_bucket_sum<0>(multi_buckets, inw, p.feat, pv.entries, pv.buckets, pv.ctrl, (uint16_t *)d_ws, stream);
+        if (p.fmt) launch_bucket_sum<1>(multi_buckets, p.in_pitch, p.feat, pv.entries, pv.buckets, pv.ctrl, (uint16_t *)d_ws, stream);
+        else launch_bucket_sum<0>(multi_buckets, p.in_pitch, p.feat, pv.entries, pv.buckets, pv.ctrl, (uint16_t *)d_ws, stream);
         prof_end(stream);
         PCX_LAUNCH_CHECK();
     }
@@ -989,7 +1010,7 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     PCX_LAUNCH_CHECK();
     if (p.nsplit > 1) {
         const int64_t slots = pv.nblocks * ROWS;
-        os_reduce_kernel<<<(unsigned)((slots * (outw / 8) + 255) / 256), 256, 0, stream>>>(p.partial, p.perm, p.bias, slots, outw, p.nsplit,
+        os_reduce_kernel<<<(unsigned)((slots * (p.out_pitch / 8) + 255) / 256), 256, 0, stream>>>(p.partial, p.perm, p.bias, slots, p.out_pitch, p.nsplit,
                                                                                            p.fmt, p.out);
         PCX_LAUNCH_CHECK();
     }

@@ -120,7 +120,7 @@ int pcx_mvmr_bias(const void *d_weight, const void *d_feat, const int32_t *d_gat
     if (T > 0) {
         bool tensor_ok = mvmr_tensor_supported(a);
         if (engine == PCX_ENGINE_TENSOR && !tensor_ok)
-            PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr: tensor engine needs fp16/bf16, G=1, tap-sorted triplets and channel counts that are multiples of 16 in [16,256]");
+            PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr: tensor engine needs fp16/bf16, tap-sorted triplets and channel counts that are multiples of 16 (of 32 beyond 256, of 48 beyond 512 ...)");
         int rc = (engine != PCX_ENGINE_CUDA_CORE && tensor_ok) ? mvmr_tensor(a, stream) : mvmr_generic(a, stream);
         if (rc != PCX_OK) return rc;
     }
@@ -168,7 +168,7 @@ int pcx_vvor(const void *d_a, const int32_t *d_a_idx, const void *d_b, const int
         if (force_engine()) engine = force_engine();
         bool tensor_ok = vvor_tensor_supported(a);
         if (engine == PCX_ENGINE_TENSOR && !tensor_ok)
-            PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_vvor: tensor engine needs fp16/bf16, G=1, sorted output index and channel counts that are multiples of 16 in [16,256]");
+            PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_vvor: tensor engine needs fp16/bf16, a sorted output index and channel counts that are multiples of 16 (of 32 beyond 256, of 48 beyond 512 ...)");
         int rc = (engine != PCX_ENGINE_CUDA_CORE && tensor_ok) ? vvor_tensor(a, stream) : vvor_generic(a, stream);
         if (rc != PCX_OK) return rc;
     }

@@ -82,6 +82,7 @@ struct ChunkCursorT {
 };
 using ChunkCursor = ChunkCursorT<CH>;
 
+constexpr int MAX_PARTS = 64;        // (group, part, part) combinations of one launch
 constexpr int MAX_TAPS_SMEM = 1024;  // taps whose chunk table fits the shared-memory copy
 
 // cum[k] = chunks of CHR triplets in the taps before k; all threads of the CTA call this.
@@ -115,12 +116,12 @@ __device__ __forceinline__ void build_chunk_table(const int64_t *__restrict__ se
 }
 
 // Gather `rows` rows of `width` 2-byte channels into a swizzled tile; the row
-// indices were staged in shared memory beforehand so that the copy loop issues
+// (`pitch` elements apart) were staged in shared memory beforehand so that the copy loop issues
 // cp.async back to back.  Rows past `rows` are zero-filled when ZERO_TAIL
 // (needed when the row index is the contraction index), untouched otherwise.
 template <bool ZERO_TAIL, int CHR = CH>
 __device__ __forceinline__ void gather_tile(uint32_t tile, const uint16_t *__restrict__ src,
-                                            const int32_t *s_idx, int rows, int width, int tid, int nthreads) {
+                                            const int32_t *s_idx, int rows, int width, int64_t pitch, int tid, int nthreads) {
     const int cpr = width >> 3;  // 16-byte pieces per row
     constexpr uint32_t BLK = CHR * 128;   // one 64-channel block of the tile
     const int rmax = ZERO_TAIL ? CHR : rows;
@@ -134,7 +135,7 @@ __device__ __forceinline__ void gather_tile(uint32_t tile, const uint16_t *__res
         for (int r = tid >> sh; r < rmax; r += rpp) {
             const uint32_t dst = dcol + (uint32_t)r * 128 + (uint32_t)(((ch ^ r) & 7) << 4);
             if (r < rows) {
-                cp_async16(dst, scol + (int64_t)s_idx[r] * width);
+                cp_async16(dst, scol + s_idx[r] * pitch);
             } else if (ZERO_TAIL) {
                 asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};" ::"r"(dst), "r"(0) : "memory");
             }
@@ -147,7 +148,7 @@ __device__ __forceinline__ void gather_tile(uint32_t tile, const uint16_t *__res
         int r = e / cpr, ch = e - r * cpr;
         uint32_t dst = tile + (uint32_t)(ch >> 3) * BLK + (uint32_t)r * 128 + (uint32_t)(((ch & 7) ^ (r & 7)) << 4);
         if (r < rows) {
-            cp_async16(dst, src + (int64_t)s_idx[r] * width + ch * 8);
+            cp_async16(dst, src + s_idx[r] * pitch + ch * 8);
         } else if (ZERO_TAIL) {
             asm volatile("st.shared.v4.b32 [%0], {%1,%1,%1,%1};" ::"r"(dst), "r"(0) : "memory");
         }
@@ -179,6 +180,12 @@ __device__ __forceinline__ float unpack_one(uint16_t v, int fmt) {
     return fmt ? __bfloat162float(__ushort_as_bfloat16(v)) : __half2float(__ushort_as_half(v));
 }
 
+// Wide and grouped layers run as parts of at most 256 x 256 channels: blockIdx.y counts (group, part of the
+// output row, part of the contraction), the parts of a contraction meet in the accumulator's reductions.
+// Every part of a width has the same size, a multiple of 16.
+int parts_of(int width) { return (width + 255) / 256; }
+bool splits_evenly(int width) { return width >= 16 && width % (16 * parts_of(width)) == 0; }
+
 struct MvmrTcParams {
     const uint16_t *weight;  // (K, C, M) as stored
     const uint16_t *feat;
@@ -188,6 +195,8 @@ struct MvmrTcParams {
     uint16_t *out;           // MODE 2: the output rows themselves (every row occurs in exactly one triplet)
     const uint16_t *bias;    // MODE 2: added before the rounding (null: none); the other modes start from it
     int reverse;             // tap k uses weight K-1-k
+    int64_t in_pitch, out_pitch, w_pitch, w_tap;   // rows of features / output / one tap's weight, elements of one tap's weight
+    int out_parts, in_parts;                       // C, M below: the part's
     int K, C, M, transpose, fmt, nbuf, slab;  // slab: columns parked per bulk reduction (32 or 64)
     int prow_log2;                            // a warp parks 2^prow_log2 rows at a time (8, 16 or 32)
     uint32_t park_bytes;                      // size of the parking area (the chunk table follows it)
@@ -213,6 +222,16 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
     __shared__ int32_t s_warp_sums[4];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int inw = p.transpose ? p.M : p.C, outw = p.transpose ? p.C : p.M;
+    {
+        const int ip = (int)blockIdx.y % p.in_parts, op = (int)blockIdx.y / p.in_parts % p.out_parts,
+                  g = (int)blockIdx.y / (p.in_parts * p.out_parts);
+        const int64_t out0 = ((int64_t)g * p.out_parts + op) * outw;
+        p.feat += ((int64_t)g * p.in_parts + ip) * inw;
+        p.acc += out0;
+        if (MODE == 2) p.out += out0, p.bias = p.bias ? p.bias + out0 : p.bias;
+        const int64_t rows = (int64_t)(p.transpose ? p.out_parts : p.in_parts) * p.C;
+        p.weight += ((int64_t)g * rows + (p.transpose ? op : ip) * p.C) * p.w_pitch + (p.transpose ? ip : op) * p.M;
+    }
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const int kb = (inw + 63) >> 6;
     const uint32_t a_bytes = (uint32_t)kb * BLK_BYTES;
@@ -256,12 +275,12 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
     bool alive = true;
 
     auto load_weight = [&](int tap) {
-        const uint16_t *w = p.weight + (int64_t)(p.reverse ? p.K - 1 - tap : tap) * p.C * p.M;
+        const uint16_t *w = p.weight + (p.reverse ? p.K - 1 - tap : tap) * p.w_tap;
         const int cpr = p.M >> 3;
         for (int e = tid; e < p.C * cpr; e += 128) {
             int c = e / cpr, ch = e - c * cpr;
             uint32_t dst = b_tile + (uint32_t)(ch >> 3) * w_blk + (uint32_t)c * 128 + (uint32_t)(((ch & 7) ^ (c & 7)) << 4);
-            cp_async16(dst, w + (int64_t)c * p.M + ch * 8);
+            cp_async16(dst, w + c * p.w_pitch + ch * 8);
         }
     };
 
@@ -279,7 +298,7 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
         load_weight(c0.tap);
         loaded_tap = c0.tap;
         __syncthreads();
-        gather_tile<false>(a_tile0, p.feat, s_gather[0], rows, inw, tid, 128);
+        gather_tile<false>(a_tile0, p.feat, s_gather[0], rows, inw, p.in_pitch, tid, 128);
         cp_async_commit();
         if (lo + 1 < hi) {
             c1.advance(s_cum, p.seg, p.K, lo + 1);
@@ -302,7 +321,7 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
         }
         __syncthreads();
         if (have_next && two)
-            gather_tile<false>(a_tile0 + (uint32_t)(b ^ 1) * a_bytes, p.feat, s_gather[b ^ 1], rows_next, inw, tid, 128);
+            gather_tile<false>(a_tile0 + (uint32_t)(b ^ 1) * a_bytes, p.feat, s_gather[b ^ 1], rows_next, inw, p.in_pitch, tid, 128);
         cp_async_commit();
         if (chunk + 2 < hi) {
             c2.advance(s_cum, p.seg, p.K, chunk + 2);
@@ -338,13 +357,13 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
             cp_async_commit();
         }
         if (have_next && !two && !p.alias) {  // single A tile: it is free as well
-            gather_tile<false>(a_tile0, p.feat, s_gather[b ^ 1], rows_next, inw, tid, 128);
+            gather_tile<false>(a_tile0, p.feat, s_gather[b ^ 1], rows_next, inw, p.in_pitch, tid, 128);
             cp_async_commit();
         }
         if (BULK && alive && warp * 32 < rows) {
             const int row = warp * 32 + lane;
             const bool row_ok = row < rows;
-            float *dst_row = p.acc + (int64_t)(row_ok ? s_scatter[b][row] : 0) * outw;
+            float *dst_row = p.acc + (row_ok ? s_scatter[b][row] : 0) * p.out_pitch;
             // a warp parks `prow` rows at a time (32, or 16 when shared memory is better spent
             // on one more resident CTA): lanes of the current batch store, the others only
             // take part in the warp-wide TMEM load
@@ -375,7 +394,7 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
             // one thread per accumulator row: 32 columns at a time, rounded and stored
             const int row = warp * 32 + lane;
             const bool row_ok = row < rows;
-            uint16_t *dst_row = p.out + (int64_t)(row_ok ? s_scatter[b][row] : 0) * outw;
+            uint16_t *dst_row = p.out + (row_ok ? s_scatter[b][row] : 0) * p.out_pitch;
             for (int col0 = 0; col0 < outw; col0 += 32) {
                 float v[32];
                 tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)col0, v);
@@ -407,7 +426,7 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
                 for (int col0 = 0; col0 < outw; col0 += 64) {
                     float v[32];
                     tmem_ld_16x64(tmem + ((uint32_t)(warp * 32 + half * 16) << 16) + (uint32_t)col0, v);
-                    scatter_block(p.acc, da, db, outw, col0, lane, v);
+                    scatter_block(p.acc, da, db, outw, p.out_pitch, col0, lane, v);
                 }
             }
         }
@@ -417,7 +436,7 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
             bulk_wait_read();
             __syncthreads();
             if (have_next) {
-                gather_tile<false>(a_tile0, p.feat, s_gather[b ^ 1], rows_next, inw, tid, 128);
+                gather_tile<false>(a_tile0, p.feat, s_gather[b ^ 1], rows_next, inw, p.in_pitch, tid, 128);
                 cp_async_commit();
             }
         }
@@ -436,8 +455,10 @@ struct VvorTcParams {
     const uint16_t *a, *b;  // (n_a, Ma), (n_b, Cb)
     const int32_t *a_idx, *b_idx;
     const int64_t *seg;
-    float *acc;             // (n_o, Ma, Cb)
-    int n_o, Ma, Cb, fmt, stages;
+    float *acc;             // (n_o, G, rows of Cb)
+    int64_t a_pitch, b_pitch, acc_pitch, acc_tap;   // rows of a / b / one tap's sums, elements of one tap's sums
+    int a_parts, b_parts;                           // blockIdx.y: (group, part of a, part of b)
+    int n_o, Ma, Cb, fmt, stages;   // Ma, Cb: the part's
     uint32_t ncols;
 };
 
@@ -461,6 +482,13 @@ __global__ void __launch_bounds__(NT) vvor_tc_kernel(VvorTcParams p) {
     __shared__ int32_t s_warp_sums[NT / 32];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    {
+        const int bp = (int)blockIdx.y % p.b_parts, ap = (int)blockIdx.y / p.b_parts % p.a_parts,
+                  g = (int)blockIdx.y / (p.b_parts * p.a_parts);
+        p.a += ((int64_t)g * p.a_parts + ap) * p.Ma;
+        p.b += ((int64_t)g * p.b_parts + bp) * p.Cb;
+        p.acc += ((int64_t)g * p.a_parts + ap) * p.Ma * p.acc_pitch + bp * p.Cb;
+    }
     const int row_tiles = (p.Ma + 127) >> 7;
     const int ablk = (p.Ma + 63) >> 6;  // blocks actually filled; an odd count borrows the next block as padding
     const int bblk = (p.Cb + 63) >> 6;
@@ -506,8 +534,8 @@ __global__ void __launch_bounds__(NT) vvor_tc_kernel(VvorTcParams p) {
     auto copy_rows = [&](int slot, int rows) {
         __syncthreads();
         const uint32_t a_tile = base + (uint32_t)slot * buf_bytes;
-        gather_tile<true, CHR>(a_tile, p.a, s_ia[slot], rows, p.Ma, tid, NT);
-        gather_tile<true, CHR>(a_tile + (uint32_t)ablk * BLK, p.b, s_ib[slot], rows, p.Cb, tid, NT);
+        gather_tile<true, CHR>(a_tile, p.a, s_ia[slot], rows, p.Ma, p.a_pitch, tid, NT);
+        gather_tile<true, CHR>(a_tile + (uint32_t)ablk * BLK, p.b, s_ib[slot], rows, p.Cb, p.b_pitch, tid, NT);
     };
     auto issue_gather = [&](const Cursor &cc, int chunk, int slot, bool from_regs) {
         copy_rows(slot, stage_indices(cc, chunk, slot, from_regs));
@@ -546,7 +574,7 @@ __global__ void __launch_bounds__(NT) vvor_tc_kernel(VvorTcParams p) {
     // a warp reads the 32 TMEM lanes of its quarter (warp % 4); the warps of a quarter share its columns
     const int quarter = warp & 3, col_part = warp >> 2;
     auto flush_tap = [&](int o) {
-        float *dst_o = p.acc + (int64_t)o * p.Ma * p.Cb;
+        float *dst_o = p.acc + o * p.acc_tap;
         for (int rt = 0; rt < row_tiles; ++rt) {
 #pragma unroll 1
             for (int half = 0; half < 2; ++half) {
@@ -557,7 +585,7 @@ __global__ void __launch_bounds__(NT) vvor_tc_kernel(VvorTcParams p) {
                 for (int c0 = col_part * 64; c0 < p.Cb; c0 += (NT / 128) * 64) {
                     float v[32];
                     tmem_ld_16x64(tmem + ((uint32_t)(quarter * 32 + half * 16) << 16) + (uint32_t)(rt * p.Cb + c0), v);
-                    scatter_block(dst_o, da, db, p.Cb, c0, lane, v);
+                    scatter_block(dst_o, da, db, p.Cb, p.acc_pitch, c0, lane, v);
                 }
             }
         }
@@ -636,8 +664,8 @@ __global__ void __launch_bounds__(NT) vvor_tc_kernel(VvorTcParams p) {
             const int rows = fill.rows(chunk);
             if (ctid >= 0) {
                 const uint32_t a_tile = base + (uint32_t)slot * buf_bytes;
-                gather_tile<true, CHR>(a_tile, p.a, s_ia[islot], rows, p.Ma, ctid, NCOPY);
-                gather_tile<true, CHR>(a_tile + (uint32_t)ablk * BLK, p.b, s_ib[islot], rows, p.Cb, ctid, NCOPY);
+                gather_tile<true, CHR>(a_tile, p.a, s_ia[islot], rows, p.Ma, p.a_pitch, ctid, NCOPY);
+                gather_tile<true, CHR>(a_tile + (uint32_t)ablk * BLK, p.b, s_ib[islot], rows, p.Cb, p.b_pitch, ctid, NCOPY);
             }
         };
         auto next = [](int v, int mod) { return v + 1 == mod ? 0 : v + 1; };
@@ -763,9 +791,9 @@ bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
 
 bool mvmr_tensor_supported(const MvmrArgs &a) {
     if (a.dtype != PCX_F16 && a.dtype != PCX_BF16) return false;
-    if (a.G != 1 || !a.seg_offs || a.T <= 0 || a.K > MAX_TAPS_SMEM) return false;
-    const int inw = a.transpose ? a.M : a.C, outw = a.transpose ? a.C : a.M;
-    if (inw % 16 || outw % 16 || inw < 16 || outw < 16 || inw > 256 || outw > 256) return false;
+    if (!a.seg_offs || a.T <= 0 || a.K > MAX_TAPS_SMEM) return false;
+    if (!splits_evenly(a.C) || !splits_evenly(a.M) || (int64_t)a.G * parts_of(a.C) * parts_of(a.M) > MAX_PARTS) return false;
+    if (a.out_rows && parts_of(a.transpose ? a.M : a.C) > 1) return false;   // rows can be stored only where one pass completes them
     if (!aligned16(a.weight) || !aligned16(a.feat)) return false;
     if (a.T / CH + a.K >= INT32_MAX) return false;
     return true;
@@ -773,20 +801,24 @@ bool mvmr_tensor_supported(const MvmrArgs &a) {
 
 bool vvor_tensor_supported(const VvorArgs &a) {
     if (a.dtype != PCX_F16 && a.dtype != PCX_BF16) return false;
-    if (a.G != 1 || !a.seg_offs || a.T <= 0 || a.n_o > MAX_TAPS_SMEM) return false;
-    if (a.Ma % 16 || a.Cb % 16 || a.Ma < 16 || a.Cb < 16 || a.Ma > 256 || a.Cb > 256) return false;
-    if (((a.Ma + 127) / 128 - 1) * a.Cb + (a.Cb + 63) / 64 * 64 > 512) return false;
+    if (!a.seg_offs || a.T <= 0 || a.n_o > MAX_TAPS_SMEM) return false;
+    if (!splits_evenly(a.Ma) || !splits_evenly(a.Cb) || (int64_t)a.G * parts_of(a.Ma) * parts_of(a.Cb) > MAX_PARTS) return false;
     if (!aligned16(a.a) || !aligned16(a.b)) return false;
     return true;
 }
 
 int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
-    const int inw = a.transpose ? a.M : a.C, outw = a.transpose ? a.C : a.M;
+    const int c_parts = parts_of(a.C), m_parts = parts_of(a.M), C = a.C / c_parts, M = a.M / m_parts;   // the part's
+    const int inw = a.transpose ? M : C, outw = a.transpose ? C : M;
     MvmrTcParams p;
+    p.in_parts = a.transpose ? m_parts : c_parts, p.out_parts = a.transpose ? c_parts : m_parts;
+    p.in_pitch = (int64_t)a.G * p.in_parts * inw, p.out_pitch = (int64_t)a.G * p.out_parts * outw;
+    p.w_pitch = a.M, p.w_tap = (int64_t)a.G * a.C * a.M;
+    const int parts = a.G * c_parts * m_parts;
     p.weight = (const uint16_t *)a.weight, p.feat = (const uint16_t *)a.feat;
     p.gather = a.gather, p.scatter = a.scatter, p.seg = a.seg_offs, p.acc = a.acc;
     p.out = (uint16_t *)a.out_rows, p.bias = (const uint16_t *)a.bias, p.reverse = a.reverse;
-    p.K = a.K, p.C = a.C, p.M = a.M, p.transpose = a.transpose, p.fmt = a.dtype == PCX_BF16 ? 1 : 0;
+    p.K = a.K, p.C = C, p.M = M, p.transpose = a.transpose, p.fmt = a.dtype == PCX_BF16 ? 1 : 0;
     p.ncols = pow2_cols((outw + 63) / 64 * 64);  // the epilogue reads blocks of up to 64 columns
     // Measured on B200: rows of exactly 64 floats leave fastest through one bulk reduction
     // each (64 vs 84 us on the 150k-point scene); narrower and wider rows from registers
@@ -796,7 +828,7 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
     if (const char *e = getenv("PCX_MVMR_SCATTER")) bulk = atoi(e) != 0;
     const bool store = a.out_rows != nullptr;
     if (store) bulk = false;
-    const int kb = (inw + 63) / 64, wb = (a.M + 63) / 64;
+    const int kb = (inw + 63) / 64, wb = (M + 63) / 64;
     const size_t static_smem = 2176;  // index rings, barrier
     const size_t table = align_up((size_t)(a.K + 1) * 4, 16);
     p.slab = outw >= 64 ? 64 : 32;  // columns parked per bulk reduction
@@ -810,7 +842,7 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
     // reductions to drain, but one more CTA fits per SM (measured: 62 vs 65 us).
     p.alias = bulk ? 1 : 0;
     if (const char *e = getenv("PCX_MVMR_ALIAS")) p.alias = bulk && atoi(e) != 0;
-    const size_t rest = 1024 + (size_t)wb * a.C * 128 + (p.alias ? 0 : p.park_bytes) + table;
+    const size_t rest = 1024 + (size_t)wb * C * 128 + (p.alias ? 0 : p.park_bytes) + table;
     // One A tile: it is free again as soon as the multiply has finished, so the
     // next gather still overlaps the scatter, and more CTAs fit on an SM.
     p.nbuf = 1;
@@ -833,12 +865,12 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
                             : kernel_registers(mvmr_tc_kernel<0>, &regs_mvmr[0]);
     const int occ = ctas_per_sm(smem + static_smem, p.ncols, regs);
     int64_t upper = a.T / CH + a.K + 1;
-    int64_t grid = std::min<int64_t>(upper, (int64_t)occ * num_sms());
+    const dim3 grid((unsigned)std::min<int64_t>(upper, std::max<int64_t>(1, (int64_t)occ * num_sms() / parts)), (unsigned)parts);
     prof_begin(store ? (a.transpose ? "mvmr_tc_kernel(dgrad, store)" : "mvmr_tc_kernel(fwd, store)")
                      : (a.transpose ? "mvmr_tc_kernel(dgrad)" : "mvmr_tc_kernel(fwd)"), stream);
-    if (store) mvmr_tc_kernel<2><<<(unsigned)grid, 128, smem, stream>>>(p);
-    else if (bulk) mvmr_tc_kernel<1><<<(unsigned)grid, 128, smem, stream>>>(p);
-    else mvmr_tc_kernel<0><<<(unsigned)grid, 128, smem, stream>>>(p);
+    if (store) mvmr_tc_kernel<2><<<grid, 128, smem, stream>>>(p);
+    else if (bulk) mvmr_tc_kernel<1><<<grid, 128, smem, stream>>>(p);
+    else mvmr_tc_kernel<0><<<grid, 128, smem, stream>>>(p);
     prof_end(stream);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
@@ -846,16 +878,16 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
 
 // One instantiation of the VVOR kernel: its shared-memory opt-in, its resident CTAs, its launch.
 template <int NT, int CHR, bool RING>
-int launch_vvor(const VvorTcParams &p, int64_t chunks_upper, size_t smem, size_t static_smem, cudaStream_t stream) {
+int launch_vvor(const VvorTcParams &p, int parts, int64_t chunks_upper, size_t smem, size_t static_smem, cudaStream_t stream) {
     static int granted[64] = {};   // per device
     static int regs = 0;
     int dev = 0;
     PCX_CUDA(cudaGetDevice(&dev));
     if (int rc = ensure_dynamic_smem(vvor_tc_kernel<NT, CHR, RING>, smem, &granted[dev & 63])) return rc;
     const int occ = ctas_per_sm(smem + static_smem, p.ncols, kernel_registers(vvor_tc_kernel<NT, CHR, RING>, &regs), NT);
-    const int64_t grid = std::min<int64_t>(chunks_upper, (int64_t)occ * num_sms());
+    const dim3 grid((unsigned)std::min<int64_t>(chunks_upper, std::max<int64_t>(1, (int64_t)occ * num_sms() / parts)), (unsigned)parts);
     prof_begin("vvor_tc_kernel", stream);
-    vvor_tc_kernel<NT, CHR, RING><<<(unsigned)grid, NT, smem, stream>>>(p);
+    vvor_tc_kernel<NT, CHR, RING><<<grid, NT, smem, stream>>>(p);
     prof_end(stream);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
@@ -865,10 +897,13 @@ int vvor_tensor(const VvorArgs &a, cudaStream_t stream) {
     VvorTcParams p;
     p.a = (const uint16_t *)a.a, p.b = (const uint16_t *)a.b, p.a_idx = a.a_idx, p.b_idx = a.b_idx;
     p.seg = a.seg_offs, p.acc = a.acc;
-    p.n_o = (int)a.n_o, p.Ma = a.Ma, p.Cb = a.Cb, p.fmt = a.dtype == PCX_BF16 ? 1 : 0;
-    const int row_tiles = (a.Ma + 127) / 128;
-    p.ncols = pow2_cols((row_tiles - 1) * a.Cb + (a.Cb + 63) / 64 * 64);  // flushed in blocks of 64 columns
-    const size_t blocks = (size_t)((a.Ma + 63) / 64 + (a.Cb + 63) / 64);
+    p.a_parts = parts_of(a.Ma), p.b_parts = parts_of(a.Cb);
+    const int Ma = a.Ma / p.a_parts, Cb = a.Cb / p.b_parts, parts = a.G * p.a_parts * p.b_parts;   // the part's widths
+    p.a_pitch = (int64_t)a.G * a.Ma, p.b_pitch = (int64_t)a.G * a.Cb, p.acc_pitch = a.Cb, p.acc_tap = (int64_t)a.G * a.Ma * a.Cb;
+    p.n_o = (int)a.n_o, p.Ma = Ma, p.Cb = Cb, p.fmt = a.dtype == PCX_BF16 ? 1 : 0;
+    const int row_tiles = (Ma + 127) / 128;
+    p.ncols = pow2_cols((row_tiles - 1) * Cb + (Cb + 63) / 64 * 64);  // flushed in blocks of 64 columns
+    const size_t blocks = (size_t)((Ma + 63) / 64 + (Cb + 63) / 64);
     // one stage = both operand tiles plus their index rows
     // (index rows: two per stage and operand, the ring variant fetches them ahead of the copies)
     auto stage_bytes = [&](int chr) { return blocks * (size_t)chr * 128 + 4 * (size_t)chr * sizeof(int32_t); };
@@ -911,17 +946,17 @@ int vvor_tensor(const VvorArgs &a, cudaStream_t stream) {
     if (smem + static_smem > 232448 - 1024) PCX_FAIL(PCX_E_UNSUPPORTED, "vvor tensor kernel does not fit (smem %zu)", smem);
     const int64_t upper = a.T / chr + a.n_o + 1;
     if (chr == 128) {
-        if (threads == 128) return launch_vvor<128, 128, false>(p, upper, smem, static_smem, stream);
-        if (threads == 256) return launch_vvor<256, 128, false>(p, upper, smem, static_smem, stream);
-        return launch_vvor<512, 128, false>(p, upper, smem, static_smem, stream);
+        if (threads == 128) return launch_vvor<128, 128, false>(p, parts, upper, smem, static_smem, stream);
+        if (threads == 256) return launch_vvor<256, 128, false>(p, parts, upper, smem, static_smem, stream);
+        return launch_vvor<512, 128, false>(p, parts, upper, smem, static_smem, stream);
     }
     if (stages == 1) {
-        if (threads == 128) return launch_vvor<128, 64, false>(p, upper, smem, static_smem, stream);
-        if (threads == 256) return launch_vvor<256, 64, false>(p, upper, smem, static_smem, stream);
-        return launch_vvor<512, 64, false>(p, upper, smem, static_smem, stream);
+        if (threads == 128) return launch_vvor<128, 64, false>(p, parts, upper, smem, static_smem, stream);
+        if (threads == 256) return launch_vvor<256, 64, false>(p, parts, upper, smem, static_smem, stream);
+        return launch_vvor<512, 64, false>(p, parts, upper, smem, static_smem, stream);
     }
-    if (threads <= 256) return launch_vvor<256, 64, true>(p, upper, smem, static_smem, stream);   // the ring wants the warps
-    return launch_vvor<512, 64, true>(p, upper, smem, static_smem, stream);
+    if (threads <= 256) return launch_vvor<256, 64, true>(p, parts, upper, smem, static_smem, stream);   // the ring wants the warps
+    return launch_vvor<512, 64, true>(p, parts, upper, smem, static_smem, stream);
 }
 
 // Device address of the status word, for kernels of other translation units.

@@ -205,11 +205,11 @@ __device__ __forceinline__ void red_add_v2(float *addr, float a, float b) {
 }
 // Adds one 16 x 64 accumulator block to fp32 rows in global memory.
 //   row_a / row_b: destination rows of this thread's two accumulator rows (-1 = skip)
-//   width: row length of the destination; col0: first column of the block
-__device__ __forceinline__ void scatter_block(float *dst, int64_t row_a, int64_t row_b, int width, int col0,
+//   width: columns of the destination tile; pitch: distance of its rows; col0: first column of the block
+__device__ __forceinline__ void scatter_block(float *dst, int64_t row_a, int64_t row_b, int width, int64_t pitch, int col0,
                                               int lane, const float *v) {
     const int c = col0 + 2 * (lane & 3);
-    float *pa = dst + row_a * width + c, *pb = dst + row_b * width + c;
+    float *pa = dst + row_a * pitch + c, *pb = dst + row_b * pitch + c;
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
         if (col0 + 8 * n < width) {

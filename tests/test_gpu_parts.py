@@ -1,0 +1,101 @@
+"""Layers whose widths the tensor engines take in parts or padded: channel counts that are not multiples of 16,
+rows wider than 256 channels, grouped weights -- on the scatter kernel, the output-stationary kernel (split by
+taps where the cloud is small, whole groups where it is not) and the weight-gradient kernel, against fp64.
+
+Tolerance: the operands are exact in the reference.  A result is rounded once (2^-9 relative at most, bf16;
+2^-12, fp16), a bucket sum of the output-stationary kernel once more; relative Frobenius errors stay below
+2^-8.5 = 2.8e-3 (bf16) and 2^-11.5 = 3.5e-4 (fp16), the fp32 sums add less than 1e-5."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+TOL = {torch.bfloat16: 2.9e-3, torch.float16: 3.7e-4}
+
+
+def _rulebook(n_out, n_in, K, T, seed):
+    g = torch.Generator(device=DEV).manual_seed(seed)
+    k = torch.sort(torch.randint(0, K, (T,), device=DEV, generator=g)).values
+    i = torch.randint(0, n_out, (T,), device=DEV, generator=g)
+    order = torch.argsort(k * n_out + i, stable=True)
+    i, j = i[order].int(), torch.randint(0, n_in, (T,), device=DEV, generator=g).int()
+    seg = torch.searchsorted(k, torch.arange(K + 1, device=DEV)).to(torch.int64)
+    return i, j, k, seg
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm().clamp_min(1e-30))
+
+
+CASES = [  # n_out, n_in, K, T, G, C, M, dtype
+    (1, 1, 1, 1, 1, 3, 16, torch.bfloat16),
+    (300, 257, 27, 4000, 1, 6, 32, torch.bfloat16),
+    (129, 200, 27, 5000, 1, 20, 20, torch.float16),
+    (500, 400, 125, 9000, 1, 3, 272, torch.bfloat16),
+    (400, 380, 27, 12000, 1, 512, 512, torch.float16),
+    (260, 300, 8, 2500, 1, 384, 320, torch.bfloat16),
+    (513, 513, 27, 9000, 2, 48, 256, torch.bfloat16),
+    (300, 300, 27, 3000, 2, 3, 10, torch.float16),
+    (200, 220, 27, 4000, 4, 16, 320, torch.bfloat16),
+    (80000, 80000, 27, 500000, 1, 32, 48, torch.bfloat16),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: "x".join(str(v) for v in c[:7]))
+def test_padded_wide_and_grouped_layers(case):
+    from pointelligence_b200 import _cabi
+    from pointelligence_b200.sparse_engines.tig import TigIndex, tig_mvmr
+
+    n_out, n_in, K, T, G, C, M, dtype = case
+    i, j, k, seg = _rulebook(n_out, n_in, K, T, 3)
+    g = torch.Generator(device=DEV).manual_seed(4)
+    w = (torch.randn(K, G, C, M, device=DEV, generator=g) / C ** 0.5).to(dtype)
+    x = torch.randn(n_in, G * C, device=DEV, generator=g).to(dtype)
+    go = torch.randn(n_out, G * M, device=DEV, generator=g).to(dtype)
+    b = torch.randn(G * M, device=DEV, generator=g).to(dtype)
+    y_ref = torch.zeros(n_out, G, M, dtype=torch.float64, device=DEV)
+    gx_ref = torch.zeros(n_in, G, C, dtype=torch.float64, device=DEV)
+    gw_ref = torch.zeros(K, G, C, M, dtype=torch.float64, device=DEV)
+    xd, gd, wd = x.double().view(n_in, G, C), go.double().view(n_out, G, M), w.double()
+    for tap in range(K):
+        a, e = int(seg[tap]), int(seg[tap + 1])
+        ii, jj = i[a:e].long(), j[a:e].long()
+        y_ref.index_add_(0, ii, torch.einsum("tgc,gcm->tgm", xd[jj], wd[tap]))
+        gx_ref.index_add_(0, jj, torch.einsum("tgm,gcm->tgc", gd[ii], wd[tap]))
+        gw_ref[tap] = torch.einsum("tgc,tgm->gcm", xd[jj], gd[ii])
+    tol = TOL[dtype]
+    # the layer: bias, forward and the three gradients
+    index = TigIndex.from_flat(i, j, seg, n_out, n_in, K)
+    ws, xs, bs = (t.clone().requires_grad_() for t in (w, x, b))
+    y = tig_mvmr(ws, xs, index, bias=bs)
+    y.backward(go)
+    assert _rel(y, y_ref.view(n_out, -1) + b.double()) < tol
+    assert _rel(xs.grad, gx_ref.view(n_in, -1)) < tol and _rel(ws.grad, gw_ref) < tol
+    assert _rel(bs.grad, go.double().sum(0)) < tol
+    # every engine that takes these widths
+    if C % 16 == 0 and M % 16 == 0 and C != 320:
+        for engine in (_cabi.ENGINE_TENSOR, _cabi.ENGINE_PLANNED):
+            out = _cabi.mvmr(w, x, j, i, seg, None, n_out, False, engine)
+            assert _rel(out, y_ref.view(n_out, -1)) < tol, engine
+            gx = _cabi.mvmr(w, go, i, j, seg, None, n_in, True, engine)
+            assert _rel(gx, gx_ref.view(n_in, -1)) < tol, engine
+        again = _cabi.mvmr(w, x, j, i, seg, None, n_out, False, _cabi.ENGINE_PLANNED)
+        assert torch.equal(out, again)            # fixed order of every sum, split or not
+    assert _cabi.device_status() == 0
+
+
+def test_output_row_count_one_above_a_whole_wave_of_groups():
+    """75 777 rows: 297 groups, the first count that is not split, and a last block of one row."""
+    from pointelligence_b200 import _cabi
+
+    n, K, T = 296 * 256 + 1, 27, 300000
+    i, j, k, seg = _rulebook(n, n, K, T, 9)
+    i[-1] = n - 1
+    w = torch.randn(K, 1, 32, 32, device=DEV).bfloat16() / 6
+    x = torch.randn(n, 32, device=DEV).bfloat16()
+    out = _cabi.mvmr(w, x, j, i, seg, None, n, False, _cabi.ENGINE_PLANNED)
+    ref = torch.zeros(n, 32, dtype=torch.float64, device=DEV)
+    for tap in range(K):
+        a, e = int(seg[tap]), int(seg[tap + 1])
+        ref.index_add_(0, i[a:e].long(), x[j[a:e].long()].double() @ w[tap, 0].double())
+    assert _rel(out, ref) < TOL[torch.bfloat16]
