@@ -549,8 +549,8 @@ def run_ours(args, rank, local_rank, world):
         balg = algorithmic_bytes(T, n, n, C, M, K)
         label_to_pass = {"mvmr_tc_kernel(fwd)": "fwd", "mvmr_tc_kernel(dgrad)": "dgrad", "vvor_tc_kernel": "wgrad",
                          "mvmr_os_kernel(fwd)": "fwd", "mvmr_os_kernel(dgrad)": "dgrad",
-                         "mvmr_sorted_kernel(fwd)": "fwd", "mvmr_sorted_kernel(dgrad)": "dgrad",
-                         "vvor_sorted_kernel": "wgrad"}
+                         "mvmr_fma_kernel(fwd)": "fwd", "mvmr_fma_kernel(dgrad)": "dgrad",
+                         "vvor_fma_kernel": "wgrad"}
         avg = {name: ms for name, ms in avg.items() if name in label_to_pass}
         dominant = max(avg, key=avg.get)
         dom_pass = label_to_pass[dominant]

@@ -46,74 +46,10 @@ constexpr int BLK_BYTES = CH * 128; // one 64-channel block of a 128-row tile
 
 using namespace tc;
 
-// Position of a CTA in the chunk sequence; the bounds of the current tap are
-// kept in registers and reloaded only when the chunk index leaves the tap.
-// The cumulative chunk table lives in shared memory (built by every CTA from
-// the segment offsets), so no separate kernel and no global table are needed.
-template <int CHR>
-struct ChunkCursorT {
-    int tap;
-    int cum_lo, cum_hi;
-    int64_t seg_lo, seg_hi;
-    __device__ __forceinline__ void load(const int32_t *cum, const int64_t *__restrict__ seg) {
-        cum_lo = cum[tap], cum_hi = cum[tap + 1];
-        seg_lo = seg[tap], seg_hi = seg[tap + 1];
-    }
-    __device__ __forceinline__ void seek(const int32_t *cum, const int64_t *__restrict__ seg, int K, int chunk) {
-        int lo = 0, hi = K;
-        while (hi - lo > 1) {
-            int mid = (lo + hi) >> 1;
-            if (cum[mid] <= chunk) lo = mid; else hi = mid;
-        }
-        tap = lo;
-        load(cum, seg);
-    }
-    __device__ __forceinline__ void advance(const int32_t *cum, const int64_t *__restrict__ seg, int K, int chunk) {
-        if (chunk < cum_hi) return;
-        while (tap + 1 < K && cum[tap + 1] <= chunk) ++tap;
-        load(cum, seg);
-    }
-    __device__ __forceinline__ int64_t first(int chunk) const { return seg_lo + (int64_t)(chunk - cum_lo) * CHR; }
-    __device__ __forceinline__ int rows(int chunk) const {
-        int64_t left = seg_hi - first(chunk);
-        return (int)(left < CHR ? left : CHR);
-    }
-    __device__ __forceinline__ bool last_of_tap(int chunk) const { return chunk + 1 >= cum_hi; }
-};
 using ChunkCursor = ChunkCursorT<CH>;
 
 constexpr int MAX_PARTS = 64;        // (group, part, part) combinations of one launch
 constexpr int MAX_TAPS_SMEM = 1024;  // taps whose chunk table fits the shared-memory copy
-
-// cum[k] = chunks of CHR triplets in the taps before k; all threads of the CTA call this.
-template <int CHR = CH>
-__device__ __forceinline__ void build_chunk_table(const int64_t *__restrict__ seg, int K, int32_t *cum,
-                                                  int32_t *warp_sums) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    int32_t carry = 0;
-    for (int base = 0; base < K; base += blockDim.x) {
-        int k = base + tid;
-        int32_t v = k < K ? (int32_t)((seg[k + 1] - seg[k] + CHR - 1) / CHR) : 0;
-        int32_t inc = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int32_t n = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += n;
-        }
-        if (lane == 31) warp_sums[warp] = inc;
-        __syncthreads();
-        int32_t before = carry, all = carry;
-        for (int w = 0; w < nwarps; ++w) {
-            if (w < warp) before += warp_sums[w];
-            all += warp_sums[w];
-        }
-        if (k < K) cum[k] = before + inc - v;
-        carry = all;
-        __syncthreads();
-    }
-    if (tid == 0) cum[K] = carry;
-    __syncthreads();
-}
 
 // Gather `rows` rows of `width` 2-byte channels into a swizzled tile; the row
 // (`pitch` elements apart) were staged in shared memory beforehand so that the copy loop issues
@@ -257,7 +193,7 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(smem_u32(&s_tmem), p.ncols);
-    build_chunk_table(p.seg, p.K, s_cum, s_warp_sums);
+    build_chunk_table<CH>(p.seg, p.K, s_cum, s_warp_sums);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
