@@ -182,6 +182,16 @@ int pcx_mvmr_plan_build(const int32_t *d_scatter, const int32_t *d_gather,
                         int64_t n_out, int group_blocks, void *d_plan,
                         size_t plan_bytes, void *d_ws, size_t ws_bytes,
                         void *stream);
+/* ... and the number of buckets with several triplets, for which both build
+ * entries synchronise `stream`.  Rulebooks whose rows ascend inside every tap
+ * (what pcx_radius_taps_fill emits) are regrouped by counting, others by
+ * sorting their triplets. */
+int pcx_mvmr_plan_build_counted(const int32_t *d_scatter,
+                                const int32_t *d_gather,
+                                const int64_t *d_seg_offs, int64_t T, int K,
+                                int64_t n_out, int group_blocks, void *d_plan,
+                                size_t plan_bytes, void *d_ws, size_t ws_bytes,
+                                int64_t *h_multi, void *stream);
 int pcx_mvmr_plan_multi_buckets(const void *d_plan, int64_t *h_count,
                                 void *stream);
 size_t pcx_mvmr_planned_workspace_bytes(int64_t multi_buckets, int in_width);

@@ -56,6 +56,8 @@ SIGNATURES = {
     "pcx_mvmr_plan_workspace_bytes": (c_size_t, [c_int64, c_int64, c_int, c_int]),
     "pcx_mvmr_plan_build": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int64, c_int, c_void_p, c_size_t, c_void_p,
                                     c_size_t, c_void_p]),
+    "pcx_mvmr_plan_build_counted": (c_int, [c_void_p] * 3 + [c_int64, c_int, c_int64, c_int, c_void_p, c_size_t,
+                                            c_void_p, c_size_t, ctypes.POINTER(c_int64), c_void_p]),
     "pcx_mvmr_plan_multi_buckets": (c_int, [c_void_p, ctypes.POINTER(c_int64), c_void_p]),
     "pcx_mvmr_planned_workspace_bytes": (c_size_t, [c_int64, c_int]),
     "pcx_mvmr_planned": (c_int, [c_void_p] * 3 + [c_size_t, c_void_p] + [c_int64] * 3 + [c_int] * 6

@@ -499,10 +499,9 @@ std::tuple<Tensor, int64_t> plan_build(const Tensor &scatter_, const Tensor &gat
                                              " K=" + std::to_string(K) + " group=" + std::to_string(group));
     }
     Tensor buf = workspace(bytes, scatter), ws = workspace(pcx_mvmr_plan_workspace_bytes(T, n_out, (int)K, (int)group), scatter);
-    check(pcx_mvmr_plan_build(ptr_as<int32_t>(scatter), ptr_as<int32_t>(gather), ptr_as<int64_t>(seg), T, (int)K, n_out, (int)group,
-                              ptr(buf), buf.numel(), ptr(ws), ws.numel(), stream()));
     int64_t multi = 0;
-    check(pcx_mvmr_plan_multi_buckets(ptr(buf), &multi, stream()));
+    check(pcx_mvmr_plan_build_counted(ptr_as<int32_t>(scatter), ptr_as<int32_t>(gather), ptr_as<int64_t>(seg), T, (int)K, n_out, (int)group,
+                                      ptr(buf), buf.numel(), ptr(ws), ws.numel(), &multi, stream()));
     return {buf, multi};
 }
 

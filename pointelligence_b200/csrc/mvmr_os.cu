@@ -64,7 +64,7 @@ constexpr unsigned STATUS_BIT = 4u;   // bit of the device status word this kern
 constexpr unsigned PLAN_MAGIC = 0x70637832u;
 
 // control words at the head of a plan
-enum { CTRL_MAGIC = 2, CTRL_GROUP = 3, CTRL_NMULTI = 4, CTRL_WORDS = 64 };
+enum { CTRL_MAGIC = 2, CTRL_GROUP = 3, CTRL_NMULTI = 4, CTRL_UNSORTED = 5, CTRL_WORDS = 64 };
 
 struct PlanView {
     uint32_t *ctrl;        // CTRL_WORDS
@@ -102,7 +102,8 @@ int bits_of(int64_t n) {
 }
 
 struct BuildWs {
-    uint32_t *sig, *sig_sorted;          // n_out
+    uint32_t *sig;                       // n_out
+    uint64_t *order, *order_sorted;      // n_out
     int32_t *row, *row_sorted, *rank;    // n_out
     uint32_t *key, *key_sorted;          // T
     int32_t *val, *val_sorted;           // T
@@ -119,7 +120,8 @@ size_t carve_build(void *base, int64_t T, int64_t n_out, int K, int G, BuildWs *
     const int64_t nblocks = (n_out + ROWS - 1) / ROWS, ngroups = (nblocks + G - 1) / G;
     const size_t n = (size_t)std::max<int64_t>(n_out, 1), t = (size_t)std::max<int64_t>(T, 1);
     const size_t g = (size_t)std::max<int64_t>(ngroups, 1);
-    w.sig = c.take<uint32_t>(n), w.sig_sorted = c.take<uint32_t>(n);
+    w.sig = c.take<uint32_t>(n);
+    w.order = c.take<uint64_t>(n), w.order_sorted = c.take<uint64_t>(n);
     w.row = c.take<int32_t>(n), w.row_sorted = c.take<int32_t>(n), w.rank = c.take<int32_t>(n);
     w.key = c.take<uint32_t>(t), w.key_sorted = c.take<uint32_t>(t);
     w.val = c.take<int32_t>(t), w.val_sorted = c.take<int32_t>(t);
@@ -127,8 +129,8 @@ size_t carve_build(void *base, int64_t T, int64_t n_out, int K, int G, BuildWs *
     w.cost = c.take<uint32_t>(g), w.cost_sorted = c.take<uint32_t>(g);
     w.gid = c.take<int32_t>(g);
     size_t b1 = 0, b2 = 0, b3 = 0, b4 = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, b1, (const uint32_t *)nullptr, (uint32_t *)nullptr, (const int32_t *)nullptr,
-                                    (int32_t *)nullptr, (int)n, 0, 32);
+    cub::DeviceRadixSort::SortPairs(nullptr, b1, (const uint64_t *)nullptr, (uint64_t *)nullptr, (const int32_t *)nullptr,
+                                    (int32_t *)nullptr, (int)n, 0, 64);
     cub::DeviceRadixSort::SortPairs(nullptr, b2, (const uint32_t *)nullptr, (uint32_t *)nullptr, (const int32_t *)nullptr,
                                     (int32_t *)nullptr, (int)t, 0, 32);
     cub::DeviceScan::ExclusiveSum(nullptr, b3, (const int32_t *)nullptr, (int32_t *)nullptr, (int)((size_t)nblocks * K + 1));
@@ -149,13 +151,18 @@ __device__ __forceinline__ uint32_t pack2(float a, float b, int fmt) {
     return *reinterpret_cast<uint32_t *>(&v);
 }
 
-__device__ __forceinline__ int tap_of(const int64_t *__restrict__ seg, int K, int64_t t) {
-    int lo = 0, hi = K;  // last k with seg[k] <= t
+// Tap of triplet t: last k with seg[k] <= t; `seg` is the CTA's copy of the segment offsets.
+__device__ __forceinline__ int tap_of(const int64_t *seg, int K, int64_t t) {
+    int lo = 0, hi = K;
     while (hi - lo > 1) {
         int mid = (lo + hi) >> 1;
         if (seg[mid] <= t) lo = mid; else hi = mid;
     }
     return lo;
+}
+__device__ __forceinline__ void copy_seg(const int64_t *__restrict__ seg, int K, int64_t *s_seg) {
+    for (int k = threadIdx.x; k <= K; k += blockDim.x) s_seg[k] = seg[k];
+    __syncthreads();
 }
 
 __global__ void plan_init_kernel(int64_t n_out, uint32_t *sig, int32_t *row, int32_t *tile_cnt, int64_t n_tiles,
@@ -167,27 +174,38 @@ __global__ void plan_init_kernel(int64_t n_out, uint32_t *sig, int32_t *row, int
 }
 
 // Tap signature of every output row.  With more than 32 taps the taps are folded onto 32
-// bits (tap mod 32): rows that share a signature then share a superset of taps.
+// bits (tap mod 32): rows that share a signature then share a superset of taps.  Notes rulebooks
+// whose rows do not ascend inside a tap.
 __global__ void plan_sig_kernel(const int32_t *__restrict__ scatter, const int64_t *__restrict__ seg, int64_t T, int K,
-                                uint32_t *sig) {
+                                uint32_t *sig, uint32_t *ctrl) {
+    __shared__ int64_t s_seg[MAX_TAPS + 1];
+    copy_seg(seg, K, s_seg);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T) return;
-    atomicOr(&sig[scatter[t]], 1u << (tap_of(seg, K, t) & 31));
+    const int k = tap_of(s_seg, K, t);
+    const int32_t r = scatter[t];
+    if (t > s_seg[k]) {
+        const int32_t before = scatter[t - 1];
+        if (before == r) return;   // the first triplet of the bucket says it
+        if (before > r) ctrl[CTRL_UNSORTED] = 1u;
+    }
+    atomicOr(&sig[r], 1u << (k & 31));
 }
 
-// Second sort key of the rows of a cubic kernel (K = ks^3 <= 32 taps, tap = (kx * ks + ky) * ks + kz):
-// which kx / ky / kz planes of the kernel a row uses at all, kz most significant.  Points of a
-// scene lie on surfaces; rows of one surface orientation share these planes even where their
-// exact tap sets differ, and sorted by (planes, signature) the blocks of 128 rows need a quarter
-// fewer (block, tap) tiles on thin rulebooks than sorted by signature alone.
-__global__ void plan_planes_kernel(const uint32_t *__restrict__ sig_sorted, int64_t n_out, int K, int ks, uint32_t *planes) {
+// Sort key of the rows: the signature and, above it for a cubic kernel (K = ks^3 <= 32 taps, tap =
+// (kx * ks + ky) * ks + kz), which kx / ky / kz planes of the kernel a row uses at all, kz most
+// significant.  Points of a scene lie on surfaces; rows of one surface orientation share these planes
+// even where their exact tap sets differ, and sorted by (planes, signature) the blocks of 128 rows need
+// a quarter fewer (block, tap) tiles on thin rulebooks than sorted by signature alone.
+__global__ void plan_order_kernel(const uint32_t *__restrict__ sig, int64_t n_out, int K, int ks, uint64_t *order) {
     const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= n_out) return;
-    const uint32_t m = sig_sorted[x];
+    const uint32_t m = sig[x];
     uint32_t px = 0, py = 0, pz = 0;
-    for (int tap = 0; tap < K; ++tap)
-        if ((m >> tap) & 1u) px |= 1u << (tap / (ks * ks)), py |= 1u << ((tap / ks) % ks), pz |= 1u << (tap % ks);
-    planes[x] = px | (py << ks) | (pz << (2 * ks));
+    if (ks)
+        for (int tap = 0; tap < K; ++tap)
+            if ((m >> tap) & 1u) px |= 1u << (tap / (ks * ks)), py |= 1u << ((tap / ks) % ks), pz |= 1u << (tap % ks);
+    order[x] = (uint64_t)m | (uint64_t)(px | (py << ks) | (pz << (2 * ks))) << (K < 32 ? K : 32);
 }
 
 __global__ void plan_rank_kernel(const int32_t *__restrict__ row_sorted, int64_t n_out, int64_t n_pad, int32_t *rank,
@@ -203,12 +221,88 @@ __global__ void plan_rank_kernel(const int32_t *__restrict__ row_sorted, int64_t
     }
 }
 
+// ---- rulebooks whose rows ascend inside a tap (what the geometry stage emits): a (row, tap) bucket is a run of
+// consecutive triplets, so everything is placed by counting and no triplet is sorted.
+
+// tile_rows[tile * 128 + slot] = first triplet of the bucket; triplets per tile
+__global__ void plan_heads_kernel(const int32_t *__restrict__ scatter, const int64_t *__restrict__ seg, const int32_t *__restrict__ rank,
+                                  int64_t T, int K, int32_t *tile_rows, int32_t *tile_cnt) {
+    __shared__ int64_t s_seg[MAX_TAPS + 1];
+    copy_seg(seg, K, s_seg);
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= T) return;
+    const int k = tap_of(s_seg, K, t);
+    const int32_t row = scatter[t];
+    if (t > s_seg[k] && scatter[t - 1] == row) return;
+    int len = 1;
+    while (t + len < s_seg[k + 1] && scatter[t + len] == row) ++len;
+    const uint32_t r = (uint32_t)rank[row], tile = (r >> 7) * (uint32_t)K + (uint32_t)k;
+    tile_rows[((int64_t)tile << 7) | (r & 127u)] = (int32_t)t;
+    atomicAdd(&tile_cnt[tile], len);
+}
+
+// One warp per (block, tap) tile: entries in slot order, the tile's source rows, its multi-triplet buckets.
+__global__ void plan_tiles_kernel(const int32_t *__restrict__ scatter, const int32_t *__restrict__ gather, const int64_t *__restrict__ seg,
+                                  int K, int64_t n_tiles, const int32_t *__restrict__ tile_offs, uint2 *entries, int32_t *tile_rows,
+                                  uint2 *buckets, uint32_t *ctrl) {
+    const int64_t tile = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int lane = threadIdx.x & 31;
+    if (tile >= n_tiles) return;
+    const int32_t first = tile_offs[tile];
+    if (tile_offs[tile + 1] == first) return;   // no triplets: its rows say "none" already
+    const int64_t end = seg[tile % K + 1];
+    int4 *slots = reinterpret_cast<int4 *>(tile_rows + (tile << 7)) + lane;
+    const int4 h = *slots;
+    const int32_t head[4] = {h.x, h.y, h.z, h.w};
+    int len[4], sum = 0, multi = 0;
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        len[s] = 0;
+        if (head[s] >= 0) {
+            const int32_t row = scatter[head[s]];
+            len[s] = 1;
+            while (head[s] + len[s] < end && scatter[head[s] + len[s]] == row) ++len[s];
+        }
+        sum += len[s], multi += len[s] > 1;
+    }
+    int at = sum, nth = multi;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int a = __shfl_up_sync(0xffffffffu, at, o), b = __shfl_up_sync(0xffffffffu, nth, o);
+        if (lane >= o) at += a, nth += b;
+    }
+    const int total = __shfl_sync(0xffffffffu, nth, 31);
+    uint32_t base = 0;
+    if (lane == 0 && total) base = atomicAdd(&ctrl[CTRL_NMULTI], (uint32_t)total);
+    base = __shfl_sync(0xffffffffu, base, 0) + (uint32_t)(nth - multi);
+    uint32_t entry = (uint32_t)(first + at - sum);
+    int32_t source[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+        source[s] = -1;
+        for (int m = 0; m < len[s]; ++m) {
+            const int32_t j = gather[head[s] + m];
+            entries[entry + m] = make_uint2((uint32_t)(lane * 4 + s) | ((uint32_t)min(m, 0xffffff) << 8), (uint32_t)j);
+            if (len[s] == 1) source[s] = j;
+        }
+        if (len[s] > 1) {
+            buckets[base] = make_uint2(entry, (uint32_t)len[s]);
+            source[s] = -2 - (int32_t)base++;
+        }
+        entry += (uint32_t)len[s];
+    }
+    *slots = make_int4(source[0], source[1], source[2], source[3]);
+}
+
+// ---- any other tap-sorted rulebook: the triplets are sorted by (block, tap, slot)
 __global__ void plan_keys_kernel(const int32_t *__restrict__ scatter, const int32_t *__restrict__ gather,
                                  const int64_t *__restrict__ seg, const int32_t *__restrict__ rank, int64_t T, int K,
                                  uint32_t *key, int32_t *val, int32_t *tile_cnt) {
+    __shared__ int64_t s_seg[MAX_TAPS + 1];
+    copy_seg(seg, K, s_seg);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T) return;
-    const int k = tap_of(seg, K, t);
+    const int k = tap_of(s_seg, K, t);
     const uint32_t r = (uint32_t)rank[scatter[t]];
     const uint32_t tile = (r >> 7) * (uint32_t)K + (uint32_t)k;
     key[t] = (tile << 7) | (r & 127u);
@@ -799,6 +893,17 @@ bool plan_sizes_ok(int64_t T, int64_t n_out, int K, int G) {
     return nblocks * K * ROWS <= ((int64_t)1 << 32) && nblocks * K < INT32_MAX;
 }
 
+// groups, most tiles first, and the tap sets of their blocks
+int order_groups(const PlanView &pv, const BuildWs &w, int K, int G, cudaStream_t stream) {
+    plan_cost_kernel<<<(unsigned)((pv.ngroups + 255) / 256), 256, 0, stream>>>(pv.tile_offs, pv.nblocks, K, G, pv.ngroups, w.cost, w.gid,
+                                                                               pv.tap_masks);
+    PCX_LAUNCH_CHECK();
+    size_t bytes = w.cub_bytes;
+    PCX_CUDA(cub::DeviceRadixSort::SortPairsDescending(w.cub_tmp, bytes, w.cost, w.cost_sorted, w.gid, pv.group_order, (int)pv.ngroups, 0,
+                                                       bits_of((int64_t)G * K + 2), stream));
+    return PCX_OK;
+}
+
 }  // namespace
 }  // namespace pcx
 
@@ -825,13 +930,21 @@ size_t pcx_mvmr_plan_workspace_bytes(int64_t T, int64_t n_out, int K, int group_
 
 int pcx_mvmr_plan_build(const int32_t *d_scatter, const int32_t *d_gather, const int64_t *d_seg_offs, int64_t T, int K,
                         int64_t n_out, int group_blocks, void *d_plan, size_t plan_bytes, void *d_ws, size_t ws_bytes,
-                        void *stream_) {
+                        void *stream) {
+    int64_t multi = 0;
+    return pcx_mvmr_plan_build_counted(d_scatter, d_gather, d_seg_offs, T, K, n_out, group_blocks, d_plan, plan_bytes, d_ws, ws_bytes,
+                                       &multi, stream);
+}
+
+int pcx_mvmr_plan_build_counted(const int32_t *d_scatter, const int32_t *d_gather, const int64_t *d_seg_offs, int64_t T, int K,
+                                int64_t n_out, int group_blocks, void *d_plan, size_t plan_bytes, void *d_ws, size_t ws_bytes,
+                                int64_t *h_multi, void *stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
     const int G = group_blocks;
     if (!plan_sizes_ok(T, n_out, K, G))
         PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_plan_build: sizes out of range (T=%lld n_out=%lld K=%d group=%d)", (long long)T,
                  (long long)n_out, K, G);
-    if (!d_plan || !d_ws || (T > 0 && (!d_scatter || !d_gather || !d_seg_offs)))
+    if (!d_plan || !d_ws || !h_multi || (T > 0 && (!d_scatter || !d_gather || !d_seg_offs)))
         PCX_FAIL(PCX_E_ARG, "pcx_mvmr_plan_build: null pointer");
     if ((uintptr_t)d_plan % 256 || (uintptr_t)d_ws % 256)
         PCX_FAIL(PCX_E_ALIGN, "pcx_mvmr_plan_build: plan and workspace must be 256-byte aligned");
@@ -849,46 +962,52 @@ int pcx_mvmr_plan_build(const int32_t *d_scatter, const int32_t *d_gather, const
     PCX_LAUNCH_CHECK();
     size_t bytes = w.cub_bytes;
     if (T > 0) {
-        plan_sig_kernel<<<blocks(T), TPB, 0, stream>>>(d_scatter, d_seg_offs, T, K, w.sig);
+        plan_sig_kernel<<<blocks(T), TPB, 0, stream>>>(d_scatter, d_seg_offs, T, K, w.sig, pv.ctrl);
         PCX_LAUNCH_CHECK();
     }
-    // rows by signature (stable: rows of equal signature keep their order) ...
-    PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, bytes, w.sig, w.sig_sorted, w.row, w.row_sorted, (int)n_out, 0,
-                                             std::min(K, 32), stream));
-    const int32_t *rows_in_order = w.row_sorted;
+    // rows by (planes, signature), stable: rows of equal keys keep their order
     int ks = 1;
     while (ks * ks * ks < K) ++ks;
-    if (ks * ks * ks == K && K <= 32 && K > 1) {
-        // ... and then, stable again, by the kernel planes they use: the order is (planes, signature)
-        plan_planes_kernel<<<blocks(n_out), TPB, 0, stream>>>(w.sig_sorted, n_out, K, ks, w.sig);
-        PCX_LAUNCH_CHECK();
-        bytes = w.cub_bytes;
-        PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, bytes, w.sig, w.sig_sorted, w.row_sorted, w.row, (int)n_out, 0,
-                                                 3 * ks, stream));
-        rows_in_order = w.row;
-    }
-    plan_rank_kernel<<<blocks(n_pad), TPB, 0, stream>>>(rows_in_order, n_out, n_pad, w.rank, pv.perm);
+    if (ks * ks * ks != K || K > 32 || K == 1) ks = 0;
+    plan_order_kernel<<<blocks(n_out), TPB, 0, stream>>>(w.sig, n_out, K, ks, w.order);
+    PCX_LAUNCH_CHECK();
+    PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, bytes, w.order, w.order_sorted, w.row, w.row_sorted, (int)n_out, 0,
+                                             std::min(K, 32) + 3 * ks, stream));
+    plan_rank_kernel<<<blocks(n_pad), TPB, 0, stream>>>(w.row_sorted, n_out, n_pad, w.rank, pv.perm);
     PCX_LAUNCH_CHECK();
     if (T > 0) {
-        plan_keys_kernel<<<blocks(T), TPB, 0, stream>>>(d_scatter, d_gather, d_seg_offs, w.rank, T, K, w.key, w.val, w.tile_cnt);
+        plan_heads_kernel<<<blocks(T), TPB, 0, stream>>>(d_scatter, d_seg_offs, w.rank, T, K, pv.tile_rows, w.tile_cnt);
         PCX_LAUNCH_CHECK();
-        bytes = w.cub_bytes;
-        PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, bytes, w.key, w.key_sorted, w.val, w.val_sorted, (int)T, 0,
-                                                 std::min(32, bits_of(n_tiles * ROWS)), stream));
     }
     bytes = w.cub_bytes;
     PCX_CUDA(cub::DeviceScan::ExclusiveSum(w.cub_tmp, bytes, w.tile_cnt, pv.tile_offs, (int)(n_tiles + 1), stream));
     if (T > 0) {
-        plan_entries_kernel<<<blocks(T), TPB, 0, stream>>>(w.key_sorted, w.val_sorted, T, pv.entries, pv.tile_rows, pv.buckets,
-                                                           pv.ctrl);
+        plan_tiles_kernel<<<blocks(n_tiles * 32), TPB, 0, stream>>>(d_scatter, d_gather, d_seg_offs, K, n_tiles, pv.tile_offs, pv.entries,
+                                                                   pv.tile_rows, pv.buckets, pv.ctrl);
         PCX_LAUNCH_CHECK();
     }
-    plan_cost_kernel<<<blocks(pv.ngroups), TPB, 0, stream>>>(pv.tile_offs, pv.nblocks, K, G, pv.ngroups, w.cost, w.gid, pv.tap_masks);
+    if (int rc = order_groups(pv, w, K, G, stream)) return rc;
+    uint32_t h[8] = {};
+    PCX_CUDA(cudaMemcpyAsync(h, pv.ctrl, sizeof(h), cudaMemcpyDeviceToHost, stream));
+    PCX_CUDA(cudaStreamSynchronize(stream));
+    *h_multi = h[CTRL_NMULTI];
+    if (!h[CTRL_UNSORTED]) return PCX_OK;
+
+    // rows out of order inside a tap: what comes after the row order once more, by sorting the triplets
+    PCX_CUDA(cudaMemsetAsync(pv.tile_rows, 0xff, (size_t)n_tiles * ROWS * sizeof(int32_t), stream));
+    PCX_CUDA(cudaMemsetAsync(w.tile_cnt, 0, (size_t)(n_tiles + 1) * sizeof(int32_t), stream));
+    PCX_CUDA(cudaMemsetAsync(pv.ctrl + CTRL_NMULTI, 0, sizeof(uint32_t), stream));
+    plan_keys_kernel<<<blocks(T), TPB, 0, stream>>>(d_scatter, d_gather, d_seg_offs, w.rank, T, K, w.key, w.val, w.tile_cnt);
     PCX_LAUNCH_CHECK();
     bytes = w.cub_bytes;
-    PCX_CUDA(cub::DeviceRadixSort::SortPairsDescending(w.cub_tmp, bytes, w.cost, w.cost_sorted, w.gid, pv.group_order,
-                                                       (int)pv.ngroups, 0, bits_of((int64_t)G * K + 2), stream));
-    return PCX_OK;
+    PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, bytes, w.key, w.key_sorted, w.val, w.val_sorted, (int)T, 0,
+                                             std::min(32, bits_of(n_tiles * ROWS)), stream));
+    bytes = w.cub_bytes;
+    PCX_CUDA(cub::DeviceScan::ExclusiveSum(w.cub_tmp, bytes, w.tile_cnt, pv.tile_offs, (int)(n_tiles + 1), stream));
+    plan_entries_kernel<<<blocks(T), TPB, 0, stream>>>(w.key_sorted, w.val_sorted, T, pv.entries, pv.tile_rows, pv.buckets, pv.ctrl);
+    PCX_LAUNCH_CHECK();
+    if (int rc = order_groups(pv, w, K, G, stream)) return rc;
+    return pcx_mvmr_plan_multi_buckets(d_plan, h_multi, stream);
 }
 
 size_t pcx_mvmr_planned_workspace_bytes(int64_t multi_buckets, int in_width) {

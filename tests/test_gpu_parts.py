@@ -118,3 +118,21 @@ def test_a_kept_sparse_rulebook_moves_to_the_output_stationary_kernel():
         _cabi.profile_enable(False)
         assert _rel(out, want.double()) < 2 * TOL[torch.bfloat16]     # two roundings apart
     assert set(labels[:-1]) == {"mvmr_tc_kernel(fwd)"} and labels[-1] == "mvmr_os_kernel(fwd)"
+
+
+def test_plan_of_rows_out_of_order_inside_a_tap():
+    """The counting path and the sorting path of the plan builder regroup the same triplets."""
+    from pointelligence_b200 import _cabi
+
+    n, K, T = 700, 27, 9000
+    i, j, k, seg = _rulebook(n, n, K, T, 13)
+    shuffle = torch.argsort(k * T + torch.randperm(T, device=DEV))
+    counted = _cabi.mvmr_plan(i, j, seg, K, n, 2)
+    sorted_ = _cabi.mvmr_plan(i[shuffle], j[shuffle], seg, K, n, 2)
+    a, b = counted.views(), sorted_.views()
+    assert torch.equal(a["perm"], b["perm"]) and torch.equal(a["tile_offs"], b["tile_offs"])
+    assert counted.multi_buckets == sorted_.multi_buckets > 0
+    assert torch.equal(a["entries"][:, 0], b["entries"][:, 0])
+    assert torch.equal(a["tile_rows"] < -1, b["tile_rows"] < -1) and torch.equal(a["tile_rows"].clamp_min(-1), b["tile_rows"].clamp_min(-1))
+    w, x = torch.randn(K, 1, 64, 64, device=DEV).bfloat16() / 8, torch.randn(n, 64, device=DEV).bfloat16()
+    assert _rel(_cabi.mvmr_planned(w, x, counted, False), _cabi.mvmr_planned(w, x, sorted_, False).double()) < TOL[torch.bfloat16]
