@@ -12,10 +12,12 @@
 //     the right cell keep their relative order (the sort is stable), so the output does not change.
 //     The low three bits of the hash are the parities of the cell coordinates, so the eight cells
 //     a query looks at always land in eight different buckets.
-//   * eight lanes serve one query, one lane per candidate cell, each walking its own short run;
-//     a block of 256 threads serves 32 consecutive queries.  The predicate runs alone over 64
-//     candidates at a time into a bit mask; the rarer accepted points are handled afterwards, and
-//     the fill pass reads the mask back instead of evaluating the predicate again.
+//   * eight lanes serve one query: each looks up the run of one of its cells, then the eight runs are walked as
+//     ONE list, 32 candidates at a time, so that lanes do not wait for the longest run (a lane per run kept
+//     22 % of them busy) and four loads per lane are in flight; the accepted points of a warp are queued and
+//     their taps computed 32 at a time.  The first 48 accepted points of a query (96 for more than 27 taps)
+//     are kept with their taps, so that the fill pass only places them; a warp with a longer list walks its
+//     runs again.  A block of 256 threads serves 32 consecutive queries.
 //   * the count pass leaves a per-block tap histogram; its prefix over blocks plus the tap
 //     segment offsets give every block its write position in every tap, so the fill pass places
 //     the pairs directly in tap-major order (a stable counting sort by tap inside the block):
@@ -47,9 +49,10 @@ struct TapsWs {
     int32_t *vals_a, *vals_b;
     float4 *sorted_pts;     // xyz + original index (bit pattern) in bucket order
     int2 *table;            // bucket -> [start, end) in the sorted order; (0,0) = empty
-    uint4 *lanes;           // Q x 8: candidate run [start, end) and the accept mask of its first 64 points
-    unsigned long long *lanes_more;   // Q x 8: accept mask of points 64 .. 127 of a run longer than 64
-    uint32_t *lane_counts;  // Q x 8 accepted pairs per (query, cell)
+    int32_t *sorted_sample; // sample ids in bucket order
+    int32_t *kept_point;    // Q x kept: the accepted points of a query, in output order
+    uint8_t *kept_tap;      // ... and their taps
+    uint32_t *counts;       // Q: accepted pairs
     uint32_t *block_hist;   // [tap][block] accepted pairs; exclusive prefix over blocks after the scan
     unsigned long long *tap_total;  // k3
     int64_t *seg;           // k3 + 1
@@ -61,10 +64,16 @@ struct TapsWs {
     int64_t buckets, nblocks;
 };
 
+int kept_per_query(int k3) { return k3 <= 27 ? 48 : 96; }
+
 int bucket_bits(int64_t P) {
     int b = 1;
     while (((int64_t)1 << b) < P) ++b;
     b += 1;
+    // The radix sort takes eight bits a pass: where two or three bits too many would cost a third pass (18 us of the
+    // search at 100 000 points), fewer buckets do -- a cell of side 2R holds several points, so that even then
+    // less than half of the buckets are taken.
+    if (b > 16 && b <= 18) b = 16;
     return b < 8 ? 8 : (b > 28 ? 28 : b);
 }
 
@@ -83,9 +92,10 @@ size_t carve_taps(void *ws, int64_t P, int64_t Q, int k3, TapsWs *out) {
     w.vals_b = c.take<int32_t>(P);
     w.sorted_pts = c.take<float4>(P);
     w.table = c.take<int2>(w.buckets);
-    w.lanes = c.take<uint4>(Q * 8);
-    w.lanes_more = c.take<unsigned long long>(Q * 8);
-    w.lane_counts = c.take<uint32_t>(Q * 8);
+    w.sorted_sample = c.take<int32_t>(P);
+    w.kept_point = c.take<int32_t>(Q * kept_per_query(k3));
+    w.kept_tap = c.take<uint8_t>(Q * kept_per_query(k3));
+    w.counts = c.take<uint32_t>(Q);
     w.block_hist = c.take<uint32_t>(w.nblocks * k3);
     w.cub_bytes = 0;
     cub::DeviceRadixSort::SortPairs(nullptr, w.cub_bytes, (const uint32_t *)nullptr, (uint32_t *)nullptr,
@@ -112,12 +122,14 @@ __global__ void taps_key_kernel(const float *__restrict__ pts, const int32_t *__
 }
 
 // Sorted copy of the points and the bucket table in one pass over the sorted keys.
-__global__ void taps_table_kernel(const float *__restrict__ pts, const uint32_t *__restrict__ keys,
-                                  const int32_t *__restrict__ perm, int64_t P, float4 *sorted_pts, int2 *table) {
+__global__ void taps_table_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, const uint32_t *__restrict__ keys,
+                                  const int32_t *__restrict__ perm, int64_t P, float4 *sorted_pts, int32_t *sorted_sample,
+                                  int2 *table) {
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (s >= P) return;
     const int32_t p = perm[s];
     sorted_pts[s] = make_float4(pts[3 * (int64_t)p], pts[3 * (int64_t)p + 1], pts[3 * (int64_t)p + 2], __int_as_float(p));
+    if (sample) sorted_sample[s] = sample[p];
     const uint32_t key = keys[s];
     if (s == 0 || keys[s - 1] != key) table[key].x = (int)s;
     if (s + 1 == P || keys[s + 1] != key) table[key].y = (int)(s + 1);
@@ -128,9 +140,11 @@ struct TapArgs {
     const int32_t *query_sample, *point_sample;
     const float4 *sorted_pts;
     const int2 *table;
-    uint4 *lanes;
-    unsigned long long *lanes_more;
-    uint32_t *lane_counts, *block_hist;
+    const int32_t *sorted_sample;   // null: no sample ids
+    int32_t *kept_point;
+    uint8_t *kept_tap;
+    int kept;
+    uint32_t *counts, *block_hist;
     int64_t *num_neighbors;
     const int64_t *seg, *ctrl;
     int64_t *ctrl_rw;
@@ -156,85 +170,120 @@ __device__ __forceinline__ bool accept_fast(const TapArgs &a, float qx, float qy
     return radius_accept(qx, qy, qz, p, a.r32, a.distance_type, a.variant, &d);
 }
 
-// Walks the run [r.x, r.y) of sorted points for query (qx, qy, qz) of sample b, 64 candidates at a
-// time: first the predicate alone over the chunk (two loads in flight, no divergent work), giving
-// a 64-bit mask, then hit(tap, j) for the set bits in run order.  The mask of the first chunk is
-// stored by the count pass (after the sample check) and read back by the fill pass, which then
-// touches accepted points only; later chunks of a long run are evaluated again.  `masks` holds the
-// masks of the first two chunks (128 candidates), which covers the runs of dense scenes.
-template <bool STORED, typename Hit>
-__device__ __forceinline__ void walk_run(const TapArgs &a, int2 r, float qx, float qy, float qz, int b,
-                                         unsigned long long (&masks)[2], Hit hit) {
-    for (int s0 = r.x; s0 < r.y; s0 += 64) {
-        const int chunk = (s0 - r.x) >> 6;
-        const bool first = chunk < 2;   // a chunk whose mask is kept
-        const int len = min(64, r.y - s0);
-        unsigned long long m = 0;
-        if (STORED && first) {
-            m = masks[chunk & 1];
-        } else {
-            uint32_t half[2] = {0u, 0u};
+// The eight candidate runs of a query as one list: lane c of the query's eight holds run c.
+struct Runs {
+    int first;   // start of this lane's run minus the candidates before it
+    int upto;    // candidates up to and including this lane's run
+    int total;   // candidates of the query
+    __device__ __forceinline__ Runs(int2 run, int c) {   // (start, length)
+        upto = run.y;
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int n = min(32, len - 32 * h);   // candidates of this half (may be <= 0)
-                const float4 *src = a.sorted_pts + s0 + 32 * h;
-                for (int t = 0; t < n; t += 4) {       // four loads in flight; the tail repeats the last point
-                    float4 p[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) p[u] = src[min(t + u, n - 1)];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-                        if (t + u < n && accept_fast(a, qx, qy, qz, p[u])) half[h] |= 1u << (t + u);
-                }
-            }
-            m = (unsigned long long)half[0] | ((unsigned long long)half[1] << 32);
+        for (int o = 1; o < 8; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, upto, o, 8);
+            if (c >= o) upto += v;
         }
-        unsigned long long keep = m;
-        while (m) {
-            const int t = __ffsll((long long)m) - 1;
-            m &= m - 1;
-            const float4 p = a.sorted_pts[s0 + t];
-            const int j = __float_as_int(p.w);
-            if (!(STORED && first) && a.point_sample && a.point_sample[j] != b) {   // a foreign cell sharing the bucket
-                keep &= ~(1ULL << t);
-                continue;
-            }
-            hit(tap_of_fast(qx, qy, qz, p, a.g32, a.inv_g, a.K), j);
+        first = run.x - (upto - run.y);
+        total = __shfl_sync(0xffffffffu, upto, 7, 8);
+    }
+    __device__ __forceinline__ int at(int p) const {   // sorted position of candidate p < total
+        int o = 0;
+        if (p >= __shfl_sync(0xffffffffu, upto, 3, 8)) o = 4;
+        if (p >= __shfl_sync(0xffffffffu, upto, o + 1, 8)) o += 2;
+        if (p >= __shfl_sync(0xffffffffu, upto, o, 8)) o += 1;
+        return __shfl_sync(0xffffffffu, first, o, 8) + p;
+    }
+};
+
+// Candidate run of cell c (0 .. 7) of a query: (start, length).
+__device__ __forceinline__ int2 run_of(const TapArgs &a, float qx, float qy, float qz, int b, int c) {
+    const int cx = corner_of(qx, a.r32, a.inv) + ((c >> 2) & 1);
+    const int cy = corner_of(qy, a.r32, a.inv) + ((c >> 1) & 1);
+    const int cz = corner_of(qz, a.r32, a.inv) + (c & 1);
+    const int2 r = a.table[cell_bucket(b, cx, cy, cz, a.mask)];
+    return make_int2(r.x, r.y - r.x);
+}
+
+constexpr int DEPTH = 4;   // candidates a lane looks at together
+
+// Walks the candidates of the warp's four queries: hit(accept bits of this query's eight lanes, this lane's
+// candidate accepted, its sorted position, its point) once per eight candidates, in list order.
+template <typename Hit>
+__device__ __forceinline__ void walk(const TapArgs &a, const Runs &runs, float qx, float qy, float qz, int b, int c, int lane, Hit hit) {
+    const int rounds = (__reduce_max_sync(0xffffffffu, runs.total) + 7) >> 3;
+    for (int r = 0; r < rounds; r += DEPTH) {
+        int pos[DEPTH], smp[DEPTH];
+        float4 pt[DEPTH];
+#pragma unroll
+        for (int u = 0; u < DEPTH; ++u) {
+            const int p = (r + u) * 8 + c, s = runs.at(min(p, max(runs.total - 1, 0)));
+            pos[u] = p < runs.total ? s : -1;
         }
-        if (!STORED && first) masks[chunk & 1] = keep;
+#pragma unroll
+        for (int u = 0; u < DEPTH; ++u) {   // a foreign cell may share the bucket: its sample differs, or the distance does
+            pt[u] = pos[u] >= 0 ? a.sorted_pts[pos[u]] : make_float4(0.f, 0.f, 0.f, 0.f);
+            smp[u] = a.sorted_sample && pos[u] >= 0 ? a.sorted_sample[pos[u]] : b;
+        }
+#pragma unroll
+        for (int u = 0; u < DEPTH; ++u) {
+            const bool ok = pos[u] >= 0 && accept_fast(a, qx, qy, qz, pt[u]) && smp[u] == b;
+            const uint32_t all = __ballot_sync(0xffffffffu, ok);
+            if (all) hit(all, ok, pt[u]);
+        }
     }
 }
 
 __global__ void __launch_bounds__(THREADS) taps_count_kernel(TapArgs a) {
     __shared__ uint32_t s_hist[MAX_K3];
+    __shared__ float4 s_queue[THREADS / 32][64];     // accepted points whose tap is still to be computed ...
+    __shared__ uint32_t s_whose[THREADS / 32][64];   // ... and their query in the warp and place in its list
     if (threadIdx.x < MAX_K3) s_hist[threadIdx.x] = 0;
     __syncthreads();
-    const int c = threadIdx.x & 7;
-    const int64_t q = (int64_t)blockIdx.x * QPB + (threadIdx.x >> 3);
-    uint32_t n = 0;
+    const int c = threadIdx.x & 7, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t q0 = (int64_t)blockIdx.x * QPB + warp * 4, q = q0 + (lane >> 3);
+    float qx = 0.f, qy = 0.f, qz = 0.f;
+    int b = 0;
+    int2 run = make_int2(0, 0);
     if (q < a.Q) {
-        const float qx = a.queries[3 * q], qy = a.queries[3 * q + 1], qz = a.queries[3 * q + 2];
-        const int b = a.query_sample ? a.query_sample[q] : 0;
-        const int cx = corner_of(qx, a.r32, a.inv) + ((c >> 2) & 1);
-        const int cy = corner_of(qy, a.r32, a.inv) + ((c >> 1) & 1);
-        const int cz = corner_of(qz, a.r32, a.inv) + (c & 1);
-        const int2 r = a.table[cell_bucket(b, cx, cy, cz, a.mask)];
-        unsigned long long masks[2] = {0ULL, 0ULL};
-        walk_run<false>(a, r, qx, qy, qz, b, masks, [&](int tap, int) {
-            ++n;
-            atomicAdd(&s_hist[tap], 1u);
-        });
-        a.lanes[q * 8 + c] = make_uint4((uint32_t)r.x, (uint32_t)r.y, (uint32_t)masks[0], (uint32_t)(masks[0] >> 32));
-        if (r.y - r.x > 64) a.lanes_more[q * 8 + c] = masks[1];
-        a.lane_counts[q * 8 + c] = n;
+        qx = a.queries[3 * q], qy = a.queries[3 * q + 1], qz = a.queries[3 * q + 2];
+        b = a.query_sample ? a.query_sample[q] : 0;
+        run = run_of(a, qx, qy, qz, b, c);
     }
-    uint32_t tot = n;
-    tot += __shfl_xor_sync(0xffffffffu, tot, 1);
-    tot += __shfl_xor_sync(0xffffffffu, tot, 2);
-    tot += __shfl_xor_sync(0xffffffffu, tot, 4);
+    const Runs runs(run, c);
+    uint32_t n = 0;
+    int head = 0, queued = 0;
+    auto taps_of_queued = [&](int count) {
+        __syncwarp();
+        const float4 p = s_queue[warp][(head + lane) & 63];
+        const uint32_t e = s_whose[warp][(head + lane) & 63];
+        const int from = lane < count ? (int)(e & 3u) * 8 : 0;
+        const float x = __shfl_sync(0xffffffffu, qx, from), y = __shfl_sync(0xffffffffu, qy, from), z = __shfl_sync(0xffffffffu, qz, from);
+        if (lane < count) {
+            const int tap = tap_of_fast(x, y, z, p, a.g32, a.inv_g, a.K);
+            atomicAdd(&s_hist[tap], 1u);
+            if ((int)(e >> 2) < a.kept) {
+                const int64_t at = (q0 + (e & 3u)) * a.kept + (e >> 2);
+                a.kept_point[at] = __float_as_int(p.w), a.kept_tap[at] = (uint8_t)tap;
+            }
+        }
+        head += count, queued -= count;
+        __syncwarp();
+    };
+    walk(a, runs, qx, qy, qz, b, c, lane, [&](uint32_t all, bool ok, const float4 &p) {
+        const uint32_t mine = (all >> (lane & 24)) & 0xffu;
+        if (ok) {
+            const int slot = (head + queued + __popc(all & ((1u << lane) - 1u))) & 63;
+            s_queue[warp][slot] = p;
+            s_whose[warp][slot] = (uint32_t)(lane >> 3) | ((n + __popc(mine & ((1u << c) - 1u))) << 2);
+        }
+        n += __popc(mine);
+        queued += __popc(all);
+        if (queued >= 32) taps_of_queued(32);
+    });
+    if (queued) taps_of_queued(queued);
     if (q < a.Q && c == 0) {
-        a.num_neighbors[q] = tot;
-        if (tot == 0) atomicAdd((unsigned long long *)&a.ctrl_rw[3], 1ULL);
+        a.counts[q] = n;
+        a.num_neighbors[q] = n;
+        if (n == 0) atomicAdd((unsigned long long *)&a.ctrl_rw[3], 1ULL);
     }
     __syncthreads();
     if ((int)threadIdx.x < a.k3) a.block_hist[(int64_t)threadIdx.x * a.nblocks + blockIdx.x] = s_hist[threadIdx.x];
@@ -295,7 +344,7 @@ __global__ void __launch_bounds__(THREADS) taps_fill_kernel(TapArgs a) {
     using Scan = cub::BlockScan<uint32_t, THREADS>;
     const int kpad = (a.k3 + 31) & ~31;
     __shared__ typename Scan::TempStorage tmp;
-    __shared__ unsigned long long s_rec[REC_MAX];   // tap << 40 | local query << 32 | point index, in output order
+    __shared__ unsigned long long s_rec[REC_MAX];   // accepted pairs in output order
     extern __shared__ uint16_t s_gcnt[];            // [GROUPS][kpad] per 32 records and tap: count, then prefix inside the round
     __shared__ uint32_t s_base[MAX_K3];             // next write position of each tap for this block
     __shared__ uint32_t s_round[MAX_K3];
@@ -305,32 +354,41 @@ __global__ void __launch_bounds__(THREADS) taps_fill_kernel(TapArgs a) {
     const int64_t q0 = (int64_t)blockIdx.x * QPB, q = q0 + ql;
     if ((int)threadIdx.x < a.k3)
         s_base[threadIdx.x] = (uint32_t)a.seg[threadIdx.x] + a.block_hist[(int64_t)threadIdx.x * a.nblocks + blockIdx.x];
-    const uint32_t n = q < a.Q ? a.lane_counts[q * 8 + c] : 0u;
-    uint32_t my_off, block_total;
-    Scan(tmp).ExclusiveSum(n, my_off, block_total);
-    float qx = 0.f, qy = 0.f, qz = 0.f;
-    int b = 0;
-    int2 r = make_int2(0, 0);
-    unsigned long long masks[2] = {0ULL, 0ULL};
-    if (n) {
-        qx = a.queries[3 * q], qy = a.queries[3 * q + 1], qz = a.queries[3 * q + 2];
-        b = a.query_sample ? a.query_sample[q] : 0;
-        const uint4 l = a.lanes[q * 8 + c];
-        r = make_int2((int)l.x, (int)l.y);
-        masks[0] = (unsigned long long)l.z | ((unsigned long long)l.w << 32);
-        if (r.y - r.x > 64) masks[1] = a.lanes_more[q * 8 + c];
-    }
+    const uint32_t nq = q < a.Q ? a.counts[q] : 0u;
+    uint32_t q_off, block_total;
+    Scan(tmp).ExclusiveSum(c == 0 ? nq : 0u, q_off, block_total);
+    q_off = __shfl_sync(0xffffffffu, q_off, 0, 8);
+    const bool kept = __all_sync(0xffffffffu, nq <= (uint32_t)a.kept);   // all accepted points of the warp's queries were kept
     __syncthreads();
     for (uint32_t lo = 0; lo < block_total; lo += REC_MAX) {
         const uint32_t hi = lo + REC_MAX;
         const int cnt = (int)min((uint32_t)REC_MAX, block_total - lo), groups = (cnt + 31) >> 5;
         for (int t = threadIdx.x; t < groups * kpad; t += THREADS) s_gcnt[t] = 0;
-        if (n && my_off < hi && my_off + n > lo) {
-            uint32_t pos = my_off;
-            walk_run<true>(a, r, qx, qy, qz, b, masks, [&](int tap, int j) {
+        // tap << 40 | local query << 32 | point index, in output order
+        if (kept) {
+            for (uint32_t e = c; e < nq; e += 8) {
+                const uint32_t pos = q_off + e;
                 if (pos >= lo && pos < hi)
-                    s_rec[pos - lo] = ((unsigned long long)tap << 40) | ((unsigned long long)ql << 32) | (uint32_t)j;
-                ++pos;
+                    s_rec[pos - lo] = ((unsigned long long)a.kept_tap[q * a.kept + e] << 40) | ((unsigned long long)ql << 32) |
+                                      (uint32_t)a.kept_point[q * a.kept + e];
+            }
+        } else {
+            float qx = 0.f, qy = 0.f, qz = 0.f;
+            int b = 0;
+            int2 run = make_int2(0, 0);
+            if (nq) {
+                qx = a.queries[3 * q], qy = a.queries[3 * q + 1], qz = a.queries[3 * q + 2];
+                b = a.query_sample ? a.query_sample[q] : 0;
+                run = run_of(a, qx, qy, qz, b, c);
+            }
+            const Runs runs(run, c);
+            uint32_t at = q_off;
+            walk(a, runs, qx, qy, qz, b, c, lane, [&](uint32_t all, bool ok, const float4 &p) {
+                const uint32_t mine = (all >> (lane & 24)) & 0xffu, pos = at + __popc(mine & ((1u << c) - 1u));
+                if (ok && pos >= lo && pos < hi)
+                    s_rec[pos - lo] = ((unsigned long long)tap_of_fast(qx, qy, qz, p, a.g32, a.inv_g, a.K) << 40) |
+                                      ((unsigned long long)ql << 32) | (uint32_t)__float_as_int(p.w);
+                at += __popc(mine);
             });
         }
         __syncthreads();
@@ -387,8 +445,9 @@ TapArgs make_args(const TapsWs &w, const float *queries, const int32_t *point_sa
                   int64_t Q, double radius, int distance_type, int kernel_size, double grid) {
     TapArgs a = {};
     a.queries = queries, a.query_sample = query_sample, a.point_sample = point_sample;
-    a.sorted_pts = w.sorted_pts, a.table = w.table, a.lanes = w.lanes, a.lanes_more = w.lanes_more;
-    a.lane_counts = w.lane_counts, a.block_hist = w.block_hist, a.seg = w.seg, a.ctrl = w.ctrl, a.ctrl_rw = w.ctrl;
+    a.sorted_pts = w.sorted_pts, a.table = w.table, a.kept_point = w.kept_point, a.kept_tap = w.kept_tap;
+    a.sorted_sample = point_sample ? w.sorted_sample : nullptr, a.kept = kept_per_query(kernel_size * kernel_size * kernel_size);
+    a.counts = w.counts, a.block_hist = w.block_hist, a.seg = w.seg, a.ctrl = w.ctrl, a.ctrl_rw = w.ctrl;
     a.Q = Q, a.nblocks = w.nblocks, a.mask = (uint32_t)(w.buckets - 1);
     a.r32 = (float)radius, a.inv = (float)(1.0 / (2.0 * radius)), a.g32 = (float)grid;
     a.inv_g = 1.0f / a.g32;
@@ -444,7 +503,7 @@ int pcx_radius_taps_count(const float *d_points, const float *d_queries, const i
     PCX_LAUNCH_CHECK();
     size_t tmp = w.cub_bytes;
     PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, tmp, w.keys_a, w.keys_b, w.vals_a, w.vals_b, P, 0, w.bits, stream));
-    taps_table_kernel<<<pblocks, 256, 0, stream>>>(d_points, w.keys_b, w.vals_b, P, w.sorted_pts, w.table);
+    taps_table_kernel<<<pblocks, 256, 0, stream>>>(d_points, d_point_sample, w.keys_b, w.vals_b, P, w.sorted_pts, w.sorted_sample, w.table);
     PCX_LAUNCH_CHECK();
     TapArgs a = make_args(w, d_queries, d_point_sample, d_query_sample, Q, radius, distance_type, kernel_size, kernel_grid_size);
     a.num_neighbors = d_num_neighbors;
