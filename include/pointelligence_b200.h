@@ -502,6 +502,14 @@ size_t pcx_grid_sample_workspace_bytes(int64_t N);
 int pcx_grid_sample_count(const float *d_points, const int32_t *d_sample,
                           int64_t N, double cell, int64_t *h_num_cells,
                           void *d_ws, size_t ws_bytes, void *stream);
+/* ... with h_info[3] = cells, smallest and largest sample id. */
+int pcx_grid_sample_count_samples(const float *d_points,
+                                  const int32_t *d_sample, int64_t N,
+                                  double cell, int64_t *h_info, void *d_ws,
+                                  size_t ws_bytes, void *stream);
+/* sizes[s] = how often s occurs in a non-decreasing list of ids (S of them). */
+int pcx_sample_sizes(const int32_t *d_sorted, int64_t N, int64_t S,
+                     int64_t *d_sizes, void *stream);
 int pcx_grid_sample_select(const float *d_points, const int32_t *d_sample,
                            int64_t N, double cell, int64_t num_cells,
                            int64_t *d_indices, float *d_out_points,

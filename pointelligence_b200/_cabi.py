@@ -114,6 +114,9 @@ SIGNATURES = {
     "pcx_grid_sample_workspace_bytes": (c_size_t, [c_int64]),
     "pcx_grid_sample_count": (c_int, [c_void_p, c_void_p, c_int64, c_double, c_void_p, c_void_p, c_size_t,
                                       c_void_p]),
+    "pcx_grid_sample_count_samples": (c_int, [c_void_p, c_void_p, c_int64, c_double, ctypes.POINTER(c_int64), c_void_p,
+                                              c_size_t, c_void_p]),
+    "pcx_sample_sizes": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p]),
     "pcx_grid_sample_select": (c_int, [c_void_p, c_void_p, c_int64, c_double, c_int64] + [c_void_p] * 4
                                + [c_void_p, c_size_t, c_void_p]),
 }
@@ -198,15 +201,6 @@ _SIDE_STREAMS = {}
 _overlap = threading.local()
 
 
-def _side_stream(device):
-    """The high-priority stream geometry runs on inside a ``geometry_overlap`` scope, else None."""
-    active = getattr(_overlap, "devices", None)
-    index = device.index if device.index is not None else torch.cuda.current_device()
-    if not active or index not in active:
-        return None
-    return _SIDE_STREAMS[index]
-
-
 class geometry_overlap:
     """Scope in which the index-building calls of this module (radius search, grid sampling, plan
     building) run on a stream of their own, so that their host hand-overs wait for the geometry
@@ -230,6 +224,8 @@ class geometry_overlap:
         active = getattr(_overlap, "devices", None)
         if active is None:
             active = _overlap.devices = set()
+            _overlap.inside = False
+            _overlap.known = {}
         if index in active:
             return self
         if index not in _SIDE_STREAMS:
@@ -242,6 +238,7 @@ class geometry_overlap:
     def __exit__(self, *exc):
         if self.owner:
             _overlap.devices.discard(self.index)
+            _overlap.known.clear()
             torch.cuda.current_stream(self.index).wait_stream(_SIDE_STREAMS[self.index])
             self.owner = False
         return False
@@ -263,33 +260,40 @@ def on_geometry_stream(fn):
                 return v.points.device
         return None
 
-    def hand_over(value, main, depth=0):
+    def collect(value, out, depth=0):
         if isinstance(value, torch.Tensor):
-            if value.is_cuda:
-                value.record_stream(main)
+            if id(value) not in _overlap.known:      # kept until the scope ends, so that ids stay unique
+                _overlap.known[id(value)] = value
+                out.append(value)
         elif isinstance(value, (tuple, list)):
             for v in value:
-                hand_over(v, main, depth)
+                collect(v, out, depth)
         elif isinstance(value, MvmrPlan):
-            value.buffer.record_stream(main)
+            out.append(value.buffer)
         elif hasattr(value, "__dataclass_fields__") and depth < 8:
             for v in vars(value).values():
-                if isinstance(v, (torch.Tensor, tuple, list)) or hasattr(v, "__dataclass_fields__"):
-                    hand_over(v, main, depth + 1)
+                if v is not None and not isinstance(v, (bool, int, float, str)):
+                    collect(v, out, depth + 1)
 
     @functools.wraps(fn)
     def wrapper(*args, **kwargs):
+        active = getattr(_overlap, "devices", None)
+        if not active or _overlap.inside:            # no scope, or already on the geometry stream
+            return fn(*args, **kwargs)
         dev = device_of(list(args) + list(kwargs.values()))
-        side = _side_stream(dev) if dev is not None else None
-        if side is None:
+        if dev is None or dev.index not in active:
             return fn(*args, **kwargs)
-        main = torch.cuda.current_stream(dev)
-        if main == side:
-            return fn(*args, **kwargs)
-        with torch.cuda.stream(side):
+        side = _SIDE_STREAMS[dev.index]
+        before = host().side_begin(side.stream_id, side.device_index, side.device_type)
+        _overlap.inside = True
+        try:
             out = fn(*args, **kwargs)
-        main.wait_stream(side)
-        hand_over(out, main)
+        finally:
+            _overlap.inside = False
+            host().side_end(*before)
+        fresh = []
+        collect(out, fresh)
+        host().record_streams(fresh)
         return out
 
     return wrapper
@@ -860,4 +864,7 @@ def _radius_taps(points, queries, radius, ps, qs, distance_type, kernel_size, ke
 def grid_sample_center_nearest(points, cell, sample, return_mapping):
     """Returns ``(indices int64 (S,), points_f (S,3), sample_f int32 (S,)|None, mapping int64|None)``."""
     require_cuda(points, sample)
-    return host().grid_sample(points, float(cell), sample, bool(return_mapping))
+    indices, out, out_sample, mapping, sizes = host().grid_sample(points, float(cell), sample, bool(return_mapping))
+    if sizes is not None:
+        out_sample.pcx_sample_sizes = sizes     # spares the caller a histogram and its hand-over
+    return indices, out, out_sample, mapping

@@ -15,6 +15,9 @@ namespace pcx {
 
 void set_error(const char *fmt, ...);
 extern std::atomic<long long> g_launches;               // kernels launched by this library
+// Where a host hand-over (an asynchronous copy and a wait for the stream, in one call) puts its words.
+constexpr int HANDOVER_WORDS = 16;
+int64_t *handover_words();
 void prof_begin(const char *name, cudaStream_t stream); // event timer around a dominant kernel
 void prof_end(cudaStream_t stream);
 

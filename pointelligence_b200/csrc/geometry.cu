@@ -489,6 +489,42 @@ __global__ void grid_select_kernel(const float *__restrict__ pts, const int32_t 
     if (out_sample) out_sample[seg] = sample ? sample[best_idx] : 0;
 }
 
+// sizes[s] = elements of a non-decreasing id list that equal s
+__global__ void sample_sizes_kernel(const int32_t *__restrict__ sorted, int64_t N, int64_t S, int64_t *sizes) {
+    const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (s >= S) return;
+    int64_t bound[2];
+    for (int e = 0; e < 2; ++e) {   // first position with a value >= s + e
+        int64_t lo = 0, hi = N;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (sorted[mid] < s + e) lo = mid + 1; else hi = mid;
+        }
+        bound[e] = lo;
+    }
+    sizes[s] = bound[1] - bound[0];
+}
+
+// Bits of the largest cell key of a cloud with these extents (min[4], max[4]); 64 where the key space is larger.
+int key_bits_for(const int32_t *ext) {
+    uint64_t span = 1;
+    for (int a = 0; a < 4; ++a) {
+        const int64_t e = (int64_t)ext[4 + a] - ext[a] + 1;
+        if (e <= 0 || __builtin_mul_overflow(span, (uint64_t)e, &span)) return 64;
+    }
+    int bits = 1;
+    while (bits < 64 && ((span - 1) >> bits)) ++bits;
+    return bits;
+}
+
+// (cell size's bit pattern << 32 | key bits) of the last cloud that was binned at about this cell size
+std::atomic<uint64_t> &key_bits_of(float cell) {
+    static std::atomic<uint64_t> table[64];
+    uint32_t u;
+    memcpy(&u, &cell, sizeof(u));
+    return table[(u * 2654435761u) >> 26];
+}
+
 int bits_for(int64_t n) {
     int b = 1;
     while (((int64_t)1 << b) < n) ++b;
@@ -700,10 +736,19 @@ size_t pcx_grid_sample_workspace_bytes(int64_t N) {
     return carve_grid(nullptr, N, nullptr);
 }
 
-int pcx_grid_sample_count(const float *d_points, const int32_t *d_sample, int64_t N, double cell,
-                          int64_t *h_num_cells, void *d_ws, size_t ws_bytes, void *stream_) {
+int pcx_grid_sample_count(const float *d_points, const int32_t *d_sample, int64_t N, double cell, int64_t *h_num_cells, void *d_ws,
+                          size_t ws_bytes, void *stream) {
+    if (!h_num_cells) PCX_FAIL(PCX_E_ARG, "pcx_grid_sample_count: bad arguments");
+    int64_t info[3];
+    if (int rc = pcx_grid_sample_count_samples(d_points, d_sample, N, cell, info, d_ws, ws_bytes, stream)) return rc;
+    *h_num_cells = info[0];
+    return PCX_OK;
+}
+
+int pcx_grid_sample_count_samples(const float *d_points, const int32_t *d_sample, int64_t N, double cell, int64_t *h_info, void *d_ws,
+                                  size_t ws_bytes, void *stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
-    if (N <= 0 || !d_points || !h_num_cells || !d_ws) PCX_FAIL(PCX_E_ARG, "pcx_grid_sample_count: bad arguments");
+    if (N <= 0 || !d_points || !h_info || !d_ws) PCX_FAIL(PCX_E_ARG, "pcx_grid_sample_count: bad arguments");
     if (N > INT32_MAX) PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_grid_sample_count: more than 2^31-1 points");
     if (!(cell > 0)) PCX_FAIL(PCX_E_ARG, "grid_size must be positive; got %g", cell);
     GridWs w;
@@ -719,34 +764,46 @@ int pcx_grid_sample_count(const float *d_points, const int32_t *d_sample, int64_
     unsigned nb = (unsigned)((N + 255) / 256);
     grid_key_kernel<<<nb, 256, 0, stream>>>(d_points, d_sample, N, c32, w.ext, w.keys_a, w.vals_a);
     PCX_LAUNCH_CHECK();
-    // The sort only has to look at the bits the largest key can use: the extents come to the host
-    // (32 bytes; the call ends with a hand-over of the cell count anyway).
-    int32_t h_ext[8];
-    PCX_CUDA(cudaMemcpyAsync(h_ext, w.ext, sizeof(h_ext), cudaMemcpyDeviceToHost, stream));
-    PCX_CUDA(cudaStreamSynchronize(stream));
-    int key_bits = 64;
-    {
-        uint64_t span = 1;
-        bool fits = true;
-        for (int a = 0; a < 4 && fits; ++a) {
-            const int64_t e = (int64_t)h_ext[4 + a] - h_ext[a] + 1;
-            fits = e > 0 && !__builtin_mul_overflow(span, (uint64_t)e, &span);
-        }
-        if (fits) {
-            key_bits = 1;
-            while (key_bits < 64 && ((span - 1) >> key_bits)) ++key_bits;
-        }
+    // The sort only has to look at the bits the largest key can use.  How many those are is known from the extents,
+    // which come to the host with the cell count; the sort is enqueued for the bits that the last cloud of this
+    // cell size needed, and repeated where this one needs more (a first call asks for the extents beforehand).
+    int32_t *h = reinterpret_cast<int32_t *>(handover_words());   // extents, then the number of cells
+    auto extents = [&]() -> int {
+        PCX_CUDA(cudaMemcpyAsync(h, w.ext, 8 * sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+        PCX_CUDA(cudaStreamSynchronize(stream));
+        return PCX_OK;
+    };
+    std::atomic<uint64_t> &known = key_bits_of(c32);
+    uint32_t cell_bits;
+    memcpy(&cell_bits, &c32, sizeof(cell_bits));
+    uint64_t seen = known.load();
+    if ((seen >> 32) != cell_bits || (seen & 0xff) == 0) {
+        if (int rc = extents()) return rc;
+        seen = ((uint64_t)cell_bits << 32) | (uint64_t)key_bits_for(h);
     }
-    size_t tmp = w.cub_bytes;
-    PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, tmp, w.keys_a, w.keys_b, w.vals_a, w.vals_b, N, 0, key_bits, stream));
-    grid_flag_kernel<<<nb, 256, 0, stream>>>(w.keys_b, N, w.flags);
+    int used = (int)(seen & 0xff);
+    for (;;) {
+        size_t tmp = w.cub_bytes;
+        PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, tmp, w.keys_a, w.keys_b, w.vals_a, w.vals_b, N, 0, used, stream));
+        grid_flag_kernel<<<nb, 256, 0, stream>>>(w.keys_b, N, w.flags);
+        PCX_LAUNCH_CHECK();
+        tmp = w.cub_bytes;
+        PCX_CUDA(cub::DeviceScan::InclusiveSum(w.cub_tmp, tmp, w.flags, w.ordinal, N, stream));
+        PCX_CUDA(cudaMemcpyAsync(h + 8, w.ordinal + (N - 1), sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+        if (int rc = extents()) return rc;
+        const int need = key_bits_for(h);
+        known.store(((uint64_t)cell_bits << 32) | (uint64_t)need);
+        if (need <= used) break;
+        used = need;
+    }
+    h_info[0] = h[8], h_info[1] = h[3], h_info[2] = h[7];
+    return PCX_OK;
+}
+
+int pcx_sample_sizes(const int32_t *d_sorted, int64_t N, int64_t S, int64_t *d_sizes, void *stream_) {
+    if (N < 0 || S <= 0 || (N > 0 && !d_sorted) || !d_sizes) PCX_FAIL(PCX_E_ARG, "pcx_sample_sizes: bad arguments");
+    sample_sizes_kernel<<<(unsigned)((S + 127) / 128), 128, 0, (cudaStream_t)stream_>>>(d_sorted, N, S, d_sizes);
     PCX_LAUNCH_CHECK();
-    tmp = w.cub_bytes;
-    PCX_CUDA(cub::DeviceScan::InclusiveSum(w.cub_tmp, tmp, w.flags, w.ordinal, N, stream));
-    int32_t last = 0;
-    PCX_CUDA(cudaMemcpyAsync(&last, w.ordinal + (N - 1), sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-    PCX_CUDA(cudaStreamSynchronize(stream));
-    *h_num_cells = last;
     return PCX_OK;
 }
 

@@ -12,6 +12,7 @@
 #include <torch/extension.h>
 
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
 
 #include "../../include/pointelligence_b200.h"
@@ -465,8 +466,9 @@ std::tuple<Tensor, Tensor, OptTensor, Tensor, Tensor, int64_t, int64_t, int64_t>
             total[2]};
 }
 
-// (indices, points, sample | undefined, mapping | undefined) of the centre-nearest point of every occupied cell
-std::tuple<Tensor, Tensor, OptTensor, OptTensor> grid_sample(const Tensor &points_, double cell, const OptTensor &sample_,
+// (indices, points, sample | undefined, mapping | undefined, points per sample | undefined) of the centre-nearest
+// point of every occupied cell
+std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor> grid_sample(const Tensor &points_, double cell, const OptTensor &sample_,
                                                              bool want_mapping) {
     require_cuda(points_), require_cuda(sample_);
     c10::cuda::CUDAGuard guard(points_.device());
@@ -474,15 +476,21 @@ std::tuple<Tensor, Tensor, OptTensor, OptTensor> grid_sample(const Tensor &point
     const int64_t N = points.size(0);
     const auto i64 = at::TensorOptions().dtype(at::kLong).device(points.device());
     Tensor ws = workspace(pcx_grid_sample_workspace_bytes(N), points);
-    int64_t cells = 0;
-    check(pcx_grid_sample_count(ptr_as<float>(points), ptr_as<int32_t>(sample), N, cell, &cells, ptr(ws), ws.numel(), stream()));
+    int64_t info[3] = {0, 0, 0};
+    check(pcx_grid_sample_count_samples(ptr_as<float>(points), ptr_as<int32_t>(sample), N, cell, info, ptr(ws), ws.numel(), stream()));
+    const int64_t cells = info[0];
     Tensor indices = at::empty({cells}, i64), out = at::empty({cells, 3}, i64.dtype(at::kFloat));
     Tensor out_sample = sample_ ? at::empty({cells}, i64.dtype(at::kInt)) : Tensor();
     Tensor mapping = want_mapping ? at::empty({N}, i64) : Tensor();
     check(pcx_grid_sample_select(ptr_as<float>(points), ptr_as<int32_t>(sample), N, cell, cells, ptr_as<int64_t>(indices),
                                  ptr_as<float>(out), ptr_as<int32_t>(out_sample), ptr_as<int64_t>(mapping), ptr(ws), ws.numel(),
                                  stream()));
-    return {indices, out, sample_ ? OptTensor(out_sample) : std::nullopt, want_mapping ? OptTensor(mapping) : std::nullopt};
+    OptTensor sizes;
+    if (sample_ && info[1] >= 0) {   // cells come in ascending sample order
+        sizes = at::empty({info[2] + 1}, i64);
+        check(pcx_sample_sizes(ptr_as<int32_t>(out_sample), cells, info[2] + 1, ptr_as<int64_t>(*sizes), stream()));
+    }
+    return {indices, out, sample_ ? OptTensor(out_sample) : std::nullopt, want_mapping ? OptTensor(mapping) : std::nullopt, sizes};
 }
 
 // (plan buffer, number of buckets with several triplets)
@@ -514,6 +522,26 @@ Tensor planned(const Tensor &weight, const Tensor &feat, const Tensor &buffer, i
     return mvmr_planned(weight.contiguous(), feat.contiguous(), plan, T, n_out, transpose ? 1 : 0, Tensor());
 }
 
+// Geometry on a stream of its own: from here on the calling thread's work on `device` goes to the given stream ...
+std::tuple<int64_t, int64_t, int64_t> side_begin(int64_t stream_id, int64_t device, int64_t type) {
+    const auto before = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).pack3();
+    c10::cuda::setCurrentCUDAStream(c10::cuda::CUDAStream::unpack3(stream_id, (c10::DeviceIndex)device, (c10::DeviceType)type));
+    return {before.stream_id, before.device_index, (int64_t)before.device_type};
+}
+// ... and back: the stream before waits for what was enqueued meanwhile.
+void side_end(int64_t stream_id, int64_t device, int64_t type) {
+    const auto before = c10::cuda::CUDAStream::unpack3(stream_id, (c10::DeviceIndex)device, (c10::DeviceType)type);
+    at::cuda::CUDAEvent event;
+    event.record(c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device));
+    event.block(before);
+    c10::cuda::setCurrentCUDAStream(before);
+}
+// The tensors are used on the calling thread's current stream from now on.
+void record_streams(const std::vector<Tensor> &tensors) {
+    for (const Tensor &t : tensors)
+        if (t.is_cuda()) t.record_stream(c10::cuda::getCurrentCUDAStream(t.device().index()).unwrap());
+}
+
 void set_hooks(py::object plan, py::object symmetric, py::object double_backward) {
     g_plan_hook = plan.release().ptr();
     g_symmetric_hook = symmetric.release().ptr();
@@ -524,6 +552,9 @@ void set_hooks(py::object plan, py::object symmetric, py::object double_backward
 
 PYBIND11_MODULE(_pcx_host, m) {
     m.def("set_hooks", &set_hooks);
+    m.def("side_begin", &side_begin);
+    m.def("side_end", &side_end);
+    m.def("record_streams", &record_streams);
     m.def("set_engine", [](int e) { g_engine = e; });
     m.def("mvmr", &mvmr);
     m.def("vvor", &vvor);

@@ -987,8 +987,8 @@ int pcx_mvmr_plan_build_counted(const int32_t *d_scatter, const int32_t *d_gathe
         PCX_LAUNCH_CHECK();
     }
     if (int rc = order_groups(pv, w, K, G, stream)) return rc;
-    uint32_t h[8] = {};
-    PCX_CUDA(cudaMemcpyAsync(h, pv.ctrl, sizeof(h), cudaMemcpyDeviceToHost, stream));
+    uint32_t *h = reinterpret_cast<uint32_t *>(handover_words());
+    PCX_CUDA(cudaMemcpyAsync(h, pv.ctrl, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
     PCX_CUDA(cudaStreamSynchronize(stream));
     *h_multi = h[CTRL_NMULTI];
     if (!h[CTRL_UNSORTED]) return PCX_OK;

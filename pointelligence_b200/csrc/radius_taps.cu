@@ -465,6 +465,17 @@ TapArgs make_args(const TapsWs &w, const float *queries, const int32_t *point_sa
     return a;
 }
 
+// ctrl[0 .. 3] and the device status word, in one wait
+int read_ctrl(const TapsWs &w, int64_t *h, cudaStream_t stream) {
+    unsigned int *d_status = nullptr;
+    if (int rc = device_status_address(&d_status)) return rc;
+    h[4] = 0;
+    PCX_CUDA(cudaMemcpyAsync(h, w.ctrl, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
+    PCX_CUDA(cudaMemcpyAsync(h + 4, d_status, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
+    PCX_CUDA(cudaStreamSynchronize(stream));
+    return PCX_OK;
+}
+
 }  // namespace
 }  // namespace pcx
 
@@ -522,13 +533,9 @@ int pcx_radius_taps_total(int64_t P, int64_t Q, int kernel_size, int64_t *h_tota
     if (!h_total || !d_ws || P <= 0 || Q <= 0 || !pcx_radius_taps_supported(kernel_size)) PCX_FAIL(PCX_E_ARG, "pcx_radius_taps_total: bad arguments");
     TapsWs w;
     if (ws_bytes < carve_taps(d_ws, P, Q, kernel_size * kernel_size * kernel_size, &w)) PCX_FAIL(PCX_E_CAPACITY, "pcx_radius_taps_total: workspace too small");
-    int64_t h[4] = {0, 0, 0, 0};
-    unsigned int status = 0, *d_status = nullptr;
-    if (int rc = device_status_address(&d_status)) return rc;
-    PCX_CUDA(cudaMemcpyAsync(h, w.ctrl, sizeof(h), cudaMemcpyDeviceToHost, stream));
-    PCX_CUDA(cudaMemcpyAsync(&status, d_status, sizeof(status), cudaMemcpyDeviceToHost, stream));
-    PCX_CUDA(cudaStreamSynchronize(stream));
-    h_total[0] = h[0], h_total[1] = h[3], h_total[2] = (int64_t)status;
+    int64_t *h = handover_words();
+    if (int rc = read_ctrl(w, h, stream)) return rc;
+    h_total[0] = h[0], h_total[1] = h[3], h_total[2] = h[4];
     if (h[1] || h[0] > INT32_MAX) PCX_FAIL(PCX_E_UNSUPPORTED, "prepared kernel-segment output currently requires fewer than 2^31 edges; got %lld", (long long)h[0]);
     return PCX_OK;
 }
@@ -554,13 +561,9 @@ int pcx_radius_taps_fill(const float *d_queries, const int32_t *d_point_sample, 
         prof_end(stream);
         PCX_LAUNCH_CHECK();
     }
-    int64_t h[4] = {0, 0, 0, 0};
-    unsigned int status = 0, *d_status = nullptr;
-    if (int rc = device_status_address(&d_status)) return rc;
-    PCX_CUDA(cudaMemcpyAsync(h, w.ctrl, sizeof(h), cudaMemcpyDeviceToHost, stream));
-    PCX_CUDA(cudaMemcpyAsync(&status, d_status, sizeof(status), cudaMemcpyDeviceToHost, stream));
-    PCX_CUDA(cudaStreamSynchronize(stream));
-    h_total[0] = h[0], h_total[1] = h[3], h_total[2] = (int64_t)status;
+    int64_t *h = handover_words();
+    if (int rc = read_ctrl(w, h, stream)) return rc;
+    h_total[0] = h[0], h_total[1] = h[3], h_total[2] = h[4];
     if (h[1] || h[0] > INT32_MAX) PCX_FAIL(PCX_E_UNSUPPORTED, "prepared kernel-segment output currently requires fewer than 2^31 edges; got %lld", (long long)h[0]);
     if (h[0] > capacity) PCX_FAIL(PCX_E_CAPACITY, "pcx_radius_taps_fill: %lld pairs do not fit the capacity of %lld; nothing was written", (long long)h[0], (long long)capacity);
     return PCX_OK;

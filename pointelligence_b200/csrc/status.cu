@@ -19,6 +19,25 @@ void set_error(const char *fmt, ...) {
 
 std::atomic<long long> g_launches{0};
 
+namespace {
+struct HandOver {   // page-locked, one per thread: copies into it neither stage nor block the stream
+    int64_t *words = nullptr;
+    int64_t pageable[HANDOVER_WORDS];
+    ~HandOver() {
+        if (words && words != pageable) cudaFreeHost(words);
+    }
+};
+}  // namespace
+
+int64_t *handover_words() {
+    static thread_local HandOver h;
+    if (!h.words && cudaHostAlloc((void **)&h.words, HANDOVER_WORDS * sizeof(int64_t), cudaHostAllocPortable) != cudaSuccess) {
+        (void)cudaGetLastError();
+        h.words = h.pageable;
+    }
+    return h.words;
+}
+
 struct ProfRecord {
     const char *name;
     cudaEvent_t start, stop;

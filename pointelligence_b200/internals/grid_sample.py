@@ -42,7 +42,12 @@ def grid_sample_filter(points, grid_size, sample_inds=None, reduction="center_ne
     need_map = return_mapping or reduction == "mean"
     indices, out_pts, out_smp, mapping = _cabi.grid_sample_center_nearest(
         pts32, float(grid_size), sample_inds, need_map)
-    sample_f = None if sample_inds is None else sample_inds[indices]
+    sample_f = None
+    if sample_inds is not None:
+        sample_f = out_smp.to(sample_inds.dtype)
+        sizes = getattr(out_smp, "pcx_sample_sizes", None)
+        if sizes is not None:
+            sample_f.pcx_sample_sizes = sizes
     if reduction in ("center_nearest", "random"):
         points_f = out_pts
     elif reduction == "center":

@@ -208,7 +208,7 @@ def handle_stride_and_build_triplets(m: MetaData, stride, kernel_size=_triple(3)
             neighbor_radius = parent.grid_size * radius_scaler
             m.points, m.sample_inds, m.grid_size, m.downsample_indices = downsample(
                 m.points, m.sample_inds, m.grid_size, stride)
-            m.sample_sizes = torch.bincount(m.sample_inds)
+            m.sample_sizes = _sizes_of(m.sample_inds)
             m.i, m.j, m.k, m.seg_offs, m.num_neighbors = _build_for(
                 parent.points, parent.sample_inds, parent.sample_sizes, neighbor_radius, kernel_size,
                 radius_scaler, sort_by, distance_type, return_num_neighbors,
@@ -222,6 +222,12 @@ def handle_stride_and_build_triplets(m: MetaData, stride, kernel_size=_triple(3)
                 sort_by, distance_type, return_num_neighbors)
     m.contract = TripletContract(k_sorted=(sort_by == "k"))
     return m
+
+
+def _sizes_of(sample_inds):
+    """Points per sample: counted by the grid sampler itself, or a histogram of the ids."""
+    sizes = getattr(sample_inds, "pcx_sample_sizes", None)
+    return torch.bincount(sample_inds) if sizes is None else sizes
 
 
 def _own_parent(m: MetaData) -> MetaData:
@@ -271,7 +277,7 @@ def handle_stride_disjoint_and_build_triplets(m: MetaData, stride, kernel_size=_
                                                                sample_inds=parent.sample_inds, reduction="center",
                                                                return_mapping=True)
         m.points, m.sample_inds, m.grid_size = centres.contiguous(), sample_c, cell_size
-        m.sample_sizes = torch.bincount(sample_c)
+        m.sample_sizes = _sizes_of(sample_c)
         m.downsample_indices = kept
         slot = partition_slots(pts, cell_size, K)
         point = torch.arange(pts.shape[0], device=pts.device)
