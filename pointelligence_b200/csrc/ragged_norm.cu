@@ -44,8 +44,13 @@ __global__ void ln_tail_kernel(int64_t *offsets, int64_t S, int64_t total) {
     if (threadIdx.x == 0 && blockIdx.x == 0) offsets[S] = total;
 }
 
-// Row offsets of a batch of a few samples in one small launch: one warp scans 32 lengths at a time.
-__global__ void ln_small_offsets_kernel(const int64_t *__restrict__ lengths, int64_t *offsets, int64_t S, int64_t total) {
+// Row offsets of a batch of a few samples, and zeros for what the backward pass accumulates into (up to three
+// arrays), in one small launch.
+__global__ void ln_small_offsets_kernel(const int64_t *__restrict__ lengths, int64_t *offsets, int64_t S, int64_t total, float *z0,
+                                        int64_t n0, float *z1, float *z2, int64_t n12) {
+    for (int64_t t = threadIdx.x; t < n0; t += blockDim.x) z0[t] = 0.f;
+    for (int64_t t = threadIdx.x; t < n12; t += blockDim.x) z1[t] = 0.f, z2[t] = 0.f;
+    if (threadIdx.x >= 32) return;
     const int lane = threadIdx.x;
     int64_t carry = 0;
     for (int64_t base = 0; base < S; base += 32) {
@@ -62,110 +67,100 @@ __global__ void ln_small_offsets_kernel(const int64_t *__restrict__ lengths, int
     if (lane == 0) offsets[S] = total;
 }
 
-// The kernels below share one shape: a block owns LN_ROWS consecutive rows, a thread
+// The kernels below share one shape: a block owns `rows` consecutive rows, a thread
 // keeps one vector column (VN channels, one 16-byte access when VN > 1) and walks the
-// rows of its row lane.  `uniform` blocks lie inside one sample (all but S - 1 of them).
+// rows of its row lane.  `uniform` blocks lie inside one sample.  The layer norm's kernels work
+// a block off in pieces that lie inside one sample each, unless it holds more than MAX_PIECES
+// samples (then every row looks its sample up); their blocks are sized for one wave of what is
+// resident (layer_rows): with blocks of 512 rows the sums pass spent a quarter of its time folding
+// blocks, and clouds of some thousand points kept a fraction of the chip busy.
+constexpr int MAX_PIECES = 8;
 struct BlockRows {
-    int64_t row0, row1, s_first;
+    int64_t row0, row1, s_first, s_last;
     bool uniform;
-    __device__ __forceinline__ BlockRows(const int64_t *__restrict__ offsets, int64_t N, int64_t S) {
-        row0 = (int64_t)blockIdx.x * LN_ROWS;
-        row1 = min(N, row0 + LN_ROWS);
+    __device__ __forceinline__ BlockRows(const int64_t *__restrict__ offsets, int64_t N, int64_t S, int rows = LN_ROWS) {
+        row0 = (int64_t)blockIdx.x * rows;
+        row1 = min(N, row0 + rows);
         s_first = segment_of_row(offsets, S, row0);
-        uniform = s_first == segment_of_row(offsets, S, row1 - 1);
+        s_last = segment_of_row(offsets, S, row1 - 1);
+        uniform = s_first == s_last;
     }
+    __device__ __forceinline__ bool in_pieces() const { return s_last - s_first < MAX_PIECES; }
 };
 
-// Statistics of the layer norm with ONE read of x from HBM.  A block first sums its rows (block
-// mean), then sums the squares centred on that mean while its rows are still in the caches, and
-// leaves (count, mean, M2) per (block, sample) piece; ln_combine_kernel merges the pieces of a
-// sample exactly (M2 = sum M2_p + n_p (mean_p - mean)^2), which keeps the accuracy of the
-// two-pass formula.  The piece of sample s in block b is record b + s (pieces are ordered, and
-// going to the next piece advances b or s by one), so a sample's pieces are consecutive records.
+// Statistics of the layer norm with ONE read of x from HBM.  A thread folds four rows of its column at a time:
+// their mean, their squares centred on it, and the exact merge of (count, mean, M2) into what it has; the
+// threads of a block merge the same way, and leave one record per (block, sample) piece, which
+// ln_combine_kernel merges again (M2 = sum M2_p + n_p (mean_p - mean)^2): the accuracy of the two-pass
+// formula, with no barrier while rows are read (sums and squares of a block in turn, each with a block-wide
+// reduction, read 1.1 M x 64 bf16 in 52 us).  The piece of sample s in block b is record b + s (pieces are
+// ordered, and going to the next piece advances b or s by one), so a sample's pieces are consecutive records.
 struct Moments { float n, mean, m2, pad; };
 
-template <typename T, int VN>
-__global__ void ln_moments_kernel(const T *__restrict__ x, const int64_t *__restrict__ offsets, Moments *rec,
-                                  int64_t N, int64_t S, int C) {
-    __shared__ float scratch[LN_THREADS / 32];
-    const BlockRows B(offsets, N, S);
-    const RowLayout L(C, VN);
-    const int64_t s_last = B.uniform ? B.s_first : segment_of_row(offsets, S, B.row1 - 1);
-    for (int64_t s = B.s_first; s <= s_last; ++s) {
-        const int64_t lo = max(B.row0, offsets[s]), hi = min(B.row1, offsets[s + 1]);
-        if (hi <= lo) continue;   // an empty sample inside the block (same decision in every thread)
-        float mu = 0.f;
-        float result[2];
-#pragma unroll
-        for (int pass = 0; pass < 2; ++pass) {
-            float acc = 0.f;
-            for (int cp = 0; cp * L.vcb < L.vc_total; ++cp) {
-                const int vcol = cp * L.vcb + L.vc;
-                if (vcol >= L.vc_total || L.lane >= L.lanes) continue;
-#pragma unroll 4
-                for (int64_t r = lo + L.lane; r < hi; r += L.lanes) {
-                    float v[VN];
-                    load_vec<T, VN>(x + r * C + (int64_t)vcol * VN, v);
-#pragma unroll
-                    for (int i = 0; i < VN; ++i) {
-                        const float d = v[i] - mu;
-                        acc += pass ? d * d : d;
-                    }
-                }
-            }
-            result[pass] = block_sum(acc, scratch);
-            if (pass == 0) mu = result[0] / ((float)(hi - lo) * (float)C);
-        }
-        if (threadIdx.x == 0) rec[blockIdx.x + s] = Moments{(float)(hi - lo) * (float)C, mu, result[1], 0.f};
-    }
+__device__ __forceinline__ void merge(Moments &a, float n, float mean, float m2) {
+    if (n == 0.f) return;
+    const float total = a.n + n, d = mean - a.mean, share = n / total;
+    a.mean += d * share;
+    a.m2 += m2 + d * d * a.n * share;
+    a.n = total;
 }
 
-// The same statistics with the block's rows held in registers (rows of at most 256 sixteen-byte
-// columns): a thread loads MOM_R rows of its column once, and both sweeps -- the sum, then the squares
-// centred on the block mean -- run over those registers.  A block covers MOM_R * (256 / columns) rows.
 constexpr int MOM_R = 4;
 
 template <typename T, int VN>
-__global__ void __launch_bounds__(LN_THREADS) ln_moments_reg_kernel(const T *__restrict__ x, const int64_t *__restrict__ offsets,
-                                                                    Moments *rec, int64_t N, int64_t S, int C, int mom_rows) {
-    __shared__ float scratch[LN_THREADS / 32];
-    const RowLayout L(C, VN);   // one pass: vc_total <= blockDim
-    const int64_t row0 = (int64_t)blockIdx.x * mom_rows, row1 = min(N, row0 + mom_rows);
-    const int64_t s_first = segment_of_row(offsets, S, row0), s_last = segment_of_row(offsets, S, row1 - 1);
-    float v[MOM_R][VN];
-    int64_t rows[MOM_R];
-#pragma unroll
-    for (int k = 0; k < MOM_R; ++k) {
-        rows[k] = row0 + L.lane + (int64_t)k * L.lanes;
-        if (L.lane < L.lanes && rows[k] < row1) {
-            load_vec<T, VN>(x + rows[k] * C + (int64_t)L.vc * VN, v[k]);
-        } else {
-            rows[k] = -1;
-#pragma unroll
-            for (int i = 0; i < VN; ++i) v[k][i] = 0.f;
-        }
-    }
-    for (int64_t s = s_first; s <= s_last; ++s) {
-        const int64_t lo = max(row0, offsets[s]), hi = min(row1, offsets[s + 1]);
+__global__ void __launch_bounds__(LN_THREADS, 4) ln_moments_kernel(const T *__restrict__ x, const int64_t *__restrict__ offsets, Moments *rec,
+                                                                   int64_t N, int64_t S, int C, int rows) {
+    __shared__ Moments scratch[LN_THREADS / 32];
+    const BlockRows B(offsets, N, S, rows);
+    const RowLayout L(C, VN);
+    for (int64_t s = B.s_first; s <= B.s_last; ++s) {
+        const int64_t lo = max(B.row0, offsets[s]), hi = min(B.row1, offsets[s + 1]);
         if (hi <= lo) continue;   // an empty sample inside the block (same decision in every thread)
-        float mu = 0.f, result[2];
+        Moments m{0.f, 0.f, 0.f, 0.f};
+        for (int cp = 0; cp * L.vcb < L.vc_total; ++cp) {
+            const int vcol = cp * L.vcb + L.vc;
+            if (vcol >= L.vc_total || L.lane >= L.lanes) continue;
+            const T *col = x + (int64_t)vcol * VN;
+            int64_t r = lo + L.lane;
+            for (; r + (MOM_R - 1) * L.lanes < hi; r += (int64_t)MOM_R * L.lanes) {
+                float v[MOM_R][VN], sum = 0.f, sq = 0.f;
 #pragma unroll
-        for (int pass = 0; pass < 2; ++pass) {
-            float acc = 0.f;
+                for (int k = 0; k < MOM_R; ++k) load_vec<T, VN>(col + (r + (int64_t)k * L.lanes) * C, v[k]);
 #pragma unroll
-            for (int k = 0; k < MOM_R; ++k) {
-                if (rows[k] >= lo && rows[k] < hi) {
+                for (int k = 0; k < MOM_R; ++k)
 #pragma unroll
-                    for (int i = 0; i < VN; ++i) {
-                        const float d = v[k][i] - mu;
-                        acc += pass ? d * d : d;
-                    }
-                }
+                    for (int i = 0; i < VN; ++i) sum += v[k][i];
+                const float mu = sum * (1.f / (MOM_R * VN));
+#pragma unroll
+                for (int k = 0; k < MOM_R; ++k)
+#pragma unroll
+                    for (int i = 0; i < VN; ++i) sq += (v[k][i] - mu) * (v[k][i] - mu);
+                merge(m, (float)(MOM_R * VN), mu, sq);
             }
-            result[pass] = block_sum(acc, scratch);
-            if (pass == 0) mu = result[0] / ((float)(hi - lo) * (float)C);
+            for (; r < hi; r += L.lanes) {
+                float v[VN], sum = 0.f, sq = 0.f;
+                load_vec<T, VN>(col + r * C, v);
+#pragma unroll
+                for (int i = 0; i < VN; ++i) sum += v[i];
+                const float mu = sum * (1.f / VN);
+#pragma unroll
+                for (int i = 0; i < VN; ++i) sq += (v[i] - mu) * (v[i] - mu);
+                merge(m, (float)VN, mu, sq);
+            }
         }
-        if (threadIdx.x == 0) rec[blockIdx.x + s] = Moments{(float)(hi - lo) * (float)C, mu, result[1], 0.f};
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float n = __shfl_xor_sync(0xffffffffu, m.n, o), mean = __shfl_xor_sync(0xffffffffu, m.mean, o),
+                        m2 = __shfl_xor_sync(0xffffffffu, m.m2, o);
+            merge(m, n, mean, m2);
+        }
+        __syncthreads();
+        if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = m;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            for (int w = 1; w < LN_THREADS / 32; ++w) merge(m, scratch[w].n, scratch[w].mean, scratch[w].m2);
+            rec[blockIdx.x + s] = m;
+        }
     }
 }
 
@@ -216,8 +211,8 @@ template <typename T, int VN>
 __global__ void __launch_bounds__(LN_THREADS, 5) ln_apply_kernel(const T *__restrict__ x, const int64_t *__restrict__ offsets,
                                 const float *__restrict__ mean, const float *__restrict__ rstd,
                                 const float *__restrict__ weight, const float *__restrict__ bias,
-                                const T *__restrict__ residual, T *y, int64_t N, int64_t S, int C, int relu) {
-    const BlockRows B(offsets, N, S);
+                                const T *__restrict__ residual, T *y, int64_t N, int64_t S, int C, int relu, int rows) {
+    const BlockRows B(offsets, N, S, rows);
     const RowLayout L(C, VN);
     for (int cp = 0; cp * L.vcb < L.vc_total; ++cp) {
         const int vcol = cp * L.vcb + L.vc;
@@ -228,10 +223,7 @@ __global__ void __launch_bounds__(LN_THREADS, 5) ln_apply_kernel(const T *__rest
             w[i] = weight ? weight[vcol * VN + i] : 1.f;
             b[i] = weight ? bias[vcol * VN + i] : 0.f;
         }
-#pragma unroll 4
-        for (int64_t r = B.row0 + L.lane; r < B.row1; r += L.lanes) {
-            const int64_t s = B.uniform ? B.s_first : segment_of_row(offsets, S, r);
-            const float mu = mean[s], rs = rstd[s];
+        auto row = [&](int64_t r, float mu, float rs) {
             const int64_t at = r * C + (int64_t)vcol * VN;
             float v[VN], res[VN];
             load_vec<T, VN>(x + at, v);
@@ -243,6 +235,19 @@ __global__ void __launch_bounds__(LN_THREADS, 5) ln_apply_kernel(const T *__rest
                 v[i] = relu ? fmaxf(o, 0.f) : o;
             }
             store_vec<T, VN>(y + at, v);
+        };
+        if (B.in_pieces()) {
+            for (int64_t s = B.s_first; s <= B.s_last; ++s) {
+                const int64_t hi = min(B.row1, offsets[s + 1]);
+                const float mu = mean[s], rs = rstd[s];
+#pragma unroll 4
+                for (int64_t r = max(B.row0, offsets[s]) + L.lane; r < hi; r += L.lanes) row(r, mu, rs);
+            }
+        } else {
+            for (int64_t r = B.row0 + L.lane; r < B.row1; r += L.lanes) {
+                const int64_t s = segment_of_row(offsets, S, r);
+                row(r, mean[s], rstd[s]);
+            }
         }
     }
 }
@@ -256,10 +261,10 @@ __global__ void __launch_bounds__(LN_THREADS, 4) ln_bwd_sums_kernel(const T *__r
                                    const int64_t *__restrict__ offsets, const float *__restrict__ mean,
                                    const float *__restrict__ rstd, const float *__restrict__ weight, float *s1,
                                    float *s2, float *dweight, float *dbias, T *dresidual, int64_t N, int64_t S,
-                                   int C, int relu) {
+                                   int C, int relu, int rows) {
     __shared__ float scratch[LN_THREADS / 32];
     __shared__ float col_w[LN_THREADS * VN], col_b[LN_THREADS * VN];
-    const BlockRows B(offsets, N, S);
+    const BlockRows B(offsets, N, S, rows);
     const RowLayout L(C, VN);
     float a = 0.f, b = 0.f;     // running sums of gh and gh * xh for sample `cur`
     int64_t cur = B.s_first;
@@ -272,32 +277,47 @@ __global__ void __launch_bounds__(LN_THREADS, 4) ln_bwd_sums_kernel(const T *__r
             w[i] = (weight && active) ? weight[vcol * VN + i] : 1.f;
             dw[i] = db[i] = 0.f;
         }
-        if (active) {
+        auto row = [&](int64_t r, float mu, float rs) {
+            const int64_t at = r * C + (int64_t)vcol * VN;
+            float gv[VN], xv[VN], yv[VN];
+            load_vec<T, VN>(g + at, gv);
+            load_vec<T, VN>(x + at, xv);
+            if (relu) load_vec<T, VN>(y + at, yv);
+#pragma unroll
+            for (int i = 0; i < VN; ++i) {
+                if (relu && !(yv[i] > 0.f)) gv[i] = 0.f;
+                const float xh = (xv[i] - mu) * rs;
+                a += gv[i] * w[i];
+                b += gv[i] * w[i] * xh;
+                dw[i] += gv[i] * xh;
+                db[i] += gv[i];
+            }
+            if (dresidual) store_vec<T, VN>(dresidual + at, gv);
+        };
+        if (B.in_pieces()) {
+            for (int64_t s = B.s_first; s <= B.s_last; ++s) {
+                const int64_t hi = active ? min(B.row1, offsets[s + 1]) : 0;
+                const float mu = mean[s], rs = rstd[s];
 #pragma unroll 2
+                for (int64_t r = max(B.row0, offsets[s]) + L.lane; r < hi; r += L.lanes) row(r, mu, rs);
+                a = block_sum(a, scratch);
+                b = block_sum(b, scratch);
+                if (threadIdx.x == 0) {
+                    atomicAdd(s1 + s, a);
+                    atomicAdd(s2 + s, b);
+                }
+                a = b = 0.f;
+            }
+        } else if (active) {
             for (int64_t r = B.row0 + L.lane; r < B.row1; r += L.lanes) {
-                const int64_t s = B.uniform ? B.s_first : segment_of_row(offsets, S, r);
+                const int64_t s = segment_of_row(offsets, S, r);
                 if (s != cur) {
                     atomicAdd(s1 + cur, a);
                     atomicAdd(s2 + cur, b);
                     a = b = 0.f;
                     cur = s;
                 }
-                const float mu = mean[s], rs = rstd[s];
-                const int64_t at = r * C + (int64_t)vcol * VN;
-                float gv[VN], xv[VN], yv[VN];
-                load_vec<T, VN>(g + at, gv);
-                load_vec<T, VN>(x + at, xv);
-                if (relu) load_vec<T, VN>(y + at, yv);
-#pragma unroll
-                for (int i = 0; i < VN; ++i) {
-                    if (relu && !(yv[i] > 0.f)) gv[i] = 0.f;
-                    const float xh = (xv[i] - mu) * rs;
-                    a += gv[i] * w[i];
-                    b += gv[i] * w[i] * xh;
-                    dw[i] += gv[i] * xh;
-                    db[i] += gv[i];
-                }
-                if (dresidual) store_vec<T, VN>(dresidual + at, gv);
+                row(r, mean[s], rstd[s]);
             }
         }
         if (dweight) {
@@ -321,26 +341,19 @@ __global__ void __launch_bounds__(LN_THREADS, 4) ln_bwd_sums_kernel(const T *__r
             __syncthreads();
         }
     }
-    if (B.uniform) {
-        a = block_sum(a, scratch);
-        b = block_sum(b, scratch);
-        if (threadIdx.x == 0) {
-            atomicAdd(s1 + B.s_first, a);
-            atomicAdd(s2 + B.s_first, b);
-        }
-    } else {
+    if (!B.in_pieces()) {
         atomicAdd(s1 + cur, a);
         atomicAdd(s2 + cur, b);
     }
 }
 
 template <typename T, int VN>
-__global__ void ln_bwd_apply_kernel(const T *__restrict__ g, const T *__restrict__ x, const T *__restrict__ y,
+__global__ void __launch_bounds__(LN_THREADS, 4) ln_bwd_apply_kernel(const T *__restrict__ g, const T *__restrict__ x, const T *__restrict__ y,
                                     const int64_t *__restrict__ offsets, const float *__restrict__ mean,
                                     const float *__restrict__ rstd, const float *__restrict__ weight,
                                     const float *__restrict__ s1, const float *__restrict__ s2, T *dx, int64_t N,
-                                    int64_t S, int C, int relu) {
-    const BlockRows B(offsets, N, S);
+                                    int64_t S, int C, int relu, int rows) {
+    const BlockRows B(offsets, N, S, rows);
     const RowLayout L(C, VN);
     for (int cp = 0; cp * L.vcb < L.vc_total; ++cp) {
         const int vcol = cp * L.vcb + L.vc;
@@ -348,12 +361,7 @@ __global__ void ln_bwd_apply_kernel(const T *__restrict__ g, const T *__restrict
         float w[VN];
 #pragma unroll
         for (int i = 0; i < VN; ++i) w[i] = weight ? weight[vcol * VN + i] : 1.f;
-#pragma unroll 2
-        for (int64_t r = B.row0 + L.lane; r < B.row1; r += L.lanes) {
-            const int64_t s = B.uniform ? B.s_first : segment_of_row(offsets, S, r);
-            const float mu = mean[s], rs = rstd[s];
-            const float inv_n = 1.f / ((float)(offsets[s + 1] - offsets[s]) * (float)C);
-            const float m1 = s1[s] * inv_n, m2 = s2[s] * inv_n;
+        auto row = [&](int64_t r, float mu, float rs, float m1, float m2) {
             const int64_t at = r * C + (int64_t)vcol * VN;
             float gv[VN], xv[VN], yv[VN];
             load_vec<T, VN>(g + at, gv);   // with relu == 0 this may be the gradient the sums pass already masked
@@ -366,6 +374,21 @@ __global__ void ln_bwd_apply_kernel(const T *__restrict__ g, const T *__restrict
                 gv[i] = rs * (gv[i] * w[i] - m1 - xh * m2);
             }
             store_vec<T, VN>(dx + at, gv);
+        };
+        if (B.in_pieces()) {
+            for (int64_t s = B.s_first; s <= B.s_last; ++s) {
+                const int64_t hi = min(B.row1, offsets[s + 1]);
+                const float mu = mean[s], rs = rstd[s], inv_n = 1.f / ((float)(offsets[s + 1] - offsets[s]) * (float)C);
+                const float m1 = s1[s] * inv_n, m2 = s2[s] * inv_n;
+#pragma unroll 2
+                for (int64_t r = max(B.row0, offsets[s]) + L.lane; r < hi; r += L.lanes) row(r, mu, rs, m1, m2);
+            }
+        } else {
+            for (int64_t r = B.row0 + L.lane; r < B.row1; r += L.lanes) {
+                const int64_t s = segment_of_row(offsets, S, r);
+                const float inv_n = 1.f / ((float)(offsets[s + 1] - offsets[s]) * (float)C);
+                row(r, mean[s], rstd[s], s1[s] * inv_n, s2[s] * inv_n);
+            }
         }
     }
 }
@@ -639,11 +662,25 @@ size_t carve_ln(void *ws, int64_t S, LnWs *out, int64_t pieces = 0) {
     return c.off;
 }
 
-int ln_offsets(const int64_t *d_lengths, int64_t S, int64_t N, const LnWs &w, cudaStream_t stream) {
+// Rows per block: one wave of `ctas` blocks per SM, whole row lanes, at least two rows per thread.
+int layer_rows(int64_t N, int C, int dtype, bool vec, int ctas) {
+    const int cols = C / (vec ? 16 / (int)elem_size(dtype) : 1), lanes = LN_THREADS / std::min(cols, LN_THREADS);
+    const int64_t wave = (int64_t)ctas * num_sms(), rows = (N + wave - 1) / wave;
+    return (int)std::min<int64_t>(((std::max<int64_t>(rows, 2 * lanes) + lanes - 1) / lanes) * lanes, (int64_t)1 << 30);
+}
+
+// `z1`, `z2` (n12 floats each, or null) and, with `zero_sums`, the workspace's sums are cleared on the way.
+int ln_offsets(const int64_t *d_lengths, int64_t S, int64_t N, const LnWs &w, cudaStream_t stream, bool zero_sums = false, float *z1 = nullptr,
+               float *z2 = nullptr, int64_t n12 = 0) {
     if (S <= 4096) {
-        ln_small_offsets_kernel<<<1, 32, 0, stream>>>(d_lengths, w.offsets, S, N);
+        ln_small_offsets_kernel<<<1, 256, 0, stream>>>(d_lengths, w.offsets, S, N, w.sums, zero_sums ? 2 * S : 0, z1, z2, z1 ? n12 : 0);
         PCX_LAUNCH_CHECK();
         return PCX_OK;
+    }
+    if (zero_sums) PCX_CUDA(cudaMemsetAsync(w.sums, 0, (size_t)2 * S * sizeof(float), stream));
+    if (z1) {
+        PCX_CUDA(cudaMemsetAsync(z1, 0, (size_t)n12 * sizeof(float), stream));
+        PCX_CUDA(cudaMemsetAsync(z2, 0, (size_t)n12 * sizeof(float), stream));
     }
     size_t bytes = w.cub_bytes;
     PCX_CUDA(cub::DeviceScan::ExclusiveSum(w.cub_tmp, bytes, d_lengths, w.offsets, (int)S, stream));
@@ -653,8 +690,8 @@ int ln_offsets(const int64_t *d_lengths, int64_t S, int64_t N, const LnWs &w, cu
 }
 
 // (block, sample) pieces of N rows in S samples: record b + s, b < blocks, s < S
-// an upper bound for every block height the statistics pass may choose (at least MOM_R rows per block)
-int64_t ln_pieces(int64_t N, int64_t S) { return (N + MOM_R - 1) / MOM_R + S; }
+// an upper bound for every block height the statistics pass may choose (at least two rows per block)
+int64_t ln_pieces(int64_t N, int64_t S) { return (N + 1) / 2 + S; }
 
 bool ln_sizes_ok(int64_t N, int64_t S, int C, int dtype) {
     return N >= 0 && S > 0 && S <= INT32_MAX && C > 0 && (dtype == PCX_F32 || dtype == PCX_F16 || dtype == PCX_BF16);
@@ -691,27 +728,20 @@ int pcx_ragged_layer_norm(const void *d_x, const int64_t *d_lengths, const float
     size_t need = carve_ln(d_ws, S, &w, ln_pieces(N, S));
     if (ws_bytes < need) PCX_FAIL(PCX_E_CAPACITY, "pcx_ragged_layer_norm: workspace %zu < %zu bytes", ws_bytes, need);
     if (int rc = ln_offsets(d_lengths, S, N, w, stream)) return rc;
-    const unsigned grid = (unsigned)((N + LN_ROWS - 1) / LN_ROWS);
     const bool vec = vec_ok(C, dtype, {d_x, d_y, d_residual});
-    int mom_rows = LN_ROWS;
-    const int vcols = C / (16 / (int)elem_size(dtype));   // sixteen-byte columns of a row (when vectorised)
-    if (vec && vcols <= LN_THREADS) mom_rows = MOM_R * (LN_THREADS / vcols);   // rows held in registers
+    const int mom_rows = layer_rows(N, C, dtype, vec, 4), rows = layer_rows(N, C, dtype, vec, 5);
     if (N > 0) {
-        if (mom_rows != LN_ROWS) {
-            const unsigned mgrid = (unsigned)((N + mom_rows - 1) / mom_rows);
-            PCX_LN_DISPATCH(dtype, true, (ln_moments_reg_kernel<T, VN><<<mgrid, LN_THREADS, 0, stream>>>((const T *)d_x, w.offsets, w.rec, N, S, C, mom_rows)));
-        } else {
-            PCX_LN_DISPATCH(dtype, vec, (ln_moments_kernel<T, VN><<<grid, LN_THREADS, 0, stream>>>((const T *)d_x, w.offsets, w.rec, N, S, C)));
-        }
+        const unsigned mgrid = (unsigned)((N + mom_rows - 1) / mom_rows);
+        PCX_LN_DISPATCH(dtype, vec, (ln_moments_kernel<T, VN><<<mgrid, LN_THREADS, 0, stream>>>((const T *)d_x, w.offsets, w.rec, N, S, C, mom_rows)));
         PCX_LAUNCH_CHECK();
     }
     ln_combine_kernel<<<(unsigned)S, COMBINE_THREADS, 0, stream>>>(w.rec, w.offsets, d_mean, d_rstd, S, (float)eps, mom_rows);
     PCX_LAUNCH_CHECK();
     if (N > 0) {
         prof_begin("ln_apply_kernel", stream);
-        PCX_LN_DISPATCH(dtype, vec, (ln_apply_kernel<T, VN><<<grid, LN_THREADS, 0, stream>>>(
+        PCX_LN_DISPATCH(dtype, vec, (ln_apply_kernel<T, VN><<<(unsigned)((N + rows - 1) / rows), LN_THREADS, 0, stream>>>(
                                    (const T *)d_x, w.offsets, d_mean, d_rstd, d_weight, d_bias, (const T *)d_residual,
-                                   (T *)d_y, N, S, C, relu)));
+                                   (T *)d_y, N, S, C, relu, rows)));
         prof_end(stream);
         PCX_LAUNCH_CHECK();
     }
@@ -731,25 +761,21 @@ int pcx_ragged_layer_norm_backward(const void *d_grad_y, const void *d_x, const 
     LnWs w;
     size_t need = carve_ln(d_ws, S, &w);
     if (ws_bytes < need) PCX_FAIL(PCX_E_CAPACITY, "pcx_ragged_layer_norm_backward: workspace %zu < %zu bytes", ws_bytes, need);
-    if (int rc = ln_offsets(d_lengths, S, N, w, stream)) return rc;
-    PCX_CUDA(cudaMemsetAsync(w.sums, 0, (size_t)2 * S * sizeof(float), stream));
-    if (d_grad_weight) {
-        PCX_CUDA(cudaMemsetAsync(d_grad_weight, 0, (size_t)C * sizeof(float), stream));
-        PCX_CUDA(cudaMemsetAsync(d_grad_bias, 0, (size_t)C * sizeof(float), stream));
-    }
+    if (int rc = ln_offsets(d_lengths, S, N, w, stream, true, d_grad_weight, d_grad_bias, C)) return rc;
     if (N == 0) return PCX_OK;
-    const unsigned grid = (unsigned)((N + LN_ROWS - 1) / LN_ROWS);
     const bool vec = vec_ok(C, dtype, {d_grad_y, d_x, d_y, d_grad_x, d_grad_residual});
+    const int rows = layer_rows(N, C, dtype, vec, 4);
+    const unsigned grid = (unsigned)((N + rows - 1) / rows);
     PCX_LN_DISPATCH(dtype, vec, (ln_bwd_sums_kernel<T, VN><<<grid, LN_THREADS, 0, stream>>>(
                                (const T *)d_grad_y, (const T *)d_x, (const T *)d_y, w.offsets, d_mean, d_rstd, d_weight,
-                               w.sums, w.sums + S, d_grad_weight, d_grad_bias, (T *)d_grad_residual, N, S, C, relu)));
+                               w.sums, w.sums + S, d_grad_weight, d_grad_bias, (T *)d_grad_residual, N, S, C, relu, rows)));
     PCX_LAUNCH_CHECK();
     // the sums pass wrote the ReLU-masked gradient as the residual's gradient: the second pass reads
     // that instead of masking again, which spares it the read of y
     const bool masked = relu && d_grad_residual;
     PCX_LN_DISPATCH(dtype, vec, (ln_bwd_apply_kernel<T, VN><<<grid, LN_THREADS, 0, stream>>>(
                                (const T *)(masked ? d_grad_residual : d_grad_y), (const T *)d_x, (const T *)d_y, w.offsets,
-                               d_mean, d_rstd, d_weight, w.sums, w.sums + S, (T *)d_grad_x, N, S, C, masked ? 0 : relu)));
+                               d_mean, d_rstd, d_weight, w.sums, w.sums + S, (T *)d_grad_x, N, S, C, masked ? 0 : relu, rows)));
     PCX_LAUNCH_CHECK();
     return PCX_OK;
 }
