@@ -424,14 +424,20 @@ __global__ void plan_cost_kernel(const int32_t *__restrict__ tile_offs, int64_t 
 }
 
 // ------------------------------------------------------------------ kernel ----
-constexpr int EPI_WARPS = 4, TEAMS = 2, TEAM_WARPS = 8, COPY_WARPS = TEAMS * TEAM_WARPS;
+constexpr int EPI_WARPS = 4, TEAMS = 4, TEAM_WARPS = 4, COPY_WARPS = TEAMS * TEAM_WARPS;
 constexpr int COPY_WARP0 = EPI_WARPS, WALK_WARP = COPY_WARP0 + COPY_WARPS, WEIGHT_WARP = WALK_WARP + 1, MMA_WARP0 = WEIGHT_WARP + 1;
 constexpr int THREADS = (MMA_WARP0 + GROUP_BLOCKS) * 32;
 constexpr int MAX_SLOTS = 8;
-constexpr int AHEAD = 8;                              // steps the walk runs ahead (even: an entry always belongs to the same team)
+constexpr int AHEAD = 8;                              // steps the walk runs ahead
 constexpr uint32_t ENTRY_BYTES = 2 * ROWS * 4;        // source rows of a step's two tiles
 // a step's word: slice << 9 | tiles that have the tap << 13 | first of its unit << 15 | end << 16
 constexpr uint32_t STEP_FIRST = 1u << 15, STEP_END = 1u << 16;
+// The MMA threads read the words from a ring of their own, each marked with the turn of the ring it belongs to.
+// The walk is at most AHEAD steps ahead of the copies and these at most MAX_SLOTS ahead of the MMAs, so with
+// WORDS entries no word is overwritten before it has been read.
+constexpr int WORDS = 32;
+static_assert(WORDS >= AHEAD + MAX_SLOTS + TEAMS, "the word ring must hold every step between the walk and the MMAs");
+constexpr uint32_t TURN_SHIFT = 17;   // turn (from 1 on) in the upper 15 bits
 
 struct OsParams {
     const uint16_t *feat, *bias;            // rows of in_pitch elements; bias: added before the rounding; null: none
@@ -444,7 +450,7 @@ struct OsParams {
     int K, C, M, transpose, reverse, fmt;   // reverse: tap k uses weight K-1-k
     int inw, outw, nkb, ngroups, nblocks, nsplit, mask_words;   // inw, outw: of a part
     int nparts, out_parts, in_pitch, out_pitch;   // parts of an output row: groups of the weight, each in out_parts
-    int nslots, nacc;
+    int nslots, nacc, teams;
     uint32_t slot_bytes, w_box_rows, w_tx_bytes, ncols, col_stride;
     uint64_t wait_limit_ns;
 };
@@ -528,11 +534,15 @@ struct Ring {
     __device__ __forceinline__ void next(int depth) {
         if (++slot == (uint32_t)depth) slot = 0, ++turn;
     }
+    __device__ __forceinline__ void skip(int by, int depth) {
+        for (slot += (uint32_t)by; slot >= (uint32_t)depth; ++turn) slot -= (uint32_t)depth;
+    }
 };
 
 __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ OsParams p) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t s_full[MAX_SLOTS], s_empty[MAX_SLOTS], s_acc_full[2], s_acc_empty[2], s_step_full[AHEAD], s_step_empty[AHEAD];
+    __shared__ uint32_t s_word[WORDS];
     __shared__ uint4 s_step[AHEAD];   // the step's word, its first feature column, the corner of its weight slice
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
@@ -542,15 +552,21 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
     const uint32_t slot0 = (smem_u32(smem_raw) + 1023u) & ~1023u, rows0 = slot0 + (uint32_t)p.nslots * p.slot_bytes;
     volatile int *abort_flag = &s_abort;
     auto wait = [&](const uint64_t &bar, uint32_t parity) {   // the verdict is the same in the whole warp
+        if (__all_sync(0xffffffffu, mbar_try_wait(smem_u32(&bar), parity & 1u))) return true;
         return __all_sync(0xffffffffu, mbar_wait_abortable(smem_u32(&bar), parity & 1u, STATUS_BIT, p.status, abort_flag, p.wait_limit_ns)) != 0;
+    };
+
+    auto wait_one = [&](const uint64_t &bar, uint32_t parity) {   // for roles of a single thread
+        return mbar_wait_abortable(smem_u32(&bar), parity & 1u, STATUS_BIT, p.status, abort_flag, p.wait_limit_ns);
     };
 
     if (tid == 0) {
         for (int s = 0; s < p.nslots; ++s)   // a team's copies and the weight slice; both MMA warps
             mbar_init(smem_u32(&s_full[s]), TEAM_WARPS * 32 + 1), mbar_init(smem_u32(&s_empty[s]), GROUP_BLOCKS);
         for (int s = 0; s < 2; ++s) mbar_init(smem_u32(&s_acc_full[s]), GROUP_BLOCKS), mbar_init(smem_u32(&s_acc_empty[s]), EPI_WARPS);
-        for (int s = 0; s < AHEAD; ++s)   // the walk's copies and its word; a team, the MMA warps and the weight warp
-            mbar_init(smem_u32(&s_step_full[s]), 33), mbar_init(smem_u32(&s_step_empty[s]), TEAM_WARPS + GROUP_BLOCKS + 1);
+        for (int s = 0; s < WORDS; ++s) s_word[s] = 0u;
+        for (int s = 0; s < AHEAD; ++s)   // the walk; a team and the weight warp
+            mbar_init(smem_u32(&s_step_full[s]), 1), mbar_init(smem_u32(&s_step_empty[s]), TEAM_WARPS + 1);
         fence_mbar_init();
         s_abort = 0;
         tma_prefetch_desc(&tmap);
@@ -616,87 +632,96 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
         }
     } else if (warp < WALK_WARP) {
         // ------------------------------------------------------------------ copies ----
-        // Two teams take the steps in turn: while one team's copies go through the load/store unit (230 clocks
-        // for a 16 KB tile) the other one waits for its slot and fetches its rows.  A warp owns 16 rows of
-        // either tile, eight lanes a row, a group of eight lanes four consecutive rows.
+        // Four teams take the steps in turn: while one team's copies go through the load/store unit (230 clocks
+        // for a 16 KB tile) the others wait for their slots and fetch their rows.  A warp owns 32 rows of either
+        // tile, eight lanes a row, a group of eight lanes eight consecutive rows.
         const int team = (warp - COPY_WARP0) / TEAM_WARPS, piece = lane & 7;
-        const int row0 = ((warp - COPY_WARP0) % TEAM_WARPS) * 16 + (lane >> 3) * 4;
-        uint32_t dst_off[4];
+        const int row0 = ((warp - COPY_WARP0) % TEAM_WARPS) * 32 + (lane >> 3) * 8;
+        uint32_t dst_off[8];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) dst_off[k] = (uint32_t)(row0 + k) * 128 + (uint32_t)((piece ^ ((row0 + k) & 7)) << 4);
+        for (int k = 0; k < 8; ++k) dst_off[k] = (uint32_t)(row0 + k) * 128 + (uint32_t)((piece ^ k) << 4);
+        const uint32_t pitch = (uint32_t)p.in_pitch * 2u;
         Ring ring, step;
-        for (int n = 0;; n ^= 1) {   // (two teams)
-            if (n == team) {
-                if (!wait(s_step_full[step.slot], step.turn)) break;
-                const uint32_t word = *(volatile uint32_t *)&s_step[step.slot].x;
-                if (word & STEP_END) break;
-                const uint32_t at = rows0 + step.slot * ENTRY_BYTES + (uint32_t)row0 * 4;
-                const uint4 rows[2] = {lds_v4(at), lds_v4(at + ROWS * 4)};
-                const uint32_t column = *(volatile uint32_t *)&s_step[step.slot].y + (uint32_t)piece * 8;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&s_step_empty[step.slot]));
-                const int slice = (int)(word >> 9) & 15;
-                const uint16_t *col = p.feat + column, *sums = p.scratch + column;
-                const bool piece_ok = piece * 8 < p.inw - slice * 64;
-                // the tensor core has finished with what was in the slot
-                if (!wait(s_empty[ring.slot], ring.turn ^ 1u)) break;
-                const uint32_t dst = slot0 + ring.slot * p.slot_bytes;
-                if (piece_ok) {
+        for (int n = 0; n < team; ++n) ring.next(p.nslots), step.next(AHEAD);
+        while (team < p.teams) {
+            if (!wait(s_step_full[step.slot], step.turn)) break;
+            const uint32_t word = *(volatile uint32_t *)&s_step[step.slot].x;
+            if (word & STEP_END) break;
+            const uint32_t at = rows0 + step.slot * ENTRY_BYTES + (uint32_t)row0 * 4;
+            const uint4 rows[4] = {lds_v4(at), lds_v4(at + 16), lds_v4(at + ROWS * 4), lds_v4(at + ROWS * 4 + 16)};
+            const uint32_t column = *(volatile uint32_t *)&s_step[step.slot].y + (uint32_t)piece * 8;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&s_step_empty[step.slot]));
+            const int slice = (int)(word >> 9) & 15;
+            const char *col = reinterpret_cast<const char *>(p.feat + column);
+            const char *sums = reinterpret_cast<const char *>(p.scratch + column) - pitch;
+            const bool piece_ok = piece * 8 < p.inw - slice * 64;
+            // the tensor core has finished with what was in the slot
+            if (!wait(s_empty[ring.slot], ring.turn ^ 1u)) break;
+            const uint32_t dst = slot0 + ring.slot * p.slot_bytes;
+            if (piece_ok) {
 #pragma unroll
-                    for (int t = 0; t < 2; ++t) {
-                        if (!((word >> (13 + t)) & 1u)) continue;
-                        const int32_t rr[4] = {(int32_t)rows[t].x, (int32_t)rows[t].y, (int32_t)rows[t].z, (int32_t)rows[t].w};
+                for (int t = 0; t < 2; ++t) {
+                    if (!((word >> (13 + t)) & 1u)) continue;
+                    const int32_t rr[8] = {(int32_t)rows[2 * t].x, (int32_t)rows[2 * t].y, (int32_t)rows[2 * t].z, (int32_t)rows[2 * t].w,
+                                           (int32_t)rows[2 * t + 1].x, (int32_t)rows[2 * t + 1].y, (int32_t)rows[2 * t + 1].z, (int32_t)rows[2 * t + 1].w};
 #pragma unroll
-                        for (int k = 0; k < 4; ++k) {
-                            // a feature row, a row of bucket sums, or nothing (zeros: source size 0)
-                            const uint32_t idx = (uint32_t)(rr[k] >= 0 ? rr[k] : rr[k] == -1 ? 0 : -2 - rr[k]);
-                            const uint16_t *src = (rr[k] < -1 ? sums : col) + (uint64_t)idx * (uint32_t)p.in_pitch;
-                            cp_async16_zfill(dst + (uint32_t)t * SLOT_BYTES + dst_off[k], src, rr[k] == -1 ? 0u : 16u);
-                        }
+                    for (int k = 0; k < 8; ++k) {
+                        // a feature row x >= 0, the row of bucket sums -2 - x, or nothing (-1: zeros, and a source that is not read)
+                        const char *src = (rr[k] < -1 ? sums : col) + (uint64_t)(uint32_t)(rr[k] ^ (rr[k] >> 31)) * pitch;
+                        cp_async16_or_zero(dst + (uint32_t)t * SLOT_BYTES + dst_off[k], src, rr[k] == -1);
                     }
                 }
-                cp_async_mbar_arrive(smem_u32(&s_full[ring.slot]));   // fires once this thread's copies have landed
             }
-            ring.next(p.nslots);
-            step.next(AHEAD);
+            cp_async_mbar_arrive(smem_u32(&s_full[ring.slot]));   // fires once this thread's copies have landed
+            ring.skip(p.teams, p.nslots);
+            step.skip(p.teams, AHEAD);
         }
         cp_async_wait<0>();
     } else if (warp == WALK_WARP) {
         // -------------------------------------------------------------------- walk ----
         // Decides the steps and brings the source rows of their tiles into shared memory, AHEAD steps early:
-        // the tables come from DRAM, once.
-        Walk w(p);
-        Ring step;
-        bool more = true;
-        for (int ends = 0; ends < TEAMS;) {   // an end mark for either team
-            if (!wait(s_step_empty[step.slot], step.turn ^ 1u)) break;
-            if (more) more = w.next();
-            const uint32_t entry = rows0 + step.slot * ENTRY_BYTES + (uint32_t)lane * 16, full = smem_u32(&s_step_full[step.slot]);
-            if (more) {
-                const int32_t *src = p.tile_rows + ((int64_t)w.block0 * p.K + w.tap) * ROWS + lane * 4;
-                if (w.has & 1u) cp_async16(entry, src);
-                if (w.has & 2u) cp_async16(entry + ROWS * 4, src + (int64_t)p.K * ROWS);
-            } else {
-                ++ends;
-            }
-            if (lane == 0) {
+        // the tables come from DRAM, once.  One thread and a bulk copy a tile: as a warp with votes, a copy a lane
+        // and the divisions of the part in every step it took 1300 clocks a step and held up everything behind it.
+        if (elect_one()) {
+            Walk w(p);
+            Ring step, word;
+            bool more = true;
+            int column = 0, wx = 0, wy = 0;   // of the unit: first feature column, corner of its weights in the (taps * groups * C, M) matrix
+            const int groups = p.nparts / p.out_parts, tap_rows = groups * p.C;
+            for (int ends = 0; ends < p.teams;) {   // an end mark for each team
+                if (!wait_one(s_step_empty[step.slot], step.turn ^ 1u)) break;
+                if (more) more = w.next();
+                const uint32_t full = smem_u32(&s_step_full[step.slot]);
                 uint4 s = make_uint4(STEP_END, 0u, 0u, 0u);
                 if (more) {
-                    // feature columns of the part's group; corner (x, y) of the weight slice in the (taps * groups * C, M) matrix
-                    const int g = w.part / p.out_parts, o = (w.part - g * p.out_parts) * p.outw;
-                    const int groups = p.nparts / p.out_parts, tap = p.reverse ? p.K - 1 - w.tap : w.tap;
+                    if (w.first) {
+                        const int g = w.part / p.out_parts, o = (w.part - g * p.out_parts) * p.outw;
+                        column = g * p.inw, wx = p.transpose ? 0 : o, wy = g * p.C + (p.transpose ? o : 0);
+                    }
+                    const int k0 = w.q * 64, tap = p.reverse ? p.K - 1 - w.tap : w.tap;
                     s.x = (uint32_t)w.q << 9 | (w.has << 13) | (w.first ? STEP_FIRST : 0u);
-                    s.y = (uint32_t)(g * p.inw + w.q * 64);
-                    s.z = (uint32_t)(p.transpose ? w.q * 64 : o);
-                    s.w = (uint32_t)((tap * groups + g) * p.C + (p.transpose ? o : w.q * 64));
+                    s.y = (uint32_t)(column + k0);
+                    s.z = (uint32_t)(wx + (p.transpose ? k0 : 0));
+                    s.w = (uint32_t)(tap * tap_rows + wy + (p.transpose ? 0 : k0));
                 }
                 s_step[step.slot] = s;
-                mbar_arrive(full);
+                *(volatile uint32_t *)&s_word[word.slot] = s.x | ((word.turn + 1u) & 0x7fffu) << TURN_SHIFT;
+                if (more) {
+                    const uint32_t entry = rows0 + step.slot * ENTRY_BYTES;
+                    const int32_t *src = p.tile_rows + ((int64_t)w.block0 * p.K + w.tap) * ROWS;
+                    mbar_arrive_expect_tx(full, w.has == 3u ? ENTRY_BYTES : ENTRY_BYTES / 2);
+                    if (w.has & 1u) bulk_load(entry, src, ROWS * 4, full);
+                    if (w.has & 2u) bulk_load(entry + ROWS * 4, src + (int64_t)p.K * ROWS, ROWS * 4, full);
+                } else {
+                    mbar_arrive(full);
+                    ++ends;
+                }
+                step.next(AHEAD);
+                word.next(WORDS);
             }
-            cp_async_mbar_arrive(full);
-            step.next(AHEAD);
         }
-        cp_async_wait<0>();
+        __syncwarp();
     } else if (warp == WEIGHT_WARP) {
         // ---------------------------------------------------------------- weights ----
         Ring ring, step;
@@ -733,35 +758,41 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
         const uint64_t a_desc0 = smem_desc(slot0 + (uint32_t)t * SLOT_BYTES, 16, 1024);
         const uint64_t b_desc0 = p.transpose ? smem_desc(w0, 16, 1024) : smem_desc(w0, p.w_box_rows * 128, 1024);
         const uint32_t b_step = p.transpose ? 2u : 128u;   // 32 bytes along a K-major row / 16 contraction rows of 128 bytes
-        Ring ring, acc, step;
-        uint32_t started = 0;
-        bool open = false, ok = true;
-        for (;;) {
-            ok = wait(s_step_full[step.slot], step.turn);
-            if (!ok) break;
-            const uint32_t word = *(volatile uint32_t *)&s_step[step.slot].x;
-            if (word & STEP_END) break;
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&s_step_empty[step.slot]));
-            if (word & STEP_FIRST) {
-                if (open) {
-                    if (elect_one()) tc_commit(smem_u32(&s_acc_full[acc.slot]));
-                    acc.next(p.nacc);
+        if (elect_one()) {   // one thread from here on: no warp-wide votes or barriers in the chain
+            Ring ring, acc, step;
+            uint32_t started = 0;
+            bool open = false, ok = true;
+            auto peek = [&]() { return *(volatile uint32_t *)&s_word[step.slot]; };
+            uint32_t word = peek();
+            for (;;) {
+                // the step's word has been written for this turn of the ring (bounded as every wait)
+                for (uint64_t t0 = 0; ok && (word >> TURN_SHIFT) != ((step.turn + 1u) & 0x7fffu); word = peek()) {
+                    const uint64_t t = global_timer_ns();
+                    if (t0 == 0) t0 = t;
+                    if (s_abort || t - t0 > p.wait_limit_ns) {
+                        if (!s_abort) atomicOr(p.status, STATUS_BIT), *abort_flag = 1;
+                        ok = false;
+                    }
                 }
-                ok = wait(s_acc_empty[acc.slot], acc.turn ^ 1u);
+                if (!ok || (word & STEP_END)) break;
+                const uint32_t now = word;
+                step.next(WORDS);
+                word = peek();   // the next step's, most likely there already
+                if (now & STEP_FIRST) {
+                    if (open) tc_commit(smem_u32(&s_acc_full[acc.slot])), acc.next(p.nacc);
+                    ok = wait_one(s_acc_empty[acc.slot], acc.turn ^ 1u);
+                    if (!ok) break;
+                    open = true, started = 0;
+                }
+                ok = wait_one(s_full[ring.slot], ring.turn);
                 if (!ok) break;
-                open = true, started = 0;
-            }
-            ok = wait(s_full[ring.slot], ring.turn);
-            if (!ok) break;
-            if ((word >> (13 + t)) & 1u) {
-                fence_async_smem();   // the copies came through the generic proxy, the tensor core reads through the async proxy
-                tc_fence_after();
-                const uint64_t at = (uint64_t)(ring.slot * (p.slot_bytes >> 4));
-                const int ksteps = min(64, p.inw - (int)((word >> 9) & 15) * 64) >> 4;
-                const uint64_t ad = a_desc0 + at, bd = b_desc0 + at;
-                const uint32_t d = tmem + (acc.slot * 2 + (uint32_t)t) * p.col_stride;
-                if (elect_one()) {
+                if ((now >> (13 + t)) & 1u) {
+                    fence_async_smem();   // the copies came through the generic proxy, the tensor core reads through the async proxy
+                    tc_fence_after();
+                    const uint64_t at = (uint64_t)(ring.slot * (p.slot_bytes >> 4));
+                    const int ksteps = min(64, p.inw - (int)((now >> 9) & 15) * 64) >> 4;
+                    const uint64_t ad = a_desc0 + at, bd = b_desc0 + at;
+                    const uint32_t d = tmem + (acc.slot * 2 + (uint32_t)t) * p.col_stride;
                     tc_mma(d, ad, bd, idesc, started);
                     if (ksteps == 4) {
                         tc_mma(d, ad + 2, bd + b_step, idesc, 1u);
@@ -771,16 +802,14 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
                         for (int k = 1; k < ksteps; ++k) tc_mma(d, ad + (uint64_t)(2 * k), bd + (uint64_t)(b_step * k), idesc, 1u);
                     }
                     tc_commit(smem_u32(&s_empty[ring.slot]));
+                    started = 1u;
+                } else {
+                    mbar_arrive(smem_u32(&s_empty[ring.slot]));
                 }
-                started = 1u;
-            } else if (lane == 0) {
-                mbar_arrive(smem_u32(&s_empty[ring.slot]));
+                ring.next(p.nslots);
             }
-            __syncwarp();
-            ring.next(p.nslots);
-            step.next(AHEAD);
+            if (ok && open) tc_commit(smem_u32(&s_acc_full[acc.slot]));
         }
-        if (ok && open && elect_one()) tc_commit(smem_u32(&s_acc_full[acc.slot]));
         __syncwarp();
     }
     tc_fence_before();
@@ -1101,6 +1130,9 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
 
     // as many slots as fit: three of 64 KB at 256 output channels, five of 40 KB at 64
     p.nslots = (int)std::min<size_t>(MAX_SLOTS, ((size_t)232448 - 1024 - 1024 - AHEAD * ENTRY_BYTES) / p.slot_bytes);
+    // A team at step n has waited for the release of step n - teams - nslots, and its next wait names step n - nslots
+    // by the parity of its turn alone: with more teams than slots that could still be a turn further back.
+    p.teams = std::min(TEAMS, p.nslots);
     if (p.nslots < 2) PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_planned: shared memory does not fit (C=%d M=%d)", C, M);
     // the fp32 sums of a split rulebook lie behind the bucket sums; a caller that made no room for them gets one part
     const size_t sums_bytes = pcx_mvmr_planned_workspace_bytes(multi_buckets, p.in_pitch);
