@@ -22,18 +22,24 @@
 //   masks    the taps that touch a block: what the walk goes through, so no task lists are built
 //
 // Per call: a small kernel sums the rows of the multi-triplet buckets into the scratch (fp32 sum,
-// one rounding), then one persistent CTA per SM works off its steps (unit, slice, tap):
+// one rounding), then one persistent CTA per SM works off its steps (unit, 64-channel slice,
+// tap; of rows of 16 or 32 channels four or two taps fill a step):
 //
-//   walk warp        decides the steps and fetches the source rows of their two tiles into shared memory
+//   walk thread      decides the steps and fetches the source rows of their two tiles into shared memory
 //                    eight steps early.  The tables come from DRAM: looked up one step ahead, every step
 //                    waited out most of that latency and a tile took 1500 - 1800 clocks
-//   copy teams       two teams fill the A tiles, a step each in turn: 16-byte cp.async copies of the
+//   copy teams       up to four teams fill the A tiles, a step each in turn: 16-byte cp.async copies of the
 //                    tiles' source rows straight into the 128-byte-swizzled slot (rows without a source
-//                    are zero-filled by the same instruction with a source size of 0).  A copy loop alone
+//                    are zero-filled by the same instruction).  A copy loop alone
 //                    moves a 16 KB tile of random rows in 230 - 290 clocks (a TMA row gather, measured: 2260)
 //   weight warp      the 64-channel slice of W[tap] for both blocks, by TMA into the same slot
-//   MMA warps        one per block: one wait per step, up to four tcgen05.mma (M = 128, N = out_width)
+//   MMA threads      one per block: one wait per step, up to four tcgen05.mma (M = 128, N = out_width)
 //                    and one commit
+//
+// What bounds a step (two tiles) is neither memory (the same time with every row in L2) nor the tensor core but
+// the instruction chains of the roles, some 1000 clocks each: hence single threads without votes, more teams of
+// fewer warps, and several taps a step where rows are narrow.  Forward, 300k points with 22 triplets a row:
+// 32 -> 32 channels 84 -> 64 us, 64 -> 64 93 us, 128 -> 128 185 us; 80k points, kernel 5, 16 -> 32: 209 -> 89 us.
 //   epilogue warps   read TMEM (tcgen05.ld), round once and write each output row; up to 128 channels
 //                    the accumulators are double-buffered, so the next group is built meanwhile
 //
@@ -429,8 +435,9 @@ constexpr int COPY_WARP0 = EPI_WARPS, WALK_WARP = COPY_WARP0 + COPY_WARPS, WEIGH
 constexpr int THREADS = (MMA_WARP0 + GROUP_BLOCKS) * 32;
 constexpr int MAX_SLOTS = 8;
 constexpr int AHEAD = 8;                              // steps the walk runs ahead
-constexpr uint32_t ENTRY_BYTES = 2 * ROWS * 4;        // source rows of a step's two tiles
-// a step's word: slice << 9 | tiles that have the tap << 13 | first of its unit << 15 | end << 16
+constexpr uint32_t ENTRY_BYTES = 2 * ROWS * 4;        // source rows of a tap's two tiles
+// a step's word: per tap of the step, which of the two tiles have it | contraction steps of 16 << 8 | tiles that have
+// any << 13 | first of its unit << 15 | end << 16
 constexpr uint32_t STEP_FIRST = 1u << 15, STEP_END = 1u << 16;
 // The MMA threads read the words from a ring of their own, each marked with the turn of the ring it belongs to.
 // The walk is at most AHEAD steps ahead of the copies and these at most MAX_SLOTS ahead of the MMAs, so with
@@ -451,7 +458,8 @@ struct OsParams {
     int inw, outw, nkb, ngroups, nblocks, nsplit, mask_words;   // inw, outw: of a part
     int nparts, out_parts, in_pitch, out_pitch;   // parts of an output row: groups of the weight, each in out_parts
     int nslots, nacc, teams;
-    uint32_t slot_bytes, w_box_rows, w_tx_bytes, ncols, col_stride;
+    const uint16_t *weight;                 // read without the tensor map: transposed weights of a step of several taps
+    uint32_t slot_bytes, w_box_rows, w_rows, w_tx_bytes, ncols, col_stride;   // w_rows: of the weight slice of all taps of a step
     uint64_t wait_limit_ns;
 };
 
@@ -504,13 +512,24 @@ struct Walk {
         tap_lo = p.K * split / p.nsplit, tap_hi = p.K * (split + 1) / p.nsplit;
         return true;
     }
+    __device__ __forceinline__ void take() {
+        const int b = __ffs(left) - 1;
+        left &= left - 1;
+        tap = word * 32 + b;
+        has = ((m0 >> b) & 1u) | (((m1 >> b) & 1u) << 1);
+    }
+    __device__ __forceinline__ bool next_here() {   // another tap of the unit (of one slice)
+        while (!left) {
+            if (word + 1 >= p.mask_words) return false;
+            load(++word);
+        }
+        take();
+        return true;
+    }
     __device__ __forceinline__ bool next() {
         for (;;) {
             if (left) {
-                const int b = __ffs(left) - 1;
-                left &= left - 1;
-                tap = word * 32 + b;
-                has = ((m0 >> b) & 1u) | (((m1 >> b) & 1u) << 1);
+                take();
                 first = opened, opened = false;
                 return true;
             }
@@ -539,17 +558,22 @@ struct Ring {
     }
 };
 
+template <int PACK>   // taps of a step
 __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ OsParams p) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t s_full[MAX_SLOTS], s_empty[MAX_SLOTS], s_acc_full[2], s_acc_empty[2], s_step_full[AHEAD], s_step_empty[AHEAD];
     __shared__ uint32_t s_word[WORDS];
-    __shared__ uint4 s_step[AHEAD];   // the step's word, its first feature column, the corner of its weight slice
+    __shared__ uint4 s_step[AHEAD];   // the step's word, its first feature column, the column of its weights
+    constexpr int PIECE_SHIFT = PACK == 4 ? 1 : PACK == 2 ? 2 : 3;   // log2 of the 16-byte pieces a tap has of the 128-byte row of a tile
+    __shared__ int s_wrow[AHEAD * PACK];   // and, of each of its taps, the first row
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // a slot: the A tiles of the group's two blocks, then the weight slice both use; behind the slots the
     // source rows of the next steps
     const uint32_t slot0 = (smem_u32(smem_raw) + 1023u) & ~1023u, rows0 = slot0 + (uint32_t)p.nslots * p.slot_bytes;
+    const uint32_t entry_bytes = (uint32_t)PACK * ENTRY_BYTES;
+    const bool w_plain = PACK > 1 && p.transpose;
     volatile int *abort_flag = &s_abort;
     auto wait = [&](const uint64_t &bar, uint32_t parity) {   // the verdict is the same in the whole warp
         if (__all_sync(0xffffffffu, mbar_try_wait(smem_u32(&bar), parity & 1u))) return true;
@@ -562,7 +586,7 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
 
     if (tid == 0) {
         for (int s = 0; s < p.nslots; ++s)   // a team's copies and the weight slice; both MMA warps
-            mbar_init(smem_u32(&s_full[s]), TEAM_WARPS * 32 + 1), mbar_init(smem_u32(&s_empty[s]), GROUP_BLOCKS);
+            mbar_init(smem_u32(&s_full[s]), TEAM_WARPS * 32 + (w_plain ? 32 : 1)), mbar_init(smem_u32(&s_empty[s]), GROUP_BLOCKS);
         for (int s = 0; s < 2; ++s) mbar_init(smem_u32(&s_acc_full[s]), GROUP_BLOCKS), mbar_init(smem_u32(&s_acc_empty[s]), EPI_WARPS);
         for (int s = 0; s < WORDS; ++s) s_word[s] = 0u;
         for (int s = 0; s < AHEAD; ++s)   // the walk; a team and the weight warp
@@ -637,6 +661,7 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
         // tile, eight lanes a row, a group of eight lanes eight consecutive rows.
         const int team = (warp - COPY_WARP0) / TEAM_WARPS, piece = lane & 7;
         const int row0 = ((warp - COPY_WARP0) % TEAM_WARPS) * 32 + (lane >> 3) * 8;
+        const int tap_slot = piece >> PIECE_SHIFT, sub = piece & ((1 << PIECE_SHIFT) - 1);
         uint32_t dst_off[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k) dst_off[k] = (uint32_t)(row0 + k) * 128 + (uint32_t)((piece ^ k) << 4);
@@ -647,15 +672,14 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
             if (!wait(s_step_full[step.slot], step.turn)) break;
             const uint32_t word = *(volatile uint32_t *)&s_step[step.slot].x;
             if (word & STEP_END) break;
-            const uint32_t at = rows0 + step.slot * ENTRY_BYTES + (uint32_t)row0 * 4;
+            const uint32_t at = rows0 + step.slot * entry_bytes + (uint32_t)tap_slot * ENTRY_BYTES + (uint32_t)row0 * 4;
             const uint4 rows[4] = {lds_v4(at), lds_v4(at + 16), lds_v4(at + ROWS * 4), lds_v4(at + ROWS * 4 + 16)};
-            const uint32_t column = *(volatile uint32_t *)&s_step[step.slot].y + (uint32_t)piece * 8;
+            const uint32_t column = *(volatile uint32_t *)&s_step[step.slot].y + (uint32_t)sub * 8;
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&s_step_empty[step.slot]));
-            const int slice = (int)(word >> 9) & 15;
             const char *col = reinterpret_cast<const char *>(p.feat + column);
             const char *sums = reinterpret_cast<const char *>(p.scratch + column) - pitch;
-            const bool piece_ok = piece * 8 < p.inw - slice * 64;
+            const bool piece_ok = piece < 2 * (int)((word >> 8) & 7u);
             // the tensor core has finished with what was in the slot
             if (!wait(s_empty[ring.slot], ring.turn ^ 1u)) break;
             const uint32_t dst = slot0 + ring.slot * p.slot_bytes;
@@ -663,8 +687,11 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
 #pragma unroll
                 for (int t = 0; t < 2; ++t) {
                     if (!((word >> (13 + t)) & 1u)) continue;
-                    const int32_t rr[8] = {(int32_t)rows[2 * t].x, (int32_t)rows[2 * t].y, (int32_t)rows[2 * t].z, (int32_t)rows[2 * t].w,
-                                           (int32_t)rows[2 * t + 1].x, (int32_t)rows[2 * t + 1].y, (int32_t)rows[2 * t + 1].z, (int32_t)rows[2 * t + 1].w};
+                    const uint32_t none = PACK == 1 || ((word >> (2 * tap_slot + t)) & 1u) ? 0u : 0xffffffffu;   // the tile has other taps of the step
+                    const int32_t rr[8] = {(int32_t)(rows[2 * t].x | none), (int32_t)(rows[2 * t].y | none),
+                                           (int32_t)(rows[2 * t].z | none), (int32_t)(rows[2 * t].w | none),
+                                           (int32_t)(rows[2 * t + 1].x | none), (int32_t)(rows[2 * t + 1].y | none),
+                                           (int32_t)(rows[2 * t + 1].z | none), (int32_t)(rows[2 * t + 1].w | none)};
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
                         // a feature row x >= 0, the row of bucket sums -2 - x, or nothing (-1: zeros, and a source that is not read)
@@ -694,25 +721,33 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
                 if (more) more = w.next();
                 const uint32_t full = smem_u32(&s_step_full[step.slot]);
                 uint4 s = make_uint4(STEP_END, 0u, 0u, 0u);
+                uint32_t tx = 0;
                 if (more) {
                     if (w.first) {
                         const int g = w.part / p.out_parts, o = (w.part - g * p.out_parts) * p.outw;
                         column = g * p.inw, wx = p.transpose ? 0 : o, wy = g * p.C + (p.transpose ? o : 0);
                     }
-                    const int k0 = w.q * 64, tap = p.reverse ? p.K - 1 - w.tap : w.tap;
-                    s.x = (uint32_t)w.q << 9 | (w.has << 13) | (w.first ? STEP_FIRST : 0u);
+                    const int k0 = w.q * 64;
+                    uint32_t entry = rows0 + step.slot * entry_bytes, any = 0;
+                    s.x = w.first ? STEP_FIRST : 0u;
+                    int n = 0;
+                    do {
+                        const int32_t *src = p.tile_rows + ((int64_t)w.block0 * p.K + w.tap) * ROWS;
+                        const int tap = p.reverse ? p.K - 1 - w.tap : w.tap;
+                        if (w.has & 1u) bulk_load(entry, src, ROWS * 4, full);
+                        if (w.has & 2u) bulk_load(entry + ROWS * 4, src + (int64_t)p.K * ROWS, ROWS * 4, full);
+                        s_wrow[step.slot * PACK + n] = tap * tap_rows + wy + (p.transpose ? 0 : k0);
+                        s.x |= w.has << (2 * n), any |= w.has, tx += (w.has & 1u) + (w.has >> 1), entry += ENTRY_BYTES;
+                    } while (++n < PACK && w.next_here());
+                    s.x |= any << 13 | (uint32_t)(PACK > 1 ? n * p.inw : min(64, p.inw - k0)) >> 4 << 8;
                     s.y = (uint32_t)(column + k0);
                     s.z = (uint32_t)(wx + (p.transpose ? k0 : 0));
-                    s.w = (uint32_t)(tap * tap_rows + wy + (p.transpose ? 0 : k0));
+                    s.w = (uint32_t)n;
                 }
                 s_step[step.slot] = s;
                 *(volatile uint32_t *)&s_word[word.slot] = s.x | ((word.turn + 1u) & 0x7fffu) << TURN_SHIFT;
                 if (more) {
-                    const uint32_t entry = rows0 + step.slot * ENTRY_BYTES;
-                    const int32_t *src = p.tile_rows + ((int64_t)w.block0 * p.K + w.tap) * ROWS;
-                    mbar_arrive_expect_tx(full, w.has == 3u ? ENTRY_BYTES : ENTRY_BYTES / 2);
-                    if (w.has & 1u) bulk_load(entry, src, ROWS * 4, full);
-                    if (w.has & 2u) bulk_load(entry + ROWS * 4, src + (int64_t)p.K * ROWS, ROWS * 4, full);
+                    mbar_arrive_expect_tx(full, tx * (ROWS * 4));
                 } else {
                     mbar_arrive(full);
                     ++ends;
@@ -729,23 +764,41 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
             if (!wait(s_step_full[step.slot], step.turn)) break;
             const uint32_t word = *(volatile uint32_t *)&s_step[step.slot].x;
             if (word & STEP_END) break;
-            const int x = *(volatile int *)&s_step[step.slot].z, y = *(volatile int *)&s_step[step.slot].w;
+            const int x = *(volatile int *)&s_step[step.slot].z, taps = PACK > 1 ? *(volatile int *)&s_step[step.slot].w : 1;
+            int y[PACK];
+#pragma unroll
+            for (int n = 0; n < PACK; ++n) y[n] = *(volatile int *)&s_wrow[step.slot * PACK + n];
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&s_step_empty[step.slot]));
             if (!wait(s_empty[ring.slot], ring.turn ^ 1u)) break;
             const uint32_t dst = slot0 + ring.slot * p.slot_bytes + 2 * SLOT_BYTES, full = smem_u32(&s_full[ring.slot]);
-            if (lane == 0) {
-                mbar_arrive_expect_tx(full, p.w_tx_bytes);
+            if (w_plain) {   // a row (output channel) holds the contraction of all taps of the step: narrower than a box of the map can place
+                const int ppt = 1 << PIECE_SHIFT;
+#pragma unroll
+                for (int n = 0; n < PACK; ++n) {
+                    if (n >= taps) continue;
+                    for (int c = lane; c < p.outw * ppt; c += 32) {
+                        const int row = c >> PIECE_SHIFT, piece = c & (ppt - 1);
+                        cp_async16(dst + (uint32_t)row * 128 + (uint32_t)(((n * ppt + piece) ^ (row & 7)) << 4),
+                                   p.weight + (int64_t)(y[n] + row) * p.M + piece * 8);
+                    }
+                }
+                cp_async_mbar_arrive(full);
+            } else if (lane == 0) {
+                mbar_arrive_expect_tx(full, p.w_tx_bytes * (uint32_t)taps);
                 if (p.transpose) {   // contraction over m: an m-block of the output channels' rows
-                    tma_load_2d(dst, &tmap, x, y, full);
-                } else {             // contraction over c: 64 rows, one box per 64 output channels
-                    for (int mb = 0; mb * 64 < p.outw; ++mb)
-                        tma_load_2d(dst + (uint32_t)mb * p.w_box_rows * 128, &tmap, x + mb * 64, y, full);
+                    tma_load_2d(dst, &tmap, x, y[0], full);
+                } else {             // contraction over c: the rows of a 64-channel slice or of several taps, one box per 64 output channels
+#pragma unroll
+                    for (int n = 0; n < PACK; ++n)
+                        for (int mb = 0; n < taps && mb * 64 < p.outw; ++mb)
+                            tma_load_2d(dst + ((uint32_t)mb * p.w_rows + (uint32_t)n * p.w_box_rows) * 128, &tmap, x + mb * 64, y[n], full);
                 }
             }
             ring.next(p.nslots);
             step.next(AHEAD);
         }
+        cp_async_wait<0>();
     } else {
         // -------------------------------------------------------------------- MMA ----
         // One warp per block of the group: the issue of a step (waits, descriptors, four tcgen05.mma, commit) is a
@@ -756,7 +809,7 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
         // slot or step is an addition to the low word
         const uint32_t w0 = slot0 + 2 * SLOT_BYTES;
         const uint64_t a_desc0 = smem_desc(slot0 + (uint32_t)t * SLOT_BYTES, 16, 1024);
-        const uint64_t b_desc0 = p.transpose ? smem_desc(w0, 16, 1024) : smem_desc(w0, p.w_box_rows * 128, 1024);
+        const uint64_t b_desc0 = p.transpose ? smem_desc(w0, 16, 1024) : smem_desc(w0, p.w_rows * 128, 1024);
         const uint32_t b_step = p.transpose ? 2u : 128u;   // 32 bytes along a K-major row / 16 contraction rows of 128 bytes
         if (elect_one()) {   // one thread from here on: no warp-wide votes or barriers in the chain
             Ring ring, acc, step;
@@ -790,7 +843,7 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
                     fence_async_smem();   // the copies came through the generic proxy, the tensor core reads through the async proxy
                     tc_fence_after();
                     const uint64_t at = (uint64_t)(ring.slot * (p.slot_bytes >> 4));
-                    const int ksteps = min(64, p.inw - (int)((now >> 9) & 15) * 64) >> 4;
+                    const int ksteps = (int)((now >> 8) & 7u);
                     const uint64_t ad = a_desc0 + at, bd = b_desc0 + at;
                     const uint32_t d = tmem + (acc.slot * 2 + (uint32_t)t) * p.col_stride;
                     tc_mma(d, ad, bd, idesc, started);
@@ -1109,9 +1162,15 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     p.nacc = 4 * p.col_stride <= 512 ? 2 : 1;   // up to 128 channels the next group starts while the last one is written
     p.ncols = 32;
     while (p.ncols < 2u * (uint32_t)p.nacc * p.col_stride) p.ncols <<= 1;
+    // A step costs its chain of waits, copies and MMA issue, some 1000 clocks, whatever the width: rows of 16 or 32
+    // channels fill the 64 of a step with four or two taps.
+    const int pack = inw == 16 ? 4 : inw == 32 ? 2 : 1;
+    p.weight = (const uint16_t *)d_weight;
     p.w_box_rows = (uint32_t)(transpose ? p.outw : std::min(64, C));
-    p.w_tx_bytes = (transpose ? 1u : (uint32_t)((p.outw + 63) / 64)) * p.w_box_rows * 128u;
-    p.slot_bytes = 2 * SLOT_BYTES + (uint32_t)align_up(p.w_tx_bytes, 1024);
+    p.w_rows = transpose ? p.w_box_rows : p.w_box_rows * (uint32_t)pack;
+    const uint32_t boxes = transpose ? 1u : (uint32_t)((p.outw + 63) / 64);
+    p.w_tx_bytes = boxes * p.w_box_rows * 128u;
+    p.slot_bytes = 2 * SLOT_BYTES + (uint32_t)align_up((size_t)boxes * p.w_rows * 128u, 1024);
     p.wait_limit_ns = wait_limit();
     if (!encode_tiled()) PCX_FAIL(PCX_E_LAUNCH, "pcx_mvmr_planned: the driver offers no cuTensorMapEncodeTiled");
 
@@ -1129,7 +1188,7 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     if (r != CUDA_SUCCESS) PCX_FAIL(PCX_E_LAUNCH, "pcx_mvmr_planned: cuTensorMapEncodeTiled failed (%d)", (int)r);
 
     // as many slots as fit: three of 64 KB at 256 output channels, five of 40 KB at 64
-    p.nslots = (int)std::min<size_t>(MAX_SLOTS, ((size_t)232448 - 1024 - 1024 - AHEAD * ENTRY_BYTES) / p.slot_bytes);
+    p.nslots = (int)std::min<size_t>(MAX_SLOTS, ((size_t)232448 - 1024 - 1024 - AHEAD * pack * ENTRY_BYTES) / p.slot_bytes);
     // A team at step n has waited for the release of step n - teams - nslots, and its next wait names step n - nslots
     // by the parity of its turn alone: with more teams than slots that could still be a turn further back.
     p.teams = std::min(TEAMS, p.nslots);
@@ -1139,13 +1198,15 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     p.nsplit = split_parts(pv.ngroups, K, nparts);
     if (p.nsplit > 1 && (!d_ws || ws_bytes < sums_bytes + partial_bytes(n_out, p.out_pitch, p.nsplit))) p.nsplit = 1;
     p.partial = p.nsplit > 1 ? (float *)((char *)d_ws + sums_bytes) : nullptr;
-    const size_t smem = 1024 + (size_t)p.nslots * p.slot_bytes + AHEAD * ENTRY_BYTES;
-    static int granted[64] = {};
+    const size_t smem = 1024 + (size_t)p.nslots * p.slot_bytes + AHEAD * pack * ENTRY_BYTES;
+    auto kernel = pack == 4 ? mvmr_os_kernel<4> : pack == 2 ? mvmr_os_kernel<2> : mvmr_os_kernel<1>;
+    static int granted[3][64] = {};
     int dev = 0;
     PCX_CUDA(cudaGetDevice(&dev));
-    if ((int)smem > granted[dev & 63]) {
-        PCX_CUDA(cudaFuncSetAttribute(mvmr_os_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        granted[dev & 63] = (int)smem;
+    int &most = granted[pack >> 1][dev & 63];
+    if ((int)smem > most) {
+        PCX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        most = (int)smem;
     }
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(pv.ngroups * p.nsplit * nparts, num_sms()));
     if (multi_buckets > 0) {
@@ -1156,7 +1217,7 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
         PCX_LAUNCH_CHECK();
     }
     prof_begin(transpose ? "mvmr_os_kernel(dgrad)" : "mvmr_os_kernel(fwd)", stream);
-    mvmr_os_kernel<<<grid, THREADS, smem, stream>>>(tmap, p);
+    kernel<<<grid, THREADS, smem, stream>>>(tmap, p);
     prof_end(stream);
     PCX_LAUNCH_CHECK();
     if (p.nsplit > 1) {

@@ -38,6 +38,9 @@ CASES = [  # n_out, n_in, K, T, G, C, M, dtype
     (300, 300, 27, 3000, 2, 3, 10, torch.float16),
     (200, 220, 27, 4000, 4, 16, 320, torch.bfloat16),
     (80000, 80000, 27, 500000, 1, 32, 48, torch.bfloat16),
+    (40000, 40000, 27, 600000, 1, 256, 256, torch.bfloat16),   # fewer slots than copy teams, many steps a block
+    (20001, 20000, 125, 600000, 1, 5, 32, torch.bfloat16),     # steps of four taps, of two on the way back
+    (3000, 3000, 70, 60000, 2, 32, 16, torch.float16),         # steps that end in a part of their taps
 ]
 
 
