@@ -463,11 +463,6 @@ struct OsParams {
     uint64_t wait_limit_ns;
 };
 
-__device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
-    uint4 v;
-    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-    return v;
-}
 __device__ __forceinline__ float bias_at(const uint16_t *b, int c, int fmt) {
     const uint16_t v = __ldg(b + c);
     return fmt ? __bfloat162float(__ushort_as_bfloat16(v)) : __half2float(__ushort_as_half(v));
@@ -545,16 +540,6 @@ struct Walk {
                 load(0);
             }
         }
-    }
-};
-
-struct Ring {
-    uint32_t slot = 0, turn = 0;   // slot, and how often the ring has gone round
-    __device__ __forceinline__ void next(int depth) {
-        if (++slot == (uint32_t)depth) slot = 0, ++turn;
-    }
-    __device__ __forceinline__ void skip(int by, int depth) {
-        for (slot += (uint32_t)by; slot >= (uint32_t)depth; ++turn) slot -= (uint32_t)depth;
     }
 };
 
@@ -962,7 +947,6 @@ int split_parts(int64_t ngroups, int K, int nparts) {
 
 // Output rows wider than the tensor memory's two accumulators (256 channels), and those of a grouped
 // weight, are worked off in parts of the same width.
-int parts_of(int width) { return (width + 255) / 256; }
 
 size_t partial_bytes(int64_t n_out, int outw, int splits) {
     return splits > 1 ? (size_t)splits * ((n_out + ROWS - 1) / ROWS) * ROWS * outw * sizeof(float) : 0;

@@ -107,6 +107,10 @@ int vvor_generic(const VvorArgs &a, cudaStream_t stream);
 int clear_accumulator(float *acc, const void *bias, int64_t rows, int width, int dtype, cudaStream_t stream);
 int round_accumulator(const float *acc, void *out, int64_t n, int dtype, cudaStream_t stream);
 
+// Rows wider than 256 channels go through the tensor engines in equal parts of at most 256.
+inline int parts_of(int width) { return (width + 255) / 256; }
+inline bool splits_evenly(int width) { return width >= 16 && width % (16 * parts_of(width)) == 0; }
+
 bool mvmr_tensor_supported(const MvmrArgs &a);
 bool vvor_tensor_supported(const VvorArgs &a);
 int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream);

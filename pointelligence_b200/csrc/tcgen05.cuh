@@ -131,6 +131,21 @@ __device__ __forceinline__ void bulk_load(uint32_t dst, const void *src, uint32_
 __device__ __forceinline__ void tma_prefetch_desc(const void *tmap) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
 }
+__device__ __forceinline__ uint4 lds_v4(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+// Place in a ring of slots that producers and consumers go round.
+struct Ring {
+    uint32_t slot = 0, turn = 0;   // slot, and how often the ring has gone round
+    __device__ __forceinline__ void next(int depth) {
+        if (++slot == (uint32_t)depth) slot = 0, ++turn;
+    }
+    __device__ __forceinline__ void skip(int by, int depth) {
+        for (slot += (uint32_t)by; slot >= (uint32_t)depth; ++turn) slot -= (uint32_t)depth;
+    }
+};
 // true in one thread of a converged warp
 __device__ __forceinline__ bool elect_one() {
     uint32_t p;

@@ -1,0 +1,299 @@
+// VVOR on sm_100a (tcgen05 + TMEM): the gradient of the weights.
+//
+//   D[Ma x Cb] += X[t x Ma]^T * G[t x Cb], t = triplets of a chunk; both operands MN-major (a gathered row
+//   is contiguous along M / N, the triplet index is the contraction), accumulated in TMEM over all chunks of
+//   a tap and added to the fp32 sums in global memory once per (CTA, tap).
+//
+// A persistent CTA per SM owns a contiguous range of chunks of tap-sorted triplets.  Its warps play roles, so
+// that index fetch, row copies, multiplies and the writing of a finished tap run at the same time:
+//
+//   index warp     the index rows of a chunk, up to eight chunks early
+//   copy teams     up to four; a team gathers the rows of a chunk with 16-byte cp.async copies straight into the
+//                  128-byte-swizzled tiles ([64-channel block][row][128 bytes]) of a slot
+//   MMA thread     up to CHR / 16 steps of tcgen05.mma per 128 rows of D
+//   flush warps    read a finished tap from TMEM and add it to global memory; up to 256 columns of
+//                  accumulators are double-buffered, so the next tap starts meanwhile
+//
+// Bound by what the L2 gives to gathers of whole rows, below 64 channels by the chain of a chunk (waits, copies,
+// MMA issue).  Before, the same warps did every step of a chunk, with a block barrier a chunk and the smaller chunks
+// several CTAs an SM leave room for; before and now, 300k points, 6.6 M triplets: 64 x 64 186 -> 148 us, 128 x 128 385 -> 294, 256 x 256 1042 -> 718
+// (11.3, 11.4 and 9.4 TB/s of gathered rows); 150k points, 0.98 M: 42 -> 34, 76 -> 54, 178 -> 120 us.
+//
+// Every wait is bounded (one second) and abortable: a role that gives up raises a flag in the status word and
+// in shared memory, the other roles leave their waits, and the CTA frees its TMEM and returns.
+#include "sparse_kernels.cuh"
+#include "tcgen05.cuh"
+
+namespace pcx {
+int device_status_address(unsigned int **d_status);
+
+namespace {
+
+using namespace tc;
+
+constexpr unsigned STATUS_BIT = 2u;
+constexpr int MAX_PARTS = 64;        // (group, part, part) combinations of one launch
+constexpr int MAX_TAPS_SMEM = 1024;  // taps whose chunk table fits the shared-memory copy
+constexpr int FLUSH_WARPS = 4, TEAMS = 4, TEAM_WARPS = 4;
+constexpr int COPY_WARP0 = FLUSH_WARPS, INDEX_WARP = COPY_WARP0 + TEAMS * TEAM_WARPS, MMA_WARP = INDEX_WARP + 1;
+constexpr int THREADS = (MMA_WARP + 1) * 32;
+constexpr int MAX_SLOTS = 6, AHEAD = 8;   // chunks whose rows / whose indices are in shared memory
+
+struct VvorTcParams {
+    const uint16_t *a, *b;  // (n_a, Ma), (n_b, Cb)
+    const int32_t *a_idx, *b_idx;
+    const int64_t *seg;
+    float *acc;             // (n_o, G, rows of Cb)
+    unsigned int *status;
+    int64_t a_pitch, b_pitch, acc_pitch, acc_tap;   // rows of a / b / one tap's sums, elements of one tap's sums
+    int a_parts, b_parts;                           // blockIdx.y: (group, part of a, part of b)
+    int n_o, Ma, Cb, fmt, nslots, nacc, teams;      // Ma, Cb: the part's
+    uint32_t ncols, acc_cols;
+};
+
+// The rows of a chunk of one operand that this lane copies: CHR / 16 consecutive rows from `row0` on, a 16-byte
+// piece of each 64-channel block of a row.  Rows from `rows` up to a multiple of 16 are zeros.
+template <int CHR>
+__device__ __forceinline__ void copy_operand(uint32_t tile, const uint16_t *src, uint32_t pitch_bytes, uint32_t idx, int row0,
+                                             int rows, int piece, int pieces) {
+    if (piece >= pieces) return;
+    const char *col = reinterpret_cast<const char *>(src + piece * 8);
+    const int blocks = (pieces - piece + 7) >> 3, end = (rows + 15) & ~15;
+#pragma unroll
+    for (int q = 0; q < CHR / 64; ++q) {
+        const int r = row0 + 4 * q;
+        if (r >= end) return;
+        const uint4 i4 = lds_v4(idx + (uint32_t)r * 4);
+        const uint32_t at[4] = {i4.x, i4.y, i4.z, i4.w};
+        const char *s[4];
+        uint32_t dst[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            s[k] = col + (uint64_t)(r + k < rows ? at[k] : 0u) * pitch_bytes;
+            dst[k] = tile + (uint32_t)(r + k) * 128 + (uint32_t)((piece ^ ((r + k) & 7)) << 4);
+        }
+        for (int c = 0;;) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) cp_async16_or_zero(dst[k], s[k], r + k >= rows);
+            if (++c == blocks) break;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) dst[k] += CHR * 128, s[k] += 128;
+        }
+    }
+}
+
+template <int CHR>   // triplets of a chunk: the contraction of one slot
+__global__ void __launch_bounds__(THREADS, 1) vvor_tc_kernel(VvorTcParams p) {
+    constexpr uint32_t BLK = CHR * 128;   // one 64-channel block of a tile
+    using Cursor = ChunkCursorT<CHR>;
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t s_full[MAX_SLOTS], s_empty[MAX_SLOTS], s_acc_full[2], s_acc_empty[2], s_idx_full[AHEAD], s_idx_empty[AHEAD];
+    __shared__ uint32_t s_tmem;
+    __shared__ int s_abort;
+    __shared__ int32_t s_warp_sums[THREADS / 32];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    {
+        const int bp = (int)blockIdx.y % p.b_parts, ap = (int)blockIdx.y / p.b_parts % p.a_parts,
+                  g = (int)blockIdx.y / (p.b_parts * p.a_parts);
+        p.a += ((int64_t)g * p.a_parts + ap) * p.Ma;
+        p.b += ((int64_t)g * p.b_parts + bp) * p.Cb;
+        p.acc += ((int64_t)g * p.a_parts + ap) * p.Ma * p.acc_pitch + bp * p.Cb;
+    }
+    const int row_tiles = (p.Ma + 127) >> 7;
+    const int ablk = (p.Ma + 63) >> 6, bblk = (p.Cb + 63) >> 6;   // an odd ablk borrows the next block as padding
+    const uint32_t slot_bytes = (uint32_t)(ablk + bblk) * BLK;
+    // behind the slots: the index rings of both operands, then the chunk table
+    const uint32_t idx0 = base + (uint32_t)p.nslots * slot_bytes;
+    int32_t *s_cum = reinterpret_cast<int32_t *>(smem_raw + (idx0 - smem_u32(smem_raw)) + 2 * AHEAD * CHR * 4);
+    volatile int *abort_flag = &s_abort;
+    auto wait_one = [&](const uint64_t &bar, uint32_t parity) {
+        return mbar_wait_abortable(smem_u32(&bar), parity & 1u, STATUS_BIT, p.status, abort_flag);
+    };
+    auto wait = [&](const uint64_t &bar, uint32_t parity) {   // the verdict is the same in the whole warp
+        if (__all_sync(0xffffffffu, mbar_try_wait(smem_u32(&bar), parity & 1u))) return true;
+        return __all_sync(0xffffffffu, wait_one(bar, parity)) != 0;
+    };
+
+    if (tid == 0) {
+        for (int s = 0; s < p.nslots; ++s) mbar_init(smem_u32(&s_full[s]), TEAM_WARPS * 32), mbar_init(smem_u32(&s_empty[s]), 1);
+        for (int s = 0; s < 2; ++s) mbar_init(smem_u32(&s_acc_full[s]), 1), mbar_init(smem_u32(&s_acc_empty[s]), FLUSH_WARPS);
+        for (int s = 0; s < AHEAD; ++s) mbar_init(smem_u32(&s_idx_full[s]), 32), mbar_init(smem_u32(&s_idx_empty[s]), TEAM_WARPS);
+        fence_mbar_init();
+        s_abort = 0;
+    }
+    if (warp == 0) tmem_alloc(smem_u32(&s_tmem), p.ncols);
+    build_chunk_table<CHR>(p.seg, p.n_o, s_cum, s_warp_sums);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = s_tmem;
+
+    const int total = s_cum[p.n_o];
+    const int per = (total + gridDim.x - 1) / gridDim.x;
+    const int lo = blockIdx.x * per, hi = min(total, lo + per);
+    Cursor cur;
+    if (lo < hi) cur.seek(s_cum, p.seg, p.n_o, lo);
+
+    if (lo >= hi) {
+    } else if (warp < FLUSH_WARPS) {
+        // ----------------------------------------------------------------- flush ----
+        // a warp reads the 32 TMEM lanes of its quarter
+        Ring acc;
+        for (int tap = cur.tap; tap < p.n_o && s_cum[tap] < hi; ++tap) {
+            if (s_cum[tap + 1] == s_cum[tap]) continue;
+            if (!wait(s_acc_full[acc.slot], acc.turn)) break;
+            tc_fence_after();
+            float *dst = p.acc + tap * p.acc_tap;
+            for (int rt = 0; rt < row_tiles; ++rt) {
+#pragma unroll 1
+                for (int half = 0; half < 2; ++half) {
+                    const int m0 = rt * 128 + warp * 32 + half * 16;
+                    if (m0 >= p.Ma) break;
+                    const int ma = m0 + (lane >> 2), mb = ma + 8;
+                    const int64_t da = ma < p.Ma ? ma : -1, db = mb < p.Ma ? mb : -1;
+                    for (int c0 = 0; c0 < p.Cb; c0 += 64) {
+                        float v[32];
+                        tmem_ld_16x64(tmem + ((uint32_t)(warp * 32 + half * 16) << 16) + acc.slot * p.acc_cols + (uint32_t)(rt * p.Cb + c0), v);
+                        scatter_block(dst, da, db, p.Cb, p.acc_pitch, c0, lane, v);
+                    }
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&s_acc_empty[acc.slot]));
+            acc.next(p.nacc);
+        }
+    } else if (warp < INDEX_WARP) {
+        // ---------------------------------------------------------------- copies ----
+        const int team = (warp - COPY_WARP0) / TEAM_WARPS, piece = lane & 7;
+        const int row0 = ((warp - COPY_WARP0) % TEAM_WARPS) * (CHR / 4) + (lane >> 3) * (CHR / 16);
+        Ring ring, idx;
+        ring.skip(team, p.nslots), idx.skip(team, AHEAD);
+        if (team < p.teams) {
+            for (int chunk = lo + team; chunk < hi; chunk += p.teams) {
+                cur.advance(s_cum, p.seg, p.n_o, chunk);
+                const int rows = cur.rows(chunk);
+                if (!wait(s_idx_full[idx.slot], idx.turn) || !wait(s_empty[ring.slot], ring.turn ^ 1u)) break;
+                const uint32_t tile = base + ring.slot * slot_bytes, ia = idx0 + idx.slot * (CHR * 4);
+                copy_operand<CHR>(tile, p.a, (uint32_t)p.a_pitch * 2u, ia, row0, rows, piece, p.Ma >> 3);
+                copy_operand<CHR>(tile + (uint32_t)ablk * BLK, p.b, (uint32_t)p.b_pitch * 2u, ia + AHEAD * CHR * 4, row0, rows, piece, p.Cb >> 3);
+                cp_async_mbar_arrive(smem_u32(&s_full[ring.slot]));   // fires once this thread's copies have landed
+                __syncwarp();
+                if (lane == 0) mbar_arrive(smem_u32(&s_idx_empty[idx.slot]));
+                ring.skip(p.teams, p.nslots);
+                idx.skip(p.teams, AHEAD);
+            }
+        }
+        cp_async_wait<0>();
+    } else if (warp == INDEX_WARP) {
+        // --------------------------------------------------------------- indices ----
+        Ring idx;
+        for (int chunk = lo; chunk < hi; ++chunk) {
+            cur.advance(s_cum, p.seg, p.n_o, chunk);
+            const int rows = cur.rows(chunk);
+            const int64_t first = cur.first(chunk);
+            if (!wait(s_idx_empty[idx.slot], idx.turn ^ 1u)) break;
+            const uint32_t ia = idx0 + idx.slot * (CHR * 4);
+#pragma unroll 4
+            for (int r = lane; r < rows; r += 32) {
+                cp_async4(ia + (uint32_t)r * 4, p.a_idx + first + r);
+                cp_async4(ia + (uint32_t)(AHEAD * CHR + r) * 4, p.b_idx + first + r);
+            }
+            cp_async_mbar_arrive(smem_u32(&s_idx_full[idx.slot]));
+            idx.next(AHEAD);
+        }
+        cp_async_wait<0>();
+    } else {
+        // ------------------------------------------------------------------- MMA ----
+        if (elect_one()) {
+            const uint32_t idesc = instr_desc(p.fmt, 128, p.Cb, 1, 1);
+            const uint64_t ad0 = smem_desc(base, BLK, 1024), bd0 = smem_desc(base + (uint32_t)ablk * BLK, BLK, 1024);
+            Ring ring, acc;
+            bool fresh = true;   // the next multiply starts a tap
+            for (int chunk = lo; chunk < hi; ++chunk) {
+                cur.advance(s_cum, p.seg, p.n_o, chunk);
+                const int ksteps = (cur.rows(chunk) + 15) >> 4;
+                if (fresh && !wait_one(s_acc_empty[acc.slot], acc.turn ^ 1u)) break;
+                if (!wait_one(s_full[ring.slot], ring.turn)) break;
+                fence_async_smem();   // the copies came through the generic proxy, the tensor core reads through the async proxy
+                tc_fence_after();
+                const uint64_t at = (uint64_t)(ring.slot * (slot_bytes >> 4));   // (descriptor addresses count 16 bytes)
+                for (int rt = 0; rt < row_tiles; ++rt) {
+                    const uint32_t d = tmem + acc.slot * p.acc_cols + (uint32_t)(rt * p.Cb);
+                    const uint64_t ad = ad0 + at + (uint64_t)(rt * 2) * (BLK >> 4), bd = bd0 + at;
+                    for (int s = 0; s < ksteps; ++s) tc_mma(d, ad + (uint64_t)(s * 128), bd + (uint64_t)(s * 128), idesc, fresh && s == 0 ? 0u : 1u);
+                }
+                tc_commit(smem_u32(&s_empty[ring.slot]));
+                ring.next(p.nslots);
+                fresh = chunk + 1 == hi || cur.last_of_tap(chunk);
+                if (fresh) tc_commit(smem_u32(&s_acc_full[acc.slot])), acc.next(p.nacc);
+            }
+        }
+        __syncwarp();
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem, p.ncols);
+}
+
+template <int CHR>
+int launch_vvor(VvorTcParams &p, int parts, int64_t T, size_t block_rows, cudaStream_t stream) {
+    const size_t slot = block_rows * CHR * 128;
+    const size_t rest = 1024 + 2 * AHEAD * CHR * 4 + align_up((size_t)(p.n_o + 1) * 4, 16);   // alignment, index rings, chunk table
+    p.nslots = (int)std::min<size_t>(MAX_SLOTS, ((size_t)232448 - 1024 - rest) / slot);
+    if (p.nslots < 2) PCX_FAIL(PCX_E_UNSUPPORTED, "vvor tensor kernel does not fit (Ma=%d Cb=%d)", p.Ma, p.Cb);
+    p.teams = std::min(TEAMS, p.nslots);   // a wait names its turn by parity: no team may be a whole ring ahead of another
+    const size_t smem = rest + p.nslots * slot;
+    static int granted[64] = {};   // per device
+    int dev = 0;
+    PCX_CUDA(cudaGetDevice(&dev));
+    if ((int)smem > granted[dev & 63]) {
+        PCX_CUDA(cudaFuncSetAttribute(vvor_tc_kernel<CHR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        granted[dev & 63] = (int)smem;
+    }
+    const dim3 grid((unsigned)std::min<int64_t>(T / CHR + p.n_o + 1, std::max(1, num_sms() / parts)), (unsigned)parts);
+    prof_begin("vvor_tc_kernel", stream);
+    vvor_tc_kernel<CHR><<<grid, THREADS, smem, stream>>>(p);
+    prof_end(stream);
+    PCX_LAUNCH_CHECK();
+    return PCX_OK;
+}
+
+}  // namespace
+
+bool vvor_tensor_supported(const VvorArgs &a) {
+    if (a.dtype != PCX_F16 && a.dtype != PCX_BF16) return false;
+    if (!a.seg_offs || a.T <= 0 || a.n_o > MAX_TAPS_SMEM) return false;
+    if (!splits_evenly(a.Ma) || !splits_evenly(a.Cb) || (int64_t)a.G * parts_of(a.Ma) * parts_of(a.Cb) > MAX_PARTS) return false;
+    if ((uintptr_t)a.a % 16 || (uintptr_t)a.b % 16) return false;
+    return a.T / 64 + a.n_o < INT32_MAX;
+}
+
+int vvor_tensor(const VvorArgs &a, cudaStream_t stream) {
+    VvorTcParams p = {};
+    p.a = (const uint16_t *)a.a, p.b = (const uint16_t *)a.b, p.a_idx = a.a_idx, p.b_idx = a.b_idx;
+    p.seg = a.seg_offs, p.acc = a.acc;
+    p.a_parts = parts_of(a.Ma), p.b_parts = parts_of(a.Cb);
+    const int parts = a.G * p.a_parts * p.b_parts;
+    p.Ma = a.Ma / p.a_parts, p.Cb = a.Cb / p.b_parts;   // the part's widths
+    p.a_pitch = (int64_t)a.G * a.Ma, p.b_pitch = (int64_t)a.G * a.Cb, p.acc_pitch = a.Cb, p.acc_tap = (int64_t)a.G * a.Ma * a.Cb;
+    p.n_o = (int)a.n_o, p.fmt = a.dtype == PCX_BF16 ? 1 : 0;
+    if (int rc = device_status_address(&p.status)) return rc;
+    p.acc_cols = (uint32_t)(((p.Ma + 127) / 128 - 1) * p.Cb + (p.Cb + 63) / 64 * 64);   // flushed in blocks of 64 columns
+    p.nacc = 2 * p.acc_cols <= 512 ? 2 : 1;
+    p.ncols = 32;
+    while (p.ncols < (uint32_t)p.nacc * p.acc_cols) p.ncols <<= 1;
+    // Slots of up to 64 KB: the chain of a chunk (waits, copies, MMA issue, some 1000 clocks whatever its size) stays
+    // below the time its copies take, and three slots fit (64 x 64, 6.6 M triplets: chunks of 64 / 128 / 256 triplets
+    // 299 / 197 / 148 us).  Few triplets: shorter chunks, so that every SM has some.
+    const size_t blocks = (size_t)((p.Ma + 63) / 64 + (p.Cb + 63) / 64);
+    const int64_t ctas = std::max(1, num_sms() / parts);
+    int chr = blocks <= 2 ? 256 : blocks <= 4 ? 128 : 64;
+    while (chr > 64 && a.T < 4 * ctas * chr) chr /= 2;
+    if (chr == 256) return launch_vvor<256>(p, parts, a.T, blocks, stream);
+    if (chr == 128) return launch_vvor<128>(p, parts, a.T, blocks, stream);
+    return launch_vvor<64>(p, parts, a.T, blocks, stream);
+}
+
+}  // namespace pcx

@@ -139,3 +139,24 @@ def test_plan_of_rows_out_of_order_inside_a_tap():
     assert torch.equal(a["tile_rows"] < -1, b["tile_rows"] < -1) and torch.equal(a["tile_rows"].clamp_min(-1), b["tile_rows"].clamp_min(-1))
     w, x = torch.randn(K, 1, 64, 64, device=DEV).bfloat16() / 8, torch.randn(n, 64, device=DEV).bfloat16()
     assert _rel(_cabi.mvmr_planned(w, x, counted, False), _cabi.mvmr_planned(w, x, sorted_, False).double()) < TOL[torch.bfloat16]
+
+
+@pytest.mark.parametrize("Ma,Cb", [(16, 16), (64, 64), (96, 160), (256, 256)])
+@pytest.mark.parametrize("scale", [1, 16])
+def test_weight_gradient_at_the_edges_of_chunks(Ma, Cb, scale):
+    """Taps of no, one, and around a multiple of 16 / 64 / 256 triplets, between taps of many chunks (which are
+    longer where the rulebook is); fp32 sums of exact products, rounded once."""
+    from pointelligence_b200 import _cabi
+
+    sizes = [0, 1, 15, 16, 17, 0, 63, 64, 65, 255, 256, 257, 12000 * scale, 3, 0, 127 * scale, 128, 129, 0]
+    seg = torch.tensor([0] + sizes, device=DEV).cumsum(0)
+    T, n = int(seg[-1]), 3001
+    g = torch.Generator(device=DEV).manual_seed(9)
+    ai, bi = (torch.randint(0, n, (T,), device=DEV, generator=g).int() for _ in range(2))
+    a, b = (torch.randn(n, 1, c, device=DEV, generator=g).to(torch.bfloat16) for c in (Ma, Cb))
+    out = _cabi.vvor(a, ai, b, bi, seg, None, len(sizes))
+    ref = torch.zeros(len(sizes), 1, Ma, Cb, dtype=torch.float64, device=DEV)
+    for k in range(len(sizes)):
+        s, e = int(seg[k]), int(seg[k + 1])
+        ref[k, 0] = a[ai[s:e].long(), 0].double().T @ b[bi[s:e].long(), 0].double()
+        assert _rel(out[k], ref[k]) < TOL[torch.bfloat16], k
