@@ -342,70 +342,106 @@ __global__ void plan_entries_kernel(const uint32_t *__restrict__ key_sorted, con
 // scratch[b] = sum of the feature rows of bucket b (fp32 sum in entry order, one rounding); one thread
 // per 16-byte piece.  The row indices of up to four members are fetched together and their pieces
 // together after that, so that a bucket costs two memory latencies instead of two per member.
-// The element format and, for the usual row widths, the pieces per row are compile-time values: the
-// first version of this kernel spent most of its instructions on a 64-bit division of the thread
-// index and on per-element format branches (749 M warp instructions for 9 M buckets, issue-bound
-// at 28 % of the DRAM bandwidth).
+// Half of its time went to issuing instructions, so: the format is a compile-time value, sums go two to an instruction,
+// the first two members (every bucket here has them) need no test and no zeros to start from.
+struct Sum8 {
+    uint64_t v[4];   // two floats each
+};
 template <int FMT>
-__device__ __forceinline__ void add_piece(float (&acc)[8], uint4 v) {
-    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+__device__ __forceinline__ Sum8 widen(uint4 p) {
+    const uint32_t w[4] = {p.x, p.y, p.z, p.w};
+    Sum8 s;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         float2 f;
         if (FMT) f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&w[q]));
         else f = __half22float2(*reinterpret_cast<const __half2 *>(&w[q]));
-        acc[2 * q] += f.x, acc[2 * q + 1] += f.y;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(s.v[q]) : "f"(f.x), "f"(f.y));
     }
+    return s;
+}
+__device__ __forceinline__ void add(Sum8 &s, const Sum8 &t) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(s.v[q]) : "l"(t.v[q]));
 }
 
-constexpr int BUCKET_SUM_THREADS = 256;
+constexpr int BUCKET_SUM_THREADS = 256, SLICE_PASSES = 2;
 
-// PPR: 16-byte pieces per row when that is a power of two (2 .. 32), else 0 (taken from inw).
-// (Two pieces per thread were tried: fewer instructions per byte, but fewer resident warps, and slower.)
-template <int FMT, int PPR>
+// LANES: threads of a bucket, a 16-byte piece each; PASSES: buckets a thread sums one after the other.
+// Bound by the latencies of the gathers and by what L1 and L2 hold, not by DRAM.  300k points, 22 triplets a row:
+// 64 channels 146 -> 132 us, 128 267 -> 242, 192 500 -> 377, 256 520 -> 474.  Tried, and slower or no faster: two
+// pieces per thread; loads that bypass the L1 (256 channels: 516 -> 625); more resident warps (623); 1024-thread or
+// looping blocks, so that an SM works on neighbouring buckets (515 - 600).
+template <int FMT, int LANES, int PASSES>
 __global__ void __launch_bounds__(BUCKET_SUM_THREADS) bucket_sum_kernel(const uint16_t *__restrict__ feat,
                                                                         const uint2 *__restrict__ entries,
                                                                         const uint2 *__restrict__ buckets,
                                                                         const uint32_t *__restrict__ ctrl, int inw,
                                                                         uint16_t *scratch) {
-    const unsigned ppr = PPR ? (unsigned)PPR : (unsigned)inw >> 3;
-    const unsigned per_block = BUCKET_SUM_THREADS / ppr;
-    const unsigned local = threadIdx.x / ppr, piece = threadIdx.x - local * ppr;
-    const unsigned b = blockIdx.x * per_block + local;
-    if (local >= per_block || b >= ctrl[CTRL_NMULTI]) return;
-    const uint2 bk = __ldg(buckets + b);
-    const uint16_t *col = feat + piece * 8;
-    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    for (uint32_t m0 = 0; m0 < bk.y; m0 += 4) {
-        uint32_t rows[4];
+    constexpr unsigned AT_ONCE = BUCKET_SUM_THREADS / LANES;
+    const unsigned piece = blockIdx.y * LANES + threadIdx.x % LANES, pitch = (unsigned)inw * 2u, nmulti = ctrl[CTRL_NMULTI];
+    if (piece * 16 >= pitch) return;
+    const char *col = reinterpret_cast<const char *>(feat + piece * 8);
+    unsigned b = blockIdx.x * (AT_ONCE * PASSES) + threadIdx.x / LANES;
+    for (int pass = 0; pass < PASSES && b < nmulti; ++pass, b += AT_ONCE) {
+        const uint2 bk = __ldg(buckets + b);
+        const uint2 *entry = entries + bk.x;
+        auto row = [&](uint32_t m) { return m < bk.y ? __ldg(&entry[m].y) : 0u; };
+        auto piece_of = [&](uint32_t r) { return __ldg(reinterpret_cast<const uint4 *>(col + (uint64_t)r * pitch)); };
+        const uint32_t r0 = __ldg(&entry[0].y), r1 = __ldg(&entry[1].y), r2 = row(2), r3 = row(3);
+        const uint4 v0 = piece_of(r0), v1 = piece_of(r1);
+        uint4 v2 = make_uint4(0, 0, 0, 0), v3 = v2;
+        if (bk.y > 2) v2 = piece_of(r2);
+        if (bk.y > 3) v3 = piece_of(r3);
+        Sum8 sum = widen<FMT>(v0);
+        add(sum, widen<FMT>(v1));
+        if (bk.y > 2) add(sum, widen<FMT>(v2));
+        if (bk.y > 3) add(sum, widen<FMT>(v3));
+        for (uint32_t m0 = 4; m0 < bk.y; m0 += 4) {
+            uint32_t rows[4];
+            uint4 v[4];
 #pragma unroll
-        for (int m = 0; m < 4; ++m) rows[m] = m0 + m < bk.y ? __ldg(&entries[bk.x + m0 + m].y) : 0u;
-        uint4 v[4];
+            for (int m = 0; m < 4; ++m) rows[m] = row(m0 + m);
 #pragma unroll
-        for (int m = 0; m < 4; ++m)
-            v[m] = m0 + m < bk.y ? __ldg(reinterpret_cast<const uint4 *>(col + (size_t)rows[m] * (unsigned)inw)) : make_uint4(0, 0, 0, 0);
+            for (int m = 0; m < 4; ++m) v[m] = m0 + m < bk.y ? piece_of(rows[m]) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) add_piece<FMT>(acc, v[m]);   // an absent member adds zeros
+            for (int m = 0; m < 4; ++m) add(sum, widen<FMT>(v[m]));   // an absent member adds zeros
+        }
+        float acc[8];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[2 * q]), "=f"(acc[2 * q + 1]) : "l"(sum.v[q]));
+        uint4 o;
+        o.x = pack2(acc[0], acc[1], FMT), o.y = pack2(acc[2], acc[3], FMT);
+        o.z = pack2(acc[4], acc[5], FMT), o.w = pack2(acc[6], acc[7], FMT);
+        // past the L2's share of the feature rows: the sums are read once, by the next kernel
+        __stcs(reinterpret_cast<uint4 *>(reinterpret_cast<char *>(scratch + piece * 8) + (uint64_t)b * pitch), o);
     }
-    uint4 o;
-    o.x = pack2(acc[0], acc[1], FMT), o.y = pack2(acc[2], acc[3], FMT);
-    o.z = pack2(acc[4], acc[5], FMT), o.w = pack2(acc[6], acc[7], FMT);
-    *reinterpret_cast<uint4 *>(scratch + (size_t)b * (unsigned)inw + piece * 8) = o;
 }
 
 template <int FMT>
 void launch_bucket_sum(int64_t multi, int inw, const uint16_t *feat, const uint2 *entries, const uint2 *buckets,
                        const uint32_t *ctrl, uint16_t *scratch, cudaStream_t stream) {
+    // A power of two of pieces up to 32: a thread each.  Other widths in slices, blockIdx.y: a bucket costs a warp
+    // about the same whatever its lanes do, and 24 pieces left some idle.  96 and 112 channels: 16 lanes, of which a
+    // quarter idle at most (96 channels: 211 us; slices of 4 lanes 230, rows of 12 lanes 248).
     const int ppr = inw >> 3;
-    const unsigned grid = (unsigned)((multi + BUCKET_SUM_THREADS / ppr - 1) / (BUCKET_SUM_THREADS / ppr));
-#define PCX_BS(P) bucket_sum_kernel<FMT, P><<<grid, BUCKET_SUM_THREADS, 0, stream>>>(feat, entries, buckets, ctrl, inw, scratch)
-    switch (ppr) {
-        case 2: PCX_BS(2); break;
-        case 4: PCX_BS(4); break;
-        case 8: PCX_BS(8); break;
-        case 16: PCX_BS(16); break;
-        case 32: PCX_BS(32); break;
-        default: PCX_BS(0); break;
+    const bool whole = ppr <= 32 && (ppr & (ppr - 1)) == 0;
+    const int lanes = whole ? ppr : ppr % 8 == 0 ? 8 : ppr == 12 || ppr == 14 ? 16 : 4, passes = whole ? 1 : SLICE_PASSES;
+    const int per_block = BUCKET_SUM_THREADS / lanes * passes;
+    const dim3 grid((unsigned)((multi + per_block - 1) / per_block), (unsigned)((ppr + lanes - 1) / lanes));
+#define PCX_BS(L, P) bucket_sum_kernel<FMT, L, P><<<grid, BUCKET_SUM_THREADS, 0, stream>>>(feat, entries, buckets, ctrl, inw, scratch)
+    if (!whole) {
+        if (lanes == 8) PCX_BS(8, SLICE_PASSES);
+        else if (lanes == 16) PCX_BS(16, SLICE_PASSES);
+        else PCX_BS(4, SLICE_PASSES);
+        return;
+    }
+    switch (lanes) {
+        case 2: PCX_BS(2, 1); break;
+        case 4: PCX_BS(4, 1); break;
+        case 8: PCX_BS(8, 1); break;
+        case 16: PCX_BS(16, 1); break;
+        default: PCX_BS(32, 1); break;
     }
 #undef PCX_BS
 }
