@@ -185,7 +185,10 @@ int pcx_mvmr_plan_build(const int32_t *d_scatter, const int32_t *d_gather,
 /* ... and the number of buckets with several triplets, for which both build
  * entries synchronise `stream`.  Rulebooks whose rows ascend inside every tap
  * (what pcx_radius_taps_fill emits) are regrouped by counting, others by
- * sorting their triplets. */
+ * sorting their triplets.  With `h_multi` null the caller vouches that the
+ * rows ascend: nothing is waited for, the count appears in 32-bit word
+ * PCX_PLAN_MULTI_WORD of the plan, and min(T / 2, n_out * K) bounds it. */
+#define PCX_PLAN_MULTI_WORD 4
 int pcx_mvmr_plan_build_counted(const int32_t *d_scatter,
                                 const int32_t *d_gather,
                                 const int64_t *d_seg_offs, int64_t T, int K,

@@ -382,11 +382,23 @@ class MvmrPlan:
     one direction (which index is scattered) and one ``group_blocks`` value.
     """
 
-    __slots__ = ("buffer", "T", "K", "n_out", "group_blocks", "multi_buckets", "__weakref__")
+    __slots__ = ("buffer", "T", "K", "n_out", "group_blocks", "_multi", "_word", "_stream", "__weakref__")
 
-    def __init__(self, buffer, T, K, n_out, group_blocks, multi_buckets):
+    def __init__(self, buffer, T, K, n_out, group_blocks, multi, word=None, stream=None):
         self.buffer, self.T, self.K, self.n_out, self.group_blocks = buffer, T, K, n_out, group_blocks
-        self.multi_buckets = multi_buckets   # (row, tap) buckets with several triplets
+        self._multi, self._word, self._stream = multi, word, stream
+
+    @property
+    def multi_buckets(self):
+        """(row, tap) buckets with several triplets; a bound while the plan of an ordered rulebook is being built."""
+        if self._word is not None:
+            n = host().peek(self._word)
+            if n < 0 and torch.cuda.current_stream(self.buffer.device) != self._stream:
+                torch.cuda.synchronize(self.buffer.device)   # another stream than the one that waits for the plan
+                n = host().peek(self._word)
+            if n >= 0:
+                self._multi, self._word = n, None
+        return self._multi
 
     def views(self):
         """The plan's arrays as tensors (for tests): perm, tile_offs, entries (T, 2), group_order."""
@@ -442,35 +454,47 @@ def mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks):
     """Build the plan of a tap-sorted rulebook: ``scatter`` indexes the rows that are summed
     into (n_out of them), ``gather`` the rows that are read."""
     require_cuda(scatter, gather, seg_offs)
-    buf, multi = host().plan_build(scatter, gather, seg_offs, int(K), int(n_out), int(group_blocks))
-    return MvmrPlan(buf, scatter.numel(), int(K), int(n_out), int(group_blocks), multi)
+    T = scatter.numel()
+    ordered = T <= _NO_WAIT_TRIPLETS and _built(scatter, gather) is not None
+    buf, multi, word = host().plan_build(scatter, gather, seg_offs, int(K), int(n_out), int(group_blocks), ordered)
+    return MvmrPlan(buf, T, int(K), int(n_out), int(group_blocks), multi, word)
 
+
+# Rulebooks of the geometry path up to this size get their plan without a wait (150 us each where a network of
+# 40 000 points builds eleven per pass).  Until the count of multi-triplet buckets has arrived, passes reserve scratch
+# for its bound, half the triplets: at 2^20 triplets and 256 channels 256 MB.
+_NO_WAIT_TRIPLETS = 1 << 20
 
 _PLAN_CACHE = {}
 _PLAN_CACHE_MAX = 64
-_SYMMETRIC = {}
+_BUILT = {}
 
 
-def mark_symmetric(i, j):
-    """Record that the rulebook ``(i, j, k)`` these index tensors belong to is its own mirror image:
-    with ``(i, j, k)`` it holds ``(j, i, K - 1 - k)``.  True for a self-search (queries are the points):
+def mark_built(i, j, symmetric):
+    """Record that ``(i, j, k)`` come from the geometry path: i ascends inside every tap.  ``symmetric``: the
+    rulebook these index tensors belong to is its own mirror image: with ``(i, j, k)`` it holds ``(j, i, K - 1 - k)``.  True for a self-search (queries are the points):
     the distance is symmetric and the tap of the opposite offset is the mirrored tap.  The input
     gradient of such a layer is then a forward pass over the SAME rulebook with the taps of the
     weight reversed, so it needs no plan of its own (``tig_grad_input``).  Remembered by tensor
     identity, like the plans."""
     import weakref
 
-    for key in [key for key, (refs, _) in _SYMMETRIC.items() if any(r() is None for r in refs)]:
-        _SYMMETRIC.pop(key, None)
-    _SYMMETRIC[(i.data_ptr(), j.data_ptr(), i.numel())] = ((weakref.ref(i), weakref.ref(j)), (i._version, j._version))
+    for key in [key for key, (refs, _, _) in _BUILT.items() if any(r() is None for r in refs)]:
+        _BUILT.pop(key, None)
+    _BUILT[(i.data_ptr(), j.data_ptr(), i.numel())] = ((weakref.ref(i), weakref.ref(j)), (i._version, j._version), bool(symmetric))
+
+
+def _built(i, j):
+    """None for a rulebook the geometry path did not build (or that was written to since), else whether it is symmetric."""
+    hit = _BUILT.get((i.data_ptr(), j.data_ptr(), i.numel()))
+    if hit is None:
+        return None
+    refs, stamp, symmetric = hit
+    return symmetric if refs[0]() is i and refs[1]() is j and stamp == (i._version, j._version) else None
 
 
 def is_symmetric(i, j):
-    hit = _SYMMETRIC.get((i.data_ptr(), j.data_ptr(), i.numel()))
-    if hit is None or os.environ.get("PCX_SYMMETRIC_DGRAD", "1") == "0":
-        return False
-    refs, stamp = hit
-    return refs[0]() is i and refs[1]() is j and stamp == (i._version, j._version)
+    return bool(_built(i, j)) and os.environ.get("PCX_SYMMETRIC_DGRAD", "1") != "0"
 
 
 def cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks):
@@ -487,6 +511,7 @@ def cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks):
         if old_stamp == stamp and all(r() is t for r, t in zip(refs, (scatter, gather, seg_offs))):
             return value
     value = mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks)
+    value._stream = torch.cuda.current_stream(scatter.device)
     for k in [k for k, (refs, _, _) in _PLAN_CACHE.items() if any(r() is None for r in refs)]:
         _PLAN_CACHE.pop(k, None)
     if len(_PLAN_CACHE) >= _PLAN_CACHE_MAX:
@@ -569,7 +594,7 @@ def _differentiable_backward(weight, feat, grad, i, j, seg_offs, n_out, n_in, K,
 
 def prepare_mvmr(weight, gather, scatter, seg_offs, n_out, transpose=False):
     """Build (and cache) now what ``mvmr`` with the automatic engine would build on its first call
-    for this rulebook -- the plan of the output-stationary kernel, whose construction ends with a
+    for this rulebook -- the plan of the output-stationary kernel, whose construction may end with a
     host hand-over -- so that the feature pass itself is kernels only.  Returns True when a plan
     was prepared, False when the policy keeps the scatter engines (which need no preparation)."""
     K, G, C, M = weight.shape

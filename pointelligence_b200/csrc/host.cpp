@@ -493,9 +493,11 @@ std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor> grid_sample(const Te
     return {indices, out, sample_ ? OptTensor(out_sample) : std::nullopt, want_mapping ? OptTensor(mapping) : std::nullopt, sizes};
 }
 
-// (plan buffer, number of buckets with several triplets)
-std::tuple<Tensor, int64_t> plan_build(const Tensor &scatter_, const Tensor &gather_, const Tensor &seg_, int64_t K, int64_t n_out,
-                                       int64_t group) {
+// (plan buffer, number of buckets with several triplets, null or a page-locked word).  A rulebook whose rows are known
+// to ascend inside every tap needs no wait: the number is a bound then, and the true one replaces the word's -1 when the
+// plan is ready.
+std::tuple<Tensor, int64_t, OptTensor> plan_build(const Tensor &scatter_, const Tensor &gather_, const Tensor &seg_, int64_t K,
+                                                  int64_t n_out, int64_t group, bool ordered) {
     require_cuda(scatter_), require_cuda(gather_), require_cuda(seg_);
     c10::cuda::CUDAGuard guard(scatter_.device());
     const Tensor scatter = as_i32(scatter_), gather = as_i32(gather_), seg = as_i64(seg_);
@@ -508,9 +510,14 @@ std::tuple<Tensor, int64_t> plan_build(const Tensor &scatter_, const Tensor &gat
     }
     Tensor buf = workspace(bytes, scatter), ws = workspace(pcx_mvmr_plan_workspace_bytes(T, n_out, (int)K, (int)group), scatter);
     int64_t multi = 0;
+    ordered = ordered && T > 0 && c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None;
     check(pcx_mvmr_plan_build_counted(ptr_as<int32_t>(scatter), ptr_as<int32_t>(gather), ptr_as<int64_t>(seg), T, (int)K, n_out, (int)group,
-                                      ptr(buf), buf.numel(), ptr(ws), ws.numel(), &multi, stream()));
-    return {buf, multi};
+                                      ptr(buf), buf.numel(), ptr(ws), ws.numel(), ordered ? nullptr : &multi, stream()));
+    if (!ordered) return {buf, multi, std::nullopt};
+    Tensor word = at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    *static_cast<volatile int32_t *>(word.data_ptr<int32_t>()) = -1;
+    word.copy_(buf.narrow(0, 4 * PCX_PLAN_MULTI_WORD, 4).view(at::kInt), true);
+    return {buf, std::min(T / 2, n_out * K), word};
 }
 
 Tensor planned(const Tensor &weight, const Tensor &feat, const Tensor &buffer, int64_t group, int64_t multi, int64_t T, int64_t n_out,
@@ -565,6 +572,7 @@ PYBIND11_MODULE(_pcx_host, m) {
     m.def("layer_norm_backward", &layer_norm_backward);
     m.def("radius_taps", &radius_taps, py::call_guard<py::gil_scoped_release>());
     m.def("grid_sample", &grid_sample, py::call_guard<py::gil_scoped_release>());
+    m.def("peek", [](const Tensor &word) { return (int64_t)*static_cast<volatile int32_t *>(word.data_ptr<int32_t>()); });
     m.def("plan_build", &plan_build, py::call_guard<py::gil_scoped_release>());
     m.def("planned", &planned);
 }

@@ -70,7 +70,7 @@ constexpr unsigned STATUS_BIT = 4u;   // bit of the device status word this kern
 constexpr unsigned PLAN_MAGIC = 0x70637832u;
 
 // control words at the head of a plan
-enum { CTRL_MAGIC = 2, CTRL_GROUP = 3, CTRL_NMULTI = 4, CTRL_UNSORTED = 5, CTRL_WORDS = 64 };
+enum { CTRL_MAGIC = 2, CTRL_GROUP = 3, CTRL_NMULTI = PCX_PLAN_MULTI_WORD, CTRL_UNSORTED = 5, CTRL_WORDS = 64 };
 
 struct PlanView {
     uint32_t *ctrl;        // CTRL_WORDS
@@ -1046,7 +1046,7 @@ int pcx_mvmr_plan_build_counted(const int32_t *d_scatter, const int32_t *d_gathe
     if (!plan_sizes_ok(T, n_out, K, G))
         PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_plan_build: sizes out of range (T=%lld n_out=%lld K=%d group=%d)", (long long)T,
                  (long long)n_out, K, G);
-    if (!d_plan || !d_ws || !h_multi || (T > 0 && (!d_scatter || !d_gather || !d_seg_offs)))
+    if (!d_plan || !d_ws || (T > 0 && (!d_scatter || !d_gather || !d_seg_offs)))
         PCX_FAIL(PCX_E_ARG, "pcx_mvmr_plan_build: null pointer");
     if ((uintptr_t)d_plan % 256 || (uintptr_t)d_ws % 256)
         PCX_FAIL(PCX_E_ALIGN, "pcx_mvmr_plan_build: plan and workspace must be 256-byte aligned");
@@ -1089,6 +1089,7 @@ int pcx_mvmr_plan_build_counted(const int32_t *d_scatter, const int32_t *d_gathe
         PCX_LAUNCH_CHECK();
     }
     if (int rc = order_groups(pv, w, K, G, stream)) return rc;
+    if (!h_multi) return PCX_OK;   // rows ascend inside every tap: the caller says so
     uint32_t *h = reinterpret_cast<uint32_t *>(handover_words());
     PCX_CUDA(cudaMemcpyAsync(h, pv.ctrl, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, stream));
     PCX_CUDA(cudaStreamSynchronize(stream));

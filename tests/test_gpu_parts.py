@@ -160,3 +160,32 @@ def test_weight_gradient_at_the_edges_of_chunks(Ma, Cb, scale):
         s, e = int(seg[k]), int(seg[k + 1])
         ref[k, 0] = a[ai[s:e].long(), 0].double().T @ b[bi[s:e].long(), 0].double()
         assert _rel(out[k], ref[k]) < TOL[torch.bfloat16], k
+
+
+@pytest.mark.parametrize("n", [300, 5000])
+def test_plan_of_a_geometry_built_rulebook_is_not_waited_for(n):
+    """The plan whose bucket count arrives later, used at once, later and on another stream, gives the bits of the
+    plan that was waited for."""
+    from pointelligence_b200 import _cabi
+    from pointelligence_b200.layers.triplets import build_triplets_segmented
+
+    g = torch.Generator(device=DEV).manual_seed(n)
+    pts = torch.rand(n, 3, device=DEV, generator=g) * n ** (1 / 3)
+    inds, sizes = torch.zeros(n, dtype=torch.int32, device=DEV), torch.tensor([n], device=DEV)
+    i, j, k, seg, _ = build_triplets_segmented(pts, inds, sizes, 1.5, 3, radius_scaler=2.5)
+    want = _cabi.mvmr_plan(i.clone(), j.clone(), seg, 27, n, 2)
+    assert want._word is None and want.multi_buckets > 0
+    w, x = torch.randn(27, 1, 64, 64, device=DEV).bfloat16() / 8, torch.randn(n, 64, device=DEV).bfloat16()
+    ref = _cabi.mvmr_planned(w, x, want, False)
+    torch.cuda.synchronize()
+    plan = _cabi.cached_mvmr_plan(i, j, seg, 27, n, 2)
+    assert want.multi_buckets <= plan.multi_buckets <= i.numel() // 2
+    assert torch.equal(_cabi.mvmr_planned(w, x, plan, False), ref)
+    fresh = _cabi.cached_mvmr_plan(i, j, seg.clone(), 27, n, 2)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        assert fresh.multi_buckets == want.multi_buckets
+        assert torch.equal(_cabi.mvmr_planned(w, x, fresh, False), ref)
+    side.synchronize()
+    torch.cuda.synchronize()
+    assert plan.multi_buckets == want.multi_buckets and plan._word is None
