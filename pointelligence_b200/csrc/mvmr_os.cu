@@ -891,27 +891,31 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
     if (warp == 0) tmem_dealloc(tmem, p.ncols);
 }
 
-// out[perm[slot]] = the parts of a split group added in order, plus the bias, rounded once
+// out[perm[slot]] = the parts of a split group added in order, plus the bias, rounded once.  Small outputs, so bound
+// by latency: four columns a thread, the loads of REDUCE_BATCH parts in flight together.
+constexpr int REDUCE_BATCH = 9;
 __global__ void os_reduce_kernel(const float *__restrict__ partial, const int32_t *__restrict__ perm, const uint16_t *__restrict__ bias,
                                  int64_t slots, int outw, int nsplit, int fmt, uint16_t *out) {
-    const int ppr = outw >> 3;
+    const int ppr = outw >> 2;
     const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= slots * ppr) return;
     const int64_t slot = x / ppr;
-    const int c = (int)(x - slot * ppr) * 8;
+    const int c = (int)(x - slot * ppr) * 4;
     const int32_t row = perm[slot];
     if (row < 0) return;
-    float v[8];
+    float v[4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = bias ? bias_at(bias, c + e, fmt) : 0.f;
-#pragma unroll 4
-    for (int s = 0; s < nsplit; ++s) {
-        const float4 *src = reinterpret_cast<const float4 *>(partial + ((int64_t)s * slots + slot) * outw + c);
-        const float4 a = __ldcs(src), b = __ldcs(src + 1);
-        v[0] += a.x, v[1] += a.y, v[2] += a.z, v[3] += a.w, v[4] += b.x, v[5] += b.y, v[6] += b.z, v[7] += b.w;
+    for (int e = 0; e < 4; ++e) v[e] = bias ? bias_at(bias, c + e, fmt) : 0.f;
+    const float *src = partial + slot * outw + c;
+    for (int s0 = 0; s0 < nsplit; s0 += REDUCE_BATCH) {
+        float4 a[REDUCE_BATCH];
+#pragma unroll
+        for (int s = 0; s < REDUCE_BATCH; ++s)
+            a[s] = s0 + s < nsplit ? __ldcs(reinterpret_cast<const float4 *>(src + (s0 + s) * slots * outw)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < REDUCE_BATCH; ++s) v[0] += a[s].x, v[1] += a[s].y, v[2] += a[s].z, v[3] += a[s].w;
     }
-    *reinterpret_cast<uint4 *>(out + (int64_t)row * outw + c) =
-        make_uint4(pack2(v[0], v[1], fmt), pack2(v[2], v[3], fmt), pack2(v[4], v[5], fmt), pack2(v[6], v[7], fmt));
+    *reinterpret_cast<uint2 *>(out + (int64_t)row * outw + c) = make_uint2(pack2(v[0], v[1], fmt), pack2(v[2], v[3], fmt));
 }
 
 // A single thread waits on an mbarrier that nothing arrives at: the bounded wait runs out,
@@ -1243,7 +1247,7 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     PCX_LAUNCH_CHECK();
     if (p.nsplit > 1) {
         const int64_t slots = pv.nblocks * ROWS;
-        os_reduce_kernel<<<(unsigned)((slots * (p.out_pitch / 8) + 255) / 256), 256, 0, stream>>>(p.partial, p.perm, p.bias, slots, p.out_pitch, p.nsplit,
+        os_reduce_kernel<<<(unsigned)((slots * (p.out_pitch / 4) + 255) / 256), 256, 0, stream>>>(p.partial, p.perm, p.bias, slots, p.out_pitch, p.nsplit,
                                                                                            p.fmt, p.out);
         PCX_LAUNCH_CHECK();
     }
