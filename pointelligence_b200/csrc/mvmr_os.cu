@@ -649,10 +649,11 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
                     }
                     if (row >= 0) {
                         if (p.nsplit > 1) {
-                            float4 *dst = reinterpret_cast<float4 *>(
-                                p.partial + ((int64_t)w.split * p.nblocks * ROWS + slot) * p.out_pitch + col0 + c0);
+                            // [split][block][four columns][row]: the lanes of a warp write next to each other
+                            float4 *dst = reinterpret_cast<float4 *>(p.partial + ((int64_t)w.split * p.nblocks + w.block0 + b) * ROWS * p.out_pitch) +
+                                          ((col0 + c0) >> 2) * ROWS + warp * 32 + lane;
 #pragma unroll
-                            for (int e = 0; e < 4; ++e) dst[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
+                            for (int e = 0; e < 4; ++e) dst[e * ROWS] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
                         } else {
                             if (p.bias) {
 #pragma unroll
@@ -892,30 +893,36 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
 }
 
 // out[perm[slot]] = the parts of a split group added in order, plus the bias, rounded once.  Small outputs, so bound
-// by latency: four columns a thread, the loads of REDUCE_BATCH parts in flight together.
+// by latency: eight columns a thread, the loads of REDUCE_BATCH parts in flight together.
 constexpr int REDUCE_BATCH = 9;
-__global__ void os_reduce_kernel(const float *__restrict__ partial, const int32_t *__restrict__ perm, const uint16_t *__restrict__ bias,
-                                 int64_t slots, int outw, int nsplit, int fmt, uint16_t *out) {
-    const int ppr = outw >> 2;
-    const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= slots * ppr) return;
-    const int64_t slot = x / ppr;
-    const int c = (int)(x - slot * ppr) * 4;
-    const int32_t row = perm[slot];
+__global__ void __launch_bounds__(128) os_reduce_kernel(const float *__restrict__ partial, const int32_t *__restrict__ perm,
+                                                        const uint16_t *__restrict__ bias, int64_t slots, int outw, int nsplit, int fmt,
+                                                        uint16_t *out) {
+    // a block of threads: the rows of a block of the plan, eight columns
+    const int64_t block = blockIdx.x;
+    const int c = (int)blockIdx.y * 8, lane = threadIdx.x;
+    const int32_t row = perm[block * ROWS + lane];
     if (row < 0) return;
-    float v[4];
+    float v[8];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) v[e] = bias ? bias_at(bias, c + e, fmt) : 0.f;
-    const float *src = partial + slot * outw + c;
+    for (int e = 0; e < 8; ++e) v[e] = bias ? bias_at(bias, c + e, fmt) : 0.f;
+    const float4 *src = reinterpret_cast<const float4 *>(partial + block * ROWS * outw) + (c >> 2) * ROWS + lane;
+    const int64_t part = slots * (outw >> 2);
     for (int s0 = 0; s0 < nsplit; s0 += REDUCE_BATCH) {
-        float4 a[REDUCE_BATCH];
+        float4 a[REDUCE_BATCH][2];
 #pragma unroll
         for (int s = 0; s < REDUCE_BATCH; ++s)
-            a[s] = s0 + s < nsplit ? __ldcs(reinterpret_cast<const float4 *>(src + (s0 + s) * slots * outw)) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int s = 0; s < REDUCE_BATCH; ++s) v[0] += a[s].x, v[1] += a[s].y, v[2] += a[s].z, v[3] += a[s].w;
+            for (int h = 0; h < 2; ++h)
+                a[s][h] = s0 + s < nsplit ? __ldcs(src + (s0 + s) * part + h * ROWS) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int s = 0; s < REDUCE_BATCH; ++s)
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                v[4 * h] += a[s][h].x, v[4 * h + 1] += a[s][h].y, v[4 * h + 2] += a[s][h].z, v[4 * h + 3] += a[s][h].w;
     }
-    *reinterpret_cast<uint2 *>(out + (int64_t)row * outw + c) = make_uint2(pack2(v[0], v[1], fmt), pack2(v[2], v[3], fmt));
+    *reinterpret_cast<uint4 *>(out + (int64_t)row * outw + c) =
+        make_uint4(pack2(v[0], v[1], fmt), pack2(v[2], v[3], fmt), pack2(v[4], v[5], fmt), pack2(v[6], v[7], fmt));
 }
 
 // A single thread waits on an mbarrier that nothing arrives at: the bounded wait runs out,
@@ -1247,8 +1254,8 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     PCX_LAUNCH_CHECK();
     if (p.nsplit > 1) {
         const int64_t slots = pv.nblocks * ROWS;
-        os_reduce_kernel<<<(unsigned)((slots * (p.out_pitch / 4) + 255) / 256), 256, 0, stream>>>(p.partial, p.perm, p.bias, slots, p.out_pitch, p.nsplit,
-                                                                                           p.fmt, p.out);
+        os_reduce_kernel<<<dim3((unsigned)pv.nblocks, (unsigned)(p.out_pitch / 8)), ROWS, 0, stream>>>(p.partial, p.perm, p.bias, slots, p.out_pitch,
+                                                                                                     p.nsplit, p.fmt, p.out);
         PCX_LAUNCH_CHECK();
     }
     return PCX_OK;
