@@ -486,7 +486,7 @@ struct OsParams {
     const uint16_t *feat, *bias;            // rows of in_pitch elements; bias: added before the rounding; null: none
     const uint16_t *scratch;                // sums of the multi-triplet buckets
     uint16_t *out;
-    float *partial;                         // nsplit > 1: [split][nblocks * ROWS][outw]
+    float *partial;                         // nsplit > 1: [split][nblocks][row of out_pitch / 4][ROWS] float4
     const int32_t *perm, *group_order, *tile_rows;
     const uint32_t *tap_masks;
     unsigned int *status;
@@ -893,36 +893,29 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
 }
 
 // out[perm[slot]] = the parts of a split group added in order, plus the bias, rounded once.  Small outputs, so bound
-// by latency: eight columns a thread, the loads of REDUCE_BATCH parts in flight together.
+// by latency: four columns a thread, the loads of REDUCE_BATCH parts in flight together.
 constexpr int REDUCE_BATCH = 9;
 __global__ void __launch_bounds__(128) os_reduce_kernel(const float *__restrict__ partial, const int32_t *__restrict__ perm,
                                                         const uint16_t *__restrict__ bias, int64_t slots, int outw, int nsplit, int fmt,
                                                         uint16_t *out) {
-    // a block of threads: the rows of a block of the plan, eight columns
+    // a block of threads: the rows of a block of the plan, four columns
     const int64_t block = blockIdx.x;
-    const int c = (int)blockIdx.y * 8, lane = threadIdx.x;
+    const int c = (int)blockIdx.y * 4, lane = threadIdx.x;
     const int32_t row = perm[block * ROWS + lane];
     if (row < 0) return;
-    float v[8];
+    float v[4];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) v[e] = bias ? bias_at(bias, c + e, fmt) : 0.f;
+    for (int e = 0; e < 4; ++e) v[e] = bias ? bias_at(bias, c + e, fmt) : 0.f;
     const float4 *src = reinterpret_cast<const float4 *>(partial + block * ROWS * outw) + (c >> 2) * ROWS + lane;
     const int64_t part = slots * (outw >> 2);
     for (int s0 = 0; s0 < nsplit; s0 += REDUCE_BATCH) {
-        float4 a[REDUCE_BATCH][2];
+        float4 a[REDUCE_BATCH];
 #pragma unroll
-        for (int s = 0; s < REDUCE_BATCH; ++s)
+        for (int s = 0; s < REDUCE_BATCH; ++s) a[s] = s0 + s < nsplit ? __ldcs(src + (s0 + s) * part) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-                a[s][h] = s0 + s < nsplit ? __ldcs(src + (s0 + s) * part + h * ROWS) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int s = 0; s < REDUCE_BATCH; ++s)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                v[4 * h] += a[s][h].x, v[4 * h + 1] += a[s][h].y, v[4 * h + 2] += a[s][h].z, v[4 * h + 3] += a[s][h].w;
+        for (int s = 0; s < REDUCE_BATCH; ++s) v[0] += a[s].x, v[1] += a[s].y, v[2] += a[s].z, v[3] += a[s].w;
     }
-    *reinterpret_cast<uint4 *>(out + (int64_t)row * outw + c) =
-        make_uint4(pack2(v[0], v[1], fmt), pack2(v[2], v[3], fmt), pack2(v[4], v[5], fmt), pack2(v[6], v[7], fmt));
+    *reinterpret_cast<uint2 *>(out + (int64_t)row * outw + c) = make_uint2(pack2(v[0], v[1], fmt), pack2(v[2], v[3], fmt));
 }
 
 // A single thread waits on an mbarrier that nothing arrives at: the bounded wait runs out,
@@ -1254,7 +1247,7 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     PCX_LAUNCH_CHECK();
     if (p.nsplit > 1) {
         const int64_t slots = pv.nblocks * ROWS;
-        os_reduce_kernel<<<dim3((unsigned)pv.nblocks, (unsigned)(p.out_pitch / 8)), ROWS, 0, stream>>>(p.partial, p.perm, p.bias, slots, p.out_pitch,
+        os_reduce_kernel<<<dim3((unsigned)pv.nblocks, (unsigned)(p.out_pitch / 4)), ROWS, 0, stream>>>(p.partial, p.perm, p.bias, slots, p.out_pitch,
                                                                                                      p.nsplit, p.fmt, p.out);
         PCX_LAUNCH_CHECK();
     }
