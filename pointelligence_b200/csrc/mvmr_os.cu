@@ -470,6 +470,9 @@ constexpr int EPI_WARPS = 4, TEAMS = 4, TEAM_WARPS = 4, COPY_WARPS = TEAMS * TEA
 constexpr int COPY_WARP0 = EPI_WARPS, WALK_WARP = COPY_WARP0 + COPY_WARPS, WEIGHT_WARP = WALK_WARP + 1, MMA_WARP0 = WEIGHT_WARP + 1;
 constexpr int THREADS = (MMA_WARP0 + GROUP_BLOCKS) * 32;
 constexpr int MAX_SLOTS = 8;
+// Output channels whose bias is kept in shared memory (wider rows read it from global memory: behind the copies in the
+// SM's memory pipeline every 16 columns waited for it, and 200k points of 256 channels took 383 us instead of 338).
+constexpr int BIAS_WIDTH = 1024;
 constexpr int AHEAD = 8;                              // steps the walk runs ahead
 constexpr uint32_t ENTRY_BYTES = 2 * ROWS * 4;        // source rows of a tap's two tiles
 // a step's word: per tap of the step, which of the two tiles have it | contraction steps of 16 << 8 | tiles that have
@@ -589,6 +592,7 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
     __shared__ int s_wrow[AHEAD * PACK];   // and, of each of its taps, the first row
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
+    __shared__ float s_bias[BIAS_WIDTH];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // a slot: the A tiles of the group's two blocks, then the weight slice both use; behind the slots the
     // source rows of the next steps
@@ -617,6 +621,9 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
         tma_prefetch_desc(&tmap);
     }
     if (warp == 0) tmem_alloc(smem_u32(&s_tmem), p.ncols);
+    const bool bias_here = p.bias && p.nsplit == 1 && p.out_pitch <= BIAS_WIDTH;
+    if (bias_here)
+        for (int c = tid; c < p.out_pitch; c += THREADS) s_bias[c] = bias_at(p.bias, c, p.fmt);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
@@ -655,7 +662,10 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
 #pragma unroll
                             for (int e = 0; e < 4; ++e) dst[e * ROWS] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
                         } else {
-                            if (p.bias) {
+                            if (bias_here) {
+#pragma unroll
+                                for (int e = 0; e < 16; ++e) v[e] += s_bias[col0 + c0 + e];
+                            } else if (p.bias) {
 #pragma unroll
                                 for (int e = 0; e < 16; ++e) v[e] += bias_at(p.bias, col0 + c0 + e, p.fmt);
                             }
@@ -1213,7 +1223,7 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     if (r != CUDA_SUCCESS) PCX_FAIL(PCX_E_LAUNCH, "pcx_mvmr_planned: cuTensorMapEncodeTiled failed (%d)", (int)r);
 
     // as many slots as fit: three of 64 KB at 256 output channels, five of 40 KB at 64
-    p.nslots = (int)std::min<size_t>(MAX_SLOTS, ((size_t)232448 - 1024 - 1024 - AHEAD * pack * ENTRY_BYTES) / p.slot_bytes);
+    p.nslots = (int)std::min<size_t>(MAX_SLOTS, ((size_t)232448 - 1024 - 1536 - BIAS_WIDTH * sizeof(float) - AHEAD * pack * ENTRY_BYTES) / p.slot_bytes);
     // A team at step n has waited for the release of step n - teams - nslots, and its next wait names step n - nslots
     // by the parity of its turn alone: with more teams than slots that could still be a turn further back.
     p.teams = std::min(TEAMS, p.nslots);
