@@ -110,11 +110,13 @@ int pcx_mvmr_bias(const void *d_weight, const void *d_feat, const int32_t *d_gat
     a.K = K, a.G = G, a.C = C, a.M = M, a.transpose = transpose ? 1 : 0, a.dtype = dtype;
     a.bias = d_bias, a.reverse = (flags & PCX_MVMR_REVERSE_TAPS) ? 1 : 0;
     if (force_engine()) engine = force_engine();
-    if (fan_in_one && T > 0 && engine != PCX_ENGINE_CUDA_CORE && mvmr_tensor_supported(a) && ((uintptr_t)d_out & 15) == 0) {
+    if (fan_in_one && T > 0 && engine != PCX_ENGINE_CUDA_CORE && ((uintptr_t)d_out & 15) == 0) {
         // every output row has exactly one triplet: the tensor kernel stores the rounded rows
-        // itself -- no accumulator to clear, no reductions, no rounding pass
+        // itself -- no accumulator to clear, no reductions, no rounding pass.  Rows of a contraction
+        // wider than 256 channels are completed by several passes and cannot be stored.
         a.out_rows = d_out;
-        return mvmr_tensor(a, stream);
+        if (mvmr_tensor_supported(a)) return mvmr_tensor(a, stream);
+        a.out_rows = nullptr;
     }
     if (int rc = clear_accumulator(a.acc, d_bias, n_out, G * outw, dtype, stream)) return rc;
     if (T > 0) {
