@@ -187,7 +187,8 @@ int pcx_mvmr_plan_build(const int32_t *d_scatter, const int32_t *d_gather,
  * (what pcx_radius_taps_fill emits) are regrouped by counting, others by
  * sorting their triplets.  With `h_multi` null the caller vouches that the
  * rows ascend: nothing is waited for, the count appears in 32-bit word
- * PCX_PLAN_MULTI_WORD of the plan, and min(T / 2, n_out * K) bounds it. */
+ * PCX_PLAN_MULTI_WORD of the plan, and min(T / 2, n_out * K) bounds it.  The
+ * word after it is set when the rows do not ascend; the plan is wrong then. */
 #define PCX_PLAN_MULTI_WORD 4
 int pcx_mvmr_plan_build_counted(const int32_t *d_scatter,
                                 const int32_t *d_gather,

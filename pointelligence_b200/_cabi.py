@@ -393,9 +393,11 @@ class MvmrPlan:
         """(row, tap) buckets with several triplets; a bound while the plan of an ordered rulebook is being built."""
         if self._word is not None:
             n = host().peek(self._word)
-            if n < 0 and torch.cuda.current_stream(self.buffer.device) != self._stream:
+            if n == -1 and torch.cuda.current_stream(self.buffer.device) != self._stream:
                 torch.cuda.synchronize(self.buffer.device)   # another stream than the one that waits for the plan
                 n = host().peek(self._word)
+            if n == -2:
+                raise RuntimeError("a plan was built for rows that ascend inside every tap, and these do not")
             if n >= 0:
                 self._multi, self._word = n, None
         return self._multi
@@ -455,7 +457,7 @@ def mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks):
     into (n_out of them), ``gather`` the rows that are read."""
     require_cuda(scatter, gather, seg_offs)
     T = scatter.numel()
-    ordered = T <= _NO_WAIT_TRIPLETS and _built(scatter, gather) is not None
+    ordered = T <= _NO_WAIT_TRIPLETS and _rows_ascend(scatter, gather, seg_offs, K)
     buf, multi, word = host().plan_build(scatter, gather, seg_offs, int(K), int(n_out), int(group_blocks), ordered)
     return MvmrPlan(buf, T, int(K), int(n_out), int(group_blocks), multi, word)
 
@@ -470,31 +472,42 @@ _PLAN_CACHE_MAX = 64
 _BUILT = {}
 
 
-def mark_built(i, j, symmetric):
-    """Record that ``(i, j, k)`` come from the geometry path: i ascends inside every tap.  ``symmetric``: the
-    rulebook these index tensors belong to is its own mirror image: with ``(i, j, k)`` it holds ``(j, i, K - 1 - k)``.  True for a self-search (queries are the points):
-    the distance is symmetric and the tap of the opposite offset is the mirrored tap.  The input
-    gradient of such a layer is then a forward pass over the SAME rulebook with the taps of the
-    weight reversed, so it needs no plan of its own (``tig_grad_input``).  Remembered by tensor
-    identity, like the plans."""
+def mark_built(i, j, seg_offs, K, symmetric):
+    """Record that ``(i, j)`` cut into ``K`` taps by ``seg_offs`` come from the geometry path: i ascends inside every
+    tap.  ``symmetric``: the rulebook is its own mirror image: with ``(i, j, k)`` it holds ``(j, i, K - 1 - k)``.
+    True for a self-search (queries are the points): the distance is symmetric and the tap of the opposite offset is
+    the mirrored tap.  The input gradient of such a layer is then a forward pass over the SAME rulebook with the taps
+    of the weight reversed, so it needs no plan of its own (``tig_grad_input``).  Remembered by tensor identity, like
+    the plans."""
     import weakref
 
-    for key in [key for key, (refs, _, _) in _BUILT.items() if any(r() is None for r in refs)]:
+    for key in [key for key, (refs, _, _, _) in _BUILT.items() if any(r() is None for r in refs)]:
         _BUILT.pop(key, None)
-    _BUILT[(i.data_ptr(), j.data_ptr(), i.numel())] = ((weakref.ref(i), weakref.ref(j)), (i._version, j._version), bool(symmetric))
+    built = (i, j, seg_offs)
+    _BUILT[(i.data_ptr(), j.data_ptr(), i.numel())] = (tuple(weakref.ref(t) for t in built),
+                                                       tuple(t._version for t in built), int(K), bool(symmetric))
 
 
 def _built(i, j):
-    """None for a rulebook the geometry path did not build (or that was written to since), else whether it is symmetric."""
+    """What ``mark_built`` recorded for these tensors (None: nothing, or they were written to since)."""
     hit = _BUILT.get((i.data_ptr(), j.data_ptr(), i.numel()))
     if hit is None:
         return None
-    refs, stamp, symmetric = hit
-    return symmetric if refs[0]() is i and refs[1]() is j and stamp == (i._version, j._version) else None
+    refs, stamp = hit[:2]
+    return hit if refs[0]() is i and refs[1]() is j and stamp[:2] == (i._version, j._version) else None
 
 
-def is_symmetric(i, j):
-    return bool(_built(i, j)) and os.environ.get("PCX_SYMMETRIC_DGRAD", "1") != "0"
+def _rows_ascend(i, j, seg_offs, K):
+    """Whether i is known to ascend inside every tap.  That is a property of the cut into taps too: where taps are
+    merged, rows fall at the seams."""
+    hit = _built(i, j)
+    return hit is not None and hit[0][2]() is seg_offs and hit[1][2] == seg_offs._version and hit[2] == int(K)
+
+
+def is_symmetric(i, j, K=None):
+    hit = _built(i, j)
+    return (hit is not None and hit[3] and (K is None or hit[2] == int(K))
+            and os.environ.get("PCX_SYMMETRIC_DGRAD", "1") != "0")
 
 
 def cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks):

@@ -25,7 +25,7 @@ namespace {
 
 // ------------------------------------------------------------------ helpers ----
 PyObject *g_plan_hook = nullptr;       // (scatter, gather, seg, K, n_out, out_width, in_width, forced) -> None | plan tuple
-PyObject *g_symmetric_hook = nullptr;  // (i, j) -> bool
+PyObject *g_symmetric_hook = nullptr;  // (i, j, K) -> bool
 PyObject *g_double_backward = nullptr; // differentiable backward of the convolution (create_graph)
 
 [[noreturn]] void raise(PyObject *type, const std::string &msg) {
@@ -234,9 +234,9 @@ std::atomic<int> g_engine{0};   // engine of the current dispatch mode (0 automa
 
 constexpr int64_t FAN_IN_ONE = PCX_ENGINE_FLAG_FAN_IN_ONE;
 
-bool is_symmetric(const Tensor &i, const Tensor &j) {
+bool is_symmetric(const Tensor &i, const Tensor &j, int64_t K) {
     py::gil_scoped_acquire gil;
-    return py::cast<bool>(py::reinterpret_borrow<py::object>(g_symmetric_hook)(i, j));
+    return py::cast<bool>(py::reinterpret_borrow<py::object>(g_symmetric_hook)(i, j, K));
 }
 
 void match(Tensor &w, Tensor &x) {
@@ -271,7 +271,7 @@ Tensor conv_grad_input(const Tensor &weight, const Tensor &grad, const Tensor &i
     int64_t engine = g_engine;
     // a self-search rulebook holds (j, i, K - 1 - k) with every (i, j, k): the input gradient is the forward
     // schedule over the same rulebook (and the same plan) with the taps of the weight in reverse order
-    if (s.n_out == s.n_in && is_symmetric(i, j))
+    if (s.n_out == s.n_in && is_symmetric(i, j, s.K))
         return mvmr_impl(w, g, j, i, seg, std::nullopt, s.n_in, 3, engine, Tensor()).to(grad.scalar_type());
     if (s.cover_in && i.numel() == s.n_in) engine |= FAN_IN_ONE;
     return mvmr_impl(w, g, i, j, seg, std::nullopt, s.n_in, 1, engine, Tensor()).to(grad.scalar_type());
@@ -493,9 +493,9 @@ std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor> grid_sample(const Te
     return {indices, out, sample_ ? OptTensor(out_sample) : std::nullopt, want_mapping ? OptTensor(mapping) : std::nullopt, sizes};
 }
 
-// (plan buffer, number of buckets with several triplets, null or a page-locked word).  A rulebook whose rows are known
-// to ascend inside every tap needs no wait: the number is a bound then, and the true one replaces the word's -1 when the
-// plan is ready.
+// (plan buffer, number of buckets with several triplets, null or page-locked words).  A rulebook whose rows are known
+// to ascend inside every tap needs no wait: the number is a bound then, and the true one and the builder's verdict on
+// the rows replace the words' -1 when the plan is ready.
 std::tuple<Tensor, int64_t, OptTensor> plan_build(const Tensor &scatter_, const Tensor &gather_, const Tensor &seg_, int64_t K,
                                                   int64_t n_out, int64_t group, bool ordered) {
     require_cuda(scatter_), require_cuda(gather_), require_cuda(seg_);
@@ -514,10 +514,17 @@ std::tuple<Tensor, int64_t, OptTensor> plan_build(const Tensor &scatter_, const 
     check(pcx_mvmr_plan_build_counted(ptr_as<int32_t>(scatter), ptr_as<int32_t>(gather), ptr_as<int64_t>(seg), T, (int)K, n_out, (int)group,
                                       ptr(buf), buf.numel(), ptr(ws), ws.numel(), ordered ? nullptr : &multi, stream()));
     if (!ordered) return {buf, multi, std::nullopt};
-    Tensor word = at::empty({1}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
-    *static_cast<volatile int32_t *>(word.data_ptr<int32_t>()) = -1;
-    word.copy_(buf.narrow(0, 4 * PCX_PLAN_MULTI_WORD, 4).view(at::kInt), true);
-    return {buf, std::min(T / 2, n_out * K), word};
+    Tensor words = at::empty({2}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    for (int n = 0; n < 2; ++n) static_cast<volatile int32_t *>(words.data_ptr<int32_t>())[n] = -1;
+    words.copy_(buf.narrow(0, 4 * PCX_PLAN_MULTI_WORD, 8).view(at::kInt), true);
+    return {buf, std::min(T / 2, n_out * K), words};
+}
+
+// The words of a plan that was not waited for: the number of buckets, -1 until it is known, -2 for rows out of order.
+int64_t peek(const Tensor &words) {
+    const volatile int32_t *w = static_cast<volatile int32_t *>(words.data_ptr<int32_t>());
+    const int32_t multi = w[0], unsorted = w[1];
+    return multi == -1 || unsorted == -1 ? -1 : unsorted ? -2 : multi;
 }
 
 Tensor planned(const Tensor &weight, const Tensor &feat, const Tensor &buffer, int64_t group, int64_t multi, int64_t T, int64_t n_out,
@@ -572,7 +579,7 @@ PYBIND11_MODULE(_pcx_host, m) {
     m.def("layer_norm_backward", &layer_norm_backward);
     m.def("radius_taps", &radius_taps, py::call_guard<py::gil_scoped_release>());
     m.def("grid_sample", &grid_sample, py::call_guard<py::gil_scoped_release>());
-    m.def("peek", [](const Tensor &word) { return (int64_t)*static_cast<volatile int32_t *>(word.data_ptr<int32_t>()); });
+    m.def("peek", &peek);
     m.def("plan_build", &plan_build, py::call_guard<py::gil_scoped_release>());
     m.def("planned", &planned);
 }

@@ -70,7 +70,7 @@ constexpr unsigned STATUS_BIT = 4u;   // bit of the device status word this kern
 constexpr unsigned PLAN_MAGIC = 0x70637832u;
 
 // control words at the head of a plan
-enum { CTRL_MAGIC = 2, CTRL_GROUP = 3, CTRL_NMULTI = PCX_PLAN_MULTI_WORD, CTRL_UNSORTED = 5, CTRL_WORDS = 64 };
+enum { CTRL_MAGIC = 2, CTRL_GROUP = 3, CTRL_NMULTI = PCX_PLAN_MULTI_WORD, CTRL_UNSORTED = CTRL_NMULTI + 1, CTRL_WORDS = 64 };
 
 struct PlanView {
     uint32_t *ctrl;        // CTRL_WORDS

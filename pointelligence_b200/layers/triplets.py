@@ -112,7 +112,7 @@ def build_triplets_segmented(points, sample_inds, sample_sizes, neighbor_radius,
             lonely = int((num_neighbors == 0).sum().item()) if num_neighbors.numel() else 0
         if lonely:
             raise AssertionError(_NO_NEIGHBOR_MSG)
-        _cabi.mark_built(i, j, symmetric=query_points is points)   # a self-search is its own mirror image
+        _cabi.mark_built(i, j, seg_offs, ks ** 3, symmetric=query_points is points)   # a self-search is its own mirror image
         out = (i, j, k, seg_offs, (num_neighbors if return_num_neighbors else None))
         cache_put(key, out, points)
         return out

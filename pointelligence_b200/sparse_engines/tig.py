@@ -97,7 +97,7 @@ def tig_grad_input(weight, grad_out, index, input_precision=None, flat_cfg=None)
     assert grad_out.size(0) == index.N, f"grad_out rows {grad_out.size(0)} != index.N {index.N}"
     out_dtype = grad_out.dtype
     w, grad_out = _match(w, grad_out)
-    if index.N == index.N_in and _cabi.is_symmetric(index.flat_i, index.flat_j):
+    if index.N == index.N_in and _cabi.is_symmetric(index.flat_i, index.flat_j, index.K):
         # a self-search rulebook holds (j, i, K - 1 - k) with every (i, j, k): the input gradient is
         # the forward schedule over the same rulebook (and the same plan) with the taps reversed
         out = mvmr_op(w.flip(0), grad_out, index.flat_j, index.flat_i, index.flat_seg, None, index.N_in, True,

@@ -29,3 +29,24 @@ def test_one_triplet_per_row_with_contractions_of_several_parts(C, M, G):
         ref = torch.zeros(n, out.shape[1], dtype=torch.float64, device=DEV)
         ref[once.long()] = torch.einsum("tgc,tgcm->tgm", x.double().view(70, G, -1)[any_row.long()], wd[k]).reshape(n, -1)
         assert _rel(out, ref) < TOL[dtype], transpose
+
+
+def test_geometry_built_triplets_with_merged_taps():
+    """Rows ascend inside the 27 taps of the search, not inside nine merged ones: that plan has to sort."""
+    from pointelligence_b200 import _cabi
+    from pointelligence_b200.layers.triplets import build_triplets_segmented
+
+    n = 3000
+    g = torch.Generator(device=DEV).manual_seed(2)
+    pts = torch.rand(n, 3, device=DEV, generator=g) * n ** (1 / 3)
+    i, j, _, seg, _ = build_triplets_segmented(pts, torch.zeros(n, dtype=torch.int32, device=DEV),
+                                               torch.tensor([n], device=DEV), 1.5, 3, radius_scaler=2.5)
+    merged = seg[::3].contiguous()
+    w = torch.randn(9, 1, 64, 64, device=DEV, generator=g).bfloat16() / 8
+    x = torch.randn(n, 64, device=DEV, generator=g).bfloat16()
+    out = _cabi.mvmr(w, x, j, i, merged, None, n, False, _cabi.ENGINE_PLANNED)
+    ref = torch.zeros(n, 64, dtype=torch.float64, device=DEV)
+    for tap in range(9):
+        a, b = int(merged[tap]), int(merged[tap + 1])
+        ref.index_add_(0, i[a:b].long(), x[j[a:b].long()].double() @ w[tap, 0].double())
+    assert _rel(out, ref) < TOL[torch.bfloat16]

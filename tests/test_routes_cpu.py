@@ -1,0 +1,32 @@
+"""Host-side rules that pick a kernel, and what they remember about a rulebook.  No GPU: the kernels are not run."""
+import pytest
+import torch
+
+from pointelligence_b200 import _cabi
+
+
+@pytest.fixture
+def rulebook():
+    """27 taps of 40 triplets, rows ascending inside each tap."""
+    g = torch.Generator().manual_seed(0)
+    i = torch.sort(torch.randint(0, 200, (27, 40), generator=g), dim=1).values.int().flatten()
+    j = torch.randint(0, 200, (1080,), generator=g).int()
+    return i, j, torch.arange(28) * 40
+
+
+def test_row_order_is_remembered_with_the_cut_into_taps(rulebook):
+    i, j, seg = rulebook
+    _cabi.mark_built(i, j, seg, 27, symmetric=True)
+    assert _cabi._rows_ascend(i, j, seg, 27) and _cabi.is_symmetric(i, j) and _cabi.is_symmetric(i, j, 27)
+    merged = seg[::3].contiguous()      # nine taps of the same triplets: rows fall at the seams
+    assert not _cabi._rows_ascend(i, j, merged, 9) and not _cabi.is_symmetric(i, j, 9)
+    assert not _cabi._rows_ascend(i, j, seg.clone(), 27)
+    seg += 0                            # written to since
+    assert not _cabi._rows_ascend(i, j, seg, 27) and _cabi.is_symmetric(i, j, 27)
+    i += 0
+    assert not _cabi.is_symmetric(i, j, 27)
+
+
+@pytest.mark.parametrize("words,want", [((-1, -1), -1), ((5, -1), -1), ((-1, 0), -1), ((5, 0), 5), ((0, 0), 0), ((5, 1), -2)])
+def test_words_of_a_plan_that_is_not_waited_for(words, want):
+    assert _cabi.host().peek(torch.tensor(words, dtype=torch.int32)) == want
