@@ -371,10 +371,7 @@ def run_ours(args, rank, local_rank, world):
             dist.barrier()
         torch.cuda.synchronize()
 
-    # steps before the warm-up: a rulebook that a program keeps gets its plan after a number of passes, outside the
-    # steady state that is timed (as the rulebook itself, whose construction is reported as geometry_ms)
-    settle = _cabi._KEPT_PASSES + 1 if args.engine == "auto" else 0
-    for _ in range(settle + max(args.warmup, 3)):
+    for _ in range(max(args.warmup, 3)):
         step_resident()
     barrier()
 
@@ -575,7 +572,7 @@ def run_ours(args, rank, local_rank, world):
             "config": {"workload": workload_label(args.points, args.channels), "points_per_rank": n, "triplets_rank0": T,
                        "triplets_per_point": T / n, "l2": "flushed between steps (256 MiB write)",
                        "collective": "all-reduce of dW per step" if world > 1 else "none", "numa_rank0": numa,
-                       "mvmr_engine": args.engine, "settle_steps": settle,
+                       "mvmr_engine": args.engine,
                        "geometry_ms": geometry_ms},
             "tflops": 6.0 * T_all * C * M / (per_step_ms * 1e-3) / 1e12,
             "roofline": roofline,
