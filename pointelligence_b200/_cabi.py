@@ -559,36 +559,10 @@ def mvmr(weight, feat, gather, scatter, seg_offs, tap_idx, n_out, transpose, eng
     return host().mvmr(weight, feat, gather, scatter, seg_offs, tap_idx, int(n_out), bool(transpose), int(engine))
 
 
-# A rulebook the program keeps: the output-stationary kernel beats the scatter kernel from about three
-# triplets per output row on (150 000 points, 6.7 per row: 62 against 83 us per pass at 64 channels, 116
-# against 195 at 128), but by less than its plan costs (0.25 ms there).  So the plan of a rulebook that does
-# not pay for itself at once is built when the rulebook has been used _KEPT_PASSES times.
-_KEPT_PASSES = 8
-_KEPT_MIN_RATIO = 3.0
-_PASSES = {}
-
-
-def _kept_rulebook_pays(scatter, gather, K, n_out):
-    if not _PLANNED_ENABLED or K <= 1 or scatter.numel() < _KEPT_MIN_RATIO * n_out:
-        return False
-    import weakref
-
-    key = (scatter.data_ptr(), gather.data_ptr(), scatter.numel())
-    entry = _PASSES.get(key)
-    if entry is None or entry[0]() is not scatter or entry[1]() is not gather or entry[2] != (scatter._version, gather._version):
-        if len(_PASSES) >= 256:
-            for k in [k for k, e in _PASSES.items() if e[0]() is None or e[1]() is None] or list(_PASSES)[:128]:
-                _PASSES.pop(k, None)
-        entry = _PASSES[key] = [weakref.ref(scatter), weakref.ref(gather), (scatter._version, gather._version), 0]
-    entry[3] += 1
-    return entry[3] > _KEPT_PASSES
-
-
 def _plan_hook(scatter, gather, seg_offs, K, n_out, outw, inw, forced):
     """Asked by the host path for every pass the output-stationary kernel could take: the plan to run
     (buffer, blocks per group, multi-triplet buckets) or None for the scatter engine."""
-    if not forced and not _planned_pays(gather.numel(), n_out, outw, K) and not _kept_rulebook_pays(
-            scatter, gather, K, n_out):
+    if not forced and not _planned_pays(gather.numel(), n_out, outw, K):
         return None
     plan = cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, plan_group_blocks(outw))
     return plan.buffer, plan.group_blocks, plan.multi_buckets

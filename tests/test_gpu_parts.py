@@ -104,25 +104,6 @@ def test_output_row_count_one_above_a_whole_wave_of_groups():
     assert _rel(out, ref) < TOL[torch.bfloat16]
 
 
-def test_a_kept_sparse_rulebook_moves_to_the_output_stationary_kernel():
-    from pointelligence_b200 import _cabi
-
-    n, K, T = 4000, 27, 16000
-    i, j, k, seg = _rulebook(n, n, K, T, 11)
-    w = torch.randn(K, 1, 64, 64, device=DEV).bfloat16() / 8
-    x = torch.randn(n, 64, device=DEV).bfloat16()
-    want = _cabi.mvmr(w, x, j, i, seg, None, n, False, _cabi.ENGINE_TENSOR)
-    labels = []
-    for _ in range(_cabi._KEPT_PASSES + 1):
-        _cabi.profile_enable(True)
-        out = _cabi.mvmr(w, x, j, i, seg, None, n, False)
-        torch.cuda.synchronize()
-        labels.append([name for name, _ in _cabi.profile_records() if name.startswith("mvmr")][-1])
-        _cabi.profile_enable(False)
-        assert _rel(out, want.double()) < 2 * TOL[torch.bfloat16]     # two roundings apart
-    assert set(labels[:-1]) == {"mvmr_tc_kernel(fwd)"} and labels[-1] == "mvmr_os_kernel(fwd)"
-
-
 def test_plan_of_rows_out_of_order_inside_a_tap():
     """The counting path and the sorting path of the plan builder regroup the same triplets."""
     from pointelligence_b200 import _cabi

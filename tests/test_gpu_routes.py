@@ -50,3 +50,28 @@ def test_geometry_built_triplets_with_merged_taps():
         a, b = int(merged[tap]), int(merged[tap + 1])
         ref.index_add_(0, i[a:b].long(), x[j[a:b].long()].double() @ w[tap, 0].double())
     assert _rel(out, ref) < TOL[torch.bfloat16]
+
+
+def test_a_chain_of_layers_on_one_sparse_rulebook_is_captured():
+    """Six layers on one rulebook of a few triplets per row: twelve passes by the end of the capture, the same bits as
+    the eager chain's engine gives."""
+    from pointelligence_b200 import _cabi
+    from pointelligence_b200.internals.two_phase import GeometryScheduler
+    from pointelligence_b200.layers.conv import PointConv3d
+    from pointelligence_b200.layers.metadata import MetaData
+    from pointelligence_b200.layers.two_phase_conv import ConvOp
+
+    g = torch.Generator(device=DEV).manual_seed(0)
+    pts, batch = torch.rand(4096, 3, generator=g, device=DEV) * 5.0, torch.arange(4096, device=DEV) // 2048
+    torch.manual_seed(1)
+    ops = [ConvOp(PointConv3d(32, 32, kernel_size=3, device=DEV, dtype=torch.bfloat16), stride=1.0) for _ in range(6)]
+    with torch.no_grad():
+        metas = [MetaData(points=pts.clone(), sample_inds=batch.clone(), sample_sizes=torch.bincount(batch), grid_size=0.2)
+                 for _ in range(2)]
+        eager = GeometryScheduler().prepare(ops, metas[0])
+        graphed = GeometryScheduler().prepare(ops, metas[1], compile_segments=True)
+        for seed in range(2):
+            x = torch.randn(4096, 32, device=DEV, generator=g.manual_seed(seed)).bfloat16()
+            want, got = eager(x), graphed(x)
+            assert torch.allclose(got.float(), want.float(), atol=2e-2, rtol=2e-2)
+    assert _cabi.device_status() == 0

@@ -30,3 +30,15 @@ def test_row_order_is_remembered_with_the_cut_into_taps(rulebook):
 @pytest.mark.parametrize("words,want", [((-1, -1), -1), ((5, -1), -1), ((-1, 0), -1), ((5, 0), 5), ((0, 0), 0), ((5, 1), -2)])
 def test_words_of_a_plan_that_is_not_waited_for(words, want):
     assert _cabi.host().peek(torch.tensor(words, dtype=torch.int32)) == want
+
+
+def test_a_rulebook_takes_the_same_engine_however_often_it_is_used(rulebook, monkeypatch):
+    """5.4 triplets per row and a small accumulator: the scatter engine, whose operands stay exact, at every pass; no
+    plan is built under way, where the stream may be capturing."""
+    i, j, seg = rulebook
+
+    def no_plan(*args):
+        raise AssertionError("a plan was built by a feature pass")
+
+    monkeypatch.setattr(_cabi, "cached_mvmr_plan", no_plan)
+    assert all(_cabi._plan_hook(i, j, seg, 27, 200, 64, 64, False) is None for _ in range(40))
