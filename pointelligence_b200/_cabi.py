@@ -438,13 +438,14 @@ def padded_width(width):
 
 
 def planned_supported(weight, feat, gather, scatter, seg_offs, n_out, transpose):
-    """Whether the output-stationary kernel takes this call (fp16 / bf16, tap-sorted int32 triplets;
-    channel counts are padded on the way)."""
+    """Whether the automatic choice may give this call to the output-stationary kernel (fp16 / bf16, one group,
+    tap-sorted int32 triplets, channel counts that need no padding, output rows of at most 256 channels).  Asked for
+    by name it takes grouped and wider layers too."""
     K, G, C, M = weight.shape
-    inw, outw = (padded_width(M), padded_width(C)) if transpose else (padded_width(C), padded_width(M))
-    if seg_offs is None or feat.dtype not in (torch.float16, torch.bfloat16) or n_out <= 0:
+    inw, outw = (M, C) if transpose else (C, M)
+    if G != 1 or seg_offs is None or feat.dtype not in (torch.float16, torch.bfloat16) or n_out <= 0:
         return False
-    if inw > 1024 or G * inw > 2048 or K > 512 or G * ((outw + 255) // 256) > 64:
+    if inw != padded_width(inw) or outw != padded_width(outw) or outw > 256 or inw > 1024 or K > 512:
         return False
     T = gather.numel()
     nblocks = (int(n_out) + 127) // 128
@@ -586,7 +587,7 @@ def prepare_mvmr(weight, gather, scatter, seg_offs, n_out, transpose=False):
     was prepared, False when the policy keeps the scatter engines (which need no preparation)."""
     K, G, C, M = weight.shape
     n_out = int(n_out)
-    outw = padded_width(C if transpose else M)
+    outw = C if transpose else M
     if not (gather is not None and gather.is_cuda and planned_supported(weight, weight, gather, scatter, seg_offs,
                                                                         n_out, transpose)):
         return False

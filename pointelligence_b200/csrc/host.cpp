@@ -125,6 +125,11 @@ bool plan_fits(at::ScalarType dtype, int64_t T, int64_t n_out, int64_t K, int64_
 }
 
 constexpr int ENGINE_PLANNED = 3;
+constexpr int64_t NO_PLAN = 0x200;   // internal flag of an engine: the automatic choice is between the scatter engines
+
+// Shapes the automatic choice may give to the output-stationary kernel.  It rounds the sums of (row, tap) buckets to 16
+// bits; grouped, padded and wider layers multiply their operands as they are unless the caller asks for that kernel.
+bool plan_unasked(int64_t K, int64_t G, int64_t outw) { return K > 1 && G == 1 && outw <= 256; }
 
 Tensor mvmr_planned(const Tensor &weight, const Tensor &feat, const Plan &plan, int64_t T, int64_t n_out, int flags,
                     const Tensor &bias) {
@@ -161,7 +166,7 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
         const Tensor w = reshape16(weight, K * G, C, M, Cp, Mp, {K, G, Cp, Mp});
         const Tensor x = inp == inw ? feat : reshape16(feat, feat.size(0) * G, 1, inw, 1, inp, {feat.size(0), G * inp});
         const Tensor b = !bias.defined() || outp == outw ? bias : reshape16(bias.contiguous(), G, 1, outw, 1, outp, {G * outp});
-        const Tensor y = mvmr_impl(w, x, gather_, scatter_, seg_, tap_, n_out, flags, engine, b);
+        const Tensor y = mvmr_impl(w, x, gather_, scatter_, seg_, tap_, n_out, flags, engine | NO_PLAN, b);
         return outp == outw ? y : reshape16(y, n_out * G, 1, outp, 1, outw, {n_out, G * outw});
     }
     if (engine == 0 || engine == ENGINE_PLANNED) {
@@ -169,15 +174,17 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
         if (engine == ENGINE_PLANNED && !fits) {
             py::gil_scoped_acquire gil;
             raise(PyExc_NotImplementedError,
-                  "the output-stationary engine needs fp16/bf16 features, one group, tap-sorted triplets, channel counts "
-                  "that are multiples of 16 and rows of at most 256 channels");
+                  "the output-stationary engine needs fp16/bf16 features, tap-sorted triplets of at most 512 taps, channel "
+                  "counts that are multiples of 16 (of 32 beyond 256, of 48 beyond 512 ...) and at most 1024 input "
+                  "channels a group");
         }
-        if (fits && (K > 1 || engine == ENGINE_PLANNED)) {
+        if (fits && (engine == ENGINE_PLANNED || plan_unasked(K, G, outw))) {
             const Plan plan = ask_plan(scatter_, gather_, *seg_, K, n_out, outw, inw, engine == ENGINE_PLANNED);
             if (plan.valid) return mvmr_planned(weight, feat, plan, T, n_out, flags, bias);
         }
         engine = 0;
     }
+    engine &= ~NO_PLAN;
     const Tensor gather = as_i32(gather_), scatter = as_i32(scatter_);
     const Tensor tap = tap_ ? as_i32(*tap_) : Tensor(), seg = seg_ ? as_i64(*seg_) : Tensor();
     Tensor out = at::empty({n_out, G * outw}, feat.options());

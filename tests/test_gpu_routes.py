@@ -75,3 +75,26 @@ def test_a_chain_of_layers_on_one_sparse_rulebook_is_captured():
             want, got = eager(x), graphed(x)
             assert torch.allclose(got.float(), want.float(), atol=2e-2, rtol=2e-2)
     assert _cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("C,M,G", [(20, 20, 1), (6, 32, 1), (32, 64, 2), (512, 512, 1), (272, 320, 1)])
+def test_dense_rulebooks_of_padded_grouped_and_wide_layers_keep_exact_operands(C, M, G):
+    """Buckets of several rows of 30 000 leave the range of fp16; the products of these rows do not."""
+    from pointelligence_b200.sparse_engines.tig import TigIndex, tig_mvmr
+
+    n, K, T = 500, 9, 10000
+    g = torch.Generator(device=DEV).manual_seed(3)
+    k = torch.sort(torch.randint(0, K, (T,), device=DEV, generator=g)).values
+    i, j = (torch.randint(0, n, (T,), device=DEV, generator=g).int() for _ in range(2))
+    seg = torch.searchsorted(k, torch.arange(K + 1, device=DEV))
+    w = (torch.randn(K, G, C, M, device=DEV, generator=g) * 1e-4).half().requires_grad_()
+    x = (30000 + 1000 * torch.randn(n, G * C, device=DEV, generator=g)).half().requires_grad_()
+    y = tig_mvmr(w, x, TigIndex.from_flat(i, j, seg, n, n, K))
+    rows = torch.einsum("tgc,tgcm->tgm", x.detach().double().view(n, G, C)[j.long()], w.detach().double()[k])
+    ref = torch.zeros(n, G, M, dtype=torch.float64, device=DEV).index_add_(0, i.long(), rows).view(n, -1)
+    assert torch.isfinite(y).all() and _rel(y.detach(), ref) < TOL[torch.float16]
+    go = torch.full_like(y, 30000.0)
+    gx, = torch.autograd.grad(y, x, go)
+    back = torch.einsum("tgm,tgcm->tgc", go.double().view(n, G, M)[i.long()], w.detach().double()[k])
+    ref = torch.zeros(n, G, C, dtype=torch.float64, device=DEV).index_add_(0, j.long(), back).view(n, -1)
+    assert torch.isfinite(gx).all() and _rel(gx, ref) < TOL[torch.float16]

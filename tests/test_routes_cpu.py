@@ -42,3 +42,13 @@ def test_a_rulebook_takes_the_same_engine_however_often_it_is_used(rulebook, mon
 
     monkeypatch.setattr(_cabi, "cached_mvmr_plan", no_plan)
     assert all(_cabi._plan_hook(i, j, seg, 27, 200, 64, 64, False) is None for _ in range(40))
+
+
+@pytest.mark.parametrize("C,M,G,transpose,takes", [
+    (64, 64, 1, False, True), (1024, 256, 1, False, True), (256, 256, 1, True, True), (16, 512, 1, True, True),
+    (64, 272, 1, False, False), (512, 64, 1, True, False), (64, 64, 2, False, False), (6, 32, 1, False, False),
+    (32, 20, 1, False, False), (1040, 64, 1, False, False)])
+def test_layers_that_may_sum_in_16_bits(rulebook, C, M, G, transpose, takes):
+    i, j, seg = rulebook
+    w, x = torch.empty(27, G, C, M, dtype=torch.bfloat16), torch.empty(1, 1, dtype=torch.bfloat16)
+    assert _cabi.planned_supported(w, x, j, i, seg, 200, transpose) is takes
