@@ -391,11 +391,12 @@ class MvmrPlan:
     @property
     def multi_buckets(self):
         """(row, tap) buckets with several triplets; a bound while the plan of an ordered rulebook is being built."""
-        if self._word is not None:
-            n = host().peek(self._word)
+        word = self._word                # threads may share the plan: one of them drops the word
+        if word is not None:
+            n = host().peek(word)
             if n == -1 and torch.cuda.current_stream(self.buffer.device) != self._stream:
                 torch.cuda.synchronize(self.buffer.device)   # another stream than the one that waits for the plan
-                n = host().peek(self._word)
+                n = host().peek(word)
             if n == -2:
                 raise RuntimeError("a plan was built for rows that ascend inside every tap, and these do not")
             if n >= 0:

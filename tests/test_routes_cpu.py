@@ -52,3 +52,33 @@ def test_layers_that_may_sum_in_16_bits(rulebook, C, M, G, transpose, takes):
     i, j, seg = rulebook
     w, x = torch.empty(27, G, C, M, dtype=torch.bfloat16), torch.empty(1, 1, dtype=torch.bfloat16)
     assert _cabi.planned_supported(w, x, j, i, seg, 200, transpose) is takes
+
+
+class _Words:
+    """Stands in for the host module: what the words of a plan say, call by call (the last value from then on)."""
+
+    def __init__(self, *values, then=lambda: None):
+        self.values, self.then, self.seen = list(values), then, []
+
+    def peek(self, word):
+        self.seen.append(word)
+        value = self.values.pop(0) if len(self.values) > 1 else self.values[0]
+        self.then()
+        return value
+
+
+def _plan(word="word", stream="built here"):
+    return _cabi.MvmrPlan(torch.empty(0), 10, 3, 4, 2, 5, word, stream)
+
+
+def test_another_thread_may_drop_the_word_of_a_plan(monkeypatch):
+    plan = _plan()
+
+    def other_thread():
+        plan._multi, plan._word = 2, None
+
+    words = _Words(-1, 2, then=other_thread)
+    monkeypatch.setattr(_cabi, "host", lambda: words)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: "elsewhere")
+    monkeypatch.setattr(torch.cuda, "synchronize", lambda device=None: None)
+    assert plan.multi_buckets == 2 and None not in words.seen
