@@ -12,6 +12,7 @@ from __future__ import annotations
 import ctypes
 import os
 import threading
+import time
 from ctypes import c_double, c_int, c_int64, c_size_t, c_void_p
 
 import torch
@@ -375,6 +376,9 @@ def _planned_pays(T, n_out, outw, K):
     return ratio >= _PLANNED_DENSE_RATIO or (ratio >= _PLANNED_MIN_RATIO and n_out * outw * 4 >= _PLANNED_MIN_ACC_BYTES)
 
 
+_PLAN_WAIT_SECONDS = 30.0   # for a plan that is being built on another stream
+
+
 class MvmrPlan:
     """A rulebook regrouped for the output-stationary MVMR kernel (``pcx_mvmr_plan_build``).
 
@@ -395,8 +399,15 @@ class MvmrPlan:
         if word is not None:
             n = host().peek(word)
             if n == -1 and torch.cuda.current_stream(self.buffer.device) != self._stream:
-                torch.cuda.synchronize(self.buffer.device)   # another stream than the one that waits for the plan
-                n = host().peek(word)
+                # another stream than the one the plan is built on: wait for the build, without a call that a stream
+                # under capture refuses
+                give_up = time.monotonic() + _PLAN_WAIT_SECONDS
+                while n == -1:
+                    if time.monotonic() > give_up:
+                        raise RuntimeError("a plan was not ready after "
+                                           f"{_PLAN_WAIT_SECONDS:g} s [pcx status -7]")
+                    time.sleep(0)
+                    n = host().peek(word)
             if n == -2:
                 raise RuntimeError("a plan was built for rows that ascend inside every tap, and these do not")
             if n >= 0:

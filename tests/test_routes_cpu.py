@@ -80,5 +80,23 @@ def test_another_thread_may_drop_the_word_of_a_plan(monkeypatch):
     words = _Words(-1, 2, then=other_thread)
     monkeypatch.setattr(_cabi, "host", lambda: words)
     monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: "elsewhere")
-    monkeypatch.setattr(torch.cuda, "synchronize", lambda device=None: None)
     assert plan.multi_buckets == 2 and None not in words.seen
+
+
+def test_a_plan_is_waited_for_without_calls_that_a_capture_refuses(monkeypatch):
+    def refused(device=None):
+        raise RuntimeError("operation not permitted when stream is capturing")
+
+    words = _Words(-1, -1, -1, 3)
+    monkeypatch.setattr(_cabi, "host", lambda: words)
+    monkeypatch.setattr(torch.cuda, "synchronize", refused)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: "elsewhere")
+    assert _plan().multi_buckets == 3
+    words.values = [-1]
+    assert _plan(stream="elsewhere").multi_buckets == 5      # the build's own stream: the bound, no wait
+    monkeypatch.setattr(_cabi, "_PLAN_WAIT_SECONDS", 0.01)
+    with pytest.raises(RuntimeError, match="not ready"):
+        _plan().multi_buckets
+    words.values = [-2]
+    with pytest.raises(RuntimeError, match="ascend"):
+        _plan().multi_buckets
