@@ -485,6 +485,12 @@ _PLAN_CACHE_MAX = 64
 _BUILT = {}
 
 
+def _stamp(*tensors):
+    """What tells whether the tensors were written to since; None for tensors of inference mode, which do not say (and
+    raise when they are asked): nothing is remembered about those."""
+    return None if any(t.is_inference() for t in tensors) else tuple(t._version for t in tensors)
+
+
 def mark_built(i, j, seg_offs, K, symmetric):
     """Record that ``(i, j)`` cut into ``K`` taps by ``seg_offs`` come from the geometry path: i ascends inside every
     tap.  ``symmetric``: the rulebook is its own mirror image: with ``(i, j, k)`` it holds ``(j, i, K - 1 - k)``.
@@ -496,9 +502,10 @@ def mark_built(i, j, seg_offs, K, symmetric):
 
     for key in [key for key, (refs, _, _, _) in _BUILT.items() if any(r() is None for r in refs)]:
         _BUILT.pop(key, None)
-    built = (i, j, seg_offs)
-    _BUILT[(i.data_ptr(), j.data_ptr(), i.numel())] = (tuple(weakref.ref(t) for t in built),
-                                                       tuple(t._version for t in built), int(K), bool(symmetric))
+    stamp = _stamp(i, j, seg_offs)
+    if stamp is not None:
+        _BUILT[(i.data_ptr(), j.data_ptr(), i.numel())] = (tuple(weakref.ref(t) for t in (i, j, seg_offs)), stamp,
+                                                           int(K), bool(symmetric))
 
 
 def _built(i, j):
@@ -507,14 +514,14 @@ def _built(i, j):
     if hit is None:
         return None
     refs, stamp = hit[:2]
-    return hit if refs[0]() is i and refs[1]() is j and stamp[:2] == (i._version, j._version) else None
+    return hit if refs[0]() is i and refs[1]() is j and stamp[:2] == _stamp(i, j) else None
 
 
 def _rows_ascend(i, j, seg_offs, K):
     """Whether i is known to ascend inside every tap.  That is a property of the cut into taps too: where taps are
     merged, rows fall at the seams."""
     hit = _built(i, j)
-    return hit is not None and hit[0][2]() is seg_offs and hit[1][2] == seg_offs._version and hit[2] == int(K)
+    return hit is not None and hit[0][2]() is seg_offs and hit[1][2:] == _stamp(seg_offs) and hit[2] == int(K)
 
 
 def is_symmetric(i, j, K=None):
@@ -530,7 +537,9 @@ def cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks):
 
     key = (scatter.data_ptr(), gather.data_ptr(), seg_offs.data_ptr(), scatter.numel(), int(K), int(n_out),
            int(group_blocks))
-    stamp = (scatter._version, gather._version, seg_offs._version)
+    stamp = _stamp(scatter, gather, seg_offs)
+    if stamp is None:
+        return mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks)
     hit = _PLAN_CACHE.get(key)
     if hit is not None:
         refs, old_stamp, value = hit
@@ -575,8 +584,8 @@ def mvmr(weight, feat, gather, scatter, seg_offs, tap_idx, n_out, transpose, eng
 def _plan_hook(scatter, gather, seg_offs, K, n_out, outw, inw, forced):
     """Asked by the host path for every pass the output-stationary kernel could take: the plan to run
     (buffer, blocks per group, multi-triplet buckets) or None for the scatter engine."""
-    if not forced and not _planned_pays(gather.numel(), n_out, outw, K):
-        return None
+    if not forced and (not _planned_pays(gather.numel(), n_out, outw, K) or _stamp(scatter, gather, seg_offs) is None):
+        return None    # (a plan of inference tensors cannot be remembered, and one per pass does not pay)
     plan = cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, plan_group_blocks(outw))
     return plan.buffer, plan.group_blocks, plan.multi_buckets
 
@@ -603,7 +612,7 @@ def prepare_mvmr(weight, gather, scatter, seg_offs, n_out, transpose=False):
     if not (gather is not None and gather.is_cuda and planned_supported(weight, weight, gather, scatter, seg_offs,
                                                                         n_out, transpose)):
         return False
-    if not _planned_pays(gather.numel(), n_out, outw, K):
+    if not _planned_pays(gather.numel(), n_out, outw, K) or _stamp(scatter, gather, seg_offs) is None:
         return False
     cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, plan_group_blocks(outw))
     return True

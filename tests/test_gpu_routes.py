@@ -98,3 +98,28 @@ def test_dense_rulebooks_of_padded_grouped_and_wide_layers_keep_exact_operands(C
     back = torch.einsum("tgm,tgcm->tgc", go.double().view(n, G, M)[i.long()], w.detach().double()[k])
     ref = torch.zeros(n, G, C, dtype=torch.float64, device=DEV).index_add_(0, j.long(), back).view(n, -1)
     assert torch.isfinite(gx).all() and _rel(gx, ref) < TOL[torch.float16]
+
+
+@pytest.mark.parametrize("density", [4.0, 40.0])
+def test_layers_under_inference_mode(density):
+    """Strided and stride-1 layers on sparse and dense clouds whose index tensors are inference tensors."""
+    from pointelligence_b200.layers import MetaData, PointConv3d, conv_with_stride
+
+    n = 3000
+    g = torch.Generator(device=DEV).manual_seed(5)
+    pts = torch.rand(n, 3, device=DEV, generator=g) * (n / density) ** (1 / 3)
+    inds, x = torch.zeros(n, dtype=torch.int64, device=DEV), torch.randn(n, 64, device=DEV, generator=g).bfloat16()
+    torch.manual_seed(6)
+    convs = [PointConv3d(64, 64, 3, device=DEV, dtype=torch.bfloat16) for _ in range(3)]
+    results = []
+    for mode in (torch.no_grad, torch.inference_mode):
+        with mode():
+            m = MetaData(points=pts, sample_inds=inds, sample_sizes=torch.bincount(inds), grid_size=0.5)
+            y, m = conv_with_stride(convs[0], x, m, 1.0)
+            m.dirty_triplets()
+            y, m = conv_with_stride(convs[1], y, m, 2.0)
+            m.dirty_triplets()
+            y, m = conv_with_stride(convs[2], y, m, 1.0)
+        results.append((y, m.i, m.j))
+    assert all(torch.equal(a, b) for a, b in zip(results[0][1:], results[1][1:]))
+    assert _rel(results[1][0], results[0][0].double()) < 6 * TOL[torch.bfloat16]   # three layers, two engines

@@ -100,3 +100,18 @@ def test_a_plan_is_waited_for_without_calls_that_a_capture_refuses(monkeypatch):
     words.values = [-2]
     with pytest.raises(RuntimeError, match="ascend"):
         _plan().multi_buckets
+
+
+def test_rulebooks_of_inference_mode(monkeypatch):
+    """Inference tensors have no version: a rulebook of them is used, and nothing is remembered about it."""
+    with torch.inference_mode():
+        i, j, seg = (torch.arange(n, dtype=t) for n, t in ((3000, torch.int32), (3000, torch.int32), (28, torch.int64)))
+    _cabi.mark_built(i, j, seg, 27, symmetric=True)
+    assert not _cabi._rows_ascend(i, j, seg, 27) and not _cabi.is_symmetric(i, j, 27)
+    built = []
+    monkeypatch.setattr(_cabi, "mvmr_plan", lambda *args: built.append(args) or _plan(word=None))
+    assert _cabi._planned_pays(3000, 100, 64, 27)
+    assert _cabi._plan_hook(i, j, seg, 27, 100, 64, 64, False) is None and not built
+    for _ in range(2):                       # asked for by name: a plan for every pass
+        assert _cabi._plan_hook(i, j, seg, 27, 100, 64, 64, True)[1:] == (2, 5)
+    assert len(built) == 2 and not any(refs[0]() is i for refs, _, _ in _cabi._PLAN_CACHE.values())
