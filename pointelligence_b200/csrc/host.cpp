@@ -165,7 +165,7 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
         const int64_t Cp = padded(C), Mp = padded(M), inp = transpose ? Mp : Cp, outp = transpose ? Cp : Mp;
         const Tensor w = reshape16(weight, K * G, C, M, Cp, Mp, {K, G, Cp, Mp});
         const Tensor x = inp == inw ? feat : reshape16(feat, feat.size(0) * G, 1, inw, 1, inp, {feat.size(0), G * inp});
-        const Tensor b = !bias.defined() || outp == outw ? bias : reshape16(bias.contiguous(), G, 1, outw, 1, outp, {G * outp});
+        const Tensor b = !bias.defined() || outp == outw ? bias : reshape16(bias, G, 1, outw, 1, outp, {G * outp});
         const Tensor y = mvmr_impl(w, x, gather_, scatter_, seg_, tap_, n_out, flags, engine | NO_PLAN, b);
         return outp == outw ? y : reshape16(y, n_out * G, 1, outp, 1, outw, {n_out, G * outw});
     }
@@ -266,9 +266,13 @@ Tensor conv_forward(const Tensor &weight, const Tensor &feat, const Tensor &bias
                 " do not fit a weight ", weight.sizes(), " of ", s.K, " taps");
     TORCH_CHECK(x.size(0) == s.n_in, "feat rows ", x.size(0), " != index.N_in ", s.n_in);
     match(w, x);
+    TORCH_CHECK(!bias.defined() || (bias.dim() == 1 && bias.numel() == w.size(1) * w.size(3) && bias.device() == x.device() &&
+                                    bias.scalar_type() == x.scalar_type()),
+                "a bias ", bias.sizes(), " does not fit a weight ", weight.sizes());   // the kernels read it by address
     int64_t engine = g_engine;
     if (s.cover_out && i.numel() == s.n_out) engine |= FAN_IN_ONE;   // one triplet per output row: stored, not reduced
-    return mvmr_impl(w, x, j, i, seg, std::nullopt, s.n_out, 0, engine, bias).to(feat.scalar_type());
+    return mvmr_impl(w, x, j, i, seg, std::nullopt, s.n_out, 0, engine, bias.defined() ? bias.contiguous() : bias)
+        .to(feat.scalar_type());
 }
 
 Tensor conv_grad_input(const Tensor &weight, const Tensor &grad, const Tensor &i, const Tensor &j, const Tensor &seg,

@@ -170,12 +170,20 @@ def _takes_host_path(*tensors):
     return True
 
 
+def _fuses(bias, weight, feat):
+    """Whether the kernels can add this bias: one element per output column, of the operands' type.  Others
+    (broadcast ones) are added, or refused, as torch does."""
+    columns = weight.shape[-1] * (weight.shape[1] if weight.dim() == 4 else 1)
+    return (bias.dim() == 1 and bias.numel() == columns and bias.dtype == feat.dtype == weight.dtype
+            and bias.device == feat.device)
+
+
 def tig_mvmr(weight, feat, index, mode="auto", input_precision: Optional[str] = None, bias: Optional[Tensor] = None):
     """Differentiable tap-sorted convolution: one autograd node, three kernel
     families (forward MVMR, transposed MVMR, VVOR).  A ``bias`` of the output's type is added
     before the rows are rounded."""
     if _takes_host_path(weight, feat, bias, index.flat_i, index.flat_j, index.flat_seg) and (
-            bias is None or bias.dtype == feat.dtype == weight.dtype):
+            bias is None or _fuses(bias, weight, feat)):
         return _cabi.host().conv(weight, feat, bias, index.flat_i, index.flat_j, index.flat_seg, index.N, index.N_in,
                                  index.K, index.exact_cover_out, index.exact_cover_in)
     if bias is not None:

@@ -123,3 +123,28 @@ def test_layers_under_inference_mode(density):
         results.append((y, m.i, m.j))
     assert all(torch.equal(a, b) for a, b in zip(results[0][1:], results[1][1:]))
     assert _rel(results[1][0], results[0][0].double()) < 6 * TOL[torch.bfloat16]   # three layers, two engines
+
+
+@pytest.mark.parametrize("M,dtype", [(32, torch.bfloat16), (20, torch.float16), (32, torch.float32)])
+def test_strided_broadcast_and_misfitting_biases(M, dtype):
+    from pointelligence_b200.sparse_engines.tig import TigIndex, tig_mvmr
+
+    n, K, T = 200, 8, 900
+    g = torch.Generator(device=DEV).manual_seed(7)
+    k = torch.sort(torch.randint(0, K, (T,), device=DEV, generator=g)).values
+    i, j = (torch.randint(0, n, (T,), device=DEV, generator=g).int() for _ in range(2))
+    index = TigIndex.from_flat(i, j, torch.searchsorted(k, torch.arange(K + 1, device=DEV)), n, n, K)
+    w = torch.randn(K, 1, 32, M, device=DEV, generator=g).to(dtype) / 6
+    x = torch.randn(n, 32, device=DEV, generator=g).to(dtype)
+    wide = torch.randn(2 * M, device=DEV, generator=g).to(dtype)
+    plain = tig_mvmr(w, x, index)
+    for bias in (wide[::2], wide[:1], wide[0], wide[:M].view(1, M)):
+        bias = bias.detach().requires_grad_()
+        y = tig_mvmr(w, x, index, bias=bias)
+        # at most: the sum rounded, and rounded again with the bias
+        assert _rel(y.detach(), plain.double() + bias.detach().double()) < 2 * TOL.get(dtype, 3e-6)
+        grad, = torch.autograd.grad(y.sum(), bias)
+        assert grad.shape == bias.shape and _rel(grad, torch.full_like(bias, y.numel() / bias.numel()).double()) < 1e-6
+    for bias in (wide[:M - 1], wide):
+        with pytest.raises(RuntimeError):
+            tig_mvmr(w, x, index, bias=bias)

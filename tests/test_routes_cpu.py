@@ -115,3 +115,13 @@ def test_rulebooks_of_inference_mode(monkeypatch):
     for _ in range(2):                       # asked for by name: a plan for every pass
         assert _cabi._plan_hook(i, j, seg, 27, 100, 64, 64, True)[1:] == (2, 5)
     assert len(built) == 2 and not any(refs[0]() is i for refs, _, _ in _cabi._PLAN_CACHE.values())
+
+
+def test_biases_the_kernels_add():
+    from pointelligence_b200.sparse_engines.tig import _fuses
+
+    w, x = torch.empty(27, 2, 8, 16), torch.empty(10, 16)
+    assert _fuses(torch.empty(32), w, x) and _fuses(torch.empty(64)[::2], w, x) and _fuses(torch.empty(16), w[:, 0], x)
+    for bias in (torch.empty(31), torch.empty(1), torch.empty(()), torch.empty(1, 32), torch.empty(32).half(),
+                 torch.empty(32, device="meta")):
+        assert not _fuses(bias, w, x)
