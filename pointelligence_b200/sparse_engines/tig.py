@@ -15,6 +15,7 @@ from typing import Optional
 
 import torch
 from torch import Tensor
+from torch.autograd import forward_ad
 
 from .. import _cabi
 from ._dispatch_override import current_engine, resolve_input_precision
@@ -160,9 +161,12 @@ _PLAIN = (Tensor, torch.nn.Parameter)
 
 
 def _takes_host_path(*tensors):
-    """Whether a call goes straight to the compiled host path: eager mode on plain CUDA tensors.
-    Tracing (``torch.compile``) and tensor subclasses see the registered operator instead."""
-    if torch.compiler.is_compiling():
+    """Whether a call goes straight to the compiled host path: eager mode on plain CUDA tensors.  Whatever watches or
+    transforms operators sees the registered one instead: tracing (``torch.compile``, ``jit.trace``, ``make_fx``),
+    dispatch modes (FLOP counters, selective checkpointing), ``torch.func`` transforms, forward-mode differentiation
+    and tensor subclasses."""
+    if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or torch._C._get_tracing_state() is not None
+            or torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0):
         return False
     for t in tensors:
         if t is not None and (type(t) not in _PLAIN or not t.is_cuda):

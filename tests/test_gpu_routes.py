@@ -148,3 +148,22 @@ def test_strided_broadcast_and_misfitting_biases(M, dtype):
     for bias in (wide[:M - 1], wide):
         with pytest.raises(RuntimeError):
             tig_mvmr(w, x, index, bias=bias)
+
+
+def test_vmap_and_tracing_of_a_convolution():
+    from torch.fx.experimental.proxy_tensor import make_fx
+
+    from pointelligence_b200.sparse_engines.tig import TigIndex, tig_mvmr
+
+    n, K, T = 100, 8, 500
+    g = torch.Generator(device=DEV).manual_seed(8)
+    k = torch.sort(torch.randint(0, K, (T,), device=DEV, generator=g)).values
+    i, j = (torch.randint(0, n, (T,), device=DEV, generator=g).int() for _ in range(2))
+    index = TigIndex.from_flat(i, j, torch.searchsorted(k, torch.arange(K + 1, device=DEV)), n, n, K)
+    w, b = torch.randn(K, 1, 32, 32, device=DEV, generator=g), torch.randn(32, device=DEV, generator=g)
+    xs = torch.randn(3, n, 32, device=DEV, generator=g)
+    want = torch.stack([tig_mvmr(w, x, index, bias=b) for x in xs])
+    assert _rel(torch.func.vmap(lambda x: tig_mvmr(w, x, index, bias=b))(xs), want.double()) < 4e-6
+    traced = make_fx(lambda x: tig_mvmr(w, x, index, bias=b))(xs[0])
+    assert "pointelligence_b200.tig_mvmr" in traced.code
+    assert _rel(traced(xs[1]), want[1].double()) < 4e-6    # and not the values it was traced with

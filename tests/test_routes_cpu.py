@@ -125,3 +125,35 @@ def test_biases_the_kernels_add():
     for bias in (torch.empty(31), torch.empty(1), torch.empty(()), torch.empty(1, 32), torch.empty(32).half(),
                  torch.empty(32, device="meta")):
         assert not _fuses(bias, w, x)
+
+
+def test_what_watches_operators_sees_the_operator(monkeypatch):
+    """The compiled path is for plain eager calls; tracers, modes and transforms get the registered operator."""
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    from pointelligence_b200.sparse_engines import tig
+
+    class Watch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    seen = []
+
+    def call(x):
+        seen.append(tig._takes_host_path())      # (what the tensors are is looked at after these)
+        return x * 2
+
+    x = torch.ones(3)
+    call(x)
+    with Watch():
+        call(x)
+    make_fx(call)(x)
+    torch.jit.trace(call, (x,), check_trace=False)
+    torch.func.vmap(call)(x)
+    torch.func.grad(lambda v: call(v).sum())(x)
+    torch.func.jvp(call, (x,), (x,))
+    with torch.autograd.forward_ad.dual_level():
+        call(x)
+    call(x)
+    assert seen == [True] + [False] * 7 + [True]
