@@ -425,9 +425,7 @@ struct LayerNorm : public torch::autograd::Function<LayerNorm> {
 
 Tensor layer_norm(const Tensor &x, const Tensor &lengths, const OptTensor &weight, const OptTensor &bias,
                   const OptTensor &residual, double eps, bool relu) {
-    const auto wants = [](const OptTensor &t) { return t && t->requires_grad(); };
-    if (!at::GradMode::is_enabled() || !(x.requires_grad() || wants(weight) || wants(bias) || wants(residual)))
-        return std::get<0>(layer_norm_forward(x, lengths, weight, bias, residual, eps, relu));
+    // also without gradients: torch.func transforms and forward-mode tangents are refused there, not dropped
     return LayerNorm::apply(x, lengths, weight, bias, residual, eps, relu);
 }
 

@@ -167,3 +167,14 @@ def test_vmap_and_tracing_of_a_convolution():
     traced = make_fx(lambda x: tig_mvmr(w, x, index, bias=b))(xs[0])
     assert "pointelligence_b200.tig_mvmr" in traced.code
     assert _rel(traced(xs[1]), want[1].double()) < 4e-6    # and not the values it was traced with
+
+
+@pytest.mark.parametrize("grad", [False, True])
+def test_forward_mode_of_the_fused_layer_norm_is_refused(grad):
+    import torch.autograd.forward_ad as fa
+
+    from pointelligence_b200.layers.norm import fused_layer_norm
+
+    x, lengths = torch.randn(5, 8, device=DEV), torch.tensor([5], device=DEV)
+    with fa.dual_level(), torch.set_grad_enabled(grad), pytest.raises((RuntimeError, NotImplementedError), match="jvp"):
+        fused_layer_norm(fa.make_dual(x, torch.ones_like(x)), lengths)

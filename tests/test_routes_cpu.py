@@ -157,3 +157,14 @@ def test_what_watches_operators_sees_the_operator(monkeypatch):
         call(x)
     call(x)
     assert seen == [True] + [False] * 7 + [True]
+
+
+def test_transforms_of_the_fused_layer_norm_are_refused():
+    """The node has one derivative rule, backward; a transform must not get past it to the kernels."""
+    from pointelligence_b200.layers.norm import fused_layer_norm
+
+    x, lengths = torch.randn(4, 8), torch.tensor([4])
+    with pytest.raises(RuntimeError, match="functorch"):
+        torch.func.vmap(lambda v: fused_layer_norm(v, lengths))(x[None])
+    with torch.no_grad(), pytest.raises(RuntimeError, match="functorch"):
+        torch.func.jvp(lambda v: fused_layer_norm(v, lengths), (x,), (x,))
