@@ -178,3 +178,26 @@ def test_forward_mode_of_the_fused_layer_norm_is_refused(grad):
     x, lengths = torch.randn(5, 8, device=DEV), torch.tensor([5], device=DEV)
     with fa.dual_level(), torch.set_grad_enabled(grad), pytest.raises((RuntimeError, NotImplementedError), match="jvp"):
         fused_layer_norm(fa.make_dual(x, torch.ones_like(x)), lengths)
+
+
+def test_operands_of_other_shapes_are_refused():
+    from pointelligence_b200 import _cabi
+    from pointelligence_b200.layers.norm import fused_layer_norm
+    from pointelligence_b200.sparse_engines.tig import TigIndex, tig_mvmr
+
+    i = j = torch.arange(10, device=DEV, dtype=torch.int32)
+    seg, w, x = torch.tensor([0, 4, 10], device=DEV), torch.randn(2, 1, 8, 8, device=DEV), torch.randn(10, 8, device=DEV)
+    index = TigIndex.from_flat(i, j, seg, 10, 10, 2)
+    assert tig_mvmr(w, x, index).shape == tig_mvmr(w[:, 0], x, index).shape == (10, 8)
+    for weight in (w[:, 0], w[..., None]):
+        with pytest.raises(ValueError):
+            _cabi.mvmr(weight, x, j, i, seg, None, 10, False)
+    with pytest.raises(AssertionError):
+        _cabi.mvmr(w, x.half(), j, i, seg, None, 10, False)
+    with pytest.raises(AssertionError):
+        _cabi.vvor(x[:, None], j, x[:, None].half(), i, seg, None, 2)
+    for feat in (x[:, :7], x[:9], torch.randn(10, 9, device=DEV)):
+        with pytest.raises(AssertionError):
+            tig_mvmr(w, feat, index)
+    with pytest.raises(ValueError):
+        fused_layer_norm(torch.randn(10, 8, 2, device=DEV), torch.tensor([10], device=DEV))

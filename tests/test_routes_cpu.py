@@ -168,3 +168,11 @@ def test_transforms_of_the_fused_layer_norm_are_refused():
         torch.func.vmap(lambda v: fused_layer_norm(v, lengths))(x[None])
     with torch.no_grad(), pytest.raises(RuntimeError, match="functorch"):
         torch.func.jvp(lambda v: fused_layer_norm(v, lengths), (x,), (x,))
+
+
+def test_layer_norm_takes_rows_only():
+    from pointelligence_b200.layers.norm import fused_layer_norm
+
+    for shape in ((4, 8, 3), (8,)):
+        with pytest.raises(ValueError):
+            fused_layer_norm(torch.randn(shape), torch.tensor([4]))
