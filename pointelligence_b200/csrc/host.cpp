@@ -510,7 +510,8 @@ std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor> grid_sample(const Te
                                  ptr_as<float>(out), ptr_as<int32_t>(out_sample), ptr_as<int64_t>(mapping), ptr(ws), ws.numel(),
                                  stream()));
     OptTensor sizes;
-    if (sample_ && info[1] >= 0) {   // cells come in ascending sample order
+    // cells come in ascending sample order; ids far beyond the number of points (hashes) are not worth an array
+    if (sample_ && info[1] >= 0 && info[2] < std::max<int64_t>(N, 4096)) {
         sizes = at::empty({info[2] + 1}, i64);
         check(pcx_sample_sizes(ptr_as<int32_t>(out_sample), cells, info[2] + 1, ptr_as<int64_t>(*sizes), stream()));
     }

@@ -44,7 +44,8 @@ def grid_sample_filter(points, grid_size, sample_inds=None, reduction="center_ne
         pts32, float(grid_size), sample_inds, need_map)
     sample_f = None
     if sample_inds is not None:
-        sample_f = out_smp.to(sample_inds.dtype)
+        # ids beyond 32 bits are grouped by their low words and returned as they came
+        sample_f = out_smp if sample_inds.dtype == torch.int32 else sample_inds[indices]
         sizes = getattr(out_smp, "pcx_sample_sizes", None)
         if sizes is not None:
             sample_f.pcx_sample_sizes = sizes

@@ -201,3 +201,22 @@ def test_operands_of_other_shapes_are_refused():
             tig_mvmr(w, feat, index)
     with pytest.raises(ValueError):
         fused_layer_norm(torch.randn(10, 8, 2, device=DEV), torch.tensor([10], device=DEV))
+
+
+@pytest.mark.parametrize("ids", [(0, 3), (7, 2 ** 31 - 2), (5, 2 ** 40 + 1), (-4, 9)])
+def test_grid_sampling_of_points_with_any_sample_ids(ids):
+    """Ids come back as they went in, and no array is made for every id up to the largest."""
+    from pointelligence_b200.internals.grid_sample import grid_sample_filter
+
+    g = torch.Generator(device=DEV).manual_seed(9)
+    pts = torch.rand(2000, 3, device=DEV, generator=g)
+    inds = torch.tensor(ids, device=DEV).repeat_interleave(1000)
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    _, sample, indices, _ = grid_sample_filter(pts, 0.2, inds)
+    assert torch.cuda.max_memory_allocated() - before < 2 ** 20 * 8
+    assert torch.equal(sample, inds[indices]) and sample.dtype == inds.dtype
+    if max(ids) < 2 ** 31:
+        sizes = getattr(sample, "pcx_sample_sizes", None)
+        assert (sizes is not None) == (ids == (0, 3))
+        assert sizes is None or torch.equal(sizes, torch.bincount(sample))
