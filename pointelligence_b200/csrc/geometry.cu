@@ -517,12 +517,23 @@ int key_bits_for(const int32_t *ext) {
     return bits;
 }
 
-// (cell size's bit pattern << 32 | key bits) of the last cloud that was binned at about this cell size
+// What the clouds binned at about this cell size need: (cell size's bit pattern << 32 | calls in a row that needed
+// less << 8 | key bits in whole passes of the radix sort).  Only a hint of how many bits to sort before the extents of a
+// cloud are known: too many cost a pass, too few a second sort.
 std::atomic<uint64_t> &key_bits_of(float cell) {
     static std::atomic<uint64_t> table[64];
     uint32_t u;
     memcpy(&u, &cell, sizeof(u));
     return table[(u * 2654435761u) >> 26];
+}
+
+// The hint after a cloud that needed `bits`: the largest of the last clouds, so that clouds of alternating extents are
+// not sorted twice; one of unusual extents is forgotten after sixteen smaller ones.
+uint64_t key_bits_hint(uint64_t seen, uint32_t cell, int bits) {
+    const uint64_t need = (uint64_t)(bits + 7) / 8 * 8, known = seen & 0xff, smaller = ((seen >> 8) & 0xff) + 1;
+    const uint64_t tag = (uint64_t)cell << 32;
+    if ((seen >> 32) != cell || need >= known || smaller == 16) return tag | need;
+    return tag | smaller << 8 | known;
 }
 
 int bits_for(int64_t n) {
@@ -765,7 +776,7 @@ int pcx_grid_sample_count_samples(const float *d_points, const int32_t *d_sample
     grid_key_kernel<<<nb, 256, 0, stream>>>(d_points, d_sample, N, c32, w.ext, w.keys_a, w.vals_a);
     PCX_LAUNCH_CHECK();
     // The sort only has to look at the bits the largest key can use.  How many those are is known from the extents,
-    // which come to the host with the cell count; the sort is enqueued for the bits that the last cloud of this
+    // which come to the host with the cell count; the sort is enqueued for the bits that the last clouds of this
     // cell size needed, and repeated where this one needs more (a first call asks for the extents beforehand).
     int32_t *h = reinterpret_cast<int32_t *>(handover_words());   // extents, then the number of cells
     auto extents = [&]() -> int {
@@ -779,7 +790,7 @@ int pcx_grid_sample_count_samples(const float *d_points, const int32_t *d_sample
     uint64_t seen = known.load();
     if ((seen >> 32) != cell_bits || (seen & 0xff) == 0) {
         if (int rc = extents()) return rc;
-        seen = ((uint64_t)cell_bits << 32) | (uint64_t)key_bits_for(h);
+        seen = key_bits_hint(0, cell_bits, key_bits_for(h));
     }
     int used = (int)(seen & 0xff);
     for (;;) {
@@ -792,7 +803,7 @@ int pcx_grid_sample_count_samples(const float *d_points, const int32_t *d_sample
         PCX_CUDA(cudaMemcpyAsync(h + 8, w.ordinal + (N - 1), sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
         if (int rc = extents()) return rc;
         const int need = key_bits_for(h);
-        known.store(((uint64_t)cell_bits << 32) | (uint64_t)need);
+        known.store(key_bits_hint(seen, cell_bits, need));
         if (need <= used) break;
         used = need;
     }

@@ -220,3 +220,23 @@ def test_grid_sampling_of_points_with_any_sample_ids(ids):
         sizes = getattr(sample, "pcx_sample_sizes", None)
         assert (sizes is not None) == (ids == (0, 3))
         assert sizes is None or torch.equal(sizes, torch.bincount(sample))
+
+
+def test_clouds_of_alternating_extents_are_sorted_once():
+    """Rooms whose cell keys need some bits more and less (here 20 and 28): from the third call on every call launches
+    the same kernels, and all of them find the cells of a cloud sorted for its own bits."""
+    from pointelligence_b200 import _cabi
+
+    g = torch.Generator(device=DEV).manual_seed(10)
+    clouds = [torch.rand(5000, 3, device=DEV, generator=g) * side for side in (4.1, 26.0)]
+    cell = 0.0413       # of this test alone: what a size needed is remembered
+    first = [_cabi.grid_sample_center_nearest(c, cell, None, True) for c in clouds]
+    launches = []
+    for n in range(8):
+        _cabi.launch_count(reset=True)
+        out = _cabi.grid_sample_center_nearest(clouds[n % 2], cell, None, True)
+        launches.append(_cabi.launch_count())
+        assert torch.equal(out[0], first[n % 2][0]) and torch.equal(out[3], first[n % 2][3])
+    assert len(set(launches)) == 1, launches
+    key = torch.div(clouds[1], cell, rounding_mode="floor").long()
+    assert first[1][0].numel() == torch.unique(key, dim=0).shape[0]
