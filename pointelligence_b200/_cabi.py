@@ -261,20 +261,20 @@ def on_geometry_stream(fn):
                 return v.points.device
         return None
 
-    def collect(value, out, depth=0):
+    def collect(value, out, caller, depth=0):
         if isinstance(value, torch.Tensor):
-            if id(value) not in _overlap.known:      # kept until the scope ends, so that ids stay unique
-                _overlap.known[id(value)] = value
+            if (id(value), caller) not in _overlap.known:      # kept until the scope ends, so that ids stay unique
+                _overlap.known[id(value), caller] = value
                 out.append(value)
         elif isinstance(value, (tuple, list)):
             for v in value:
-                collect(v, out, depth)
+                collect(v, out, caller, depth)
         elif isinstance(value, MvmrPlan):
             out.append(value.buffer)
         elif hasattr(value, "__dataclass_fields__") and depth < 8:
             for v in vars(value).values():
                 if v is not None and not isinstance(v, (bool, int, float, str)):
-                    collect(v, out, depth + 1)
+                    collect(v, out, caller, depth + 1)
 
     @functools.wraps(fn)
     def wrapper(*args, **kwargs):
@@ -293,7 +293,7 @@ def on_geometry_stream(fn):
             _overlap.inside = False
             host().side_end(*before)
         fresh = []
-        collect(out, fresh)
+        collect(out, fresh, before)
         host().record_streams(fresh)
         return out
 

@@ -240,3 +240,28 @@ def test_clouds_of_alternating_extents_are_sorted_once():
     assert len(set(launches)) == 1, launches
     key = torch.div(clouds[1], cell, rounding_mode="floor").long()
     assert first[1][0].numel() == torch.unique(key, dim=0).shape[0]
+
+
+def test_geometry_handed_to_two_streams_is_known_to_both(monkeypatch):
+    """The allocator has to hear of every stream that a result of the geometry stream is used on."""
+    from pointelligence_b200 import _cabi
+
+    real, heard = _cabi.host(), []
+
+    class Host:
+        def __getattr__(self, name):
+            return getattr(real, name)
+
+        def record_streams(self, tensors):
+            heard.extend((id(t), torch.cuda.current_stream().cuda_stream) for t in tensors)
+            real.record_streams(tensors)
+
+    monkeypatch.setattr(_cabi, "host", Host)
+    result = torch.ones(8, device=DEV)
+    build = _cabi.on_geometry_stream(lambda x: result)     # as a builder that finds its rulebook in the cache
+    side = torch.cuda.Stream()
+    with _cabi.geometry_overlap(torch.device(DEV)):
+        for stream in (torch.cuda.current_stream(), torch.cuda.current_stream(), side):
+            with torch.cuda.stream(stream):
+                build(result)
+    assert heard == [(id(result), s.cuda_stream) for s in (torch.cuda.current_stream(), side)]
