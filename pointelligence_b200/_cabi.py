@@ -488,7 +488,10 @@ _BUILT = {}
 def _stamp(*tensors):
     """What tells whether the tensors were written to since; None for tensors of inference mode, which do not say (and
     raise when they are asked): nothing is remembered about those."""
-    return None if any(t.is_inference() for t in tensors) else tuple(t._version for t in tensors)
+    try:
+        return tuple([t._version for t in tensors])
+    except RuntimeError:
+        return None
 
 
 def mark_built(i, j, seg_offs, K, symmetric):
@@ -584,7 +587,8 @@ def mvmr(weight, feat, gather, scatter, seg_offs, tap_idx, n_out, transpose, eng
 def _plan_hook(scatter, gather, seg_offs, K, n_out, outw, inw, forced):
     """Asked by the host path for every pass the output-stationary kernel could take: the plan to run
     (buffer, blocks per group, multi-triplet buckets) or None for the scatter engine."""
-    if not forced and (not _planned_pays(gather.numel(), n_out, outw, K) or _stamp(scatter, gather, seg_offs) is None):
+    if not forced and (not _planned_pays(gather.numel(), n_out, outw, K) or scatter.is_inference()
+                       or gather.is_inference() or seg_offs.is_inference()):
         return None    # (a plan of inference tensors cannot be remembered, and one per pass does not pay)
     plan = cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, plan_group_blocks(outw))
     return plan.buffer, plan.group_blocks, plan.multi_buckets

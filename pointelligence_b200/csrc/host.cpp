@@ -56,10 +56,12 @@ void require_cuda(const OptTensor &t) {
     if (t) require_cuda(*t);
 }
 
-void require(bool ok, PyObject *type, const std::string &msg) {
+// `message` makes the text, once it is needed
+template <typename F>
+void require(bool ok, PyObject *type, F message) {
     if (ok) return;
     py::gil_scoped_acquire gil;
-    raise(type, msg);
+    raise(type, message());
 }
 std::string str(at::IntArrayRef sizes) {
     std::ostringstream s;
@@ -163,8 +165,9 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
     require_cuda(weight), require_cuda(feat), require_cuda(gather_), require_cuda(scatter_);
     require_cuda(seg_), require_cuda(tap_);
     const int code = dtype_code(feat.scalar_type());
-    require(weight.dim() == 4, PyExc_ValueError, "expected a weight (taps, groups, inputs, outputs), got " + str(weight.sizes()));
-    require(weight.scalar_type() == feat.scalar_type(), PyExc_AssertionError, "weight and features differ in type");
+    require(weight.dim() == 4, PyExc_ValueError,
+            [&] { return "expected a weight (taps, groups, inputs, outputs), got " + str(weight.sizes()); });
+    require(weight.scalar_type() == feat.scalar_type(), PyExc_AssertionError, [] { return std::string("weight and features differ in type"); });
     weight = weight.contiguous(), feat = feat.contiguous();
     const int64_t K = weight.size(0), G = weight.size(1), C = weight.size(2), M = weight.size(3);
     const bool transpose = flags & 1;
@@ -217,7 +220,7 @@ Tensor vvor(Tensor a, const Tensor &a_idx_, Tensor b, const Tensor &b_idx_, cons
             int64_t n_o, int64_t engine) {
     require_cuda(a), require_cuda(b), require_cuda(a_idx_), require_cuda(b_idx_), require_cuda(seg_), require_cuda(o_idx_);
     const int code = dtype_code(a.scalar_type());
-    require(a.scalar_type() == b.scalar_type(), PyExc_AssertionError, "operands differ in type");
+    require(a.scalar_type() == b.scalar_type(), PyExc_AssertionError, [] { return std::string("operands differ in type"); });
     a = a.contiguous(), b = b.contiguous();
     const int64_t G = a.size(1), Ma = a.size(2), Cb = b.size(2);
     c10::cuda::CUDAGuard guard(a.device());
@@ -274,15 +277,17 @@ Tensor as4(const Tensor &w) { return w.dim() == 4 ? w : w.unsqueeze(1); }
 Tensor conv_forward(const Tensor &weight, const Tensor &feat, const Tensor &bias, const Tensor &i, const Tensor &j,
                     const Tensor &seg, const ConvSizes &s) {
     Tensor w = as4(weight), x = feat;
-    require(w.dim() == 4, PyExc_ValueError, "expected a weight (taps, groups, inputs, outputs), got " + str(weight.sizes()));
-    require(w.size(0) == s.K && x.dim() == 2 && x.size(1) == w.size(1) * w.size(2), PyExc_AssertionError,
-            "features " + str(x.sizes()) + " do not fit a weight " + str(weight.sizes()) + " of " + std::to_string(s.K) + " taps");
+    require(w.dim() == 4, PyExc_ValueError,
+            [&] { return "expected a weight (taps, groups, inputs, outputs), got " + str(weight.sizes()); });
+    require(w.size(0) == s.K && x.dim() == 2 && x.size(1) == w.size(1) * w.size(2), PyExc_AssertionError, [&] {
+        return "features " + str(x.sizes()) + " do not fit a weight " + str(weight.sizes()) + " of " + std::to_string(s.K) + " taps";
+    });
     require(x.size(0) == s.n_in, PyExc_AssertionError,
-            "feat rows " + std::to_string(x.size(0)) + " != index.N_in " + std::to_string(s.n_in));
+            [&] { return "feat rows " + std::to_string(x.size(0)) + " != index.N_in " + std::to_string(s.n_in); });
     match(w, x);
     require(!bias.defined() || (bias.dim() == 1 && bias.numel() == w.size(1) * w.size(3) && bias.device() == x.device() &&
                                 bias.scalar_type() == x.scalar_type()),   // the kernels read it by address
-            PyExc_ValueError, "the bias does not fit a weight " + str(weight.sizes()));
+            PyExc_ValueError, [&] { return "the bias does not fit a weight " + str(weight.sizes()); });
     int64_t engine = g_engine;
     if (s.cover_out && i.numel() == s.n_out) engine |= FAN_IN_ONE;   // one triplet per output row: stored, not reduced
     return mvmr_impl(w, x, j, i, seg, std::nullopt, s.n_out, 0, engine, bias.defined() ? bias.contiguous() : bias)
@@ -361,7 +366,7 @@ Tensor f32_or_none(const OptTensor &t) { return t ? t->detach().to(at::kFloat).c
 
 std::tuple<Tensor, Tensor, Tensor> layer_norm_forward(Tensor x, const Tensor &lengths_, const OptTensor &weight_,
                                                       const OptTensor &bias_, const OptTensor &residual_, double eps, bool relu) {
-    require(x.dim() == 2, PyExc_ValueError, "expected rows (points, channels), got " + str(x.sizes()));
+    require(x.dim() == 2, PyExc_ValueError, [&] { return "expected rows (points, channels), got " + str(x.sizes()); });
     require_cuda(x), require_cuda(lengths_), require_cuda(weight_), require_cuda(bias_), require_cuda(residual_);
     const int code = dtype_code(x.scalar_type());
     c10::cuda::CUDAGuard guard(x.device());

@@ -158,6 +158,8 @@ _tig_mvmr_op.register_autograd(_tig_backward, setup_context=_tig_setup)
 
 
 _PLAIN = (Tensor, torch.nn.Parameter)
+_is_compiling, _dispatch_modes = torch.compiler.is_compiling, torch._C._len_torch_dispatch_stack
+_tracing, _transforms = torch._C._get_tracing_state, torch._C._are_functorch_transforms_active
 
 
 def _takes_host_path(*tensors):
@@ -165,8 +167,7 @@ def _takes_host_path(*tensors):
     transforms operators sees the registered one instead: tracing (``torch.compile``, ``jit.trace``, ``make_fx``),
     dispatch modes (FLOP counters, selective checkpointing), ``torch.func`` transforms, forward-mode differentiation
     and tensor subclasses."""
-    if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() or torch._C._get_tracing_state() is not None
-            or torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0):
+    if _is_compiling() or _dispatch_modes() or _tracing() is not None or _transforms() or forward_ad._current_level >= 0:
         return False
     for t in tensors:
         if t is not None and (type(t) not in _PLAIN or not t.is_cuda):
