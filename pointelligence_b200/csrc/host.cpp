@@ -445,7 +445,13 @@ struct LayerNorm : public torch::autograd::Function<LayerNorm> {
 
 Tensor layer_norm(const Tensor &x, const Tensor &lengths, const OptTensor &weight, const OptTensor &bias,
                   const OptTensor &residual, double eps, bool relu) {
-    // also without gradients: torch.func transforms and forward-mode tangents are refused there, not dropped
+    // the node refuses torch.func transforms and forward-mode tangents; the kernels alone would drop them
+    const bool transforms = c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+    const auto wants = [](const OptTensor &t) {
+        return t && ((at::GradMode::is_enabled() && t->requires_grad()) || t->_fw_grad(0).defined());
+    };
+    if (!transforms && !wants(x) && !wants(weight) && !wants(bias) && !wants(residual))
+        return std::get<0>(layer_norm_forward(x, lengths, weight, bias, residual, eps, relu));
     return LayerNorm::apply(x, lengths, weight, bias, residual, eps, relu);
 }
 

@@ -178,9 +178,9 @@ def _takes_host_path(*tensors):
 def _fuses(bias, weight, feat):
     """Whether the kernels can add this bias: one element per output column, of the operands' type.  Others
     (broadcast ones) are added, or refused, as torch does."""
-    columns = weight.shape[-1] * (weight.shape[1] if weight.dim() == 4 else 1)
-    return (bias.dim() == 1 and bias.numel() == columns and bias.dtype == feat.dtype == weight.dtype
-            and bias.device == feat.device)
+    shape = weight.shape
+    columns = shape[1] * shape[3] if len(shape) == 4 else shape[-1]
+    return bias.shape == (columns,) and bias.dtype == feat.dtype == weight.dtype
 
 
 def tig_mvmr(weight, feat, index, mode="auto", input_precision: Optional[str] = None, bias: Optional[Tensor] = None):
