@@ -193,7 +193,8 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
                   "counts that are multiples of 16 (of 32 beyond 256, of 48 beyond 512 ...) and at most 1024 input "
                   "channels a group");
         }
-        if (fits && (engine == ENGINE_PLANNED || plan_unasked(K, G, outw))) {
+        const bool aligned = ((uintptr_t)ptr(weight) | (uintptr_t)ptr(feat)) % 16 == 0;   // else the CUDA-core engine
+        if (fits && (engine == ENGINE_PLANNED || (plan_unasked(K, G, outw) && aligned))) {
             const Plan plan = ask_plan(scatter_, gather_, *seg_, K, n_out, outw, inw, engine == ENGINE_PLANNED);
             if (plan.valid) return mvmr_planned(weight, feat, plan, T, n_out, flags, bias);
         }

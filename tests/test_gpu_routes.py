@@ -265,3 +265,19 @@ def test_geometry_handed_to_two_streams_is_known_to_both(monkeypatch):
             with torch.cuda.stream(stream):
                 build(result)
     assert heard == [(id(result), s.cuda_stream) for s in (torch.cuda.current_stream(), side)]
+
+
+@pytest.mark.parametrize("C", [64, 384])
+def test_features_at_odd_addresses_on_a_dense_rulebook(C):
+    from pointelligence_b200 import _cabi
+
+    n, K, T = 300, 9, 6000
+    g = torch.Generator(device=DEV).manual_seed(11)
+    k = torch.sort(torch.randint(0, K, (T,), device=DEV, generator=g)).values
+    i, j = (torch.randint(0, n, (T,), device=DEV, generator=g).int() for _ in range(2))
+    seg = torch.searchsorted(k, torch.arange(K + 1, device=DEV))
+    w = torch.randn(K, 1, C, 64, device=DEV, generator=g).bfloat16() / C ** 0.5
+    x = torch.randn(n * C + 1, device=DEV, generator=g).bfloat16()[1:].view(n, C)
+    out = _cabi.mvmr(w, x, j, i, seg, None, n, False)
+    rows = torch.einsum("tc,tcm->tm", x.double()[j.long()], w[:, 0].double()[k])
+    assert _rel(out, torch.zeros(n, 64, dtype=torch.float64, device=DEV).index_add_(0, i.long(), rows)) < TOL[torch.bfloat16]
