@@ -281,3 +281,24 @@ def test_features_at_odd_addresses_on_a_dense_rulebook(C):
     out = _cabi.mvmr(w, x, j, i, seg, None, n, False)
     rows = torch.einsum("tc,tcm->tm", x.double()[j.long()], w[:, 0].double()[k])
     assert _rel(out, torch.zeros(n, 64, dtype=torch.float64, device=DEV).index_add_(0, i.long(), rows)) < TOL[torch.bfloat16]
+
+
+@pytest.mark.parametrize("C,M", [(32, 32), (70, 96), (256, 64)])
+def test_short_chunks_of_the_cuda_core_engine(C, M):
+    """Taps of no, one and around 16, 32, 64 and 128 triplets: what is multiplied of a chunk goes by its rows.  fp32
+    sums of at most 256 products of size one over 129 rows each, 2^-24 relative each: below 4e-6."""
+    from pointelligence_b200 import _cabi
+
+    sizes = [0, 1, 15, 16, 17, 31, 32, 33, 0, 63, 64, 65, 127, 128, 129, 200]
+    seg = torch.tensor([0] + sizes, device=DEV).cumsum(0)
+    T, n = int(seg[-1]), 301
+    g = torch.Generator(device=DEV).manual_seed(12)
+    k = torch.repeat_interleave(torch.arange(len(sizes), device=DEV), torch.tensor(sizes, device=DEV))
+    i, j = (torch.randint(0, n, (T,), device=DEV, generator=g).int() for _ in range(2))
+    w = torch.randn(len(sizes), 1, C, M, device=DEV, generator=g)
+    x, go = torch.randn(n, C, device=DEV, generator=g), torch.randn(n, M, device=DEV, generator=g)
+    y, gx = _cabi.mvmr(w, x, j, i, seg, None, n, False), _cabi.mvmr(w, go, i, j, seg, None, n, True)
+    wd = w[:, 0].double()[k]
+    y_ref = torch.zeros(n, M, dtype=torch.float64, device=DEV).index_add_(0, i.long(), torch.einsum("tc,tcm->tm", x.double()[j.long()], wd))
+    gx_ref = torch.zeros(n, C, dtype=torch.float64, device=DEV).index_add_(0, j.long(), torch.einsum("tm,tcm->tc", go.double()[i.long()], wd))
+    assert _rel(y, y_ref) < 4e-6 and _rel(gx, gx_ref) < 4e-6
