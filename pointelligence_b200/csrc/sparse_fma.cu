@@ -53,6 +53,7 @@ __device__ __forceinline__ void gather_f32(uint32_t tile, const T *__restrict__ 
 constexpr int MC = 128;      // triplets per chunk
 constexpr int MK = 32;       // contraction slice
 constexpr int MXP = MK + 4;  // row pitch of the gathered tile: neighbouring rows four banks apart
+constexpr int WPAD = 4;      // the same for the rows of the weight slices, which a transposed weight fills column by column
 
 struct MvmrFmaParams {
     const int32_t *gather, *scatter;
@@ -69,10 +70,10 @@ constexpr int VVOR_CTAS = 4;
 
 template <typename T, bool TRANSPOSE, int NT>
 __global__ void __launch_bounds__(NT * 4, mvmr_ctas(NT)) mvmr_fma_kernel(const T *__restrict__ W, const T *__restrict__ feat, MvmrFmaParams p) {
-    constexpr int THREADS = NT * 4;
+    constexpr int THREADS = NT * 4, WP = NT + WPAD;
     extern __shared__ __align__(16) uint8_t raw[];
     __shared__ int32_t s_cum[TABLE_TAPS + 1], s_warp_sums[THREADS / 32], s_gather[MC], s_scatter[MC];
-    const uint32_t xs = smem_u32(raw), ws = xs + MC * MXP * 4;   // gathered tile | weight slices [slice][MK][NT]
+    const uint32_t xs = smem_u32(raw), ws = xs + MC * MXP * 4;   // gathered tile | weight slices [slice][MK][WP]
     const int tid = threadIdx.x, tx = tid % (NT / 4), ty = tid / (NT / 4);   // columns 4 tx .., rows ty + 16 r
     const int32_t *cum = p.table;
     if (!cum) {
@@ -99,7 +100,7 @@ __global__ void __launch_bounds__(NT * 4, mvmr_ctas(NT)) mvmr_fma_kernel(const T
             if (TRANSPOSE) n = e / MK, kk = e % MK; else kk = e / NT, n = e % NT;
             const int k = slice * MK + kk;
             const bool ok = k < p.inw && n0 + n < p.outw;
-            sts_f32(dst + (uint32_t)(kk * NT + n) * 4, ok ? to_f32(w[TRANSPOSE ? (int64_t)(n0 + n) * p.M + k : (int64_t)k * p.M + n0 + n]) : 0.f);
+            sts_f32(dst + (uint32_t)(kk * WP + n) * 4, ok ? to_f32(w[TRANSPOSE ? (int64_t)(n0 + n) * p.M + k : (int64_t)k * p.M + n0 + n]) : 0.f);
         }
     };
     fetch(lo);
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(NT * 4, mvmr_ctas(NT)) mvmr_fma_kernel(const T
         for (int r = 0; r < 8; ++r) s[r] = make_float4(0.f, 0.f, 0.f, 0.f);
         for (int slice = 0; slice < slices; ++slice) {
             if (slice) __syncthreads();
-            const uint32_t w_at = ws + (p.keep ? (uint32_t)slice * (MK * NT * 4) : 0u);
+            const uint32_t w_at = ws + (p.keep ? (uint32_t)slice * (MK * WP * 4) : 0u);
             if (p.vec_in) gather_f32<T, MK, MXP, MC, sizeof(T) == 4>(xs, feat, s_gather, rows, slice * MK, p.inw, in_pitch, tid, THREADS);
             else gather_f32<T, MK, MXP, MC, false>(xs, feat, s_gather, rows, slice * MK, p.inw, in_pitch, tid, THREADS);
             if (!p.keep || loaded != tap) load_weight(tap, slice, w_at);
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(NT * 4, mvmr_ctas(NT)) mvmr_fma_kernel(const T
                 for (int k = 0; k < depth; k += 4) {
                     float4 w[4];
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) w[q] = lds_f4(wt + (uint32_t)((k + q) * NT) * 4);
+                    for (int q = 0; q < 4; ++q) w[q] = lds_f4(wt + (uint32_t)((k + q) * WP) * 4);
 #pragma unroll
                     for (int r = 0; r < R; ++r) {
                         const float4 x = lds_f4(x_at + (uint32_t)(16 * r * MXP + k) * 4);
@@ -269,8 +270,8 @@ __global__ void __launch_bounds__(128, VVOR_CTAS) vvor_fma_kernel(const T *__res
 }
 
 // --------------------------------------------------------------------- host ----
-int granted_smem(const void *kernel, size_t smem) {   // above 48 KB a kernel has to ask once per device
-    if (smem <= 48 * 1024) return PCX_OK;
+int granted_smem(const void *kernel, size_t smem) {   // above 48 KB, its static 5 KB included, a kernel has to ask
+    if (smem <= 42 * 1024) return PCX_OK;
     PCX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024));
     return PCX_OK;
 }
@@ -280,7 +281,7 @@ template <typename T, bool TRANSPOSE, int NT>
 int launch_mvmr(const MvmrArgs &a, MvmrFmaParams p, cudaStream_t stream) {
     const int slices = (p.inw + MK - 1) / MK;
     p.keep = slices * MK * NT * 4 <= 64 * 1024;
-    const size_t smem = (size_t)MC * MXP * 4 + (size_t)(p.keep ? slices : 1) * MK * NT * 4;
+    const size_t smem = (size_t)MC * MXP * 4 + (size_t)(p.keep ? slices : 1) * MK * (NT + WPAD) * 4;
     if (int rc = granted_smem((const void *)mvmr_fma_kernel<T, TRANSPOSE, NT>, smem)) return rc;
     const int64_t tiles = (int64_t)((p.outw + NT - 1) / NT) * p.G;
     const int occ = (int)std::max<size_t>(1, std::min<size_t>(mvmr_ctas(NT), (size_t)220 * 1024 / (smem + 6 * 1024)));
