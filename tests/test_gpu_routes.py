@@ -302,3 +302,16 @@ def test_short_chunks_of_the_cuda_core_engine(C, M):
     y_ref = torch.zeros(n, M, dtype=torch.float64, device=DEV).index_add_(0, i.long(), torch.einsum("tc,tcm->tm", x.double()[j.long()], wd))
     gx_ref = torch.zeros(n, C, dtype=torch.float64, device=DEV).index_add_(0, j.long(), torch.einsum("tm,tcm->tc", go.double()[i.long()], wd))
     assert _rel(y, y_ref) < 4e-6 and _rel(gx, gx_ref) < 4e-6
+
+
+def test_weight_gradient_of_one_tap_over_many_chunks():
+    """One tap and more chunks than CTAs add to it, in fp32: sums of up to 30 011 products of size one, whose partial
+    sums grow like the root of their number, stay below 4e-6 relative."""
+    from pointelligence_b200 import _cabi
+
+    n = 30011
+    g = torch.Generator(device=DEV).manual_seed(13)
+    ai, bi = (torch.randint(0, n, (n,), device=DEV, generator=g).int() for _ in range(2))
+    a, b = torch.randn(n, 1, 32, device=DEV, generator=g), torch.randn(n, 1, 29, device=DEV, generator=g)
+    out = _cabi.vvor(a, ai, b, bi, torch.tensor([0, n], device=DEV), None, 1)
+    assert _rel(out[0, 0], a[ai.long(), 0].double().T @ b[bi.long(), 0].double()) < 4e-6
