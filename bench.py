@@ -779,17 +779,15 @@ def backbone_setup(args, rank, world, dev):
 def backbone_split(step, params, world):
     """One instrumented step: where its time goes.  Geometry = wall clock of the library's two
     geometry entry points (each ends with a host hand-over, so the wall clock is the device time
-    plus the hand-over); convolution = the library's event timer around the MVMR / VVOR kernels;
-    norm = CUDA events around the fused layer-norm calls; all-reduce = CUDA events around it."""
+    plus the hand-over); convolution and norm = the library's event timer around the MVMR / VVOR kernels and
+    around the layer norm's; all-reduce = CUDA events around it."""
     import torch
 
     from pointelligence_b200 import _cabi
     from pointelligence_b200.dist import allreduce_gradients
 
     wall = {"geometry": 0.0}
-    norm_events = []
-    originals = {name: getattr(_cabi, name) for name in
-                 ("radius_search", "grid_sample_center_nearest", "ragged_layer_norm", "ragged_layer_norm_backward")}
+    originals = {name: getattr(_cabi, name) for name in ("radius_search", "grid_sample_center_nearest")}
 
     def timed_wall(fn):
         def inner(*a, **kw):
@@ -801,21 +799,9 @@ def backbone_split(step, params, world):
             return out
         return inner
 
-    def timed_events(fn):
-        def inner(*a, **kw):
-            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-            e0.record()
-            out = fn(*a, **kw)
-            e1.record()
-            norm_events.append((e0, e1))
-            return out
-        return inner
-
     try:
         _cabi.radius_search = timed_wall(originals["radius_search"])
         _cabi.grid_sample_center_nearest = timed_wall(originals["grid_sample_center_nearest"])
-        _cabi.ragged_layer_norm = timed_events(originals["ragged_layer_norm"])
-        _cabi.ragged_layer_norm_backward = timed_events(originals["ragged_layer_norm_backward"])
         _cabi.profile_enable(True)
         t0, t1, t2 = (torch.cuda.Event(enable_timing=True) for _ in range(3))
         torch.cuda.synchronize()
@@ -831,9 +817,9 @@ def backbone_split(step, params, world):
         _cabi.profile_enable(False)
         for name, fn in originals.items():
             setattr(_cabi, name, fn)
-    # the event timer also brackets geometry and norm kernels: keep the convolution engines' only
+    # (the event timer brackets geometry kernels too)
     conv = sum(ms for name, ms in records if name.startswith(("mvmr", "vvor", "bucket_sum")))
-    norm = sum(a.elapsed_time(b) for a, b in norm_events)
+    norm = sum(ms for name, ms in records if name.startswith("layer_norm"))
     total = t0.elapsed_time(t2)
     return {"instrumented_step_ms": total, "geometry_ms": wall["geometry"], "conv_kernels_ms": conv,
             "norm_kernels_ms": norm, "allreduce_ms": t1.elapsed_time(t2),

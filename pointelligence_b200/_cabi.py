@@ -724,17 +724,6 @@ def _f32_or_none(t):
     return None if t is None else t.detach().to(torch.float32).contiguous()
 
 
-def ragged_layer_norm(x, lengths, weight, bias, residual, eps, relu):
-    """Fused ``relu?(layer_norm_per_sample(x) * weight + bias (+ residual))``; returns ``(y, mean, rstd)``."""
-    return host().layer_norm_forward(x, lengths, weight, bias, residual, float(eps), bool(relu))
-
-
-def ragged_layer_norm_backward(grad_y, x, y, lengths, weight, mean, rstd, relu, want_affine, want_residual):
-    """Returns ``(grad_x, grad_weight|None, grad_bias|None, grad_residual|None)`` (affine gradients in fp32)."""
-    return host().layer_norm_backward(grad_y, x, y, lengths, weight, mean, rstd, bool(relu), bool(want_affine),
-                                      bool(want_residual))
-
-
 def ragged_group_norm(x, lengths, weight, bias, groups, eps):
     """Group norm per sample (``groups`` blocks of consecutive channels; ``groups == C`` is the
     instance norm); returns ``(y, mean, rstd)`` with the statistics as (S * groups,) fp32."""

@@ -612,8 +612,6 @@ PYBIND11_MODULE(_pcx_host, m) {
     m.def("conv", &conv);
     m.def("column_sums", &column_sums);
     m.def("layer_norm", &layer_norm);
-    m.def("layer_norm_forward", &layer_norm_forward);
-    m.def("layer_norm_backward", &layer_norm_backward);
     m.def("radius_taps", &radius_taps, py::call_guard<py::gil_scoped_release>());
     m.def("grid_sample", &grid_sample, py::call_guard<py::gil_scoped_release>());
     m.def("peek", &peek);

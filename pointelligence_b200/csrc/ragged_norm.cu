@@ -727,6 +727,7 @@ int pcx_ragged_layer_norm(const void *d_x, const int64_t *d_lengths, const float
     LnWs w;
     size_t need = carve_ln(d_ws, S, &w, ln_pieces(N, S));
     if (ws_bytes < need) PCX_FAIL(PCX_E_CAPACITY, "pcx_ragged_layer_norm: workspace %zu < %zu bytes", ws_bytes, need);
+    prof_begin("layer_norm(fwd)", stream);   // all of its kernels
     if (int rc = ln_offsets(d_lengths, S, N, w, stream)) return rc;
     const bool vec = vec_ok(C, dtype, {d_x, d_y, d_residual});
     const int mom_rows = layer_rows(N, C, dtype, vec, 4), rows = layer_rows(N, C, dtype, vec, 5);
@@ -738,13 +739,12 @@ int pcx_ragged_layer_norm(const void *d_x, const int64_t *d_lengths, const float
     ln_combine_kernel<<<(unsigned)S, COMBINE_THREADS, 0, stream>>>(w.rec, w.offsets, d_mean, d_rstd, S, (float)eps, mom_rows);
     PCX_LAUNCH_CHECK();
     if (N > 0) {
-        prof_begin("ln_apply_kernel", stream);
         PCX_LN_DISPATCH(dtype, vec, (ln_apply_kernel<T, VN><<<(unsigned)((N + rows - 1) / rows), LN_THREADS, 0, stream>>>(
                                    (const T *)d_x, w.offsets, d_mean, d_rstd, d_weight, d_bias, (const T *)d_residual,
                                    (T *)d_y, N, S, C, relu, rows)));
-        prof_end(stream);
         PCX_LAUNCH_CHECK();
     }
+    prof_end(stream);
     return PCX_OK;
 }
 
@@ -761,6 +761,7 @@ int pcx_ragged_layer_norm_backward(const void *d_grad_y, const void *d_x, const 
     LnWs w;
     size_t need = carve_ln(d_ws, S, &w);
     if (ws_bytes < need) PCX_FAIL(PCX_E_CAPACITY, "pcx_ragged_layer_norm_backward: workspace %zu < %zu bytes", ws_bytes, need);
+    prof_begin("layer_norm(bwd)", stream);
     if (int rc = ln_offsets(d_lengths, S, N, w, stream, true, d_grad_weight, d_grad_bias, C)) return rc;
     if (N == 0) return PCX_OK;
     const bool vec = vec_ok(C, dtype, {d_grad_y, d_x, d_y, d_grad_x, d_grad_residual});
@@ -776,6 +777,7 @@ int pcx_ragged_layer_norm_backward(const void *d_grad_y, const void *d_x, const 
     PCX_LN_DISPATCH(dtype, vec, (ln_bwd_apply_kernel<T, VN><<<grid, LN_THREADS, 0, stream>>>(
                                (const T *)(masked ? d_grad_residual : d_grad_y), (const T *)d_x, (const T *)d_y, w.offsets,
                                d_mean, d_rstd, d_weight, w.sums, w.sums + S, (T *)d_grad_x, N, S, C, masked ? 0 : relu, rows)));
+    prof_end(stream);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
 }
