@@ -421,18 +421,20 @@ __global__ void __launch_bounds__(BUCKET_SUM_THREADS) bucket_sum_kernel(const ui
 template <int FMT>
 void launch_bucket_sum(int64_t multi, int inw, const uint16_t *feat, const uint2 *entries, const uint2 *buckets,
                        const uint32_t *ctrl, uint16_t *scratch, cudaStream_t stream) {
-    // A power of two of pieces up to 32: a thread each.  Other widths in slices, blockIdx.y: a bucket costs a warp
-    // about the same whatever its lanes do, and 24 pieces left some idle.  96 and 112 channels: 16 lanes, of which a
-    // quarter idle at most (96 channels: 211 us; slices of 4 lanes 230, rows of 12 lanes 248).
+    // A power of two of pieces up to 32: a thread each.  Multiples of eight in slices of eight lanes, blockIdx.y.  Other
+    // widths take a row of the next power of two of lanes where a quarter of them idles at most, else slices of four: a
+    // bucket costs a warp about the same whatever its lanes do.  300k points, 22 triplets a row: 96 channels 207 us in 16
+    // lanes (230 in slices of four), 208 / 224 / 240 channels 384 / 391 / 406 in 32 (580 / 539 / 662), 256 457.
     const int ppr = inw >> 3;
     const bool whole = ppr <= 32 && (ppr & (ppr - 1)) == 0;
-    const int lanes = whole ? ppr : ppr % 8 == 0 ? 8 : ppr == 12 || ppr == 14 ? 16 : 4, passes = whole ? 1 : SLICE_PASSES;
+    const int lanes = whole ? ppr : ppr % 8 == 0 ? 8 : ppr == 12 || ppr == 14 ? 16 : ppr == 26 || ppr == 28 || ppr == 30 ? 32 : 4, passes = whole ? 1 : SLICE_PASSES;
     const int per_block = BUCKET_SUM_THREADS / lanes * passes;
     const dim3 grid((unsigned)((multi + per_block - 1) / per_block), (unsigned)((ppr + lanes - 1) / lanes));
 #define PCX_BS(L, P) bucket_sum_kernel<FMT, L, P><<<grid, BUCKET_SUM_THREADS, 0, stream>>>(feat, entries, buckets, ctrl, inw, scratch)
     if (!whole) {
         if (lanes == 8) PCX_BS(8, SLICE_PASSES);
         else if (lanes == 16) PCX_BS(16, SLICE_PASSES);
+        else if (lanes == 32) PCX_BS(32, SLICE_PASSES);
         else PCX_BS(4, SLICE_PASSES);
         return;
     }

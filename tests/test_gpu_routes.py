@@ -331,3 +331,20 @@ def test_time_of_the_layer_norm_is_recorded():
     _cabi.profile_enable(False)
     # 51 MB in, 51 MB out at 8 TB/s: more than 5 us each way even from the caches
     assert [name for name, ms in records if ms > 5e-3] == ["layer_norm(fwd)", "layer_norm(bwd)"]
+
+
+@pytest.mark.parametrize("C", [112, 176, 208, 224, 240])
+def test_bucket_sums_of_widths_between_the_powers_of_two(C):
+    """Rows of 14, 22, 26, 28 and 30 pieces of 16 bytes: the last lanes of a row have nothing to do."""
+    from pointelligence_b200 import _cabi
+
+    n, K, T = 300, 9, 6000
+    g = torch.Generator(device=DEV).manual_seed(14)
+    k = torch.sort(torch.randint(0, K, (T,), device=DEV, generator=g)).values
+    i, j = (torch.randint(0, n, (T,), device=DEV, generator=g).int() for _ in range(2))
+    seg = torch.searchsorted(k, torch.arange(K + 1, device=DEV))
+    w = torch.randn(K, 1, C, 64, device=DEV, generator=g).bfloat16() / C ** 0.5
+    x = torch.randn(n, C, device=DEV, generator=g).bfloat16()
+    out = _cabi.mvmr(w, x, j, i, seg, None, n, False, _cabi.ENGINE_PLANNED)
+    rows = torch.einsum("tc,tcm->tm", x.double()[j.long()], w[:, 0].double()[k])
+    assert _rel(out, torch.zeros(n, 64, dtype=torch.float64, device=DEV).index_add_(0, i.long(), rows)) < TOL[torch.bfloat16]
