@@ -140,8 +140,10 @@ int pcx_column_sums(const void *d_x, void *d_out, int64_t N, int C, int dtype,
                     void *d_ws, size_t ws_bytes, void *stream);
 
 /* ------------------------------------------------------------------------
- * Output-stationary MVMR: same result as pcx_mvmr (fp16 / bf16, one group,
- * tap-sorted triplets), computed from a "plan" of the rulebook.
+ * Output-stationary MVMR: the sums of pcx_mvmr (fp16 / bf16, tap-sorted
+ * triplets), computed from a "plan" of the rulebook.  One rounding more than
+ * pcx_mvmr: the sum of a (row, tap) bucket with several triplets is rounded to
+ * the feature type before it is multiplied, and in fp16 may leave its range.
  *
  * Replaces the same reference code as pcx_mvmr and, for the regrouping of the
  * rulebook by output row with its (row, tap) buckets summed before the
@@ -155,8 +157,9 @@ int pcx_column_sums(const void *d_x, void *d_out, int64_t N, int C, int dtype,
  * gradient: the two swapped) and use it for every layer and step that shares
  * the rulebook.  pcx_mvmr_planned then keeps the fp32 sums of every block in
  * tensor memory across all taps and writes each output row once: no
- * workspace, no zero-fill, no atomics, bit-reproducible.  Rows that no
- * triplet touches are written as zero.
+ * zero-fill, no atomics, bit-reproducible.  Rows that no triplet touches are
+ * written as zero.  The workspace holds the bucket sums and, for a small
+ * rulebook that is split over the whole chip, its fp32 sums.
  *
  *   group_blocks  blocks that share the weight tiles they stream;
  *                 pcx_mvmr_plan_group_blocks(out_width) gives the value to use
@@ -165,7 +168,9 @@ int pcx_column_sums(const void *d_x, void *d_out, int64_t N, int C, int dtype,
  *                 not valid for another).
  *   d_plan        caller-owned, 256-byte aligned, pcx_mvmr_plan_bytes(); not
  *                 written after the build
- *   limits        K <= 512, channel counts multiples of 16, out_width <= 256,
+ *   limits        K <= 512, in_width a multiple of 16 and at most 1024 (2048
+ *                 over all groups), out_width equal parts of at most 256
+ *                 channels in sixteens, at most 64 of them over all groups,
  *                 T < 2^31, ceil(n_out / 128) * K * 128 <= 2^32
  * The feature rows of a (row, tap) bucket with several triplets are summed
  * first (fp32 sum, one rounding to the feature type) into the workspace, by a

@@ -347,18 +347,29 @@ def profile_records():
 # Engine choice of ``mvmr`` with the automatic engine.  The output-stationary kernel
 # (``pcx_mvmr_planned``: accumulators in tensor memory across all taps, every output row written
 # once) needs a plan of the rulebook, built once per rulebook and direction and remembered by the
-# identity of the index tensors.  Measured on B200 it beats the scatter kernel of ``pcx_mvmr``
-#   - for dense neighbourhoods (a dozen triplets per output row and more: the deeper levels of a
-#     U-Net, dense scans), at every width, and
-#   - from four triplets per row on once the scatter kernel's fp32 accumulator (n_out x width x 4
-#     bytes) outgrows half of the 126 MB L2 and its reductions start to go to HBM: wide layers and
-#     large clouds (on the residual U-Net of the benchmark: 282 ms per step on the scatter kernel
-#     alone, 203 ms with this rule).
-# Sparse rulebooks over small accumulators and single-tap rulebooks (nothing to keep across taps)
-# stay on the scatter kernel.  So do rulebooks that are thin in tap space (fewer than 0.18 triplets
-# per output row and tap): their 128-row tiles are mostly padding.  The 125-tap stem of the benchmark
-# (16.5 triplets per row, 0.13 per row and tap, 16 input channels) takes 1.03 ms on the scatter kernel
-# against 2.56 ms plus its plan; the 27-tap layers of the finest level (0.23) stay planned.
+# identity of the index tensors.  Rooms of the benchmark's kind on B200, 27 taps, us per forward
+# pass on the scatter kernel / on this one (its plan):
+#
+#   triplets per row          16 -> 32        64 -> 64      128 -> 128     256 -> 256
+#    6.5 (150 000 points)      63 /  31        84 /  49      209 /  96      490 / 212   (179)
+#   10.1 (150 000)             85 /  38       114 /  72      295 / 132      705 / 293   (203)
+#   13.5 (150 000)            110 /  44       149 /  87      381 / 162      924 / 351   (217)
+#   21.9 (300 000)            321 /  97       403 / 215     1175 / 412                  (361)
+#    6.3 (600 000)            210 /  89       402 / 158     1054 / 304                  (337)
+#   15.3 (20 000)              32 /  27        37 /  35       78 /  51      163 / 105   (144)
+#
+# It is chosen
+#   - from twelve triplets per output row on (the deeper levels of a U-Net, dense scans), and
+#   - from four on once the scatter kernel's fp32 accumulator (n_out x width x 4 bytes) outgrows half
+#     of the 126 MB L2 and its reductions start to go to HBM: wide layers and large clouds.
+# Below that a pass gains less than the plan costs, and a rulebook may be used once.  The kernel also
+# rounds the sums of (row, tap) buckets to 16 bits, which the scatter kernel does not: the lines are
+# not moved for time alone.  Single-tap rulebooks (nothing to keep across taps) and rulebooks
+# that are thin in tap space (fewer than 0.18 triplets per output row and tap: tiles mostly padding)
+# stay on the scatter kernel.  125 taps, 130 000 points, the same pairs of widths:
+#
+#   17.5 per row, 0.14 per tap  123 / 119      157 / 250     413 / 497     1009 / 1215  (307)
+#   39.6, 0.32                  264 / 158      306 / 327     878 / 652                  (442)
 ENGINE_PLANNED = 3
 _PLANNED_DENSE_RATIO = float(os.environ.get("PCX_PLANNED_DENSE_RATIO", "12"))   # triplets per output row: always planned
 _PLANNED_MIN_RATIO = float(os.environ.get("PCX_PLANNED_MIN_RATIO", "4"))        # ... planned when the accumulator is large

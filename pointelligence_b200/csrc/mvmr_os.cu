@@ -35,13 +35,14 @@
 //   weight warp      the 64-channel slice of W[tap] for both blocks, by TMA into the same slot
 //   MMA threads      one per block: one wait per step, up to four tcgen05.mma (M = 128, N = out_width)
 //                    and one commit
+//   epilogue warps   read TMEM (tcgen05.ld), add the bias, round once and write each output row; up to 128
+//                    channels the accumulators are double-buffered, so the next group is built meanwhile
 //
 // What bounds a step (two tiles) is neither memory (the same time with every row in L2) nor the tensor core but
 // the instruction chains of the roles, some 1000 clocks each: hence single threads without votes, more teams of
 // fewer warps, and several taps a step where rows are narrow.  Forward, 300k points with 22 triplets a row:
-// 32 -> 32 channels 84 -> 64 us, 64 -> 64 93 us, 128 -> 128 185 us; 80k points, kernel 5, 16 -> 32: 209 -> 89 us.
-//   epilogue warps   read TMEM (tcgen05.ld), round once and write each output row; up to 128 channels
-//                    the accumulators are double-buffered, so the next group is built meanwhile
+// 32 -> 32 channels 64 us (84 with one tap a step), 64 -> 64 93 us, 128 -> 128 185 us; 80k points, kernel 5,
+// 16 -> 32: 89 us (209).
 //
 // Units are groups; where those do not fill the chip (small clouds, deep levels) their taps are split
 // over several CTAs, which leave fp32 sums that a last kernel adds in a fixed order.
@@ -997,9 +998,7 @@ int split_parts(int64_t ngroups, int K, int nparts) {
     return best;
 }
 
-// Output rows wider than the tensor memory's two accumulators (256 channels), and those of a grouped
-// weight, are worked off in parts of the same width.
-
+// fp32 sums of a rulebook whose taps are split
 size_t partial_bytes(int64_t n_out, int outw, int splits) {
     return splits > 1 ? (size_t)splits * ((n_out + ROWS - 1) / ROWS) * ROWS * outw * sizeof(float) : 0;
 }
@@ -1170,6 +1169,8 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
         PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_planned: sizes out of range (T=%lld n_out=%lld K=%d group=%d)", (long long)T,
                  (long long)n_out, K, G);
     const int inw = transpose ? M : C, outw = transpose ? C : M;
+    // output rows wider than the tensor memory's two accumulators (256 channels), and those of a grouped weight, are
+    // worked off in parts of the same width
     const int out_parts = parts_of(outw), nparts = groups * out_parts;
     if (inw % 16 || outw % (16 * out_parts) || inw > 1024 || groups * inw > 2048 || nparts > 64)
         PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_planned: channel counts must be multiples of 16 and the parts of an output row equal (groups=%d C=%d M=%d)", groups, C, M);

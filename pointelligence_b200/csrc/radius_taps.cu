@@ -64,6 +64,9 @@ struct TapsWs {
     int64_t buckets, nblocks;
 };
 
+// Accepted points of a query that the count pass keeps, at 5 bytes each: 240 bytes a query for kernels of up to 27 taps,
+// 480 for larger ones (half a gigabyte of workspace at a million queries).  Rooms of 2 cm voxels have 6 to 25 and 16 to
+// 75 neighbours there; the runs of a warp with a longer list are walked again.
 int kept_per_query(int k3) { return k3 <= 27 ? 48 : 96; }
 
 int bucket_bits(int64_t P) {

@@ -15,9 +15,10 @@
 //                  accumulators are double-buffered, so the next tap starts meanwhile
 //
 // Bound by what the L2 gives to gathers of whole rows, below 64 channels by the chain of a chunk (waits, copies,
-// MMA issue).  Before, the same warps did every step of a chunk, with a block barrier a chunk and the smaller chunks
-// several CTAs an SM leave room for; before and now, 300k points, 6.6 M triplets: 64 x 64 186 -> 148 us, 128 x 128 385 -> 294, 256 x 256 1042 -> 718
-// (11.3, 11.4 and 9.4 TB/s of gathered rows); 150k points, 0.98 M: 42 -> 34, 76 -> 54, 178 -> 120 us.
+// MMA issue).  300k points, 6.6 M triplets: 64 x 64 148 us, 128 x 128 294, 256 x 256 718 (11.3, 11.4 and 9.4 TB/s of
+// gathered rows); 150k points, 0.98 M: 34, 54, 120 us.  With the same warps doing every step of a chunk, and a block
+// barrier a chunk: 186, 385, 1042 and 42, 76, 178 us.  16 x 16 is 10 % slower than with those (6 of 8 lanes of a copy
+// have nothing to do): 200 000 points, 3.6 M triplets 82 against 73 us.
 //
 // Every wait is bounded (one second) and abortable: a role that gives up raises a flag in the status word and
 // in shared memory, the other roles leave their waits, and the CTA frees its TMEM and returns.
