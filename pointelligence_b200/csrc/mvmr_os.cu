@@ -340,111 +340,112 @@ __global__ void plan_entries_kernel(const uint32_t *__restrict__ key_sorted, con
     }
 }
 
-// scratch[b] = sum of the feature rows of bucket b (fp32 sum in entry order, one rounding); one thread
-// per 16-byte piece.  The row indices of up to four members are fetched together and their pieces
-// together after that, so that a bucket costs two memory latencies instead of two per member.
-// Half of its time went to issuing instructions, so: the format is a compile-time value, sums go two to an instruction,
-// the first two members (every bucket here has them) need no test and no zeros to start from.
-struct Sum8 {
-    uint64_t v[4];   // two floats each
-};
+// scratch[b] = sum of the feature rows of bucket b (fp32 sum in entry order, one rounding); a thread per 16-byte piece.
+// Widening and adding is one instruction a value (add.f32 takes a 16-bit operand); a sum starts from its first member.
 template <int FMT>
-__device__ __forceinline__ Sum8 widen(uint4 p) {
+__device__ __forceinline__ void widen(uint4 p, float *s) {
     const uint32_t w[4] = {p.x, p.y, p.z, p.w};
-    Sum8 s;
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        float2 f;
-        if (FMT) f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&w[q]));
-        else f = __half22float2(*reinterpret_cast<const __half2 *>(&w[q]));
-        asm("mov.b64 %0, {%1, %2};" : "=l"(s.v[q]) : "f"(f.x), "f"(f.y));
+        const float2 f = FMT ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162 *>(&w[q])) : __half22float2(*reinterpret_cast<const __half2 *>(&w[q]));
+        s[2 * q] = f.x, s[2 * q + 1] = f.y;
     }
-    return s;
 }
-__device__ __forceinline__ void add(Sum8 &s, const Sum8 &t) {
+template <int FMT>
+__device__ __forceinline__ void add(uint4 p, float *s) {
+    const uint32_t w[4] = {p.x, p.y, p.z, p.w};
 #pragma unroll
-    for (int q = 0; q < 4; ++q) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(s.v[q]) : "l"(t.v[q]));
+    for (int q = 0; q < 4; ++q) {
+        float &a = s[2 * q], &b = s[2 * q + 1];
+        if (FMT) asm("{.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.bf16 %0, l, %0;\n\tadd.rn.f32.bf16 %1, h, %1;}" : "+f"(a), "+f"(b) : "r"(w[q]));
+        else asm("{.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.f16 %0, l, %0;\n\tadd.rn.f32.f16 %1, h, %1;}" : "+f"(a), "+f"(b) : "r"(w[q]));
+    }
 }
 
-constexpr int BUCKET_SUM_THREADS = 256, SLICE_PASSES = 2;
+constexpr int BUCKET_SUM_THREADS = 256, BUCKET_SUM_WARPS = BUCKET_SUM_THREADS / 32, BUCKET_SUM_CTAS = 4;
 
-// LANES: threads of a bucket, a 16-byte piece each; PASSES: buckets a thread sums one after the other.
-// Bound by the latencies of the gathers and by what L1 and L2 hold, not by DRAM.  300k points, 22 triplets a row:
-// 64 channels 146 -> 132 us, 128 267 -> 242, 192 500 -> 377, 256 520 -> 474.  Tried, and slower or no faster: two
-// pieces per thread; loads that bypass the L1 (256 channels: 516 -> 625); more resident warps (623); 1024-thread or
-// looping blocks, so that an SM works on neighbouring buckets (515 - 600).
-template <int FMT, int LANES, int PASSES>
-__global__ void __launch_bounds__(BUCKET_SUM_THREADS) bucket_sum_kernel(const uint16_t *__restrict__ feat,
-                                                                        const uint2 *__restrict__ entries,
-                                                                        const uint2 *__restrict__ buckets,
-                                                                        const uint32_t *__restrict__ ctrl, int inw,
-                                                                        uint16_t *scratch) {
-    constexpr unsigned AT_ONCE = BUCKET_SUM_THREADS / LANES;
-    const unsigned piece = blockIdx.y * LANES + threadIdx.x % LANES, pitch = (unsigned)inw * 2u, nmulti = ctrl[CTRL_NMULTI];
-    if (piece * 16 >= pitch) return;
-    const char *col = reinterpret_cast<const char *>(feat + piece * 8);
-    unsigned b = blockIdx.x * (AT_ONCE * PASSES) + threadIdx.x / LANES;
-    for (int pass = 0; pass < PASSES && b < nmulti; ++pass, b += AT_ONCE) {
-        const uint2 bk = __ldg(buckets + b);
-        const uint2 *entry = entries + bk.x;
-        auto row = [&](uint32_t m) { return m < bk.y ? __ldg(&entry[m].y) : 0u; };
-        auto piece_of = [&](uint32_t r) { return __ldg(reinterpret_cast<const uint4 *>(col + (uint64_t)r * pitch)); };
-        const uint32_t r0 = __ldg(&entry[0].y), r1 = __ldg(&entry[1].y), r2 = row(2), r3 = row(3);
-        const uint4 v0 = piece_of(r0), v1 = piece_of(r1);
-        uint4 v2 = make_uint4(0, 0, 0, 0), v3 = v2;
-        if (bk.y > 2) v2 = piece_of(r2);
-        if (bk.y > 3) v3 = piece_of(r3);
-        Sum8 sum = widen<FMT>(v0);
-        add(sum, widen<FMT>(v1));
-        if (bk.y > 2) add(sum, widen<FMT>(v2));
-        if (bk.y > 3) add(sum, widen<FMT>(v3));
-        for (uint32_t m0 = 4; m0 < bk.y; m0 += 4) {
-            uint32_t rows[4];
-            uint4 v[4];
+// LANES: threads of a bucket.  A warp fetches the descriptors and the first four rows of up to 32 consecutive buckets at
+// once, a lane each, then sums them 32 / LANES at a time.
+//
+// Bound by the latency of the gathers.  With a bucket per LANES threads of a grid that covers them all, each waited for
+// its descriptor, its rows' indices and its rows in turn and took 144 instructions (72 now).  The warps of the whole chip
+// walk through the buckets together (round after round, not a range each): what they gather at one time lies in few blocks
+// of the plan, 250 against 297 us.  Rounds are of equal size: a last one of few buckets left 13 % of the chip idle.
+// 200k points, 22 triplets a row: 32 channels 50 -> 44 us, 64 88 -> 70, 96 141 -> 106, 128 160 -> 113, 192 245 -> 197,
+// 256 305 -> 250, 512 647 -> 517.  Slower: 5 and 6 CTAs an SM (spills), the next bucket's rows fetched early at 3 CTAs
+// (368), several pieces a thread (550 - 1090).
+template <int FMT, int LANES>
+__global__ void __launch_bounds__(BUCKET_SUM_THREADS, BUCKET_SUM_CTAS) bucket_sum_kernel(const uint16_t *__restrict__ feat,
+                                                                                         const uint2 *__restrict__ entries,
+                                                                                         const uint2 *__restrict__ buckets,
+                                                                                         const uint32_t *__restrict__ ctrl, int inw,
+                                                                                         uint16_t *__restrict__ scratch) {
+    constexpr int AT_ONCE = 32 / LANES;
+    const int lane = threadIdx.x & 31, sub = lane / LANES, nmulti = (int)ctrl[CTRL_NMULTI];
+    const unsigned piece = blockIdx.y * LANES + lane % LANES, pitch = (unsigned)inw * 2u;
+    const bool piece_ok = piece * 16 < pitch;   // a lane without a piece takes part in the shuffles
+    const char *col = reinterpret_cast<const char *>(feat) + (piece_ok ? piece * 16 : 0);
+    char *dst = reinterpret_cast<char *>(scratch) + piece * 16;
+    const int warps = (int)gridDim.x * BUCKET_SUM_WARPS, rounds = max((nmulti + 32 * warps - 1) / (32 * warps), 1);
+    const int batch = ((nmulti + warps * rounds - 1) / (warps * rounds) + AT_ONCE - 1) / AT_ONCE * AT_ONCE;   // at most 32
+    for (int b0 = ((int)blockIdx.x * BUCKET_SUM_WARPS + (int)(threadIdx.x >> 5)) * batch; b0 < nmulti; b0 += warps * batch) {
+        const int n = min(batch, nmulti - b0);
+        const uint2 bk = lane < n ? __ldg(buckets + b0 + lane) : make_uint2(0u, 0u);
+        uint32_t row[4];
 #pragma unroll
-            for (int m = 0; m < 4; ++m) rows[m] = row(m0 + m);
-#pragma unroll
-            for (int m = 0; m < 4; ++m) v[m] = m0 + m < bk.y ? piece_of(rows[m]) : make_uint4(0, 0, 0, 0);
-#pragma unroll
-            for (int m = 0; m < 4; ++m) add(sum, widen<FMT>(v[m]));   // an absent member adds zeros
+        for (int m = 0; m < 4; ++m) row[m] = m < (int)bk.y ? __ldg(&entries[bk.x + m].y) : 0u;
+#pragma unroll 1
+        for (int i = 0; i < n; i += AT_ONCE) {
+            const int src = i + sub;   // (below 32: n is at most the batch, a multiple of AT_ONCE)
+            auto piece_of = [&](uint32_t r) { return __ldg(reinterpret_cast<const uint4 *>(col + (uint64_t)r * pitch)); };
+            auto member = [&](int m) { return piece_of(__shfl_sync(0xffffffffu, row[m], src)); };   // an absent one reads row 0
+            const uint32_t len = __shfl_sync(0xffffffffu, bk.y, src);   // 0 behind the end
+            const bool three = __any_sync(0xffffffffu, len > 2), four = __any_sync(0xffffffffu, len > 3);
+            const uint4 v0 = member(0), v1 = member(1);
+            uint4 v2, v3;
+            if (three) v2 = member(2);
+            if (four) v3 = member(3);
+            float s[8];
+            widen<FMT>(v0, s);
+            add<FMT>(v1, s);
+            if (len > 2) add<FMT>(v2, s);
+            if (len > 3) add<FMT>(v3, s);
+            if (four) {
+                const uint32_t first = __shfl_sync(0xffffffffu, bk.x, src);
+                for (uint32_t m = 4; m < len; ++m) add<FMT>(piece_of(__ldg(&entries[first + m].y)), s);
+            }
+            uint4 o;
+            o.x = pack2(s[0], s[1], FMT), o.y = pack2(s[2], s[3], FMT);
+            o.z = pack2(s[4], s[5], FMT), o.w = pack2(s[6], s[7], FMT);
+            // past the L2's share of the feature rows: the sums are read once, by the next kernel
+            if (piece_ok && len) __stcs(reinterpret_cast<uint4 *>(dst + (uint64_t)(uint32_t)(b0 + src) * pitch), o);
         }
-        float acc[8];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) asm("mov.b64 {%0, %1}, %2;" : "=f"(acc[2 * q]), "=f"(acc[2 * q + 1]) : "l"(sum.v[q]));
-        uint4 o;
-        o.x = pack2(acc[0], acc[1], FMT), o.y = pack2(acc[2], acc[3], FMT);
-        o.z = pack2(acc[4], acc[5], FMT), o.w = pack2(acc[6], acc[7], FMT);
-        // past the L2's share of the feature rows: the sums are read once, by the next kernel
-        __stcs(reinterpret_cast<uint4 *>(reinterpret_cast<char *>(scratch + piece * 8) + (uint64_t)b * pitch), o);
     }
 }
 
 template <int FMT>
 void launch_bucket_sum(int64_t multi, int inw, const uint16_t *feat, const uint2 *entries, const uint2 *buckets,
                        const uint32_t *ctrl, uint16_t *scratch, cudaStream_t stream) {
-    // A power of two of pieces up to 32: a thread each.  Multiples of eight in slices of eight lanes, blockIdx.y.  Other
-    // widths take a row of the next power of two of lanes where a quarter of them idles at most, else slices of four: a
-    // bucket costs a warp about the same whatever its lanes do.  300k points, 22 triplets a row: 96 channels 207 us in 16
-    // lanes (230 in slices of four), 208 / 224 / 240 channels 384 / 391 / 406 in 32 (580 / 539 / 662), 256 457.
+    // Up to 128 channels the next power of two of lanes, beyond that slices (blockIdx.y) of 32, 16 or 8 lanes, whichever
+    // idles least: 192 channels 197 us in slices of 8 (223 of 32), 384 386 of 16 (444 of 8, 429 of 32), 256 255 of 32
+    // (245 of 16, 268 of 8), 208 241 of 32 (249 of 16).  Below: 48 channels 63 us in 8 lanes (80 in slices of 2).
     const int ppr = inw >> 3;
-    const bool whole = ppr <= 32 && (ppr & (ppr - 1)) == 0;
-    const int lanes = whole ? ppr : ppr % 8 == 0 ? 8 : ppr == 12 || ppr == 14 ? 16 : ppr == 26 || ppr == 28 || ppr == 30 ? 32 : 4, passes = whole ? 1 : SLICE_PASSES;
-    const int per_block = BUCKET_SUM_THREADS / lanes * passes;
-    const dim3 grid((unsigned)((multi + per_block - 1) / per_block), (unsigned)((ppr + lanes - 1) / lanes));
-#define PCX_BS(L, P) bucket_sum_kernel<FMT, L, P><<<grid, BUCKET_SUM_THREADS, 0, stream>>>(feat, entries, buckets, ctrl, inw, scratch)
-    if (!whole) {
-        if (lanes == 8) PCX_BS(8, SLICE_PASSES);
-        else if (lanes == 16) PCX_BS(16, SLICE_PASSES);
-        else if (lanes == 32) PCX_BS(32, SLICE_PASSES);
-        else PCX_BS(4, SLICE_PASSES);
-        return;
+    int lanes = 2;
+    while (lanes < ppr && lanes < 16) lanes <<= 1;
+    if (ppr > 16) {
+        lanes = 32;
+        for (const int l : {16, 8})
+            if ((ppr + l - 1) / l * l < (ppr + lanes - 1) / lanes * lanes) lanes = l;
     }
+    const int slices = (ppr + lanes - 1) / lanes, at_once = BUCKET_SUM_THREADS / lanes;
+    const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>((multi + at_once - 1) / at_once, num_sms() * BUCKET_SUM_CTAS / slices)), (unsigned)slices);
+#define PCX_BS(L) bucket_sum_kernel<FMT, L><<<grid, BUCKET_SUM_THREADS, 0, stream>>>(feat, entries, buckets, ctrl, inw, scratch)
     switch (lanes) {
-        case 2: PCX_BS(2, 1); break;
-        case 4: PCX_BS(4, 1); break;
-        case 8: PCX_BS(8, 1); break;
-        case 16: PCX_BS(16, 1); break;
-        default: PCX_BS(32, 1); break;
+        case 2: PCX_BS(2); break;
+        case 4: PCX_BS(4); break;
+        case 8: PCX_BS(8); break;
+        case 16: PCX_BS(16); break;
+        default: PCX_BS(32); break;
     }
 #undef PCX_BS
 }

@@ -250,3 +250,29 @@ def test_symmetric_rulebook_input_gradient_reuses_the_forward_plan(monkeypatch):
     for mode in ("1", "0"):
         err = (grads[mode][0].double() - want).norm() / want.norm()
         assert float(err) < 1e-2, (mode, float(err))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("width", [16, 32, 48, 64, 80, 128, 160, 192, 208, 240, 256])   # every split of a row over lanes and slices
+@pytest.mark.parametrize("rows", [1, 33, 20000])   # one bucket, a batch and one more, several rounds of the chip
+def test_bucket_sums_bit_for_bit(rows, width, dtype):
+    """One tap and the identity as its weight: a row of the result is the sum of its bucket, added in fp32 in the order of
+    the triplets and rounded once."""
+    from pointelligence_b200 import _cabi
+
+    rng = np.random.default_rng(rows + width)
+    lens = rng.integers(1, 10, rows)
+    lens[0] = 7
+    i = np.repeat(np.arange(rows), lens).astype(np.int32)
+    j = rng.integers(0, 500, len(i)).astype(np.int32)
+    x = _t(rng.standard_normal((500, width))).to(dtype)
+    seg = np.array([0, len(i)], np.int64)
+    plan = _cabi.mvmr_plan(_t(i), _t(j), _t(seg), 1, rows, _cabi.plan_group_blocks(width))
+    out = _cabi.mvmr_planned(torch.eye(width, device=DEV, dtype=dtype).view(1, 1, width, width), x, plan, False)
+    first = np.cumsum(lens) - lens
+    want = torch.zeros(rows, width, device=DEV)
+    for m in range(int(lens.max())):
+        have = _t(lens > m)
+        want[have] += x[_t(j[np.minimum(first + m, len(j) - 1)].astype(np.int64))].float()[have]
+    assert torch.equal(out, want.to(dtype))
+    assert _cabi.device_status() == 0
