@@ -72,11 +72,12 @@ __device__ __forceinline__ int tap_of(float qx, float qy, float qz, float4 p, fl
 // The same tap without the three IEEE divisions where that is safe: rint(d / g) equals rint(d * (1 / g))
 // unless the quotient lies within a few ulp of a half-integer, because the product differs from the
 // correctly rounded quotient by at most about two ulp.  A component whose product is farther than
-// 0.49 from its nearest integer (or large) is decided by the exact division, as in tap_of.
+// 0.4999 from its nearest integer, or beyond 64 (where two ulp are 1.5e-5), is decided by the exact division, as in tap_of.
+// (At 0.49 one axis in fifty took the division, and so a warp with 32 points nearly always.)
 __device__ __forceinline__ int tap_axis_fast(float d, float g32, float inv_g) {
     const float t = __fmul_rn(d, inv_g);
     const float r = rintf(t);
-    if (fabsf(t - r) > 0.49f || fabsf(t) > 4096.f) return __float2int_rn(__fdiv_rn(d, g32));
+    if (!(fabsf(t - r) <= 0.4999f && fabsf(t) <= 64.f)) return __float2int_rn(__fdiv_rn(d, g32));
     return (int)r;
 }
 __device__ __forceinline__ int tap_of_fast(float qx, float qy, float qz, float4 p, float g32, float inv_g, int K) {

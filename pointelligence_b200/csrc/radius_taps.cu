@@ -12,16 +12,17 @@
 //     the right cell keep their relative order (the sort is stable), so the output does not change.
 //     The low three bits of the hash are the parities of the cell coordinates, so the eight cells
 //     a query looks at always land in eight different buckets.
-//   * eight lanes serve one query: each looks up the run of one of its cells, then the eight runs are walked as
-//     ONE list, 32 candidates at a time, so that lanes do not wait for the longest run (a lane per run kept
-//     22 % of them busy) and four loads per lane are in flight; the accepted points of a warp are queued and
-//     their taps computed 32 at a time.  The first 48 accepted points of a query (96 for more than 27 taps)
-//     are kept with their taps, so that the fill pass only places them; a warp with a longer list walks its
-//     runs again.  A block of 256 threads serves 32 consecutive queries.
+//   * a warp serves four queries: a lane looks up the run of one of their 32 cells (cells the ball does not reach are
+//     left out) and lists it in shared memory in fours of candidates.  The list of the warp is worked off 32
+//     candidates at a time, whatever query and cell they are of, so that no lane waits for a longer run or a query
+//     with more candidates, four loads per lane in flight.  Accepted candidates are queued and their taps computed
+//     32 at a time.  The first 64 accepted points of a query (96 for more than 27 taps) are kept with their taps, so
+//     that the fill pass only places them; a warp with a longer list walks its runs again.  A block of 256 threads
+//     serves 32 consecutive queries.
 //   * the count pass leaves a per-block tap histogram; its prefix over blocks plus the tap
-//     segment offsets give every block its write position in every tap, so the fill pass places
-//     the pairs directly in tap-major order (a stable counting sort by tap inside the block):
-//     no sort of the edges, no per-query offsets.
+//     segment offsets give every block its write position in every tap, so the fill pass sorts the
+//     pairs of a block by tap (a stable counting sort in shared memory, by counts per tap and query)
+//     and writes them where they belong, neighbours next to each other: no sort of the edges, no per-query offsets.
 //   * the fill pass writes into caller buffers of a given capacity; when the total exceeds it,
 //     nothing is written and the call reports PCX_E_CAPACITY with the total, so that the caller
 //     can retry with the exact size from the state kept in the workspace.
@@ -41,7 +42,8 @@ namespace {
 constexpr int QPB = 32;           // queries per block
 constexpr int THREADS = QPB * 8;  // one lane per (query, candidate cell)
 constexpr int MAX_K3 = 128;       // taps this path handles (kernel_size 3 and 5)
-constexpr int REC_MAX = 2048;     // accepted pairs staged per round of the fill pass
+constexpr int REC_MAX = 1024;     // accepted pairs staged per round of the fill pass
+constexpr int FOURS = 64;         // fours of candidates that a warp lists at a time
 constexpr int SCAN_THREADS = 1024, SCAN_ITEMS = 4;
 
 struct TapsWs {
@@ -64,10 +66,10 @@ struct TapsWs {
     int64_t buckets, nblocks;
 };
 
-// Accepted points of a query that the count pass keeps, at 5 bytes each: 240 bytes a query for kernels of up to 27 taps,
+// Accepted points of a query that the count pass keeps, at 5 bytes each: 320 bytes a query for kernels of up to 27 taps,
 // 480 for larger ones (half a gigabyte of workspace at a million queries).  Rooms of 2 cm voxels have 6 to 25 and 16 to
 // 75 neighbours there; the runs of a warp with a longer list are walked again.
-int kept_per_query(int k3) { return k3 <= 27 ? 48 : 96; }
+int kept_per_query(int k3) { return k3 <= 27 ? 64 : 96; }
 
 int bucket_bits(int64_t P) {
     int b = 1;
@@ -154,7 +156,7 @@ struct TapArgs {
     int32_t *out_i, *out_j, *out_k;
     int64_t Q, nblocks, capacity;
     uint32_t mask;
-    float r32, inv, g32, inv_g, s_max;
+    float r32, inv, g32, inv_g, s_max, cell, reach;   // cell: side of a cell; reach: square of the radius, with a margin
     int distance_type, variant, K, k3, use_s_max;
 };
 
@@ -162,10 +164,12 @@ struct TapArgs {
 // rounded, so sqrt(s) <= R holds exactly for the sums s up to the largest float whose root is <= R
 // (s_max, found on the host).  The approximate-root variant and the Chebyshev distance keep the
 // shared expression.
+// FUSED: the usual case (Euclidean distance, sums of squares by fused multiply-adds) as a compile-time constant.
+template <bool FUSED>
 __device__ __forceinline__ bool accept_fast(const TapArgs &a, float qx, float qy, float qz, float4 p) {
-    if (a.use_s_max) {
+    if (FUSED || a.use_s_max) {
         const float dx = __fsub_rn(qx, p.x), dy = __fsub_rn(qy, p.y), dz = __fsub_rn(qz, p.z);
-        const float s = a.variant == 0 ? __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz))
+        const float s = !FUSED && a.variant == 0 ? __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz))
                                        : __fmaf_rn(dz, dz, __fmaf_rn(dx, dx, __fmul_rn(dy, dy)));
         return s <= a.s_max;
     }
@@ -173,117 +177,159 @@ __device__ __forceinline__ bool accept_fast(const TapArgs &a, float qx, float qy
     return radius_accept(qx, qy, qz, p, a.r32, a.distance_type, a.variant, &d);
 }
 
-// The eight candidate runs of a query as one list: lane c of the query's eight holds run c.
-struct Runs {
-    int first;   // start of this lane's run minus the candidates before it
-    int upto;    // candidates up to and including this lane's run
-    int total;   // candidates of the query
-    __device__ __forceinline__ Runs(int2 run, int c) {   // (start, length)
-        upto = run.y;
-#pragma unroll
-        for (int o = 1; o < 8; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, upto, o, 8);
-            if (c >= o) upto += v;
-        }
-        first = run.x - (upto - run.y);
-        total = __shfl_sync(0xffffffffu, upto, 7, 8);
-    }
-    __device__ __forceinline__ int at(int p) const {   // sorted position of candidate p < total
-        int o = 0;
-        if (p >= __shfl_sync(0xffffffffu, upto, 3, 8)) o = 4;
-        if (p >= __shfl_sync(0xffffffffu, upto, o + 1, 8)) o += 2;
-        if (p >= __shfl_sync(0xffffffffu, upto, o, 8)) o += 1;
-        return __shfl_sync(0xffffffffu, first, o, 8) + p;
-    }
-};
-
 // Candidate run of cell c (0 .. 7) of a query: (start, length).
 __device__ __forceinline__ int2 run_of(const TapArgs &a, float qx, float qy, float qz, int b, int c) {
     const int cx = corner_of(qx, a.r32, a.inv) + ((c >> 2) & 1);
     const int cy = corner_of(qy, a.r32, a.inv) + ((c >> 1) & 1);
     const int cz = corner_of(qz, a.r32, a.inv) + (c & 1);
+    // A cell farther from the query than the radius holds no neighbour.  A point of cell k lies at 2 R k or behind it up to
+    // the rounding of its cell, some 3e-7 of the coordinate; the predicate's own rounding is some 1e-6 of R^2.
+    if (a.distance_type == 0) {
+        auto gap = [&](float v, int k) {
+            const float lo = (float)k * a.cell, slack = 1e-6f * (fabsf(v) + 2.f * a.cell);
+            return fmaxf(fmaxf(lo - v, v - (lo + a.cell)) - slack, 0.f);
+        };
+        const float gx = gap(qx, cx), gy = gap(qy, cy), gz = gap(qz, cz);
+        if (gx * gx + gy * gy + gz * gz > a.reach) return make_int2(0, 0);
+    }
     const int2 r = a.table[cell_bucket(b, cx, cy, cz, a.mask)];
     return make_int2(r.x, r.y - r.x);
 }
 
-constexpr int DEPTH = 4;   // candidates a lane looks at together
+struct Four {
+    int first;        // sorted position of its first candidate
+    uint32_t about;   // candidates (0 - 4) | query in the warp << 3
+};
 
-// Walks the candidates of the warp's four queries: hit(accept bits of this query's eight lanes, this lane's
-// candidate accepted, its sorted position, its point) once per eight candidates, in list order.
-template <typename Hit>
-__device__ __forceinline__ void walk(const TapArgs &a, const Runs &runs, float qx, float qy, float qz, int b, int c, int lane, Hit hit) {
-    const int rounds = (__reduce_max_sync(0xffffffffu, runs.total) + 7) >> 3;
-    for (int r = 0; r < rounds; r += DEPTH) {
-        int pos[DEPTH], smp[DEPTH];
-        float4 pt[DEPTH];
-#pragma unroll
-        for (int u = 0; u < DEPTH; ++u) {
-            const int p = (r + u) * 8 + c, s = runs.at(min(p, max(runs.total - 1, 0)));
-            pos[u] = p < runs.total ? s : -1;
+// The four queries of a warp; lane l looks after cell l & 7 of query l >> 3.
+struct Queries {
+    float4 *at;   // in shared memory: coordinates, sample id (bit pattern)
+    int2 run;     // candidate run of this lane's cell: (start, length)
+    __device__ __forceinline__ Queries(const TapArgs &a, int64_t q, int lane, float4 *room) : at(room), run(make_int2(0, 0)) {
+        if (q < a.Q) {
+            const float x = a.queries[3 * q], y = a.queries[3 * q + 1], z = a.queries[3 * q + 2];
+            const int b = a.query_sample ? a.query_sample[q] : 0;
+            run = run_of(a, x, y, z, b, lane & 7);
+            if ((lane & 7) == 0) at[lane >> 3] = make_float4(x, y, z, __int_as_float(b));
         }
+        __syncwarp();
+    }
+};
+
+// Walks the candidates of a warp: hit(which of this lane's four are accepted, the first one's sorted position, its query)
+// once per 32 fours, lanes in the order of queries, cells and sorted positions.  `list`: room for FOURS entries.
+template <bool FUSED, typename Hit>
+__device__ __forceinline__ void walk(const TapArgs &a, const Queries &w, Four *list, int lane, Hit hit) {
+    const int fours = (w.run.y + 3) >> 2;
+    int upto = fours;   // fours of the cells up to this lane's
 #pragma unroll
-        for (int u = 0; u < DEPTH; ++u) {   // a foreign cell may share the bucket: its sample differs, or the distance does
-            pt[u] = pos[u] >= 0 ? a.sorted_pts[pos[u]] : make_float4(0.f, 0.f, 0.f, 0.f);
-            smp[u] = a.sorted_sample && pos[u] >= 0 ? a.sorted_sample[pos[u]] : b;
-        }
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, upto, 31), before = upto - fours;
+    for (int lo = 0; lo < total; lo += FOURS) {
+        const int here = min(total - lo, FOURS);
+        for (int k = max(lo - before, 0); k < fours && before + k < lo + FOURS; ++k)
+            list[before + k - lo] = Four{w.run.x + 4 * k, (uint32_t)min(w.run.y - 4 * k, 4) | (uint32_t)(lane >> 3) << 3};
+        __syncwarp();
+#pragma unroll 1
+        for (int t = 0; t < here; t += 32) {   // a four a lane
+            const Four e = t + lane < here ? list[t + lane] : Four{0, 0u};
+            const int query = (int)(e.about >> 3), size = (int)(e.about & 7u);
+            const float4 q = w.at[query];
+            float4 pt[4];
+            bool ok[4];
 #pragma unroll
-        for (int u = 0; u < DEPTH; ++u) {
-            const bool ok = pos[u] >= 0 && accept_fast(a, qx, qy, qz, pt[u]) && smp[u] == b;
-            const uint32_t all = __ballot_sync(0xffffffffu, ok);
-            if (all) hit(all, ok, pt[u]);
+            for (int u = 0; u < 4; ++u) pt[u] = u < size ? a.sorted_pts[e.first + u] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) ok[u] = u < size && accept_fast<FUSED>(a, q.x, q.y, q.z, pt[u]);
+            if (a.sorted_sample) {   // a foreign cell may share the bucket: its sample differs, or the distance does
+                int smp[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) smp[u] = ok[u] ? a.sorted_sample[e.first + u] : 0;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) ok[u] = ok[u] && smp[u] == __float_as_int(q.w);
+            }
+            hit(ok, e.first, query);
         }
+        __syncwarp();
     }
 }
 
+// Accepted candidates of a warp, looked at 32 at a time in the order they came: use(there, sorted position, query, place
+// among the accepted of its query).  The whole warp calls `use`.
+struct Accepted {
+    static constexpr int ROOM = 256;   // a power of two that 31 left over and four of each lane fit
+    int2 *queue;                       // ROOM entries in shared memory: sorted position, query
+    int head = 0, size = 0;
+    int n[4] = {0, 0, 0, 0};
+    __device__ __forceinline__ explicit Accepted(int2 *room) : queue(room) {}
+    template <typename Use>
+    __device__ __forceinline__ void take(int lane, int count, Use use) {
+        __syncwarp();
+        const bool there = lane < count;
+        const int2 e = queue[(head + lane) & (ROOM - 1)];
+        int place = 0;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t of = __ballot_sync(0xffffffffu, there && e.y == q);
+            if (e.y == q) place = n[q] + __popc(of & ((1u << lane) - 1u));
+            n[q] += __popc(of);
+        }
+        use(there, there ? e.x : 0, there ? e.y : 0, place);
+        head += count, size -= count;
+        __syncwarp();
+    }
+    template <typename Use>
+    __device__ __forceinline__ void add(int lane, const bool (&ok)[4], int pos, int query, Use use) {
+        const uint32_t below = (1u << lane) - 1u;
+        int at = head + size;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const uint32_t all = __ballot_sync(0xffffffffu, ok[u]);
+            at += __popc(all & below), size += __popc(all);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (ok[u]) queue[at++ & (ROOM - 1)] = make_int2(pos + u, query);
+        while (size >= 32) take(lane, 32, use);
+    }
+    template <typename Use>
+    __device__ __forceinline__ void finish(int lane, Use use) {
+        if (size) take(lane, size, use);
+    }
+};
+
+// Bound by issuing instructions (1140 a warp of four queries and some 330 candidates).  One list of candidates a warp and
+// a four a lane: 1 M points in eight rooms, 512 000 queries at a stride of two, 230 -> 170 us; 150 000 points 50 -> 35;
+// four LiDAR sweeps 68 -> 53.  Eight lanes a query with a list of their own, and pieces of eight candidates: 207, 48, 74.
+template <bool FUSED>
 __global__ void __launch_bounds__(THREADS) taps_count_kernel(TapArgs a) {
     __shared__ uint32_t s_hist[MAX_K3];
-    __shared__ float4 s_queue[THREADS / 32][64];     // accepted points whose tap is still to be computed ...
-    __shared__ uint32_t s_whose[THREADS / 32][64];   // ... and their query in the warp and place in its list
+    __shared__ __align__(16) Four s_list[THREADS / 32][FOURS];
+    __shared__ float4 s_query[THREADS / 32][4];
+    __shared__ int2 s_queue[THREADS / 32][Accepted::ROOM];
     if (threadIdx.x < MAX_K3) s_hist[threadIdx.x] = 0;
     __syncthreads();
-    const int c = threadIdx.x & 7, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t q0 = (int64_t)blockIdx.x * QPB + warp * 4, q = q0 + (lane >> 3);
-    float qx = 0.f, qy = 0.f, qz = 0.f;
-    int b = 0;
-    int2 run = make_int2(0, 0);
-    if (q < a.Q) {
-        qx = a.queries[3 * q], qy = a.queries[3 * q + 1], qz = a.queries[3 * q + 2];
-        b = a.query_sample ? a.query_sample[q] : 0;
-        run = run_of(a, qx, qy, qz, b, c);
-    }
-    const Runs runs(run, c);
-    uint32_t n = 0;
-    int head = 0, queued = 0;
-    auto taps_of_queued = [&](int count) {
-        __syncwarp();
-        const float4 p = s_queue[warp][(head + lane) & 63];
-        const uint32_t e = s_whose[warp][(head + lane) & 63];
-        const int from = lane < count ? (int)(e & 3u) * 8 : 0;
-        const float x = __shfl_sync(0xffffffffu, qx, from), y = __shfl_sync(0xffffffffu, qy, from), z = __shfl_sync(0xffffffffu, qz, from);
-        if (lane < count) {
-            const int tap = tap_of_fast(x, y, z, p, a.g32, a.inv_g, a.K);
-            atomicAdd(&s_hist[tap], 1u);
-            if ((int)(e >> 2) < a.kept) {
-                const int64_t at = (q0 + (e & 3u)) * a.kept + (e >> 2);
-                a.kept_point[at] = __float_as_int(p.w), a.kept_tap[at] = (uint8_t)tap;
-            }
+    const Queries queries(a, q, lane, s_query[warp]);
+    Accepted accepted(s_queue[warp]);
+    auto count = [&](bool there, int pos, int query, int place) {
+        if (!there) return;
+        const float4 p = a.sorted_pts[pos], c = queries.at[query];
+        const int tap = tap_of_fast(c.x, c.y, c.z, p, a.g32, a.inv_g, a.K);
+        atomicAdd(&s_hist[tap], 1u);
+        if (place < a.kept) {
+            const int64_t at = (q0 + query) * a.kept + place;
+            a.kept_point[at] = __float_as_int(p.w), a.kept_tap[at] = (uint8_t)tap;
         }
-        head += count, queued -= count;
-        __syncwarp();
     };
-    walk(a, runs, qx, qy, qz, b, c, lane, [&](uint32_t all, bool ok, const float4 &p) {
-        const uint32_t mine = (all >> (lane & 24)) & 0xffu;
-        if (ok) {
-            const int slot = (head + queued + __popc(all & ((1u << lane) - 1u))) & 63;
-            s_queue[warp][slot] = p;
-            s_whose[warp][slot] = (uint32_t)(lane >> 3) | ((n + __popc(mine & ((1u << c) - 1u))) << 2);
-        }
-        n += __popc(mine);
-        queued += __popc(all);
-        if (queued >= 32) taps_of_queued(32);
-    });
-    if (queued) taps_of_queued(queued);
-    if (q < a.Q && c == 0) {
+    walk<FUSED>(a, queries, s_list[warp], lane, [&](const bool (&ok)[4], int first, int query) { accepted.add(lane, ok, first, query, count); });
+    accepted.finish(lane, count);
+    if (q < a.Q && (lane & 7) == 0) {
+        const int n = lane == 0 ? accepted.n[0] : lane == 8 ? accepted.n[1] : lane == 16 ? accepted.n[2] : accepted.n[3];
         a.counts[q] = n;
         a.num_neighbors[q] = n;
         if (n == 0) atomicAdd((unsigned long long *)&a.ctrl_rw[3], 1ULL);
@@ -343,91 +389,156 @@ __global__ void __launch_bounds__(SCAN_THREADS) taps_colscan_kernel(uint32_t *bl
     }
 }
 
-__global__ void __launch_bounds__(THREADS) taps_fill_kernel(TapArgs a) {
-    using Scan = cub::BlockScan<uint32_t, THREADS>;
-    const int kpad = (a.k3 + 31) & ~31;
-    __shared__ typename Scan::TempStorage tmp;
-    __shared__ unsigned long long s_rec[REC_MAX];   // accepted pairs in output order
-    extern __shared__ uint16_t s_gcnt[];            // [GROUPS][kpad] per 32 records and tap: count, then prefix inside the round
-    __shared__ uint32_t s_base[MAX_K3];             // next write position of each tap for this block
-    __shared__ uint32_t s_round[MAX_K3];
-    if (a.ctrl[0] > a.capacity || a.ctrl[1]) return;
+// Up to 64 kept pairs a query (kernels of up to 27 taps) set bits, from which their places follow in any order; matching
+// lanes by tap kept one pipe 63 % busy and took 141 us instead of 111 below.  Before pairs were sorted in shared memory
+// and written side by side: 512 000 queries with 13 neighbours 175 -> 111 us, 150 000 points 37 -> 27, LiDAR 67 -> 35
+// (with 64 instead of 48 kept pairs; 65 with 48: one query in ninety has more, and its warp keeps the block waiting).
+template <bool FUSED, bool MASKS>
+__global__ void __launch_bounds__(THREADS, 5) taps_fill_kernel(TapArgs a) {
+    constexpr int WARPS = THREADS / 32;
+    struct Walk {
+        Four list[WARPS][FOURS];
+        float4 query[WARPS][4];
+        int2 queue[WARPS][Accepted::ROOM];
+    };
+    // pairs of a round as they come (point, tap | query << 8 | place among the query's pairs of that tap << 16), then by tap.
+    // Warps that walk their runs again do so before the pairs are sorted.
+    __shared__ uint2 s_rec[REC_MAX];
+    __shared__ union {
+        uint2 sorted[REC_MAX];
+        Walk walk;
+    } s_u;
+    extern __shared__ uint16_t s_cnt[];                     // [tap][query]: pairs, then those of the queries before
+    uint2 *s_mask = reinterpret_cast<uint2 *>(s_cnt + a.k3 * QPB);   // MASKS: [tap][query], a bit for each kept pair of that tap
+    __shared__ uint32_t s_base[MAX_K3];                     // next write position of each tap for this block
+    __shared__ uint32_t s_start[MAX_K3], s_total[MAX_K3];   // first place of each tap among the sorted, its pairs in this round
+    const bool fits = a.ctrl[0] <= a.capacity && !a.ctrl[1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int c = threadIdx.x & 7, ql = threadIdx.x >> 3;
     const int64_t q0 = (int64_t)blockIdx.x * QPB, q = q0 + ql;
     if ((int)threadIdx.x < a.k3)
         s_base[threadIdx.x] = (uint32_t)a.seg[threadIdx.x] + a.block_hist[(int64_t)threadIdx.x * a.nblocks + blockIdx.x];
-    const uint32_t nq = q < a.Q ? a.counts[q] : 0u;
-    uint32_t q_off, block_total;
-    Scan(tmp).ExclusiveSum(c == 0 ? nq : 0u, q_off, block_total);
-    q_off = __shfl_sync(0xffffffffu, q_off, 0, 8);
+    // pairs of the block's queries and where each query's begin: every warp for itself, a query a lane
+    const uint32_t n_lane = q0 + lane < a.Q ? a.counts[q0 + lane] : 0u;
+    if (!fits) return;   // (the counts were on their way meanwhile)
+    uint32_t upto = n_lane;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xffffffffu, upto, o);
+        if (lane >= o) upto += v;
+    }
+    const uint32_t block_total = __shfl_sync(0xffffffffu, upto, 31);
+    const uint32_t nq = __shfl_sync(0xffffffffu, n_lane, ql), q_off = __shfl_sync(0xffffffffu, upto, ql) - nq;
     const bool kept = __all_sync(0xffffffffu, nq <= (uint32_t)a.kept);   // all accepted points of the warp's queries were kept
-    __syncthreads();
     for (uint32_t lo = 0; lo < block_total; lo += REC_MAX) {
-        const uint32_t hi = lo + REC_MAX;
-        const int cnt = (int)min((uint32_t)REC_MAX, block_total - lo), groups = (cnt + 31) >> 5;
-        for (int t = threadIdx.x; t < groups * kpad; t += THREADS) s_gcnt[t] = 0;
-        // tap << 40 | local query << 32 | point index, in output order
-        if (kept) {
-            for (uint32_t e = c; e < nq; e += 8) {
-                const uint32_t pos = q_off + e;
-                if (pos >= lo && pos < hi)
-                    s_rec[pos - lo] = ((unsigned long long)a.kept_tap[q * a.kept + e] << 40) | ((unsigned long long)ql << 32) |
-                                      (uint32_t)a.kept_point[q * a.kept + e];
+        const uint32_t cnt = min((uint32_t)REC_MAX, block_total - lo);
+        for (int t = threadIdx.x; t < a.k3 * QPB / 2 * (MASKS ? 5 : 1); t += THREADS) reinterpret_cast<uint32_t *>(s_cnt)[t] = 0u;   // s_mask too
+        __syncthreads();
+        // A pair of query x of the block: its place among that query's pairs of the same tap, and into s_rec.  The whole warp
+        // calls; pairs of a query come in order, the lanes' queries do not fall.
+        auto place = [&](bool there, uint32_t pos, int x, int point, int tap) {
+            there = there && pos - lo < (uint32_t)REC_MAX;
+            const uint32_t same = __match_any_sync(0xffffffffu, there ? tap | x << 8 : 0x10000 + lane);
+            uint16_t *count = s_cnt + tap * QPB + x;
+            const uint32_t before = there ? *count : 0u, lower = same & ((1u << lane) - 1u);
+            __syncwarp();
+            if (there) {
+                s_rec[pos - lo] = make_uint2((uint32_t)point, (uint32_t)tap | (uint32_t)x << 8 | (before + __popc(lower)) << 16);
+                if (!lower) *count = (uint16_t)(before + __popc(same));
+            }
+            __syncwarp();
+        };
+        if (kept && MASKS) {
+            // a bit for each pair: whatever the order in which they come, those before one are the bits below its own
+            const uint32_t most = __reduce_max_sync(0xffffffffu, nq);
+            for (uint32_t e0 = c; e0 < most; e0 += 32) {
+                uint32_t tap[4], point[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const int64_t at = q * a.kept + e0 + 8 * u;
+                    if (e0 + 8 * u < nq) tap[u] = a.kept_tap[at], point[u] = (uint32_t)a.kept_point[at];
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const uint32_t e = e0 + 8 * u, pos = q_off + e - lo;
+                    if (e >= nq || pos >= (uint32_t)REC_MAX) continue;
+                    uint2 *mask = s_mask + tap[u] * QPB + ql;
+                    atomicOr(e < 32 ? &mask->x : &mask->y, 1u << (e & 31));
+                    s_rec[pos] = make_uint2(point[u], tap[u] | (uint32_t)ql << 8 | e << 16);
+                }
+            }
+        } else if (kept) {
+            const uint32_t most = (__reduce_max_sync(0xffffffffu, nq) + 7) & ~7u;
+            for (uint32_t e = c; e < most; e += 8) {
+                const bool there = e < nq;
+                place(there, q_off + e, ql, there ? a.kept_point[q * a.kept + e] : 0, there ? a.kept_tap[q * a.kept + e] : 0);
             }
         } else {
-            float qx = 0.f, qy = 0.f, qz = 0.f;
-            int b = 0;
-            int2 run = make_int2(0, 0);
-            if (nq) {
-                qx = a.queries[3 * q], qy = a.queries[3 * q + 1], qz = a.queries[3 * q + 2];
-                b = a.query_sample ? a.query_sample[q] : 0;
-                run = run_of(a, qx, qy, qz, b, c);
+            const Queries queries(a, q, lane, s_u.walk.query[warp]);
+            Accepted accepted(s_u.walk.queue[warp]);
+            auto put = [&](bool there, int pos, int query, int nth) {
+                const float4 p = a.sorted_pts[pos], at = queries.at[query];
+                const int tap = there ? tap_of_fast(at.x, at.y, at.z, p, a.g32, a.inv_g, a.K) : 0;
+                place(there, __shfl_sync(0xffffffffu, q_off, query * 8) + (uint32_t)nth, warp * 4 + query, __float_as_int(p.w), tap);
+            };
+            walk<FUSED>(a, queries, s_u.walk.list[warp], lane, [&](const bool (&ok)[4], int first, int query) { accepted.add(lane, ok, first, query, put); });
+            accepted.finish(lane, put);
+        }
+        __syncthreads();
+        // a warp per tap: the pairs of the queries before each query
+        for (int tap = warp; tap < a.k3; tap += WARPS) {
+            uint32_t v = s_cnt[tap * QPB + lane];
+            if (MASKS) {
+                const uint2 m = s_mask[tap * QPB + lane];
+                v += __popc(m.x) + __popc(m.y);   // a warp's pairs are in one or the other
             }
-            const Runs runs(run, c);
-            uint32_t at = q_off;
-            walk(a, runs, qx, qy, qz, b, c, lane, [&](uint32_t all, bool ok, const float4 &p) {
-                const uint32_t mine = (all >> (lane & 24)) & 0xffu, pos = at + __popc(mine & ((1u << c) - 1u));
-                if (ok && pos >= lo && pos < hi)
-                    s_rec[pos - lo] = ((unsigned long long)tap_of_fast(qx, qy, qz, p, a.g32, a.inv_g, a.K) << 40) |
-                                      ((unsigned long long)ql << 32) | (uint32_t)__float_as_int(p.w);
-                at += __popc(mine);
-            });
-        }
-        __syncthreads();
-        // stable counting sort by tap: count per (32 records, tap), prefix over the groups, place
-        for (int g = warp; g < groups; g += THREADS / 32) {
-            const int idx = g * 32 + lane;
-            const int tap = idx < cnt ? (int)(s_rec[idx] >> 40) : 0xffff;
-            const unsigned m = __match_any_sync(0xffffffffu, tap);
-            if (idx < cnt && lane == __ffs(m) - 1) s_gcnt[g * kpad + tap] = (uint16_t)__popc(m);
-        }
-        __syncthreads();
-        if ((int)threadIdx.x < a.k3) {
-            uint32_t run = 0;
-            for (int g = 0; g < groups; ++g) {
-                const uint32_t v = s_gcnt[g * kpad + threadIdx.x];
-                s_gcnt[g * kpad + threadIdx.x] = (uint16_t)run;
-                run += v;
+            uint32_t incl = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += up;
             }
-            s_round[threadIdx.x] = run;
+            s_cnt[tap * QPB + lane] = (uint16_t)(incl - v);
+            if (lane == 31) s_total[tap] = incl;
         }
         __syncthreads();
-        for (int g = warp; g < groups; g += THREADS / 32) {
-            const int idx = g * 32 + lane;
-            const unsigned long long rec = idx < cnt ? s_rec[idx] : ~0ULL;
-            const int tap = idx < cnt ? (int)(rec >> 40) : 0xffff;
-            const unsigned m = __match_any_sync(0xffffffffu, tap);
-            if (idx < cnt) {
-                const uint32_t pos = s_base[tap] + s_gcnt[g * kpad + tap] + __popc(m & ((1u << lane) - 1u));
-                a.out_i[pos] = (int32_t)(q0 + (int)((rec >> 32) & 0xff));
-                a.out_j[pos] = (int32_t)(uint32_t)rec;
-                if (a.out_k) a.out_k[pos] = tap;
+        if (warp == 0) {   // k3 <= 128: four taps per lane
+            uint32_t v[4], sum = 0;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = lane * 4 + u < a.k3 ? s_total[lane * 4 + u] : 0u, sum += v[u];
+            uint32_t incl = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += up;
             }
+            uint32_t first = incl - sum;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) s_start[lane * 4 + u] = first, first += v[u];
         }
         __syncthreads();
-        if ((int)threadIdx.x < a.k3) s_base[threadIdx.x] += s_round[threadIdx.x];
+        for (uint32_t x = threadIdx.x; x < cnt; x += THREADS) {
+            const uint2 rec = s_rec[x];
+            const uint32_t tap = rec.y & 0xffu;
+            const uint32_t at = tap * QPB + ((rec.y >> 8) & 0xffu);
+            uint32_t nth = rec.y >> 16;
+            if (MASKS) {
+                const uint2 m = s_mask[at];
+                if (m.x | m.y) nth = __popc(m.x & (nth < 32 ? (1u << nth) - 1u : ~0u)) + __popc(m.y & (nth < 32 ? 0u : (1u << (nth - 32)) - 1u));
+            }
+            s_u.sorted[s_start[tap] + s_cnt[at] + nth] = rec;
+        }
         __syncthreads();
+        for (uint32_t x = threadIdx.x; x < cnt; x += THREADS) {
+            const uint2 rec = s_u.sorted[x];
+            const uint32_t tap = rec.y & 0xffu, pos = s_base[tap] + x - s_start[tap];
+            a.out_i[pos] = (int32_t)(q0 + (int)((rec.y >> 8) & 0xffu));
+            a.out_j[pos] = (int32_t)rec.x;
+            if (a.out_k) a.out_k[pos] = (int32_t)tap;
+        }
+        if (lo + REC_MAX >= block_total) break;
+        __syncthreads();
+        if ((int)threadIdx.x < a.k3) s_base[threadIdx.x] += s_total[threadIdx.x];
     }
 }
 
@@ -454,6 +565,7 @@ TapArgs make_args(const TapsWs &w, const float *queries, const int32_t *point_sa
     a.Q = Q, a.nblocks = w.nblocks, a.mask = (uint32_t)(w.buckets - 1);
     a.r32 = (float)radius, a.inv = (float)(1.0 / (2.0 * radius)), a.g32 = (float)grid;
     a.inv_g = 1.0f / a.g32;
+    a.cell = (float)(2.0 * radius), a.reach = a.r32 * a.r32 * 1.0001f;
     a.distance_type = distance_type, a.variant = radius_variant(), a.K = kernel_size;
     a.k3 = kernel_size * kernel_size * kernel_size;
     a.use_s_max = distance_type == 0 && a.variant != 2;
@@ -467,6 +579,8 @@ TapArgs make_args(const TapsWs &w, const float *queries, const int32_t *point_sa
     }
     return a;
 }
+
+bool fused(const TapArgs &a) { return a.use_s_max && a.variant == 1; }
 
 // ctrl[0 .. 3] and the device status word, in one wait
 int read_ctrl(const TapsWs &w, int64_t *h, cudaStream_t stream) {
@@ -522,7 +636,7 @@ int pcx_radius_taps_count(const float *d_points, const float *d_queries, const i
     TapArgs a = make_args(w, d_queries, d_point_sample, d_query_sample, Q, radius, distance_type, kernel_size, kernel_grid_size);
     a.num_neighbors = d_num_neighbors;
     prof_begin("taps_count_kernel", stream);
-    taps_count_kernel<<<(unsigned)w.nblocks, THREADS, 0, stream>>>(a);
+    (fused(a) ? taps_count_kernel<true> : taps_count_kernel<false>)<<<(unsigned)w.nblocks, THREADS, 0, stream>>>(a);
     prof_end(stream);
     PCX_LAUNCH_CHECK();
     taps_colscan_kernel<<<k3, SCAN_THREADS, 0, stream>>>(w.block_hist, w.nblocks, k3, w.tap_total, w.seg, d_seg_offs, w.ctrl);
@@ -560,7 +674,8 @@ int pcx_radius_taps_fill(const float *d_queries, const int32_t *d_point_sample, 
     a.out_i = d_out_i, a.out_j = d_out_j, a.out_k = d_out_k, a.capacity = capacity;
     if (capacity > 0) {
         prof_begin("taps_fill_kernel", stream);
-        taps_fill_kernel<<<(unsigned)w.nblocks, THREADS, (size_t)(REC_MAX / 32) * ((k3 + 31) & ~31) * sizeof(uint16_t), stream>>>(a);
+        if (a.kept <= 64) (fused(a) ? taps_fill_kernel<true, true> : taps_fill_kernel<false, true>)<<<(unsigned)w.nblocks, THREADS, (size_t)k3 * QPB * 10, stream>>>(a);
+        else (fused(a) ? taps_fill_kernel<true, false> : taps_fill_kernel<false, false>)<<<(unsigned)w.nblocks, THREADS, (size_t)k3 * QPB * 2, stream>>>(a);
         prof_end(stream);
         PCX_LAUNCH_CHECK();
     }

@@ -206,3 +206,37 @@ def test_tap_ties_on_a_half_grid_lattice():
         ref, got = _both(pts, pts, None, None, radius, k, g)
         _assert_same(ref, got)
         assert got[0].numel() > 20 * pts.shape[0]
+
+
+# neighbours about the number that is kept of a query (64, 96), the pairs a block places at a time (1024 for 32 queries) and
+# the fours of candidates a warp lists at a time (64 for four queries); clusters a cell apart keep the runs apart
+@pytest.mark.parametrize("per", [1, 7, 31, 32, 33, 63, 64, 65, 95, 96, 97, 260])
+@pytest.mark.parametrize("k", [3, 5])
+def test_lists_of_any_length(per, k):
+    from pointelligence_b200 import _cabi
+
+    dev = torch.device("cuda:0")
+    gen = torch.Generator().manual_seed(per * k)
+    centre = torch.arange(41).float()[:, None] * torch.tensor([[0.11, 0.07, 0.0]])
+    size = torch.randint(max(1, per - 1), per + 2, (41,), generator=gen)
+    pts = torch.repeat_interleave(centre, size, 0)
+    pts = (pts + 0.01 * torch.randn(pts.shape, generator=gen))[torch.randperm(pts.shape[0], generator=gen)].to(dev)
+    _cabi._TAPS_RATIO.clear()
+    _assert_same(*_both(pts, pts, None, None, 0.05, k, 0.02))
+
+
+@pytest.mark.parametrize("shift", [0.0, -3.0, 1000.0, -20000.0])
+def test_cells_out_of_reach(shift):
+    """Points and queries on the faces, edges and corners of the search cells and a few ulp off them, where a cell is left out
+    of the search if it is farther than the radius."""
+    from pointelligence_b200 import _cabi
+
+    dev, radius = torch.device("cuda:0"), 0.05
+    rng = np.random.default_rng(5)
+    p = (np.round(rng.uniform(-8, 8, (6000, 3))) * radius + shift).astype(np.float32)   # cells are two radii wide
+    for _ in range(3):
+        p = np.where(rng.random(p.shape) < 0.3, np.nextafter(p, np.float32(np.inf) * rng.choice([-1, 1], p.shape).astype(np.float32)), p)
+    q = p[rng.permutation(len(p))][:3000]
+    q = np.where(rng.random(q.shape) < 0.3, q + rng.uniform(-radius, radius, q.shape).astype(np.float32), q).astype(np.float32)
+    _cabi._TAPS_RATIO.clear()
+    _assert_same(*_both(torch.from_numpy(p).to(dev), torch.from_numpy(q).to(dev), None, None, radius, 3, 0.02))
