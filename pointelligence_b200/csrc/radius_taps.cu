@@ -16,7 +16,7 @@
 //     left out) and lists it in shared memory in fours of candidates.  The list of the warp is worked off 32
 //     candidates at a time, whatever query and cell they are of, so that no lane waits for a longer run or a query
 //     with more candidates, four loads per lane in flight.  Accepted candidates are queued and their taps computed
-//     32 at a time.  The first 64 accepted points of a query (96 for more than 27 taps) are kept with their taps, so
+//     32 at a time.  The first 64 accepted points of a query (128 for more than 27 taps) are kept with their taps, so
 //     that the fill pass only places them; a warp with a longer list walks its runs again.  A block of 256 threads
 //     serves 32 consecutive queries.
 //   * the count pass leaves a per-block tap histogram; its prefix over blocks plus the tap
@@ -42,7 +42,6 @@ namespace {
 constexpr int QPB = 32;           // queries per block
 constexpr int THREADS = QPB * 8;  // one lane per (query, candidate cell)
 constexpr int MAX_K3 = 128;       // taps this path handles (kernel_size 3 and 5)
-constexpr int REC_MAX = 1024;     // accepted pairs staged per round of the fill pass
 constexpr int FOURS = 64;         // fours of candidates that a warp lists at a time
 constexpr int SCAN_THREADS = 1024, SCAN_ITEMS = 4;
 
@@ -67,9 +66,9 @@ struct TapsWs {
 };
 
 // Accepted points of a query that the count pass keeps, at 5 bytes each: 320 bytes a query for kernels of up to 27 taps,
-// 480 for larger ones (half a gigabyte of workspace at a million queries).  Rooms of 2 cm voxels have 6 to 25 and 16 to
+// 640 for larger ones (0.6 gigabytes of workspace at a million queries).  Rooms of 2 cm voxels have 6 to 25 and 16 to
 // 75 neighbours there; the runs of a warp with a longer list are walked again.
-int kept_per_query(int k3) { return k3 <= 27 ? 64 : 96; }
+int kept_per_query(int k3) { return k3 <= 27 ? 64 : 128; }
 
 int bucket_bits(int64_t P) {
     int b = 1;
@@ -389,27 +388,29 @@ __global__ void __launch_bounds__(SCAN_THREADS) taps_colscan_kernel(uint32_t *bl
     }
 }
 
-// Up to 64 kept pairs a query (kernels of up to 27 taps) set bits, from which their places follow in any order; matching
-// lanes by tap kept one pipe 63 % busy and took 141 us instead of 111 below.  Before pairs were sorted in shared memory
-// and written side by side: 512 000 queries with 13 neighbours 175 -> 111 us, 150 000 points 37 -> 27, LiDAR 67 -> 35
-// (with 64 instead of 48 kept pairs; 65 with 48: one query in ninety has more, and its warp keeps the block waiting).
-template <bool FUSED, bool MASKS>
-__global__ void __launch_bounds__(THREADS, 5) taps_fill_kernel(TapArgs a) {
+// Kept pairs are counted by shared-memory additions in any order and put in order within their few neighbours of the same
+// query and tap when they are written; matching lanes by tap kept one pipe 63 % busy and took 141 us instead of 111 below.
+// Before pairs were sorted in shared memory and written side by side: 512 000 queries with 13 neighbours 175 -> 112 us,
+// 150 000 points 37 -> 26, LiDAR 67 -> 38 (with 64 instead of 48 kept pairs; 65 with 48: one query in ninety has more,
+// and its warp keeps the block waiting), 125 taps, 100 000 queries with 41 152 -> 110
+template <bool FUSED, int REC_MAX>   // pairs staged per round
+__global__ void __launch_bounds__(THREADS, REC_MAX > 1024 ? 4 : 5) taps_fill_kernel(TapArgs a) {
     constexpr int WARPS = THREADS / 32;
     struct Walk {
         Four list[WARPS][FOURS];
         float4 query[WARPS][4];
         int2 queue[WARPS][Accepted::ROOM];
     };
-    // pairs of a round as they come (point, tap | query << 8 | place among the query's pairs of that tap << 16), then by tap.
+    // pairs of a round as they come (point, tap | query << 8 | place among the query's pairs << 16), then by tap.
     // Warps that walk their runs again do so before the pairs are sorted.
+    constexpr uint32_t UNORDERED = 1u << 31;
     __shared__ uint2 s_rec[REC_MAX];
+    __shared__ uint16_t s_nth[REC_MAX];                     // where a pair goes among those of its query and tap
     __shared__ union {
         uint2 sorted[REC_MAX];
         Walk walk;
     } s_u;
     extern __shared__ uint16_t s_cnt[];                     // [tap][query]: pairs, then those of the queries before
-    uint2 *s_mask = reinterpret_cast<uint2 *>(s_cnt + a.k3 * QPB);   // MASKS: [tap][query], a bit for each kept pair of that tap
     __shared__ uint32_t s_base[MAX_K3];                     // next write position of each tap for this block
     __shared__ uint32_t s_start[MAX_K3], s_total[MAX_K3];   // first place of each tap among the sorted, its pairs in this round
     const bool fits = a.ctrl[0] <= a.capacity && !a.ctrl[1];
@@ -432,7 +433,7 @@ __global__ void __launch_bounds__(THREADS, 5) taps_fill_kernel(TapArgs a) {
     const bool kept = __all_sync(0xffffffffu, nq <= (uint32_t)a.kept);   // all accepted points of the warp's queries were kept
     for (uint32_t lo = 0; lo < block_total; lo += REC_MAX) {
         const uint32_t cnt = min((uint32_t)REC_MAX, block_total - lo);
-        for (int t = threadIdx.x; t < a.k3 * QPB / 2 * (MASKS ? 5 : 1); t += THREADS) reinterpret_cast<uint32_t *>(s_cnt)[t] = 0u;   // s_mask too
+        for (int t = threadIdx.x; t < a.k3 * QPB / 2; t += THREADS) reinterpret_cast<uint32_t *>(s_cnt)[t] = 0u;
         __syncthreads();
         // A pair of query x of the block: its place among that query's pairs of the same tap, and into s_rec.  The whole warp
         // calls; pairs of a query come in order, the lanes' queries do not fall.
@@ -443,13 +444,15 @@ __global__ void __launch_bounds__(THREADS, 5) taps_fill_kernel(TapArgs a) {
             const uint32_t before = there ? *count : 0u, lower = same & ((1u << lane) - 1u);
             __syncwarp();
             if (there) {
-                s_rec[pos - lo] = make_uint2((uint32_t)point, (uint32_t)tap | (uint32_t)x << 8 | (before + __popc(lower)) << 16);
+                const uint32_t nth = before + __popc(lower);
+                s_rec[pos - lo] = make_uint2((uint32_t)point, (uint32_t)tap | (uint32_t)x << 8 | nth << 16), s_nth[pos - lo] = (uint16_t)nth;
                 if (!lower) *count = (uint16_t)(before + __popc(same));
             }
             __syncwarp();
         };
-        if (kept && MASKS) {
-            // a bit for each pair: whatever the order in which they come, those before one are the bits below its own
+        if (kept) {
+            // Counted in any order: what is stored is a pair's place in its query's list, and the few pairs of a query and
+            // tap are put in order when they are written.
             const uint32_t most = __reduce_max_sync(0xffffffffu, nq);
             for (uint32_t e0 = c; e0 < most; e0 += 32) {
                 uint32_t tap[4], point[4];
@@ -462,16 +465,11 @@ __global__ void __launch_bounds__(THREADS, 5) taps_fill_kernel(TapArgs a) {
                 for (int u = 0; u < 4; ++u) {
                     const uint32_t e = e0 + 8 * u, pos = q_off + e - lo;
                     if (e >= nq || pos >= (uint32_t)REC_MAX) continue;
-                    uint2 *mask = s_mask + tap[u] * QPB + ql;
-                    atomicOr(e < 32 ? &mask->x : &mask->y, 1u << (e & 31));
-                    s_rec[pos] = make_uint2(point[u], tap[u] | (uint32_t)ql << 8 | e << 16);
+                    const uint32_t shift = (ql & 1) * 16;   // (two queries of one warp share a word)
+                    const uint32_t nth = atomicAdd(reinterpret_cast<uint32_t *>(s_cnt) + (tap[u] * QPB + ql) / 2, 1u << shift) >> shift & 0xffffu;
+                    s_rec[pos] = make_uint2(point[u], tap[u] | (uint32_t)ql << 8 | e << 16 | UNORDERED);
+                    s_nth[pos] = (uint16_t)nth;
                 }
-            }
-        } else if (kept) {
-            const uint32_t most = (__reduce_max_sync(0xffffffffu, nq) + 7) & ~7u;
-            for (uint32_t e = c; e < most; e += 8) {
-                const bool there = e < nq;
-                place(there, q_off + e, ql, there ? a.kept_point[q * a.kept + e] : 0, there ? a.kept_tap[q * a.kept + e] : 0);
             }
         } else {
             const Queries queries(a, q, lane, s_u.walk.query[warp]);
@@ -487,11 +485,7 @@ __global__ void __launch_bounds__(THREADS, 5) taps_fill_kernel(TapArgs a) {
         __syncthreads();
         // a warp per tap: the pairs of the queries before each query
         for (int tap = warp; tap < a.k3; tap += WARPS) {
-            uint32_t v = s_cnt[tap * QPB + lane];
-            if (MASKS) {
-                const uint2 m = s_mask[tap * QPB + lane];
-                v += __popc(m.x) + __popc(m.y);   // a warp's pairs are in one or the other
-            }
+            const uint32_t v = s_cnt[tap * QPB + lane];
             uint32_t incl = v;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -520,18 +514,20 @@ __global__ void __launch_bounds__(THREADS, 5) taps_fill_kernel(TapArgs a) {
         for (uint32_t x = threadIdx.x; x < cnt; x += THREADS) {
             const uint2 rec = s_rec[x];
             const uint32_t tap = rec.y & 0xffu;
-            const uint32_t at = tap * QPB + ((rec.y >> 8) & 0xffu);
-            uint32_t nth = rec.y >> 16;
-            if (MASKS) {
-                const uint2 m = s_mask[at];
-                if (m.x | m.y) nth = __popc(m.x & (nth < 32 ? (1u << nth) - 1u : ~0u)) + __popc(m.y & (nth < 32 ? 0u : (1u << (nth - 32)) - 1u));
-            }
-            s_u.sorted[s_start[tap] + s_cnt[at] + nth] = rec;
+            s_u.sorted[s_start[tap] + s_cnt[tap * QPB + ((rec.y >> 8) & 0xffu)] + s_nth[x]] = rec;
         }
         __syncthreads();
         for (uint32_t x = threadIdx.x; x < cnt; x += THREADS) {
             const uint2 rec = s_u.sorted[x];
-            const uint32_t tap = rec.y & 0xffu, pos = s_base[tap] + x - s_start[tap];
+            const uint32_t tap = rec.y & 0xffu, of = (rec.y >> 8) & 0xffu, first = s_cnt[tap * QPB + of];
+            uint32_t place = x - s_start[tap];
+            if (rec.y & UNORDERED) {
+                place = first;
+                const uint32_t end = of + 1 < QPB ? s_cnt[tap * QPB + of + 1] : s_total[tap];
+                if (end - first > 1)
+                    for (uint32_t y = first; y < end; ++y) place += s_u.sorted[s_start[tap] + y].y < rec.y;   // (they differ in the list place alone)
+            }
+            const uint32_t pos = s_base[tap] + place;
             a.out_i[pos] = (int32_t)(q0 + (int)((rec.y >> 8) & 0xffu));
             a.out_j[pos] = (int32_t)rec.x;
             if (a.out_k) a.out_k[pos] = (int32_t)tap;
@@ -674,8 +670,9 @@ int pcx_radius_taps_fill(const float *d_queries, const int32_t *d_point_sample, 
     a.out_i = d_out_i, a.out_j = d_out_j, a.out_k = d_out_k, a.capacity = capacity;
     if (capacity > 0) {
         prof_begin("taps_fill_kernel", stream);
-        if (a.kept <= 64) (fused(a) ? taps_fill_kernel<true, true> : taps_fill_kernel<false, true>)<<<(unsigned)w.nblocks, THREADS, (size_t)k3 * QPB * 10, stream>>>(a);
-        else (fused(a) ? taps_fill_kernel<true, false> : taps_fill_kernel<false, false>)<<<(unsigned)w.nblocks, THREADS, (size_t)k3 * QPB * 2, stream>>>(a);
+        const auto kernel = k3 <= 27 ? (fused(a) ? taps_fill_kernel<true, 1024> : taps_fill_kernel<false, 1024>)
+                                     : (fused(a) ? taps_fill_kernel<true, 1536> : taps_fill_kernel<false, 1536>);
+        kernel<<<(unsigned)w.nblocks, THREADS, (size_t)k3 * QPB * sizeof(uint16_t), stream>>>(a);
         prof_end(stream);
         PCX_LAUNCH_CHECK();
     }

@@ -208,9 +208,9 @@ def test_tap_ties_on_a_half_grid_lattice():
         assert got[0].numel() > 20 * pts.shape[0]
 
 
-# neighbours about the number that is kept of a query (64, 96), the pairs a block places at a time (1024 for 32 queries) and
-# the fours of candidates a warp lists at a time (64 for four queries); clusters a cell apart keep the runs apart
-@pytest.mark.parametrize("per", [1, 7, 31, 32, 33, 63, 64, 65, 95, 96, 97, 260])
+# neighbours about the number that is kept of a query (64, 128), the pairs a block places at a time (1024 or 1536 for 32
+# queries) and the fours of candidates a warp lists at a time (64 for four queries); clusters a cell apart keep the runs apart
+@pytest.mark.parametrize("per", [1, 7, 31, 32, 33, 63, 64, 65, 127, 128, 129, 260])
 @pytest.mark.parametrize("k", [3, 5])
 def test_lists_of_any_length(per, k):
     from pointelligence_b200 import _cabi
