@@ -120,6 +120,7 @@ int pcx_mvmr(const void *d_weight, const void *d_feat, const int32_t *d_gather,
  * layers/conv.py:430-465. */
 #define PCX_MVMR_TRANSPOSE 1
 #define PCX_MVMR_REVERSE_TAPS 2
+#define PCX_MVMR_SPLIT_SUMS 4 /* pcx_mvmr_planned_bias alone: see there */
 int pcx_mvmr_bias(const void *d_weight, const void *d_feat,
                   const int32_t *d_gather, const int32_t *d_scatter,
                   const int64_t *d_seg_offs, const int32_t *d_tap_idx,
@@ -214,7 +215,11 @@ int pcx_mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan,
  * ceil(width / 256) equal parts of a multiple of 16 channels make them up.  A
  * workspace of pcx_mvmr_planned_scratch_bytes() lets a small rulebook be split
  * over the whole chip (its fp32 sums go through the workspace); with less it
- * runs on as many SMs as it has groups. */
+ * runs on as many SMs as it has groups.  PCX_MVMR_SPLIT_SUMS keeps every bucket
+ * sum as two numbers of the feature type, the rounded sum and what the rounding
+ * left over, and multiplies both (bf16: as exact as fp32 sums of the products
+ * once the row is rounded); the workspace is then the one for twice in_width.
+ * In fp16 sums beyond 65504 are not finite with or without it. */
 size_t pcx_mvmr_planned_scratch_bytes(int64_t multi_buckets, int in_width,
                                       int64_t n_out, int out_width, int K,
                                       int G);

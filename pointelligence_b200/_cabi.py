@@ -387,6 +387,27 @@ def _planned_pays(T, n_out, outw, K):
     return ratio >= _PLANNED_DENSE_RATIO or (ratio >= _PLANNED_MIN_RATIO and n_out * outw * 4 >= _PLANNED_MIN_ACC_BYTES)
 
 
+# Grouped layers and rows wider than 256 channels go to the output-stationary kernel with its bucket sums in two parts
+# (bf16 alone): as exact as the scatter kernels (relative error against fp64 1.65e-3 on both over all shapes below), for a
+# contraction twice as long.  One pass on a built plan, scatter / split, and the plan, us:
+#
+#   triplets per row (rows)     512 -> 512    128 -> 384    32 -> 512    2 x 128 -> 128    plan
+#   33.8 (942)                    81 /  50      35 / 30       38 / 27        30 /  27        74
+#   11.4 (5000)                  123 / 122      54 / 48       62 / 35        42 /  42       128
+#    7.3 (15 000)                217 / 291      82 / 83       96 / 43        57 /  78       135
+#   25.4 (15 000)                672 / 350     232 / 95      277 / 49       150 / 100       139
+#
+# It is chosen where the scatter kernel's fp32 reductions (triplets x width x 4 bytes) are half a gigabyte, so that one
+# pass pays for most of a plan, and the two-part sums stay within 4 GB.  The input gradient of an up-sampling layer 384 ->
+# 128 with 134 triplets a row (18.9 M) took 10.1 ms on the scatter kernel; the training step around it went from 113.0 to
+# 104.7 ms, its plan included.
+_SPLIT_MIN_REDUCED_BYTES, _SPLIT_MAX_SCRATCH_BYTES = 512 << 20, 4 << 30
+
+
+def _split_pays(T, n_out, outw, inw, K):
+    return T * outw * 4 >= _SPLIT_MIN_REDUCED_BYTES and min(T // 2, n_out * K) * inw * 4 <= _SPLIT_MAX_SCRATCH_BYTES
+
+
 _PLAN_WAIT_SECONDS = 30.0   # for a plan that is being built on another stream
 
 
@@ -475,6 +496,17 @@ def planned_supported(weight, feat, gather, scatter, seg_offs, n_out, transpose)
     return T < 2 ** 31 and nblocks * K * 128 <= 2 ** 32
 
 
+def _split_supported(weight, gather, seg_offs, n_out, transpose):
+    """Whether the automatic choice may give this call to the output-stationary kernel with its sums in two parts."""
+    K, G, C, M = weight.shape
+    inw, outw = (M, C) if transpose else (C, M)
+    if seg_offs is None or weight.dtype != torch.bfloat16 or K <= 1 or K > 512 or n_out <= 0 or not (G > 1 or outw > 256):
+        return False
+    if inw != padded_width(inw) or outw != padded_width(outw) or inw > 1024 or G * inw > 2048 or G * ((outw + 255) // 256) > 64:
+        return False
+    return gather.numel() < 2 ** 31 and (int(n_out) + 127) // 128 * K * 128 <= 2 ** 32
+
+
 @on_geometry_stream
 def mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks):
     """Build the plan of a tap-sorted rulebook: ``scatter`` indexes the rows that are summed
@@ -544,21 +576,32 @@ def is_symmetric(i, j, K=None):
             and os.environ.get("PCX_SYMMETRIC_DGRAD", "1") != "0")
 
 
+def _plan_key(scatter, gather, seg_offs, K, n_out, group_blocks):
+    return (scatter.data_ptr(), gather.data_ptr(), seg_offs.data_ptr(), scatter.numel(), int(K), int(n_out),
+            int(group_blocks))
+
+
+def _remembered_plan(scatter, gather, seg_offs, K, n_out, group_blocks):
+    hit = _PLAN_CACHE.get(_plan_key(scatter, gather, seg_offs, K, n_out, group_blocks))
+    if hit is not None:
+        refs, old_stamp, value = hit
+        if old_stamp == _stamp(scatter, gather, seg_offs) and all(r() is t for r, t in zip(refs, (scatter, gather, seg_offs))):
+            return value
+    return None
+
+
 def cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks):
     """``mvmr_plan`` remembered by the identity (and version) of the index tensors, so that every
     layer and every step that shares a rulebook builds its plan once."""
     import weakref
 
-    key = (scatter.data_ptr(), gather.data_ptr(), seg_offs.data_ptr(), scatter.numel(), int(K), int(n_out),
-           int(group_blocks))
+    key = _plan_key(scatter, gather, seg_offs, K, n_out, group_blocks)
     stamp = _stamp(scatter, gather, seg_offs)
     if stamp is None:
         return mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks)
-    hit = _PLAN_CACHE.get(key)
-    if hit is not None:
-        refs, old_stamp, value = hit
-        if old_stamp == stamp and all(r() is t for r, t in zip(refs, (scatter, gather, seg_offs))):
-            return value
+    value = _remembered_plan(scatter, gather, seg_offs, K, n_out, group_blocks)
+    if value is not None:
+        return value
     value = mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks)
     value._stream = torch.cuda.current_stream(scatter.device)
     for k in [k for k, (refs, _, _) in _PLAN_CACHE.items() if any(r() is None for r in refs)]:
@@ -570,14 +613,14 @@ def cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks):
     return value
 
 
-def mvmr_planned(weight, feat, plan, transpose):
+def mvmr_planned(weight, feat, plan, transpose, split=False):
     """``out[scatter[t]] += feat[gather[t]] @ W[tap(t)]`` for the rulebook of ``plan``
-    (``transpose``: use W^T); returns (plan.n_out, out_width) in feat.dtype."""
+    (``transpose``: use W^T; ``split``: bucket sums in two parts); returns (plan.n_out, G * out_width) in feat.dtype."""
     require_cuda(weight, feat)
     K, G, C, M = weight.shape
-    assert G == 1 and K == plan.K and weight.dtype == feat.dtype, (weight.shape, plan.K, weight.dtype, feat.dtype)
+    assert K == plan.K and weight.dtype == feat.dtype, (weight.shape, plan.K, weight.dtype, feat.dtype)
     return host().planned(weight, feat, plan.buffer, plan.group_blocks, plan.multi_buckets, plan.T, plan.n_out,
-                          bool(transpose))
+                          bool(transpose), bool(split))
 
 
 def debug_wait_runs_out(limit_ns=1_000_000):
@@ -595,12 +638,17 @@ def mvmr(weight, feat, gather, scatter, seg_offs, tap_idx, n_out, transpose, eng
     return host().mvmr(weight, feat, gather, scatter, seg_offs, tap_idx, int(n_out), bool(transpose), int(engine))
 
 
-def _plan_hook(scatter, gather, seg_offs, K, n_out, outw, inw, forced):
+def _plan_hook(scatter, gather, seg_offs, K, n_out, outw, inw, forced, split=False):
     """Asked by the host path for every pass the output-stationary kernel could take: the plan to run
     (buffer, blocks per group, multi-triplet buckets) or None for the scatter engine."""
     if not forced and (not _planned_pays(gather.numel(), n_out, outw, K) or scatter.is_inference()
                        or gather.is_inference() or seg_offs.is_inference()):
         return None    # (a plan of inference tensors cannot be remembered, and one per pass does not pay)
+    if split and not _split_pays(gather.numel(), n_out, outw, inw, K):
+        return None
+    if split and torch.cuda.is_current_stream_capturing() and _remembered_plan(
+            scatter, gather, seg_offs, K, n_out, plan_group_blocks(outw)) is None:
+        return None    # building it may wait for the device: the scatter kernels can be captured as they are
     plan = cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, plan_group_blocks(outw))
     return plan.buffer, plan.group_blocks, plan.multi_buckets
 
@@ -623,9 +671,11 @@ def prepare_mvmr(weight, gather, scatter, seg_offs, n_out, transpose=False):
     was prepared, False when the policy keeps the scatter engines (which need no preparation)."""
     K, G, C, M = weight.shape
     n_out = int(n_out)
-    outw = C if transpose else M
-    if not (gather is not None and gather.is_cuda and planned_supported(weight, weight, gather, scatter, seg_offs,
-                                                                        n_out, transpose)):
+    inw, outw = (G * M, G * C) if transpose else (G * C, G * M)
+    if gather is None or not gather.is_cuda:
+        return False
+    if not planned_supported(weight, weight, gather, scatter, seg_offs, n_out, transpose) and not (
+            _split_supported(weight, gather, seg_offs, n_out, transpose) and _split_pays(gather.numel(), n_out, outw, inw, K)):
         return False
     if not _planned_pays(gather.numel(), n_out, outw, K) or _stamp(scatter, gather, seg_offs) is None:
         return False

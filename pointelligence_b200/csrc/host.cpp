@@ -24,7 +24,7 @@ using OptTensor = std::optional<Tensor>;
 namespace {
 
 // ------------------------------------------------------------------ helpers ----
-PyObject *g_plan_hook = nullptr;       // (scatter, gather, seg, K, n_out, out_width, in_width, forced) -> None | plan tuple
+PyObject *g_plan_hook = nullptr;       // (scatter, gather, seg, K, n_out, out_width, in_width, forced, split) -> None | plan tuple
 PyObject *g_symmetric_hook = nullptr;  // (i, j, K) -> bool
 PyObject *g_double_backward = nullptr; // differentiable backward of the convolution (create_graph)
 
@@ -101,10 +101,10 @@ struct Plan {
 };
 
 Plan ask_plan(const Tensor &scatter, const Tensor &gather, const Tensor &seg, int64_t K, int64_t n_out, int64_t outw,
-              int64_t inw, bool forced) {
+              int64_t inw, bool forced, bool split) {
     Plan plan;
     py::gil_scoped_acquire gil;
-    py::object r = py::reinterpret_borrow<py::object>(g_plan_hook)(scatter, gather, seg, K, n_out, outw, inw, forced);
+    py::object r = py::reinterpret_borrow<py::object>(g_plan_hook)(scatter, gather, seg, K, n_out, outw, inw, forced, split);
     if (!r.is_none()) {
         py::tuple t = py::cast<py::tuple>(r);
         plan.buffer = py::cast<Tensor>(t[0]);
@@ -143,6 +143,10 @@ constexpr int64_t NO_PLAN = 0x200;   // internal flag of an engine: the automati
 // Shapes the automatic choice may give to the output-stationary kernel.  It rounds the sums of (row, tap) buckets to 16
 // bits; grouped, padded and wider layers multiply their operands as they are unless the caller asks for that kernel.
 bool plan_unasked(int64_t K, int64_t G, int64_t outw) { return K > 1 && G == 1 && outw <= 256; }
+// ... and those it may be given with the sums in two parts (bf16: as exact as the scatter kernels; in fp16 a sum could
+// leave the type's range, which the scatter kernels' products do not).
+bool plan_split(at::ScalarType dtype, int64_t K, int64_t G, int64_t outw) { return K > 1 && (G > 1 || outw > 256) && dtype == at::kBFloat16; }
+constexpr int SPLIT_SUMS = PCX_MVMR_SPLIT_SUMS;
 
 Tensor mvmr_planned(const Tensor &weight, const Tensor &feat, const Plan &plan, int64_t T, int64_t n_out, int flags,
                     const Tensor &bias) {
@@ -150,7 +154,7 @@ Tensor mvmr_planned(const Tensor &weight, const Tensor &feat, const Plan &plan, 
     const bool transpose = flags & 1;
     const int64_t inw = transpose ? M : C, outw = transpose ? C : M;
     Tensor out = at::empty({n_out, G * outw}, feat.options());
-    const size_t bytes = pcx_mvmr_planned_scratch_bytes(plan.multi, (int)inw, n_out, (int)outw, (int)K, (int)G);
+    const size_t bytes = pcx_mvmr_planned_scratch_bytes(plan.multi, (int)inw * (flags & SPLIT_SUMS ? 2 : 1), n_out, (int)outw, (int)K, (int)G);
     Tensor ws = workspace(bytes, feat);
     check(pcx_mvmr_planned_bias(ptr(weight), ptr(feat), ptr(plan.buffer), plan.buffer.numel(), ptr(bias), ptr(out), T, feat.size(0),
                                 n_out, (int)K, (int)G, (int)C, (int)M, flags, dtype_code(feat.scalar_type()), (int)plan.group, plan.multi,
@@ -196,9 +200,10 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
                   "channels a group");
         }
         const bool aligned = ((uintptr_t)ptr(weight) | (uintptr_t)ptr(feat)) % 16 == 0;   // else the CUDA-core engine
-        if (fits && (engine == ENGINE_PLANNED || (plan_unasked(K, G, outw) && aligned))) {
-            const Plan plan = ask_plan(scatter_, gather_, *seg_, K, n_out, outw, inw, engine == ENGINE_PLANNED);
-            if (plan.valid) return mvmr_planned(weight, feat, plan, T, n_out, flags, bias);
+        const bool forced = engine == ENGINE_PLANNED, split = !forced && plan_split(feat.scalar_type(), K, G, outw);
+        if (fits && (forced || (aligned && (split || plan_unasked(K, G, outw))))) {
+            const Plan plan = ask_plan(scatter_, gather_, *seg_, K, n_out, G * outw, G * inw, forced, split);
+            if (plan.valid) return mvmr_planned(weight, feat, plan, T, n_out, flags | (split ? SPLIT_SUMS : 0), bias);
         }
         engine = 0;
     }
@@ -567,12 +572,12 @@ int64_t peek(const Tensor &words) {
 }
 
 Tensor planned(const Tensor &weight, const Tensor &feat, const Tensor &buffer, int64_t group, int64_t multi, int64_t T, int64_t n_out,
-               bool transpose) {
+               bool transpose, bool split) {
     require_cuda(weight), require_cuda(feat);
     c10::cuda::CUDAGuard guard(feat.device());
     Plan plan;
     plan.buffer = buffer, plan.group = group, plan.multi = multi;
-    return mvmr_planned(weight.contiguous(), feat.contiguous(), plan, T, n_out, transpose ? 1 : 0, Tensor());
+    return mvmr_planned(weight.contiguous(), feat.contiguous(), plan, T, n_out, (transpose ? 1 : 0) | (split ? SPLIT_SUMS : 0), Tensor());
 }
 
 // Geometry on a stream of its own: from here on the calling thread's work on `device` goes to the given stream ...

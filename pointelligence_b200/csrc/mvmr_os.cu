@@ -374,7 +374,7 @@ constexpr int BUCKET_SUM_THREADS = 256, BUCKET_SUM_WARPS = BUCKET_SUM_THREADS / 
 // 200k points, 22 triplets a row: 32 channels 50 -> 44 us, 64 88 -> 70, 96 141 -> 106, 128 160 -> 113, 192 245 -> 197,
 // 256 305 -> 250, 512 647 -> 517.  Slower: 5 and 6 CTAs an SM (spills), the next bucket's rows fetched early at 3 CTAs
 // (368), several pieces a thread (550 - 1090).
-template <int FMT, int LANES>
+template <int FMT, int LANES, bool SPLIT>
 __global__ void __launch_bounds__(BUCKET_SUM_THREADS, BUCKET_SUM_CTAS) bucket_sum_kernel(const uint16_t *__restrict__ feat,
                                                                                          const uint2 *__restrict__ entries,
                                                                                          const uint2 *__restrict__ buckets,
@@ -418,12 +418,21 @@ __global__ void __launch_bounds__(BUCKET_SUM_THREADS, BUCKET_SUM_CTAS) bucket_su
             o.x = pack2(s[0], s[1], FMT), o.y = pack2(s[2], s[3], FMT);
             o.z = pack2(s[4], s[5], FMT), o.w = pack2(s[6], s[7], FMT);
             // past the L2's share of the feature rows: the sums are read once, by the next kernel
-            if (piece_ok && len) __stcs(reinterpret_cast<uint4 *>(dst + (uint64_t)(uint32_t)(b0 + src) * pitch), o);
+            const bool store = piece_ok && len;
+            uint4 *at = reinterpret_cast<uint4 *>(dst + (uint64_t)(uint32_t)(b0 + src) * (SPLIT ? 2 * pitch : pitch));
+            if (store) __stcs(at, o);
+            if (SPLIT) {   // ... and behind it what the rounding left over
+                float hi[8];
+                widen<FMT>(o, hi);
+                o.x = pack2(s[0] - hi[0], s[1] - hi[1], FMT), o.y = pack2(s[2] - hi[2], s[3] - hi[3], FMT);
+                o.z = pack2(s[4] - hi[4], s[5] - hi[5], FMT), o.w = pack2(s[6] - hi[6], s[7] - hi[7], FMT);
+                if (store) __stcs(reinterpret_cast<uint4 *>(reinterpret_cast<char *>(at) + pitch), o);
+            }
         }
     }
 }
 
-template <int FMT>
+template <int FMT, bool SPLIT>
 void launch_bucket_sum(int64_t multi, int inw, const uint16_t *feat, const uint2 *entries, const uint2 *buckets,
                        const uint32_t *ctrl, uint16_t *scratch, cudaStream_t stream) {
     // Up to 128 channels the next power of two of lanes, beyond that slices (blockIdx.y) of 32, 16 or 8 lanes, whichever
@@ -439,7 +448,7 @@ void launch_bucket_sum(int64_t multi, int inw, const uint16_t *feat, const uint2
     }
     const int slices = (ppr + lanes - 1) / lanes, at_once = BUCKET_SUM_THREADS / lanes;
     const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>((multi + at_once - 1) / at_once, num_sms() * BUCKET_SUM_CTAS / slices)), (unsigned)slices);
-#define PCX_BS(L) bucket_sum_kernel<FMT, L><<<grid, BUCKET_SUM_THREADS, 0, stream>>>(feat, entries, buckets, ctrl, inw, scratch)
+#define PCX_BS(L) bucket_sum_kernel<FMT, L, SPLIT><<<grid, BUCKET_SUM_THREADS, 0, stream>>>(feat, entries, buckets, ctrl, inw, scratch)
     switch (lanes) {
         case 2: PCX_BS(2); break;
         case 4: PCX_BS(4); break;
@@ -479,9 +488,10 @@ constexpr int MAX_SLOTS = 8;
 constexpr int BIAS_WIDTH = 1024;
 constexpr int AHEAD = 8;                              // steps the walk runs ahead
 constexpr uint32_t ENTRY_BYTES = 2 * ROWS * 4;        // source rows of a tap's two tiles
-// a step's word: per tap of the step, which of the two tiles have it | contraction steps of 16 << 8 | tiles that have
+// a step's word: per tap of the step, which of the two tiles have it | contraction steps of 16 << 8 | low parts of split
+// sums << 11 | tiles that have
 // any << 13 | first of its unit << 15 | end << 16
-constexpr uint32_t STEP_FIRST = 1u << 15, STEP_END = 1u << 16;
+constexpr uint32_t STEP_LOW = 1u << 11, STEP_FIRST = 1u << 15, STEP_END = 1u << 16;
 // The MMA threads read the words from a ring of their own, each marked with the turn of the ring it belongs to.
 // The walk is at most AHEAD steps ahead of the copies and these at most MAX_SLOTS ahead of the MMAs, so with
 // WORDS entries no word is overwritten before it has been read.
@@ -498,7 +508,7 @@ struct OsParams {
     const uint32_t *tap_masks;
     unsigned int *status;
     int K, C, M, transpose, reverse, fmt;   // reverse: tap k uses weight K-1-k
-    int inw, outw, nkb, ngroups, nblocks, nsplit, mask_words;   // inw, outw: of a part
+    int inw, outw, nkb, ngroups, nblocks, nsplit, mask_words;   // inw, outw: of a part; nkb: slices of the contraction
     int nparts, out_parts, in_pitch, out_pitch;   // parts of an output row: groups of the weight, each in out_parts
     int nslots, nacc, teams;
     const uint16_t *weight;                 // read without the tensor map: transposed weights of a step of several taps
@@ -524,12 +534,13 @@ __device__ __forceinline__ int unit_at(int n, int units) {
 struct Walk {
     const OsParams &p;
     int n = -1, split = 0, part = 0, block0 = 0, q = 0, word = 0, tap = 0;
+    int slices;                     // of the contraction; those of the low parts follow those of the high ones
     int tap_lo = 0, tap_hi = 0;     // taps of this part of the group
     uint32_t m0 = 0, m1 = 0, left = 0;
     uint32_t has = 0;               // of the current step: bit b = block b of the group has the tap
     bool opened = false;            // no step of the unit yet
     bool first = false;             // the current step is the first of its unit
-    __device__ __forceinline__ explicit Walk(const OsParams &params) : p(params) { q = params.nkb; }
+    __device__ __forceinline__ Walk(const OsParams &params, bool split_sums) : p(params), slices(split_sums ? 2 * params.nkb : params.nkb) { q = slices; }
 
     __device__ __forceinline__ static uint32_t below(int w, int tap) {   // bits of mask word w that belong to taps < tap
         const int n = min(max(tap - 32 * w, 0), 32);
@@ -571,9 +582,9 @@ struct Walk {
                 first = opened, opened = false;
                 return true;
             }
-            if (q < p.nkb && ++word < p.mask_words) {
+            if (q < slices && ++word < p.mask_words) {
                 load(word);
-            } else if (++q < p.nkb) {
+            } else if (++q < slices) {
                 word = 0;
                 if (p.mask_words > 1) load(0);
                 else left = m0 | m1;
@@ -586,7 +597,10 @@ struct Walk {
     }
 };
 
-template <int PACK>   // taps of a step
+// PACK: taps of a step.  SPLIT: the scratch holds every bucket's sum as two 16-bit rows, the rounded sum and what the
+// rounding left over, and the contraction goes over both: sums of 16 bits more (bf16: 2^-16 of the sum is lost where
+// one row loses 2^-8), for a second pass over the taps.
+template <int PACK, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ OsParams p) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t s_full[MAX_SLOTS], s_empty[MAX_SLOTS], s_acc_full[2], s_acc_empty[2], s_step_full[AHEAD], s_step_empty[AHEAD];
@@ -635,7 +649,7 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
 
     if (warp < EPI_WARPS) {
         // -------------------------------------------------------------- epilogue ----
-        Walk w(p);
+        Walk w(p, false);
         Ring acc;
         for (int n = 0; w.open(n); ++n) {
             uint32_t any0 = 0, any1 = 0;
@@ -714,7 +728,9 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&s_step_empty[step.slot]));
             const char *col = reinterpret_cast<const char *>(p.feat + column);
-            const char *sums = reinterpret_cast<const char *>(p.scratch + column) - pitch;
+            const bool low = SPLIT && (word & STEP_LOW);
+            const uint32_t sum_pitch = SPLIT ? 2 * pitch : pitch;
+            const char *sums = reinterpret_cast<const char *>(p.scratch + column) + (low ? pitch : 0u) - sum_pitch;
             const bool piece_ok = piece < 2 * (int)((word >> 8) & 7u);
             // the tensor core has finished with what was in the slot
             if (!wait(s_empty[ring.slot], ring.turn ^ 1u)) break;
@@ -731,8 +747,8 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
 #pragma unroll
                     for (int k = 0; k < 8; ++k) {
                         // a feature row x >= 0, the row of bucket sums -2 - x, or nothing (-1: zeros, and a source that is not read)
-                        const char *src = (rr[k] < -1 ? sums : col) + (uint64_t)(uint32_t)(rr[k] ^ (rr[k] >> 31)) * pitch;
-                        cp_async16_or_zero(dst + (uint32_t)t * SLOT_BYTES + dst_off[k], src, rr[k] == -1);
+                        const char *src = (rr[k] < -1 ? sums : col) + (uint64_t)(uint32_t)(rr[k] ^ (rr[k] >> 31)) * (SPLIT && rr[k] < -1 ? sum_pitch : pitch);
+                        cp_async16_or_zero(dst + (uint32_t)t * SLOT_BYTES + dst_off[k], src, rr[k] == -1 || (SPLIT && low && rr[k] >= 0));
                     }
                 }
             }
@@ -747,7 +763,7 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
         // the tables come from DRAM, once.  One thread and a bulk copy a tile: as a warp with votes, a copy a lane
         // and the divisions of the part in every step it took 1300 clocks a step and held up everything behind it.
         if (elect_one()) {
-            Walk w(p);
+            Walk w(p, SPLIT);
             Ring step, word;
             bool more = true;
             int column = 0, wx = 0, wy = 0;   // of the unit: first feature column, corner of its weights in the (taps * groups * C, M) matrix
@@ -763,9 +779,9 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
                         const int g = w.part / p.out_parts, o = (w.part - g * p.out_parts) * p.outw;
                         column = g * p.inw, wx = p.transpose ? 0 : o, wy = g * p.C + (p.transpose ? o : 0);
                     }
-                    const int k0 = w.q * 64;
+                    const int k0 = (SPLIT && w.q >= p.nkb ? w.q - p.nkb : w.q) * 64;
                     uint32_t entry = rows0 + step.slot * entry_bytes, any = 0;
-                    s.x = w.first ? STEP_FIRST : 0u;
+                    s.x = (w.first ? STEP_FIRST : 0u) | (SPLIT && w.q >= p.nkb ? STEP_LOW : 0u);
                     int n = 0;
                     do {
                         const int32_t *src = p.tile_rows + ((int64_t)w.block0 * p.K + w.tap) * ROWS;
@@ -1162,6 +1178,7 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
                           int64_t T, int64_t n_feat, int64_t n_out, int K, int groups, int C, int M, int flags, int dtype,
                           int group_blocks, int64_t multi_buckets, void *d_ws, size_t ws_bytes, void *stream_) {
     const int transpose = flags & PCX_MVMR_TRANSPOSE;
+    const bool split_sums = (flags & PCX_MVMR_SPLIT_SUMS) != 0;
     cudaStream_t stream = (cudaStream_t)stream_;
     const int G = group_blocks;
     if (dtype != PCX_F16 && dtype != PCX_BF16) PCX_FAIL(PCX_E_DTYPE, "pcx_mvmr_planned: fp16 or bf16 only (dtype %d)", dtype);
@@ -1179,9 +1196,9 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     if ((uintptr_t)d_weight % 16 || (uintptr_t)d_feat % 16 || (uintptr_t)d_out % 16 || (uintptr_t)d_plan % 256 || (uintptr_t)d_ws % 256)
         PCX_FAIL(PCX_E_ALIGN, "pcx_mvmr_planned: weight, features and output must be 16-byte aligned, plan and workspace 256-byte aligned");
     if (multi_buckets < 0 || multi_buckets > T / 2) PCX_FAIL(PCX_E_ARG, "pcx_mvmr_planned: multi_buckets out of range");
-    if (multi_buckets > 0 && (!d_ws || ws_bytes < pcx_mvmr_planned_workspace_bytes(multi_buckets, groups * inw)))
-        PCX_FAIL(PCX_E_CAPACITY, "pcx_mvmr_planned: workspace %zu < %zu bytes", ws_bytes,
-                 pcx_mvmr_planned_workspace_bytes(multi_buckets, groups * inw));
+    const size_t sums_bytes = pcx_mvmr_planned_workspace_bytes(multi_buckets, groups * inw * (split_sums ? 2 : 1));
+    if (multi_buckets > 0 && (!d_ws || ws_bytes < sums_bytes))
+        PCX_FAIL(PCX_E_CAPACITY, "pcx_mvmr_planned: workspace %zu < %zu bytes", ws_bytes, sums_bytes);
     PlanView pv;
     const size_t need_plan = carve_plan(d_plan, T, n_out, K, G, &pv);
     if (plan_bytes < need_plan) PCX_FAIL(PCX_E_CAPACITY, "pcx_mvmr_planned: plan buffer %zu < %zu bytes", plan_bytes, need_plan);
@@ -1233,16 +1250,16 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     p.teams = std::min(TEAMS, p.nslots);
     if (p.nslots < 2) PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_planned: shared memory does not fit (C=%d M=%d)", C, M);
     // the fp32 sums of a split rulebook lie behind the bucket sums; a caller that made no room for them gets one part
-    const size_t sums_bytes = pcx_mvmr_planned_workspace_bytes(multi_buckets, p.in_pitch);
     p.nsplit = split_parts(pv.ngroups, K, nparts);
     if (p.nsplit > 1 && (!d_ws || ws_bytes < sums_bytes + partial_bytes(n_out, p.out_pitch, p.nsplit))) p.nsplit = 1;
     p.partial = p.nsplit > 1 ? (float *)((char *)d_ws + sums_bytes) : nullptr;
     const size_t smem = 1024 + (size_t)p.nslots * p.slot_bytes + AHEAD * pack * ENTRY_BYTES;
-    auto kernel = pack == 4 ? mvmr_os_kernel<4> : pack == 2 ? mvmr_os_kernel<2> : mvmr_os_kernel<1>;
-    static int granted[3][64] = {};
+    auto kernel = split_sums ? (pack == 4 ? mvmr_os_kernel<4, true> : pack == 2 ? mvmr_os_kernel<2, true> : mvmr_os_kernel<1, true>)
+                             : (pack == 4 ? mvmr_os_kernel<4, false> : pack == 2 ? mvmr_os_kernel<2, false> : mvmr_os_kernel<1, false>);
+    static int granted[6][64] = {};
     int dev = 0;
     PCX_CUDA(cudaGetDevice(&dev));
-    int &most = granted[pack >> 1][dev & 63];
+    int &most = granted[(pack >> 1) + (split_sums ? 3 : 0)][dev & 63];
     if ((int)smem > most) {
         PCX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         most = (int)smem;
@@ -1250,8 +1267,8 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(pv.ngroups * p.nsplit * nparts, num_sms()));
     if (multi_buckets > 0) {
         prof_begin("bucket_sum_kernel", stream);
-        if (p.fmt) launch_bucket_sum<1>(multi_buckets, p.in_pitch, p.feat, pv.entries, pv.buckets, pv.ctrl, (uint16_t *)d_ws, stream);
-        else launch_bucket_sum<0>(multi_buckets, p.in_pitch, p.feat, pv.entries, pv.buckets, pv.ctrl, (uint16_t *)d_ws, stream);
+        auto sum = split_sums ? (p.fmt ? launch_bucket_sum<1, true> : launch_bucket_sum<0, true>) : (p.fmt ? launch_bucket_sum<1, false> : launch_bucket_sum<0, false>);
+        sum(multi_buckets, p.in_pitch, p.feat, pv.entries, pv.buckets, pv.ctrl, (uint16_t *)d_ws, stream);
         prof_end(stream);
         PCX_LAUNCH_CHECK();
     }

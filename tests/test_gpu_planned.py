@@ -276,3 +276,68 @@ def test_bucket_sums_bit_for_bit(rows, width, dtype):
         want[have] += x[_t(j[np.minimum(first + m, len(j) - 1)].astype(np.int64))].float()[have]
     assert torch.equal(out, want.to(dtype))
     assert _cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("K,G,C,M,transpose", [(27, 1, 64, 64, 0), (27, 1, 16, 48, 0), (27, 1, 32, 96, 1), (27, 1, 80, 16, 0), (8, 1, 512, 320, 0),
+                                               (27, 1, 384, 128, 1), (40, 2, 32, 48, 0), (27, 2, 96, 64, 1), (1, 1, 48, 48, 0)])
+@pytest.mark.parametrize("rows", [130, 6000])   # taps split over the chip, and not
+def test_sums_in_two_parts_are_exact(rows, K, G, C, M, transpose):
+    """bf16 bucket sums as a rounded part and the rest.  Of a sum s the first part leaves up to 2^-8 |s|, of which the second
+    loses 2^-8: 2^-16 of the magnitudes that made an element up, and 2^-19 of them for the fp32 additions (some hundred
+    at 2^-24 each, in random order far less); then one rounding, 2^-8 of the element and of what was lost."""
+    from pointelligence_b200 import _cabi
+
+    rng = np.random.default_rng(rows + C)
+    n_in, T = 400, rows * 20
+    i, k = np.sort(rng.integers(0, rows, T)), rng.integers(0, K, T)
+    k[rng.random(T) < 0.5] = K // 2      # long buckets
+    order = np.lexsort((i, k))
+    i, k, j = i[order].astype(np.int32), k[order], rng.integers(0, n_in, T).astype(np.int32)
+    seg = np.searchsorted(k, np.arange(K + 1)).astype(np.int64)
+    inw, outw = (M, C) if transpose else (C, M)
+    w = _t(rng.standard_normal((K, G, C, M)) / np.sqrt(inw)).bfloat16()
+    x = _t(rng.standard_normal((n_in, G * inw))).bfloat16()
+    plan = _cabi.mvmr_plan(_t(i), _t(j), _t(seg), K, rows, _cabi.plan_group_blocks(outw))
+    assert plan.multi_buckets > 0
+    out = _cabi.mvmr_planned(w, x, plan, transpose, True)
+    want, size = (torch.zeros(rows, G, outw, dtype=torch.float64, device=DEV) for _ in range(2))
+    for t in range(K):
+        ii, jj = (_t(a[seg[t]:seg[t + 1]]).long() for a in (i, j))
+        wt = w[t].double().transpose(1, 2) if transpose else w[t].double()
+        want.index_add_(0, ii, torch.einsum("tgc,gcm->tgm", x[jj].double().view(-1, G, inw), wt))
+        size.index_add_(0, ii, torch.einsum("tgc,gcm->tgm", x[jj].double().abs().view(-1, G, inw), wt.abs()))
+    err = (out.double().view(rows, G, outw) - want).abs()
+    lost = size * (2.0 ** -16 + 2.0 ** -19)
+    assert bool((err <= want.abs() * 2.0 ** -8 + lost * (1 + 2.0 ** -8)).all())
+    assert torch.equal(out, _cabi.mvmr_planned(w, x, plan, transpose, True))
+    assert _cabi.device_status() == 0
+
+
+def test_wide_and_grouped_layers_choose_the_kernel_by_their_reductions():
+    from pointelligence_b200 import _cabi
+
+    i, j, k, seg = _rulebook(3, 20000, 20000, 27, 400000)     # 20 triplets per output row
+    ti, tj, ts = _t(i), _t(j), _t(seg)
+
+    def kernel(G, C, M, dtype=torch.bfloat16):
+        w = torch.randn(27, G, C, M, device=DEV).to(dtype) / 8
+        x = torch.randn(20000, G * C, device=DEV).to(dtype)
+        out, names = _kernels_of(lambda: _cabi.mvmr(w, x, tj, ti, ts, None, 20000, False))
+        return [n for n in names if n != "bucket_sum_kernel"], out, w, x
+
+    names, out, w, x = kernel(1, 64, 352)
+    assert names == ["mvmr_os_kernel(fwd)"]
+    scatter = _cabi.mvmr(w, x, tj, ti, ts, None, 20000, False, _cabi.ENGINE_TENSOR)
+    assert float((out.float() - scatter.float()).norm() / scatter.float().norm()) < 1e-3   # ties of the one rounding
+    assert kernel(2, 64, 176)[0] == ["mvmr_os_kernel(fwd)"]
+    assert kernel(1, 64, 288)[0] == ["mvmr_tc_kernel(fwd)"]                     # 461 MB of reductions
+    assert kernel(1, 64, 352, torch.float16)[0] == ["mvmr_tc_kernel(fwd)"]      # sums may leave the range of fp16
+    # a capture builds no plan
+    w, x = torch.randn(27, 1, 64, 384, device=DEV).bfloat16() / 8, torch.randn(20000, 64, device=DEV).bfloat16()
+    fresh = ti.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = _cabi.mvmr(w, x, tj, fresh, ts, None, 20000, False)
+    graph.replay()
+    ref = _cabi.mvmr(w, x, tj, ti, ts, None, 20000, False)
+    assert float((y.float() - ref.float()).norm() / ref.float().norm()) < 1e-3
