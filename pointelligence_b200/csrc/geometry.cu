@@ -425,6 +425,7 @@ __device__ __forceinline__ int floor_div_cell(float a, float b) {
 
 __global__ void grid_extent_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample,
                                    int64_t N, float cell, int32_t *ext) {
+    start_after_previous();
     Extent4 e;
     e.reset();
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < N; t += (int64_t)gridDim.x * blockDim.x) {
@@ -438,6 +439,7 @@ __global__ void grid_extent_kernel(const float *__restrict__ pts, const int32_t 
 __global__ void grid_key_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample,
                                 int64_t N, float cell, const int32_t *__restrict__ ext,
                                 int64_t *keys, int32_t *vals) {
+    start_after_previous();
     int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (n >= N) return;
     int64_t ex = (int64_t)ext[4] - ext[0] + 1, ey = (int64_t)ext[5] - ext[1] + 1,
@@ -450,6 +452,7 @@ __global__ void grid_key_kernel(const float *__restrict__ pts, const int32_t *__
 }
 
 __global__ void grid_flag_kernel(const int64_t *__restrict__ keys, int64_t N, int32_t *flags) {
+    start_after_previous();
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= N) return;
     flags[p] = (p == 0 || keys[p] != keys[p - 1]) ? 1 : 0;
@@ -460,6 +463,7 @@ __global__ void grid_select_kernel(const float *__restrict__ pts, const int32_t 
                                    const int32_t *__restrict__ flags, const int32_t *__restrict__ ordinal,
                                    int64_t N, float cell, int64_t *indices, float *out_pts,
                                    int32_t *out_sample, int64_t *mapping) {
+    start_after_previous();
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= N) return;
     int32_t seg = ordinal[p] - 1;
@@ -491,6 +495,7 @@ __global__ void grid_select_kernel(const float *__restrict__ pts, const int32_t 
 
 // sizes[s] = elements of a non-decreasing id list that equal s
 __global__ void sample_sizes_kernel(const int32_t *__restrict__ sorted, int64_t N, int64_t S, int64_t *sizes) {
+    start_after_previous();
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (s >= S) return;
     int64_t bound[2];
@@ -770,10 +775,10 @@ int pcx_grid_sample_count_samples(const float *d_points, const int32_t *d_sample
     PCX_CUDA(cudaMemsetAsync(w.ext, 0x7f, 4 * sizeof(int32_t), stream));
     PCX_CUDA(cudaMemsetAsync(w.ext + 4, 0x80, 4 * sizeof(int32_t), stream));
     int blocks = (int)std::min<int64_t>((N + 255) / 256, 8 * num_sms());
-    grid_extent_kernel<<<blocks, 256, 0, stream>>>(d_points, d_sample, N, c32, w.ext);
+    launch_after(grid_extent_kernel, blocks, 256, 0, stream, d_points, d_sample, N, c32, w.ext);
     PCX_LAUNCH_CHECK();
     unsigned nb = (unsigned)((N + 255) / 256);
-    grid_key_kernel<<<nb, 256, 0, stream>>>(d_points, d_sample, N, c32, w.ext, w.keys_a, w.vals_a);
+    launch_after(grid_key_kernel, nb, 256, 0, stream, d_points, d_sample, N, c32, w.ext, w.keys_a, w.vals_a);
     PCX_LAUNCH_CHECK();
     // The sort only has to look at the bits the largest key can use.  How many those are is known from the extents,
     // which come to the host with the cell count; the sort is enqueued for the bits that the last clouds of this
@@ -796,7 +801,7 @@ int pcx_grid_sample_count_samples(const float *d_points, const int32_t *d_sample
     for (;;) {
         size_t tmp = w.cub_bytes;
         PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, tmp, w.keys_a, w.keys_b, w.vals_a, w.vals_b, N, 0, used, stream));
-        grid_flag_kernel<<<nb, 256, 0, stream>>>(w.keys_b, N, w.flags);
+        launch_after(grid_flag_kernel, nb, 256, 0, stream, w.keys_b, N, w.flags);
         PCX_LAUNCH_CHECK();
         tmp = w.cub_bytes;
         PCX_CUDA(cub::DeviceScan::InclusiveSum(w.cub_tmp, tmp, w.flags, w.ordinal, N, stream));
@@ -813,7 +818,7 @@ int pcx_grid_sample_count_samples(const float *d_points, const int32_t *d_sample
 
 int pcx_sample_sizes(const int32_t *d_sorted, int64_t N, int64_t S, int64_t *d_sizes, void *stream_) {
     if (N < 0 || S <= 0 || (N > 0 && !d_sorted) || !d_sizes) PCX_FAIL(PCX_E_ARG, "pcx_sample_sizes: bad arguments");
-    sample_sizes_kernel<<<(unsigned)((S + 127) / 128), 128, 0, (cudaStream_t)stream_>>>(d_sorted, N, S, d_sizes);
+    launch_after(sample_sizes_kernel, (unsigned)((S + 127) / 128), 128, 0, (cudaStream_t)stream_, d_sorted, N, S, d_sizes);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
 }
@@ -827,7 +832,7 @@ int pcx_grid_sample_select(const float *d_points, const int32_t *d_sample, int64
     GridWs w;
     size_t need = carve_grid(d_ws, N, &w);
     if (ws_bytes < need) PCX_FAIL(PCX_E_CAPACITY, "pcx_grid_sample_select: workspace %zu < %zu bytes", ws_bytes, need);
-    grid_select_kernel<<<(unsigned)((N + 255) / 256), 256, 0, stream>>>(
+    launch_after(grid_select_kernel, (unsigned)((N + 255) / 256), 256, 0, stream, 
         d_points, d_sample, w.keys_b, w.vals_b, w.flags, w.ordinal, N, (float)cell, d_indices,
         d_out_points, d_out_sample, d_mapping);
     PCX_LAUNCH_CHECK();

@@ -174,6 +174,7 @@ __device__ __forceinline__ void copy_seg(const int64_t *__restrict__ seg, int K,
 
 __global__ void plan_init_kernel(int64_t n_out, uint32_t *sig, int32_t *row, int32_t *tile_cnt, int64_t n_tiles,
                                  uint32_t *ctrl, int G) {
+    start_after_previous();
     const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (x < n_out) sig[x] = 0u, row[x] = (int32_t)x;
     if (x <= n_tiles) tile_cnt[x] = 0;
@@ -185,6 +186,7 @@ __global__ void plan_init_kernel(int64_t n_out, uint32_t *sig, int32_t *row, int
 // whose rows do not ascend inside a tap.
 __global__ void plan_sig_kernel(const int32_t *__restrict__ scatter, const int64_t *__restrict__ seg, int64_t T, int K,
                                 uint32_t *sig, uint32_t *ctrl) {
+    start_after_previous();
     __shared__ int64_t s_seg[MAX_TAPS + 1];
     copy_seg(seg, K, s_seg);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -205,6 +207,7 @@ __global__ void plan_sig_kernel(const int32_t *__restrict__ scatter, const int64
 // even where their exact tap sets differ, and sorted by (planes, signature) the blocks of 128 rows need
 // a quarter fewer (block, tap) tiles on thin rulebooks than sorted by signature alone.
 __global__ void plan_order_kernel(const uint32_t *__restrict__ sig, int64_t n_out, int K, int ks, uint64_t *order) {
+    start_after_previous();
     const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= n_out) return;
     const uint32_t m = sig[x];
@@ -217,6 +220,7 @@ __global__ void plan_order_kernel(const uint32_t *__restrict__ sig, int64_t n_ou
 
 __global__ void plan_rank_kernel(const int32_t *__restrict__ row_sorted, int64_t n_out, int64_t n_pad, int32_t *rank,
                                  int32_t *perm) {
+    start_after_previous();
     const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= n_pad) return;
     if (x < n_out) {
@@ -234,6 +238,7 @@ __global__ void plan_rank_kernel(const int32_t *__restrict__ row_sorted, int64_t
 // tile_rows[tile * 128 + slot] = first triplet of the bucket; triplets per tile
 __global__ void plan_heads_kernel(const int32_t *__restrict__ scatter, const int64_t *__restrict__ seg, const int32_t *__restrict__ rank,
                                   int64_t T, int K, int32_t *tile_rows, int32_t *tile_cnt) {
+    start_after_previous();
     __shared__ int64_t s_seg[MAX_TAPS + 1];
     copy_seg(seg, K, s_seg);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -252,6 +257,7 @@ __global__ void plan_heads_kernel(const int32_t *__restrict__ scatter, const int
 __global__ void plan_tiles_kernel(const int32_t *__restrict__ scatter, const int32_t *__restrict__ gather, const int64_t *__restrict__ seg,
                                   int K, int64_t n_tiles, const int32_t *__restrict__ tile_offs, uint2 *entries, int32_t *tile_rows,
                                   uint2 *buckets, uint32_t *ctrl) {
+    start_after_previous();
     const int64_t tile = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
     if (tile >= n_tiles) return;
@@ -305,6 +311,7 @@ __global__ void plan_tiles_kernel(const int32_t *__restrict__ scatter, const int
 __global__ void plan_keys_kernel(const int32_t *__restrict__ scatter, const int32_t *__restrict__ gather,
                                  const int64_t *__restrict__ seg, const int32_t *__restrict__ rank, int64_t T, int K,
                                  uint32_t *key, int32_t *val, int32_t *tile_cnt) {
+    start_after_previous();
     __shared__ int64_t s_seg[MAX_TAPS + 1];
     copy_seg(seg, K, s_seg);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -322,6 +329,7 @@ __global__ void plan_keys_kernel(const int32_t *__restrict__ scatter, const int3
 // when more triplets follow, the scratch row the bucket's sum will be written to
 __global__ void plan_entries_kernel(const uint32_t *__restrict__ key_sorted, const int32_t *__restrict__ val_sorted,
                                     int64_t T, uint2 *entries, int32_t *tile_rows, uint2 *buckets, uint32_t *ctrl) {
+    start_after_previous();
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T) return;
     const uint32_t k = key_sorted[t];
@@ -380,6 +388,7 @@ __global__ void __launch_bounds__(BUCKET_SUM_THREADS, BUCKET_SUM_CTAS) bucket_su
                                                                                          const uint2 *__restrict__ buckets,
                                                                                          const uint32_t *__restrict__ ctrl, int inw,
                                                                                          uint16_t *__restrict__ scratch) {
+    start_after_previous();
     constexpr int AT_ONCE = 32 / LANES;
     const int lane = threadIdx.x & 31, sub = lane / LANES, nmulti = (int)ctrl[CTRL_NMULTI];
     const unsigned piece = blockIdx.y * LANES + lane % LANES, pitch = (unsigned)inw * 2u;
@@ -448,7 +457,7 @@ void launch_bucket_sum(int64_t multi, int inw, const uint16_t *feat, const uint2
     }
     const int slices = (ppr + lanes - 1) / lanes, at_once = BUCKET_SUM_THREADS / lanes;
     const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>((multi + at_once - 1) / at_once, num_sms() * BUCKET_SUM_CTAS / slices)), (unsigned)slices);
-#define PCX_BS(L) bucket_sum_kernel<FMT, L, SPLIT><<<grid, BUCKET_SUM_THREADS, 0, stream>>>(feat, entries, buckets, ctrl, inw, scratch)
+#define PCX_BS(L) launch_after(bucket_sum_kernel<FMT, L, SPLIT>, grid, BUCKET_SUM_THREADS, 0, stream, feat, entries, buckets, ctrl, inw, scratch)
     switch (lanes) {
         case 2: PCX_BS(2); break;
         case 4: PCX_BS(4); break;
@@ -462,6 +471,7 @@ void launch_bucket_sum(int64_t multi, int inw, const uint16_t *feat, const uint2
 // cost of a group = its non-empty tiles (each is one A tile to copy and multiply); the tap sets of its blocks
 __global__ void plan_cost_kernel(const int32_t *__restrict__ tile_offs, int64_t nblocks, int K, int G, int64_t ngroups,
                                  uint32_t *cost, int32_t *gid, uint32_t *tap_masks) {
+    start_after_previous();
     const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= ngroups) return;
     const int words = (K + 31) / 32;
@@ -602,6 +612,7 @@ struct Walk {
 // one row loses 2^-8), for a second pass over the taps.
 template <int PACK, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ OsParams p) {
+    start_after_previous();
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t s_full[MAX_SLOTS], s_empty[MAX_SLOTS], s_acc_full[2], s_acc_empty[2], s_step_full[AHEAD], s_step_empty[AHEAD];
     __shared__ uint32_t s_word[WORDS];
@@ -928,6 +939,7 @@ constexpr int REDUCE_BATCH = 9;
 __global__ void __launch_bounds__(128) os_reduce_kernel(const float *__restrict__ partial, const int32_t *__restrict__ perm,
                                                         const uint16_t *__restrict__ bias, int64_t slots, int outw, int nsplit, int fmt,
                                                         uint16_t *out) {
+    start_after_previous();
     // a block of threads: the rows of a block of the plan, four columns
     const int64_t block = blockIdx.x;
     const int c = (int)blockIdx.y * 4, lane = threadIdx.x;
@@ -1029,7 +1041,7 @@ bool plan_sizes_ok(int64_t T, int64_t n_out, int K, int G) {
 
 // groups, most tiles first, and the tap sets of their blocks
 int order_groups(const PlanView &pv, const BuildWs &w, int K, int G, cudaStream_t stream) {
-    plan_cost_kernel<<<(unsigned)((pv.ngroups + 255) / 256), 256, 0, stream>>>(pv.tile_offs, pv.nblocks, K, G, pv.ngroups, w.cost, w.gid,
+    launch_after(plan_cost_kernel, (unsigned)((pv.ngroups + 255) / 256), 256, 0, stream, pv.tile_offs, pv.nblocks, K, G, pv.ngroups, w.cost, w.gid,
                                                                                pv.tap_masks);
     PCX_LAUNCH_CHECK();
     size_t bytes = w.cub_bytes;
@@ -1092,31 +1104,31 @@ int pcx_mvmr_plan_build_counted(const int32_t *d_scatter, const int32_t *d_gathe
     auto blocks = [&](int64_t n) { return (unsigned)((n + TPB - 1) / TPB); };
     const int64_t init_n = std::max<int64_t>(std::max<int64_t>(n_out, n_tiles + 1), CTRL_WORDS);
     PCX_CUDA(cudaMemsetAsync(pv.tile_rows, 0xff, (size_t)n_tiles * ROWS * sizeof(int32_t), stream));
-    plan_init_kernel<<<blocks(init_n), TPB, 0, stream>>>(n_out, w.sig, w.row, w.tile_cnt, n_tiles, pv.ctrl, G);
+    launch_after(plan_init_kernel, blocks(init_n), TPB, 0, stream, n_out, w.sig, w.row, w.tile_cnt, n_tiles, pv.ctrl, G);
     PCX_LAUNCH_CHECK();
     size_t bytes = w.cub_bytes;
     if (T > 0) {
-        plan_sig_kernel<<<blocks(T), TPB, 0, stream>>>(d_scatter, d_seg_offs, T, K, w.sig, pv.ctrl);
+        launch_after(plan_sig_kernel, blocks(T), TPB, 0, stream, d_scatter, d_seg_offs, T, K, w.sig, pv.ctrl);
         PCX_LAUNCH_CHECK();
     }
     // rows by (planes, signature), stable: rows of equal keys keep their order
     int ks = 1;
     while (ks * ks * ks < K) ++ks;
     if (ks * ks * ks != K || K > 32 || K == 1) ks = 0;
-    plan_order_kernel<<<blocks(n_out), TPB, 0, stream>>>(w.sig, n_out, K, ks, w.order);
+    launch_after(plan_order_kernel, blocks(n_out), TPB, 0, stream, w.sig, n_out, K, ks, w.order);
     PCX_LAUNCH_CHECK();
     PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, bytes, w.order, w.order_sorted, w.row, w.row_sorted, (int)n_out, 0,
                                              std::min(K, 32) + 3 * ks, stream));
-    plan_rank_kernel<<<blocks(n_pad), TPB, 0, stream>>>(w.row_sorted, n_out, n_pad, w.rank, pv.perm);
+    launch_after(plan_rank_kernel, blocks(n_pad), TPB, 0, stream, w.row_sorted, n_out, n_pad, w.rank, pv.perm);
     PCX_LAUNCH_CHECK();
     if (T > 0) {
-        plan_heads_kernel<<<blocks(T), TPB, 0, stream>>>(d_scatter, d_seg_offs, w.rank, T, K, pv.tile_rows, w.tile_cnt);
+        launch_after(plan_heads_kernel, blocks(T), TPB, 0, stream, d_scatter, d_seg_offs, w.rank, T, K, pv.tile_rows, w.tile_cnt);
         PCX_LAUNCH_CHECK();
     }
     bytes = w.cub_bytes;
     PCX_CUDA(cub::DeviceScan::ExclusiveSum(w.cub_tmp, bytes, w.tile_cnt, pv.tile_offs, (int)(n_tiles + 1), stream));
     if (T > 0) {
-        plan_tiles_kernel<<<blocks(n_tiles * 32), TPB, 0, stream>>>(d_scatter, d_gather, d_seg_offs, K, n_tiles, pv.tile_offs, pv.entries,
+        launch_after(plan_tiles_kernel, blocks(n_tiles * 32), TPB, 0, stream, d_scatter, d_gather, d_seg_offs, K, n_tiles, pv.tile_offs, pv.entries,
                                                                    pv.tile_rows, pv.buckets, pv.ctrl);
         PCX_LAUNCH_CHECK();
     }
@@ -1132,14 +1144,14 @@ int pcx_mvmr_plan_build_counted(const int32_t *d_scatter, const int32_t *d_gathe
     PCX_CUDA(cudaMemsetAsync(pv.tile_rows, 0xff, (size_t)n_tiles * ROWS * sizeof(int32_t), stream));
     PCX_CUDA(cudaMemsetAsync(w.tile_cnt, 0, (size_t)(n_tiles + 1) * sizeof(int32_t), stream));
     PCX_CUDA(cudaMemsetAsync(pv.ctrl + CTRL_NMULTI, 0, sizeof(uint32_t), stream));
-    plan_keys_kernel<<<blocks(T), TPB, 0, stream>>>(d_scatter, d_gather, d_seg_offs, w.rank, T, K, w.key, w.val, w.tile_cnt);
+    launch_after(plan_keys_kernel, blocks(T), TPB, 0, stream, d_scatter, d_gather, d_seg_offs, w.rank, T, K, w.key, w.val, w.tile_cnt);
     PCX_LAUNCH_CHECK();
     bytes = w.cub_bytes;
     PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, bytes, w.key, w.key_sorted, w.val, w.val_sorted, (int)T, 0,
                                              std::min(32, bits_of(n_tiles * ROWS)), stream));
     bytes = w.cub_bytes;
     PCX_CUDA(cub::DeviceScan::ExclusiveSum(w.cub_tmp, bytes, w.tile_cnt, pv.tile_offs, (int)(n_tiles + 1), stream));
-    plan_entries_kernel<<<blocks(T), TPB, 0, stream>>>(w.key_sorted, w.val_sorted, T, pv.entries, pv.tile_rows, pv.buckets, pv.ctrl);
+    launch_after(plan_entries_kernel, blocks(T), TPB, 0, stream, w.key_sorted, w.val_sorted, T, pv.entries, pv.tile_rows, pv.buckets, pv.ctrl);
     PCX_LAUNCH_CHECK();
     if (int rc = order_groups(pv, w, K, G, stream)) return rc;
     return pcx_mvmr_plan_multi_buckets(d_plan, h_multi, stream);
@@ -1273,12 +1285,12 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
         PCX_LAUNCH_CHECK();
     }
     prof_begin(transpose ? "mvmr_os_kernel(dgrad)" : "mvmr_os_kernel(fwd)", stream);
-    kernel<<<grid, THREADS, smem, stream>>>(tmap, p);
+    launch_after(kernel, grid, THREADS, smem, stream, tmap, p);
     prof_end(stream);
     PCX_LAUNCH_CHECK();
     if (p.nsplit > 1) {
         const int64_t slots = pv.nblocks * ROWS;
-        os_reduce_kernel<<<dim3((unsigned)pv.nblocks, (unsigned)(p.out_pitch / 4)), ROWS, 0, stream>>>(p.partial, p.perm, p.bias, slots, p.out_pitch,
+        launch_after(os_reduce_kernel, dim3((unsigned)pv.nblocks, (unsigned)(p.out_pitch / 4)), ROWS, 0, stream, p.partial, p.perm, p.bias, slots, p.out_pitch,
                                                                                                      p.nsplit, p.fmt, p.out);
         PCX_LAUNCH_CHECK();
     }

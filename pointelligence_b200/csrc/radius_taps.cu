@@ -118,6 +118,7 @@ __device__ __forceinline__ uint32_t cell_bucket(int b, int cx, int cy, int cz, u
 
 __global__ void taps_key_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, int64_t P,
                                 float inv, uint32_t mask, uint32_t *keys, int32_t *vals) {
+    start_after_previous();
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= P) return;
     keys[p] = cell_bucket(sample ? sample[p] : 0, cell_of(pts[3 * p], inv), cell_of(pts[3 * p + 1], inv),
@@ -129,6 +130,7 @@ __global__ void taps_key_kernel(const float *__restrict__ pts, const int32_t *__
 __global__ void taps_table_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, const uint32_t *__restrict__ keys,
                                   const int32_t *__restrict__ perm, int64_t P, float4 *sorted_pts, int32_t *sorted_sample,
                                   int2 *table) {
+    start_after_previous();
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (s >= P) return;
     const int32_t p = perm[s];
@@ -305,6 +307,7 @@ struct Accepted {
 // four LiDAR sweeps 68 -> 53.  Eight lanes a query with a list of their own, and pieces of eight candidates: 207, 48, 74.
 template <bool FUSED>
 __global__ void __launch_bounds__(THREADS) taps_count_kernel(TapArgs a) {
+    start_after_previous();
     __shared__ uint32_t s_hist[MAX_K3];
     __shared__ __align__(16) Four s_list[THREADS / 32][FOURS];
     __shared__ float4 s_query[THREADS / 32][4];
@@ -342,6 +345,7 @@ __global__ void __launch_bounds__(THREADS) taps_count_kernel(TapArgs a) {
 __global__ void __launch_bounds__(SCAN_THREADS) taps_colscan_kernel(uint32_t *block_hist, int64_t nblocks, int k3,
                                                                      unsigned long long *tap_total, int64_t *seg,
                                                                      int64_t *seg_out, int64_t *ctrl) {
+    start_after_previous();
     using Scan = cub::BlockScan<uint32_t, SCAN_THREADS>;
     __shared__ typename Scan::TempStorage tmp;
     __shared__ int s_last;
@@ -395,6 +399,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) taps_colscan_kernel(uint32_t *bl
 // and its warp keeps the block waiting), 125 taps, 100 000 queries with 41 152 -> 110
 template <bool FUSED, int REC_MAX>   // pairs staged per round
 __global__ void __launch_bounds__(THREADS, REC_MAX > 1024 ? 4 : 5) taps_fill_kernel(TapArgs a) {
+    start_after_previous();
     constexpr int WARPS = THREADS / 32;
     struct Walk {
         Four list[WARPS][FOURS];
@@ -623,19 +628,19 @@ int pcx_radius_taps_count(const float *d_points, const float *d_queries, const i
     const unsigned pblocks = (unsigned)((P + 255) / 256);
     PCX_CUDA(cudaMemsetAsync(w.ctrl, 0, 8 * sizeof(int64_t), stream));
     PCX_CUDA(cudaMemsetAsync(w.table, 0, (size_t)w.buckets * sizeof(int2), stream));
-    taps_key_kernel<<<pblocks, 256, 0, stream>>>(d_points, d_point_sample, P, inv, mask, w.keys_a, w.vals_a);
+    launch_after(taps_key_kernel, pblocks, 256, 0, stream, d_points, d_point_sample, P, inv, mask, w.keys_a, w.vals_a);
     PCX_LAUNCH_CHECK();
     size_t tmp = w.cub_bytes;
     PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, tmp, w.keys_a, w.keys_b, w.vals_a, w.vals_b, P, 0, w.bits, stream));
-    taps_table_kernel<<<pblocks, 256, 0, stream>>>(d_points, d_point_sample, w.keys_b, w.vals_b, P, w.sorted_pts, w.sorted_sample, w.table);
+    launch_after(taps_table_kernel, pblocks, 256, 0, stream, d_points, d_point_sample, w.keys_b, w.vals_b, P, w.sorted_pts, w.sorted_sample, w.table);
     PCX_LAUNCH_CHECK();
     TapArgs a = make_args(w, d_queries, d_point_sample, d_query_sample, Q, radius, distance_type, kernel_size, kernel_grid_size);
     a.num_neighbors = d_num_neighbors;
     prof_begin("taps_count_kernel", stream);
-    (fused(a) ? taps_count_kernel<true> : taps_count_kernel<false>)<<<(unsigned)w.nblocks, THREADS, 0, stream>>>(a);
+    launch_after((fused(a) ? taps_count_kernel<true> : taps_count_kernel<false>), (unsigned)w.nblocks, THREADS, 0, stream, a);
     prof_end(stream);
     PCX_LAUNCH_CHECK();
-    taps_colscan_kernel<<<k3, SCAN_THREADS, 0, stream>>>(w.block_hist, w.nblocks, k3, w.tap_total, w.seg, d_seg_offs, w.ctrl);
+    launch_after(taps_colscan_kernel, k3, SCAN_THREADS, 0, stream, w.block_hist, w.nblocks, k3, w.tap_total, w.seg, d_seg_offs, w.ctrl);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
 }
@@ -672,7 +677,7 @@ int pcx_radius_taps_fill(const float *d_queries, const int32_t *d_point_sample, 
         prof_begin("taps_fill_kernel", stream);
         const auto kernel = k3 <= 27 ? (fused(a) ? taps_fill_kernel<true, 1024> : taps_fill_kernel<false, 1024>)
                                      : (fused(a) ? taps_fill_kernel<true, 1536> : taps_fill_kernel<false, 1536>);
-        kernel<<<(unsigned)w.nblocks, THREADS, (size_t)k3 * QPB * sizeof(uint16_t), stream>>>(a);
+        launch_after(kernel, (unsigned)w.nblocks, THREADS, (size_t)k3 * QPB * sizeof(uint16_t), stream, a);
         prof_end(stream);
         PCX_LAUNCH_CHECK();
     }

@@ -48,6 +48,7 @@ __global__ void ln_tail_kernel(int64_t *offsets, int64_t S, int64_t total) {
 // arrays), in one small launch.
 __global__ void ln_small_offsets_kernel(const int64_t *__restrict__ lengths, int64_t *offsets, int64_t S, int64_t total, float *z0,
                                         int64_t n0, float *z1, float *z2, int64_t n12) {
+    start_after_previous();
     for (int64_t t = threadIdx.x; t < n0; t += blockDim.x) z0[t] = 0.f;
     for (int64_t t = threadIdx.x; t < n12; t += blockDim.x) z1[t] = 0.f, z2[t] = 0.f;
     if (threadIdx.x >= 32) return;
@@ -110,6 +111,7 @@ constexpr int MOM_R = 4;
 template <typename T, int VN>
 __global__ void __launch_bounds__(LN_THREADS, 4) ln_moments_kernel(const T *__restrict__ x, const int64_t *__restrict__ offsets, Moments *rec,
                                                                    int64_t N, int64_t S, int C, int rows) {
+    start_after_previous();
     __shared__ Moments scratch[LN_THREADS / 32];
     const BlockRows B(offsets, N, S, rows);
     const RowLayout L(C, VN);
@@ -181,6 +183,7 @@ __device__ __forceinline__ double block_sum_f64(double v, double *scratch) {
 __global__ void __launch_bounds__(COMBINE_THREADS) ln_combine_kernel(const Moments *__restrict__ rec,
                                                                      const int64_t *__restrict__ offsets, float *mean,
                                                                      float *rstd, int64_t S, float eps, int mom_rows) {
+    start_after_previous();
     __shared__ double scratch[COMBINE_THREADS / 32];
     const int64_t s = blockIdx.x;
     const int64_t lo = offsets[s], hi = offsets[s + 1];
@@ -212,6 +215,7 @@ __global__ void __launch_bounds__(LN_THREADS, 5) ln_apply_kernel(const T *__rest
                                 const float *__restrict__ mean, const float *__restrict__ rstd,
                                 const float *__restrict__ weight, const float *__restrict__ bias,
                                 const T *__restrict__ residual, T *y, int64_t N, int64_t S, int C, int relu, int rows) {
+    start_after_previous();
     const BlockRows B(offsets, N, S, rows);
     const RowLayout L(C, VN);
     for (int cp = 0; cp * L.vcb < L.vc_total; ++cp) {
@@ -262,6 +266,7 @@ __global__ void __launch_bounds__(LN_THREADS, 4) ln_bwd_sums_kernel(const T *__r
                                    const float *__restrict__ rstd, const float *__restrict__ weight, float *s1,
                                    float *s2, float *dweight, float *dbias, T *dresidual, int64_t N, int64_t S,
                                    int C, int relu, int rows) {
+    start_after_previous();
     __shared__ float scratch[LN_THREADS / 32];
     __shared__ float col_w[LN_THREADS * VN], col_b[LN_THREADS * VN];
     const BlockRows B(offsets, N, S, rows);
@@ -353,6 +358,7 @@ __global__ void __launch_bounds__(LN_THREADS, 4) ln_bwd_apply_kernel(const T *__
                                     const float *__restrict__ rstd, const float *__restrict__ weight,
                                     const float *__restrict__ s1, const float *__restrict__ s2, T *dx, int64_t N,
                                     int64_t S, int C, int relu, int rows) {
+    start_after_previous();
     const BlockRows B(offsets, N, S, rows);
     const RowLayout L(C, VN);
     for (int cp = 0; cp * L.vcb < L.vc_total; ++cp) {
@@ -673,7 +679,7 @@ int layer_rows(int64_t N, int C, int dtype, bool vec, int ctas) {
 int ln_offsets(const int64_t *d_lengths, int64_t S, int64_t N, const LnWs &w, cudaStream_t stream, bool zero_sums = false, float *z1 = nullptr,
                float *z2 = nullptr, int64_t n12 = 0) {
     if (S <= 4096) {
-        ln_small_offsets_kernel<<<1, 256, 0, stream>>>(d_lengths, w.offsets, S, N, w.sums, zero_sums ? 2 * S : 0, z1, z2, z1 ? n12 : 0);
+        launch_after(ln_small_offsets_kernel, 1, 256, 0, stream, d_lengths, w.offsets, S, N, w.sums, zero_sums ? 2 * S : 0, z1, z2, z1 ? n12 : 0);
         PCX_LAUNCH_CHECK();
         return PCX_OK;
     }
@@ -733,13 +739,13 @@ int pcx_ragged_layer_norm(const void *d_x, const int64_t *d_lengths, const float
     const int mom_rows = layer_rows(N, C, dtype, vec, 4), rows = layer_rows(N, C, dtype, vec, 5);
     if (N > 0) {
         const unsigned mgrid = (unsigned)((N + mom_rows - 1) / mom_rows);
-        PCX_LN_DISPATCH(dtype, vec, (ln_moments_kernel<T, VN><<<mgrid, LN_THREADS, 0, stream>>>((const T *)d_x, w.offsets, w.rec, N, S, C, mom_rows)));
+        PCX_LN_DISPATCH(dtype, vec, (launch_after(ln_moments_kernel<T, VN>, mgrid, LN_THREADS, 0, stream, (const T *)d_x, w.offsets, w.rec, N, S, C, mom_rows)));
         PCX_LAUNCH_CHECK();
     }
-    ln_combine_kernel<<<(unsigned)S, COMBINE_THREADS, 0, stream>>>(w.rec, w.offsets, d_mean, d_rstd, S, (float)eps, mom_rows);
+    launch_after(ln_combine_kernel, (unsigned)S, COMBINE_THREADS, 0, stream, w.rec, w.offsets, d_mean, d_rstd, S, (float)eps, mom_rows);
     PCX_LAUNCH_CHECK();
     if (N > 0) {
-        PCX_LN_DISPATCH(dtype, vec, (ln_apply_kernel<T, VN><<<(unsigned)((N + rows - 1) / rows), LN_THREADS, 0, stream>>>(
+        PCX_LN_DISPATCH(dtype, vec, (launch_after(ln_apply_kernel<T, VN>, (unsigned)((N + rows - 1) / rows), LN_THREADS, 0, stream, 
                                    (const T *)d_x, w.offsets, d_mean, d_rstd, d_weight, d_bias, (const T *)d_residual,
                                    (T *)d_y, N, S, C, relu, rows)));
         PCX_LAUNCH_CHECK();
@@ -767,14 +773,14 @@ int pcx_ragged_layer_norm_backward(const void *d_grad_y, const void *d_x, const 
     const bool vec = vec_ok(C, dtype, {d_grad_y, d_x, d_y, d_grad_x, d_grad_residual});
     const int rows = layer_rows(N, C, dtype, vec, 4);
     const unsigned grid = (unsigned)((N + rows - 1) / rows);
-    PCX_LN_DISPATCH(dtype, vec, (ln_bwd_sums_kernel<T, VN><<<grid, LN_THREADS, 0, stream>>>(
+    PCX_LN_DISPATCH(dtype, vec, (launch_after(ln_bwd_sums_kernel<T, VN>, grid, LN_THREADS, 0, stream, 
                                (const T *)d_grad_y, (const T *)d_x, (const T *)d_y, w.offsets, d_mean, d_rstd, d_weight,
                                w.sums, w.sums + S, d_grad_weight, d_grad_bias, (T *)d_grad_residual, N, S, C, relu, rows)));
     PCX_LAUNCH_CHECK();
     // the sums pass wrote the ReLU-masked gradient as the residual's gradient: the second pass reads
     // that instead of masking again, which spares it the read of y
     const bool masked = relu && d_grad_residual;
-    PCX_LN_DISPATCH(dtype, vec, (ln_bwd_apply_kernel<T, VN><<<grid, LN_THREADS, 0, stream>>>(
+    PCX_LN_DISPATCH(dtype, vec, (launch_after(ln_bwd_apply_kernel<T, VN>, grid, LN_THREADS, 0, stream, 
                                (const T *)(masked ? d_grad_residual : d_grad_y), (const T *)d_x, (const T *)d_y, w.offsets,
                                d_mean, d_rstd, d_weight, w.sums, w.sums + S, (T *)d_grad_x, N, S, C, masked ? 0 : relu, rows)));
     prof_end(stream);

@@ -70,6 +70,7 @@ constexpr int VVOR_CTAS = 4;
 
 template <typename T, bool TRANSPOSE, int NT>
 __global__ void __launch_bounds__(NT * 4, mvmr_ctas(NT)) mvmr_fma_kernel(const T *__restrict__ W, const T *__restrict__ feat, MvmrFmaParams p) {
+    start_after_previous();
     constexpr int THREADS = NT * 4, WP = NT + WPAD;
     extern __shared__ __align__(16) uint8_t raw[];
     __shared__ int32_t s_cum[TABLE_TAPS + 1], s_warp_sums[THREADS / 32], s_gather[MC], s_scatter[MC];
@@ -188,6 +189,7 @@ struct VvorFmaParams {
 // chunk (two groups for TE = 64) and each adds its own sums when the tap ends.
 template <typename T, int TE>
 __global__ void __launch_bounds__(128, VVOR_CTAS) vvor_fma_kernel(const T *__restrict__ A, const T *__restrict__ B, VvorFmaParams p) {
+    start_after_previous();
     constexpr int TP = TE + 4, PER = (TE / 8) * (TE / 8), TEAMS = 128 / PER;
     extern __shared__ __align__(16) uint8_t raw[];
     __shared__ int32_t s_cum[TABLE_TAPS + 1], s_warp_sums[4], s_a[VC], s_b[VC];
@@ -288,7 +290,7 @@ int launch_mvmr(const MvmrArgs &a, MvmrFmaParams p, cudaStream_t stream) {
     const int64_t upper = a.T / MC + a.K + 1;
     const dim3 grid((unsigned)std::min<int64_t>(upper, std::max<int64_t>(1, (int64_t)occ * num_sms() / tiles)), (unsigned)(tiles / p.G), (unsigned)p.G);
     prof_begin(TRANSPOSE ? "mvmr_fma_kernel(dgrad)" : "mvmr_fma_kernel(fwd)", stream);
-    mvmr_fma_kernel<T, TRANSPOSE, NT><<<grid, NT * 4, smem, stream>>>((const T *)a.weight, (const T *)a.feat, p);
+    launch_after(mvmr_fma_kernel<T, TRANSPOSE, NT>, grid, NT * 4, smem, stream, (const T *)a.weight, (const T *)a.feat, p);
     prof_end(stream);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
@@ -306,7 +308,7 @@ int launch_vvor(const VvorArgs &a, const VvorFmaParams &p, cudaStream_t stream) 
     if (TE == 32 && a.Ma * a.Cb > 512) upper = std::min(upper, a.n_o * 256);
     const dim3 grid((unsigned)std::min<int64_t>(upper, std::max<int64_t>(1, (int64_t)VVOR_CTAS * num_sms() / tiles)), (unsigned)(tiles / p.G), (unsigned)p.G);
     prof_begin("vvor_fma_kernel", stream);
-    vvor_fma_kernel<T, TE><<<grid, 128, smem, stream>>>((const T *)a.a, (const T *)a.b, p);
+    launch_after(vvor_fma_kernel<T, TE>, grid, 128, smem, stream, (const T *)a.a, (const T *)a.b, p);
     prof_end(stream);
     PCX_LAUNCH_CHECK();
     return PCX_OK;

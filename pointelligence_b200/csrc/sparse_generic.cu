@@ -86,6 +86,7 @@ __global__ void vvor_unsorted_kernel(const T *__restrict__ A, const int32_t *__r
 
 template <typename T>
 __global__ void round_kernel(const float *__restrict__ acc, T *__restrict__ out, int64_t n) {
+    start_after_previous();
     int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * 4;
     if (i + 3 < n) {
         float4 v = *reinterpret_cast<const float4 *>(acc + i);
@@ -150,8 +151,8 @@ int vvor_generic(const VvorArgs &a, cudaStream_t stream) {
 int round_accumulator(const float *acc, void *out, int64_t n, int dtype, cudaStream_t stream) {
     if (n == 0) return PCX_OK;
     unsigned blocks = (unsigned)((n / 4 + 255) / 256 + 1);
-    if (dtype == PCX_F16) round_kernel<__half><<<blocks, 256, 0, stream>>>(acc, (__half *)out, n);
-    else if (dtype == PCX_BF16) round_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(acc, (__nv_bfloat16 *)out, n);
+    if (dtype == PCX_F16) launch_after(round_kernel<__half>, blocks, 256, 0, stream, acc, (__half *)out, n);
+    else if (dtype == PCX_BF16) launch_after(round_kernel<__nv_bfloat16>, blocks, 256, 0, stream, acc, (__nv_bfloat16 *)out, n);
     else PCX_FAIL(PCX_E_DTYPE, "round_accumulator: dtype %d", dtype);
     PCX_LAUNCH_CHECK();
     return PCX_OK;

@@ -129,6 +129,7 @@ struct MvmrTcParams {
 // row occurs in exactly one triplet (fan-in 1: nothing to accumulate, clear or round afterwards).
 template <int MODE>
 __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
+    start_after_previous();
     constexpr bool BULK = MODE == 1;
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t s_bar;
@@ -489,9 +490,9 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
     const dim3 grid((unsigned)std::min<int64_t>(upper, std::max<int64_t>(1, (int64_t)occ * num_sms() / parts)), (unsigned)parts);
     prof_begin(store ? (a.transpose ? "mvmr_tc_kernel(dgrad, store)" : "mvmr_tc_kernel(fwd, store)")
                      : (a.transpose ? "mvmr_tc_kernel(dgrad)" : "mvmr_tc_kernel(fwd)"), stream);
-    if (store) mvmr_tc_kernel<2><<<grid, 128, smem, stream>>>(p);
-    else if (bulk) mvmr_tc_kernel<1><<<grid, 128, smem, stream>>>(p);
-    else mvmr_tc_kernel<0><<<grid, 128, smem, stream>>>(p);
+    if (store) launch_after(mvmr_tc_kernel<2>, grid, 128, smem, stream, p);
+    else if (bulk) launch_after(mvmr_tc_kernel<1>, grid, 128, smem, stream, p);
+    else launch_after(mvmr_tc_kernel<0>, grid, 128, smem, stream, p);
     prof_end(stream);
     PCX_LAUNCH_CHECK();
     return PCX_OK;

@@ -85,6 +85,7 @@ __device__ __forceinline__ void copy_operand(uint32_t tile, const uint16_t *src,
 
 template <int CHR>   // triplets of a chunk: the contraction of one slot
 __global__ void __launch_bounds__(THREADS, 1) vvor_tc_kernel(VvorTcParams p) {
+    start_after_previous();
     constexpr uint32_t BLK = CHR * 128;   // one 64-channel block of a tile
     using Cursor = ChunkCursorT<CHR>;
     extern __shared__ uint8_t smem_raw[];
@@ -255,7 +256,7 @@ int launch_vvor(VvorTcParams &p, int parts, int64_t T, size_t block_rows, cudaSt
     }
     const dim3 grid((unsigned)std::min<int64_t>(T / CHR + p.n_o + 1, std::max(1, num_sms() / parts)), (unsigned)parts);
     prof_begin("vvor_tc_kernel", stream);
-    vvor_tc_kernel<CHR><<<grid, THREADS, smem, stream>>>(p);
+    launch_after(vvor_tc_kernel<CHR>, grid, THREADS, smem, stream, p);
     prof_end(stream);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
