@@ -173,9 +173,10 @@ __device__ __forceinline__ void copy_seg(const int64_t *__restrict__ seg, int K,
 }
 
 __global__ void plan_init_kernel(int64_t n_out, uint32_t *sig, int32_t *row, int32_t *tile_cnt, int64_t n_tiles,
-                                 uint32_t *ctrl, int G) {
+                                 uint32_t *ctrl, int G, int4 *tile_rows) {
     start_after_previous();
-    const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, threads = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t t = x; t < n_tiles * (ROWS / 4); t += threads) tile_rows[t] = make_int4(-1, -1, -1, -1);   // no source anywhere
     if (x < n_out) sig[x] = 0u, row[x] = (int32_t)x;
     if (x <= n_tiles) tile_cnt[x] = 0;
     if (x < CTRL_WORDS) ctrl[x] = x == CTRL_MAGIC ? PLAN_MAGIC : x == CTRL_GROUP ? (uint32_t)G : 0u;
@@ -1102,9 +1103,10 @@ int pcx_mvmr_plan_build_counted(const int32_t *d_scatter, const int32_t *d_gathe
     const int TPB = 256;
     const int64_t n_tiles = pv.nblocks * K, n_pad = pv.nblocks * ROWS;
     auto blocks = [&](int64_t n) { return (unsigned)((n + TPB - 1) / TPB); };
-    const int64_t init_n = std::max<int64_t>(std::max<int64_t>(n_out, n_tiles + 1), CTRL_WORDS);
-    PCX_CUDA(cudaMemsetAsync(pv.tile_rows, 0xff, (size_t)n_tiles * ROWS * sizeof(int32_t), stream));
-    launch_after(plan_init_kernel, blocks(init_n), TPB, 0, stream, n_out, w.sig, w.row, w.tile_cnt, n_tiles, pv.ctrl, G);
+    const int64_t init_n = std::max(std::max<int64_t>(n_out, n_tiles + 1),
+                                    std::max<int64_t>(CTRL_WORDS, std::min<int64_t>(n_tiles * (ROWS / 4), (int64_t)num_sms() * 2048)));
+    launch_after(plan_init_kernel, blocks(init_n), TPB, 0, stream, n_out, w.sig, w.row, w.tile_cnt, n_tiles, pv.ctrl, G,
+                 reinterpret_cast<int4 *>(pv.tile_rows));
     PCX_LAUNCH_CHECK();
     size_t bytes = w.cub_bytes;
     if (T > 0) {

@@ -117,9 +117,11 @@ __device__ __forceinline__ uint32_t cell_bucket(int b, int cx, int cy, int cz, u
 }
 
 __global__ void taps_key_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, int64_t P,
-                                float inv, uint32_t mask, uint32_t *keys, int32_t *vals) {
+                                float inv, uint32_t mask, uint32_t *keys, int32_t *vals, int2 *table, int64_t *ctrl) {
     start_after_previous();
-    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, threads = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t t = p; t <= (int64_t)mask; t += threads) table[t] = make_int2(0, 0);   // every bucket empty
+    if (p < 8) ctrl[p] = 0;
     if (p >= P) return;
     keys[p] = cell_bucket(sample ? sample[p] : 0, cell_of(pts[3 * p], inv), cell_of(pts[3 * p + 1], inv),
                           cell_of(pts[3 * p + 2], inv), mask);
@@ -626,9 +628,7 @@ int pcx_radius_taps_count(const float *d_points, const float *d_queries, const i
     const float inv = (float)(1.0 / (2.0 * radius));
     const uint32_t mask = (uint32_t)(w.buckets - 1);
     const unsigned pblocks = (unsigned)((P + 255) / 256);
-    PCX_CUDA(cudaMemsetAsync(w.ctrl, 0, 8 * sizeof(int64_t), stream));
-    PCX_CUDA(cudaMemsetAsync(w.table, 0, (size_t)w.buckets * sizeof(int2), stream));
-    launch_after(taps_key_kernel, pblocks, 256, 0, stream, d_points, d_point_sample, P, inv, mask, w.keys_a, w.vals_a);
+    launch_after(taps_key_kernel, pblocks, 256, 0, stream, d_points, d_point_sample, P, inv, mask, w.keys_a, w.vals_a, w.table, w.ctrl);
     PCX_LAUNCH_CHECK();
     size_t tmp = w.cub_bytes;
     PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, tmp, w.keys_a, w.keys_b, w.vals_a, w.vals_b, P, 0, w.bits, stream));

@@ -165,7 +165,7 @@ int pcx_vvor(const void *d_a, const int32_t *d_a_idx, const void *d_b, const int
     a.acc = dtype == PCX_F32 ? (float *)d_out : w.acc;
     a.chunk_table = w.chunk_table;
     a.T = T, a.n_a = n_a, a.n_b = n_b, a.n_o = n_o, a.G = G, a.Ma = Ma, a.Cb = Cb, a.dtype = dtype;
-    PCX_CUDA(cudaMemsetAsync(a.acc, 0, (size_t)out_elems * sizeof(float), stream));
+    if (int rc = clear_accumulator(a.acc, nullptr, n_o * G * Ma, Cb, dtype, stream)) return rc;
     if (T > 0) {
         if (force_engine()) engine = force_engine();
         bool tensor_ok = vvor_tensor_supported(a);
