@@ -472,7 +472,14 @@ class MvmrPlan:
 
 def plan_group_blocks(out_width):
     """Blocks of 128 output rows that share the weight tiles they stream, for rows of ``out_width`` channels."""
-    return int(lib().pcx_mvmr_plan_group_blocks(min(int(out_width), 256)))
+    width = min(int(out_width), 256)
+    blocks = _GROUP_BLOCKS.get(width)
+    if blocks is None:
+        blocks = _GROUP_BLOCKS[width] = int(lib().pcx_mvmr_plan_group_blocks(width))
+    return blocks
+
+
+_GROUP_BLOCKS = {}
 
 
 def padded_width(width):
@@ -581,11 +588,11 @@ def _plan_key(scatter, gather, seg_offs, K, n_out, group_blocks):
             int(group_blocks))
 
 
-def _remembered_plan(scatter, gather, seg_offs, K, n_out, group_blocks):
-    hit = _PLAN_CACHE.get(_plan_key(scatter, gather, seg_offs, K, n_out, group_blocks))
+def _remembered_plan(key, scatter, gather, seg_offs):
+    hit = _PLAN_CACHE.get(key)
     if hit is not None:
-        refs, old_stamp, value = hit
-        if old_stamp == _stamp(scatter, gather, seg_offs) and all(r() is t for r, t in zip(refs, (scatter, gather, seg_offs))):
+        (i, j, seg), stamp, value = hit
+        if i() is scatter and j() is gather and seg() is seg_offs and stamp == _stamp(scatter, gather, seg_offs):
             return value
     return None
 
@@ -596,12 +603,12 @@ def cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks):
     import weakref
 
     key = _plan_key(scatter, gather, seg_offs, K, n_out, group_blocks)
+    value = _remembered_plan(key, scatter, gather, seg_offs)
+    if value is not None:
+        return value
     stamp = _stamp(scatter, gather, seg_offs)
     if stamp is None:
         return mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks)
-    value = _remembered_plan(scatter, gather, seg_offs, K, n_out, group_blocks)
-    if value is not None:
-        return value
     value = mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks)
     value._stream = torch.cuda.current_stream(scatter.device)
     for k in [k for k, (refs, _, _) in _PLAN_CACHE.items() if any(r() is None for r in refs)]:
@@ -641,15 +648,18 @@ def mvmr(weight, feat, gather, scatter, seg_offs, tap_idx, n_out, transpose, eng
 def _plan_hook(scatter, gather, seg_offs, K, n_out, outw, inw, forced, split=False):
     """Asked by the host path for every pass the output-stationary kernel could take: the plan to run
     (buffer, blocks per group, multi-triplet buckets) or None for the scatter engine."""
-    if not forced and (not _planned_pays(gather.numel(), n_out, outw, K) or scatter.is_inference()
-                       or gather.is_inference() or seg_offs.is_inference()):
-        return None    # (a plan of inference tensors cannot be remembered, and one per pass does not pay)
-    if split and not _split_pays(gather.numel(), n_out, outw, inw, K):
+    T, blocks = gather.numel(), plan_group_blocks(outw)
+    if not forced and not _planned_pays(T, n_out, outw, K):
         return None
-    if split and torch.cuda.is_current_stream_capturing() and _remembered_plan(
-            scatter, gather, seg_offs, K, n_out, plan_group_blocks(outw)) is None:
-        return None    # building it may wait for the device: the scatter kernels can be captured as they are
-    plan = cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, plan_group_blocks(outw))
+    plan = _remembered_plan(_plan_key(scatter, gather, seg_offs, K, n_out, blocks), scatter, gather, seg_offs)
+    if split and not _split_pays(T, n_out, outw, inw, K):
+        return None
+    if plan is None:
+        if not forced and (scatter.is_inference() or gather.is_inference() or seg_offs.is_inference()):
+            return None    # (a plan of inference tensors cannot be remembered, and one per pass does not pay)
+        if split and torch.cuda.is_current_stream_capturing():
+            return None    # building it may wait for the device: the scatter kernels can be captured as they are
+        plan = cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, blocks)
     return plan.buffer, plan.group_blocks, plan.multi_buckets
 
 
