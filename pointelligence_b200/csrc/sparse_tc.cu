@@ -98,9 +98,13 @@ __device__ __forceinline__ float unpack_one(uint16_t v, int fmt) {
     return fmt ? __bfloat162float(__ushort_as_bfloat16(v)) : __half2float(__ushort_as_half(v));
 }
 
-// Wide and grouped layers run as parts of at most 256 x 256 channels: blockIdx.y counts (group, part of the
-// output row, part of the contraction), the parts of a contraction meet in the accumulator's reductions.
-// Every part of a width has the same size, a multiple of 16.
+// Wide and grouped layers run as parts of at most 256 x 256 channels, every part of a width of the same size, a
+// multiple of 16.  blockIdx.y counts (group, part of the output row, link of the contraction): a block takes up to
+// p.chain parts of a contraction one after another, each into tensor memory columns of its own, and reduces their
+// sum.  (As blocks of their own they meet in the accumulator, with as many reductions more: fp16, 31 852 triplets of
+// 512 x 512 channels 75 us, chained 65; 408 976 triplets 726 and 676; 2048 to 128 channels 895 and 817.)  One column
+// range for all of them would need no additions (676 would be 657), but the tensor cores drop bits at each step of a
+// chain: rows of 2048 channels of one sign came out with ten times the error against fp64, 1.2e-5.
 
 struct MvmrTcParams {
     const uint16_t *weight;  // (K, C, M) as stored
@@ -112,12 +116,12 @@ struct MvmrTcParams {
     const uint16_t *bias;    // MODE 2: added before the rounding (null: none); the other modes start from it
     int reverse;             // tap k uses weight K-1-k
     int64_t in_pitch, out_pitch, w_pitch, w_tap;   // rows of features / output / one tap's weight, elements of one tap's weight
-    int out_parts, in_parts;                       // C, M below: the part's
+    int out_parts, in_parts, chain;                // C, M below: the part's; contraction parts a block takes
     int K, C, M, transpose, fmt, nbuf, slab;  // slab: columns parked per bulk reduction (32 or 64)
     int prow_log2;                            // a warp parks 2^prow_log2 rows at a time (8, 16 or 32)
     uint32_t park_bytes;                      // size of the parking area (the chunk table follows it)
     int alias;                                // parking area shares the feature tile's memory
-    uint32_t ncols;
+    uint32_t ncols, acc_cols;                 // tensor memory columns of a block, of one part
 };
 
 // One A tile by default: the next gather is issued as soon as the multiply has finished (or,
@@ -127,8 +131,11 @@ struct MvmrTcParams {
 // MODE 0: sums leave through two-float reductions from registers; 1: one bulk reduction per row
 // (rows of 64 floats); 2: plain 16-byte stores of the rounded row, for rulebooks in which every output
 // row occurs in exactly one triplet (fan-in 1: nothing to accumulate, clear or round afterwards).
-template <int MODE>
-__global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
+// NT: 128 threads, or 256 where shared memory leaves room for few CTAs (mode 0): with four warps an SM a 256 x 256 part
+// waited for its own copies and reductions (31 852 triplets of 512 x 512 fp16 channels 69 us, with eight warps 65;
+// 256 x 256 channels, 408 976 triplets 212 and 201).
+template <int MODE, int NT, bool CHAINED>
+__global__ void __launch_bounds__(NT, NT == 256 ? 1 : 0) mvmr_tc_kernel(MvmrTcParams p) {
     start_after_previous();
     constexpr bool BULK = MODE == 1;
     extern __shared__ uint8_t smem_raw[];
@@ -136,12 +143,14 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
     __shared__ uint32_t s_tmem;
     __shared__ __align__(16) int32_t s_scatter[2][CH];
     __shared__ int32_t s_gather[2][CH];
-    __shared__ int32_t s_warp_sums[4];
+    __shared__ int32_t s_warp_sums[NT / 32];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int inw = p.transpose ? p.M : p.C, outw = p.transpose ? p.C : p.M;
+    int parts;   // of the contraction, in this block
     {
-        const int ip = (int)blockIdx.y % p.in_parts, op = (int)blockIdx.y / p.in_parts % p.out_parts,
-                  g = (int)blockIdx.y / (p.in_parts * p.out_parts);
+        const int links = (p.in_parts + p.chain - 1) / p.chain, ip = (int)blockIdx.y % links * p.chain,
+                  op = (int)blockIdx.y / links % p.out_parts, g = (int)blockIdx.y / (links * p.out_parts);
+        parts = CHAINED ? min(p.chain, p.in_parts - ip) : 1;
         const int64_t out0 = ((int64_t)g * p.out_parts + op) * outw;
         p.feat += ((int64_t)g * p.in_parts + ip) * inw;
         p.acc += out0;
@@ -191,13 +200,17 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
     int loaded_tap = -1;
     bool alive = true;
 
-    auto load_weight = [&](int tap) {
-        const uint16_t *w = p.weight + (p.reverse ? p.K - 1 - tap : tap) * p.w_tap;
+    auto load_weight = [&](int tap, int part) {
+        const uint16_t *w = p.weight + (p.reverse ? p.K - 1 - tap : tap) * p.w_tap +
+                            (p.transpose ? (int64_t)part * p.M : part * p.C * p.w_pitch);
         const int cpr = p.M >> 3;
-        for (int e = tid; e < p.C * cpr; e += 128) {
-            int c = e / cpr, ch = e - c * cpr;
+        const int dc = NT / cpr, dch = NT - dc * cpr;   // from one piece of a thread to its next
+        int c = tid / cpr, ch = tid - c * cpr;
+        for (int e = tid; e < p.C * cpr; e += NT) {
             uint32_t dst = b_tile + (uint32_t)(ch >> 3) * w_blk + (uint32_t)c * 128 + (uint32_t)(((ch & 7) ^ (c & 7)) << 4);
             cp_async16(dst, w + c * p.w_pitch + ch * 8);
+            c += dc, ch += dch;
+            if (ch >= cpr) ch -= cpr, ++c;
         }
     };
 
@@ -212,10 +225,10 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
             s_gather[0][tid] = p.gather[c0.first(lo) + tid];
             s_scatter[0][tid] = p.scatter[c0.first(lo) + tid];
         }
-        load_weight(c0.tap);
+        load_weight(c0.tap, 0);
         loaded_tap = c0.tap;
         __syncthreads();
-        gather_tile(a_tile0, p.feat, s_gather[0], rows, inw, p.in_pitch, tid, 128);
+        gather_tile(a_tile0, p.feat, s_gather[0], rows, inw, p.in_pitch, tid, NT);
         cp_async_commit();
         if (lo + 1 < hi) {
             c1.advance(s_cum, p.seg, p.K, lo + 1);
@@ -238,7 +251,7 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
         }
         __syncthreads();
         if (have_next && two)
-            gather_tile(a_tile0 + (uint32_t)(b ^ 1) * a_bytes, p.feat, s_gather[b ^ 1], rows_next, inw, p.in_pitch, tid, 128);
+            gather_tile(a_tile0 + (uint32_t)(b ^ 1) * a_bytes, p.feat, s_gather[b ^ 1], rows_next, inw, p.in_pitch, tid, NT);
         cp_async_commit();
         if (chunk + 2 < hi) {
             c2.advance(s_cum, p.seg, p.K, chunk + 2);
@@ -247,34 +260,40 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
                 pre_s = p.scatter[c2.first(chunk + 2) + tid];
             }
         }
-        if (two) cp_async_wait<1>();  // everything but the gather just issued has landed
-        else cp_async_wait<0>();
-        fence_async_smem();
-        __syncthreads();
+        for (int part = 0;; ++part) {
+            if (two) cp_async_wait<1>();  // everything but the gather just issued has landed
+            else cp_async_wait<0>();
+            fence_async_smem();
+            __syncthreads();
 
-        if (tid == 0) {
-            tc_fence_after();
-            const uint32_t a_tile = a_tile0 + (two ? (uint32_t)b * a_bytes : 0u);
-            for (int s = 0; s < ksteps; ++s) {
-                uint64_t ad = smem_desc(a_tile + (uint32_t)(s >> 2) * BLK_BYTES + (uint32_t)(s & 3) * 32, 16, 1024);
-                uint64_t bd = p.transpose
-                                  ? smem_desc(b_tile + (uint32_t)(s >> 2) * w_blk + (uint32_t)(s & 3) * 32, 16, 1024)
-                                  : smem_desc(b_tile + (uint32_t)s * 2048, w_blk, 1024);
-                tc_mma(tmem, ad, bd, idesc, s > 0 ? 1u : 0u);
+            if (tid == 0) {
+                tc_fence_after();
+                const uint32_t a_tile = a_tile0 + (two ? (uint32_t)b * a_bytes : 0u);
+                for (int s = 0; s < ksteps; ++s) {
+                    uint64_t ad = smem_desc(a_tile + (uint32_t)(s >> 2) * BLK_BYTES + (uint32_t)(s & 3) * 32, 16, 1024);
+                    uint64_t bd = p.transpose
+                                      ? smem_desc(b_tile + (uint32_t)(s >> 2) * w_blk + (uint32_t)(s & 3) * 32, 16, 1024)
+                                      : smem_desc(b_tile + (uint32_t)s * 2048, w_blk, 1024);
+                    tc_mma(tmem + (uint32_t)part * p.acc_cols, ad, bd, idesc, s > 0 ? 1u : 0u);
+                }
+                tc_commit(bar);
             }
-            tc_commit(bar);
+            alive = __syncthreads_and(mbar_wait(bar, phase, 1u, &g_device_status));
+            phase ^= 1u;
+            tc_fence_after();
+            if (part + 1 >= parts || !alive) break;
+            load_weight(c0.tap, part + 1);   // the next part, over both tiles
+            gather_tile(a_tile0, p.feat + (int64_t)(part + 1) * inw, s_gather[b], rows, inw, p.in_pitch, tid, NT);
+            cp_async_commit();
         }
-        alive = __syncthreads_and(mbar_wait(bar, phase, 1u, &g_device_status));
-        phase ^= 1u;
-        tc_fence_after();
         // the weight tile is free now: fetch the next tap's if the next chunk needs it
-        if (have_next && c1.tap != loaded_tap) {
-            load_weight(c1.tap);
+        if (have_next && (c1.tap != loaded_tap || parts > 1)) {
+            load_weight(c1.tap, 0);
             loaded_tap = c1.tap;
             cp_async_commit();
         }
         if (have_next && !two && !p.alias) {  // single A tile: it is free as well
-            gather_tile(a_tile0, p.feat, s_gather[b ^ 1], rows_next, inw, p.in_pitch, tid, 128);
+            gather_tile(a_tile0, p.feat, s_gather[b ^ 1], rows_next, inw, p.in_pitch, tid, NT);
             cp_async_commit();
         }
         if (BULK && alive && warp * 32 < rows) {
@@ -331,18 +350,26 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
                     }
                 }
             }
-        } else if (MODE == 0 && alive && warp * 32 < rows) {
+        } else if (MODE == 0 && alive && (warp & 3) * 32 < rows) {
             // wide rows: scatter from registers (two-float vector reductions); with several
             // 64-column blocks per row the single parking area would serialise the bulk reductions
             const int32_t *sc = s_scatter[b];
+            const int quarter = warp & 3;   // the lanes of tensor memory a warp can read
 #pragma unroll 1
             for (int half = 0; half < 2; ++half) {
-                if (warp * 32 + half * 16 >= rows) break;
-                const int ra = warp * 32 + half * 16 + (lane >> 2), rb = ra + 8;
+                if (quarter * 32 + half * 16 >= rows) break;
+                const int ra = quarter * 32 + half * 16 + (lane >> 2), rb = ra + 8;
                 const int64_t da = ra < rows ? sc[ra] : -1, db = rb < rows ? sc[rb] : -1;
-                for (int col0 = 0; col0 < outw; col0 += 64) {
+                for (int col0 = (warp >> 2) * 64; col0 < outw; col0 += 64 * (NT / 128)) {
                     float v[32];
-                    tmem_ld_16x64(tmem + ((uint32_t)(warp * 32 + half * 16) << 16) + (uint32_t)col0, v);
+                    const uint32_t from = tmem + ((uint32_t)(quarter * 32 + half * 16) << 16) + (uint32_t)col0;
+                    tmem_ld_16x64(from, v);
+                    for (int part = 1; CHAINED && part < parts; ++part) {
+                        float u[32];
+                        tmem_ld_16x64(from + (uint32_t)part * p.acc_cols, u);
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) v[e] += u[e];
+                    }
                     scatter_block(p.acc, da, db, outw, p.out_pitch, col0, lane, v);
                 }
             }
@@ -353,7 +380,7 @@ __global__ void __launch_bounds__(128) mvmr_tc_kernel(MvmrTcParams p) {
             bulk_wait_read();
             __syncthreads();
             if (have_next) {
-                gather_tile(a_tile0, p.feat, s_gather[b ^ 1], rows_next, inw, p.in_pitch, tid, 128);
+                gather_tile(a_tile0, p.feat, s_gather[b ^ 1], rows_next, inw, p.in_pitch, tid, NT);
                 cp_async_commit();
             }
         }
@@ -436,12 +463,12 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
     p.in_parts = a.transpose ? m_parts : c_parts, p.out_parts = a.transpose ? c_parts : m_parts;
     p.in_pitch = (int64_t)a.G * p.in_parts * inw, p.out_pitch = (int64_t)a.G * p.out_parts * outw;
     p.w_pitch = a.M, p.w_tap = (int64_t)a.G * a.C * a.M;
-    const int parts = a.G * c_parts * m_parts;
+    const int64_t upper = a.T / CH + a.K + 1;   // tiles of triplets, at most
     p.weight = (const uint16_t *)a.weight, p.feat = (const uint16_t *)a.feat;
     p.gather = a.gather, p.scatter = a.scatter, p.seg = a.seg_offs, p.acc = a.acc;
     p.out = (uint16_t *)a.out_rows, p.bias = (const uint16_t *)a.bias, p.reverse = a.reverse;
     p.K = a.K, p.C = C, p.M = M, p.transpose = a.transpose, p.fmt = a.dtype == PCX_BF16 ? 1 : 0;
-    p.ncols = pow2_cols((outw + 63) / 64 * 64);  // the epilogue reads blocks of up to 64 columns
+    p.ncols = p.acc_cols = pow2_cols((outw + 63) / 64 * 64);  // the epilogue reads blocks of up to 64 columns
     // Measured on B200: rows of exactly 64 floats leave fastest through one bulk reduction
     // each (64 vs 84 us on the 150k-point scene); narrower and wider rows from registers
     // (C = 32: 50 vs 59 us, C = 128: 160 vs 180 us, C = 256: 390 vs 671 us).  Folding rows
@@ -472,27 +499,36 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
         if (atoi(e) == 2 && rest + 2 * (size_t)kb * BLK_BYTES + static_smem <= 232448 - 1024) p.nbuf = 2;
     if (p.alias) p.nbuf = 1;
     size_t smem = rest + std::max((size_t)p.nbuf * kb * BLK_BYTES, p.alias ? (size_t)p.park_bytes : (size_t)0);
+    // 256 threads, and the parts of a contraction in one block, where one CTA fills an SM's shared memory.  The parts
+    // stay blocks of their own where the chip would not be filled without: 1 920 triplets, 2048 to 128 channels, took
+    // 34.6 us with eight parts in one block and 17.7 in eight.  Plain reductions into an accumulator much larger than
+    // the L2 cache keep 128 threads: they are bound by its misses (256 x 256 into 184 MB 584 us and with 256 threads
+    // 620; into 123 MB 398 and 388, 61 MB 208 and 202).
+    const bool one_cta = !store && !bulk && outw > 64 && 2 * (smem + static_smem + 1024) > 232448;
+    p.chain = one_cta && p.nbuf == 1 ? std::min(p.in_parts, (int)(512 / p.acc_cols)) : 1;
+    auto blocks = [&] { return a.G * p.out_parts * ((p.in_parts + p.chain - 1) / p.chain); };
+    if (upper * blocks() < num_sms()) p.chain = 1;
+    const int parts = blocks();
+    p.ncols = pow2_cols(p.acc_cols * p.chain);
+    const bool more = one_cta && (p.chain > 1 || a.n_out * p.out_pitch * 4 <= (int64_t)160 << 20);
     smem = pad_for_tmem(smem, p.ncols);
     if (smem + static_smem > 232448 - 1024) PCX_FAIL(PCX_E_UNSUPPORTED, "mvmr tensor kernel does not fit (smem %zu)", smem);
-    static int granted_mvmr[3][64] = {};   // per output mode and device
+    const int mode = store ? 2 : bulk ? 1 : p.chain > 1 ? 4 : more ? 3 : 0, threads = more ? 256 : 128;
+    static int granted_mvmr[5][64] = {}, regs_mvmr[5] = {};   // per kernel (and device)
+    const auto kernel = mode == 4   ? mvmr_tc_kernel<0, 256, true>
+                        : mode == 3 ? mvmr_tc_kernel<0, 256, false>
+                        : mode == 2 ? mvmr_tc_kernel<2, 128, false>
+                        : mode == 1 ? mvmr_tc_kernel<1, 128, false>
+                                    : mvmr_tc_kernel<0, 128, false>;
     int dev = 0;
     PCX_CUDA(cudaGetDevice(&dev));
-    if (int rc = store ? ensure_dynamic_smem(mvmr_tc_kernel<2>, smem, &granted_mvmr[2][dev & 63])
-                 : bulk ? ensure_dynamic_smem(mvmr_tc_kernel<1>, smem, &granted_mvmr[1][dev & 63])
-                        : ensure_dynamic_smem(mvmr_tc_kernel<0>, smem, &granted_mvmr[0][dev & 63]))
-        return rc;
-    static int regs_mvmr[3] = {0, 0, 0};
-    const int regs = store ? kernel_registers(mvmr_tc_kernel<2>, &regs_mvmr[2])
-                     : bulk ? kernel_registers(mvmr_tc_kernel<1>, &regs_mvmr[1])
-                            : kernel_registers(mvmr_tc_kernel<0>, &regs_mvmr[0]);
-    const int occ = ctas_per_sm(smem + static_smem, p.ncols, regs);
-    int64_t upper = a.T / CH + a.K + 1;
+    if (int rc = ensure_dynamic_smem(kernel, smem, &granted_mvmr[mode][dev & 63])) return rc;
+    const int regs = kernel_registers(kernel, &regs_mvmr[mode]);
+    const int occ = ctas_per_sm(smem + static_smem, p.ncols, regs, threads);
     const dim3 grid((unsigned)std::min<int64_t>(upper, std::max<int64_t>(1, (int64_t)occ * num_sms() / parts)), (unsigned)parts);
     prof_begin(store ? (a.transpose ? "mvmr_tc_kernel(dgrad, store)" : "mvmr_tc_kernel(fwd, store)")
                      : (a.transpose ? "mvmr_tc_kernel(dgrad)" : "mvmr_tc_kernel(fwd)"), stream);
-    if (store) launch_after(mvmr_tc_kernel<2>, grid, 128, smem, stream, p);
-    else if (bulk) launch_after(mvmr_tc_kernel<1>, grid, 128, smem, stream, p);
-    else launch_after(mvmr_tc_kernel<0>, grid, 128, smem, stream, p);
+    launch_after(kernel, grid, threads, smem, stream, p);
     prof_end(stream);
     PCX_LAUNCH_CHECK();
     return PCX_OK;

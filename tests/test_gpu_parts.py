@@ -170,3 +170,32 @@ def test_plan_of_a_geometry_built_rulebook_is_not_waited_for(n):
     side.synchronize()
     torch.cuda.synchronize()
     assert plan.multi_buckets == want.multi_buckets and plan._word is None
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("T", [1, 300, 9000])
+@pytest.mark.parametrize("C,M,G", [(512, 64, 1), (320, 288, 1), (768, 288, 1), (2048, 16, 1), (384, 512, 2)])
+def test_parts_of_a_contraction_in_one_block(C, M, G, T, dtype):
+    """Few tiles: each part a block of its own; many: one block takes them one after another.  Operands of -1, 0 and 1
+    keep every sum a whole number below 2^8, exact in fp32 and after the rounding, in any order."""
+    from pointelligence_b200 import _cabi
+
+    n = max(2, T // 4)
+    i, j, k, seg = _rulebook(n, n, 27, T, 7)
+    g = torch.Generator(device=DEV).manual_seed(8)
+
+    def few(*shape):   # one in eight is -1 or 1
+        sign = 2 * torch.randint(0, 2, shape, device=DEV, generator=g) - 1
+        return (torch.randint(0, 8, shape, device=DEV, generator=g) // 7 * sign).to(dtype)
+
+    w, x, go = few(27, G, C, M), few(n, G * C), few(n, G * M)
+    y_ref = torch.zeros(n, G, M, dtype=torch.float64, device=DEV)
+    gx_ref = torch.zeros(n, G, C, dtype=torch.float64, device=DEV)
+    for t in range(27):
+        s = slice(int(seg[t]), int(seg[t + 1]))
+        y_ref.index_add_(0, i[s].long(), torch.einsum("tgc,gcm->tgm", x[j[s].long()].view(-1, G, C).double(), w[t].double()))
+        gx_ref.index_add_(0, j[s].long(), torch.einsum("tgm,gcm->tgc", go[i[s].long()].view(-1, G, M).double(), w[t].double()))
+    assert max(y_ref.abs().max(), gx_ref.abs().max()) < 256
+    y = _cabi.mvmr(w, x, j, i, seg, None, n, False, _cabi.ENGINE_TENSOR)
+    gx = _cabi.mvmr(w, go, i, j, seg, None, n, True, _cabi.ENGINE_TENSOR)
+    assert torch.equal(y.double(), y_ref.flatten(1)) and torch.equal(gx.double(), gx_ref.flatten(1))
