@@ -186,9 +186,11 @@ __device__ __forceinline__ int2 run_of(const TapArgs &a, float qx, float qy, flo
     const int cy = corner_of(qy, a.r32, a.inv) + ((c >> 1) & 1);
     const int cz = corner_of(qz, a.r32, a.inv) + (c & 1);
     // A cell farther from the query than the radius holds no neighbour.  A point of cell k lies at 2 R k or behind it up to
-    // the rounding of its cell, some 3e-7 of the coordinate; the predicate's own rounding is some 1e-6 of R^2.
+    // the rounding of its cell, some 3e-7 of the coordinate; the predicate's own rounding is some 1e-6 of R^2.  A cell number
+    // at the end of the integers says no more than that the point lies there or beyond: such a cell is always looked at.
     if (a.distance_type == 0) {
         auto gap = [&](float v, int k) {
+            if (k >= 1 << 30 || k <= -(1 << 30)) return 0.f;
             const float lo = (float)k * a.cell, slack = 1e-6f * (fabsf(v) + 2.f * a.cell);
             return fmaxf(fmaxf(lo - v, v - (lo + a.cell)) - slack, 0.f);
         };

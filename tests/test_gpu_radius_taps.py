@@ -240,3 +240,18 @@ def test_cells_out_of_reach(shift):
     q = np.where(rng.random(q.shape) < 0.3, q + rng.uniform(-radius, radius, q.shape).astype(np.float32), q).astype(np.float32)
     _cabi._TAPS_RATIO.clear()
     _assert_same(*_both(torch.from_numpy(p).to(dev), torch.from_numpy(q).to(dev), None, None, radius, 3, 0.02))
+
+
+@pytest.mark.parametrize("at", [5e6, -5e6, 1e30, 2.0 ** 30 * 2e-3, -(2.0 ** 30) * 2e-3, 2.0 ** 31 * 2e-3])
+@pytest.mark.parametrize("axis", [0, 2])
+def test_cells_beyond_the_integers(at, axis):
+    """Coordinates whose cell number does not fit 32 bits, or lies about where the search stops trusting it: all of them share
+    a cell at the end, and a point still finds itself and its copies."""
+    dev, radius = torch.device("cuda:0"), 1e-3
+    g = torch.Generator().manual_seed(7)
+    p = torch.rand(50, 3, generator=g) * 0.01
+    p[:, axis] = (at + abs(at) * 2e-5 * torch.rand(50, generator=g)).float()
+    p = torch.cat([p, p[:20]]).to(dev)
+    ref, got = _both(p, p, None, None, radius, 3, 1e-3)
+    _assert_same(ref, got)
+    assert got[0].numel() >= p.shape[0]
