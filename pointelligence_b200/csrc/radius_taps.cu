@@ -400,7 +400,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) taps_colscan_kernel(uint32_t *bl
 // query and tap when they are written; matching lanes by tap kept one pipe 63 % busy and took 141 us instead of 111 below.
 // Before pairs were sorted in shared memory and written side by side: 512 000 queries with 13 neighbours 175 -> 112 us,
 // 150 000 points 37 -> 26, LiDAR 67 -> 38 (with 64 instead of 48 kept pairs; 65 with 48: one query in ninety has more,
-// and its warp keeps the block waiting), 125 taps, 100 000 queries with 41 152 -> 110
+// and its warp keeps the block waiting), 125 taps, 100 000 queries with 41 152 -> 110.
+// Queries with more pairs than are kept: 40 000 with 145 of them 766 us, with 374 4.2 ms (125 taps: 637, 3.3 ms); 1389 and
+// 8.5 ms (901, 5.4 ms) when every warp walked its runs again in every round of the block.
 template <bool FUSED, int REC_MAX>   // pairs staged per round
 __global__ void __launch_bounds__(THREADS, REC_MAX > 1024 ? 4 : 5) taps_fill_kernel(TapArgs a) {
     start_after_previous();
@@ -440,6 +442,7 @@ __global__ void __launch_bounds__(THREADS, REC_MAX > 1024 ? 4 : 5) taps_fill_ker
     const uint32_t block_total = __shfl_sync(0xffffffffu, upto, 31);
     const uint32_t nq = __shfl_sync(0xffffffffu, n_lane, ql), q_off = __shfl_sync(0xffffffffu, upto, ql) - nq;
     const bool kept = __all_sync(0xffffffffu, nq <= (uint32_t)a.kept);   // all accepted points of the warp's queries were kept
+    const uint32_t warp_first = __shfl_sync(0xffffffffu, q_off, 0), warp_end = __shfl_sync(0xffffffffu, q_off + nq, 31);
     for (uint32_t lo = 0; lo < block_total; lo += REC_MAX) {
         const uint32_t cnt = min((uint32_t)REC_MAX, block_total - lo);
         for (int t = threadIdx.x; t < a.k3 * QPB / 2; t += THREADS) reinterpret_cast<uint32_t *>(s_cnt)[t] = 0u;
@@ -480,7 +483,7 @@ __global__ void __launch_bounds__(THREADS, REC_MAX > 1024 ? 4 : 5) taps_fill_ker
                     s_nth[pos] = (uint16_t)nth;
                 }
             }
-        } else {
+        } else if (warp_first < lo + REC_MAX && warp_end > lo) {   // only in the rounds that hold pairs of the warp's queries
             const Queries queries(a, q, lane, s_u.walk.query[warp]);
             Accepted accepted(s_u.walk.queue[warp]);
             auto put = [&](bool there, int pos, int query, int nth) {

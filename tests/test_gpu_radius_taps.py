@@ -255,3 +255,23 @@ def test_cells_beyond_the_integers(at, axis):
     ref, got = _both(p, p, None, None, radius, 3, 1e-3)
     _assert_same(ref, got)
     assert got[0].numel() >= p.shape[0]
+
+
+@pytest.mark.parametrize("k", [3, 5])
+@pytest.mark.parametrize("long", [300, 1600])
+def test_long_lists_among_short_ones(long, k):
+    """Queries with more pairs than a block places at a time among queries with few or none: a warp walks its runs again in
+    the rounds that hold pairs of its queries, and in those alone."""
+    from pointelligence_b200 import _cabi
+
+    dev = torch.device("cuda:0")
+    gen = torch.Generator().manual_seed(long + k)
+    centre = torch.arange(4).float()[:, None] * torch.tensor([[0.31, 0.0, 0.0]])
+    pts = torch.repeat_interleave(centre, torch.tensor([long, 3, long // 2, 70]), 0)
+    pts = (pts + 0.008 * torch.randn(pts.shape, generator=gen)).to(dev)
+    which = torch.randint(0, 6, (200,), generator=gen)        # clusters 4 and 5: nothing there
+    qry = (which.float()[:, None] * torch.tensor([[0.31, 0.0, 0.0]]) + 0.004 * torch.randn(200, 3, generator=gen)).to(dev)
+    _cabi._TAPS_RATIO.clear()
+    ref, got = _both(pts, qry, None, None, 0.05, k, 0.02)
+    _assert_same(ref, got)
+    assert int(got[4].max()) > long // 2 and int(got[4].min()) == 0
