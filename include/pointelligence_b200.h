@@ -217,9 +217,12 @@ int pcx_mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan,
  * over the whole chip (its fp32 sums go through the workspace); with less it
  * runs on as many SMs as it has groups.  PCX_MVMR_SPLIT_SUMS keeps every bucket
  * sum as two numbers of the feature type, the rounded sum and what the rounding
- * left over, and multiplies both (bf16: as exact as fp32 sums of the products
- * once the row is rounded); the workspace is then the one for twice in_width.
- * In fp16 sums beyond 65504 are not finite with or without it. */
+ * left over (zero where the rounded sum is not finite), and multiplies both
+ * (bf16: 16 bits of the sum); the workspace is then the one for twice in_width.
+ * In fp16 sums beyond 65504 are not finite with or without it.  Operands that
+ * are not finite: every row of a block of 128 is multiplied with every tap that
+ * one of them has, rows without it as zeros, so an infinite weight makes rows
+ * NaN that never meet its tap.  pcx_mvmr and pcx_mvmr_split keep rows apart. */
 size_t pcx_mvmr_planned_scratch_bytes(int64_t multi_buckets, int in_width,
                                       int64_t n_out, int out_width, int K,
                                       int G);
@@ -229,6 +232,23 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat,
                           int K, int G, int C, int M, int flags, int dtype,
                           int group_blocks, int64_t multi_buckets, void *d_ws,
                           size_t ws_bytes, void *stream);
+
+/* pcx_mvmr_bias (bf16, tensor engine) by way of a plan: pcx_mvmr_planned_bias
+ * with PCX_MVMR_SPLIT_SUMS, and where a weight or a rounded bucket sum is not
+ * finite the kernels of pcx_mvmr_bias afterwards, over the same output, so that
+ * infinities and NaN are where those put them.  The device decides: nothing is
+ * waited for.  `flags`: PCX_MVMR_TRANSPOSE, PCX_MVMR_REVERSE_TAPS; d_gather,
+ * d_scatter, d_seg_offs: the rulebook the plan was built from. */
+size_t pcx_mvmr_split_workspace_bytes(int64_t multi_buckets, int64_t n_out,
+                                      int K, int G, int C, int M,
+                                      int transpose);
+int pcx_mvmr_split(const void *d_weight, const void *d_feat,
+                   const int32_t *d_gather, const int32_t *d_scatter,
+                   const int64_t *d_seg_offs, void *d_plan, size_t plan_bytes,
+                   const void *d_bias, void *d_out, int64_t T, int64_t n_feat,
+                   int64_t n_out, int K, int G, int C, int M, int flags,
+                   int group_blocks, int64_t multi_buckets, void *d_ws,
+                   size_t ws_bytes, void *stream);
 
 /* Launches one thread that waits on a barrier nothing arrives at: the bounded
  * wait gives up after limit_ns (at most 100 ms), sets bit 8 of the device

@@ -66,6 +66,9 @@ SIGNATURES = {
     "pcx_mvmr_planned_scratch_bytes": (c_size_t, [c_int64, c_int, c_int64, c_int, c_int, c_int]),
     "pcx_mvmr_planned_bias": (c_int, [c_void_p] * 3 + [c_size_t] + [c_void_p] * 2 + [c_int64] * 3 + [c_int] * 7
                               + [c_int64, c_void_p, c_size_t, c_void_p]),
+    "pcx_mvmr_split_workspace_bytes": (c_size_t, [c_int64, c_int64] + [c_int] * 5),
+    "pcx_mvmr_split": (c_int, [c_void_p] * 6 + [c_size_t] + [c_void_p] * 2 + [c_int64] * 3 + [c_int] * 6
+                       + [c_int64, c_void_p, c_size_t, c_void_p]),
     "pcx_debug_wait_runs_out": (c_int, [ctypes.c_ulonglong, c_void_p]),
     "pcx_vvor_workspace_bytes": (c_size_t, [c_int64, c_int, c_int, c_int, c_int]),
     "pcx_vvor": (c_int, [c_void_p] * 7 + [c_int64] * 4 + [c_int] * 5 + [c_void_p, c_size_t, c_void_p]),
@@ -397,6 +400,7 @@ def _planned_pays(T, n_out, outw, K):
 #    7.3 (15 000)                217 / 291      82 / 83       96 / 43        57 /  78       135
 #   25.4 (15 000)                672 / 350     232 / 95      277 / 49       150 / 100       139
 #
+# (these and below without the scatter kernels behind, which return at once where all operands are finite: 9 us more.)
 # It is chosen where the scatter kernel's fp32 reductions (triplets x width x 4 bytes) are half a gigabyte, so that one
 # pass pays for most of a plan, and the two-part sums stay within 4 GB.  The input gradient of an up-sampling layer 384 ->
 # 128 with 134 triplets a row (18.9 M) took 10.1 ms on the scatter kernel; the training step around it went from 113.0 to
@@ -509,7 +513,7 @@ def _split_supported(weight, gather, seg_offs, n_out, transpose):
     inw, outw = (M, C) if transpose else (C, M)
     if seg_offs is None or weight.dtype != torch.bfloat16 or K <= 1 or K > 512 or n_out <= 0 or not (G > 1 or outw > 256):
         return False
-    if inw != padded_width(inw) or outw != padded_width(outw) or inw > 1024 or G * inw > 2048 or G * ((outw + 255) // 256) > 64:
+    if inw != padded_width(inw) or outw != padded_width(outw) or inw > 1024 or G * inw > 2048 or G * ((inw + 255) // 256) * ((outw + 255) // 256) > 64:
         return False
     return gather.numel() < 2 ** 31 and (int(n_out) + 127) // 128 * K * 128 <= 2 ** 32
 

@@ -112,8 +112,9 @@ int launch_column_sums(const void *x, void *out, int64_t N, int C, float *partia
 // 64-bit remainder for every one of them, 150 000 x 64 took 8.1 us instead of some 5 (a memset of that size: 4.6, and no kernel
 // can be set up behind it).
 template <typename T, int W>
-__global__ void fill_rows_kernel(float *__restrict__ acc, const T *__restrict__ bias, int64_t n, int width) {
+__global__ void fill_rows_kernel(float *__restrict__ acc, const T *__restrict__ bias, int64_t n, int width, OnlyIf only_if) {
     start_after_previous();
+    if (!only_if.holds()) return;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x * W;
     int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * W;
     int c = bias ? (int)(i % width) : 0;
@@ -137,12 +138,12 @@ __global__ void fill_rows_kernel(float *__restrict__ acc, const T *__restrict__ 
 }
 
 template <typename T>
-int launch_fill(float *acc, const void *bias, int64_t rows, int width, cudaStream_t stream) {
+int launch_fill(float *acc, const void *bias, int64_t rows, int width, OnlyIf only_if, cudaStream_t stream) {
     const int64_t n = rows * width;
     const int w = (bias ? width : n) % 4 == 0 && (uintptr_t)acc % 16 == 0 ? 4 : 1;
-    const unsigned grid = (unsigned)std::min<int64_t>((n / w + 255) / 256, (int64_t)num_sms() * 16);
-    if (w == 4) launch_after(fill_rows_kernel<T, 4>, grid, 256, 0, stream, acc, (const T *)bias, n, width);
-    else launch_after(fill_rows_kernel<T, 1>, grid, 256, 0, stream, acc, (const T *)bias, n, width);
+    const unsigned grid = (unsigned)std::min<int64_t>((n / w + 255) / 256, (int64_t)num_sms() * (only_if.words ? 4 : 16));
+    if (w == 4) launch_after(fill_rows_kernel<T, 4>, grid, 256, 0, stream, acc, (const T *)bias, n, width, only_if);
+    else launch_after(fill_rows_kernel<T, 1>, grid, 256, 0, stream, acc, (const T *)bias, n, width, only_if);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
 }
@@ -169,11 +170,11 @@ __global__ void reshape16_kernel(const uint16_t *__restrict__ src, uint16_t *__r
 
 // Every row of the accumulator starts as `bias` (zeros when null): the bias of a layer costs the store
 // that clearing the accumulator costs anyway, not a pass over its output.
-int clear_accumulator(float *acc, const void *bias, int64_t rows, int width, int dtype, cudaStream_t stream) {
+int clear_accumulator(float *acc, const void *bias, int64_t rows, int width, int dtype, cudaStream_t stream, OnlyIf only_if) {
     switch (dtype) {
-        case PCX_F32: return launch_fill<float>(acc, bias, rows, width, stream);
-        case PCX_F16: return launch_fill<__half>(acc, bias, rows, width, stream);
-        case PCX_BF16: return launch_fill<__nv_bfloat16>(acc, bias, rows, width, stream);
+        case PCX_F32: return launch_fill<float>(acc, bias, rows, width, only_if, stream);
+        case PCX_F16: return launch_fill<__half>(acc, bias, rows, width, only_if, stream);
+        case PCX_BF16: return launch_fill<__nv_bfloat16>(acc, bias, rows, width, only_if, stream);
     }
     PCX_FAIL(PCX_E_DTYPE, "unsupported dtype %d", dtype);
 }

@@ -62,6 +62,19 @@ void launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
     (void)cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);   // PCX_LAUNCH_CHECK asks for the error
 }
 
+// What a kernel is launched for only if an earlier one found a reason: a word from each of that one's blocks, zero where it
+// found none.  No words: always.  Asked by a whole block.
+struct OnlyIf {
+    const uint32_t *words = nullptr;
+    int n = 0;
+    __device__ __forceinline__ bool holds() const {
+        if (!words) return true;
+        bool any = false;
+        for (int t = threadIdx.x; t < n; t += blockDim.x) any |= words[t] != 0;
+        return __syncthreads_or(any);
+    }
+};
+
 static inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 // Bump allocator over a caller-owned workspace; every block 256-byte aligned.

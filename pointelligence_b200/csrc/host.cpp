@@ -143,9 +143,12 @@ constexpr int64_t NO_PLAN = 0x200;   // internal flag of an engine: the automati
 // Shapes the automatic choice may give to the output-stationary kernel.  It rounds the sums of (row, tap) buckets to 16
 // bits; grouped, padded and wider layers multiply their operands as they are unless the caller asks for that kernel.
 bool plan_unasked(int64_t K, int64_t G, int64_t outw) { return K > 1 && G == 1 && outw <= 256; }
-// ... and those it may be given with the sums in two parts (bf16: as exact as the scatter kernels; in fp16 a sum could
-// leave the type's range, which the scatter kernels' products do not).
-bool plan_split(at::ScalarType dtype, int64_t K, int64_t G, int64_t outw) { return K > 1 && (G > 1 || outw > 256) && dtype == at::kBFloat16; }
+// ... and those it may be given with the sums in two parts (bf16: as exact as the scatter kernels once a row is rounded; in
+// fp16 a sum could leave the type's range, which the scatter kernels' products do not).  The scatter kernels have to take
+// them too: they follow where an operand is not finite.
+bool plan_split(at::ScalarType dtype, int64_t K, int64_t G, int64_t inw, int64_t outw) {
+    return K > 1 && (G > 1 || outw > 256) && dtype == at::kBFloat16 && G * ((inw + 255) / 256) * ((outw + 255) / 256) <= 64;
+}
 constexpr int SPLIT_SUMS = PCX_MVMR_SPLIT_SUMS;
 
 Tensor mvmr_planned(const Tensor &weight, const Tensor &feat, const Plan &plan, int64_t T, int64_t n_out, int flags,
@@ -159,6 +162,19 @@ Tensor mvmr_planned(const Tensor &weight, const Tensor &feat, const Plan &plan, 
     check(pcx_mvmr_planned_bias(ptr(weight), ptr(feat), ptr(plan.buffer), plan.buffer.numel(), ptr(bias), ptr(out), T, feat.size(0),
                                 n_out, (int)K, (int)G, (int)C, (int)M, flags, dtype_code(feat.scalar_type()), (int)plan.group, plan.multi,
                                 ptr(ws), ws.numel(), stream()));
+    return out;
+}
+
+Tensor mvmr_split(const Tensor &weight, const Tensor &feat, const Tensor &gather_, const Tensor &scatter_, const Tensor &seg_,
+                  const Plan &plan, int64_t n_out, int flags, const Tensor &bias) {
+    const int64_t K = weight.size(0), G = weight.size(1), C = weight.size(2), M = weight.size(3);
+    const int transpose = flags & 1;
+    const Tensor gather = as_i32(gather_), scatter = as_i32(scatter_), seg = as_i64(seg_);
+    Tensor out = at::empty({n_out, G * (transpose ? C : M)}, feat.options());
+    Tensor ws = workspace(pcx_mvmr_split_workspace_bytes(plan.multi, n_out, (int)K, (int)G, (int)C, (int)M, transpose), feat);
+    check(pcx_mvmr_split(ptr(weight), ptr(feat), ptr_as<int32_t>(gather), ptr_as<int32_t>(scatter), ptr_as<int64_t>(seg), ptr(plan.buffer),
+                         plan.buffer.numel(), ptr(bias), ptr(out), gather.numel(), feat.size(0), n_out, (int)K, (int)G, (int)C, (int)M,
+                         flags, (int)plan.group, plan.multi, ptr(ws), ws.numel(), stream()));
     return out;
 }
 
@@ -200,10 +216,11 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
                   "channels a group");
         }
         const bool aligned = ((uintptr_t)ptr(weight) | (uintptr_t)ptr(feat)) % 16 == 0;   // else the CUDA-core engine
-        const bool forced = engine == ENGINE_PLANNED, split = !forced && plan_split(feat.scalar_type(), K, G, outw);
+        const bool forced = engine == ENGINE_PLANNED, split = !forced && plan_split(feat.scalar_type(), K, G, inw, outw);
         if (fits && (forced || (aligned && (split || plan_unasked(K, G, outw))))) {
             const Plan plan = ask_plan(scatter_, gather_, *seg_, K, n_out, G * outw, G * inw, forced, split);
-            if (plan.valid) return mvmr_planned(weight, feat, plan, T, n_out, flags | (split ? SPLIT_SUMS : 0), bias);
+            if (plan.valid && split) return mvmr_split(weight, feat, gather_, scatter_, *seg_, plan, n_out, flags, bias);
+            if (plan.valid) return mvmr_planned(weight, feat, plan, T, n_out, flags, bias);
         }
         engine = 0;
     }

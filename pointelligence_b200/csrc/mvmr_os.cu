@@ -371,6 +371,22 @@ __device__ __forceinline__ void add(uint4 p, float *s) {
     }
 }
 
+// whether one of a word's two numbers is infinite or no number
+template <int FMT>
+__device__ __forceinline__ bool not_finite(uint32_t w) {
+    constexpr uint32_t EXP = FMT ? 0x7f80u : 0x7c00u;   // all ones
+    return (w & EXP) == EXP || (w & EXP << 16) == EXP << 16;
+}
+
+// a + 0 w, two numbers each: stays what it is while the numbers of w are finite, then no number
+template <int FMT>
+__device__ __forceinline__ uint32_t times_zero(uint32_t w, uint32_t a) {
+    uint32_t r;
+    if (FMT) asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(0u), "r"(a));
+    else asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(w), "r"(0u), "r"(a));
+    return r;
+}
+
 constexpr int BUCKET_SUM_THREADS = 256, BUCKET_SUM_WARPS = BUCKET_SUM_THREADS / 32, BUCKET_SUM_CTAS = 4;
 
 // LANES: threads of a bucket.  A warp fetches the descriptors and the first four rows of up to 32 consecutive buckets at
@@ -383,15 +399,31 @@ constexpr int BUCKET_SUM_THREADS = 256, BUCKET_SUM_WARPS = BUCKET_SUM_THREADS / 
 // 200k points, 22 triplets a row: 32 channels 50 -> 44 us, 64 88 -> 70, 96 141 -> 106, 128 160 -> 113, 192 245 -> 197,
 // 256 305 -> 250, 512 647 -> 517.  Slower: 5 and 6 CTAs an SM (spills), the next bucket's rows fetched early at 3 CTAs
 // (368), several pieces a thread (550 - 1090).
+//
+// SPLIT: what rounding a sum to `hi` left over goes behind it.  With `odd` given, sums that are not finite, and weights that
+// are not (16-byte pieces of them, looked at in passing), are reported in odd[block] and the caller does all of it again;
+// without, zero goes behind such sums (infinity less infinity is no number).
 template <int FMT, int LANES, bool SPLIT>
 __global__ void __launch_bounds__(BUCKET_SUM_THREADS, BUCKET_SUM_CTAS) bucket_sum_kernel(const uint16_t *__restrict__ feat,
                                                                                          const uint2 *__restrict__ entries,
                                                                                          const uint2 *__restrict__ buckets,
                                                                                          const uint32_t *__restrict__ ctrl, int inw,
-                                                                                         uint16_t *__restrict__ scratch) {
+                                                                                         int most, uint16_t *__restrict__ scratch,
+                                                                                         const uint4 *__restrict__ weight,
+                                                                                         int64_t weight_pieces, uint32_t *odd) {
     start_after_previous();
+    bool seen = false;   // something that is not finite
+    uint32_t rest = 0;   // two zeros until what a rounding left over is not finite
+    if (SPLIT && odd) {
+        const int64_t threads = (int64_t)gridDim.x * gridDim.y * BUCKET_SUM_THREADS;
+        const int64_t first = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * BUCKET_SUM_THREADS + threadIdx.x;
+        for (int64_t t = first; t < weight_pieces; t += threads) {
+            const uint4 v = __ldg(weight + t);
+            seen |= not_finite<FMT>(v.x) || not_finite<FMT>(v.y) || not_finite<FMT>(v.z) || not_finite<FMT>(v.w);
+        }
+    }
     constexpr int AT_ONCE = 32 / LANES;
-    const int lane = threadIdx.x & 31, sub = lane / LANES, nmulti = (int)ctrl[CTRL_NMULTI];
+    const int lane = threadIdx.x & 31, sub = lane / LANES, nmulti = min((int)ctrl[CTRL_NMULTI], most);   // never beyond the scratch
     const unsigned piece = blockIdx.y * LANES + lane % LANES, pitch = (unsigned)inw * 2u;
     const bool piece_ok = piece * 16 < pitch;   // a lane without a piece takes part in the shuffles
     const char *col = reinterpret_cast<const char *>(feat) + (piece_ok ? piece * 16 : 0);
@@ -434,17 +466,30 @@ __global__ void __launch_bounds__(BUCKET_SUM_THREADS, BUCKET_SUM_CTAS) bucket_su
             if (SPLIT) {   // ... and behind it what the rounding left over
                 float hi[8];
                 widen<FMT>(o, hi);
-                o.x = pack2(s[0] - hi[0], s[1] - hi[1], FMT), o.y = pack2(s[2] - hi[2], s[3] - hi[3], FMT);
-                o.z = pack2(s[4] - hi[4], s[5] - hi[5], FMT), o.w = pack2(s[6] - hi[6], s[7] - hi[7], FMT);
-                if (store) __stcs(reinterpret_cast<uint4 *>(reinterpret_cast<char *>(at) + pitch), o);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) s[e] -= hi[e];   // no number or infinite where hi is not finite
+                if (!odd) {
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) s[e] = fabsf(s[e]) < INFINITY ? s[e] : 0.f;
+                }
+                o.x = pack2(s[0], s[1], FMT), o.y = pack2(s[2], s[3], FMT);
+                o.z = pack2(s[4], s[5], FMT), o.w = pack2(s[6], s[7], FMT);
+                if (store) {
+                    __stcs(reinterpret_cast<uint4 *>(reinterpret_cast<char *>(at) + pitch), o);
+                    rest = times_zero<FMT>(o.x, times_zero<FMT>(o.y, times_zero<FMT>(o.z, times_zero<FMT>(o.w, rest))));
+                }
             }
         }
+    }
+    if (SPLIT && odd) {
+        const int any = __syncthreads_or(seen || (rest & 0x7fff7fffu));
+        if (threadIdx.x == 0) odd[blockIdx.y * gridDim.x + blockIdx.x] = (uint32_t)any;
     }
 }
 
 template <int FMT, bool SPLIT>
-void launch_bucket_sum(int64_t multi, int inw, const uint16_t *feat, const uint2 *entries, const uint2 *buckets,
-                       const uint32_t *ctrl, uint16_t *scratch, cudaStream_t stream) {
+int launch_bucket_sum(int64_t multi, int inw, const uint16_t *feat, const uint2 *entries, const uint2 *buckets,
+                       const uint32_t *ctrl, uint16_t *scratch, const uint4 *weight, int64_t weight_pieces, uint32_t *odd, cudaStream_t stream) {
     // Up to 128 channels the next power of two of lanes, beyond that slices (blockIdx.y) of 32, 16 or 8 lanes, whichever
     // idles least: 192 channels 197 us in slices of 8 (223 of 32), 384 386 of 16 (444 of 8, 429 of 32), 256 255 of 32
     // (245 of 16, 268 of 8), 208 241 of 32 (249 of 16).  Below: 48 channels 63 us in 8 lanes (80 in slices of 2).
@@ -457,8 +502,9 @@ void launch_bucket_sum(int64_t multi, int inw, const uint16_t *feat, const uint2
             if ((ppr + l - 1) / l * l < (ppr + lanes - 1) / lanes * lanes) lanes = l;
     }
     const int slices = (ppr + lanes - 1) / lanes, at_once = BUCKET_SUM_THREADS / lanes;
-    const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>((multi + at_once - 1) / at_once, num_sms() * BUCKET_SUM_CTAS / slices)), (unsigned)slices);
-#define PCX_BS(L) launch_after(bucket_sum_kernel<FMT, L, SPLIT>, grid, BUCKET_SUM_THREADS, 0, stream, feat, entries, buckets, ctrl, inw, scratch)
+    const int64_t work = std::max((multi + at_once - 1) / at_once, odd ? (weight_pieces + BUCKET_SUM_THREADS - 1) / BUCKET_SUM_THREADS : 0);
+    const dim3 grid((unsigned)std::max<int64_t>(1, std::min<int64_t>(work, std::min(num_sms() * BUCKET_SUM_CTAS, MAX_ODD) / slices)), (unsigned)slices);
+#define PCX_BS(L) launch_after(bucket_sum_kernel<FMT, L, SPLIT>, grid, BUCKET_SUM_THREADS, 0, stream, feat, entries, buckets, ctrl, inw, (int)multi, scratch, weight, weight_pieces, odd)
     switch (lanes) {
         case 2: PCX_BS(2); break;
         case 4: PCX_BS(4); break;
@@ -467,6 +513,7 @@ void launch_bucket_sum(int64_t multi, int inw, const uint16_t *feat, const uint2
         default: PCX_BS(32); break;
     }
 #undef PCX_BS
+    return (int)(grid.x * grid.y);
 }
 
 // cost of a group = its non-empty tiles (each is one A tile to copy and multiply); the tap sets of its blocks
@@ -1190,7 +1237,28 @@ int pcx_mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan, siz
 
 int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan, size_t plan_bytes, const void *d_bias, void *d_out,
                           int64_t T, int64_t n_feat, int64_t n_out, int K, int groups, int C, int M, int flags, int dtype,
-                          int group_blocks, int64_t multi_buckets, void *d_ws, size_t ws_bytes, void *stream_) {
+                          int group_blocks, int64_t multi_buckets, void *d_ws, size_t ws_bytes, void *stream) {
+    return mvmr_planned(d_weight, d_feat, d_plan, plan_bytes, d_bias, d_out, T, n_feat, n_out, K, groups, C, M, flags, dtype, group_blocks,
+                        multi_buckets, nullptr, nullptr, d_ws, ws_bytes, stream);
+}
+
+int pcx_debug_wait_runs_out(unsigned long long limit_ns, void *stream_) {
+    cudaStream_t stream = (cudaStream_t)stream_;
+    if (limit_ns == 0 || limit_ns > 100000000ull) PCX_FAIL(PCX_E_ARG, "pcx_debug_wait_runs_out: limit must be within (0, 100 ms]");
+    unsigned int *status = status_word();
+    if (!status) PCX_FAIL(PCX_E_LAUNCH, "pcx_debug_wait_runs_out: no device status word");
+    wait_runs_out_kernel<<<1, 32, 0, stream>>>(status, 8u, (uint64_t)limit_ns);
+    PCX_LAUNCH_CHECK();
+    return PCX_OK;
+}
+
+}  // extern "C"
+
+// The call itself.  odd: null, or room for MAX_ODD words, of which the first *n_odd say afterwards (zero or not) whether a
+// split sum or a weight was not finite.
+int pcx::mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan, size_t plan_bytes, const void *d_bias, void *d_out, int64_t T,
+                      int64_t n_feat, int64_t n_out, int K, int groups, int C, int M, int flags, int dtype, int group_blocks,
+                      int64_t multi_buckets, uint32_t *odd, int *n_odd, void *d_ws, size_t ws_bytes, void *stream_) {
     const int transpose = flags & PCX_MVMR_TRANSPOSE;
     const bool split_sums = (flags & PCX_MVMR_SPLIT_SUMS) != 0;
     cudaStream_t stream = (cudaStream_t)stream_;
@@ -1279,10 +1347,12 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
         most = (int)smem;
     }
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(pv.ngroups * p.nsplit * nparts, num_sms()));
-    if (multi_buckets > 0) {
+    if (multi_buckets > 0 || odd) {   // (with no sums it looks at the weights alone)
         prof_begin("bucket_sum_kernel", stream);
         auto sum = split_sums ? (p.fmt ? launch_bucket_sum<1, true> : launch_bucket_sum<0, true>) : (p.fmt ? launch_bucket_sum<1, false> : launch_bucket_sum<0, false>);
-        sum(multi_buckets, p.in_pitch, p.feat, pv.entries, pv.buckets, pv.ctrl, (uint16_t *)d_ws, stream);
+        const int blocks = sum(multi_buckets, p.in_pitch, p.feat, pv.entries, pv.buckets, pv.ctrl, (uint16_t *)d_ws, (const uint4 *)d_weight,
+                               (int64_t)K * groups * C * M / 8, odd, stream);
+        if (odd) *n_odd = blocks;
         prof_end(stream);
         PCX_LAUNCH_CHECK();
     }
@@ -1298,15 +1368,3 @@ int pcx_mvmr_planned_bias(const void *d_weight, const void *d_feat, void *d_plan
     }
     return PCX_OK;
 }
-
-int pcx_debug_wait_runs_out(unsigned long long limit_ns, void *stream_) {
-    cudaStream_t stream = (cudaStream_t)stream_;
-    if (limit_ns == 0 || limit_ns > 100000000ull) PCX_FAIL(PCX_E_ARG, "pcx_debug_wait_runs_out: limit must be within (0, 100 ms]");
-    unsigned int *status = status_word();
-    if (!status) PCX_FAIL(PCX_E_LAUNCH, "pcx_debug_wait_runs_out: no device status word");
-    wait_runs_out_kernel<<<1, 32, 0, stream>>>(status, 8u, (uint64_t)limit_ns);
-    PCX_LAUNCH_CHECK();
-    return PCX_OK;
-}
-
-}  // extern "C"

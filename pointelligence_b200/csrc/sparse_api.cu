@@ -130,6 +130,49 @@ int pcx_mvmr_bias(const void *d_weight, const void *d_feat, const int32_t *d_gat
     return PCX_OK;
 }
 
+// Words that say whether the scatter kernels have to do it all again, and room for one of the two at a time.
+constexpr size_t SPLIT_HEAD = MAX_ODD * sizeof(uint32_t);
+
+size_t pcx_mvmr_split_workspace_bytes(int64_t multi_buckets, int64_t n_out, int K, int G, int C, int M, int transpose) {
+    const size_t scatter = pcx_mvmr_workspace_bytes(n_out, K, G, C, M, transpose, PCX_BF16);
+    const int inw = transpose ? M : C, outw = transpose ? C : M;
+    if (scatter == 0 || inw > 1024) return 0;
+    const size_t planned = pcx_mvmr_planned_scratch_bytes(multi_buckets, 2 * inw, n_out, outw, K, G);
+    return planned ? SPLIT_HEAD + std::max(planned, scatter) : 0;
+}
+
+int pcx_mvmr_split(const void *d_weight, const void *d_feat, const int32_t *d_gather, const int32_t *d_scatter,
+                   const int64_t *d_seg_offs, void *d_plan, size_t plan_bytes, const void *d_bias, void *d_out, int64_t T,
+                   int64_t n_feat, int64_t n_out, int K, int G, int C, int M, int flags, int group_blocks, int64_t multi_buckets,
+                   void *d_ws, size_t ws_bytes, void *stream_) {
+    cudaStream_t stream = (cudaStream_t)stream_;
+    const int transpose = flags & PCX_MVMR_TRANSPOSE;
+    const size_t need = pcx_mvmr_split_workspace_bytes(multi_buckets, n_out, K, G, C, M, transpose);
+    if (need == 0) PCX_FAIL(PCX_E_ARG, "pcx_mvmr_split: sizes out of range");
+    if (!d_gather || !d_scatter || !d_seg_offs || !d_ws) PCX_FAIL(PCX_E_ARG, "pcx_mvmr_split: null pointer");
+    if ((uintptr_t)d_ws % 256) PCX_FAIL(PCX_E_ALIGN, "pcx_mvmr_split: workspace must be 256-byte aligned");
+    if (ws_bytes < need) PCX_FAIL(PCX_E_CAPACITY, "pcx_mvmr_split: workspace %zu < %zu bytes", ws_bytes, need);
+    uint32_t *odd = (uint32_t *)d_ws;
+    void *ws = (char *)d_ws + SPLIT_HEAD;
+    MvmrWs w;
+    carve_mvmr(ws, n_out, K, G, C, M, transpose, PCX_BF16, &w);
+    MvmrArgs a = {};
+    a.weight = d_weight, a.feat = d_feat, a.gather = d_gather, a.scatter = d_scatter, a.seg_offs = d_seg_offs;
+    a.acc = w.acc, a.chunk_table = w.chunk_table;
+    a.T = T, a.n_feat = n_feat, a.n_out = n_out;
+    a.K = K, a.G = G, a.C = C, a.M = M, a.transpose = transpose ? 1 : 0, a.dtype = PCX_BF16;
+    a.bias = d_bias, a.reverse = (flags & PCX_MVMR_REVERSE_TAPS) ? 1 : 0;
+    if (!mvmr_tensor_supported(a)) PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_split: not a call of the tensor engine of pcx_mvmr");
+    if (int rc = mvmr_planned(d_weight, d_feat, d_plan, plan_bytes, d_bias, d_out, T, n_feat, n_out, K, G, C, M, flags | PCX_MVMR_SPLIT_SUMS, PCX_BF16,
+                              group_blocks, multi_buckets, odd, &a.only_if.n, ws, ws_bytes - SPLIT_HEAD, stream_))
+        return rc;
+    a.only_if.words = odd;
+    const int width = G * (transpose ? C : M);
+    if (int rc = clear_accumulator(a.acc, d_bias, n_out, width, PCX_BF16, stream, a.only_if)) return rc;
+    if (int rc = mvmr_tensor(a, stream)) return rc;
+    return round_accumulator(a.acc, d_out, n_out * width, PCX_BF16, stream, a.only_if);
+}
+
 size_t pcx_vvor_workspace_bytes(int64_t n_o, int G, int Ma, int Cb, int dtype) {
     if (n_o < 0 || G <= 0 || Ma <= 0 || Cb <= 0) return 0;
     uint64_t checked = 0;

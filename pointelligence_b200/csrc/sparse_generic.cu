@@ -85,17 +85,19 @@ __global__ void vvor_unsorted_kernel(const T *__restrict__ A, const int32_t *__r
 }
 
 template <typename T>
-__global__ void round_kernel(const float *__restrict__ acc, T *__restrict__ out, int64_t n) {
+__global__ void round_kernel(const float *__restrict__ acc, T *__restrict__ out, int64_t n, OnlyIf only_if) {
     start_after_previous();
-    int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * 4;
-    if (i + 3 < n) {
-        float4 v = *reinterpret_cast<const float4 *>(acc + i);
-        out[i] = from_f32<T>(v.x);
-        out[i + 1] = from_f32<T>(v.y);
-        out[i + 2] = from_f32<T>(v.z);
-        out[i + 3] = from_f32<T>(v.w);
-    } else {
-        for (; i < n; ++i) out[i] = from_f32<T>(acc[i]);
+    if (!only_if.holds()) return;
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * 4; i < n; i += (int64_t)gridDim.x * blockDim.x * 4) {
+        if (i + 3 < n) {
+            float4 v = *reinterpret_cast<const float4 *>(acc + i);
+            out[i] = from_f32<T>(v.x);
+            out[i + 1] = from_f32<T>(v.y);
+            out[i + 2] = from_f32<T>(v.z);
+            out[i + 3] = from_f32<T>(v.w);
+        } else {
+            for (int64_t e = i; e < n; ++e) out[e] = from_f32<T>(acc[e]);
+        }
     }
 }
 
@@ -148,11 +150,12 @@ int vvor_generic(const VvorArgs &a, cudaStream_t stream) {
     PCX_FAIL(PCX_E_DTYPE, "unsupported dtype %d", a.dtype);
 }
 
-int round_accumulator(const float *acc, void *out, int64_t n, int dtype, cudaStream_t stream) {
+int round_accumulator(const float *acc, void *out, int64_t n, int dtype, cudaStream_t stream, OnlyIf only_if) {
     if (n == 0) return PCX_OK;
     unsigned blocks = (unsigned)((n / 4 + 255) / 256 + 1);
-    if (dtype == PCX_F16) launch_after(round_kernel<__half>, blocks, 256, 0, stream, acc, (__half *)out, n);
-    else if (dtype == PCX_BF16) launch_after(round_kernel<__nv_bfloat16>, blocks, 256, 0, stream, acc, (__nv_bfloat16 *)out, n);
+    if (only_if.words) blocks = std::min(blocks, (unsigned)num_sms() * 4);   // mostly there is nothing to do
+    if (dtype == PCX_F16) launch_after(round_kernel<__half>, blocks, 256, 0, stream, acc, (__half *)out, n, only_if);
+    else if (dtype == PCX_BF16) launch_after(round_kernel<__nv_bfloat16>, blocks, 256, 0, stream, acc, (__nv_bfloat16 *)out, n, only_if);
     else PCX_FAIL(PCX_E_DTYPE, "round_accumulator: dtype %d", dtype);
     PCX_LAUNCH_CHECK();
     return PCX_OK;

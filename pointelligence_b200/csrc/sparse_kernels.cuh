@@ -18,6 +18,7 @@ struct MvmrArgs {
     const void *bias;        // (G*outw) of dtype or null; only the fan-in 1 stores read it, elsewhere acc starts as it
     int K, G, C, M, transpose, dtype;
     int reverse;             // tap k uses weight K-1-k
+    OnlyIf only_if;          // (tensor engine)
 };
 
 struct VvorArgs {
@@ -104,8 +105,12 @@ int mvmr_sorted_fma(const MvmrArgs &a, cudaStream_t stream);   // CUDA cores, ta
 int vvor_sorted_fma(const VvorArgs &a, cudaStream_t stream);
 int mvmr_generic(const MvmrArgs &a, cudaStream_t stream);
 int vvor_generic(const VvorArgs &a, cudaStream_t stream);
-int clear_accumulator(float *acc, const void *bias, int64_t rows, int width, int dtype, cudaStream_t stream);
-int round_accumulator(const float *acc, void *out, int64_t n, int dtype, cudaStream_t stream);
+int clear_accumulator(float *acc, const void *bias, int64_t rows, int width, int dtype, cudaStream_t stream, OnlyIf only_if = {});
+int round_accumulator(const float *acc, void *out, int64_t n, int dtype, cudaStream_t stream, OnlyIf only_if = {});
+constexpr int MAX_ODD = 1024;
+int mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan, size_t plan_bytes, const void *d_bias, void *d_out, int64_t T,
+                 int64_t n_feat, int64_t n_out, int K, int groups, int C, int M, int flags, int dtype, int group_blocks,
+                 int64_t multi_buckets, uint32_t *odd, int *n_odd, void *d_ws, size_t ws_bytes, void *stream);   // (mvmr_os.cu)
 
 // Rows wider than 256 channels go through the tensor engines in equal parts of at most 256.
 inline int parts_of(int width) { return (width + 255) / 256; }

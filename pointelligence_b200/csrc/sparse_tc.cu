@@ -115,6 +115,7 @@ struct MvmrTcParams {
     uint16_t *out;           // MODE 2: the output rows themselves (every row occurs in exactly one triplet)
     const uint16_t *bias;    // MODE 2: added before the rounding (null: none); the other modes start from it
     int reverse;             // tap k uses weight K-1-k
+    OnlyIf only_if;
     int64_t in_pitch, out_pitch, w_pitch, w_tap;   // rows of features / output / one tap's weight, elements of one tap's weight
     int out_parts, in_parts, chain;                // C, M below: the part's; contraction parts a block takes
     int K, C, M, transpose, fmt, nbuf, slab;  // slab: columns parked per bulk reduction (32 or 64)
@@ -137,6 +138,7 @@ struct MvmrTcParams {
 template <int MODE, int NT, bool CHAINED>
 __global__ void __launch_bounds__(NT, NT == 256 ? 1 : 0) mvmr_tc_kernel(MvmrTcParams p) {
     start_after_previous();
+    if (!p.only_if.holds()) return;
     constexpr bool BULK = MODE == 1;
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t s_bar;
@@ -466,7 +468,7 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
     const int64_t upper = a.T / CH + a.K + 1;   // tiles of triplets, at most
     p.weight = (const uint16_t *)a.weight, p.feat = (const uint16_t *)a.feat;
     p.gather = a.gather, p.scatter = a.scatter, p.seg = a.seg_offs, p.acc = a.acc;
-    p.out = (uint16_t *)a.out_rows, p.bias = (const uint16_t *)a.bias, p.reverse = a.reverse;
+    p.out = (uint16_t *)a.out_rows, p.bias = (const uint16_t *)a.bias, p.reverse = a.reverse, p.only_if = a.only_if;
     p.K = a.K, p.C = C, p.M = M, p.transpose = a.transpose, p.fmt = a.dtype == PCX_BF16 ? 1 : 0;
     p.ncols = p.acc_cols = pow2_cols((outw + 63) / 64 * 64);  // the epilogue reads blocks of up to 64 columns
     // Measured on B200: rows of exactly 64 floats leave fastest through one bulk reduction
@@ -526,10 +528,11 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
     const int regs = kernel_registers(kernel, &regs_mvmr[mode]);
     const int occ = ctas_per_sm(smem + static_smem, p.ncols, regs, threads);
     const dim3 grid((unsigned)std::min<int64_t>(upper, std::max<int64_t>(1, (int64_t)occ * num_sms() / parts)), (unsigned)parts);
-    prof_begin(store ? (a.transpose ? "mvmr_tc_kernel(dgrad, store)" : "mvmr_tc_kernel(fwd, store)")
-                     : (a.transpose ? "mvmr_tc_kernel(dgrad)" : "mvmr_tc_kernel(fwd)"), stream);
+    if (!a.only_if.words)
+        prof_begin(store ? (a.transpose ? "mvmr_tc_kernel(dgrad, store)" : "mvmr_tc_kernel(fwd, store)")
+                         : (a.transpose ? "mvmr_tc_kernel(dgrad)" : "mvmr_tc_kernel(fwd)"), stream);
     launch_after(kernel, grid, threads, smem, stream, p);
-    prof_end(stream);
+    if (!a.only_if.words) prof_end(stream);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
 }

@@ -1,0 +1,91 @@
+"""GPU tests of what wide and grouped bf16 layers get by way of a plan: bucket sums in two parts and, where an operand is not
+finite, the scatter kernels over the same output (``pcx_mvmr_split``)."""
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _rulebook(seed, n_in, n_out, K, T, distinct=False):
+    """Tap-sorted triplets; ``distinct``: no (row, tap) pair twice, so that no sums are taken."""
+    rng = np.random.default_rng(seed)
+    if distinct:
+        pair = rng.permutation(n_out * K)[:T]
+        i, k = pair // K, pair % K
+    else:
+        i, k = rng.integers(0, n_out, T), rng.integers(0, K, T)
+        k[rng.random(T) < 0.5] = K // 2
+    j = rng.integers(0, n_in, T)
+    order = np.lexsort((i, k))
+    i, j, k = i[order].astype(np.int32), j[order].astype(np.int32), k[order]
+    seg = np.searchsorted(k, np.arange(K + 1)).astype(np.int64)
+    return tuple(torch.from_numpy(a).to(DEV) for a in (i, j, seg))
+
+
+@pytest.fixture
+def always(monkeypatch):
+    """Every wide or grouped bf16 layer takes the plan, whatever its size."""
+    from pointelligence_b200 import _cabi
+
+    monkeypatch.setattr(_cabi, "_planned_pays", lambda *a: True)
+    monkeypatch.setattr(_cabi, "_split_pays", lambda *a: True)
+    return _cabi
+
+
+def _kernels(cabi, fn):
+    cabi.profile_enable(True)
+    try:
+        out = fn()
+        torch.cuda.synchronize()
+        return out, [name for name, _ in cabi.profile_records()]
+    finally:
+        cabi.profile_enable(False)
+
+
+@pytest.mark.parametrize("K,G,C,M,transpose", [(27, 1, 64, 288, False), (27, 1, 288, 64, True), (27, 2, 32, 48, False), (8, 4, 16, 16, True)])
+@pytest.mark.parametrize("what", ["feature inf", "feature -inf and inf", "feature nan", "weight inf", "weight nan", "sum beyond bf16",
+                                  "weight inf, no sums"])
+def test_operands_that_are_not_finite(always, what, K, G, C, M, transpose):
+    """Infinities and NaN are exactly where the scatter kernels put them; all else is as close as ever."""
+    n_in, n_out = 300, 700
+    distinct = what.endswith("no sums")
+    i, j, seg = _rulebook(C + M, n_in, n_out, K, 4000 if distinct else 14000, distinct)
+    inw = M if transpose else C
+    g = torch.Generator(device=DEV).manual_seed(1)
+    w = torch.rand(K, G, C, M, device=DEV, generator=g).bfloat16() / 8    # of one sign: an infinity stays one
+    x = torch.rand(n_in, G * inw, device=DEV, generator=g).bfloat16()
+    if what == "feature inf":
+        x[17, 3] = float("inf")
+    elif what == "feature -inf and inf":
+        x[17, 3], x[18, 3], x[19, 5] = float("inf"), -float("inf"), -float("inf")
+    elif what == "feature nan":
+        x[17, 3] = float("nan")
+    elif what == "sum beyond bf16":
+        x.fill_(3e38)
+        w *= 1e-4
+    else:
+        w[1, 0, 3, 7] = float("nan") if what == "weight nan" else float("inf")
+    out, names = _kernels(always, lambda: always.mvmr(w, x, j, i, seg, None, n_out, transpose))
+    assert [n for n in names if n != "bucket_sum_kernel"] == [f"mvmr_os_kernel({'dgrad' if transpose else 'fwd'})"]
+    want = always.mvmr(w, x, j, i, seg, None, n_out, transpose, always.ENGINE_TENSOR)
+    finite = torch.isfinite(want)
+    assert torch.equal(torch.isnan(out), torch.isnan(want))
+    assert torch.equal(out[torch.isinf(want)], want[torch.isinf(want)]) and torch.equal(finite, torch.isfinite(out))
+    if what == "sum beyond bf16":
+        assert bool(finite.all())
+    else:
+        assert not bool(finite.all()) and bool(finite.all(1).any())    # rows that do not meet it stay whole
+    # as the scatter kernels' sums, in another order: the one rounding may fall to the other side (2^-7 of a value of one sign)
+    assert bool(((out - want).abs() <= 2.0 ** -7 * want.abs())[finite].all())
+    assert always.device_status() == 0
+
+
+def test_finite_operands_are_not_done_again(always):
+    """What follows the output-stationary kernel leaves its rows alone: they are those of the kernel by itself."""
+    i, j, seg = _rulebook(3, 500, 900, 27, 20000)
+    w = (torch.randn(27, 2, 48, 64, device=DEV) / 7).bfloat16()
+    x = torch.randn(500, 96, device=DEV).bfloat16()
+    plan = always.mvmr_plan(i, j, seg, 27, 900, always.plan_group_blocks(128))
+    assert torch.equal(always.mvmr(w, x, j, i, seg, None, 900, False), always.mvmr_planned(w, x, plan, False, True))
