@@ -649,20 +649,20 @@ def mvmr(weight, feat, gather, scatter, seg_offs, tap_idx, n_out, transpose, eng
     return host().mvmr(weight, feat, gather, scatter, seg_offs, tap_idx, int(n_out), bool(transpose), int(engine))
 
 
-def _plan_hook(scatter, gather, seg_offs, K, n_out, outw, inw, forced, split=False):
+def _plan_hook(scatter, gather, seg_offs, K, n_out, outw, inw, forced, split=False, capturing=False):
     """Asked by the host path for every pass the output-stationary kernel could take: the plan to run
     (buffer, blocks per group, multi-triplet buckets) or None for the scatter engine."""
     T, blocks = gather.numel(), plan_group_blocks(outw)
     if not forced and not _planned_pays(T, n_out, outw, K):
         return None
-    plan = _remembered_plan(_plan_key(scatter, gather, seg_offs, K, n_out, blocks), scatter, gather, seg_offs)
-    if split and not _split_pays(T, n_out, outw, inw, K):
+    # Wide and grouped layers are captured on the scatter kernels, whether or not a plan exists: these read the caller's
+    # tensors alone, so that a replay follows what is written into them.
+    if split and (capturing or not _split_pays(T, n_out, outw, inw, K)):
         return None
+    plan = _remembered_plan(_plan_key(scatter, gather, seg_offs, K, n_out, blocks), scatter, gather, seg_offs)
     if plan is None:
         if not forced and (scatter.is_inference() or gather.is_inference() or seg_offs.is_inference()):
             return None    # (a plan of inference tensors cannot be remembered, and one per pass does not pay)
-        if split and torch.cuda.is_current_stream_capturing():
-            return None    # building it may wait for the device: the scatter kernels can be captured as they are
         plan = cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, blocks)
     return plan.buffer, plan.group_blocks, plan.multi_buckets
 

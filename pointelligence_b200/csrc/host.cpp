@@ -24,7 +24,7 @@ using OptTensor = std::optional<Tensor>;
 namespace {
 
 // ------------------------------------------------------------------ helpers ----
-PyObject *g_plan_hook = nullptr;       // (scatter, gather, seg, K, n_out, out_width, in_width, forced, split) -> None | plan tuple
+PyObject *g_plan_hook = nullptr;       // (scatter, gather, seg, K, n_out, out_width, in_width, forced, split, capturing) -> None | plan tuple
 PyObject *g_symmetric_hook = nullptr;  // (i, j, K) -> bool
 PyObject *g_double_backward = nullptr; // differentiable backward of the convolution (create_graph)
 
@@ -101,10 +101,10 @@ struct Plan {
 };
 
 Plan ask_plan(const Tensor &scatter, const Tensor &gather, const Tensor &seg, int64_t K, int64_t n_out, int64_t outw,
-              int64_t inw, bool forced, bool split) {
+              int64_t inw, bool forced, bool split, bool capturing) {
     Plan plan;
     py::gil_scoped_acquire gil;
-    py::object r = py::reinterpret_borrow<py::object>(g_plan_hook)(scatter, gather, seg, K, n_out, outw, inw, forced, split);
+    py::object r = py::reinterpret_borrow<py::object>(g_plan_hook)(scatter, gather, seg, K, n_out, outw, inw, forced, split, capturing);
     if (!r.is_none()) {
         py::tuple t = py::cast<py::tuple>(r);
         plan.buffer = py::cast<Tensor>(t[0]);
@@ -218,7 +218,8 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
         const bool aligned = ((uintptr_t)ptr(weight) | (uintptr_t)ptr(feat)) % 16 == 0;   // else the CUDA-core engine
         const bool forced = engine == ENGINE_PLANNED, split = !forced && plan_split(feat.scalar_type(), K, G, inw, outw);
         if (fits && (forced || (aligned && (split || plan_unasked(K, G, outw))))) {
-            const Plan plan = ask_plan(scatter_, gather_, *seg_, K, n_out, G * outw, G * inw, forced, split);
+            const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
+            const Plan plan = ask_plan(scatter_, gather_, *seg_, K, n_out, G * outw, G * inw, forced, split, capturing);
             if (plan.valid && split) return mvmr_split(weight, feat, gather_, scatter_, *seg_, plan, n_out, flags, bias);
             if (plan.valid) return mvmr_planned(weight, feat, plan, T, n_out, flags, bias);
         }

@@ -175,3 +175,17 @@ def test_layer_norm_takes_rows_only():
     for shape in ((4, 8, 3), (8,)):
         with pytest.raises(ValueError):
             fused_layer_norm(torch.randn(shape), torch.tensor([4]))
+
+
+def _dense(monkeypatch):
+    monkeypatch.setattr(_cabi, "mvmr_plan", lambda *args: _plan(word=None))
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda device=None: "here")
+    return lambda: tuple(torch.arange(n, dtype=t) for n, t in ((3000, torch.int32), (3000, torch.int32), (28, torch.int64)))
+
+
+def test_wide_and_grouped_layers_are_captured_on_the_scatter_kernels(monkeypatch):
+    """... with a remembered plan too: what a graph reads are the caller's tensors."""
+    i, j, seg = _dense(monkeypatch)()
+    monkeypatch.setattr(_cabi, "_split_pays", lambda *args: True)
+    assert _cabi._plan_hook(i, j, seg, 27, 100, 512, 64, False, True, False) is not None
+    assert _cabi._plan_hook(i, j, seg, 27, 100, 512, 64, False, True, True) is None
