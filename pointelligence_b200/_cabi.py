@@ -624,6 +624,18 @@ def cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, group_blocks):
     return value
 
 
+_CAPTURED_PLANS = {}
+
+
+def _keep_for_graph(plan, scatter):
+    """A pass that is being captured reads the plan at every replay: it lives as long as the index tensor it was built
+    from, which is what the owner of a graph keeps anyway, whatever becomes of it in the cache."""
+    import weakref
+
+    if plan not in _CAPTURED_PLANS:
+        _CAPTURED_PLANS[plan] = weakref.ref(scatter, lambda _, kept=_CAPTURED_PLANS: kept.pop(plan, None))
+
+
 def mvmr_planned(weight, feat, plan, transpose, split=False):
     """``out[scatter[t]] += feat[gather[t]] @ W[tap(t)]`` for the rulebook of ``plan``
     (``transpose``: use W^T; ``split``: bucket sums in two parts); returns (plan.n_out, G * out_width) in feat.dtype."""
@@ -664,6 +676,8 @@ def _plan_hook(scatter, gather, seg_offs, K, n_out, outw, inw, forced, split=Fal
         if not forced and (scatter.is_inference() or gather.is_inference() or seg_offs.is_inference()):
             return None    # (a plan of inference tensors cannot be remembered, and one per pass does not pay)
         plan = cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, blocks)
+    if capturing:
+        _keep_for_graph(plan, scatter)
     return plan.buffer, plan.group_blocks, plan.multi_buckets
 
 

@@ -183,6 +183,31 @@ def _dense(monkeypatch):
     return lambda: tuple(torch.arange(n, dtype=t) for n, t in ((3000, torch.int32), (3000, torch.int32), (28, torch.int64)))
 
 
+@pytest.mark.parametrize("forced", [False, True])
+def test_a_plan_that_a_capture_reads_lives_as_long_as_its_rulebook(monkeypatch, forced):
+    """Sixty-four other plans, or a write to the index tensors, push it out of the cache; a graph goes on reading it."""
+    import gc
+    import weakref
+
+    dense = _dense(monkeypatch)
+    i, j, seg = dense()
+    call = lambda capturing: _cabi._plan_hook(i, j, seg, 27, 100, 64, 64, forced, False, capturing)
+    remembered = lambda: _cabi._remembered_plan(_cabi._plan_key(i, j, seg, 27, 100, _cabi.plan_group_blocks(64)), i, j, seg)
+    assert call(False) is not None
+    plan = weakref.ref(remembered())
+    assert call(True)[0] is plan().buffer and call(True)[0] is plan().buffer
+    others = [dense() for _ in range(_cabi._PLAN_CACHE_MAX + 1)]
+    for other in others:
+        _cabi._plan_hook(*other, 27, 100, 64, 64, forced)
+    i += 1
+    assert call(False) is not None
+    gc.collect()
+    assert plan() is not None and remembered() is not plan()
+    del i, call, remembered
+    gc.collect()
+    assert plan() is None
+
+
 def test_wide_and_grouped_layers_are_captured_on_the_scatter_kernels(monkeypatch):
     """... with a remembered plan too: what a graph reads are the caller's tensors."""
     i, j, seg = _dense(monkeypatch)()
