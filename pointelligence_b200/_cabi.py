@@ -675,7 +675,12 @@ def _plan_hook(scatter, gather, seg_offs, K, n_out, outw, inw, forced, split=Fal
     if plan is None:
         if not forced and (scatter.is_inference() or gather.is_inference() or seg_offs.is_inference()):
             return None    # (a plan of inference tensors cannot be remembered, and one per pass does not pay)
-        plan = cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, blocks)
+        try:
+            plan = cached_mvmr_plan(scatter, gather, seg_offs, K, n_out, blocks)
+        except torch.OutOfMemoryError:
+            if not split:
+                raise
+            return None    # wide and grouped layers fit without a plan
     if capturing:
         _keep_for_graph(plan, scatter)
     return plan.buffer, plan.group_blocks, plan.multi_buckets

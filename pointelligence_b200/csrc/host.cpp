@@ -165,13 +165,19 @@ Tensor mvmr_planned(const Tensor &weight, const Tensor &feat, const Plan &plan, 
     return out;
 }
 
+// (undefined where the device has no room for its scratch)
 Tensor mvmr_split(const Tensor &weight, const Tensor &feat, const Tensor &gather_, const Tensor &scatter_, const Tensor &seg_,
                   const Plan &plan, int64_t n_out, int flags, const Tensor &bias) {
     const int64_t K = weight.size(0), G = weight.size(1), C = weight.size(2), M = weight.size(3);
     const int transpose = flags & 1;
     const Tensor gather = as_i32(gather_), scatter = as_i32(scatter_), seg = as_i64(seg_);
     Tensor out = at::empty({n_out, G * (transpose ? C : M)}, feat.options());
-    Tensor ws = workspace(pcx_mvmr_split_workspace_bytes(plan.multi, n_out, (int)K, (int)G, (int)C, (int)M, transpose), feat);
+    Tensor ws;
+    try {
+        ws = workspace(pcx_mvmr_split_workspace_bytes(plan.multi, n_out, (int)K, (int)G, (int)C, (int)M, transpose), feat);
+    } catch (const c10::OutOfMemoryError &) {
+        return Tensor();
+    }
     check(pcx_mvmr_split(ptr(weight), ptr(feat), ptr_as<int32_t>(gather), ptr_as<int32_t>(scatter), ptr_as<int64_t>(seg), ptr(plan.buffer),
                          plan.buffer.numel(), ptr(bias), ptr(out), gather.numel(), feat.size(0), n_out, (int)K, (int)G, (int)C, (int)M,
                          flags, (int)plan.group, plan.multi, ptr(ws), ws.numel(), stream()));
@@ -220,8 +226,11 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
         if (fits && (forced || (aligned && (split || plan_unasked(K, G, outw))))) {
             const bool capturing = c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None;
             const Plan plan = ask_plan(scatter_, gather_, *seg_, K, n_out, G * outw, G * inw, forced, split, capturing);
-            if (plan.valid && split) return mvmr_split(weight, feat, gather_, scatter_, *seg_, plan, n_out, flags, bias);
-            if (plan.valid) return mvmr_planned(weight, feat, plan, T, n_out, flags, bias);
+            if (plan.valid && !split) return mvmr_planned(weight, feat, plan, T, n_out, flags, bias);
+            if (plan.valid) {
+                const Tensor out = mvmr_split(weight, feat, gather_, scatter_, *seg_, plan, n_out, flags, bias);
+                if (out.defined()) return out;
+            }
         }
         engine = 0;
     }

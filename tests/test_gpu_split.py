@@ -89,3 +89,24 @@ def test_finite_operands_are_not_done_again(always):
     x = torch.randn(500, 96, device=DEV).bfloat16()
     plan = always.mvmr_plan(i, j, seg, 27, 900, always.plan_group_blocks(128))
     assert torch.equal(always.mvmr(w, x, j, i, seg, None, 900, False), always.mvmr_planned(w, x, plan, False, True))
+
+
+@pytest.mark.parametrize("room,T", [(64, 8000000), (150, 400000)])   # MB: the plan does not fit; the plan does, the sums do not
+def test_a_device_without_room_for_plan_or_sums(always, room, T):
+    """The scatter kernels take the call, as they did before there was a choice."""
+    n = 20000
+    i, j, seg = _rulebook(4, n, n, 27, T)
+    w = (torch.randn(27, 1, 1024, 288, device=DEV) / 32).bfloat16()
+    x = torch.randn(n, 1024, device=DEV).bfloat16()
+    plan = lambda: always._remembered_plan(always._plan_key(i, j, seg, 27, n, always.plan_group_blocks(288)), i, j, seg)
+    want = always.mvmr(w, x, j, i, seg, None, n, False, always.ENGINE_TENSOR)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + (room << 20)) / total)
+    try:
+        out, names = _kernels(always, lambda: always.mvmr(w, x, j, i, seg, None, n, False))
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert names == ["mvmr_tc_kernel(fwd)"] and (plan() is not None) is (room == 150)
+    assert float((out.float() - want.float()).norm() / want.float().norm()) < 1e-3     # ties of the one rounding
