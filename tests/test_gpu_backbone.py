@@ -115,3 +115,31 @@ def test_geometry_on_its_own_stream_gives_the_same_step(monkeypatch):
         books.append(m)
     for name in ("i", "j", "k", "seg_offs", "points", "sample_inds", "downsample_indices"):
         assert torch.equal(getattr(books[0], name), getattr(books[1], name)), name
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.bfloat16, 2.0 ** -8), (torch.float16, 2.0 ** -11), (torch.float32, 1e-5)])
+@pytest.mark.parametrize("n,taken,C,M", [(1000, None, 64, 96), (1000, 400, 64, 96), (500, None, 20, 36), (500, 130, 20, 36),
+                                         (300, None, 384, 300), (300, 100, 384, 64), (1, None, 32, 32), (1, 1, 32, 32)])
+def test_shortcut_projection_and_its_gradients(n, taken, C, M, dtype, tol):
+    """Rows stored as they are computed, or gathered ones; padded widths, contractions of several parts, one row.  An
+    element is a sum of fp32 accuracy rounded once: half an ulp of it, and 2^-20 of the magnitudes that made it up."""
+    from pointelligence_b200.backbone import project_rows
+
+    dev = "cuda:0"
+    g = torch.Generator(device=dev).manual_seed(n + C)
+    x = torch.randn(n, C, device=dev, generator=g).to(dtype).requires_grad_()
+    w = (torch.randn(M, C, device=dev, generator=g) / C ** 0.5).to(dtype).requires_grad_()
+    rows = None if taken is None else torch.randperm(n, device=dev, generator=g)[:taken]
+    y = project_rows(x, rows, w)
+    go = torch.randn(y.shape, device=dev, generator=g).to(dtype)
+    gx, gw = torch.autograd.grad(y, (x, w), go)
+    at = torch.arange(n, device=dev) if rows is None else rows
+    xd, wd, god = x.detach().double()[at], w.detach().double(), go.double()
+
+    def spread(v):
+        return torch.zeros(n, C, dtype=torch.float64, device=dev).index_add_(0, at, v)
+
+    for got, want, size in ((y.detach(), xd @ wd.T, xd.abs() @ wd.abs().T), (gx, spread(god @ wd), spread(god.abs() @ wd.abs())),
+                            (gw, god.T @ xd, god.abs().T @ xd.abs())):
+        assert got.dtype == dtype and got.shape == want.shape
+        assert bool(((got.double() - want).abs() <= tol * want.abs() + 2.0 ** -20 * size).all())

@@ -110,3 +110,45 @@ def test_a_device_without_room_for_plan_or_sums(always, room, T):
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert names == ["mvmr_tc_kernel(fwd)"] and (plan() is not None) is (room == 150)
     assert float((out.float() - want.float()).norm() / want.float().norm()) < 1e-3     # ties of the one rounding
+
+
+@pytest.mark.parametrize("G,C,M", [(2, 32, 48), (1, 64, 288), (1, 288, 64)])
+def test_layer_on_a_self_search_rulebook(always, G, C, M):
+    """A bias, and the input gradient over the forward plan with the taps of the weight reversed.  Bounds as for two-part sums
+    in general: 2^-8 of an element for its one rounding, 2^-16 + 2^-19 of the magnitudes that made it up."""
+    from pointelligence_b200.layers import PointConv3d
+
+    g = torch.Generator(device=DEV).manual_seed(C)
+    pts = torch.rand(900, 3, device=DEV, generator=g)
+    i, j, k, seg, _ = always.radius_search(pts, pts, 0.25, None, None, 0, 3, 0.1, want_k=True)
+    always.mark_built(i, j, seg, 27, True)
+    conv = PointConv3d(G * C, G * M, 3, groups=G, bias=True, device=DEV, dtype=torch.bfloat16)
+    with torch.no_grad():
+        conv.bias.normal_()
+    x = torch.randn(900, G * C, device=DEV, generator=g).bfloat16().requires_grad_()
+    go = torch.randn(900, G * M, device=DEV, generator=g).bfloat16()
+
+    def step():
+        y = conv(x, i, j, k, 900, seg_offs=seg)
+        return y.detach(), torch.autograd.grad(y, x, go)[0]
+
+    (y, gx), names = _kernels(always, step)
+    assert [n for n in names if "mvmr" in n] == ["mvmr_os_kernel(fwd)", "mvmr_os_kernel(dgrad)"]
+    w = conv.weight.detach().double().view(27, G, C, M)
+    bias = conv.bias.detach().double()
+
+    def sums(x, w, scatter, gather, width):
+        out = torch.zeros(900, G, width, dtype=torch.float64, device=DEV)
+        for t in range(27):
+            s = slice(int(seg[t]), int(seg[t + 1]))
+            out.index_add_(0, scatter[s].long(), torch.einsum("tgc,gcm->tgm", x.view(900, G, -1)[gather[s].long()], w[t]))
+        return out.flatten(1)
+
+    xd, god = x.detach().double(), go.double()
+    for got, want, size, part in ((y, sums(xd, w, i, j, M) + bias, sums(xd.abs(), w.abs(), i, j, M) + bias.abs(), M),
+                                  (gx, sums(god, w.transpose(2, 3), j, i, C), sums(god.abs(), w.abs().transpose(2, 3), j, i, C), C)):
+        if G == 1 and part <= 256:
+            continue    # sums rounded to 16 bits, as the layers of that width have them
+        lost = size * (2.0 ** -16 + 2.0 ** -19)
+        assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + lost * (1 + 2.0 ** -8)).all())
+    assert always.device_status() == 0
