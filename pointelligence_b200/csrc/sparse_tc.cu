@@ -99,7 +99,7 @@ __device__ __forceinline__ float unpack_one(uint16_t v, int fmt) {
 }
 
 // Wide and grouped layers run as parts of at most 256 x 256 channels, every part of a width of the same size, a
-// multiple of 16.  blockIdx.y counts (group, part of the output row, link of the contraction): a block takes up to
+// multiple of 16.  blockIdx.y counts (group, part of the output row, link of the contraction): a block takes
 // p.chain parts of a contraction one after another, each into tensor memory columns of its own, and reduces their
 // sum.  (As blocks of their own they meet in the accumulator, with as many reductions more: fp16, 31 852 triplets of
 // 512 x 512 channels 75 us, chained 65; 408 976 triplets 726 and 676; 2048 to 128 channels 895 and 817.)  One column
@@ -150,9 +150,9 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 1 : 0) mvmr_tc_kernel(MvmrTcPa
     const int inw = p.transpose ? p.M : p.C, outw = p.transpose ? p.C : p.M;
     int parts;   // of the contraction, in this block
     {
-        const int links = (p.in_parts + p.chain - 1) / p.chain, ip = (int)blockIdx.y % links * p.chain,
+        const int links = p.in_parts / p.chain, ip = (int)blockIdx.y % links * p.chain,
                   op = (int)blockIdx.y / links % p.out_parts, g = (int)blockIdx.y / (links * p.out_parts);
-        parts = CHAINED ? min(p.chain, p.in_parts - ip) : 1;
+        parts = CHAINED ? p.chain : 1;
         const int64_t out0 = ((int64_t)g * p.out_parts + op) * outw;
         p.feat += ((int64_t)g * p.in_parts + ip) * inw;
         p.acc += out0;
@@ -501,16 +501,22 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
         if (atoi(e) == 2 && rest + 2 * (size_t)kb * BLK_BYTES + static_smem <= 232448 - 1024) p.nbuf = 2;
     if (p.alias) p.nbuf = 1;
     size_t smem = rest + std::max((size_t)p.nbuf * kb * BLK_BYTES, p.alias ? (size_t)p.park_bytes : (size_t)0);
-    // 256 threads, and the parts of a contraction in one block, where one CTA fills an SM's shared memory.  The parts
-    // stay blocks of their own where the chip would not be filled without: 1 920 triplets, 2048 to 128 channels, took
-    // 34.6 us with eight parts in one block and 17.7 in eight.  Plain reductions into an accumulator much larger than
+    // 256 threads, and parts of a contraction in one block, where one CTA fills an SM's shared memory: as many parts as
+    // tensor memory holds, in links of the same length.  Every link gets the same share of the chip, so a shorter one would
+    // leave its share idle (300 000 triplets, us, in links as equal as parts allow / of one part / as long as possible:
+    // 768 to 512 channels, three parts, two fit: 779 / 779 / 908; 1280 to 128, five, four fit: 409 / 409 / 562; 1536 to 128,
+    // six: 450 / 487 / 567; 2048 to 128, eight: 580 / 634 / 580).  A link saves an eighth of its parts' time;
+    // where the tiles of so few blocks make more turns of the chip than that, the parts stay blocks of their own (174 tiles:
+    // 1024 to 128 channels 38 us, in one link 46, 2048 to 128 60.5 and 62.6; 276 tiles: 1024 to 128 54 and 46, 512 to 512 87 and
+    // 71; 808: 768 to 128 99 and 93).  Plain reductions into an accumulator much larger than
     // the L2 cache keep 128 threads: they are bound by its misses (256 x 256 into 184 MB 584 us and with 256 threads
     // 620; into 123 MB 398 and 388, 61 MB 208 and 202).
     const bool one_cta = !store && !bulk && outw > 64 && 2 * (smem + static_smem + 1024) > 232448;
     p.chain = one_cta && p.nbuf == 1 ? std::min(p.in_parts, (int)(512 / p.acc_cols)) : 1;
-    auto blocks = [&] { return a.G * p.out_parts * ((p.in_parts + p.chain - 1) / p.chain); };
-    if (upper * blocks() < num_sms()) p.chain = 1;
-    const int parts = blocks();
+    while (p.in_parts % p.chain) --p.chain;
+    int parts = a.G * p.out_parts * (p.in_parts / p.chain);
+    auto turns = [&](int n) { return (upper + std::max(1, num_sms() / n) - 1) / std::max(1, num_sms() / n); };
+    if (7 * p.chain * turns(parts) > 8 * turns(parts * p.chain)) parts *= p.chain, p.chain = 1;
     p.ncols = pow2_cols(p.acc_cols * p.chain);
     const bool more = one_cta && (p.chain > 1 || a.n_out * p.out_pitch * 4 <= (int64_t)160 << 20);
     smem = pad_for_tmem(smem, p.ncols);

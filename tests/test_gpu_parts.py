@@ -199,3 +199,47 @@ def test_parts_of_a_contraction_in_one_block(C, M, G, T, dtype):
     y = _cabi.mvmr(w, x, j, i, seg, None, n, False, _cabi.ENGINE_TENSOR)
     gx = _cabi.mvmr(w, go, i, j, seg, None, n, True, _cabi.ENGINE_TENSOR)
     assert torch.equal(y.double(), y_ref.flatten(1)) and torch.equal(gx.double(), gx_ref.flatten(1))
+
+
+def _whole_numbers(dtype, seed, T, n, C, M, n_in=None):
+    """Operands of -1, 0 and 1, one in eight not 0: every sum a whole number, exact in fp32 and, below 2^8, after the rounding."""
+    n_in = n_in or n
+    i, j, k, seg = _rulebook(n, n_in, 27, T, seed)
+    g = torch.Generator(device=DEV).manual_seed(seed)
+
+    def few(*shape):
+        sign = 2 * torch.randint(0, 2, shape, device=DEV, generator=g) - 1
+        return (torch.randint(0, 8, shape, device=DEV, generator=g) // 7 * sign).to(dtype)
+
+    w, x, go = few(27, 1, C, M), few(n_in, C), few(n, M)
+    y, gx = (torch.zeros(rows, width, dtype=torch.float64, device=DEV) for rows, width in ((n, M), (n_in, C)))
+    for t in range(27):
+        s = slice(int(seg[t]), int(seg[t + 1]))
+        y.index_add_(0, i[s].long(), x[j[s].long()].double() @ w[t, 0].double())
+        gx.index_add_(0, j[s].long(), go[i[s].long()].double() @ w[t, 0].double().T)
+    assert max(y.abs().max(), gx.abs().max()) < 256
+    return i, j, seg, w, x, go, y, gx
+
+
+# parts of the contraction, what tensor memory holds of them, links: 3 / 4 / 1, 4 / 4 / 1, 5 / 4 / 5, 6 / 4 / 2, 7 / 4 / 7, 8 / 4 / 2;
+# 3 / 2 / 3, 4 / 2 / 2; three narrow parts
+@pytest.mark.parametrize("C,M", [(768, 128), (1024, 128), (1280, 80), (1536, 128), (1792, 96), (2048, 128), (768, 512), (1024, 256), (528, 80)])
+@pytest.mark.parametrize("T", [20000, 60000])   # too few tiles for links of several parts, and enough
+def test_links_of_a_contraction(C, M, T):
+    from pointelligence_b200 import _cabi
+
+    i, j, seg, w, x, go, y, gx = _whole_numbers(torch.float16, C + M, T, T // 4, C, M)
+    assert torch.equal(_cabi.mvmr(w, x, j, i, seg, None, T // 4, False, _cabi.ENGINE_TENSOR).double(), y)
+    assert torch.equal(_cabi.mvmr(w, go, i, j, seg, None, T // 4, True, _cabi.ENGINE_TENSOR).double(), gx)
+    wt = w.transpose(2, 3).contiguous()     # the same links in the other direction
+    assert torch.equal(_cabi.mvmr(wt, x, j, i, seg, None, T // 4, True, _cabi.ENGINE_TENSOR).double(), y)
+    assert _cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [163840, 163841])   # accumulators of 160 MB and a row more: eight warps a block, and four
+def test_accumulators_about_the_size_that_keeps_four_warps(n):
+    from pointelligence_b200 import _cabi
+
+    i, j, seg, w, x, go, y, gx = _whole_numbers(torch.float16, 3, 30000, n, 256, 256, n_in=9000)
+    assert torch.equal(_cabi.mvmr(w, x, j, i, seg, None, n, False, _cabi.ENGINE_TENSOR).double(), y)
+    assert torch.equal(_cabi.mvmr(w, go, i, j, seg, None, 9000, True, _cabi.ENGINE_TENSOR).double(), gx)
