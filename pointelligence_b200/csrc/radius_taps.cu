@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(THREADS, REC_MAX > 1024 ? 4 : 5) taps_fill_ker
         uint2 sorted[REC_MAX];
         Walk walk;
     } s_u;
-    extern __shared__ uint16_t s_cnt[];                     // [tap][query]: pairs, then those of the queries before
+    extern __shared__ __align__(16) uint16_t s_cnt[];       // [tap][query]: pairs, then those of the queries before (32-bit words, too)
     __shared__ uint32_t s_base[MAX_K3];                     // next write position of each tap for this block
     __shared__ uint32_t s_start[MAX_K3], s_total[MAX_K3];   // first place of each tap among the sorted, its pairs in this round
     const bool fits = a.ctrl[0] <= a.capacity && !a.ctrl[1];
