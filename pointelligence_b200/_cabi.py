@@ -401,15 +401,29 @@ def _planned_pays(T, n_out, outw, K):
 #   25.4 (15 000)                672 / 350     232 / 95      277 / 49       150 / 100       139
 #
 # (these and below without the scatter kernels behind, which return at once where all operands are finite: 9 us more.)
-# It is chosen where the scatter kernel's fp32 reductions (triplets x width x 4 bytes) are half a gigabyte, so that one
-# pass pays for most of a plan, and the two-part sums stay within 4 GB.  The input gradient of an up-sampling layer 384 ->
+# It is chosen where the scatter kernel's fp32 reductions (triplets x width x 4 bytes) are half a gigabyte and the two-part
+# sums stay within 4 GB.  On a plan that exists it would pay far below that (the first line: 65 and 390 MB); the line is
+# for rulebooks that are used once or twice.  At half a gigabyte a pass over a dense rulebook gains a quarter of a plan
+# (2 x 64 -> 64, 22.5 triplets a row: 180 / 128, plan 190) to twice one (1024 -> 288, 15.7: 1074 / 777, plan 163).  Thin
+# rulebooks gain less, and a contraction much longer than the row loses on a plan that exists, too, since the low parts are
+# multiplied tile by tile whether or not a tile holds a sum.  Below six triplets a row, scatter / split / plan:
+#
+#   4.9 (60 000)     512 -> 512    514 /  462 / 163 (574 MB)    1024 -> 512   942 /  907     32 -> 512  260 /  75
+#   5.0 (120 000)    512 -> 512   1037 /  858 / 182 (1182 MB)   1024 -> 512  1914 / 1683     1024 -> 288  1439 / 1498 (665 MB)
+#   6.8 (60 000)     512 -> 512    679 /  519 / 168 (800 MB)    1024 -> 512  1274 / 1034     128 -> 384  273 / 145
+#
+# There it takes a gigabyte, and a contraction of at most twice the row.  The input gradient of an up-sampling layer 384 ->
 # 128 with 134 triplets a row (18.9 M) took 10.1 ms on the scatter kernel; the training step around it went from 113.0 to
 # 104.7 ms, its plan included.
 _SPLIT_MIN_REDUCED_BYTES, _SPLIT_MAX_SCRATCH_BYTES = 512 << 20, 4 << 30
 
 
 def _split_pays(T, n_out, outw, inw, K):
-    return T * outw * 4 >= _SPLIT_MIN_REDUCED_BYTES and min(T // 2, n_out * K) * inw * 4 <= _SPLIT_MAX_SCRATCH_BYTES
+    thin = T < 6 * n_out
+    if thin and inw > 2 * outw:
+        return False
+    return (T * outw * 4 >= _SPLIT_MIN_REDUCED_BYTES * (2 if thin else 1)
+            and min(T // 2, n_out * K) * inw * 4 <= _SPLIT_MAX_SCRATCH_BYTES)
 
 
 _PLAN_WAIT_SECONDS = 30.0   # for a plan that is being built on another stream

@@ -214,3 +214,12 @@ def test_wide_and_grouped_layers_are_captured_on_the_scatter_kernels(monkeypatch
     monkeypatch.setattr(_cabi, "_split_pays", lambda *args: True)
     assert _cabi._plan_hook(i, j, seg, 27, 100, 512, 64, False, True, False) is not None
     assert _cabi._plan_hook(i, j, seg, 27, 100, 512, 64, False, True, True) is None
+
+
+@pytest.mark.parametrize("T,n,outw,inw,pays", [
+    (605_000, 120_000, 288, 1024, False), (1_300_000, 260_000, 288, 1024, False),    # thin, and a long contraction
+    (294_000, 60_000, 512, 512, False), (605_000, 120_000, 512, 1024, True),         # thin: from a gigabyte
+    (409_000, 60_000, 512, 512, True), (450_000, 60_000, 288, 1024, False), (847_000, 120_000, 288, 1024, True),
+    (18_900_000, 141_000, 384, 128, True), (18_900_000, 141_000, 384, 1024, False)])  # 15 GB of sums
+def test_rulebooks_on_which_two_part_sums_pay(T, n, outw, inw, pays):
+    assert _cabi._planned_pays(T, n, outw, 27) and _cabi._split_pays(T, n, outw, inw, 27) is pays
