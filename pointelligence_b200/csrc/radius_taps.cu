@@ -306,7 +306,7 @@ struct Accepted {
     }
 };
 
-// Bound by issuing instructions (1140 a warp of four queries and some 330 candidates).  One list of candidates a warp and
+// Bound by issuing instructions (150 000 points with six neighbours: 745 a warp of four queries, issue slots 76 % busy).  One list of candidates a warp and
 // a four a lane: 1 M points in eight rooms, 512 000 queries at a stride of two, 230 -> 170 us; 150 000 points 50 -> 35;
 // four LiDAR sweeps 68 -> 53.  Eight lanes a query with a list of their own, and pieces of eight candidates: 207, 48, 74.
 template <bool FUSED>
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) taps_colscan_kernel(uint32_t *bl
 }
 
 // Kept pairs are counted by shared-memory additions in any order and put in order within their few neighbours of the same
-// query and tap when they are written; matching lanes by tap kept one pipe 63 % busy and took 141 us instead of 111 below.
+// query and tap when they are written; matching lanes by tap took 141 us instead of 111 below.
 // Before pairs were sorted in shared memory and written side by side: 512 000 queries with 13 neighbours 175 -> 112 us,
 // 150 000 points 37 -> 26, LiDAR 67 -> 38 (with 64 instead of 48 kept pairs; 65 with 48: one query in ninety has more,
 // and its warp keeps the block waiting), 125 taps, 100 000 queries with 41 152 -> 110.
