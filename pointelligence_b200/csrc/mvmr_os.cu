@@ -491,8 +491,9 @@ template <int FMT, bool SPLIT>
 int launch_bucket_sum(int64_t multi, int inw, const uint16_t *feat, const uint2 *entries, const uint2 *buckets,
                        const uint32_t *ctrl, uint16_t *scratch, const uint4 *weight, int64_t weight_pieces, uint32_t *odd, cudaStream_t stream) {
     // Up to 128 channels the next power of two of lanes, beyond that slices (blockIdx.y) of 32, 16 or 8 lanes, whichever
-    // idles least: 192 channels 197 us in slices of 8 (223 of 32), 384 386 of 16 (444 of 8, 429 of 32), 256 255 of 32
-    // (245 of 16, 268 of 8), 208 241 of 32 (249 of 16).  Below: 48 channels 63 us in 8 lanes (80 in slices of 2).
+    // idles least, the widest of equals (200k points, 22 triplets a row): 256 channels 258 us in slices of 32 (266 of 16, 300 of 8),
+    // 512 561 (577, 707), 208 247 (274, 292), 192 214 of 8 (222 of 32, 241 of 16), 384 417 of 16 (472 of 32, 511 of 8).
+    // Below: 48 channels 63 us in 8 lanes (80 in slices of 2).
     const int ppr = inw >> 3;
     int lanes = 2;
     while (lanes < ppr && lanes < 16) lanes <<= 1;
@@ -656,7 +657,7 @@ struct Walk {
 };
 
 // PACK: taps of a step.  SPLIT: the scratch holds every bucket's sum as two 16-bit rows, the rounded sum and what the
-// rounding left over, and the contraction goes over both: sums of 16 bits more (bf16: 2^-16 of the sum is lost where
+// rounding left over, and the contraction goes over both: sums of twice as many bits (bf16: 2^-16 of the sum is lost where
 // one row loses 2^-8), for a second pass over the taps.
 template <int PACK, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ OsParams p) {
