@@ -189,13 +189,14 @@ __device__ __forceinline__ int2 run_of(const TapArgs &a, float qx, float qy, flo
     // the rounding of its cell, some 3e-7 of the coordinate; the predicate's own rounding is some 1e-6 of R^2.  A cell number
     // at the end of the integers says no more than that the point lies there or beyond: such a cell is always looked at.
     if (a.distance_type == 0) {
+        float far = 0.f;
         auto gap = [&](float v, int k) {
-            if (k >= 1 << 30 || k <= -(1 << 30)) return 0.f;
+            far = fmaxf(far, fabsf((float)k));
             const float lo = (float)k * a.cell, slack = 1e-6f * (fabsf(v) + 2.f * a.cell);
             return fmaxf(fmaxf(lo - v, v - (lo + a.cell)) - slack, 0.f);
         };
         const float gx = gap(qx, cx), gy = gap(qy, cy), gz = gap(qz, cz);
-        if (gx * gx + gy * gy + gz * gz > a.reach) return make_int2(0, 0);
+        if (gx * gx + gy * gy + gz * gz > a.reach && far < 0x1p30f) return make_int2(0, 0);
     }
     const int2 r = a.table[cell_bucket(b, cx, cy, cz, a.mask)];
     return make_int2(r.x, r.y - r.x);
