@@ -152,3 +152,42 @@ def test_layer_on_a_self_search_rulebook(always, G, C, M):
         lost = size * (2.0 ** -16 + 2.0 ** -19)
         assert bool(((got.double() - want).abs() <= want.abs() * 2.0 ** -8 + lost * (1 + 2.0 ** -8)).all())
     assert always.device_status() == 0
+
+
+def _captured(fn):
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        fn()                                  # the usual warm-up: a plan is built and remembered
+    torch.cuda.current_stream().wait_stream(side)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = fn()
+    return graph, out
+
+
+@pytest.mark.parametrize("G,C,M", [(1, 64, 288), (2, 32, 48)])
+def test_a_replay_of_a_wide_or_grouped_layer_follows_its_index_tensors(always, G, C, M):
+    i, j, seg = _rulebook(8, 500, 900, 27, 20000)
+    w, x = (torch.randn(27, G, C, M, device=DEV) / 8).bfloat16(), torch.randn(500, G * C, device=DEV).bfloat16()
+    graph, out = _captured(lambda: always.mvmr(w, x, j, i, seg, None, 900, False))
+    for t, other in zip((i, j, seg), _rulebook(9, 500, 900, 27, 20000)):
+        t.copy_(other)
+    graph.replay()
+    want = always.mvmr(w, x, j, i, seg, None, 900, False, always.ENGINE_TENSOR)
+    assert float((out.float() - want.float()).norm() / want.float().norm()) < 1e-3
+
+
+def test_a_replay_reads_a_plan_that_the_cache_has_dropped(always):
+    i, j, seg = _rulebook(10, 500, 900, 27, 20000)
+    w, x = (torch.randn(27, 1, 64, 64, device=DEV) / 8).bfloat16(), torch.randn(500, 64, device=DEV).bfloat16()
+    graph, out = _captured(lambda: always.mvmr(w, x, j, i, seg, None, 900, False))
+    want = always.mvmr(w, x, j, i, seg, None, 900, False)
+    plan = always._remembered_plan(always._plan_key(i, j, seg, 27, 900, always.plan_group_blocks(64)), i, j, seg)
+    size, address = plan.buffer.numel(), plan.buffer.data_ptr()
+    del plan
+    always._PLAN_CACHE.clear()
+    taken = [torch.empty(size, dtype=torch.uint8, device=DEV) for _ in range(8)]    # what a freed buffer's place would go to
+    assert address not in [t.data_ptr() for t in taken]
+    graph.replay()
+    assert torch.equal(out, want)
