@@ -111,10 +111,10 @@ int launch_column_sums(const void *x, void *out, int64_t N, int C, float *partia
 // acc[r][c] = bias[c], or zero; W divides the row width, so a thread's W columns lie in one row.  Bound by the stores: with a
 // 64-bit remainder for every one of them, 150 000 x 64 took 8.1 us instead of some 5 (a memset of that size: 4.6, and no kernel
 // can be set up behind it).
-template <typename T, int W>
+template <typename T, int W, bool AGAIN>
 __global__ void fill_rows_kernel(float *__restrict__ acc, const T *__restrict__ bias, int64_t n, int width, OnlyIf only_if) {
     start_after_previous();
-    if (!only_if.holds()) return;
+    if (AGAIN && !only_if.holds()) return;
     const int64_t stride = (int64_t)gridDim.x * blockDim.x * W;
     int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * W;
     int c = bias ? (int)(i % width) : 0;
@@ -142,8 +142,9 @@ int launch_fill(float *acc, const void *bias, int64_t rows, int width, OnlyIf on
     const int64_t n = rows * width;
     const int w = (bias ? width : n) % 4 == 0 && (uintptr_t)acc % 16 == 0 ? 4 : 1;
     const unsigned grid = (unsigned)std::min<int64_t>((n / w + 255) / 256, (int64_t)num_sms() * (only_if.words ? 4 : 16));
-    if (w == 4) launch_after(fill_rows_kernel<T, 4>, grid, 256, 0, stream, acc, (const T *)bias, n, width, only_if);
-    else launch_after(fill_rows_kernel<T, 1>, grid, 256, 0, stream, acc, (const T *)bias, n, width, only_if);
+    const bool again = only_if.words != nullptr;
+    if (w == 4) launch_after((again ? fill_rows_kernel<T, 4, true> : fill_rows_kernel<T, 4, false>), grid, 256, 0, stream, acc, (const T *)bias, n, width, only_if);
+    else launch_after((again ? fill_rows_kernel<T, 1, true> : fill_rows_kernel<T, 1, false>), grid, 256, 0, stream, acc, (const T *)bias, n, width, only_if);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
 }

@@ -63,12 +63,12 @@ void launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
 }
 
 // What a kernel is launched for only if an earlier one found a reason: a word from each of that one's blocks, zero where it
-// found none.  No words: always.  Asked by a whole block.
+// found none.  No words: always.  Asked by a whole block, in variants of their own (AGAIN) of kernels that are mostly launched
+// without: asked at run time, a pass over 150 000 points and 64 channels (clear, scatter, round) took 82 us instead of 81.
 struct OnlyIf {
     const uint32_t *words = nullptr;
     int n = 0;
     __device__ __forceinline__ bool holds() const {
-        if (!words) return true;
         bool any = false;
         for (int t = threadIdx.x; t < n; t += blockDim.x) any |= words[t] != 0;
         return __syncthreads_or(any);

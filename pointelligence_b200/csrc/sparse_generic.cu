@@ -84,11 +84,12 @@ __global__ void vvor_unsorted_kernel(const T *__restrict__ A, const int32_t *__r
     }
 }
 
-template <typename T>
+template <typename T, bool AGAIN>
 __global__ void round_kernel(const float *__restrict__ acc, T *__restrict__ out, int64_t n, OnlyIf only_if) {
     start_after_previous();
-    if (!only_if.holds()) return;
-    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * 4; i < n; i += (int64_t)gridDim.x * blockDim.x * 4) {
+    if (AGAIN && !only_if.holds()) return;
+    // (blocks for all of it, or fewer that mostly have nothing to do)
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * 4; i < n; i += AGAIN ? (int64_t)gridDim.x * blockDim.x * 4 : n) {
         if (i + 3 < n) {
             float4 v = *reinterpret_cast<const float4 *>(acc + i);
             out[i] = from_f32<T>(v.x);
@@ -153,9 +154,10 @@ int vvor_generic(const VvorArgs &a, cudaStream_t stream) {
 int round_accumulator(const float *acc, void *out, int64_t n, int dtype, cudaStream_t stream, OnlyIf only_if) {
     if (n == 0) return PCX_OK;
     unsigned blocks = (unsigned)((n / 4 + 255) / 256 + 1);
-    if (only_if.words) blocks = std::min(blocks, (unsigned)num_sms() * 4);   // mostly there is nothing to do
-    if (dtype == PCX_F16) launch_after(round_kernel<__half>, blocks, 256, 0, stream, acc, (__half *)out, n, only_if);
-    else if (dtype == PCX_BF16) launch_after(round_kernel<__nv_bfloat16>, blocks, 256, 0, stream, acc, (__nv_bfloat16 *)out, n, only_if);
+    const bool again = only_if.words != nullptr;
+    if (again) blocks = std::min(blocks, (unsigned)num_sms() * 4);
+    if (dtype == PCX_F16) launch_after((again ? round_kernel<__half, true> : round_kernel<__half, false>), blocks, 256, 0, stream, acc, (__half *)out, n, only_if);
+    else if (dtype == PCX_BF16) launch_after((again ? round_kernel<__nv_bfloat16, true> : round_kernel<__nv_bfloat16, false>), blocks, 256, 0, stream, acc, (__nv_bfloat16 *)out, n, only_if);
     else PCX_FAIL(PCX_E_DTYPE, "round_accumulator: dtype %d", dtype);
     PCX_LAUNCH_CHECK();
     return PCX_OK;

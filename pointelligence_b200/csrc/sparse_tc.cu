@@ -135,10 +135,10 @@ struct MvmrTcParams {
 // NT: 128 threads, or 256 where shared memory leaves room for few CTAs (mode 0): with four warps an SM a 256 x 256 part
 // waited for its own copies and reductions (31 852 triplets of 512 x 512 fp16 channels 69 us, with eight warps 65;
 // 256 x 256 channels, 408 976 triplets 212 and 201).
-template <int MODE, int NT, bool CHAINED>
+template <int MODE, int NT, bool CHAINED, bool AGAIN>
 __global__ void __launch_bounds__(NT, NT == 256 ? 1 : 0) mvmr_tc_kernel(MvmrTcParams p) {
     start_after_previous();
-    if (!p.only_if.holds()) return;
+    if (AGAIN && !p.only_if.holds()) return;
     constexpr bool BULK = MODE == 1;
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t s_bar;
@@ -521,13 +521,16 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
     const bool more = one_cta && (p.chain > 1 || a.n_out * p.out_pitch * 4 <= (int64_t)160 << 20);
     smem = pad_for_tmem(smem, p.ncols);
     if (smem + static_smem > 232448 - 1024) PCX_FAIL(PCX_E_UNSUPPORTED, "mvmr tensor kernel does not fit (smem %zu)", smem);
-    const int mode = store ? 2 : bulk ? 1 : p.chain > 1 ? 4 : more ? 3 : 0, threads = more ? 256 : 128;
-    static int granted_mvmr[5][64] = {}, regs_mvmr[5] = {};   // per kernel (and device)
-    const auto kernel = mode == 4   ? mvmr_tc_kernel<0, 256, true>
-                        : mode == 3 ? mvmr_tc_kernel<0, 256, false>
-                        : mode == 2 ? mvmr_tc_kernel<2, 128, false>
-                        : mode == 1 ? mvmr_tc_kernel<1, 128, false>
-                                    : mvmr_tc_kernel<0, 128, false>;
+    // (rows are never stored in a call that may do one again)
+    const int mode = (store ? 2 : bulk ? 1 : p.chain > 1 ? 4 : more ? 3 : 0) + (a.only_if.words ? 5 : 0), threads = more ? 256 : 128;
+    static int granted_mvmr[10][64] = {}, regs_mvmr[10] = {};   // per kernel (and device)
+    decltype(&mvmr_tc_kernel<0, 128, false, false>) const kernels[10] = {
+        mvmr_tc_kernel<0, 128, false, false>, mvmr_tc_kernel<1, 128, false, false>, mvmr_tc_kernel<2, 128, false, false>,
+        mvmr_tc_kernel<0, 256, false, false>, mvmr_tc_kernel<0, 256, true, false>,  mvmr_tc_kernel<0, 128, false, true>,
+        mvmr_tc_kernel<1, 128, false, true>,  nullptr,                              mvmr_tc_kernel<0, 256, false, true>,
+        mvmr_tc_kernel<0, 256, true, true>};
+    const auto kernel = kernels[mode];
+    if (!kernel) PCX_FAIL(PCX_E_ARG, "mvmr tensor kernel: no such variant");
     int dev = 0;
     PCX_CUDA(cudaGetDevice(&dev));
     if (int rc = ensure_dynamic_smem(kernel, smem, &granted_mvmr[mode][dev & 63])) return rc;
