@@ -6,10 +6,13 @@
 // layers/triplets.py:431-520) -- but built for latency instead of generality:
 //
 //   * points are binned by a HASH of their cell (side 2R), not by an injective key, so no extent
-//     pass and no key-range hand-over precede the radix sort, and the bucket of a cell is found
+//     pass and no key-range hand-over precede the binning, and the bucket of a cell is found
 //     with one load from a direct table.  Two cells may share a bucket: the foreign points are
 //     ordinary candidates that fail the radius predicate (or the sample check), and the points of
-//     the right cell keep their relative order (the sort is stable), so the output does not change.
+//     the right cell keep their relative order (ascending index), so the output does not change.
+//   * nothing needs the buckets themselves in any order, so the points are not sorted by key: they are
+//     counted per bucket (an atomic addition a point), the buckets are given room as their first points come,
+//     and a point goes as many places behind its bucket's start as the bucket has points of lower index.
 //     The low three bits of the hash are the parities of the cell coordinates, so the eight cells
 //     a query looks at always land in eight different buckets.
 //   * a warp serves four queries: a lane looks up the run of one of their 32 cells (cells the ball does not reach are
@@ -27,8 +30,8 @@
 //     nothing is written and the call reports PCX_E_CAPACITY with the total, so that the caller
 //     can retry with the exact size from the state kept in the workspace.
 #include <cub/block/block_scan.cuh>
-#include <cub/device/device_radix_sort.cuh>
 
+#include <algorithm>
 #include <cfloat>
 #include <cmath>
 
@@ -44,12 +47,16 @@ constexpr int THREADS = QPB * 8;  // one lane per (query, candidate cell)
 constexpr int MAX_K3 = 128;       // taps this path handles (kernel_size 3 and 5)
 constexpr int FOURS = 64;         // fours of candidates that a warp lists at a time
 constexpr int SCAN_THREADS = 1024, SCAN_ITEMS = 4;
+constexpr int BIN_THREADS = 256;
+constexpr int CROWDED = 1024;     // points of a bucket that are put in order by counting the lower ones
 
 struct TapsWs {
-    uint32_t *keys_a, *keys_b;
-    int32_t *vals_a, *vals_b;
-    float4 *sorted_pts;     // xyz + original index (bit pattern) in bucket order
-    int2 *table;            // bucket -> [start, end) in the sorted order; (0,0) = empty
+    uint32_t *keys;         // bucket of a point
+    int32_t *arrival;       // ... and how many of the bucket's points were counted before it
+    int32_t *order;         // the points, bucket by bucket, as they arrived
+    int32_t *crowded;       // buckets with more than CROWDED points
+    float4 *sorted_pts;     // xyz + original index (bit pattern), bucket by bucket, ascending inside a bucket
+    int2 *table;            // bucket -> (start, points); 0 points = empty
     int32_t *sorted_sample; // sample ids in bucket order
     int32_t *kept_point;    // Q x kept: the accepted points of a query, in output order
     uint8_t *kept_tap;      // ... and their taps
@@ -58,9 +65,7 @@ struct TapsWs {
     unsigned long long *tap_total;  // k3
     int64_t *seg;           // k3 + 1
     int64_t *ctrl;          // [0] total pairs, [1] a tap's count does not fit 31 bits, [2] taps scanned,
-                            // [3] queries without a neighbour
-    void *cub_tmp;
-    size_t cub_bytes;
+                            // [3] queries without a neighbour, [4] points given room, [5] crowded buckets
     int bits;
     int64_t buckets, nblocks;
 };
@@ -70,14 +75,11 @@ struct TapsWs {
 // 75 neighbours there; the runs of a warp with a longer list are walked again.
 int kept_per_query(int k3) { return k3 <= 27 ? 64 : 128; }
 
+// Two to four buckets a point: a cell of side 2R holds several points, so that most buckets stay empty and few cells share one.
 int bucket_bits(int64_t P) {
     int b = 1;
     while (((int64_t)1 << b) < P) ++b;
     b += 1;
-    // The radix sort takes eight bits a pass: where two or three bits too many would cost a third pass (18 us of the
-    // search at 100 000 points), fewer buckets do -- a cell of side 2R holds several points, so that even then
-    // less than half of the buckets are taken.
-    if (b > 16 && b <= 18) b = 16;
     return b < 8 ? 8 : (b > 28 ? 28 : b);
 }
 
@@ -90,10 +92,10 @@ size_t carve_taps(void *ws, int64_t P, int64_t Q, int k3, TapsWs *out) {
     w.ctrl = c.take<int64_t>(8);
     w.tap_total = c.take<unsigned long long>(k3);
     w.seg = c.take<int64_t>(k3 + 1);
-    w.keys_a = c.take<uint32_t>(P);
-    w.keys_b = c.take<uint32_t>(P);
-    w.vals_a = c.take<int32_t>(P);
-    w.vals_b = c.take<int32_t>(P);
+    w.keys = c.take<uint32_t>(P);
+    w.arrival = c.take<int32_t>(P);
+    w.order = c.take<int32_t>(P);
+    w.crowded = c.take<int32_t>(P / CROWDED + 1);
     w.sorted_pts = c.take<float4>(P);
     w.table = c.take<int2>(w.buckets);
     w.sorted_sample = c.take<int32_t>(P);
@@ -101,10 +103,6 @@ size_t carve_taps(void *ws, int64_t P, int64_t Q, int k3, TapsWs *out) {
     w.kept_tap = c.take<uint8_t>(Q * kept_per_query(k3));
     w.counts = c.take<uint32_t>(Q);
     w.block_hist = c.take<uint32_t>(w.nblocks * k3);
-    w.cub_bytes = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, w.cub_bytes, (const uint32_t *)nullptr, (uint32_t *)nullptr,
-                                    (const int32_t *)nullptr, (int32_t *)nullptr, P);
-    w.cub_tmp = c.take<char>(w.cub_bytes);
     if (out) *out = w;
     return c.off;
 }
@@ -116,31 +114,96 @@ __device__ __forceinline__ uint32_t cell_bucket(int b, int cx, int cy, int cz, u
     return ((h << 3) | ((uint32_t)(cx & 1) << 2) | ((uint32_t)(cy & 1) << 1) | (uint32_t)(cz & 1)) & mask;
 }
 
-__global__ void taps_key_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, int64_t P,
-                                float inv, uint32_t mask, uint32_t *keys, int32_t *vals, int2 *table, int64_t *ctrl) {
+// Binning, five kernels: every bucket empty; bucket of every point and its turn there; room for the buckets; the points
+// bucket by bucket; ascending inside them.  The turn depends on which atomic addition came first, the result does not.
+//
+// Bound by launches and latency up to some 200 000 points, then by the random accesses.  Before, the keys went through a
+// library's radix sort (two or three passes of 23 to 150 blocks, nine launches): 150 000 points 77 -> 23 us, a million 100 -> 52.
+__global__ void taps_clear_kernel(int4 *table, int64_t pairs, int64_t *ctrl) {
     start_after_previous();
-    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, threads = (int64_t)gridDim.x * blockDim.x;
-    for (int64_t t = p; t <= (int64_t)mask; t += threads) table[t] = make_int2(0, 0);   // every bucket empty
-    if (p < 8) ctrl[p] = 0;
-    if (p >= P) return;
-    keys[p] = cell_bucket(sample ? sample[p] : 0, cell_of(pts[3 * p], inv), cell_of(pts[3 * p + 1], inv),
-                          cell_of(pts[3 * p + 2], inv), mask);
-    vals[p] = (int32_t)p;
+    const int64_t t0 = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, threads = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t t = t0; t < pairs; t += threads) table[t] = make_int4(0, 0, 0, 0);
+    if (t0 < 8) ctrl[t0] = 0;
 }
 
-// Sorted copy of the points and the bucket table in one pass over the sorted keys.
-__global__ void taps_table_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, const uint32_t *__restrict__ keys,
-                                  const int32_t *__restrict__ perm, int64_t P, float4 *sorted_pts, int32_t *sorted_sample,
-                                  int2 *table) {
+__global__ void __launch_bounds__(BIN_THREADS) taps_key_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, int64_t P,
+                                                               float inv, uint32_t mask, uint32_t *keys, int32_t *arrival, int2 *table) {
     start_after_previous();
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (p >= P) return;
+    const uint32_t key = cell_bucket(sample ? sample[p] : 0, cell_of(pts[3 * p], inv), cell_of(pts[3 * p + 1], inv),
+                                     cell_of(pts[3 * p + 2], inv), mask);
+    keys[p] = key;
+    arrival[p] = atomicAdd(&table[key].y, 1);
+}
+
+// The first to arrive takes room for its bucket: buckets lie in the order of their points' blocks, an addition a block.
+__global__ void __launch_bounds__(BIN_THREADS) taps_room_kernel(const uint32_t *__restrict__ keys, const int32_t *__restrict__ arrival, int64_t P,
+                                                                int2 *table, int32_t *crowded, int64_t *ctrl) {
+    start_after_previous();
+    using Scan = cub::BlockScan<int32_t, BIN_THREADS>;
+    __shared__ typename Scan::TempStorage tmp;
+    __shared__ int32_t s_first;
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const bool takes = p < P && arrival[p] == 0;
+    const uint32_t key = takes ? keys[p] : 0u;
+    const int32_t points = takes ? table[key].y : 0;
+    int32_t at, all;
+    Scan(tmp).ExclusiveSum(points, at, all);
+    if (threadIdx.x == 0) s_first = all ? (int32_t)atomicAdd((unsigned long long *)&ctrl[4], (unsigned long long)all) : 0;
+    __syncthreads();
+    if (takes) table[key].x = s_first + at;
+    if (points > CROWDED) crowded[atomicAdd((unsigned long long *)&ctrl[5], 1ULL)] = (int32_t)key;
+}
+
+__global__ void __launch_bounds__(BIN_THREADS) taps_order_kernel(const uint32_t *__restrict__ keys, const int32_t *__restrict__ arrival, int64_t P,
+                                                                 const int2 *__restrict__ table, int32_t *order) {
+    start_after_previous();
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (p < P) order[table[keys[p]].x + arrival[p]] = (int32_t)p;
+}
+
+__global__ void __launch_bounds__(BIN_THREADS) taps_place_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample,
+                                                                 const uint32_t *__restrict__ keys, const int32_t *__restrict__ order, int64_t P,
+                                                                 const int2 *__restrict__ table, const int32_t *__restrict__ crowded,
+                                                                 const int64_t *__restrict__ ctrl, float4 *sorted_pts, int32_t *sorted_sample) {
+    start_after_previous();
+    auto put = [&](int32_t p, int32_t at) {
+        sorted_pts[at] = make_float4(pts[3 * (int64_t)p], pts[3 * (int64_t)p + 1], pts[3 * (int64_t)p + 2], __int_as_float(p));
+        if (sample) sorted_sample[at] = sample[p];
+    };
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s >= P) return;
-    const int32_t p = perm[s];
-    sorted_pts[s] = make_float4(pts[3 * (int64_t)p], pts[3 * (int64_t)p + 1], pts[3 * (int64_t)p + 2], __int_as_float(p));
-    if (sample) sorted_sample[s] = sample[p];
-    const uint32_t key = keys[s];
-    if (s == 0 || keys[s - 1] != key) table[key].x = (int)s;
-    if (s + 1 == P || keys[s + 1] != key) table[key].y = (int)(s + 1);
+    if (s < P) {
+        const int32_t p = order[s];
+        const int2 run = table[keys[p]];
+        if (run.y <= CROWDED) {
+            int32_t lower = 0;
+#pragma unroll 4
+            for (int t = 0; t < run.y; ++t) lower += order[run.x + t] < p;
+            put(p, run.x + lower);
+        }
+    }
+    // Crowded buckets, a block each: all points are gone through in order.  There are at most P / CROWDED of them; a
+    // million points in buckets of 1500 take 1 ms.
+    const int64_t n = ctrl[5];
+    for (int64_t x = blockIdx.x; x < n; x += gridDim.x) {
+        using Scan = cub::BlockScan<int32_t, BIN_THREADS>;
+        __shared__ typename Scan::TempStorage tmp;
+        const uint32_t key = (uint32_t)crowded[x];
+        int32_t at = table[key].x;
+        for (int64_t first = 0; first < P; first += 4 * BIN_THREADS) {
+            const int64_t p = first + 4 * (int64_t)threadIdx.x;
+            int32_t mine[4], before, all;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) mine[u] = p + u < P && keys[p + u] == key;
+            Scan(tmp).ExclusiveSum(mine[0] + mine[1] + mine[2] + mine[3], before, all);
+            before += at, at += all;
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (mine[u]) put((int32_t)(p + u), before++);
+            __syncthreads();
+        }
+    }
 }
 
 struct TapArgs {
@@ -198,8 +261,7 @@ __device__ __forceinline__ int2 run_of(const TapArgs &a, float qx, float qy, flo
         const float gx = gap(qx, cx), gy = gap(qy, cy), gz = gap(qz, cz);
         if (gx * gx + gy * gy + gz * gz > a.reach && far < 0x1p30f) return make_int2(0, 0);
     }
-    const int2 r = a.table[cell_bucket(b, cx, cy, cz, a.mask)];
-    return make_int2(r.x, r.y - r.x);
+    return a.table[cell_bucket(b, cx, cy, cz, a.mask)];
 }
 
 struct Four {
@@ -633,12 +695,19 @@ int pcx_radius_taps_count(const float *d_points, const float *d_queries, const i
     if ((uintptr_t)d_ws % 256) PCX_FAIL(PCX_E_ALIGN, "pcx_radius_taps_count: workspace must be 256-byte aligned");
     const float inv = (float)(1.0 / (2.0 * radius));
     const uint32_t mask = (uint32_t)(w.buckets - 1);
-    const unsigned pblocks = (unsigned)((P + 255) / 256);
-    launch_after(taps_key_kernel, pblocks, 256, 0, stream, d_points, d_point_sample, P, inv, mask, w.keys_a, w.vals_a, w.table, w.ctrl);
+    const unsigned pblocks = (unsigned)((P + BIN_THREADS - 1) / BIN_THREADS);
+    const int64_t pairs = w.buckets / 2;
+    launch_after(taps_clear_kernel, (unsigned)std::min<int64_t>((pairs + BIN_THREADS - 1) / BIN_THREADS, 8 * num_sms()), BIN_THREADS, 0, stream,
+                 reinterpret_cast<int4 *>(w.table), pairs, w.ctrl);
     PCX_LAUNCH_CHECK();
-    size_t tmp = w.cub_bytes;
-    PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, tmp, w.keys_a, w.keys_b, w.vals_a, w.vals_b, P, 0, w.bits, stream));
-    launch_after(taps_table_kernel, pblocks, 256, 0, stream, d_points, d_point_sample, w.keys_b, w.vals_b, P, w.sorted_pts, w.sorted_sample, w.table);
+    launch_after(taps_key_kernel, pblocks, BIN_THREADS, 0, stream, d_points, d_point_sample, P, inv, mask, w.keys, w.arrival, w.table);
+    PCX_LAUNCH_CHECK();
+    launch_after(taps_room_kernel, pblocks, BIN_THREADS, 0, stream, w.keys, w.arrival, P, w.table, w.crowded, w.ctrl);
+    PCX_LAUNCH_CHECK();
+    launch_after(taps_order_kernel, pblocks, BIN_THREADS, 0, stream, w.keys, w.arrival, P, w.table, w.order);
+    PCX_LAUNCH_CHECK();
+    launch_after(taps_place_kernel, pblocks, BIN_THREADS, 0, stream, d_points, d_point_sample, w.keys, w.order, P, w.table, w.crowded, w.ctrl,
+                 w.sorted_pts, w.sorted_sample);
     PCX_LAUNCH_CHECK();
     TapArgs a = make_args(w, d_queries, d_point_sample, d_query_sample, Q, radius, distance_type, kernel_size, kernel_grid_size);
     a.num_neighbors = d_num_neighbors;

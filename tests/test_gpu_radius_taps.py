@@ -275,3 +275,22 @@ def test_long_lists_among_short_ones(long, k):
     ref, got = _both(pts, qry, None, None, 0.05, k, 0.02)
     _assert_same(ref, got)
     assert int(got[4].max()) > long // 2 and int(got[4].min()) == 0
+
+
+@pytest.mark.parametrize("crowd", [(1023,), (1024,), (1025, 1024, 3), (5000, 1, 2049, 700)])
+def test_crowded_cells_keep_their_points_in_order(crowd):
+    """Up to 1024 points of a bucket are ordered by counting, more by going through all points; the order of the points
+    inside a cell decides the order of the pairs."""
+    from pointelligence_b200 import _cabi
+
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(sum(crowd))
+    pts = torch.cat([torch.rand(n, 3, device=dev, generator=g) * 0.19 + 0.005 + 0.6 * c for c, n in enumerate(crowd)])
+    pts = torch.cat([pts, torch.rand(3000, 3, device=dev, generator=g) * 4.0 - 1.0])
+    pts = pts[torch.randperm(pts.shape[0], device=dev, generator=g)].contiguous()
+    qry = pts[::17].contiguous()
+    _cabi._TAPS_RATIO.clear()
+    for _ in range(2):      # counted, then with a capacity from the first
+        _assert_same(*_both(pts, qry, None, None, 0.1, 3, 0.08))
+    smp = torch.arange(pts.shape[0], device=dev) // ((pts.shape[0] + 2) // 3)
+    _assert_same(*_both(pts, qry, smp, smp[::17].contiguous(), 0.1, 3, 0.08))
