@@ -16,9 +16,25 @@ namespace pcx {
 
 void set_error(const char *fmt, ...);
 extern std::atomic<long long> g_launches;               // kernels launched by this library
-// Where a host hand-over (an asynchronous copy and a wait for the stream, in one call) puts its words.
+// Where a host hand-over (a copy or stores of a kernel, and a wait, in one call) puts its words.
 constexpr int HANDOVER_WORDS = 16;
 int64_t *handover_words();
+
+// A hand-over by stores: a kernel puts its words and then the ticket where the host reads them, and the host waits for the
+// ticket, not for the kernel's end.  Against two copies and a wait for the stream: some 20 us less
+// a search; with the host free while the pairs are written, a rulebook of 150 000 points 211 -> 128 us, binning included.
+struct HandOver {
+    int64_t *words = nullptr;   // page-locked; null where there is none: the host copies after the kernel's end
+    int64_t ticket = 0;
+    static constexpr int TICKET = HANDOVER_WORDS - 1;
+    __device__ __forceinline__ void put(int n, int64_t v) const { *(volatile int64_t *)(words + n) = v; }
+    __device__ __forceinline__ void done() const {
+        __threadfence_system();
+        *(volatile int64_t *)(words + TICKET) = ticket;
+    }
+};
+HandOver new_hand_over();                                        // of this thread: one at a time
+int wait_for_hand_over(const HandOver &h, cudaStream_t stream);
 void prof_begin(const char *name, cudaStream_t stream); // event timer around a dominant kernel
 void prof_end(cudaStream_t stream);
 

@@ -220,6 +220,8 @@ struct TapArgs {
     const int64_t *seg, *ctrl;
     int64_t *ctrl_rw;
     int32_t *out_i, *out_j, *out_k;
+    HandOver host;                  // fill pass: ctrl[0 .. 3] and the device status word
+    const unsigned int *status;
     int64_t Q, nblocks, capacity;
     uint32_t mask;
     float r32, inv, g32, inv_g, s_max, cell, reach;   // cell: side of a cell; reach: square of the radius, with a margin
@@ -487,6 +489,11 @@ __global__ void __launch_bounds__(THREADS, REC_MAX > 1024 ? 4 : 5) taps_fill_ker
     extern __shared__ __align__(16) uint16_t s_cnt[];       // [tap][query]: pairs, then those of the queries before (32-bit words, too)
     __shared__ uint32_t s_base[MAX_K3];                     // next write position of each tap for this block
     __shared__ uint32_t s_start[MAX_K3], s_total[MAX_K3];   // first place of each tap among the sorted, its pairs in this round
+    if (blockIdx.x == 0 && threadIdx.x == 0 && a.host.words) {   // all there is to hand over is known before this pass
+        for (int n = 0; n < 4; ++n) a.host.put(n, a.ctrl[n]);
+        a.host.put(4, *(const volatile unsigned int *)a.status);
+        a.host.done();
+    }
     const bool fits = a.ctrl[0] <= a.capacity && !a.ctrl[1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int c = threadIdx.x & 7, ql = threadIdx.x >> 3;
@@ -748,7 +755,11 @@ int pcx_radius_taps_fill(const float *d_queries, const int32_t *d_point_sample, 
     if (ws_bytes < need) PCX_FAIL(PCX_E_CAPACITY, "pcx_radius_taps_fill: workspace %zu < %zu bytes", ws_bytes, need);
     TapArgs a = make_args(w, d_queries, d_point_sample, d_query_sample, Q, radius, distance_type, kernel_size, kernel_grid_size);
     a.out_i = d_out_i, a.out_j = d_out_j, a.out_k = d_out_k, a.capacity = capacity;
+    int64_t *h = handover_words();
     if (capacity > 0) {
+        unsigned int *status = nullptr;
+        if (int rc = device_status_address(&status)) return rc;
+        a.host = new_hand_over(), a.status = status;
         prof_begin("taps_fill_kernel", stream);
         const auto kernel = k3 <= 27 ? (fused(a) ? taps_fill_kernel<true, 1024> : taps_fill_kernel<false, 1024>)
                                      : (fused(a) ? taps_fill_kernel<true, 1536> : taps_fill_kernel<false, 1536>);
@@ -756,8 +767,7 @@ int pcx_radius_taps_fill(const float *d_queries, const int32_t *d_point_sample, 
         prof_end(stream);
         PCX_LAUNCH_CHECK();
     }
-    int64_t *h = handover_words();
-    if (int rc = read_ctrl(w, h, stream)) return rc;
+    if (int rc = a.host.words ? wait_for_hand_over(a.host, stream) : read_ctrl(w, h, stream)) return rc;
     h_total[0] = h[0], h_total[1] = h[3], h_total[2] = h[4];
     if (h[1] || h[0] > INT32_MAX) PCX_FAIL(PCX_E_UNSUPPORTED, "prepared kernel-segment output currently requires fewer than 2^31 edges; got %lld", (long long)h[0]);
     if (h[0] > capacity) PCX_FAIL(PCX_E_CAPACITY, "pcx_radius_taps_fill: %lld pairs do not fit the capacity of %lld; nothing was written", (long long)h[0], (long long)capacity);

@@ -20,22 +20,53 @@ void set_error(const char *fmt, ...) {
 std::atomic<long long> g_launches{0};
 
 namespace {
-struct HandOver {   // page-locked, one per thread: copies into it neither stage nor block the stream
+struct Words {   // page-locked, one set per thread: copies into it neither stage nor block the stream
     int64_t *words = nullptr;
     int64_t pageable[HANDOVER_WORDS];
-    ~HandOver() {
+    int64_t tickets = 0;
+    ~Words() {
         if (words && words != pageable) cudaFreeHost(words);
     }
 };
+Words &this_threads_words() {
+    static thread_local Words h;
+    if (!h.words) {
+        if (cudaHostAlloc((void **)&h.words, HANDOVER_WORDS * sizeof(int64_t), cudaHostAllocPortable) != cudaSuccess) {
+            (void)cudaGetLastError();
+            h.words = h.pageable;
+        }
+        h.words[HandOver::TICKET] = 0;
+    }
+    return h;
+}
 }  // namespace
 
-int64_t *handover_words() {
-    static thread_local HandOver h;
-    if (!h.words && cudaHostAlloc((void **)&h.words, HANDOVER_WORDS * sizeof(int64_t), cudaHostAllocPortable) != cudaSuccess) {
-        (void)cudaGetLastError();
-        h.words = h.pageable;
+int64_t *handover_words() { return this_threads_words().words; }
+
+HandOver new_hand_over() {
+    Words &w = this_threads_words();
+    HandOver h;
+    if (w.words != w.pageable) h.words = w.words;
+    h.ticket = ++w.tickets;
+    return h;
+}
+
+int wait_for_hand_over(const HandOver &h, cudaStream_t stream) {
+    const volatile int64_t *ticket = h.words + HandOver::TICKET;
+    for (bool ended = false;;) {
+        for (int n = 0; n < 1000; ++n) {
+            if (*ticket == h.ticket) {
+                std::atomic_thread_fence(std::memory_order_acquire);
+                return PCX_OK;
+            }
+            __builtin_ia32_pause();
+        }
+        if (ended) PCX_FAIL(PCX_E_LAUNCH, "a kernel ended without its hand-over");
+        const cudaError_t e = cudaStreamQuery(stream);   // (so that a failed launch ends the wait)
+        if (e == cudaErrorNotReady) (void)cudaGetLastError();
+        else if (e != cudaSuccess) PCX_FAIL(PCX_E_LAUNCH, "waiting for a kernel failed: %s", cudaGetErrorString(e));
+        else ended = true;
     }
-    return h.words;
 }
 
 struct ProfRecord {
