@@ -250,6 +250,23 @@ int pcx_mvmr_split(const void *d_weight, const void *d_feat,
                    int group_blocks, int64_t multi_buckets, void *d_ws,
                    size_t ws_bytes, void *stream);
 
+/* pcx_mvmr_bias for layers of few input channels (fp16 / bf16, one group, a
+ * contraction of at most 8 channels, at most 512 taps and 1024 output
+ * channels, 0 < T < 2^27 - 1) on a rulebook whose output rows ascend inside every
+ * tap, as the searches write them (nothing checks it: where they do not, triplets
+ * are left out).  The sums of a row stay on the chip, operands are multiplied as
+ * they are and a row is rounded once.  Weights that are not finite are worked off
+ * triplet by triplet, slowly.  Features and weights may lie at any address of
+ * their type. */
+size_t pcx_mvmr_thin_workspace_bytes(int64_t n_feat, int64_t n_out, int K,
+                                     int C, int M, int transpose);
+int pcx_mvmr_thin(const void *d_weight, const void *d_feat,
+                  const int32_t *d_gather, const int32_t *d_scatter,
+                  const int64_t *d_seg_offs, const void *d_bias, void *d_out,
+                  int64_t T, int64_t n_feat, int64_t n_out, int K, int C, int M,
+                  int flags, int dtype, void *d_ws, size_t ws_bytes,
+                  void *stream);
+
 /* Launches one thread that waits on a barrier nothing arrives at: the bounded
  * wait gives up after limit_ns (at most 100 ms), sets bit 8 of the device
  * status word and the kernel returns.  For tests of the status path; no

@@ -66,6 +66,8 @@ SIGNATURES = {
     "pcx_mvmr_planned_scratch_bytes": (c_size_t, [c_int64, c_int, c_int64, c_int, c_int, c_int]),
     "pcx_mvmr_planned_bias": (c_int, [c_void_p] * 3 + [c_size_t] + [c_void_p] * 2 + [c_int64] * 3 + [c_int] * 7
                               + [c_int64, c_void_p, c_size_t, c_void_p]),
+    "pcx_mvmr_thin_workspace_bytes": (c_size_t, [c_int64] * 2 + [c_int] * 4),
+    "pcx_mvmr_thin": (c_int, [c_void_p] * 7 + [c_int64] * 3 + [c_int] * 5 + [c_void_p, c_size_t, c_void_p]),
     "pcx_mvmr_split_workspace_bytes": (c_size_t, [c_int64, c_int64] + [c_int] * 5),
     "pcx_mvmr_split": (c_int, [c_void_p] * 6 + [c_size_t] + [c_void_p] * 2 + [c_int64] * 3 + [c_int] * 6
                        + [c_int64, c_void_p, c_size_t, c_void_p]),
@@ -158,7 +160,7 @@ def host():
         except ImportError as exc:
             raise RuntimeError("pointelligence_b200/lib/_pcx_host.so is missing or does not load: build it with "
                                f"`python -m pointelligence_b200.build` ({exc})") from exc
-        _pcx_host.set_hooks(_plan_hook, is_symmetric, _differentiable_backward)
+        _pcx_host.set_hooks(_plan_hook, is_symmetric, _rows_ascend, _differentiable_backward)
         from .sparse_engines._dispatch_override import current_engine
 
         _pcx_host.set_engine(current_engine())

@@ -19,7 +19,6 @@ from typing import List, Sequence, Tuple
 
 import torch
 import torch.nn as nn
-import torch.nn.functional as F
 from torch import Tensor
 
 from . import _cabi
@@ -32,27 +31,14 @@ from .layers.triplets import (build_triplets_segmented, handle_stride_and_build_
 RFS = 2.5   # receptive_field_scaler of every convolution, as in the reference's model
 
 
-def _pad_to(n, multiple=16):
-    return (n + multiple - 1) // multiple * multiple
-
-
 class Bf16PointConv3d(PointConv3d):
     """``PointConv3d`` with bf16 operands: the fp32 master weight is cast on the fly and the
-    input is taken as bf16.  Channel counts that are not multiples of 16 (the 3-channel input,
-    the class logits) are zero-padded so that they take the tensor-core engine as well; the
-    padding carries no gradient."""
+    input is taken as bf16."""
 
     def forward(self, input, i, j, k, n, contract=None, seg_offs=None):
         w = self.weight.to(torch.bfloat16)
-        K, G, C, M = w.shape
-        Cp, Mp = _pad_to(C), _pad_to(M)
         x = input.to(torch.bfloat16)
-        if (Cp, Mp) != (C, M):
-            w = F.pad(w, (0, Mp - M, 0, Cp - C))
-            x = F.pad(x, (0, Cp - C))
         out = self._conv_forward(x, i, j, k, n, w, None, contract=contract, seg_offs=seg_offs)
-        if Mp != M:
-            out = out.view(n, -1)[:, :M]
         if self.bias is not None:
             out = out + self.bias.to(out.dtype)
         return out

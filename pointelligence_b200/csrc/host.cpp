@@ -26,6 +26,7 @@ namespace {
 // ------------------------------------------------------------------ helpers ----
 PyObject *g_plan_hook = nullptr;       // (scatter, gather, seg, K, n_out, out_width, in_width, forced, split, capturing) -> None | plan tuple
 PyObject *g_symmetric_hook = nullptr;  // (i, j, K) -> bool
+PyObject *g_ascending_hook = nullptr;  // (scatter, gather, seg, K) -> bool: rows are known to ascend inside every tap
 PyObject *g_double_backward = nullptr; // differentiable backward of the convolution (create_graph)
 
 [[noreturn]] void raise(PyObject *type, const std::string &msg) {
@@ -184,6 +185,30 @@ Tensor mvmr_split(const Tensor &weight, const Tensor &feat, const Tensor &gather
     return out;
 }
 
+// Layers of up to 8 channels of the contraction on rulebooks of the geometry path (pcx_mvmr_thin: rows known to ascend
+// inside every tap).  That kernel's time goes with the (128 rows x 8 taps x 64 output channels) it multiplies, 8 to 16 ns each,
+// the scatter kernel's with the fp32 sums it adds, 2.2 to 3.3 TB/s: taken from 26 000 bytes of sums for each.  Measured, scatter
+// (with its padded copies) / this, us, and the bytes:
+//
+//   27 taps    20 000 rows, 1.7 a row    -> 32  18 / 27 (7 000)     -> 64  21 / 29 (14 000)    -> 256  35 / 42 (14 000)
+//             150 000, 6.4                      70 / 61 (26 000)           90 / 70 (53 000)           437 / 192 (53 000)
+//              40 000, 16.4                     49 / 47 (67 000)           59 / 51 (134 000)          252 / 99 (134 000)
+//             600 000, 22.6                    649 / 319 (93 000)         871 / 356 (185 000)
+//   125 taps   80 000, 11.2                     63 / 99 (11 500)           76 / 106 (23 000)          336 / 286 (23 000)
+//              80 000, 23.4                    104 / 128 (24 000)         131 / 136 (48 000)          652 / 381 (48 000)
+//             150 000, 20.0                    154 / 176 (21 000)         195 / 188 (41 000)         1088 / 611 (41 000)
+bool thin_pays(at::ScalarType dtype, int64_t T, int64_t n_in, int64_t n_out, int64_t K, int64_t G, int64_t inw, int64_t outw) {
+    if (!is_half(dtype) || G != 1 || K <= 1 || K > 512 || inw <= 0 || inw > 8 || outw <= 0 || outw > 1024 || T <= 0 || T >= (int64_t(1) << 27) - 1 ||
+        n_in <= 0 || n_out <= 0)
+        return false;
+    const int64_t products = ((n_out + 127) / 128) * ((K + 7) / 8) * ((outw + 63) / 64);
+    return products < (int64_t(1) << 31) && T * outw * 4 >= 26000 * products;
+}
+bool rows_ascend(const Tensor &scatter, const Tensor &gather, const Tensor &seg, int64_t K) {
+    py::gil_scoped_acquire gil;
+    return py::cast<bool>(py::reinterpret_borrow<py::object>(g_ascending_hook)(scatter, gather, seg, K));
+}
+
 // out[scatter[t]] += feat[gather[t]] @ W[tap(t)] (+ bias).  flags: 1 = W transposed, 2 = taps of the weight
 // in reverse order.  Rows of the result are (G * out width) in feat's type.
 Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor &scatter_, const OptTensor &seg_,
@@ -199,6 +224,16 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
     const bool transpose = flags & 1;
     const int64_t inw = transpose ? M : C, outw = transpose ? C : M, T = gather_.numel();
     c10::cuda::CUDAGuard guard(feat.device());
+    if (engine == 0 && seg_ && thin_pays(feat.scalar_type(), T, feat.size(0), n_out, K, G, inw, outw) &&
+        // (a captured pass is replayed on whatever the index tensors hold then: on the kernels that take any order)
+        c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None && rows_ascend(scatter_, gather_, *seg_, K)) {
+        const Tensor gather = as_i32(gather_), scatter = as_i32(scatter_), seg = as_i64(*seg_);
+        Tensor out = at::empty({n_out, outw}, feat.options());
+        Tensor ws = workspace(pcx_mvmr_thin_workspace_bytes(feat.size(0), n_out, (int)K, (int)C, (int)M, transpose), feat);
+        check(pcx_mvmr_thin(ptr(weight), ptr(feat), ptr_as<int32_t>(gather), ptr_as<int32_t>(scatter), ptr_as<int64_t>(seg), ptr(bias), ptr(out),
+                            T, feat.size(0), n_out, (int)K, (int)C, (int)M, flags, code, ptr(ws), ws.numel(), stream()));
+        return out;
+    }
     if ((engine & 0xff) == 0 && is_half(feat.scalar_type()) && seg_ && T > 0 && n_out > 0 && K <= 1024 && G <= 64 &&
         (C != padded(C) || M != padded(M))) {
         // channel counts the tensor engines do not take (the 3 or 6 channels of an input, 20 classes): zero columns make
@@ -627,9 +662,10 @@ void record_streams(const std::vector<Tensor> &tensors) {
         if (t.is_cuda()) t.record_stream(c10::cuda::getCurrentCUDAStream(t.device().index()).unwrap());
 }
 
-void set_hooks(py::object plan, py::object symmetric, py::object double_backward) {
+void set_hooks(py::object plan, py::object symmetric, py::object ascending, py::object double_backward) {
     g_plan_hook = plan.release().ptr();
     g_symmetric_hook = symmetric.release().ptr();
+    g_ascending_hook = ascending.release().ptr();
     g_double_backward = double_backward.release().ptr();
 }
 

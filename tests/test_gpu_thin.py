@@ -1,0 +1,135 @@
+"""Layers of few input channels (``pcx_mvmr_thin``) against fp64, over the sizes where its tiles end."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+# one rounding of the result: at most the type's unit roundoff in every element, and so in the norm; sums in fp32 are below
+BOUND = {torch.bfloat16: 2.0 ** -8 * 0.5 * 1.01, torch.float16: 2.0 ** -11 * 1.01}
+
+
+def _rulebook(n_out, n_in, K, ratio, seed, empty=()):
+    """Tap-sorted, rows ascending inside a tap, with (row, tap) buckets of several triplets."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    T = max(int(n_out * ratio), 1)
+    i = torch.randint(0, n_out, (T,), device="cuda", generator=g)
+    j = torch.randint(0, n_in, (T,), device="cuda", generator=g)
+    k = torch.randint(0, K, (T,), device="cuda", generator=g)
+    for e in empty:
+        k = torch.where(k == e, (e + 1) % K, k)
+    order = torch.argsort(k * n_out + i, stable=True)
+    i, j, k = i[order], j[order], k[order]
+    seg = torch.searchsorted(k.contiguous(), torch.arange(K + 1, device="cuda"))
+    return i.int().contiguous(), j.int().contiguous(), k, seg
+
+
+def _exact(w, x, i, j, k, n_out):
+    out = torch.zeros(n_out, w.shape[-1], dtype=torch.float64, device="cuda")
+    for tap in range(w.shape[0]):
+        t = k == tap
+        if bool(t.any()):
+            out.index_add_(0, i[t].long(), x[j[t].long()].double() @ w[tap].double())
+    return out
+
+
+def _thin(weight, feat, i, j, seg, bias, n_out, flags=0):
+    from pointelligence_b200 import _cabi
+
+    K, C, M = weight.shape
+    width = C if flags & 1 else M
+    out = torch.full((n_out, width), float("nan"), device="cuda", dtype=feat.dtype)
+    L, ptr = _cabi.lib(), _cabi.ptr
+    ws = _cabi.workspace(L.pcx_mvmr_thin_workspace_bytes(feat.shape[0], n_out, K, C, M, flags & 1), feat.device)
+    _cabi.check(L.pcx_mvmr_thin(ptr(weight), ptr(feat), ptr(j), ptr(i), ptr(seg), ptr(bias), ptr(out), i.numel(), feat.shape[0],
+                                n_out, K, C, M, flags, _cabi.dtype_code(feat.dtype), ptr(ws), ws.numel(), _cabi.stream_ptr()))
+    return out
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm().clamp_min(1e-300))
+
+
+@pytest.mark.parametrize("n_out,K,C,M,ratio,empty", [
+    (1, 2, 1, 16, 1.0, ()), (127, 8, 8, 16, 3.0, ()), (128, 9, 3, 32, 4.0, (0,)), (129, 27, 3, 20, 6.0, (0, 13, 26)),
+    (1000, 27, 6, 64, 40.0, ()), (5000, 125, 6, 32, 25.0, (7, 8, 9)), (5000, 125, 8, 48, 25.0, ()), (20000, 27, 7, 96, 6.0, ()),
+    (30000, 27, 2, 256, 5.0, ()), (3000, 27, 4, 3, 200.0, ()), (40001, 125, 5, 72, 3.0, ()), (300, 343, 6, 1000, 30.0, (342,)),
+    (150, 27, 8, 24, 900.0, ())])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_against_fp64(n_out, K, C, M, ratio, empty, dtype):
+    g = torch.Generator(device="cuda").manual_seed(n_out)
+    n_in = n_out + 37
+    i, j, k, seg = _rulebook(n_out, n_in, K, ratio, n_out + K, empty)
+    w = (torch.randn(K, C, M, device="cuda", generator=g) / C ** 0.5).to(dtype)
+    x = torch.randn(n_in, C, device="cuda", generator=g).to(dtype)
+    b = torch.randn(M, device="cuda", generator=g).to(dtype)
+    assert _rel(_thin(w, x, i, j, seg, None, n_out), _exact(w, x, i, j, k, n_out)) <= BOUND[dtype]
+    assert _rel(_thin(w, x, i, j, seg, b, n_out), _exact(w, x, i, j, k, n_out) + b.double()) <= BOUND[dtype]
+    wt, flipped = w.transpose(1, 2).contiguous(), w.flip(0).contiguous()
+    assert _rel(_thin(wt, x, i, j, seg, None, n_out, 1), _exact(w, x, i, j, k, n_out)) <= BOUND[dtype]
+    assert _rel(_thin(flipped, x, i, j, seg, None, n_out, 2), _exact(w, x, i, j, k, n_out)) <= BOUND[dtype]
+
+
+@pytest.mark.parametrize("K,C,M", [(27, 6, 32), (125, 8, 80)])
+def test_odd_addresses_and_operands_that_are_not_finite(K, C, M):
+    from pointelligence_b200 import _cabi
+
+    g = torch.Generator(device="cuda").manual_seed(K)
+    n = 3001
+    i, j, k, seg = _rulebook(n, n, K, 8.0, K)
+    w = (torch.randn(K, C, M, device="cuda", generator=g) / C ** 0.5).bfloat16()
+    x = torch.randn(n, C, device="cuda", generator=g).bfloat16()
+    exact = _exact(w, x, i, j, k, n)
+    # operands that begin at an odd element
+    odd = lambda t: torch.cat([t.new_zeros(1), t.flatten()])[1:].view(t.shape)
+    assert _rel(_thin(odd(w), odd(x), i, j, seg, None, n), exact) <= BOUND[torch.bfloat16]
+    # infinities and NaN reach the rows whose triplets meet them, and no others
+    for spoil_w, spoil_x in ((True, False), (False, True), (True, True)):
+        w2, x2 = w.clone(), x.clone()
+        if spoil_w:
+            w2[5, 1, 3], w2[K - 1, 0, 0] = float("inf"), float("nan")
+        if spoil_x:
+            x2[17, 0], x2[1234, C - 1] = float("nan"), float("-inf")
+        got = _thin(w2, x2, i, j, seg, None, n)
+        ref = _cabi.mvmr(w2.unsqueeze(1), x2, j, i, seg, None, n, False, _cabi.ENGINE_CUDA_CORE)
+        assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got.isinf(), ref.isinf())
+        ok = ref.isfinite()
+        assert _rel(got[ok], ref[ok].double()) <= 2 * BOUND[torch.bfloat16]
+
+
+def test_the_layers_that_take_it():
+    """Rulebooks of the search, forward and, where the rulebook is its own mirror image, the input gradient."""
+    from pointelligence_b200 import _cabi
+    from pointelligence_b200.layers import MetaData, PointConv3d
+
+    pts = torch.rand(20000, 3, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    m = MetaData(points=pts, sample_inds=torch.zeros(len(pts), dtype=torch.int64, device="cuda"),
+                 sample_sizes=torch.tensor([len(pts)], device="cuda"), grid_size=0.025, kernel_size=(5, 5, 5), receptive_field_scaler=2.5)
+    def kernels(call):
+        _cabi.profile_enable(True)
+        out = call()
+        torch.cuda.synchronize()
+        names = [n for n, _ in _cabi.profile_records()]
+        _cabi.profile_enable(False)
+        return out, names
+
+    i, j, k = m.i, m.j, m.k
+    conv = PointConv3d(6, 64, 5, device="cuda", dtype=torch.bfloat16)
+    x = torch.randn(len(pts), 6, device="cuda", dtype=torch.bfloat16)
+    with torch.no_grad():
+        y, names = kernels(lambda: conv(x, i, j, k, len(pts), contract=m.contract, seg_offs=m.seg_offs))
+    assert names == ["mvmr_thin_kernel"]
+    assert _rel(y, _exact(conv.weight[:, 0], x, i, j, k, len(pts)) + conv.bias.double()) <= BOUND[torch.bfloat16]
+    narrow = PointConv3d(64, 6, 5, device="cuda", dtype=torch.float16)
+    x64 = torch.randn(len(pts), 64, device="cuda", dtype=torch.float16, requires_grad=True)
+    z = narrow(x64, i, j, k, len(pts), contract=m.contract, seg_offs=m.seg_offs)
+    go = torch.randn_like(z)
+    (gx,), names = kernels(lambda: torch.autograd.grad(z, (x64,), go))
+    assert names == ["mvmr_thin_kernel"]
+    assert _rel(gx, _exact(narrow.weight[:, 0].transpose(1, 2), go, j, i, k, len(pts))) <= BOUND[torch.float16]
+    with torch.no_grad():
+        few = PointConv3d(6, 4, 5, device="cuda", dtype=torch.bfloat16)      # too few sums to save
+        _, names = kernels(lambda: few(x, i, j, k, len(pts), contract=m.contract, seg_offs=m.seg_offs))
+        assert "mvmr_thin_kernel" not in names
+        i.add_(0)      # written to since the search: nothing is known about the order
+        _, names = kernels(lambda: conv(x, i, j, k, len(pts), contract=m.contract, seg_offs=m.seg_offs))
+        assert "mvmr_thin_kernel" not in names
