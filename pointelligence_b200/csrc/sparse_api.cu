@@ -208,10 +208,14 @@ int pcx_vvor(const void *d_a, const int32_t *d_a_idx, const void *d_b, const int
     a.acc = dtype == PCX_F32 ? (float *)d_out : w.acc;
     a.chunk_table = w.chunk_table;
     a.T = T, a.n_a = n_a, a.n_b = n_b, a.n_o = n_o, a.G = G, a.Ma = Ma, a.Cb = Cb, a.dtype = dtype;
+    if (force_engine()) engine = force_engine();
+    const bool tensor_ok = T > 0 && vvor_tensor_supported(a);
+    if (engine != PCX_ENGINE_CUDA_CORE && tensor_ok && vvor_stores(a)) {
+        a.out = d_out;
+        return vvor_tensor(a, stream);
+    }
     if (int rc = clear_accumulator(a.acc, nullptr, n_o * G * Ma, Cb, dtype, stream)) return rc;
     if (T > 0) {
-        if (force_engine()) engine = force_engine();
-        bool tensor_ok = vvor_tensor_supported(a);
         if (engine == PCX_ENGINE_TENSOR && !tensor_ok)
             PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_vvor: tensor engine needs fp16/bf16, a sorted output index and channel counts that are multiples of 16 (of 32 beyond 256, of 48 beyond 512 ...)");
         int rc = (engine != PCX_ENGINE_CUDA_CORE && tensor_ok) ? vvor_tensor(a, stream) : vvor_generic(a, stream);

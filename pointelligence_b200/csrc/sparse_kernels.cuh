@@ -29,6 +29,7 @@ struct VvorArgs {
     const int64_t *seg_offs; // (n_o+1) or null
     const int32_t *o_idx;    // (T) when seg_offs is null
     float *acc;              // (n_o, G, Ma, Cb) fp32, zeroed by the caller
+    void *out;               // tensor engine: the output itself, where every tap is completed by one block (acc unused); else null
     int32_t *chunk_table;    // (n_o+1) scratch
     int64_t T, n_a, n_b, n_o;
     int G, Ma, Cb, dtype;
@@ -118,6 +119,7 @@ inline bool splits_evenly(int width) { return width >= 16 && width % (16 * parts
 
 bool mvmr_tensor_supported(const MvmrArgs &a);
 bool vvor_tensor_supported(const VvorArgs &a);
+bool vvor_stores(const VvorArgs &a);   // whether the tensor engine should store rows itself
 int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream);
 int vvor_tensor(const VvorArgs &a, cudaStream_t stream);
 

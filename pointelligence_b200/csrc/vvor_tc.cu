@@ -20,6 +20,9 @@
 // barrier a chunk: 186, 385, 1042 and 42, 76, 178 us.  16 x 16 is 10 % slower than with those (6 of 8 lanes of a copy
 // have nothing to do): 200 000 points, 3.6 M triplets 82 against 73 us.
 //
+// Few triplets a tap (the deep levels of a network): a CTA takes whole taps, rounds what tensor memory holds and stores it
+// (STORE), so that there are no fp32 sums to clear, to add to and to round: the figures stand at vvor_stores().
+//
 // Every wait is bounded (one second) and abortable: a role that gives up raises a flag in the status word and
 // in shared memory, the other roles leave their waits, and the CTA frees its TMEM and returns.
 #include "sparse_kernels.cuh"
@@ -45,6 +48,7 @@ struct VvorTcParams {
     const int32_t *a_idx, *b_idx;
     const int64_t *seg;
     float *acc;             // (n_o, G, rows of Cb)
+    uint16_t *out;          // STORE: the same, rounded
     unsigned int *status;
     int64_t a_pitch, b_pitch, acc_pitch, acc_tap;   // rows of a / b / one tap's sums, elements of one tap's sums
     int a_parts, b_parts;                           // blockIdx.y: (group, part of a, part of b)
@@ -83,7 +87,30 @@ __device__ __forceinline__ void copy_operand(uint32_t tile, const uint16_t *src,
     }
 }
 
-template <int CHR>   // triplets of a chunk: the contraction of one slot
+// 32 rounded columns of a row (those below `left`) from tensor memory, or zeros; the row may begin at any even address
+__device__ __forceinline__ void store_columns(uint16_t *dst, const float *v, int left, int fmt, bool wide) {
+    uint32_t o[16];
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        if (fmt) {
+            const __nv_bfloat162 h = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+            o[e] = *reinterpret_cast<const uint32_t *>(&h);
+        } else {
+            const __half2 h = __floats2half2_rn(v[2 * e], v[2 * e + 1]);
+            o[e] = *reinterpret_cast<const uint32_t *>(&h);
+        }
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {   // (widths are multiples of 16)
+        if (8 * e >= left) continue;
+        if (wide) reinterpret_cast<uint4 *>(dst)[e] = make_uint4(o[4 * e], o[4 * e + 1], o[4 * e + 2], o[4 * e + 3]);
+        else
+#pragma unroll
+            for (int q = 0; q < 8; ++q) dst[8 * e + q] = (uint16_t)(o[4 * e + q / 2] >> (16 * (q & 1)));
+    }
+}
+
+template <int CHR, bool STORE>   // triplets of a chunk: the contraction of one slot
 __global__ void __launch_bounds__(THREADS, 1) vvor_tc_kernel(VvorTcParams p) {
     start_after_previous();
     constexpr uint32_t BLK = CHR * 128;   // one 64-channel block of a tile
@@ -100,7 +127,9 @@ __global__ void __launch_bounds__(THREADS, 1) vvor_tc_kernel(VvorTcParams p) {
                   g = (int)blockIdx.y / (p.b_parts * p.a_parts);
         p.a += ((int64_t)g * p.a_parts + ap) * p.Ma;
         p.b += ((int64_t)g * p.b_parts + bp) * p.Cb;
-        p.acc += ((int64_t)g * p.a_parts + ap) * p.Ma * p.acc_pitch + bp * p.Cb;
+        const int64_t first = ((int64_t)g * p.a_parts + ap) * p.Ma * p.acc_pitch + bp * p.Cb;
+        if (STORE) p.out += first;
+        else p.acc += first;
     }
     const int row_tiles = (p.Ma + 127) >> 7;
     const int ablk = (p.Ma + 63) >> 6, bblk = (p.Cb + 63) >> 6;   // an odd ablk borrows the next block as padding
@@ -133,12 +162,45 @@ __global__ void __launch_bounds__(THREADS, 1) vvor_tc_kernel(VvorTcParams p) {
 
     const int total = s_cum[p.n_o];
     const int per = (total + gridDim.x - 1) / gridDim.x;
-    const int lo = blockIdx.x * per, hi = min(total, lo + per);
+    const int tap0 = STORE ? (int)((int64_t)p.n_o * blockIdx.x / gridDim.x) : 0, tap1 = STORE ? (int)((int64_t)p.n_o * (blockIdx.x + 1) / gridDim.x) : p.n_o;
+    const int lo = STORE ? s_cum[tap0] : blockIdx.x * per, hi = STORE ? s_cum[tap1] : min(total, lo + per);
     Cursor cur;
     if (lo < hi) cur.seek(s_cum, p.seg, p.n_o, lo);
 
-    if (lo >= hi) {
-    } else if (warp < FLUSH_WARPS) {
+    if (STORE && warp < FLUSH_WARPS) {
+        // ----------------------------------------------------------------- store ----
+        Ring acc;
+        const bool wide = ((uintptr_t)p.out & 15) == 0 && p.acc_pitch % 8 == 0;
+        for (int tap = tap0; tap < tap1; ++tap) {
+            const bool none = s_cum[tap + 1] == s_cum[tap];
+            if (!none) {
+                if (!wait(s_acc_full[acc.slot], acc.turn)) break;
+                tc_fence_after();
+            }
+            for (int rt = 0; rt < row_tiles; ++rt) {
+                const int m = rt * 128 + warp * 32 + lane;
+                if (rt * 128 + warp * 32 >= p.Ma) break;
+                uint16_t *dst = p.out + tap * p.acc_tap + m * p.acc_pitch;
+                for (int c0 = 0; c0 < p.Cb; c0 += 32) {
+                    float v[32];
+                    if (none) {
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) v[e] = 0.f;
+                    } else {
+                        tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + acc.slot * p.acc_cols + (uint32_t)(rt * p.Cb + c0), v);
+                    }
+                    if (m < p.Ma) store_columns(dst + c0, v, p.Cb - c0, p.fmt, wide);
+                    __syncwarp();
+                }
+            }
+            if (none) continue;
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&s_acc_empty[acc.slot]));
+            acc.next(p.nacc);
+        }
+    } else if (lo >= hi) {
+    } else if (!STORE && warp < FLUSH_WARPS) {
         // ----------------------------------------------------------------- flush ----
         // a warp reads the 32 TMEM lanes of its quarter
         Ring acc;
@@ -239,7 +301,7 @@ __global__ void __launch_bounds__(THREADS, 1) vvor_tc_kernel(VvorTcParams p) {
     if (warp == 0) tmem_dealloc(tmem, p.ncols);
 }
 
-template <int CHR>
+template <int CHR, bool STORE>
 int launch_vvor(VvorTcParams &p, int parts, int64_t T, size_t block_rows, cudaStream_t stream) {
     const size_t slot = block_rows * CHR * 128;
     const size_t rest = 1024 + 2 * AHEAD * CHR * 4 + align_up((size_t)(p.n_o + 1) * 4, 16);   // alignment, index rings, chunk table
@@ -251,12 +313,12 @@ int launch_vvor(VvorTcParams &p, int parts, int64_t T, size_t block_rows, cudaSt
     int dev = 0;
     PCX_CUDA(cudaGetDevice(&dev));
     if ((int)smem > granted[dev & 63]) {
-        PCX_CUDA(cudaFuncSetAttribute(vvor_tc_kernel<CHR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PCX_CUDA(cudaFuncSetAttribute(vvor_tc_kernel<CHR, STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         granted[dev & 63] = (int)smem;
     }
-    const dim3 grid((unsigned)std::min<int64_t>(T / CHR + p.n_o + 1, std::max(1, num_sms() / parts)), (unsigned)parts);
+    const dim3 grid((unsigned)std::min<int64_t>(STORE ? p.n_o : T / CHR + p.n_o + 1, std::max(1, num_sms() / parts)), (unsigned)parts);
     prof_begin("vvor_tc_kernel", stream);
-    launch_after(vvor_tc_kernel<CHR>, grid, THREADS, smem, stream, p);
+    launch_after(vvor_tc_kernel<CHR, STORE>, grid, THREADS, smem, stream, p);
     prof_end(stream);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
@@ -272,17 +334,47 @@ bool vvor_tensor_supported(const VvorArgs &a) {
     return a.T / 64 + a.n_o < INT32_MAX;
 }
 
+namespace {
+
+// Parts of both operands for CTAs that take whole taps: as few as 256 columns ask for, then halves while that gives the
+// chip more CTAs and a part keeps 64 columns.
+void store_parts(const VvorArgs &a, int *a_parts, int *b_parts) {
+    *a_parts = parts_of(a.Ma), *b_parts = parts_of(a.Cb);
+    auto halves = [](int width, int parts) { return width % (32 * parts) == 0 && width / parts >= 128; };
+    while (2 * a.n_o * a.G * *a_parts * *b_parts <= num_sms() && 2 * a.G * *a_parts * *b_parts <= MAX_PARTS) {
+        const bool b_wider = a.Cb / *b_parts > a.Ma / *a_parts;
+        if (b_wider && halves(a.Cb, *b_parts)) *b_parts *= 2;
+        else if (halves(a.Ma, *a_parts)) *a_parts *= 2;
+        else if (halves(a.Cb, *b_parts)) *b_parts *= 2;
+        else break;
+    }
+}
+
+}  // namespace
+
+// Whether CTAs take whole taps.  The fullest tap decides how long that takes, 10 ns a triplet of 256 x 256 channels and 7 of
+// 64 x 64 or 128 x 128; a rulebook of a cloud on itself has a triplet of every point in its centre tap, so that it holds the
+// average or the points, whichever is more.  The fp32 sums cost a microsecond a megabyte.  27 taps, fullest tap 950 / 3056 / 5150,
+// sums and stored, us: 512 x 512 (28 MB) 44 / 54 / 57 and 29 / 51 / 74, 256 x 256 (7 MB) 28 / 30 / 40 and 18 / 33 / 47,
+// 128 x 128 (2 MB) 18 / 20 / 22 and 16 / 31 / 43, 64 x 64 15 / 15 / 17 and 16 / 31 / 43; 125 taps, 5050: 512 x 512 (131 MB) 143 and 96.
+bool vvor_stores(const VvorArgs &a) {
+    const int64_t fullest = std::max(a.T / a.n_o, std::min(a.n_a, a.n_b)), sums = a.n_o * a.G * a.Ma * a.Cb * 4;
+    return sums >= (1 << 20) && fullest <= 300 + sums / 10000;
+}
+
 int vvor_tensor(const VvorArgs &a, cudaStream_t stream) {
     VvorTcParams p = {};
     p.a = (const uint16_t *)a.a, p.b = (const uint16_t *)a.b, p.a_idx = a.a_idx, p.b_idx = a.b_idx;
-    p.seg = a.seg_offs, p.acc = a.acc;
+    p.seg = a.seg_offs, p.acc = a.acc, p.out = (uint16_t *)a.out;
+    const bool store = a.out != nullptr;
     p.a_parts = parts_of(a.Ma), p.b_parts = parts_of(a.Cb);
+    if (store) store_parts(a, &p.a_parts, &p.b_parts);
     const int parts = a.G * p.a_parts * p.b_parts;
     p.Ma = a.Ma / p.a_parts, p.Cb = a.Cb / p.b_parts;   // the part's widths
     p.a_pitch = (int64_t)a.G * a.Ma, p.b_pitch = (int64_t)a.G * a.Cb, p.acc_pitch = a.Cb, p.acc_tap = (int64_t)a.G * a.Ma * a.Cb;
     p.n_o = (int)a.n_o, p.fmt = a.dtype == PCX_BF16 ? 1 : 0;
     if (int rc = device_status_address(&p.status)) return rc;
-    p.acc_cols = (uint32_t)(((p.Ma + 127) / 128 - 1) * p.Cb + (p.Cb + 63) / 64 * 64);   // flushed in blocks of 64 columns
+    p.acc_cols = (uint32_t)(((p.Ma + 127) / 128 - 1) * p.Cb + (p.Cb + 63) / 64 * 64);   // read in blocks of 64 (stored: 32) columns
     p.nacc = 2 * p.acc_cols <= 512 ? 2 : 1;
     p.ncols = 32;
     while (p.ncols < (uint32_t)p.nacc * p.acc_cols) p.ncols <<= 1;
@@ -293,9 +385,14 @@ int vvor_tensor(const VvorArgs &a, cudaStream_t stream) {
     const int64_t ctas = std::max(1, num_sms() / parts);
     int chr = blocks <= 2 ? 256 : blocks <= 4 ? 128 : 64;
     while (chr > 64 && a.T < 4 * ctas * chr) chr /= 2;
-    if (chr == 256) return launch_vvor<256>(p, parts, a.T, blocks, stream);
-    if (chr == 128) return launch_vvor<128>(p, parts, a.T, blocks, stream);
-    return launch_vvor<64>(p, parts, a.T, blocks, stream);
+    if (store) {
+        if (chr == 256) return launch_vvor<256, true>(p, parts, a.T, blocks, stream);
+        if (chr == 128) return launch_vvor<128, true>(p, parts, a.T, blocks, stream);
+        return launch_vvor<64, true>(p, parts, a.T, blocks, stream);
+    }
+    if (chr == 256) return launch_vvor<256, false>(p, parts, a.T, blocks, stream);
+    if (chr == 128) return launch_vvor<128, false>(p, parts, a.T, blocks, stream);
+    return launch_vvor<64, false>(p, parts, a.T, blocks, stream);
 }
 
 }  // namespace pcx
