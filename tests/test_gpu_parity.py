@@ -650,3 +650,23 @@ def test_triplet_cache_scope_reuses_rulebooks():
         assert e[0] is not c[0]
     f = build_triplets_segmented(pts, s, n, 0.1, 3, radius_scaler=2.0)
     assert f[0] is not c[0] and torch.equal(f[0], c[0])
+
+
+@pytest.mark.parametrize("n,cell,spread", [(1, 0.1, 1.0), (257, 0.5, 3.0), (4097, 0.02, 1.0), (50000, 0.3, 1.0), (50000, 0.05, 1e3), (30000, 0.004, 1.0),
+                                           (60000, 0.001, 4e2)])
+@pytest.mark.parametrize("outlier", [False, True])
+def test_down_sampling_in_any_spread(n, cell, spread, outlier):
+    """Cells in order by counting, and by a sort where points crowd in few ranges of keys or the key space is too wide."""
+    from pointelligence_b200 import _cabi
+
+    rng = np.random.default_rng(n)
+    pts = (rng.random((n, 3)) * spread - spread / 3).astype(np.float32)
+    if outlier:
+        pts[n // 2] = [2e5 * cell, -2e5 * cell, 1.5e5 * cell]
+    inds = np.sort(rng.integers(0, 5, n)).astype(np.int32)
+    ref_p, ref_i, ref_idx, ref_map = og.grid_sample_center_nearest(pts, cell, inds, True)
+    for _ in range(2):
+        idx, p, smp, mapping = _cabi.grid_sample_center_nearest(_t(pts), cell, _t(inds), True)
+        assert torch.equal(idx.cpu(), torch.from_numpy(np.asarray(ref_idx)).long()) and torch.equal(p.cpu(), torch.from_numpy(np.asarray(ref_p)))
+        assert torch.equal(mapping.cpu(), torch.from_numpy(np.asarray(ref_map)).long())
+        assert torch.equal(smp.pcx_sample_sizes.cpu(), torch.bincount(torch.from_numpy(np.asarray(ref_i)).long(), minlength=int(inds.max()) + 1))
