@@ -517,7 +517,12 @@ int pcx_radius_fill(const float *d_points, const float *d_queries, int64_t P,
  *   layers/triplets.py:431-520; the count saves the caller a pass and a
  *   hand-over of its own), [2] the device status word of pcx_device_status as
  *   it stood at this hand-over (not cleared).
+ *   `distance_type` 0 (ball) or 1 (Chebyshev); with PCX_RADIUS_WIDE_POINT_IDS or
+ *   PCX_RADIUS_WIDE_QUERY_IDS OR-ed in, those sample ids are int64, of which the
+ *   low words count (little endian).
  *   pcx_radius_taps_supported  1 when kernel_size is served by this path. */
+#define PCX_RADIUS_WIDE_POINT_IDS 0x100
+#define PCX_RADIUS_WIDE_QUERY_IDS 0x200
 int pcx_radius_taps_supported(int kernel_size);
 size_t pcx_radius_taps_workspace_bytes(int64_t P, int64_t Q, int kernel_size);
 int pcx_radius_taps_count(const float *d_points, const float *d_queries,
@@ -567,6 +572,17 @@ int pcx_grid_sample_select(const float *d_points, const int32_t *d_sample,
                            int64_t *d_indices, float *d_out_points,
                            int32_t *d_out_sample, int64_t *d_mapping,
                            void *d_ws, size_t ws_bytes, void *stream);
+/* The same two with int64 ids, grouped by their low words and returned as they
+ * came; with d_sizes, how often 0 .. S - 1 occur among the low words returned. */
+int pcx_grid_sample_count_ids(const float *d_points, const int64_t *d_ids,
+                              int64_t N, double cell, int64_t *h_info, void *d_ws,
+                              size_t ws_bytes, void *stream);
+int pcx_grid_sample_select_ids(const float *d_points, const int64_t *d_ids,
+                               int64_t N, double cell, int64_t num_cells,
+                               int64_t *d_indices, float *d_out_points,
+                               int64_t *d_out_ids, int64_t *d_mapping,
+                               int64_t *d_sizes, int64_t S, void *d_ws,
+                               size_t ws_bytes, void *stream);
 
 #ifdef __cplusplus
 }

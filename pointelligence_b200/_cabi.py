@@ -123,6 +123,9 @@ SIGNATURES = {
     "pcx_grid_sample_count_samples": (c_int, [c_void_p, c_void_p, c_int64, c_double, ctypes.POINTER(c_int64), c_void_p,
                                               c_size_t, c_void_p]),
     "pcx_sample_sizes": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_void_p]),
+    "pcx_grid_sample_count_ids": (c_int, [c_void_p, c_void_p, c_int64, c_double, ctypes.POINTER(c_int64), c_void_p, c_size_t, c_void_p]),
+    "pcx_grid_sample_select_ids": (c_int, [c_void_p, c_void_p, c_int64, c_double, c_int64] + [c_void_p] * 5
+                                   + [c_int64, c_void_p, c_size_t, c_void_p]),
     "pcx_grid_sample_select": (c_int, [c_void_p, c_void_p, c_int64, c_double, c_int64] + [c_void_p] * 4
                                + [c_void_p, c_size_t, c_void_p]),
 }
@@ -204,6 +207,7 @@ def workspace(nbytes, device):
 
 # ---------------------------------------------------- geometry beside the features ----
 _SIDE_STREAMS = {}
+_VALUES = frozenset((type(None), bool, int, float, str))
 _overlap = threading.local()
 
 
@@ -273,12 +277,13 @@ def on_geometry_stream(fn):
                 out.append(value)
         elif isinstance(value, (tuple, list)):
             for v in value:
-                collect(v, out, caller, depth)
+                if type(v) not in _VALUES:
+                    collect(v, out, caller, depth)
         elif isinstance(value, MvmrPlan):
             out.append(value.buffer)
         elif hasattr(value, "__dataclass_fields__") and depth < 8:
             for v in vars(value).values():
-                if v is not None and not isinstance(v, (bool, int, float, str)):
+                if type(v) not in _VALUES:
                     collect(v, out, caller, depth + 1)
 
     @functools.wraps(fn)
@@ -937,14 +942,14 @@ def radius_search(points, queries, radius, point_sample, query_sample, distance_
     """
     require_cuda(points, queries, point_sample, query_sample)
     dev = points.device
+    if takes_taps(kernel_size):
+        return radius_taps(points, queries, radius, point_sample, query_sample, distance_type, kernel_size, kernel_grid_size, want_k)
     points, queries = points.contiguous(), queries.contiguous()
     ps = as_i32(point_sample)
     qs = ps if query_sample is point_sample else as_i32(query_sample)
     P, Q = points.shape[0], queries.shape[0]
     L = lib()
     k3 = kernel_size ** 3
-    if kernel_size > 0 and L.pcx_radius_taps_supported(kernel_size) and os.environ.get("PCX_RADIUS_TAPS", "1") != "0":
-        return _radius_taps(points, queries, radius, ps, qs, distance_type, kernel_size, kernel_grid_size, want_k)
     with torch.cuda.device(dev):
         ws = workspace(L.pcx_radius_workspace_bytes(P, Q, kernel_size), dev)
         num_neighbors = torch.empty(Q, dtype=torch.int64, device=dev)
@@ -980,7 +985,13 @@ def radius_search(points, queries, radius, point_sample, query_sample, distance_
 _TAPS_RATIO = {}
 
 
-def _radius_taps(points, queries, radius, ps, qs, distance_type, kernel_size, kernel_grid_size, want_k):
+def takes_taps(kernel_size):
+    """Whether the tap-segmented search serves this kernel (and is not switched off)."""
+    return (kernel_size > 0 and lib().pcx_radius_taps_supported(kernel_size)
+            and os.environ.get("PCX_RADIUS_TAPS", "1") != "0")
+
+
+def radius_taps(points, queries, radius, ps, qs, distance_type, kernel_size, kernel_grid_size, want_k):
     """Tap-segmented search through ``pcx_radius_taps_*``: the pairs are written into buffers sized
     from the density of earlier searches (exactly sized after a counted first call or when the
     estimate turns out too small) and returned as views of the first ``total`` entries."""
@@ -1000,7 +1011,8 @@ def _radius_taps(points, queries, radius, ps, qs, distance_type, kernel_size, ke
 
 @on_geometry_stream
 def grid_sample_center_nearest(points, cell, sample, return_mapping):
-    """Returns ``(indices int64 (S,), points_f (S,3), sample_f int32 (S,)|None, mapping int64|None)``."""
+    """Returns ``(indices int64 (S,), points_f (S,3), sample_f (S,)|None, mapping int64|None)``; ``sample_f`` in the type
+    of int32 and int64 ids, in int32 for others."""
     require_cuda(points, sample)
     indices, out, out_sample, mapping, sizes = host().grid_sample(points, float(cell), sample, bool(return_mapping))
     if sizes is not None:

@@ -15,6 +15,8 @@ cloud instead of inheriting the up-sampling layer's.
 """
 from __future__ import annotations
 
+import threading
+from contextlib import contextmanager
 from typing import List, Sequence, Tuple
 
 import torch
@@ -31,12 +33,35 @@ from .layers.triplets import (build_triplets_segmented, handle_stride_and_build_
 RFS = 2.5   # receptive_field_scaler of every convolution, as in the reference's model
 
 
+_cast = threading.local()
+
+
+@contextmanager
+def weights_cast_together(convs):
+    """Inside, ``convs`` take their bf16 weights from one cast (without gradients): a launch for all of them, not one each."""
+    together = [c for c in convs if c.weight.is_cuda and c.weight.dtype is torch.float32 and c.weight.numel() % 8 == 0]   # (16-byte addresses)
+    if torch.is_grad_enabled() or len(together) < 2 or torch.compiler.is_compiling() or len({c.weight.device for c in together}) > 1:
+        yield
+        return
+    flat = torch.cat([c.weight.detach().reshape(-1) for c in together]).to(torch.bfloat16)
+    parts = flat.split([c.weight.numel() for c in together])
+    outer = getattr(_cast, "weights", None)
+    _cast.weights = {id(c): p.view(c.weight.shape) for c, p in zip(together, parts)}
+    try:
+        yield
+    finally:
+        _cast.weights = outer
+
+
 class Bf16PointConv3d(PointConv3d):
     """``PointConv3d`` with bf16 operands: the fp32 master weight is cast on the fly and the
     input is taken as bf16."""
 
     def forward(self, input, i, j, k, n, contract=None, seg_offs=None):
-        w = self.weight.to(torch.bfloat16)
+        together = getattr(_cast, "weights", None)
+        w = together.get(id(self)) if together and not torch.is_grad_enabled() else None
+        if w is None:
+            w = self.weight.to(torch.bfloat16)
         x = input.to(torch.bfloat16)
         out = self._conv_forward(x, i, j, k, n, w, None, contract=contract, seg_offs=seg_offs)
         if self.bias is not None:
@@ -149,7 +174,8 @@ class ResUNet(nn.Module):
         # and the geometry of a level is built on a stream of its own while the feature kernels of
         # the level before it are still running (every point cloud of the network derives from
         # the input cloud through the library's geometry calls alone)
-        with triplet_cache_scope(), _cabi.geometry_overlap(points.device):
+        convs = [mod for mod in self.modules() if isinstance(mod, Bf16PointConv3d)] if not torch.is_grad_enabled() else []
+        with triplet_cache_scope(), _cabi.geometry_overlap(points.device), weights_cast_together(convs):
             return self._forward(feat, points, sample_inds, sample_sizes, grid_size)
 
     def _forward(self, feat, points, sample_inds, sample_sizes, grid_size):

@@ -459,7 +459,8 @@ __global__ void grid_clear_kernel(int4 *ranges, int64_t fours, int32_t *ext) {
     if (t0 < EXT_WORDS) ext[t0] = t0 < 4 ? INT_MAX : t0 < 8 ? INT_MIN : 0;
 }
 
-__global__ void grid_extent_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample,
+// (sample: words of the ids, 1 << wide apart)
+__global__ void grid_extent_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, int wide,
                                    int64_t N, float cell, int32_t *ext) {
     start_after_previous();
     Extent4 e;
@@ -467,7 +468,7 @@ __global__ void grid_extent_kernel(const float *__restrict__ pts, const int32_t 
     for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < N; t += (int64_t)gridDim.x * blockDim.x) {
         e.add(0, floor_div_cell(pts[3 * t], cell)), e.add(1, floor_div_cell(pts[3 * t + 1], cell));
         e.add(2, floor_div_cell(pts[3 * t + 2], cell));
-        e.add(3, sample ? sample[t] : 0);
+        e.add(3, sample ? sample[t << wide] : 0);
     }
     block_minmax(e, 4, ext);
 }
@@ -477,11 +478,11 @@ __global__ void grid_extent_kernel(const float *__restrict__ pts, const int32_t 
 // Before, three or four passes of a library's radix sort over 64-bit keys (12 us each at 424 000 points, 18 at a million, with 8 us
 // of launches and clears between them): from the extents to the count on the host 140 -> 76 us for a million points of rooms at
 // twice their spacing, 113 -> 97 for four LiDAR sweeps (424 000 points, where 2^23 ranges are cleared and summed in 30).
-__device__ __forceinline__ int64_t grid_key(const float *__restrict__ pts, const int32_t *__restrict__ sample, int64_t n, float cell,
+__device__ __forceinline__ int64_t grid_key(const float *__restrict__ pts, const int32_t *__restrict__ sample, int wide, int64_t n, float cell,
                                             const int32_t *__restrict__ ext) {
     const int64_t ex = (int64_t)ext[4] - ext[0] + 1, ey = (int64_t)ext[5] - ext[1] + 1, ez = (int64_t)ext[6] - ext[2] + 1;
     const int64_t x = floor_div_cell(pts[3 * n], cell) - (int64_t)ext[0], y = floor_div_cell(pts[3 * n + 1], cell) - (int64_t)ext[1],
-                  z = floor_div_cell(pts[3 * n + 2], cell) - (int64_t)ext[2], b = (int64_t)(sample ? sample[n] : 0) - ext[3];
+                  z = floor_div_cell(pts[3 * n + 2], cell) - (int64_t)ext[2], b = (int64_t)(sample ? sample[n << wide] : 0) - ext[3];
     return x + ex * (y + ey * (z + ez * b));  // x fastest, sample slowest
 }
 
@@ -497,7 +498,7 @@ __device__ __forceinline__ int range_shift(const int32_t *__restrict__ ext, int6
     return max(0, 64 - __clzll((long long)(span - 1)) - (63 - __clzll(num_ranges)));
 }
 
-__global__ void grid_count_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, int64_t N, float cell, int32_t *ext,
+__global__ void grid_count_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, int wide, int64_t N, float cell, int32_t *ext,
                                   int64_t num_ranges, int64_t *keys, int32_t *arrival, int32_t *ranges) {
     start_after_previous();
     const int shift = range_shift(ext, num_ranges);
@@ -507,7 +508,7 @@ __global__ void grid_count_kernel(const float *__restrict__ pts, const int32_t *
         return;
     }
     if (n >= N) return;
-    const int64_t key = grid_key(pts, sample, n, cell, ext);
+    const int64_t key = grid_key(pts, sample, wide, n, cell, ext);
     keys[n] = key;
     arrival[n] = atomicAdd(&ranges[key >> shift], 1);
 }
@@ -599,13 +600,13 @@ __global__ void grid_report_kernel(const int32_t *__restrict__ ext, const int32_
     host.done();
 }
 
-__global__ void grid_key_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample,
+__global__ void grid_key_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, int wide,
                                 int64_t N, float cell, const int32_t *__restrict__ ext,
                                 int64_t *keys, int32_t *vals) {
     start_after_previous();
     int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (n >= N) return;
-    keys[n] = grid_key(pts, sample, n, cell, ext);
+    keys[n] = grid_key(pts, sample, wide, n, cell, ext);
     vals[n] = (int32_t)n;
 }
 
@@ -616,11 +617,11 @@ __global__ void grid_flag_kernel(const int64_t *__restrict__ keys, int64_t N, in
     flags[p] = (p == 0 || keys[p] != keys[p - 1]) ? 1 : 0;
 }
 
-__global__ void grid_select_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample,
+__global__ void grid_select_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, const int64_t *__restrict__ ids,
                                    const int64_t *__restrict__ keys, const int32_t *__restrict__ perm,
                                    const int32_t *__restrict__ flags, const int32_t *__restrict__ ordinal,
                                    int64_t N, float cell, int64_t *indices, float *out_pts,
-                                   int32_t *out_sample, int64_t *mapping) {
+                                   int32_t *out_sample, int64_t *out_ids, int64_t *mapping) {
     start_after_previous();
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= N) return;
@@ -649,11 +650,12 @@ __global__ void grid_select_kernel(const float *__restrict__ pts, const int32_t 
     out_pts[3 * (int64_t)seg + 1] = pts[3 * (int64_t)best_idx + 1];
     out_pts[3 * (int64_t)seg + 2] = pts[3 * (int64_t)best_idx + 2];
     if (out_sample) out_sample[seg] = sample ? sample[best_idx] : 0;
+    if (out_ids) out_ids[seg] = ids[best_idx];
 }
 
 // sizes[s] = elements of a non-decreasing id list that equal s; a warp a sample, 32 places looked at together: a million ids in four
 // steps instead of twenty, 15 -> 8 us.
-__global__ void sample_sizes_kernel(const int32_t *__restrict__ sorted, int64_t N, int64_t S, int64_t *sizes) {
+__global__ void sample_sizes_kernel(const int32_t *__restrict__ sorted, int wide, int64_t N, int64_t S, int64_t *sizes) {
     start_after_previous();
     const int64_t s = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
@@ -664,7 +666,7 @@ __global__ void sample_sizes_kernel(const int32_t *__restrict__ sorted, int64_t 
         int64_t lo = 0, hi = N;     // in [lo, hi]
         while (lo < hi) {
             const int64_t step = (hi - lo + 31) / 32, at = lo + lane * step;
-            const uint32_t below = __ballot_sync(0xffffffffu, at < hi && sorted[at] < s + e);   // a run of lanes from 0 on
+            const uint32_t below = __ballot_sync(0xffffffffu, at < hi && sorted[at << wide] < s + e);   // a run of lanes from 0 on
             const int n = __popc(below);
             if (n == 0) hi = lo;
             else hi = min(hi, lo + n * step), lo += (n - 1) * step + 1;
@@ -719,6 +721,91 @@ int bits_for(int64_t n) {
     int b = 1;
     while (((int64_t)1 << b) < n) ++b;
     return b;
+}
+
+// Cells of the points in order, in the workspace; h_info: cells, smallest and largest id.
+int count_cells(const float *d_points, const int32_t *d_sample, int wide, int64_t N, double cell, int64_t *h_info, void *d_ws, size_t ws_bytes,
+                cudaStream_t stream) {
+    if (N <= 0 || !d_points || !h_info || !d_ws) PCX_FAIL(PCX_E_ARG, "pcx_grid_sample_count: bad arguments");
+    if (N > INT32_MAX) PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_grid_sample_count: more than 2^31-1 points");
+    if (!(cell > 0)) PCX_FAIL(PCX_E_ARG, "grid_size must be positive; got %g", cell);
+    GridWs w;
+    size_t need = carve_grid(d_ws, N, &w);
+    if (ws_bytes < need) PCX_FAIL(PCX_E_CAPACITY, "pcx_grid_sample_count: workspace %zu < %zu bytes", ws_bytes, need);
+    if ((uintptr_t)d_ws % 256) PCX_FAIL(PCX_E_ALIGN, "pcx_grid_sample_count: workspace must be 256-byte aligned");
+    const float c32 = (float)cell;
+    uint32_t cell_bits;
+    memcpy(&cell_bits, &c32, sizeof(cell_bits));
+    std::atomic<uint64_t> &hint = order_hint(c32);
+    const uint64_t seen_hint = hint.load(), last = (seen_hint >> 32) == cell_bits ? seen_hint & 0xffffffffu : 0;
+    if (last & MORE_RANGES) w.num_ranges = w.more_ranges;
+    const int64_t fours = w.num_ranges / 4;
+    launch_after(grid_clear_kernel, (unsigned)std::min<int64_t>((fours + 255) / 256, 8 * num_sms()), 256, 0, stream, reinterpret_cast<int4 *>(w.ranges),
+                 fours, w.ext);
+    PCX_LAUNCH_CHECK();
+    int blocks = (int)std::min<int64_t>((N + 255) / 256, 8 * num_sms());
+    launch_after(grid_extent_kernel, blocks, 256, 0, stream, d_points, d_sample, wide, N, c32, w.ext);
+    PCX_LAUNCH_CHECK();
+    unsigned nb = (unsigned)((N + 255) / 256);
+    const HandOver host = new_hand_over();
+    if (host.words && !(last & 0xff)) {
+        launch_after(grid_count_kernel, nb, 256, 0, stream, d_points, d_sample, wide, N, c32, w.ext, w.num_ranges, w.keys_b, w.vals_b, w.ranges);
+        PCX_LAUNCH_CHECK();
+        launch_after(grid_ranges_kernel, (unsigned)(w.num_ranges / SCAN_BLOCK), SCAN_THREADS, 0, stream, w.ranges, w.range_sums, w.ext);
+        PCX_LAUNCH_CHECK();
+        launch_after(grid_order_kernel, nb, 256, 0, stream, w.keys_b, w.vals_b, N, w.ranges, w.range_sums, w.ext, w.num_ranges, w.keys_a, w.vals_a);
+        PCX_LAUNCH_CHECK();
+        launch_after(grid_place_kernel, nb, 256, 0, stream, w.keys_a, w.vals_a, N, w.ranges, w.range_sums, w.ext, w.num_ranges, w.keys_b, w.vals_b, w.flags);
+        PCX_LAUNCH_CHECK();
+        size_t tmp = w.cub_bytes;
+        PCX_CUDA(cub::DeviceScan::InclusiveSum(w.cub_tmp, tmp, w.flags, w.ordinal, N, stream));
+        launch_after(grid_report_kernel, 1, 1, 0, stream, w.ext, w.ordinal + (N - 1), host);
+        PCX_LAUNCH_CHECK();
+        if (int rc = wait_for_hand_over(host, stream)) return rc;
+        const int32_t *h = reinterpret_cast<const int32_t *>(host.words);
+        if (!crowded(h, N)) {
+            h_info[0] = host.words[EXT_WORDS / 2], h_info[1] = h[3], h_info[2] = h[7];
+            return PCX_OK;
+        }
+        // too unevenly spread over their extents: sorted, and the next of that cell size with more ranges, or sorted at once
+        hint.store((uint64_t)cell_bits << 32 | (last & MORE_RANGES || h[EXT_WIDE] ? 16 : MORE_RANGES));
+    } else if (last & 0xff) {
+        hint.store(seen_hint - 1);
+    }
+    launch_after(grid_key_kernel, nb, 256, 0, stream, d_points, d_sample, wide, N, c32, w.ext, w.keys_a, w.vals_a);
+    PCX_LAUNCH_CHECK();
+    // The sort only has to look at the bits the largest key can use.  How many those are is known from the extents,
+    // which come to the host with the cell count; the sort is enqueued for the bits that the last clouds of this
+    // cell size needed, and repeated where this one needs more (a first call asks for the extents beforehand).
+    int32_t *h = reinterpret_cast<int32_t *>(handover_words());   // extents, then the number of cells
+    auto extents = [&]() -> int {
+        PCX_CUDA(cudaMemcpyAsync(h, w.ext, 8 * sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+        PCX_CUDA(cudaStreamSynchronize(stream));
+        return PCX_OK;
+    };
+    std::atomic<uint64_t> &known = key_bits_of(c32);
+    uint64_t seen = known.load();
+    if ((seen >> 32) != cell_bits || (seen & 0xff) == 0) {
+        if (int rc = extents()) return rc;
+        seen = key_bits_hint(0, cell_bits, key_bits_for(h));
+    }
+    int used = (int)(seen & 0xff);
+    for (;;) {
+        size_t tmp = w.cub_bytes;
+        PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, tmp, w.keys_a, w.keys_b, w.vals_a, w.vals_b, N, 0, used, stream));
+        launch_after(grid_flag_kernel, nb, 256, 0, stream, w.keys_b, N, w.flags);
+        PCX_LAUNCH_CHECK();
+        tmp = w.cub_bytes;
+        PCX_CUDA(cub::DeviceScan::InclusiveSum(w.cub_tmp, tmp, w.flags, w.ordinal, N, stream));
+        PCX_CUDA(cudaMemcpyAsync(h + 8, w.ordinal + (N - 1), sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
+        if (int rc = extents()) return rc;
+        const int need = key_bits_for(h);
+        known.store(key_bits_hint(seen, cell_bits, need));
+        if (need <= used) break;
+        used = need;
+    }
+    h_info[0] = h[8], h_info[1] = h[3], h_info[2] = h[7];
+    return PCX_OK;
 }
 
 }  // namespace
@@ -936,93 +1023,18 @@ int pcx_grid_sample_count(const float *d_points, const int32_t *d_sample, int64_
 }
 
 int pcx_grid_sample_count_samples(const float *d_points, const int32_t *d_sample, int64_t N, double cell, int64_t *h_info, void *d_ws,
-                                  size_t ws_bytes, void *stream_) {
-    cudaStream_t stream = (cudaStream_t)stream_;
-    if (N <= 0 || !d_points || !h_info || !d_ws) PCX_FAIL(PCX_E_ARG, "pcx_grid_sample_count: bad arguments");
-    if (N > INT32_MAX) PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_grid_sample_count: more than 2^31-1 points");
-    if (!(cell > 0)) PCX_FAIL(PCX_E_ARG, "grid_size must be positive; got %g", cell);
-    GridWs w;
-    size_t need = carve_grid(d_ws, N, &w);
-    if (ws_bytes < need) PCX_FAIL(PCX_E_CAPACITY, "pcx_grid_sample_count: workspace %zu < %zu bytes", ws_bytes, need);
-    if ((uintptr_t)d_ws % 256) PCX_FAIL(PCX_E_ALIGN, "pcx_grid_sample_count: workspace must be 256-byte aligned");
-    const float c32 = (float)cell;
-    uint32_t cell_bits;
-    memcpy(&cell_bits, &c32, sizeof(cell_bits));
-    std::atomic<uint64_t> &hint = order_hint(c32);
-    const uint64_t seen_hint = hint.load(), last = (seen_hint >> 32) == cell_bits ? seen_hint & 0xffffffffu : 0;
-    if (last & MORE_RANGES) w.num_ranges = w.more_ranges;
-    const int64_t fours = w.num_ranges / 4;
-    launch_after(grid_clear_kernel, (unsigned)std::min<int64_t>((fours + 255) / 256, 8 * num_sms()), 256, 0, stream, reinterpret_cast<int4 *>(w.ranges),
-                 fours, w.ext);
-    PCX_LAUNCH_CHECK();
-    int blocks = (int)std::min<int64_t>((N + 255) / 256, 8 * num_sms());
-    launch_after(grid_extent_kernel, blocks, 256, 0, stream, d_points, d_sample, N, c32, w.ext);
-    PCX_LAUNCH_CHECK();
-    unsigned nb = (unsigned)((N + 255) / 256);
-    const HandOver host = new_hand_over();
-    if (host.words && !(last & 0xff)) {
-        launch_after(grid_count_kernel, nb, 256, 0, stream, d_points, d_sample, N, c32, w.ext, w.num_ranges, w.keys_b, w.vals_b, w.ranges);
-        PCX_LAUNCH_CHECK();
-        launch_after(grid_ranges_kernel, (unsigned)(w.num_ranges / SCAN_BLOCK), SCAN_THREADS, 0, stream, w.ranges, w.range_sums, w.ext);
-        PCX_LAUNCH_CHECK();
-        launch_after(grid_order_kernel, nb, 256, 0, stream, w.keys_b, w.vals_b, N, w.ranges, w.range_sums, w.ext, w.num_ranges, w.keys_a, w.vals_a);
-        PCX_LAUNCH_CHECK();
-        launch_after(grid_place_kernel, nb, 256, 0, stream, w.keys_a, w.vals_a, N, w.ranges, w.range_sums, w.ext, w.num_ranges, w.keys_b, w.vals_b, w.flags);
-        PCX_LAUNCH_CHECK();
-        size_t tmp = w.cub_bytes;
-        PCX_CUDA(cub::DeviceScan::InclusiveSum(w.cub_tmp, tmp, w.flags, w.ordinal, N, stream));
-        launch_after(grid_report_kernel, 1, 1, 0, stream, w.ext, w.ordinal + (N - 1), host);
-        PCX_LAUNCH_CHECK();
-        if (int rc = wait_for_hand_over(host, stream)) return rc;
-        const int32_t *h = reinterpret_cast<const int32_t *>(host.words);
-        if (!crowded(h, N)) {
-            h_info[0] = host.words[EXT_WORDS / 2], h_info[1] = h[3], h_info[2] = h[7];
-            return PCX_OK;
-        }
-        // too unevenly spread over their extents: sorted, and the next of that cell size with more ranges, or sorted at once
-        hint.store((uint64_t)cell_bits << 32 | (last & MORE_RANGES || h[EXT_WIDE] ? 16 : MORE_RANGES));
-    } else if (last & 0xff) {
-        hint.store(seen_hint - 1);
-    }
-    launch_after(grid_key_kernel, nb, 256, 0, stream, d_points, d_sample, N, c32, w.ext, w.keys_a, w.vals_a);
-    PCX_LAUNCH_CHECK();
-    // The sort only has to look at the bits the largest key can use.  How many those are is known from the extents,
-    // which come to the host with the cell count; the sort is enqueued for the bits that the last clouds of this
-    // cell size needed, and repeated where this one needs more (a first call asks for the extents beforehand).
-    int32_t *h = reinterpret_cast<int32_t *>(handover_words());   // extents, then the number of cells
-    auto extents = [&]() -> int {
-        PCX_CUDA(cudaMemcpyAsync(h, w.ext, 8 * sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-        PCX_CUDA(cudaStreamSynchronize(stream));
-        return PCX_OK;
-    };
-    std::atomic<uint64_t> &known = key_bits_of(c32);
-    uint64_t seen = known.load();
-    if ((seen >> 32) != cell_bits || (seen & 0xff) == 0) {
-        if (int rc = extents()) return rc;
-        seen = key_bits_hint(0, cell_bits, key_bits_for(h));
-    }
-    int used = (int)(seen & 0xff);
-    for (;;) {
-        size_t tmp = w.cub_bytes;
-        PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, tmp, w.keys_a, w.keys_b, w.vals_a, w.vals_b, N, 0, used, stream));
-        launch_after(grid_flag_kernel, nb, 256, 0, stream, w.keys_b, N, w.flags);
-        PCX_LAUNCH_CHECK();
-        tmp = w.cub_bytes;
-        PCX_CUDA(cub::DeviceScan::InclusiveSum(w.cub_tmp, tmp, w.flags, w.ordinal, N, stream));
-        PCX_CUDA(cudaMemcpyAsync(h + 8, w.ordinal + (N - 1), sizeof(int32_t), cudaMemcpyDeviceToHost, stream));
-        if (int rc = extents()) return rc;
-        const int need = key_bits_for(h);
-        known.store(key_bits_hint(seen, cell_bits, need));
-        if (need <= used) break;
-        used = need;
-    }
-    h_info[0] = h[8], h_info[1] = h[3], h_info[2] = h[7];
-    return PCX_OK;
+                                  size_t ws_bytes, void *stream) {
+    return count_cells(d_points, d_sample, 0, N, cell, h_info, d_ws, ws_bytes, (cudaStream_t)stream);
+}
+
+int pcx_grid_sample_count_ids(const float *d_points, const int64_t *d_ids, int64_t N, double cell, int64_t *h_info, void *d_ws, size_t ws_bytes,
+                              void *stream) {
+    return count_cells(d_points, (const int32_t *)d_ids, 1, N, cell, h_info, d_ws, ws_bytes, (cudaStream_t)stream);
 }
 
 int pcx_sample_sizes(const int32_t *d_sorted, int64_t N, int64_t S, int64_t *d_sizes, void *stream_) {
     if (N < 0 || S <= 0 || (N > 0 && !d_sorted) || !d_sizes) PCX_FAIL(PCX_E_ARG, "pcx_sample_sizes: bad arguments");
-    launch_after(sample_sizes_kernel, (unsigned)((S + 3) / 4), 128, 0, (cudaStream_t)stream_, d_sorted, N, S, d_sizes);
+    launch_after(sample_sizes_kernel, (unsigned)((S + 3) / 4), 128, 0, (cudaStream_t)stream_, d_sorted, 0, N, S, d_sizes);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
 }
@@ -1036,10 +1048,28 @@ int pcx_grid_sample_select(const float *d_points, const int32_t *d_sample, int64
     GridWs w;
     size_t need = carve_grid(d_ws, N, &w);
     if (ws_bytes < need) PCX_FAIL(PCX_E_CAPACITY, "pcx_grid_sample_select: workspace %zu < %zu bytes", ws_bytes, need);
-    launch_after(grid_select_kernel, (unsigned)((N + 255) / 256), 256, 0, stream, 
-        d_points, d_sample, w.keys_b, w.vals_b, w.flags, w.ordinal, N, (float)cell, d_indices,
-        d_out_points, d_out_sample, d_mapping);
+    launch_after(grid_select_kernel, (unsigned)((N + 255) / 256), 256, 0, stream, d_points, d_sample, (const int64_t *)nullptr, w.keys_b, w.vals_b,
+                 w.flags, w.ordinal, N, (float)cell, d_indices, d_out_points, d_out_sample, (int64_t *)nullptr, d_mapping);
     PCX_LAUNCH_CHECK();
+    return PCX_OK;
+}
+
+int pcx_grid_sample_select_ids(const float *d_points, const int64_t *d_ids, int64_t N, double cell, int64_t num_cells, int64_t *d_indices,
+                               float *d_out_points, int64_t *d_out_ids, int64_t *d_mapping, int64_t *d_sizes, int64_t S, void *d_ws,
+                               size_t ws_bytes, void *stream_) {
+    cudaStream_t stream = (cudaStream_t)stream_;
+    if (N <= 0 || num_cells <= 0 || !d_points || !d_ids || !d_indices || !d_out_points || !d_out_ids || !d_ws || (d_sizes && S <= 0))
+        PCX_FAIL(PCX_E_ARG, "pcx_grid_sample_select_ids: bad arguments");
+    GridWs w;
+    const size_t need = carve_grid(d_ws, N, &w);
+    if (ws_bytes < need) PCX_FAIL(PCX_E_CAPACITY, "pcx_grid_sample_select_ids: workspace %zu < %zu bytes", ws_bytes, need);
+    launch_after(grid_select_kernel, (unsigned)((N + 255) / 256), 256, 0, stream, d_points, (const int32_t *)nullptr, d_ids, w.keys_b, w.vals_b,
+                 w.flags, w.ordinal, N, (float)cell, d_indices, d_out_points, (int32_t *)nullptr, d_out_ids, d_mapping);
+    PCX_LAUNCH_CHECK();
+    if (d_sizes) {
+        launch_after(sample_sizes_kernel, (unsigned)((S + 3) / 4), 128, 0, stream, (const int32_t *)d_out_ids, 1, num_cells, S, d_sizes);
+        PCX_LAUNCH_CHECK();
+    }
     return PCX_OK;
 }
 

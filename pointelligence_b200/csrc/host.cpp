@@ -526,6 +526,9 @@ Tensor layer_norm(const Tensor &x, const Tensor &lengths, const OptTensor &weigh
 }
 
 // ----------------------------------------------------------------- geometry ----
+// Sample ids as the searches and the down-sampling read them: 64-bit ones by their low words, where they lie.
+Tensor ids(const Tensor &t) { return t.scalar_type() == at::kLong ? t.contiguous() : as_i32(t); }
+
 // Tap-segmented search: enqueue, fill into buffers sized from `ratio` (pairs per query of earlier searches
 // of this kind; negative: count first) and one hand-over.  Returns
 // (i, j, k | undefined, seg, num_neighbors, total, queries without neighbour, device status).
@@ -535,8 +538,10 @@ std::tuple<Tensor, Tensor, OptTensor, Tensor, Tensor, int64_t, int64_t, int64_t>
     require_cuda(points_), require_cuda(queries_), require_cuda(ps_), require_cuda(qs_);
     c10::cuda::CUDAGuard guard(points_.device());
     const Tensor points = points_.contiguous(), queries = queries_.contiguous();
-    const Tensor ps = ps_ ? as_i32(*ps_) : Tensor();
-    const Tensor qs = !qs_ ? Tensor() : (ps_ && qs_->is_same(*ps_)) ? ps : as_i32(*qs_);
+    const Tensor ps = ps_ ? ids(*ps_) : Tensor();
+    const Tensor qs = !qs_ ? Tensor() : (ps_ && qs_->is_same(*ps_)) ? ps : ids(*qs_);
+    if (ps.defined() && ps.scalar_type() == at::kLong) distance_type |= PCX_RADIUS_WIDE_POINT_IDS;
+    if (qs.defined() && qs.scalar_type() == at::kLong) distance_type |= PCX_RADIUS_WIDE_QUERY_IDS;
     const int64_t P = points.size(0), Q = queries.size(0), k3 = kernel_size * kernel_size * kernel_size;
     const auto i32 = at::TensorOptions().dtype(at::kInt).device(points.device());
     const auto i64 = i32.dtype(at::kLong);
@@ -577,25 +582,31 @@ std::tuple<Tensor, Tensor, OptTensor, OptTensor, OptTensor> grid_sample(const Te
                                                              bool want_mapping) {
     require_cuda(points_), require_cuda(sample_);
     c10::cuda::CUDAGuard guard(points_.device());
-    const Tensor points = points_.contiguous(), sample = sample_ ? as_i32(*sample_) : Tensor();
+    const Tensor points = points_.contiguous(), sample = sample_ ? ids(*sample_) : Tensor();
+    const bool wide = sample.defined() && sample.scalar_type() == at::kLong;
     const int64_t N = points.size(0);
     const auto i64 = at::TensorOptions().dtype(at::kLong).device(points.device());
     Tensor ws = workspace(pcx_grid_sample_workspace_bytes(N), points);
     int64_t info[3] = {0, 0, 0};
-    check(pcx_grid_sample_count_samples(ptr_as<float>(points), ptr_as<int32_t>(sample), N, cell, info, ptr(ws), ws.numel(), stream()));
+    if (wide) check(pcx_grid_sample_count_ids(ptr_as<float>(points), ptr_as<int64_t>(sample), N, cell, info, ptr(ws), ws.numel(), stream()));
+    else check(pcx_grid_sample_count_samples(ptr_as<float>(points), ptr_as<int32_t>(sample), N, cell, info, ptr(ws), ws.numel(), stream()));
     const int64_t cells = info[0];
     Tensor indices = at::empty({cells}, i64), out = at::empty({cells, 3}, i64.dtype(at::kFloat));
-    Tensor out_sample = sample_ ? at::empty({cells}, i64.dtype(at::kInt)) : Tensor();
+    Tensor out_sample = sample_ ? at::empty({cells}, wide ? i64 : i64.dtype(at::kInt)) : Tensor();
     Tensor mapping = want_mapping ? at::empty({N}, i64) : Tensor();
+    OptTensor sizes;
+    // cells come in ascending sample order; ids far beyond the number of points (hashes) are not worth an array
+    if (sample_ && info[1] >= 0 && info[2] < std::max<int64_t>(N, 4096)) sizes = at::empty({info[2] + 1}, i64);
+    if (wide) {
+        check(pcx_grid_sample_select_ids(ptr_as<float>(points), ptr_as<int64_t>(sample), N, cell, cells, ptr_as<int64_t>(indices), ptr_as<float>(out),
+                                         ptr_as<int64_t>(out_sample), ptr_as<int64_t>(mapping), sizes ? ptr_as<int64_t>(*sizes) : nullptr,
+                                         info[2] + 1, ptr(ws), ws.numel(), stream()));
+        return {indices, out, OptTensor(out_sample), want_mapping ? OptTensor(mapping) : std::nullopt, sizes};
+    }
     check(pcx_grid_sample_select(ptr_as<float>(points), ptr_as<int32_t>(sample), N, cell, cells, ptr_as<int64_t>(indices),
                                  ptr_as<float>(out), ptr_as<int32_t>(out_sample), ptr_as<int64_t>(mapping), ptr(ws), ws.numel(),
                                  stream()));
-    OptTensor sizes;
-    // cells come in ascending sample order; ids far beyond the number of points (hashes) are not worth an array
-    if (sample_ && info[1] >= 0 && info[2] < std::max<int64_t>(N, 4096)) {
-        sizes = at::empty({info[2] + 1}, i64);
-        check(pcx_sample_sizes(ptr_as<int32_t>(out_sample), cells, info[2] + 1, ptr_as<int64_t>(*sizes), stream()));
-    }
+    if (sizes) check(pcx_sample_sizes(ptr_as<int32_t>(out_sample), cells, info[2] + 1, ptr_as<int64_t>(*sizes), stream()));
     return {indices, out, sample_ ? OptTensor(out_sample) : std::nullopt, want_mapping ? OptTensor(mapping) : std::nullopt, sizes};
 }
 

@@ -47,6 +47,7 @@ constexpr int THREADS = QPB * 8;  // one lane per (query, candidate cell)
 constexpr int MAX_K3 = 128;       // taps this path handles (kernel_size 3 and 5)
 constexpr int FOURS = 64;         // fours of candidates that a warp lists at a time
 constexpr int SCAN_THREADS = 1024, SCAN_ITEMS = 4;
+constexpr int DISTANCE = ~(PCX_RADIUS_WIDE_POINT_IDS | PCX_RADIUS_WIDE_QUERY_IDS);
 constexpr int BIN_THREADS = 256;
 constexpr int CROWDED = 1024;     // points of a bucket that are put in order by counting the lower ones
 
@@ -126,12 +127,12 @@ __global__ void taps_clear_kernel(int4 *table, int64_t pairs, int64_t *ctrl) {
     if (t0 < 8) ctrl[t0] = 0;
 }
 
-__global__ void __launch_bounds__(BIN_THREADS) taps_key_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, int64_t P,
+__global__ void __launch_bounds__(BIN_THREADS) taps_key_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, int wide, int64_t P,
                                                                float inv, uint32_t mask, uint32_t *keys, int32_t *arrival, int2 *table) {
     start_after_previous();
     const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= P) return;
-    const uint32_t key = cell_bucket(sample ? sample[p] : 0, cell_of(pts[3 * p], inv), cell_of(pts[3 * p + 1], inv),
+    const uint32_t key = cell_bucket(sample ? sample[p << wide] : 0, cell_of(pts[3 * p], inv), cell_of(pts[3 * p + 1], inv),
                                      cell_of(pts[3 * p + 2], inv), mask);
     keys[p] = key;
     arrival[p] = atomicAdd(&table[key].y, 1);
@@ -163,14 +164,14 @@ __global__ void __launch_bounds__(BIN_THREADS) taps_order_kernel(const uint32_t 
     if (p < P) order[table[keys[p]].x + arrival[p]] = (int32_t)p;
 }
 
-__global__ void __launch_bounds__(BIN_THREADS) taps_place_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample,
+__global__ void __launch_bounds__(BIN_THREADS) taps_place_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, int wide,
                                                                  const uint32_t *__restrict__ keys, const int32_t *__restrict__ order, int64_t P,
                                                                  const int2 *__restrict__ table, const int32_t *__restrict__ crowded,
                                                                  const int64_t *__restrict__ ctrl, float4 *sorted_pts, int32_t *sorted_sample) {
     start_after_previous();
     auto put = [&](int32_t p, int32_t at) {
         sorted_pts[at] = make_float4(pts[3 * (int64_t)p], pts[3 * (int64_t)p + 1], pts[3 * (int64_t)p + 2], __int_as_float(p));
-        if (sample) sorted_sample[at] = sample[p];
+        if (sample) sorted_sample[at] = sample[(int64_t)p << wide];
     };
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (s < P) {
@@ -208,7 +209,8 @@ __global__ void __launch_bounds__(BIN_THREADS) taps_place_kernel(const float *__
 
 struct TapArgs {
     const float *queries;
-    const int32_t *query_sample, *point_sample;
+    const int32_t *query_sample, *point_sample;   // every second word of wide ids (1 << query_wide words apart)
+    int query_wide;
     const float4 *sorted_pts;
     const int2 *table;
     const int32_t *sorted_sample;   // null: no sample ids
@@ -278,7 +280,7 @@ struct Queries {
     __device__ __forceinline__ Queries(const TapArgs &a, int64_t q, int lane, float4 *room) : at(room), run(make_int2(0, 0)) {
         if (q < a.Q) {
             const float x = a.queries[3 * q], y = a.queries[3 * q + 1], z = a.queries[3 * q + 2];
-            const int b = a.query_sample ? a.query_sample[q] : 0;
+            const int b = a.query_sample ? a.query_sample[q << a.query_wide] : 0;
             run = run_of(a, x, y, z, b, lane & 7);
             if ((lane & 7) == 0) at[lane >> 3] = make_float4(x, y, z, __int_as_float(b));
         }
@@ -625,6 +627,7 @@ int check_common(int64_t P, int64_t Q, double radius, int distance_type, int ker
     if (P <= 0 || Q <= 0) PCX_FAIL(PCX_E_ARG, "%s: P and Q must be positive (got %lld, %lld)", who, (long long)P, (long long)Q);
     if (P > INT32_MAX || Q > INT32_MAX) PCX_FAIL(PCX_E_UNSUPPORTED, "%s: more than 2^31-1 rows", who);
     if (!(radius > 0)) PCX_FAIL(PCX_E_ARG, "radius must be positive; got %g", radius);
+    distance_type &= DISTANCE;
     if (distance_type != 0 && distance_type != 1) PCX_FAIL(PCX_E_ARG, "distance_type must be 0 (ball) or 1 (chebyshev)");
     if (kernel_size <= 0 || kernel_size % 2 == 0) PCX_FAIL(PCX_E_ARG, "kernel_size must be a positive odd integer; got %d", kernel_size);
     if (kernel_size * kernel_size * kernel_size > MAX_K3)
@@ -636,7 +639,8 @@ int check_common(int64_t P, int64_t Q, double radius, int distance_type, int ker
 TapArgs make_args(const TapsWs &w, const float *queries, const int32_t *point_sample, const int32_t *query_sample,
                   int64_t Q, double radius, int distance_type, int kernel_size, double grid) {
     TapArgs a = {};
-    a.queries = queries, a.query_sample = query_sample, a.point_sample = point_sample;
+    a.queries = queries, a.query_sample = query_sample, a.point_sample = point_sample, a.query_wide = distance_type & PCX_RADIUS_WIDE_QUERY_IDS ? 1 : 0;
+    distance_type &= DISTANCE;
     a.sorted_pts = w.sorted_pts, a.table = w.table, a.kept_point = w.kept_point, a.kept_tap = w.kept_tap;
     a.sorted_sample = point_sample ? w.sorted_sample : nullptr, a.kept = kept_per_query(kernel_size * kernel_size * kernel_size);
     a.counts = w.counts, a.block_hist = w.block_hist, a.seg = w.seg, a.ctrl = w.ctrl, a.ctrl_rw = w.ctrl;
@@ -700,6 +704,7 @@ int pcx_radius_taps_count(const float *d_points, const float *d_queries, const i
     const size_t need = carve_taps(d_ws, P, Q, k3, &w);
     if (ws_bytes < need) PCX_FAIL(PCX_E_CAPACITY, "pcx_radius_taps_count: workspace %zu < %zu bytes", ws_bytes, need);
     if ((uintptr_t)d_ws % 256) PCX_FAIL(PCX_E_ALIGN, "pcx_radius_taps_count: workspace must be 256-byte aligned");
+    const int wide = distance_type & PCX_RADIUS_WIDE_POINT_IDS ? 1 : 0;
     const float inv = (float)(1.0 / (2.0 * radius));
     const uint32_t mask = (uint32_t)(w.buckets - 1);
     const unsigned pblocks = (unsigned)((P + BIN_THREADS - 1) / BIN_THREADS);
@@ -707,13 +712,13 @@ int pcx_radius_taps_count(const float *d_points, const float *d_queries, const i
     launch_after(taps_clear_kernel, (unsigned)std::min<int64_t>((pairs + BIN_THREADS - 1) / BIN_THREADS, 8 * num_sms()), BIN_THREADS, 0, stream,
                  reinterpret_cast<int4 *>(w.table), pairs, w.ctrl);
     PCX_LAUNCH_CHECK();
-    launch_after(taps_key_kernel, pblocks, BIN_THREADS, 0, stream, d_points, d_point_sample, P, inv, mask, w.keys, w.arrival, w.table);
+    launch_after(taps_key_kernel, pblocks, BIN_THREADS, 0, stream, d_points, d_point_sample, wide, P, inv, mask, w.keys, w.arrival, w.table);
     PCX_LAUNCH_CHECK();
     launch_after(taps_room_kernel, pblocks, BIN_THREADS, 0, stream, w.keys, w.arrival, P, w.table, w.crowded, w.ctrl);
     PCX_LAUNCH_CHECK();
     launch_after(taps_order_kernel, pblocks, BIN_THREADS, 0, stream, w.keys, w.arrival, P, w.table, w.order);
     PCX_LAUNCH_CHECK();
-    launch_after(taps_place_kernel, pblocks, BIN_THREADS, 0, stream, d_points, d_point_sample, w.keys, w.order, P, w.table, w.crowded, w.ctrl,
+    launch_after(taps_place_kernel, pblocks, BIN_THREADS, 0, stream, d_points, d_point_sample, wide, w.keys, w.order, P, w.table, w.crowded, w.ctrl,
                  w.sorted_pts, w.sorted_sample);
     PCX_LAUNCH_CHECK();
     TapArgs a = make_args(w, d_queries, d_point_sample, d_query_sample, Q, radius, distance_type, kernel_size, kernel_grid_size);

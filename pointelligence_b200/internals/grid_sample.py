@@ -45,7 +45,7 @@ def grid_sample_filter(points, grid_size, sample_inds=None, reduction="center_ne
     sample_f = None
     if sample_inds is not None:
         # ids beyond 32 bits are grouped by their low words and returned as they came
-        sample_f = out_smp if sample_inds.dtype == torch.int32 else sample_inds.index_select(0, indices)
+        sample_f = out_smp if sample_inds.dtype == out_smp.dtype else sample_inds.index_select(0, indices)
         sizes = getattr(out_smp, "pcx_sample_sizes", None)
         if sizes is not None:
             sample_f.pcx_sample_sizes = sizes

@@ -67,6 +67,10 @@ def triplet_key(points, query_points, neighbor_radius, radius_scaler, sort_by, r
             sort_by, bool(return_num_neighbors), ident)
 
 
+def cache_active():
+    return _active_cache() is not None
+
+
 def cache_get(key):
     cache = _active_cache()
     if cache is None or key is None:

@@ -19,7 +19,7 @@ from torch.nn.modules.utils import _triple
 from .. import _cabi
 from ..internals.indexing import cumsum_exclusive, repeat_interleave_indices
 from ..internals.neighbors import radius_search, radius_search_sorted_grid8_segments
-from ..internals.triplet_cache import cache_get, cache_put, triplet_key
+from ..internals.triplet_cache import cache_active, cache_get, cache_put, triplet_key
 from ..sparse_engines._seg_offs import kernel_offset_segments
 from .contract import TripletContract
 from .downsample import downsample
@@ -83,6 +83,29 @@ def build_triplets_segmented(points, sample_inds, sample_sizes, neighbor_radius,
                              return_num_neighbors=False, radius_scaler=None, tap_stripes=32):
     """Returns ``(i, j, k int32, seg_offs int64, num_neighbors or None)`` with the
     triplets grouped by tap.  Raises when a query has no neighbour."""
+    return _segmented(points, sample_inds, sample_sizes, neighbor_radius, kernel_size, query_points, query_sample_inds,
+                      query_sample_sizes, return_num_neighbors, radius_scaler, tap_stripes)
+
+
+def _searched(points, queries, sample_inds, query_sample_inds, radius, ks, kernel_grid_size, tap_stripes):
+    """``radius_search_sorted_grid8_segments``; ordinary clouds without its layers of checks, casts and scopes, some
+    25 us of the host's time per search."""
+    if (points.dtype is torch.float32 and queries.dtype is torch.float32 and points.is_cuda and queries.device == points.device
+            and points.dim() == 2 and queries.dim() == 2 and points.shape[1] == 3 and queries.shape[1] == 3
+            and points.shape[0] and queries.shape[0] and float(radius) > 0 and tap_stripes == 32
+            and sample_inds is not None and query_sample_inds is not None and sample_inds.is_cuda and query_sample_inds.is_cuda
+            and _cabi.takes_taps(ks)):
+        i, j, k, seg_offs, counts = _cabi.radius_taps(points, queries, float(radius), sample_inds, query_sample_inds, 0, ks,
+                                                      kernel_grid_size, True)
+        return i, j, seg_offs, counts, k
+    return radius_search_sorted_grid8_segments(
+        points=points, queries=queries, radius=radius, kernel_size=ks, kernel_grid_size=kernel_grid_size, sample_inds=sample_inds,
+        query_sample_inds=query_sample_inds, dtype_num_neighbors=torch.int64, distance_type="ball", tap_stripes=tap_stripes,
+        return_k=True)
+
+
+def _segmented(points, sample_inds, sample_sizes, neighbor_radius, kernel_size, query_points=None, query_sample_inds=None,
+               query_sample_sizes=None, return_num_neighbors=False, radius_scaler=None, tap_stripes=32):
     sizes = _triple(kernel_size)
     if not (sizes[0] == sizes[1] == sizes[2]):
         raise ValueError(f"segmented triplet construction requires a cubic kernel; got {sizes}")
@@ -95,18 +118,17 @@ def build_triplets_segmented(points, sample_inds, sample_sizes, neighbor_radius,
     with torch.no_grad():
         query_points, query_sample_inds, query_sample_sizes = _resolve_queries(
             points, sample_inds, sample_sizes, query_points, query_sample_inds, query_sample_sizes)
-        key = triplet_key(points, query_points, neighbor_radius, radius_scaler, "k", return_num_neighbors,
-                          sample_inds, query_sample_inds, partial(voxelize_3d, kernel_size=sizes))
-        if key is not None:
-            key = key + ("segmented",)
-        hit = cache_get(key)
-        if hit is not None:
-            return hit
-        i, j, seg_offs, num_neighbors, k = radius_search_sorted_grid8_segments(
-            points=points, queries=query_points, radius=neighbor_radius, kernel_size=ks,
-            kernel_grid_size=kernel_grid_size, sample_inds=sample_inds,
-            query_sample_inds=query_sample_inds, dtype_num_neighbors=torch.int64,
-            distance_type="ball", tap_stripes=tap_stripes, return_k=True)
+        key = None
+        if cache_active():
+            key = triplet_key(points, query_points, neighbor_radius, radius_scaler, "k", return_num_neighbors,
+                              sample_inds, query_sample_inds, partial(voxelize_3d, kernel_size=sizes))
+            if key is not None:
+                key = key + ("segmented",)
+            hit = cache_get(key)
+            if hit is not None:
+                return hit
+        i, j, seg_offs, num_neighbors, k = _searched(points, query_points, sample_inds, query_sample_inds, neighbor_radius, ks,
+                                                     kernel_grid_size, tap_stripes)
         lonely = getattr(num_neighbors, "pcx_queries_without_neighbor", None)   # counted by the search itself
         if lonely is None:
             lonely = int((num_neighbors == 0).sum().item()) if num_neighbors.numel() else 0
@@ -173,7 +195,7 @@ def _build_for(m_points, m_sample_inds, m_sample_sizes, neighbor_radius, kernel_
                sort_by, distance_type, return_num_neighbors, query=None):
     qp, qi, qs = query if query is not None else (None, None, None)
     if sort_by == "k" and distance_type == "ball" and should_use_direct_segmented_triplets(kernel_size):
-        return build_triplets_segmented(
+        return _segmented(   # (inside the scopes of the caller)
             points=m_points, sample_inds=m_sample_inds, sample_sizes=m_sample_sizes,
             neighbor_radius=neighbor_radius, kernel_size=kernel_size, query_points=qp,
             query_sample_inds=qi, query_sample_sizes=qs, return_num_neighbors=return_num_neighbors,
