@@ -60,7 +60,10 @@ void prof_end(cudaStream_t stream);
 
 // A kernel launched by launch_after() is set up on the chip while the one before it in the stream is still finishing; it
 // starts with start_after_previous(), which returns when that one has ended and its writes can be read, and allows the
-// next one the same.  Every thread calls it before anything else, so that an end implies the ends of all before.
+// next one the same.  Every thread calls it before it reads or writes global memory, so that an end implies the ends of all
+// before.  A kernel with tensor memory takes it, and passes a barrier, before that call: the next one may take its own early, on
+// the same multiprocessor, and would be waited for by one that still has to.  With the barriers of its pipeline it is then ready
+// when the kernel before it ends: a training call of 942 points and 512 channels 166 -> 159 us.
 // A gap between kernels shrinks by 1 to 1.5 us: a training call of 942 points and 512 channels (11 launches) 230 -> 214 us,
 // 150 000 points and 64 channels (11) 224 -> 212, an fp32 one (8) 204 -> 194, a norm with its gradient (7) 229 -> 215.
 __device__ __forceinline__ void start_after_previous() {

@@ -661,7 +661,6 @@ struct Walk {
 // one row loses 2^-8), for a second pass over the taps.
 template <int PACK, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_constant__ CUtensorMap tmap, const __grid_constant__ OsParams p) {
-    start_after_previous();
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t s_full[MAX_SLOTS], s_empty[MAX_SLOTS], s_acc_full[2], s_acc_empty[2], s_step_full[AHEAD], s_step_empty[AHEAD];
     __shared__ uint32_t s_word[WORDS];
@@ -699,13 +698,16 @@ __global__ void __launch_bounds__(THREADS, 1) mvmr_os_kernel(const __grid_consta
         tma_prefetch_desc(&tmap);
     }
     if (warp == 0) tmem_alloc(smem_u32(&s_tmem), p.ncols);
-    const bool bias_here = p.bias && p.nsplit == 1 && p.out_pitch <= BIAS_WIDTH;
-    if (bias_here)
-        for (int c = tid; c < p.out_pitch; c += THREADS) s_bias[c] = bias_at(p.bias, c, p.fmt);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
+    start_after_previous();   // (tensor memory is held by now: see there)
+    const bool bias_here = p.bias && p.nsplit == 1 && p.out_pitch <= BIAS_WIDTH;
+    if (bias_here) {
+        for (int c = tid; c < p.out_pitch; c += THREADS) s_bias[c] = bias_at(p.bias, c, p.fmt);
+        __syncthreads();
+    }
 
     if (warp < EPI_WARPS) {
         // -------------------------------------------------------------- epilogue ----

@@ -253,7 +253,6 @@ __device__ __forceinline__ int32_t load_if(bool there, const int32_t *a, int32_t
 }
 
 __global__ void __launch_bounds__(THREADS, CTAS) mvmr_thin_kernel(const __grid_constant__ ThinParams p) {
-    start_after_previous();
     constexpr int CELLS = TPS / 2;   // taps of a lane
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t s_full[SLOTS], s_empty[SLOTS], s_acc_full[2], s_acc_empty[2];   // a step's operands are there / have been used; a block's sums
@@ -261,14 +260,6 @@ __global__ void __launch_bounds__(THREADS, CTAS) mvmr_thin_kernel(const __grid_c
     __shared__ int s_abort;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, part = blockIdx.y;
     const uint32_t slot0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    {
-        uint32_t odd = 0;
-        for (int x = tid; x < p.n_odd; x += THREADS) odd |= p.odd[x];
-        if (__syncthreads_or(odd)) {
-            one_by_one(p, reinterpret_cast<float *>(smem_raw), part);
-            return;
-        }
-    }
     volatile int *abort_flag = &s_abort;
     auto wait_one = [&](const uint64_t &bar, uint32_t parity) {
         return mbar_wait_abortable(smem_u32(&bar), parity & 1u, STATUS_BIT, p.status, abort_flag);
@@ -289,6 +280,16 @@ __global__ void __launch_bounds__(THREADS, CTAS) mvmr_thin_kernel(const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
+    start_after_previous();   // (tensor memory is held by now: see there)
+    {
+        uint32_t odd = 0;
+        for (int x = tid; x < p.n_odd; x += THREADS) odd |= p.odd[x];
+        if (__syncthreads_or(odd)) {
+            one_by_one(p, reinterpret_cast<float *>(smem_raw), part);
+            if (warp == MMA_WARP) tmem_dealloc(tmem, p.ncols);
+            return;
+        }
+    }
     const int blocks = (p.nblocks - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // of this CTA
     auto block_of = [&](int n) { return (int64_t)blockIdx.x + (int64_t)n * gridDim.x; };
     auto most_of = [&](const At &at) { return at.n < blocks ? __ldg(p.most + block_of(at.n) * p.nq + at.q) : 0; };

@@ -137,8 +137,6 @@ struct MvmrTcParams {
 // 256 x 256 channels, 408 976 triplets 212 and 201).
 template <int MODE, int NT, bool CHAINED, bool AGAIN>
 __global__ void __launch_bounds__(NT, NT == 256 ? 1 : 0) mvmr_tc_kernel(MvmrTcParams p) {
-    start_after_previous();
-    if (AGAIN && !p.only_if.holds()) return;
     constexpr bool BULK = MODE == 1;
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t s_bar;
@@ -185,11 +183,16 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 1 : 0) mvmr_tc_kernel(MvmrTcPa
         fence_mbar_init();
     }
     if (warp == 0) tmem_alloc(smem_u32(&s_tmem), p.ncols);
-    build_chunk_table<CH>(p.seg, p.K, s_cum, s_warp_sums);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
+    start_after_previous();   // (tensor memory is held by now: see there)
+    if (AGAIN && !p.only_if.holds()) {
+        if (warp == 0) tmem_dealloc(tmem, p.ncols);
+        return;
+    }
+    build_chunk_table<CH>(p.seg, p.K, s_cum, s_warp_sums);
 
     const int total = s_cum[p.K];
     const int per = (total + gridDim.x - 1) / gridDim.x;

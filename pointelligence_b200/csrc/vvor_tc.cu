@@ -112,7 +112,6 @@ __device__ __forceinline__ void store_columns(uint16_t *dst, const float *v, int
 
 template <int CHR, bool STORE>   // triplets of a chunk: the contraction of one slot
 __global__ void __launch_bounds__(THREADS, 1) vvor_tc_kernel(VvorTcParams p) {
-    start_after_previous();
     constexpr uint32_t BLK = CHR * 128;   // one 64-channel block of a tile
     using Cursor = ChunkCursorT<CHR>;
     extern __shared__ uint8_t smem_raw[];
@@ -154,11 +153,12 @@ __global__ void __launch_bounds__(THREADS, 1) vvor_tc_kernel(VvorTcParams p) {
         s_abort = 0;
     }
     if (warp == 0) tmem_alloc(smem_u32(&s_tmem), p.ncols);
-    build_chunk_table<CHR>(p.seg, p.n_o, s_cum, s_warp_sums);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = s_tmem;
+    start_after_previous();   // (tensor memory is held by now: see there)
+    build_chunk_table<CHR>(p.seg, p.n_o, s_cum, s_warp_sums);
 
     const int total = s_cum[p.n_o];
     const int per = (total + gridDim.x - 1) / gridDim.x;

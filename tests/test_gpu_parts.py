@@ -243,3 +243,24 @@ def test_accumulators_about_the_size_that_keeps_four_warps(n):
     i, j, seg, w, x, go, y, gx = _whole_numbers(torch.float16, 3, 30000, n, 256, 256, n_in=9000)
     assert torch.equal(_cabi.mvmr(w, x, j, i, seg, None, n, False, _cabi.ENGINE_TENSOR).double(), y)
     assert torch.equal(_cabi.mvmr(w, go, i, j, seg, None, 9000, True, _cabi.ENGINE_TENSOR).double(), gx)
+
+
+@pytest.mark.parametrize("rows", [1, 2, 3, 5, 170, 171, 1365, 1366, 30001])
+@pytest.mark.parametrize("offset", [0, 1, 8])   # of the first element of the output, in elements: 8 is a 16-byte boundary again
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_sums_are_rounded_to_rows_of_any_size_and_address(rows, offset, dtype):
+    """No triplets and a bias: every row is the bias, exactly, and nothing beyond the rows is written."""
+    from pointelligence_b200 import _cabi
+
+    lib, M = _cabi.lib(), 3
+    bias = torch.tensor([1.5, -2.0, 0.25], dtype=dtype, device=DEV)
+    w = torch.zeros(1, 1, 3, M, dtype=dtype, device=DEV)
+    seg = torch.zeros(2, dtype=torch.int64, device=DEV)
+    out = torch.full((rows * M + 24,), 7.0, dtype=dtype, device=DEV)
+    code = 1 if dtype == torch.float16 else 2
+    need = lib.pcx_mvmr_workspace_bytes(rows, 1, 1, 3, M, 0, code)
+    ws = torch.empty(need, dtype=torch.uint8, device=DEV)
+    _cabi.check(lib.pcx_mvmr_bias(w.data_ptr(), None, None, None, seg.data_ptr(), None, bias.data_ptr(), out.data_ptr() + 2 * offset,
+                                  0, 1, rows, 1, 1, 3, M, 0, code, 0, ws.data_ptr(), need, torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(out[offset:offset + rows * M].view(rows, M), bias.expand(rows, M))
+    assert (out[:offset] == 7).all() and (out[offset + rows * M:] == 7).all()
