@@ -1064,19 +1064,35 @@ uint64_t wait_limit() {
     return v;
 }
 
-// Parts the taps of a group are split into when the groups alone do not fill the chip: the count with the
-// smallest time, a part costing a tenth of a whole group more than its share (its fp32 sums go through
-// memory).  1000 points of 256 channels, 4 groups: 183 us on 4 CTAs, 28 us in 27 parts per group.
-int split_parts(int64_t ngroups, int K, int nparts) {
-    const int sms = num_sms();
-    int best = 1;
-    double best_cost = 1e30;
-    for (int s = 1; s <= std::min(K, 64) && ngroups * nparts < 2 * sms; ++s) {
-        const double waves = (double)((ngroups * nparts * s + sms - 1) / sms), cost = waves * (1.0 / s + (s > 1 ? 0.1 : 0.0));
-        if (cost < best_cost * 0.999) best_cost = cost, best = s;
+// What a group is split into when the groups alone do not fill the chip: parts of its taps, whose fp32 sums go through memory
+// to os_reduce_kernel, and of its columns, whose rows are copied once per part.  The pair with the smallest time, by what the
+// kernels measured on B200 (in us): 0.6 a step, 0.015 a column of the epilogue, both for every unit a CTA works off in turn;
+// 0.27 for a MB of sums, written and read; 0.2 for reading the rows once more.  27 taps and 22 triplets a row, against the
+// taps alone at a tenth of a group for every part (ten calls in a graph: alone, a call of 942 points is bound by its host):
+//   points  channels   taps x columns   us             points  channels   taps x columns   us
+//      942    256       27 -> 14 x 2    22.6 -> 20.1     3000     64        12 -> 9         16.8 -> 14.5
+//     2000    256       14 -> 9 x 2     26.8 -> 23.5      500    512        27 -> 14 x 2    25.3 -> 24.4
+//     4000 points and more, and 942 of 512 channels: as before
+// `slices` of 64 channels the contraction has, `pack` taps a step; `width` columns of a part.
+struct Split { int taps, columns; };
+Split split_of(int64_t ngroups, int K, int nparts, int width, int slices, int pack, int64_t row_floats) {
+    const int64_t sms = num_sms(), units = ngroups * nparts;
+    Split best = {1, 1};
+    if (units >= 2 * sms) return best;
+    const float mb_us = 0.27e-6f * 4.f * (float)(ngroups * GROUP_BLOCKS * ROWS * row_floats);
+    float best_us = 1e30f;
+    // the fewest parts for every number of taps a part may have: few candidates, as every call asks
+    for (int s = 1, taps = K; s <= 64; s = (K + taps - 2) / (taps - 1), taps = (K + s - 1) / s) {
+        const float steps = 0.6f * (float)((taps + pack - 1) / pack * slices);
+        for (int q = 1; q <= 4 && width % (16 * q) == 0 && (q == 1 || width / q >= 64) && nparts * q <= 64; q *= 2) {
+            const float us = (float)((units * q * s + sms - 1) / sms) * (steps + 0.015f * (float)(width / q)) + (s > 1 ? mb_us * (float)s : 0.f) + 0.2f * (float)(q - 1);
+            if (us < best_us * 0.999f) best_us = us, best = {s, q};
+        }
+        if (taps == 1) break;
     }
     return best;
 }
+int taps_of_a_step(int inw) { return inw == 16 ? 4 : inw == 32 ? 2 : 1; }
 
 // fp32 sums of a rulebook whose taps are split
 size_t partial_bytes(int64_t n_out, int outw, int splits) {
@@ -1218,7 +1234,8 @@ size_t pcx_mvmr_planned_scratch_bytes(int64_t multi_buckets, int in_width, int64
     if (multi_buckets < 0 || in_width <= 0 || n_out <= 0 || out_width <= 0 || K <= 0 || G <= 0) return 0;
     const int64_t ngroups = (n_out + GROUP_BLOCKS * ROWS - 1) / (GROUP_BLOCKS * ROWS);
     return pcx_mvmr_planned_workspace_bytes(multi_buckets, G * in_width) +
-           partial_bytes(n_out, G * out_width, split_parts(ngroups, K, G * parts_of(out_width)));
+           partial_bytes(n_out, G * out_width, split_of(ngroups, K, G * parts_of(out_width), out_width / parts_of(out_width), (in_width + 63) / 64,
+                                                        taps_of_a_step(in_width), G * out_width).taps);
 }
 
 int pcx_mvmr_plan_multi_buckets(const void *d_plan, int64_t *h_count, void *stream_) {
@@ -1274,7 +1291,7 @@ int pcx::mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan, si
     const int inw = transpose ? M : C, outw = transpose ? C : M;
     // output rows wider than the tensor memory's two accumulators (256 channels), and those of a grouped weight, are
     // worked off in parts of the same width
-    const int out_parts = parts_of(outw), nparts = groups * out_parts;
+    int out_parts = parts_of(outw), nparts = groups * out_parts;
     if (inw % 16 || outw % (16 * out_parts) || inw > 1024 || groups * inw > 2048 || nparts > 64)
         PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_planned: channel counts must be multiples of 16 and the parts of an output row equal (groups=%d C=%d M=%d)", groups, C, M);
     if (!d_weight || !d_plan || !d_out || (T > 0 && !d_feat)) PCX_FAIL(PCX_E_ARG, "pcx_mvmr_planned: null pointer");
@@ -1288,7 +1305,14 @@ int pcx::mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan, si
     const size_t need_plan = carve_plan(d_plan, T, n_out, K, G, &pv);
     if (plan_bytes < need_plan) PCX_FAIL(PCX_E_CAPACITY, "pcx_mvmr_planned: plan buffer %zu < %zu bytes", plan_bytes, need_plan);
 
+    // the fp32 sums of split taps lie behind the bucket sums; a caller that made no room for them gets one part
+    Split split = split_of(pv.ngroups, K, nparts, outw / out_parts, (inw * (split_sums ? 2 : 1) + 63) / 64, taps_of_a_step(inw * (split_sums ? 2 : 1)),
+                           (int64_t)groups * outw);
+    if (split.taps > 1 && (!d_ws || ws_bytes < sums_bytes + partial_bytes(n_out, groups * outw, split.taps))) split = {1, 1};
+    out_parts *= split.columns, nparts *= split.columns;
+
     OsParams p = {};
+    p.nsplit = split.taps, p.partial = p.nsplit > 1 ? (float *)((char *)d_ws + sums_bytes) : nullptr;
     p.feat = (const uint16_t *)d_feat, p.out = (uint16_t *)d_out, p.bias = (const uint16_t *)d_bias;
     p.perm = pv.perm, p.group_order = pv.group_order, p.tile_rows = pv.tile_rows, p.tap_masks = pv.tap_masks;
     p.scratch = (const uint16_t *)d_ws;
@@ -1305,7 +1329,7 @@ int pcx::mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan, si
     while (p.ncols < 2u * (uint32_t)p.nacc * p.col_stride) p.ncols <<= 1;
     // A step costs its chain of waits, copies and MMA issue, some 1000 clocks, whatever the width: rows of 16 or 32
     // channels fill the 64 of a step with four or two taps.
-    const int pack = inw == 16 ? 4 : inw == 32 ? 2 : 1;
+    const int pack = taps_of_a_step(inw);
     p.weight = (const uint16_t *)d_weight;
     p.w_box_rows = (uint32_t)(transpose ? p.outw : std::min(64, C));
     p.w_rows = transpose ? p.w_box_rows : p.w_box_rows * (uint32_t)pack;
@@ -1334,10 +1358,6 @@ int pcx::mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan, si
     // by the parity of its turn alone: with more teams than slots that could still be a turn further back.
     p.teams = std::min(TEAMS, p.nslots);
     if (p.nslots < 2) PCX_FAIL(PCX_E_UNSUPPORTED, "pcx_mvmr_planned: shared memory does not fit (C=%d M=%d)", C, M);
-    // the fp32 sums of a split rulebook lie behind the bucket sums; a caller that made no room for them gets one part
-    p.nsplit = split_parts(pv.ngroups, K, nparts);
-    if (p.nsplit > 1 && (!d_ws || ws_bytes < sums_bytes + partial_bytes(n_out, p.out_pitch, p.nsplit))) p.nsplit = 1;
-    p.partial = p.nsplit > 1 ? (float *)((char *)d_ws + sums_bytes) : nullptr;
     const size_t smem = 1024 + (size_t)p.nslots * p.slot_bytes + AHEAD * pack * ENTRY_BYTES;
     auto kernel = split_sums ? (pack == 4 ? mvmr_os_kernel<4, true> : pack == 2 ? mvmr_os_kernel<2, true> : mvmr_os_kernel<1, true>)
                              : (pack == 4 ? mvmr_os_kernel<4, false> : pack == 2 ? mvmr_os_kernel<2, false> : mvmr_os_kernel<1, false>);

@@ -341,3 +341,36 @@ def test_wide_and_grouped_layers_choose_the_kernel_by_their_reductions():
     graph.replay()
     ref = _cabi.mvmr(w, x, tj, ti, ts, None, 20000, False)
     assert float((y.float() - ref.float()).norm() / ref.float().norm()) < 1e-3
+
+
+@pytest.mark.parametrize("G,C,M", [(1, 256, 256), (1, 64, 256), (1, 256, 192), (1, 512, 512), (1, 32, 144), (1, 16, 128), (2, 64, 256), (1, 320, 64)])
+@pytest.mark.parametrize("n", [1, 129, 300, 942, 2100])   # one to nine groups: taps split alone, and with the columns in two or four parts
+def test_small_clouds_split_by_taps_and_columns(n, G, C, M):
+    """Operands of -1, 0 and 1, one in eight not 0: sums of some hundred products are whole numbers below 2^8, exact in fp32 in any
+    split and after the rounding to fp16 (2^11).  Bucket sums are whole as well."""
+    from pointelligence_b200 import _cabi
+
+    g = torch.Generator(device=DEV).manual_seed(n + C + M)
+    K, T = 27, 22 * n
+    k = torch.sort(torch.randint(0, K, (T,), device=DEV, generator=g)).values
+    i = torch.randint(0, n, (T,), device=DEV, generator=g)
+    order = torch.argsort(k * n + i, stable=True)
+    i, j = i[order].int(), torch.randint(0, n, (T,), device=DEV, generator=g).int()
+    seg = torch.searchsorted(k, torch.arange(K + 1, device=DEV)).to(torch.int64)
+
+    def few(*shape):
+        sign = 2 * torch.randint(0, 2, shape, device=DEV, generator=g) - 1
+        return (torch.randint(0, 8, shape, device=DEV, generator=g) // 7 * sign).to(torch.float16)
+
+    w, x, go = few(K, G, C, M), few(n, G, C), few(n, G, M)
+    y, gx = torch.zeros(n, G, M, dtype=torch.float64, device=DEV), torch.zeros(n, G, C, dtype=torch.float64, device=DEV)
+    for t in range(K):
+        s = slice(int(seg[t]), int(seg[t + 1]))
+        y.index_add_(0, i[s].long(), torch.einsum("tgc,gcm->tgm", x[j[s].long()].double(), w[t].double()))
+        gx.index_add_(0, i[s].long(), torch.einsum("tgm,gcm->tgc", go[j[s].long()].double(), w[t].double()))
+    assert max(y.abs().max(), gx.abs().max()) < 2048
+    got = _cabi.mvmr(w, x.flatten(1), j, i, seg, None, n, False, _cabi.ENGINE_PLANNED)
+    assert torch.equal(got.double(), y.flatten(1))
+    got = _cabi.mvmr(w, go.flatten(1), j, i, seg, None, n, True, _cabi.ENGINE_PLANNED)
+    assert torch.equal(got.double(), gx.flatten(1))
+    assert _cabi.device_status() == 0
