@@ -234,12 +234,14 @@ __global__ void plan_rank_kernel(const int32_t *__restrict__ row_sorted, int64_t
 }
 
 // ---- rulebooks whose rows ascend inside a tap (what the geometry stage emits): a (row, tap) bucket is a run of
-// consecutive triplets, so everything is placed by counting and no triplet is sorted.
+// consecutive triplets, so everything is placed by counting and no triplet is sorted.  Of any other rulebook these two kernels
+// touch nothing: placed in vain and cleared again, the strided rulebooks of a training step on 1.04 M points, taken backwards, cost 1.1 ms.
 
 // tile_rows[tile * 128 + slot] = first triplet of the bucket; triplets per tile
 __global__ void plan_heads_kernel(const int32_t *__restrict__ scatter, const int64_t *__restrict__ seg, const int32_t *__restrict__ rank,
-                                  int64_t T, int K, int32_t *tile_rows, int32_t *tile_cnt) {
+                                  int64_t T, int K, const uint32_t *__restrict__ ctrl, int32_t *tile_rows, int32_t *tile_cnt) {
     start_after_previous();
+    if (ctrl[CTRL_UNSORTED]) return;
     __shared__ int64_t s_seg[MAX_TAPS + 1];
     copy_seg(seg, K, s_seg);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -263,7 +265,7 @@ __global__ void plan_tiles_kernel(const int32_t *__restrict__ scatter, const int
     const int lane = threadIdx.x & 31;
     if (tile >= n_tiles) return;
     const int32_t first = tile_offs[tile];
-    if (tile_offs[tile + 1] == first) return;   // no triplets: its rows say "none" already
+    if (tile_offs[tile + 1] == first) return;   // no triplets, or none placed here: its rows say "none" already
     const int64_t end = seg[tile % K + 1];
     int4 *slots = reinterpret_cast<int4 *>(tile_rows + (tile << 7)) + lane;
     const int4 h = *slots;
@@ -1190,7 +1192,7 @@ int pcx_mvmr_plan_build_counted(const int32_t *d_scatter, const int32_t *d_gathe
     launch_after(plan_rank_kernel, blocks(n_pad), TPB, 0, stream, w.row_sorted, n_out, n_pad, w.rank, pv.perm);
     PCX_LAUNCH_CHECK();
     if (T > 0) {
-        launch_after(plan_heads_kernel, blocks(T), TPB, 0, stream, d_scatter, d_seg_offs, w.rank, T, K, pv.tile_rows, w.tile_cnt);
+        launch_after(plan_heads_kernel, blocks(T), TPB, 0, stream, d_scatter, d_seg_offs, w.rank, T, K, pv.ctrl, pv.tile_rows, w.tile_cnt);
         PCX_LAUNCH_CHECK();
     }
     bytes = w.cub_bytes;
@@ -1208,10 +1210,7 @@ int pcx_mvmr_plan_build_counted(const int32_t *d_scatter, const int32_t *d_gathe
     *h_multi = h[CTRL_NMULTI];
     if (!h[CTRL_UNSORTED]) return PCX_OK;
 
-    // rows out of order inside a tap: what comes after the row order once more, by sorting the triplets
-    PCX_CUDA(cudaMemsetAsync(pv.tile_rows, 0xff, (size_t)n_tiles * ROWS * sizeof(int32_t), stream));
-    PCX_CUDA(cudaMemsetAsync(w.tile_cnt, 0, (size_t)(n_tiles + 1) * sizeof(int32_t), stream));
-    PCX_CUDA(cudaMemsetAsync(pv.ctrl + CTRL_NMULTI, 0, sizeof(uint32_t), stream));
+    // rows out of order inside a tap: nothing has been placed yet, the triplets are sorted
     launch_after(plan_keys_kernel, blocks(T), TPB, 0, stream, d_scatter, d_gather, d_seg_offs, w.rank, T, K, w.key, w.val, w.tile_cnt);
     PCX_LAUNCH_CHECK();
     bytes = w.cub_bytes;
