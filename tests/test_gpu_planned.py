@@ -374,3 +374,35 @@ def test_small_clouds_split_by_taps_and_columns(n, G, C, M):
     got = _cabi.mvmr(w, go.flatten(1), j, i, seg, None, n, True, _cabi.ENGINE_PLANNED)
     assert torch.equal(got.double(), gx.flatten(1))
     assert _cabi.device_status() == 0
+
+
+@pytest.mark.parametrize("n", [65535, 65536, 65599, 150001, 1050000])   # below the clouds that are binned, the smallest, a last bin of a row, wider bins
+@pytest.mark.parametrize("shuffled", [False, True])                      # rows that lie together, and rows that do not
+def test_buckets_are_numbered_once_each(n, shuffled):
+    """Whatever order the buckets are numbered in: every number from 0 on is used by one slot of a tile, and its entries are those of
+    the slot's row, in the order of the rulebook."""
+    from pointelligence_b200 import _cabi
+
+    g = torch.Generator(device=DEV).manual_seed(n)
+    K, per = 8, 2   # of every tap, two triplets for two rows in three
+    rows = torch.arange(n, device=DEV)
+    rows = rows[rows % 3 != 0]
+    i = rows.repeat_interleave(per).repeat(K)
+    near = (i + torch.randint(-3, 4, (i.numel(),), device=DEV, generator=g)).clamp(0, n - 1)
+    j = torch.randint(0, n, (i.numel(),), device=DEV, generator=g) if shuffled else near
+    seg = torch.arange(K + 1, device=DEV) * (rows.numel() * per)
+    plan = _cabi.mvmr_plan(i.int(), j.int(), seg, K, n, 2)
+    v, T = plan.views(), i.numel()
+    m = rows.numel() * K
+    assert plan.multi_buckets == m
+    looked, near_ = int(v["ctrl"][16]), int(v["ctrl"][17])
+    assert (2 * near_ > looked) == (n >= 65536 and not shuffled)
+    where = (v["tile_rows"] < -1).nonzero()
+    ids = (-2 - v["tile_rows"][where[:, 0], where[:, 1]]).long()
+    assert torch.equal(torch.sort(ids).values, torch.arange(m, device=DEV))
+    row = v["perm"].view(-1, 128)[where[:, 0] // K, where[:, 1]].long()
+    first = v["buckets"][ids, 0].long()
+    assert (v["buckets"][ids, 1] == per).all()
+    at = (where[:, 0] % K) * (rows.numel() * per) + (row // 3 * 2 + row % 3 - 1) * per   # the row's first triplet of the tap
+    for p in range(per):
+        assert torch.equal(v["entries"][first + p, 1].long(), j[at + p])
