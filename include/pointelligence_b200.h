@@ -68,7 +68,7 @@ const char *pcx_last_error_string(void);
 
 /* Device-side status word: kernels that give up on a bounded wait set a bit
  * (1 = MVMR tensor kernel, 2 = VVOR tensor kernel, 4 = output-stationary MVMR
- * kernel, 8 = pcx_debug_wait_runs_out).  Synchronises `stream`,
+ * kernel, 8 = pcx_debug_wait_runs_out, 16 = thin MVMR kernel).  Synchronises `stream`,
  * copies the word to *h_status and clears it when `clear` is non-zero.
  * No counterpart in the reference (its kernels have no device-side waits). */
 int pcx_device_status(unsigned int *h_status, int clear, void *stream);
