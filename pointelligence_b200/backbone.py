@@ -29,6 +29,7 @@ from .layers import MetaData, PointConv3d, RaggedLayerNorm, Upsample
 from .layers.norm import fused_layer_norm
 from .layers.triplets import (build_triplets_segmented, handle_stride_and_build_triplets,
                               radius_scaler_for_kernel_size)
+from .sparse_engines.tig import _takes_host_path
 
 RFS = 2.5   # receptive_field_scaler of every convolution, as in the reference's model
 
@@ -36,21 +37,42 @@ RFS = 2.5   # receptive_field_scaler of every convolution, as in the reference's
 _cast = threading.local()
 
 
+def _hooked(modules):
+    shared = nn.modules.module
+    return bool(shared._global_forward_pre_hooks or shared._global_forward_hooks
+                or any(mod._forward_pre_hooks or mod._forward_hooks for mod in modules))
+
+
 @contextmanager
-def weights_cast_together(convs):
-    """Inside, ``convs`` take their bf16 weights from one cast (without gradients): a launch for all of them, not one each."""
-    together = [c for c in convs if c.weight.is_cuda and c.weight.dtype is torch.float32 and c.weight.numel() % 8 == 0]   # (16-byte addresses)
-    if torch.is_grad_enabled() or len(together) < 2 or torch.compiler.is_compiling() or len({c.weight.device for c in together}) > 1:
+def weights_cast_together(network):
+    """Inside, and without gradients, the layers of ``network`` find their bf16 weights in one cast: a launch for all of them, not
+    one each.  A layer takes it only while its weight is the tensor that was cast, with nothing written to it since; where a hook
+    could run between the cast and the layer, or a weight is anything but the layer's own parameter, the layer casts by itself."""
+    modules = [] if torch.is_grad_enabled() or torch.compiler.is_compiling() else list(network.modules())
+    own = [(mod, mod._parameters.get("weight")) for mod in modules if type(mod) is Bf16PointConv3d]
+    own = [(mod, w) for mod, w in own if w is not None and w.dtype is torch.float32 and w.numel() % 8 == 0 and not w.is_inference()]   # (16-byte addresses)
+    if len(own) < 2 or len({w.device for _, w in own}) > 1 or not _takes_host_path(*[w for _, w in own]) or _hooked(modules):
         yield
         return
-    flat = torch.cat([c.weight.detach().reshape(-1) for c in together]).to(torch.bfloat16)
-    parts = flat.split([c.weight.numel() for c in together])
+    flat = torch.cat([w.detach().reshape(-1) for _, w in own]).to(torch.bfloat16)
+    parts = flat.split([w.numel() for _, w in own])
     outer = getattr(_cast, "weights", None)
-    _cast.weights = {id(c): p.view(c.weight.shape) for c, p in zip(together, parts)}
+    _cast.weights = {id(mod): (w, w.data_ptr(), w._version, part.view(w.shape)) for (mod, w), part in zip(own, parts)}
     try:
         yield
     finally:
         _cast.weights = outer
+
+
+def _joint_cast(conv):
+    """The layer's weight of ``weights_cast_together``; None where there is none, or the weight is another by now."""
+    kept = getattr(_cast, "weights", None)
+    hit = kept.get(id(conv)) if kept and not torch.is_grad_enabled() else None
+    if hit is None:
+        return None
+    weight, address, version, cast = hit
+    now = conv.weight
+    return cast if now is weight and now.data_ptr() == address and now._version == version else None
 
 
 class Bf16PointConv3d(PointConv3d):
@@ -58,8 +80,7 @@ class Bf16PointConv3d(PointConv3d):
     input is taken as bf16."""
 
     def forward(self, input, i, j, k, n, contract=None, seg_offs=None):
-        together = getattr(_cast, "weights", None)
-        w = together.get(id(self)) if together and not torch.is_grad_enabled() else None
+        w = _joint_cast(self)
         if w is None:
             w = self.weight.to(torch.bfloat16)
         x = input.to(torch.bfloat16)
@@ -174,8 +195,7 @@ class ResUNet(nn.Module):
         # and the geometry of a level is built on a stream of its own while the feature kernels of
         # the level before it are still running (every point cloud of the network derives from
         # the input cloud through the library's geometry calls alone)
-        convs = [mod for mod in self.modules() if isinstance(mod, Bf16PointConv3d)] if not torch.is_grad_enabled() else []
-        with triplet_cache_scope(), _cabi.geometry_overlap(points.device), weights_cast_together(convs):
+        with triplet_cache_scope(), _cabi.geometry_overlap(points.device), weights_cast_together(self):
             return self._forward(feat, points, sample_inds, sample_sizes, grid_size)
 
     def _forward(self, feat, points, sample_inds, sample_sizes, grid_size):

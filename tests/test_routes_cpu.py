@@ -223,3 +223,30 @@ def test_wide_and_grouped_layers_are_captured_on_the_scatter_kernels(monkeypatch
     (18_900_000, 141_000, 384, 128, True), (18_900_000, 141_000, 384, 1024, False)])  # 15 GB of sums
 def test_rulebooks_on_which_two_part_sums_pay(T, n, outw, inw, pays):
     assert _cabi._planned_pays(T, n, outw, 27) and _cabi._split_pays(T, n, outw, inw, 27) is pays
+
+
+def test_joined_casts_are_those_of_the_weights_as_they_are(monkeypatch):
+    """(The library's kernels do not run: the check for CUDA tensors is taken out.)"""
+    from torch.nn.utils import prune
+
+    from pointelligence_b200 import backbone
+
+    monkeypatch.setattr(backbone, "_takes_host_path", lambda *tensors: True)
+    make = lambda: torch.nn.Sequential(*(backbone.Bf16PointConv3d(16, width, 3) for width in (16, 24, 8)))
+    changes = [lambda c: c.weight.add_(1), lambda c: setattr(c.weight, "data", torch.zeros_like(c.weight)),
+               lambda c: setattr(c, "weight", torch.nn.Parameter(c.weight.clone()))]
+    for change in changes:
+        net = make()
+        with torch.no_grad(), backbone.weights_cast_together(net):
+            assert all(torch.equal(backbone._joint_cast(c), c.weight.bfloat16()) for c in net)
+            with torch.enable_grad():
+                assert backbone._joint_cast(net[0]) is None
+            change(net[1])
+            assert backbone._joint_cast(net[1]) is None and backbone._joint_cast(net[0]) is not None
+    nets = [make() for _ in range(3)]
+    prune.random_unstructured(nets[0][2], "weight", 0.3)
+    nets[1].register_forward_pre_hook(lambda *_: None)
+    nets[2][1].register_forward_hook(lambda *_: None)
+    for net in nets:
+        with torch.no_grad(), backbone.weights_cast_together(net):
+            assert all(backbone._joint_cast(c) is None for c in net)
