@@ -21,6 +21,7 @@ from typing import List, Sequence, Tuple
 
 import torch
 import torch.nn as nn
+import torch.nn.functional as F
 from torch import Tensor
 
 from . import _cabi
@@ -77,14 +78,25 @@ def _joint_cast(conv):
 
 class Bf16PointConv3d(PointConv3d):
     """``PointConv3d`` with bf16 operands: the fp32 master weight is cast on the fly and the
-    input is taken as bf16."""
+    input is taken as bf16.  Channel counts that are not multiples of 16 (the 3-channel input, the
+    class logits) take the engines of the next ones, with columns of zeros: padded by the host path, or here
+    where calls are traced or transformed."""
+
+    _plan_padded = True
 
     def forward(self, input, i, j, k, n, contract=None, seg_offs=None):
         w = _joint_cast(self)
         if w is None:
             w = self.weight.to(torch.bfloat16)
         x = input.to(torch.bfloat16)
+        G, C, M = w.shape[1:]
+        pad_here = G == 1 and (C % 16 or M % 16) and not _takes_host_path(w, x, i, j, seg_offs)
+        if pad_here:
+            w = F.pad(w, (0, -M % 16, 0, -C % 16))
+            x = F.pad(x, (0, -C % 16))
         out = self._conv_forward(x, i, j, k, n, w, None, contract=contract, seg_offs=seg_offs)
+        if pad_here:
+            out = out.view(n, -1)[:, :M]
         if self.bias is not None:
             out = out + self.bias.to(out.dtype)
         return out

@@ -140,6 +140,9 @@ bool plan_fits(at::ScalarType dtype, int64_t T, int64_t n_out, int64_t K, int64_
 
 constexpr int ENGINE_PLANNED = 3;
 constexpr int64_t NO_PLAN = 0x200;   // internal flag of an engine: the automatic choice is between the scatter engines
+// ... and of the automatic choice: a layer of widths that have to be padded takes the engines of the padded widths, the
+// output-stationary kernel included (the caller's operands are bf16 copies, whose sums it may round)
+constexpr int64_t PLAN_PADDED = 0x400;
 
 // Shapes the automatic choice may give to the output-stationary kernel.  It rounds the sums of (row, tap) buckets to 16
 // bits; grouped, padded and wider layers multiply their operands as they are unless the caller asks for that kernel.
@@ -224,6 +227,8 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
     const bool transpose = flags & 1;
     const int64_t inw = transpose ? M : C, outw = transpose ? C : M, T = gather_.numel();
     c10::cuda::CUDAGuard guard(feat.device());
+    const bool plan_padded = engine & PLAN_PADDED && padded(C) == (C + 15) / 16 * 16 && padded(M) == (M + 15) / 16 * 16;
+    engine &= ~PLAN_PADDED;
     if (engine == 0 && seg_ && thin_pays(feat.scalar_type(), T, feat.size(0), n_out, K, G, inw, outw) &&
         // (a captured pass is replayed on whatever the index tensors hold then: on the kernels that take any order)
         c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None && rows_ascend(scatter_, gather_, *seg_, K)) {
@@ -244,7 +249,7 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
         const Tensor w = reshape16(weight, K * G, C, M, Cp, Mp, {K, G, Cp, Mp});
         const Tensor x = inp == inw ? feat : reshape16(feat, feat.size(0) * G, 1, inw, 1, inp, {feat.size(0), G * inp});
         const Tensor b = !bias.defined() || outp == outw ? bias : reshape16(bias, G, 1, outw, 1, outp, {G * outp});
-        const Tensor y = mvmr_impl(w, x, gather_, scatter_, seg_, tap_, n_out, flags, engine | NO_PLAN, b);
+        const Tensor y = mvmr_impl(w, x, gather_, scatter_, seg_, tap_, n_out, flags, plan_padded ? engine : engine | NO_PLAN, b);
         return outp == outw ? y : reshape16(y, n_out * G, 1, outp, 1, outw, {n_out, G * outw});
     }
     if (engine == 0 || engine == ENGINE_PLANNED) {
@@ -339,7 +344,8 @@ void match(Tensor &w, Tensor &x) {
 
 struct ConvSizes {
     int64_t n_out, n_in, K;
-    bool cover_out, cover_in;
+    bool cover_out, cover_in, plan_padded;
+    int64_t engine() const { return plan_padded && g_engine == 0 ? PLAN_PADDED : (int64_t)g_engine; }
 };
 
 Tensor as4(const Tensor &w) { return w.dim() == 4 ? w : w.unsqueeze(1); }
@@ -358,7 +364,7 @@ Tensor conv_forward(const Tensor &weight, const Tensor &feat, const Tensor &bias
     require(!bias.defined() || (bias.dim() == 1 && bias.numel() == w.size(1) * w.size(3) && bias.device() == x.device() &&
                                 bias.scalar_type() == x.scalar_type()),   // the kernels read it by address
             PyExc_ValueError, [&] { return "the bias does not fit a weight " + str(weight.sizes()); });
-    int64_t engine = g_engine;
+    int64_t engine = s.engine();
     if (s.cover_out && i.numel() == s.n_out) engine |= FAN_IN_ONE;   // one triplet per output row: stored, not reduced
     return mvmr_impl(w, x, j, i, seg, std::nullopt, s.n_out, 0, engine, bias.defined() ? bias.contiguous() : bias)
         .to(feat.scalar_type());
@@ -368,7 +374,7 @@ Tensor conv_grad_input(const Tensor &weight, const Tensor &grad, const Tensor &i
                        const ConvSizes &s) {
     Tensor w = as4(weight), g = grad;
     match(w, g);
-    int64_t engine = g_engine;
+    int64_t engine = s.engine();
     // a self-search rulebook holds (j, i, K - 1 - k) with every (i, j, k): the input gradient is the forward
     // schedule over the same rulebook (and the same plan) with the taps of the weight in reverse order
     if (s.n_out == s.n_in && is_symmetric(i, j, s.K))
@@ -391,18 +397,18 @@ Tensor conv_grad_weight(const Tensor &feat, const Tensor &grad, const Tensor &i,
 struct Conv : public torch::autograd::Function<Conv> {
     static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &weight, const Tensor &feat, const OptTensor &bias,
                           const Tensor &i, const Tensor &j, const Tensor &seg, int64_t n_out, int64_t n_in, int64_t K,
-                          bool cover_out, bool cover_in) {
+                          bool cover_out, bool cover_in, bool plan_padded) {
         ctx->save_for_backward({weight, feat, i, j, seg});
-        ctx->saved_data["sizes"] = std::vector<int64_t>{n_out, n_in, K, cover_out, cover_in, bias.has_value()};
-        return conv_forward(weight, feat, bias ? *bias : Tensor(), i, j, seg, {n_out, n_in, K, cover_out, cover_in});
+        ctx->saved_data["sizes"] = std::vector<int64_t>{n_out, n_in, K, cover_out, cover_in, bias.has_value(), plan_padded};
+        return conv_forward(weight, feat, bias ? *bias : Tensor(), i, j, seg, {n_out, n_in, K, cover_out, cover_in, plan_padded});
     }
 
     static torch::autograd::variable_list backward(torch::autograd::AutogradContext *ctx, torch::autograd::variable_list grads) {
         const auto saved = ctx->get_saved_variables();
         const Tensor &weight = saved[0], &feat = saved[1], &i = saved[2], &j = saved[3], &seg = saved[4];
         const auto v = ctx->saved_data["sizes"].toIntVector();
-        const ConvSizes s{v[0], v[1], v[2], v[3] != 0, v[4] != 0};
-        torch::autograd::variable_list out(11);
+        const ConvSizes s{v[0], v[1], v[2], v[3] != 0, v[4] != 0, v[6] != 0};
+        torch::autograd::variable_list out(12);
         if (!grads[0].defined()) return out;
         const Tensor &go = grads[0];
         const bool want_w = ctx->needs_input_grad(0), want_x = ctx->needs_input_grad(1), want_b = v[5] && ctx->needs_input_grad(2);
@@ -424,11 +430,11 @@ struct Conv : public torch::autograd::Function<Conv> {
 };
 
 Tensor conv(const Tensor &weight, const Tensor &feat, const OptTensor &bias, const Tensor &i, const Tensor &j, const Tensor &seg,
-            int64_t n_out, int64_t n_in, int64_t K, bool cover_out, bool cover_in) {
+            int64_t n_out, int64_t n_in, int64_t K, bool cover_out, bool cover_in, bool plan_padded) {
     if (!at::GradMode::is_enabled() ||
         !(weight.requires_grad() || feat.requires_grad() || (bias && bias->requires_grad())))
-        return conv_forward(weight, feat, bias ? *bias : Tensor(), i, j, seg, {n_out, n_in, K, cover_out, cover_in});
-    return Conv::apply(weight, feat, bias, i, j, seg, n_out, n_in, K, cover_out, cover_in);
+        return conv_forward(weight, feat, bias ? *bias : Tensor(), i, j, seg, {n_out, n_in, K, cover_out, cover_in, plan_padded});
+    return Conv::apply(weight, feat, bias, i, j, seg, n_out, n_in, K, cover_out, cover_in, plan_padded);
 }
 
 // --------------------------------------------------- ragged layer norm (autograd) ----
@@ -690,7 +696,8 @@ PYBIND11_MODULE(_pcx_host, m) {
     m.def("set_engine", [](int e) { g_engine = e; });
     m.def("mvmr", &mvmr);
     m.def("vvor", &vvor);
-    m.def("conv", &conv);
+    m.def("conv", &conv, py::arg("weight"), py::arg("feat"), py::arg("bias"), py::arg("i"), py::arg("j"), py::arg("seg"), py::arg("n_out"),
+          py::arg("n_in"), py::arg("K"), py::arg("cover_out"), py::arg("cover_in"), py::arg("plan_padded") = false);
     m.def("column_sums", &column_sums);
     m.def("layer_norm", &layer_norm);
     m.def("radius_taps", &radius_taps, py::call_guard<py::gil_scoped_release>());

@@ -77,6 +77,8 @@ class GeneralConv(Module):
             s += ", bias=False"
         return s
 
+    _plan_padded = False   # see tig_mvmr
+
     def _conv_forward(self, input: Tensor, i: Tensor, j: Tensor, k: Tensor, n: int, weight: Tensor,
                       bias: Optional[Tensor], *, contract: Optional[TripletContract] = None,
                       seg_offs: Optional[Tensor] = None) -> Tensor:
@@ -105,7 +107,7 @@ class GeneralConv(Module):
                                exact_cover_out=contract.exact_cover_out,
                                exact_cover_in=contract.exact_cover_in)
             output = tig_mvmr(weight, x3.view(n_in, -1), idx,
-                              input_precision=resolve_input_precision(x3.dtype), bias=bias)
+                              input_precision=resolve_input_precision(x3.dtype), bias=bias, plan_padded=self._plan_padded)
             bias = None
         else:
             output = sparse_matrix_vector_multiplication_reduction(weight, k, x3, j, i, n)

@@ -183,14 +183,16 @@ def _fuses(bias, weight, feat):
     return bias.shape == (columns,) and bias.dtype == feat.dtype == weight.dtype
 
 
-def tig_mvmr(weight, feat, index, mode="auto", input_precision: Optional[str] = None, bias: Optional[Tensor] = None):
+def tig_mvmr(weight, feat, index, mode="auto", input_precision: Optional[str] = None, bias: Optional[Tensor] = None,
+             plan_padded: bool = False):
     """Differentiable tap-sorted convolution: one autograd node, three kernel
     families (forward MVMR, transposed MVMR, VVOR).  A ``bias`` of the output's type is added
-    before the rows are rounded."""
+    before the rows are rounded.  ``plan_padded``: widths that are not multiples of 16 may take the
+    output-stationary kernel as the padded widths would (plain eager calls; else the caller pads)."""
     if _takes_host_path(weight, feat, bias, index.flat_i, index.flat_j, index.flat_seg) and (
             bias is None or _fuses(bias, weight, feat)):
         return _cabi.host().conv(weight, feat, bias, index.flat_i, index.flat_j, index.flat_seg, index.N, index.N_in,
-                                 index.K, index.exact_cover_out, index.exact_cover_in)
+                                 index.K, index.exact_cover_out, index.exact_cover_in, plan_padded)
     if bias is not None:
         return tig_mvmr(weight, feat, index, mode, input_precision) + bias
     if input_precision is None:

@@ -142,3 +142,68 @@ def test_weights_computed_on_use_and_networks_inside_networks(scene):
     with torch.inference_mode():
         got = net.first(*scene)
     assert _same(got, net.first(*scene).detach())
+
+
+def _kernels(call):
+    from pointelligence_b200 import _cabi
+
+    _cabi.profile_enable(True)
+    out = call()
+    torch.cuda.synchronize()
+    names = [n for n, _ in _cabi.profile_records()]
+    _cabi.profile_enable(False)
+    return out, names
+
+
+@pytest.mark.parametrize("C,M", [(24, 40), (40, 24), (3, 24), (24, 6), (40, 40)])
+def test_padded_widths_choose_their_kernels_like_others(C, M):
+    """A dense rulebook (about 17 triplets a row of 27 taps): the output-stationary kernel, which a layer of the next
+    multiples of 16 takes in both directions; three input channels forward, and six output channels backward, take the
+    kernel of thin layers instead."""
+    from pointelligence_b200.backbone import Bf16PointConv3d
+    from pointelligence_b200.layers import MetaData, PointConv3d
+    from pointelligence_b200.layers.triplets import handle_stride_and_build_triplets
+
+    g = torch.Generator(device="cuda").manual_seed(C + M)
+    pts = torch.rand(6000, 3, device="cuda", generator=g)
+    m = MetaData(points=pts, sample_inds=torch.zeros(6000, dtype=torch.int64, device="cuda"),
+                 sample_sizes=torch.tensor([6000], device="cuda"), grid_size=0.0362)
+    m = handle_stride_and_build_triplets(m, 1.0, (3, 3, 3), 2.5)
+    assert 13 < m.i.numel() / 6000 < 30
+    conv = Bf16PointConv3d(C, M, 3, device="cuda")
+    x = torch.randn(6000, C, device="cuda", generator=g).bfloat16().requires_grad_()
+    go = torch.randn(6000, M, device="cuda", generator=g).bfloat16()
+    y, forward = _kernels(lambda: conv(x, m.i, m.j, m.k, 6000, contract=m.contract, seg_offs=m.seg_offs))
+    (gx, gw), backward = _kernels(lambda: torch.autograd.grad(y, (x, conv.weight), go))
+    convolutions = lambda names: [n.split("(")[0] for n in names if n.startswith(("bucket_sum", "mvmr_"))]
+    assert convolutions(forward) == (["mvmr_thin_kernel"] if C <= 8 else ["bucket_sum_kernel", "mvmr_os_kernel"])
+    assert convolutions(backward) == (["mvmr_thin_kernel"] if M <= 8 else ["bucket_sum_kernel", "mvmr_os_kernel"])
+    w64, x64 = conv.weight.detach().bfloat16().double()[:, 0], x.detach().double()
+    ref, gref, wref = torch.zeros(6000, M, device="cuda").double(), torch.zeros(6000, C, device="cuda").double(), torch.zeros_like(w64)
+    for t in range(27):
+        s = slice(int(m.seg_offs[t]), int(m.seg_offs[t + 1]))
+        ref.index_add_(0, m.i[s].long(), x64[m.j[s].long()] @ w64[t])
+        gref.index_add_(0, m.j[s].long(), go[m.i[s].long()].double() @ w64[t].t())
+        wref[t] = x64[m.j[s].long()].t() @ go[m.i[s].long()].double()
+    # sums of a (row, tap) rounded to bf16, their products summed in fp32, rounded: two roundings of 2^-9
+    for a, r in ((y.detach() - conv.bias.detach().bfloat16(), ref), (gx, gref), (gw[:, 0], wref)):
+        assert a.shape == r.shape and float((a.double() - r).norm() / r.norm()) < 1.5 * 2.0 ** -8
+    # other layers of such widths keep exact operands
+    plain = PointConv3d(C, M, 3, device="cuda", dtype=torch.bfloat16)
+    _, names = _kernels(lambda: plain(x, m.i, m.j, m.k, 6000, contract=m.contract, seg_offs=m.seg_offs))
+    assert "mvmr_os_kernel" not in convolutions(names)
+
+
+def test_network_of_padded_widths(scene):
+    from pointelligence_b200.backbone import ResUNet
+
+    torch.manual_seed(0)
+    model = ResUNet(in_channels=5, num_classes=13, base_channels=24, channels=(24, 40, 40, 72), tr_channels=(24, 40, 56, 72), layers=(1,) * 8).cuda()
+    feat = torch.randn(scene[0].shape[0], 5, device="cuda")
+    with torch.no_grad():
+        got, names = _kernels(lambda: model(feat, *scene[1:4], 0.1))
+    assert any(n.startswith("mvmr_os_kernel") for n in names)
+    logits = model(feat, *scene[1:4], 0.1)
+    assert logits.shape == (feat.shape[0], 13) and _same(got, logits.detach())
+    logits.float().square().mean().backward()
+    assert all(p.grad is not None and bool(p.grad.isfinite().all()) for p in model.parameters())
