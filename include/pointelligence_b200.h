@@ -255,9 +255,12 @@ int pcx_mvmr_split(const void *d_weight, const void *d_feat,
  * channels, 0 < T < 2^27 - 1) on a rulebook whose output rows ascend inside every
  * tap, as the searches write them (nothing checks it: where they do not, triplets
  * are left out).  The sums of a row stay on the chip, operands are multiplied as
- * they are and a row is rounded once.  Weights that are not finite are worked off
- * triplet by triplet, slowly.  Features and weights may lie at any address of
- * their type. */
+ * they are and a row is rounded once.  Where more than eight triplets share a row
+ * and a tap their features are added up in fp32 first, without loss from there on;
+ * pcx_mvmr_thin_workspace_bytes has room for n_out such sums, 48 bytes more than
+ * that hold one more each, and what has no room, or leaves the type's range, takes
+ * a step for every triplet.  Weights that are not finite are worked off triplet by
+ * triplet, slowly.  Features and weights may lie at any address of their type. */
 size_t pcx_mvmr_thin_workspace_bytes(int64_t n_feat, int64_t n_out, int K,
                                      int C, int M, int transpose);
 int pcx_mvmr_thin(const void *d_weight, const void *d_feat,

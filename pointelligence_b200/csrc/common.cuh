@@ -66,9 +66,11 @@ void prof_end(cudaStream_t stream);
 // when the kernel before it ends: a training call of 942 points and 512 channels 166 -> 159 us.
 // A gap between kernels shrinks by 1 to 1.5 us: a training call of 942 points and 512 channels (11 launches) 230 -> 214 us,
 // 150 000 points and 64 channels (11) 224 -> 212, an fp32 one (8) 204 -> 194, a norm with its gradient (7) 229 -> 215.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_be_set_up() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void start_after_previous() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    wait_for_previous();
+    let_next_be_set_up();
 }
 template <typename... Params, typename... Args>
 void launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args) {

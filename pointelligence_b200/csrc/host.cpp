@@ -234,7 +234,8 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
         c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None && rows_ascend(scatter_, gather_, *seg_, K)) {
         const Tensor gather = as_i32(gather_), scatter = as_i32(scatter_), seg = as_i64(*seg_);
         Tensor out = at::empty({n_out, outw}, feat.options());
-        Tensor ws = workspace(pcx_mvmr_thin_workspace_bytes(feat.size(0), n_out, (int)K, (int)C, (int)M, transpose), feat);
+        // (a sum of triplets, 48 bytes, is made of nine or more)
+        Tensor ws = workspace(pcx_mvmr_thin_workspace_bytes(feat.size(0), n_out, (int)K, (int)C, (int)M, transpose) + 48 * std::max<int64_t>(T / 9 - n_out, 0), feat);
         check(pcx_mvmr_thin(ptr(weight), ptr(feat), ptr_as<int32_t>(gather), ptr_as<int32_t>(scatter), ptr_as<int64_t>(seg), ptr(bias), ptr(out),
                             T, feat.size(0), n_out, (int)K, (int)C, (int)M, flags, code, ptr(ws), ws.numel(), stream()));
         return out;

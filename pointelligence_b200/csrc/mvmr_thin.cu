@@ -4,11 +4,16 @@
 // Here the sums of 128 consecutive output rows stay in tensor memory: the operand of a block is the matrix (128 rows) x
 // (taps x 8 channels), a row's features of all its taps side by side, built 64 columns at a time in shared memory, and
 // multiplied with the weights as one long contraction.  No plan, no accumulator to clear, to add
-// to or to round, and operands as they are: nothing is summed before it is multiplied.
+// to or to round, and operands as they are: up to eight triplets of a (row, tap) are multiplied one by one.
 //
 //   preparation   two kernels: the table of a block, [tap][row], holds a feature row, where a (row, tap) has one triplet, or
 //                 the first of its several triplets and their number (rows ascend inside a tap, so that they are neighbours);
 //                 the weights as the tiles that the tensor core reads; feature rows of eight channels
+//   clumps        the features of more than eight triplets are added up in fp32, and the sum is handed on as three 16-bit rows that
+//                 hold all its bits, so that a step is taken for at most eight triplets, not for each of the fullest (row, tap)
+//                 of 128 rows and eight taps: 100 000 points, of which 200 / 400 / 1000 lie within a centimetre, rows in random order,
+//                 27 taps, 6 -> 64 channels 269 / 567 / 1474 -> 56 / 59 / 69 us (scatter kernel 61 / 74 / 144).  Sums beyond the
+//                 type's range (and infinities, NaN) stay triplets
 //   copies        eight warps, eight taps a step: every (row, tap) a 16-byte copy, or zeros, straight into the
 //                 128-byte-swizzled tile.  Where a (row, tap) has several triplets the columns take a step for the
 //                 first of each, one for the second of those that have one, and so on
@@ -16,7 +21,7 @@
 //   epilogue      tensor memory + bias, rounded once, rows written side by side
 //
 // 80 000 points, 125 taps, 3.3 M triplets, 6 -> 32 channels: 170 us on the scatter kernel with its padded copies, clear and rounding,
-// 146 here (preparation 8 and 18, this kernel 117).  A step takes some 2000 clocks of a CTA, three of which share an SM: bound
+// 142 here (preparation 8 and 18, this kernel 116).  A step takes some 2000 clocks of a CTA, three of which share an SM: bound
 // by the load/store unit and by the fill warps' own instructions.  16-byte copies of 32 rows are taken a lane a clock, whether or
 // not a lane has a source, so that zeros are stores.  Slower: tables of a block built by warps beside the copies (in three
 // forms, 107 -> 190 us of the kernel at 3 M triplets), second triplets multiplied by the warp that finds them and added in shared
@@ -43,17 +48,21 @@ constexpr int MAX_TAPS = 512, MAX_N = 64, MAX_WIDTH = 1024;
 constexpr int SLOTS = 3;                              // operand tiles on their way or in use
 constexpr int WARPS = 8, MMA_WARP = WARPS, THREADS = (WARPS + 1) * 32, CTAS = 3;   // CTAs of an SM
 constexpr int PREP_THREADS = 256, PREP_CTAS = 8;      // of an SM
-// an entry of the table: a feature row; none; or the first of several triplets | their number - 2 << 27 | 1 << 31
+// an entry of the table: a feature row; none; or 1 << 31 | a code << 27 | the first of several triplets, or the number of a sum.
+// The code is the number of triplets - 2, or:
 constexpr int32_t NONE = -1;
-constexpr int FIRST_BITS = 27, MOST = 17;             // 17: that many or more
+constexpr int FIRST_BITS = 27, LISTED = 8;            // triplets that are multiplied one by one, at most
+constexpr int MORE = 14, SUMMED = 15;                 // more than that, to be counted; the sum of more than that
 constexpr int64_t MAX_T = ((int64_t)1 << FIRST_BITS) - 1;
+constexpr int PARTS = 3;                              // rows of a sum: 3 x 8 bits of bf16, 3 x 11 of fp16
+constexpr size_t SUM_BYTES = PARTS * CW * 2;
 
 struct ThinParams {
-    const uint16_t *feat;                 // rows of CW elements
+    const uint16_t *feat;                 // rows of CW elements: the points, then PARTS for every sum
     const int32_t *gather, *scatter;
     const int64_t *seg;
     const int32_t *table;                 // [block][tap][row]
-    const int32_t *most;                  // [block][slot]: triplets of the fullest (row, tap), at least 1
+    const int2 *most;                     // [block][slot]: steps of the fullest (row, tap), at least 1; whether codes are beyond LISTED
     const uint16_t *image;                // [part][slot][N][64]: the weights' tiles, swizzled
     const uint32_t *odd;                  // whether weights are not finite, a word for each block of the preparation
     const uint16_t *bias;
@@ -62,17 +71,20 @@ struct ThinParams {
     int64_t n_out;
     int K, nq, N, width, nblocks, n_odd, fmt;   // nq: slots (of 64 columns) of a block; N: output channels of a part; width: all
     uint32_t ncols, col_stride, slot_bytes;
+    uint32_t first_sum;                   // row of the first sum
 };
 
 struct PrepParams {
     const uint16_t *weight, *feat_in;
-    uint16_t *feat;                       // null: the features' rows are taken as they are
+    uint16_t *feat;
     const int32_t *scatter, *gather;
     const int64_t *seg;
-    int32_t *table, *most;
+    int32_t *table;
+    int2 *most;
     uint16_t *image;
-    uint32_t *odd;
-    int64_t T, n_feat, image_pieces, feat_pieces, table_pieces, most_pieces;
+    uint32_t *odd, *n_sums;
+    int64_t T, n_feat, image_pieces, table_pieces, most_pieces;
+    uint32_t max_sums;
     int K, inw, width, nq, N, transpose, reverse, fmt;
 };
 
@@ -93,7 +105,7 @@ __global__ void __launch_bounds__(PREP_THREADS) thin_prepare_kernel(PrepParams p
     start_after_previous();
     const int64_t x0 = blockIdx.x * (int64_t)PREP_THREADS + threadIdx.x, threads = (int64_t)gridDim.x * PREP_THREADS;
     for (int64_t x = x0; x < p.table_pieces; x += threads) reinterpret_cast<int4 *>(p.table)[x] = make_int4(NONE, NONE, NONE, NONE);
-    for (int64_t x = x0; x < p.most_pieces; x += threads) p.most[x] = 1;
+    for (int64_t x = x0; x < p.most_pieces; x += threads) p.most[x] = make_int2(1, 0);
     bool odd = false;
     for (int64_t x = x0; x < p.image_pieces; x += threads) {
         // [part][slot][n][piece]
@@ -115,7 +127,8 @@ __global__ void __launch_bounds__(PREP_THREADS) thin_prepare_kernel(PrepParams p
         // (N is a multiple of 16, so that rows of a tile keep their place modulo 8)
         reinterpret_cast<uint4 *>(p.image)[(x >> 3) * 8 + (piece ^ (n & 7))] = make_uint4(v[0], v[1], v[2], v[3]);
     }
-    for (int64_t x = x0; x < p.feat_pieces; x += threads) {
+    if (x0 == 0) *p.n_sums = 0u;
+    for (int64_t x = x0; x < p.n_feat; x += threads) {
         uint32_t v[4] = {0u, 0u, 0u, 0u};
 #pragma unroll
         for (int e = 0; e < 8; ++e)
@@ -126,19 +139,84 @@ __global__ void __launch_bounds__(PREP_THREADS) thin_prepare_kernel(PrepParams p
     if (threadIdx.x == 0) p.odd[blockIdx.x] = (uint32_t)any;
 }
 
-// The first triplet of every (row, tap) enters the table.
-__global__ void __launch_bounds__(PREP_THREADS) thin_table_kernel(PrepParams p) {
-    start_after_previous();
+// The triplets from `first` on that have this row (of the tap that ends at `end`), by a whole warp: what enters the table for
+// them, and the steps that takes.  An iteration takes 64, three loads one after the other: a clump of 400 points among 100 000 takes 8 us,
+// one of 1000 17.
+__device__ __forceinline__ int2 sum_up(const PrepParams &p, int64_t first, int64_t end, int32_t row) {
+    const int lane = threadIdx.x & 31;
+    float sum[CW];
+#pragma unroll
+    for (int c = 0; c < CW; ++c) sum[c] = 0.f;
+    int n = 0;
+    for (int64_t t0 = first;; t0 += 64) {
+        bool mine[2];
+        uint4 v[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const int64_t t = t0 + 32 * u + lane;
+            mine[u] = t < end && __ldg(p.scatter + t) == row;
+            v[u] = mine[u] ? *reinterpret_cast<const uint4 *>(p.feat + (int64_t)__ldg(p.gather + t) * CW) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            const uint32_t word[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+            for (int c = 0; c < CW; ++c)
+                if (mine[u]) sum[c] += widen_one(word[c >> 1] >> (16 * (c & 1)) & 0xffffu, p.fmt);
+        }
+        n += __popc(__ballot_sync(0xffffffffu, mine[0])) + __popc(__ballot_sync(0xffffffffu, mine[1]));
+        if (!__all_sync(0xffffffffu, mine[1])) break;   // (they are neighbours)
+    }
+    uint32_t word[4] = {0u, 0u, 0u, 0u};   // lane q: part q
+    bool in_range = true;
+#pragma unroll
+    for (int c = 0; c < CW; ++c) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum[c] += __shfl_xor_sync(0xffffffffu, sum[c], o);
+        float rest = sum[c];
+#pragma unroll
+        for (int q = 0; q < PARTS; ++q) {   // (each difference is exact, the last part leaves none)
+            const uint32_t part = pack2(rest, 0.f, p.fmt) & 0xffffu, most = p.fmt ? 0x7f80u : 0x7c00u;
+            rest -= widen_one(part, p.fmt);
+            if (q == 0) in_range = in_range && (part & most) != most;
+            if (q == lane) word[c >> 1] |= part << (16 * (c & 1));
+        }
+    }
+    uint32_t id = p.max_sums;
+    if (in_range) {
+        if (lane == 0) id = atomicAdd(p.n_sums, 1u);
+        id = __shfl_sync(0xffffffffu, id, 0);
+    }
+    if (id >= p.max_sums) return make_int2((int32_t)(1u << 31 | (uint32_t)MORE << FIRST_BITS | (uint32_t)first), n);
+    if (lane < PARTS) *reinterpret_cast<uint4 *>(p.feat + (p.n_feat + (int64_t)id * PARTS + lane) * CW) = make_uint4(word[0], word[1], word[2], word[3]);
+    return make_int2((int32_t)(1u << 31 | (uint32_t)SUMMED << FIRST_BITS | id), PARTS);
+}
+
+// The first triplet of every (row, tap) enters the table, or the sum of its triplets.
+__global__ void __launch_bounds__(PREP_THREADS, 8) thin_table_kernel(const __grid_constant__ PrepParams p) {
+    wait_for_previous();
     constexpr int EACH = 4;   // triplets of a thread
+    constexpr int CLUMPS = (32 * EACH + LISTED) / (LISTED + 1);   // runs of more than LISTED that begin among the triplets of a warp
     __shared__ int64_t s_seg[MAX_TAPS + 1];
+    __shared__ int4 s_clump[PREP_THREADS / 32][CLUMPS];   // first triplet, tap, row
+    __shared__ int s_clumps[PREP_THREADS / 32];
     for (int k = threadIdx.x; k <= p.K; k += PREP_THREADS) s_seg[k] = p.seg[k];
+    if (threadIdx.x < PREP_THREADS / 32) s_clumps[threadIdx.x] = 0;
     __syncthreads();
-    const int64_t t0 = (blockIdx.x * (int64_t)(PREP_THREADS / 32) + (threadIdx.x >> 5)) * (32 * EACH) + (threadIdx.x & 31);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t t0 = (blockIdx.x * (int64_t)(PREP_THREADS / 32) + warp) * (32 * EACH) + lane;
     int k = 0, hi = p.K;   // last tap that begins at t0 or before
     while (hi - k > 1) {
         const int mid = (k + hi) >> 1;
         if (s_seg[mid] <= t0) k = mid; else hi = mid;
     }
+    auto enter = [&](int32_t row, int tap, int32_t entry, int steps, bool beyond) {
+        const int64_t block = row >> 7;
+        p.table[(block * p.K + tap) * ROWS + (row & (ROWS - 1))] = entry;
+        int2 *most = p.most + block * p.nq + tap / TPS;
+        if (steps > 1 && *(volatile int32_t *)&most->x < steps) atomicMax(&most->x, steps);
+        if (beyond) most->y = 1;
+    };
     int32_t row[EACH], prev[EACH], point[EACH];
 #pragma unroll
     for (int u = 0; u < EACH; ++u) {
@@ -153,16 +231,17 @@ __global__ void __launch_bounds__(PREP_THREADS) thin_table_kernel(PrepParams p) 
         while (k + 1 < p.K && s_seg[k + 1] <= t) ++k;
         if (t >= p.T || t < s_seg[k] || t >= s_seg[k + 1] || (t > s_seg[k] && prev[u] == row[u])) continue;
         int many = 1;
-        while (many < MOST && t + many < s_seg[k + 1] && __ldg(p.scatter + t + many) == row[u]) ++many;
-        const int64_t block = row[u] >> 7;
-        p.table[(block * p.K + k) * ROWS + (row[u] & (ROWS - 1))] = many == 1 ? point[u] : (int32_t)(1u << 31 | (uint32_t)(many - 2) << FIRST_BITS | (uint32_t)t);
-        if (many > 1) {
-            if (many == MOST)
-                while (t + many < s_seg[k + 1] && __ldg(p.scatter + t + many) == row[u]) ++many;
-            int32_t *most = p.most + block * p.nq + k / TPS;
-            if (*(volatile int32_t *)most < many) atomicMax(most, many);
-        }
+        while (many <= LISTED && t + many < s_seg[k + 1] && __ldg(p.scatter + t + many) == row[u]) ++many;
+        if (many > LISTED) s_clump[warp][atomicAdd(&s_clumps[warp], 1)] = make_int4((int32_t)t, k, row[u], 0);
+        else enter(row[u], k, many == 1 ? point[u] : (int32_t)(1u << 31 | (uint32_t)(many - 2) << FIRST_BITS | (uint32_t)t), many, false);
     }
+    __syncwarp();
+    for (int x = 0, n = s_clumps[warp]; x < n; ++x) {
+        const int4 c = s_clump[warp][x];
+        const int2 entry = sum_up(p, c.x, s_seg[c.y + 1], c.z);
+        if (lane == 0) enter(c.z, c.y, entry.x, entry.y, true);
+    }
+    let_next_be_set_up();   // only now: see mvmr_thin_kernel
 }
 
 // A row of a part: sums (+ bias), rounded.
@@ -236,11 +315,11 @@ struct At {
     }
 };
 
-// Row `j` of `base` (rows of 16 bytes), or, below zero, zeros: by a store, four clocks for 32 lanes, where a copy
+// Row `j` of `base` (rows of 16 bytes), or, for NONE, zeros: by a store, four clocks for 32 lanes, where a copy
 // takes a clock a lane with or without a source.
 __device__ __forceinline__ void copy_or_zeros(uint32_t dst, const uint16_t *base, int32_t j) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t.reg .b64 s;\n\tsetp.ge.s32 p, %2, 0;\n\tmad.wide.u32 s, %2, %3, %1;\n\t"
+        "{\n\t.reg .pred p;\n\t.reg .b64 s;\n\tsetp.ne.s32 p, %2, -1;\n\tmad.wide.u32 s, %2, %3, %1;\n\t"
         "@p cp.async.cg.shared.global [%0], [s], 16;\n\t@!p st.shared.v4.b32 [%0], {%4, %4, %4, %4};\n\t}"
         ::"r"(dst), "l"(base), "r"(j), "r"(CW * 2), "r"(0u) : "memory");
 }
@@ -252,6 +331,62 @@ __device__ __forceinline__ int32_t load_if(bool there, const int32_t *a, int32_t
     return v;
 }
 
+// The copies of a slot where some row has the sum of a clump, or more than LISTED triplets, of one of the eight taps: in a function
+// of its own, so that the registers and the schedule of the ordinary slots stay as they are.  What the ring, the verdict and the last
+// weights are afterwards.
+__device__ __noinline__ int4 clump_slot(const ThinParams &p, uint64_t *s_full, uint64_t *s_empty, volatile int *abort_flag, const At now, const int row, const int x0,
+                                        const int part, const uint32_t slot0, const int4 e4, const int steps, Ring ring, uint32_t last_load) {
+    constexpr int CELLS = TPS / 2;
+    const int32_t e[CELLS] = {e4.x, e4.y, e4.z, e4.w};
+    const int64_t block = (int64_t)blockIdx.x + (int64_t)now.n * gridDim.x;
+    int32_t j[CELLS], left[CELLS], t[CELLS];
+    uint32_t sums = 0;   // of this lane's cells; t of a sum is its first row
+    // (what a load may replace is known before: nothing waits for one here)
+#pragma unroll
+    for (int x = 0; x < CELLS; ++x) {
+        const bool several = e[x] < NONE;
+        t[x] = (e[x] & (int32_t)MAX_T) + 1;
+        left[x] = several ? (int)((uint32_t)e[x] >> FIRST_BITS & 15u) + 1 : 0;
+        const bool sum = left[x] == SUMMED + 1;
+        if (sum) sums |= 1u << x, t[x] = (int32_t)(p.first_sum + (uint32_t)(t[x] - 1) * PARTS), left[x] = 0;
+        if (left[x] == MORE + 1) {
+            const int64_t end = p.seg[now.q * TPS + x0 + x + 1], i = block * ROWS + row;
+            left[x] = LISTED;
+            while ((int64_t)t[x] + left[x] < end && p.scatter[t[x] + left[x]] == i) ++left[x];
+        }
+        j[x] = load_if(several && !sum, p.gather - 1, t[x], sum ? t[x] : e[x]);
+    }
+    bool ok = true;
+    for (int m = 0; m < steps; ++m) {
+        int32_t j_next[CELLS];
+#pragma unroll
+        for (int x = 0; x < CELLS; ++x) j_next[x] = load_if(left[x] > m, p.gather, t[x] + m, (sums >> x & 1u) && m + 1 < PARTS ? t[x] + m + 1 : NONE);
+        const uint32_t empty = smem_u32(&s_empty[ring.slot]), parity = (ring.turn ^ 1u) & 1u;
+        ok = __all_sync(0xffffffffu, mbar_try_wait(empty, parity)) ||
+             __all_sync(0xffffffffu, mbar_wait_abortable(empty, parity, STATUS_BIT, p.status, abort_flag));
+        if (!ok) break;
+        const uint32_t tile = slot0 + ring.slot * p.slot_bytes, full = smem_u32(&s_full[ring.slot]);
+        if (threadIdx.x == 0) {
+            mbar_arrive_expect_tx(full, (uint32_t)p.N * 128u);
+            bulk_load(tile + A_BYTES, p.image + ((int64_t)(part * p.nq + now.q) * p.N) * 64, (uint32_t)p.N * 128u, full);
+            last_load = ring.slot | (ring.turn & 1u) << 8 | 1u << 16;
+        }
+#pragma unroll
+        for (int x = 0; x < CELLS; ++x) {
+            copy_or_zeros(tile + (uint32_t)row * 128 + (uint32_t)(((x0 + x) ^ (row & 7)) << 4), p.feat, j[x]);
+            j[x] = j_next[x];
+        }
+        cp_async_mbar_arrive(full);
+        __syncwarp();
+        if ((threadIdx.x & 31) == 0) mbar_arrive(full);
+        ring.next(SLOTS);
+    }
+    return make_int4((int)ring.slot, (int)ring.turn, ok, (int)last_load);
+}
+
+// The grid is one wave, three CTAs on every multiprocessor, of which some have a block more to do than others; where the CTAs lie
+// decides how many of those share a multiprocessor.  Set up while the blocks of the table kernel still held theirs, they lay
+// differently from call to call: 200 000 points, 125 taps 267 to 287 us; the table kernel allows it at its end now: 243.
 __global__ void __launch_bounds__(THREADS, CTAS) mvmr_thin_kernel(const __grid_constant__ ThinParams p) {
     constexpr int CELLS = TPS / 2;   // taps of a lane
     extern __shared__ uint8_t smem_raw[];
@@ -292,7 +427,7 @@ __global__ void __launch_bounds__(THREADS, CTAS) mvmr_thin_kernel(const __grid_c
     }
     const int blocks = (p.nblocks - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // of this CTA
     auto block_of = [&](int n) { return (int64_t)blockIdx.x + (int64_t)n * gridDim.x; };
-    auto most_of = [&](const At &at) { return at.n < blocks ? __ldg(p.most + block_of(at.n) * p.nq + at.q) : 0; };
+    auto most_of = [&](const At &at) { return at.n < blocks ? __ldg(p.most + block_of(at.n) * p.nq + at.q) : make_int2(0, 0); };
     Ring ring;
 
     if (warp < WARPS) {
@@ -313,47 +448,48 @@ __global__ void __launch_bounds__(THREADS, CTAS) mvmr_thin_kernel(const __grid_c
         next.next(p.nq);
         int32_t e[CELLS], e_next[CELLS];
         cells_of(now, e);
-        int steps = most_of(now);
+        int2 most = most_of(now);
         bool ok = true;
         for (; now.n < blocks && ok; now = next, next.next(p.nq)) {
             cells_of(next, e_next);
-            const int steps_next = most_of(next);
-            // this step's feature rows; of several triplets the second, and how many more
-            int32_t j[CELLS], left[CELLS], t[CELLS];
-#pragma unroll
-            for (int x = 0; x < CELLS; ++x) {
-                const bool several = e[x] < NONE;
-                t[x] = (e[x] & (int32_t)MAX_T) + 1;
-                left[x] = several ? (int)((uint32_t)e[x] >> FIRST_BITS & 15u) + 1 : 0;
-                j[x] = load_if(several, p.gather - 1, t[x], e[x]);
-                if (left[x] == MOST - 1) {   // that many or more
-                    const int64_t end = p.seg[now.q * TPS + x0 + x + 1], i = block_of(now.n) * ROWS + row;
-                    while ((int64_t)t[x] + left[x] < end && p.scatter[t[x] + left[x]] == i) ++left[x];
-                }
-            }
-            for (int m = 0; m < steps; ++m) {
-                int32_t j_next[CELLS];
-#pragma unroll
-                for (int x = 0; x < CELLS; ++x) j_next[x] = load_if(left[x] > m, p.gather, t[x] + m, NONE);
-                ok = wait(s_empty[ring.slot], ring.turn ^ 1u);
-                if (!ok) break;
-                const uint32_t tile = slot0 + ring.slot * p.slot_bytes, full = smem_u32(&s_full[ring.slot]);
-                if (tid == 0) {
-                    mbar_arrive_expect_tx(full, (uint32_t)p.N * 128u);
-                    bulk_load(tile + A_BYTES, p.image + ((int64_t)(part * p.nq + now.q) * p.N) * 64, (uint32_t)p.N * 128u, full);
-                    last_load = ring.slot | (ring.turn & 1u) << 8 | 1u << 16;
-                }
+            const int2 most_next = most_of(next);
+            if (most.y) {
+                const int4 r = clump_slot(p, s_full, s_empty, abort_flag, now, row, x0, part, slot0, make_int4(e[0], e[1], e[2], e[3]), most.x, ring, last_load);
+                ring.slot = (uint32_t)r.x, ring.turn = (uint32_t)r.y, ok = r.z != 0, last_load = (uint32_t)r.w;
+            } else {
+                // this step's feature rows; of several triplets the second, and how many more
+                int32_t j[CELLS], left[CELLS], t[CELLS];
 #pragma unroll
                 for (int x = 0; x < CELLS; ++x) {
-                    copy_or_zeros(tile + at[x], p.feat, j[x]);
-                    j[x] = j_next[x];
+                    const bool several = e[x] < NONE;
+                    t[x] = (e[x] & (int32_t)MAX_T) + 1;
+                    left[x] = several ? (int)((uint32_t)e[x] >> FIRST_BITS & 15u) + 1 : 0;
+                    j[x] = load_if(several, p.gather - 1, t[x], e[x]);
                 }
-                cp_async_mbar_arrive(full);   // fires once this lane's copies have landed
-                __syncwarp();
-                if (lane == 0) mbar_arrive(full);   // the warp's zeros
-                ring.next(SLOTS);
+                for (int m = 0; m < most.x; ++m) {
+                    int32_t j_next[CELLS];
+#pragma unroll
+                    for (int x = 0; x < CELLS; ++x) j_next[x] = load_if(left[x] > m, p.gather, t[x] + m, NONE);
+                    ok = wait(s_empty[ring.slot], ring.turn ^ 1u);
+                    if (!ok) break;
+                    const uint32_t tile = slot0 + ring.slot * p.slot_bytes, full = smem_u32(&s_full[ring.slot]);
+                    if (tid == 0) {
+                        mbar_arrive_expect_tx(full, (uint32_t)p.N * 128u);
+                        bulk_load(tile + A_BYTES, p.image + ((int64_t)(part * p.nq + now.q) * p.N) * 64, (uint32_t)p.N * 128u, full);
+                        last_load = ring.slot | (ring.turn & 1u) << 8 | 1u << 16;
+                    }
+#pragma unroll
+                    for (int x = 0; x < CELLS; ++x) {
+                        copy_or_zeros(tile + at[x], p.feat, j[x]);
+                        j[x] = j_next[x];
+                    }
+                    cp_async_mbar_arrive(full);   // fires once this lane's copies have landed
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(full);   // the warp's zeros
+                    ring.next(SLOTS);
+                }
             }
-            steps = steps_next;
+            most = most_next;
 #pragma unroll
             for (int x = 0; x < CELLS; ++x) e[x] = e_next[x];
             if (ok && warp < 4 && now.q + 1 == p.nq) {
@@ -384,9 +520,9 @@ __global__ void __launch_bounds__(THREADS, CTAS) mvmr_thin_kernel(const __grid_c
         bool ok = true;
         At now, next;
         next.next(p.nq);
-        int steps = most_of(now);
+        int steps = most_of(now).x;
         for (; now.n < blocks && ok; now = next, next.next(p.nq)) {
-            const int steps_next = most_of(next);
+            const int steps_next = most_of(next).x;
             if (now.q == 0 && !wait_one(s_acc_empty[now.n & 1], ((uint32_t)now.n >> 1) ^ 1u)) break;
             const uint32_t d = tmem + (uint32_t)(now.n & 1) * p.col_stride;
             for (int m = 0; m < steps; ++m) {
@@ -411,8 +547,9 @@ __global__ void __launch_bounds__(THREADS, CTAS) mvmr_thin_kernel(const __grid_c
 }
 
 struct ThinWs {
-    uint32_t *odd;
-    int32_t *table, *most;
+    uint32_t *odd, *n_sums;
+    int32_t *table;
+    int2 *most;
     uint16_t *image, *feat;
 };
 
@@ -433,20 +570,20 @@ bool shape_of(int64_t n_out, int K, int C, int M, int transpose, Shape *s) {
 
 int prep_blocks() { return num_sms() * PREP_CTAS; }
 
-size_t carve_thin(void *base, int64_t n_feat, int K, const Shape &s, ThinWs *out) {
+size_t carve_thin(void *base, int64_t n_feat, int K, const Shape &s, int64_t sums, ThinWs *out) {
     Carver c(base);
     ThinWs w;
-    w.odd = c.take<uint32_t>(prep_blocks());
+    w.odd = c.take<uint32_t>(prep_blocks() + 1), w.n_sums = w.odd + prep_blocks();
     w.table = c.take<int32_t>((size_t)s.nblocks * K * ROWS);
-    w.most = c.take<int32_t>((size_t)s.nblocks * s.nq);
+    w.most = c.take<int2>((size_t)s.nblocks * s.nq);
     w.image = c.take<uint16_t>((size_t)s.parts * s.nq * s.N * 64);
-    w.feat = c.take<uint16_t>((size_t)n_feat * CW);
+    w.feat = c.take<uint16_t>((size_t)(n_feat + PARTS * sums) * CW);
     if (out) *out = w;
     return c.off;
 }
 
 int launch_thin(const PrepParams &prep, ThinParams p, const Shape &s, cudaStream_t stream) {
-    const int64_t work = std::max(std::max(prep.table_pieces / 8, prep.most_pieces), std::max(prep.image_pieces, prep.feat_pieces));
+    const int64_t work = std::max(std::max(prep.table_pieces / 8, prep.most_pieces), std::max(prep.image_pieces, prep.n_feat));
     p.n_odd = (int)std::min<int64_t>((work + PREP_THREADS - 1) / PREP_THREADS, prep_blocks());
     launch_after(thin_prepare_kernel, (unsigned)p.n_odd, PREP_THREADS, 0, stream, prep);
     PCX_LAUNCH_CHECK();
@@ -478,7 +615,7 @@ extern "C" {
 size_t pcx_mvmr_thin_workspace_bytes(int64_t n_feat, int64_t n_out, int K, int C, int M, int transpose) {
     Shape s;
     if (n_feat < 0 || n_feat > INT32_MAX || !shape_of(n_out, K, C, M, transpose, &s)) return 0;
-    return carve_thin(nullptr, n_feat, K, s, nullptr);
+    return carve_thin(nullptr, n_feat, K, s, n_out, nullptr);
 }
 
 int pcx_mvmr_thin(const void *d_weight, const void *d_feat, const int32_t *d_gather, const int32_t *d_scatter, const int64_t *d_seg_offs,
@@ -494,19 +631,21 @@ int pcx_mvmr_thin(const void *d_weight, const void *d_feat, const int32_t *d_gat
     if (!d_weight || !d_feat || !d_gather || !d_scatter || !d_seg_offs || !d_out || !d_ws) PCX_FAIL(PCX_E_ARG, "pcx_mvmr_thin: null pointer");
     if ((uintptr_t)d_ws % 256 || (uintptr_t)d_out % 16) PCX_FAIL(PCX_E_ALIGN, "pcx_mvmr_thin: workspace must be 256-byte, output 16-byte aligned");
     ThinWs w;
-    const size_t need = carve_thin(d_ws, n_feat, K, s, &w);
+    const size_t need = carve_thin(nullptr, n_feat, K, s, 0, nullptr);
     if (ws_bytes < need) PCX_FAIL(PCX_E_CAPACITY, "pcx_mvmr_thin: workspace %zu < %zu bytes", ws_bytes, need);
-    const bool as_they_are = s.inw == CW && (uintptr_t)d_feat % 16 == 0;
+    // as many sums as there can be, as there is room for, and as the rows' numbers reach
+    const int64_t max_sums = std::min(std::min(T / (LISTED + 1), (int64_t)((ws_bytes - need) / SUM_BYTES)), ((int64_t)UINT32_MAX - 1 - n_feat) / PARTS);
+    carve_thin(d_ws, n_feat, K, s, max_sums, &w);
     PrepParams prep = {};
-    prep.weight = (const uint16_t *)d_weight, prep.feat_in = (const uint16_t *)d_feat, prep.feat = as_they_are ? nullptr : w.feat;
+    prep.weight = (const uint16_t *)d_weight, prep.feat_in = (const uint16_t *)d_feat, prep.feat = w.feat;
+    prep.n_sums = w.n_sums, prep.max_sums = (uint32_t)max_sums;
     prep.scatter = d_scatter, prep.gather = d_gather, prep.seg = d_seg_offs, prep.table = w.table, prep.most = w.most, prep.image = w.image, prep.odd = w.odd;
     prep.T = T, prep.n_feat = n_feat, prep.image_pieces = (int64_t)s.parts * s.nq * s.N * 8;
-    prep.feat_pieces = as_they_are ? 0 : n_feat;
     prep.table_pieces = s.nblocks * K * (ROWS / 4), prep.most_pieces = s.nblocks * s.nq;
     prep.K = K, prep.inw = s.inw, prep.width = s.width, prep.nq = s.nq, prep.N = s.N;
     prep.transpose = transpose, prep.reverse = flags & PCX_MVMR_REVERSE_TAPS ? 1 : 0, prep.fmt = dtype == PCX_BF16 ? 1 : 0;
     ThinParams p = {};
-    p.feat = as_they_are ? (const uint16_t *)d_feat : w.feat;
+    p.feat = w.feat, p.first_sum = (uint32_t)n_feat;
     p.gather = d_gather, p.scatter = d_scatter, p.seg = d_seg_offs, p.table = w.table, p.most = w.most, p.image = w.image, p.odd = w.odd;
     p.bias = (const uint16_t *)d_bias, p.out = (uint16_t *)d_out;
     if (int rc = device_status_address(&p.status)) return rc;

@@ -32,7 +32,7 @@ def _exact(w, x, i, j, k, n_out):
     return out
 
 
-def _thin(weight, feat, i, j, seg, bias, n_out, flags=0):
+def _thin(weight, feat, i, j, seg, bias, n_out, flags=0, keep=False):
     from pointelligence_b200 import _cabi
 
     K, C, M = weight.shape
@@ -42,7 +42,7 @@ def _thin(weight, feat, i, j, seg, bias, n_out, flags=0):
     ws = _cabi.workspace(L.pcx_mvmr_thin_workspace_bytes(feat.shape[0], n_out, K, C, M, flags & 1), feat.device)
     _cabi.check(L.pcx_mvmr_thin(ptr(weight), ptr(feat), ptr(j), ptr(i), ptr(seg), ptr(bias), ptr(out), i.numel(), feat.shape[0],
                                 n_out, K, C, M, flags, _cabi.dtype_code(feat.dtype), ptr(ws), ws.numel(), _cabi.stream_ptr()))
-    return out
+    return (out, ws) if keep else out
 
 
 def _rel(a, b):
@@ -133,3 +133,74 @@ def test_the_layers_that_take_it():
         i.add_(0)      # written to since the search: nothing is known about the order
         _, names = kernels(lambda: conv(x, i, j, k, len(pts), contract=m.contract, seg_offs=m.seg_offs))
         assert "mvmr_thin_kernel" not in names
+
+
+def _clumped(n, members, K, C, ratio, seed, spread=1):
+    """``_rulebook`` with, for the first ``members`` of ``n`` points in random order, triplets of each with each of them
+    in ``spread`` taps from the middle on: rows of which every one has as many triplets in a tap."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    i, j, k, _ = _rulebook(n, n, K, ratio, seed)
+    clump = torch.randperm(n, device="cuda", generator=g)[:members]
+    a, b = (t.flatten() for t in torch.meshgrid(clump, clump, indexing="ij"))
+    i = torch.cat([i.long()] + [a] * spread)
+    j = torch.cat([j.long()] + [b] * spread)
+    k = torch.cat([k] + [torch.full_like(a, K // 2 + s) for s in range(spread)])
+    order = torch.argsort(k * n + i, stable=True)
+    i, j, k = i[order], j[order], k[order]
+    seg = torch.searchsorted(k.contiguous(), torch.arange(K + 1, device="cuda"))
+    return i.int().contiguous(), j.int().contiguous(), k, seg
+
+
+def _steps(ws, n_out, K):
+    """Steps of every (block, slot of eight taps), from the workspace of a call."""
+    up = lambda n: (n + 255) // 256 * 256
+    blocks = (n_out + 127) // 128
+    at = up(4 * 8 * torch.cuda.get_device_properties(0).multi_processor_count) + up(4 * blocks * K * 128)
+    return ws[at:at + 8 * blocks * ((K + 7) // 8)].view(torch.int32)[::2]
+
+
+@pytest.mark.parametrize("members,K,C,spread", [(8, 27, 3, 1), (9, 27, 6, 1), (10, 27, 6, 14), (33, 27, 8, 2), (64, 125, 6, 1), (65, 125, 3, 3),
+                                                (400, 27, 6, 1), (1000, 27, 8, 2)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("sign", [False, True])
+def test_rows_of_many_triplets_in_a_tap(members, K, C, spread, dtype, sign):
+    """Points within a centimetre of each other: a block takes eight steps at most for eight taps, as long as the sums of such
+    a (row, tap) stay within the type's range, and loses nothing (fp32 sums before the product, handed on in three parts)."""
+    n, M = 5000, 48
+    g = torch.Generator(device="cuda").manual_seed(members)
+    i, j, k, seg = _clumped(n, members, K, C, 6.0, members + K, spread)
+    w = (torch.randn(K, C, M, device="cuda", generator=g) / C ** 0.5).to(dtype)
+    x = torch.randn(n, C, device="cuda", generator=g).to(dtype)
+    if sign:
+        w, x = w.abs(), x.abs()
+    got, ws = _thin(w, x, i, j, seg, None, n, keep=True)
+    assert _rel(got, _exact(w, x, i, j, k, n)) <= BOUND[dtype]
+    assert 3 <= int(_steps(ws, n, K).max()) <= 8
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_sums_that_leave_the_range_or_are_no_numbers(dtype):
+    """Those of a (row, tap) are then taken triplet by triplet: infinities and NaN as the scatter kernel has them, and finite
+    rows where the sum of the features alone would be infinite."""
+    from pointelligence_b200 import _cabi
+
+    n, K, C, M, members = 1000, 27, 6, 32, 40
+    g = torch.Generator(device="cuda").manual_seed(5)
+    i, j, k, seg = _clumped(n, members, K, C, 4.0, 9)
+    top = torch.finfo(dtype).max
+    x = torch.randn(n, C, device="cuda", generator=g).to(dtype)
+    x[:, 1] = top / 4
+    w = (torch.randn(K, C, M, device="cuda", generator=g) / 64).to(dtype)
+    got = _thin(w, x, i, j, seg, None, n)
+    exact = _exact(w, x, i, j, k, n)
+    fits = exact.abs() < top / 2
+    assert bool(fits.any()) and bool(got[fits].isfinite().all()) and _rel(got[fits], exact[fits]) <= 4 * BOUND[dtype]
+    heavy = torch.bincount(i[k == K // 2].long(), minlength=n).argmax()
+    x = torch.randn(n, C, device="cuda", generator=g).to(dtype)
+    members_of = j[(k == K // 2) & (i == heavy)].long()
+    x[members_of[7], 2], x[members_of[30], 3] = float("inf"), float("nan")
+    got = _thin(w, x, i, j, seg, None, n)
+    ref = _cabi.mvmr(w.unsqueeze(1), x, j, i, seg, None, n, False, _cabi.ENGINE_CUDA_CORE)
+    assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got.isinf(), ref.isinf()) and bool(got.isnan().any())
+    ok = ref.isfinite()
+    assert _rel(got[ok], ref[ok].double()) <= 2 * BOUND[dtype]
