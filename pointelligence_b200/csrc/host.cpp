@@ -212,6 +212,28 @@ bool rows_ascend(const Tensor &scatter, const Tensor &gather, const Tensor &seg,
     return py::cast<bool>(py::reinterpret_borrow<py::object>(g_ascending_hook)(scatter, gather, seg, K));
 }
 
+// (undefined where its table, a number for every row and tap, is beyond 4 GB or finds no room: the scatter kernels need less)
+constexpr size_t THIN_MAX_SCRATCH = size_t(4) << 30;
+Tensor mvmr_thin(const Tensor &weight, const Tensor &feat, const Tensor &gather_, const Tensor &scatter_, const Tensor &seg_, int64_t n_out,
+                 int flags, const Tensor &bias) {
+    const int64_t K = weight.size(0), C = weight.size(2), M = weight.size(3), T = gather_.numel();
+    const int transpose = flags & 1;
+    // (a sum of triplets, 48 bytes, is made of nine or more)
+    const size_t bytes = pcx_mvmr_thin_workspace_bytes(feat.size(0), n_out, (int)K, (int)C, (int)M, transpose) + 48 * std::max<int64_t>(T / 9 - n_out, 0);
+    if (bytes > THIN_MAX_SCRATCH) return Tensor();
+    Tensor ws;
+    try {
+        ws = workspace(bytes, feat);
+    } catch (const c10::OutOfMemoryError &) {
+        return Tensor();
+    }
+    const Tensor gather = as_i32(gather_), scatter = as_i32(scatter_), seg = as_i64(seg_);
+    Tensor out = at::empty({n_out, transpose ? C : M}, feat.options());
+    check(pcx_mvmr_thin(ptr(weight), ptr(feat), ptr_as<int32_t>(gather), ptr_as<int32_t>(scatter), ptr_as<int64_t>(seg), ptr(bias), ptr(out), T,
+                        feat.size(0), n_out, (int)K, (int)C, (int)M, flags, dtype_code(feat.scalar_type()), ptr(ws), ws.numel(), stream()));
+    return out;
+}
+
 // out[scatter[t]] += feat[gather[t]] @ W[tap(t)] (+ bias).  flags: 1 = W transposed, 2 = taps of the weight
 // in reverse order.  Rows of the result are (G * out width) in feat's type.
 Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor &scatter_, const OptTensor &seg_,
@@ -232,13 +254,8 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
     if (engine == 0 && seg_ && thin_pays(feat.scalar_type(), T, feat.size(0), n_out, K, G, inw, outw) &&
         // (a captured pass is replayed on whatever the index tensors hold then: on the kernels that take any order)
         c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None && rows_ascend(scatter_, gather_, *seg_, K)) {
-        const Tensor gather = as_i32(gather_), scatter = as_i32(scatter_), seg = as_i64(*seg_);
-        Tensor out = at::empty({n_out, outw}, feat.options());
-        // (a sum of triplets, 48 bytes, is made of nine or more)
-        Tensor ws = workspace(pcx_mvmr_thin_workspace_bytes(feat.size(0), n_out, (int)K, (int)C, (int)M, transpose) + 48 * std::max<int64_t>(T / 9 - n_out, 0), feat);
-        check(pcx_mvmr_thin(ptr(weight), ptr(feat), ptr_as<int32_t>(gather), ptr_as<int32_t>(scatter), ptr_as<int64_t>(seg), ptr(bias), ptr(out),
-                            T, feat.size(0), n_out, (int)K, (int)C, (int)M, flags, code, ptr(ws), ws.numel(), stream()));
-        return out;
+        const Tensor y = mvmr_thin(weight, feat, gather_, scatter_, *seg_, n_out, flags, bias);
+        if (y.defined()) return y;
     }
     if ((engine & 0xff) == 0 && is_half(feat.scalar_type()) && seg_ && T > 0 && n_out > 0 && K <= 1024 && G <= 64 &&
         (C != padded(C) || M != padded(M))) {

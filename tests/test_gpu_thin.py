@@ -204,3 +204,38 @@ def test_sums_that_leave_the_range_or_are_no_numbers(dtype):
     assert torch.equal(got.isnan(), ref.isnan()) and torch.equal(got.isinf(), ref.isinf()) and bool(got.isnan().any())
     ok = ref.isfinite()
     assert _rel(got[ok], ref[ok].double()) <= 2 * BOUND[dtype]
+
+
+def test_too_little_memory_for_the_table():
+    """A call that the scatter kernels have room for is no error where the table of this one does not fit."""
+    from pointelligence_b200 import _cabi
+    from pointelligence_b200.layers.triplets import build_triplets_segmented
+
+    n, K = 200_000, 125
+    pts = torch.rand(n, 3, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1))
+    pts = pts * torch.tensor([1.0, 1.0, 0.02], device="cuda")
+    ids, sizes = torch.zeros(n, dtype=torch.int64, device="cuda"), torch.tensor([n], device="cuda")
+    i, j, k, seg, _ = build_triplets_segmented(pts, ids, sizes, 0.0115, 5, radius_scaler=2.1)
+    w = (torch.randn(K, 1, 4, 32, device="cuda") / 2).bfloat16()
+    x = torch.randn(n, 4, device="cuda").bfloat16()
+
+    def call():
+        _cabi.profile_enable(True)
+        y = _cabi.mvmr(w, x, j, i, seg, None, n, False)
+        names = [name for name, _ in _cabi.profile_records()]
+        _cabi.profile_enable(False)
+        return y, names
+
+    want, names = call()
+    assert names == ["mvmr_thin_kernel"], (names, i.numel() / n)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    limit = torch.cuda.memory_reserved() + (84 << 20)      # the table takes 100 MB, the scatter kernel's sums 26
+    torch.cuda.set_per_process_memory_fraction(limit / total)
+    try:
+        got, names = call()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert "mvmr_thin_kernel" not in names
+    assert _rel(got, want.double()) < 1e-2
