@@ -377,16 +377,19 @@ __global__ void expand_taps_kernel(const int64_t *__restrict__ seg, int K, int64
 // Ranges of cell keys, for points that are put in order by counting: two for a point, or sixteen, at most 2^23.
 constexpr int RANGE_BITS = 23, SCAN_THREADS = 1024, SCAN_EACH = 4, SCAN_BLOCK = SCAN_THREADS * SCAN_EACH;
 constexpr int SCAN_BLOCKS = (1 << RANGE_BITS) / SCAN_BLOCK;
-enum { EXT_FULLEST = 8, EXT_WIDE = 9, EXT_PAIRS = 10 /* 64 bits */, EXT_WORDS = 16 };
+enum { EXT_FULLEST = 8, EXT_WIDE = 9, EXT_PAIRS = 10 /* 64 bits */, EXT_FEW_FULLEST = 12, EXT_FEW_SHIFT = 13, EXT_FEW_PAIRS = 14 /* 64 bits */, EXT_WORDS = 16 };
 // Points are put in order by comparing those of a range in pairs, as long as that is little work: up to 2048 in a range and up to
 // 128 a point on average (a million points: some 25 us); sorted otherwise.  Two ranges for a point do for rooms; sweeps of a
-// spinning LiDAR, few points in wide extents, crowd in them and take sixteen.
+// spinning LiDAR, few points in wide extents, crowd in them and take sixteen (which tell what two would have held: FEW).
+__host__ __device__ __forceinline__ bool too_full(const int32_t *fullest, const int32_t *pairs, int64_t N, int margin) {
+    return *fullest > 2048 / margin || *reinterpret_cast<const int64_t *>(pairs) > 128 / margin * N;
+}
 __host__ __device__ __forceinline__ bool crowded(const int32_t *ext, int64_t N) {
-    return ext[EXT_WIDE] || ext[EXT_FULLEST] > 2048 || *reinterpret_cast<const int64_t *>(ext + EXT_PAIRS) > 128 * N;
+    return ext[EXT_WIDE] || too_full(ext + EXT_FULLEST, ext + EXT_PAIRS, N, 1);
 }
 
 struct GridWs {
-    int32_t *ext;  // min[4], max[4] of (x, y, z, sample); points of the fullest range; whether keys need more than 62 bits
+    int32_t *ext;  // min[4], max[4] of (x, y, z, sample); points of the fullest range; whether keys need more than 62 bits; pairs
     int32_t *ranges, *range_sums;   // first point of a range within its block of the scan; points of the blocks
     int64_t num_ranges, more_ranges;   // two for a point, sixteen: there is room for the latter
     int64_t *keys_a, *keys_b;
@@ -499,7 +502,7 @@ __device__ __forceinline__ int range_shift(const int32_t *__restrict__ ext, int6
 }
 
 __global__ void grid_count_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, int wide, int64_t N, float cell, int32_t *ext,
-                                  int64_t num_ranges, int64_t *keys, int32_t *arrival, int32_t *ranges) {
+                                  int64_t num_ranges, int64_t few, int64_t *keys, int32_t *arrival, int32_t *ranges) {
     start_after_previous();
     const int shift = range_shift(ext, num_ranges);
     const int64_t n = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -507,14 +510,16 @@ __global__ void grid_count_kernel(const float *__restrict__ pts, const int32_t *
         if (n == 0) ext[EXT_WIDE] = 1;
         return;
     }
+    if (n == 0 && few < num_ranges) ext[EXT_FEW_SHIFT] = range_shift(ext, few) - shift;
     if (n >= N) return;
     const int64_t key = grid_key(pts, sample, wide, n, cell, ext);
     keys[n] = key;
     arrival[n] = atomicAdd(&ranges[key >> shift], 1);
 }
 
-// Points of a range -> first point of the range within the block's; points of the block; the fullest range.
-__global__ void __launch_bounds__(SCAN_THREADS) grid_ranges_kernel(int32_t *ranges, int32_t *sums, int32_t *ext) {
+// Points of a range -> first point of the range within the block's; points of the block; the fullest range, and points by points of
+// the same range; asked for, the same of the fewer ranges, of which each holds 1 to 8 of these.
+__global__ void __launch_bounds__(SCAN_THREADS) grid_ranges_kernel(int32_t *ranges, int32_t *sums, int32_t *ext, bool asked) {
     start_after_previous();
     using Scan = cub::BlockScan<int32_t, SCAN_THREADS>;
     __shared__ typename Scan::TempStorage tmp;
@@ -522,14 +527,41 @@ __global__ void __launch_bounds__(SCAN_THREADS) grid_ranges_kernel(int32_t *rang
     const int4 v = *mine;
     int32_t at, all;
     Scan(tmp).ExclusiveSum(v.x + v.y + v.z + v.w, at, all);
-    *mine = make_int4(at, at + v.x, at + v.x + v.y, at + v.x + v.y + v.z);
-    const int fullest = __reduce_max_sync(0xffffffffu, max(max(v.x, v.y), max(v.z, v.w)));
-    if ((threadIdx.x & 31) == 0 && fullest > 1) atomicMax(&ext[EXT_FULLEST], fullest);
     if (threadIdx.x == 0) sums[blockIdx.x] = all;
-    int64_t pairs = (int64_t)v.x * v.x + (int64_t)v.y * v.y + (int64_t)v.z * v.z + (int64_t)v.w * v.w;
+    if (all == 0) return;   // zeros already
+    *mine = make_int4(at, at + v.x, at + v.x + v.y, at + v.x + v.y + v.z);
+    // (an atomic addition a block, none from an empty one: one a warp, all to the same address, and a million points took 16 us
+    // here instead of 8, four LiDAR sweeps 26 instead of 24)
+    __shared__ int32_t s_fullest[2][SCAN_THREADS / 32];
+    __shared__ uint32_t s_pairs[2][SCAN_THREADS / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // (ranges of more than 2048 are crowded whatever the pairs; up to that a warp's stay below 2^30)
+    auto add_up = [&](int which, const int4 &n) {
+        const int32_t fullest = __reduce_max_sync(0xffffffffu, max(max(n.x, n.y), max(n.z, n.w)));
+        const uint32_t x = min(n.x, 2048), y = min(n.y, 2048), z = min(n.z, 2048), w = min(n.w, 2048);
+        const uint32_t pairs = __reduce_add_sync(0xffffffffu, x * x + y * y + z * z + w * w);
+        if (lane == 0) s_fullest[which][warp] = fullest, s_pairs[which][warp] = pairs;
+    };
+    add_up(0, v);
+    if (asked) {
+        const int more = ext[EXT_FEW_SHIFT];   // log2 of ranges in one of the few
+        int4 n = v;
+        if (more >= 1) n = make_int4(v.x + v.y, v.z + v.w, 0, 0);
+        if (more >= 2) n = make_int4(n.x + n.y, 0, 0, 0);
+        if (more >= 3) n.x += __shfl_xor_sync(0xffffffffu, n.x, 1), n.x = threadIdx.x & 1 ? 0 : n.x;
+        add_up(1, n);
+    }
+    __syncthreads();
+    if (warp < (asked ? 2 : 1)) {
+        const int32_t fullest = __reduce_max_sync(0xffffffffu, s_fullest[warp][lane]);
+        unsigned long long pairs = s_pairs[warp][lane];
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
-    if ((threadIdx.x & 31) == 0 && pairs) atomicAdd(reinterpret_cast<unsigned long long *>(ext + EXT_PAIRS), (unsigned long long)pairs);
+        for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+        if (lane == 0 && pairs) {
+            atomicMax(&ext[warp ? EXT_FEW_FULLEST : EXT_FULLEST], fullest);
+            atomicAdd(reinterpret_cast<unsigned long long *>(ext + (warp ? EXT_FEW_PAIRS : EXT_PAIRS)), pairs);
+        }
+    }
 }
 
 // First point of every block of ranges, in shared memory (SCAN_BLOCKS + 1 entries); 256 threads.
@@ -707,9 +739,11 @@ uint64_t key_bits_hint(uint64_t seen, uint32_t cell, int bits) {
     return tag | smaller << 8 | known;
 }
 
-// What clouds binned at about this cell size lately took to be put in order: (cell size's bit pattern << 32 | 0x100 for sixteen ranges
-// a point | clouds left that are sorted at once).  A hint only: where it is wrong, the cloud is put in order again.
-constexpr uint64_t MORE_RANGES = 0x100;
+// What clouds binned at about this cell size lately took to be put in order: (cell size's bit pattern << 32 | clouds in a row that had
+// sixteen ranges a point and would have been far from crowded in two << 9 | 0x100 for sixteen | clouds left that are sorted at once).  A hint
+// only: where it is wrong, the cloud is put in order again.  Sixteen ranges cost rooms that do not need them 7 us of 62 (40 000
+// points, down-sampled) to 20 of 85 (200 000); a cloud that crowds in two is put in order twice.
+constexpr uint64_t MORE_RANGES = 0x100, ONE_UNNEEDED = 0x200, UNNEEDED = 4 * ONE_UNNEEDED;
 std::atomic<uint64_t> &order_hint(float cell) {
     static std::atomic<uint64_t> table[64];
     uint32_t u;
@@ -738,6 +772,7 @@ int count_cells(const float *d_points, const int32_t *d_sample, int wide, int64_
     memcpy(&cell_bits, &c32, sizeof(cell_bits));
     std::atomic<uint64_t> &hint = order_hint(c32);
     const uint64_t seen_hint = hint.load(), last = (seen_hint >> 32) == cell_bits ? seen_hint & 0xffffffffu : 0;
+    const int64_t few = w.num_ranges;
     if (last & MORE_RANGES) w.num_ranges = w.more_ranges;
     const int64_t fours = w.num_ranges / 4;
     launch_after(grid_clear_kernel, (unsigned)std::min<int64_t>((fours + 255) / 256, 8 * num_sms()), 256, 0, stream, reinterpret_cast<int4 *>(w.ranges),
@@ -749,9 +784,9 @@ int count_cells(const float *d_points, const int32_t *d_sample, int wide, int64_
     unsigned nb = (unsigned)((N + 255) / 256);
     const HandOver host = new_hand_over();
     if (host.words && !(last & 0xff)) {
-        launch_after(grid_count_kernel, nb, 256, 0, stream, d_points, d_sample, wide, N, c32, w.ext, w.num_ranges, w.keys_b, w.vals_b, w.ranges);
+        launch_after(grid_count_kernel, nb, 256, 0, stream, d_points, d_sample, wide, N, c32, w.ext, w.num_ranges, few, w.keys_b, w.vals_b, w.ranges);
         PCX_LAUNCH_CHECK();
-        launch_after(grid_ranges_kernel, (unsigned)(w.num_ranges / SCAN_BLOCK), SCAN_THREADS, 0, stream, w.ranges, w.range_sums, w.ext);
+        launch_after(grid_ranges_kernel, (unsigned)(w.num_ranges / SCAN_BLOCK), SCAN_THREADS, 0, stream, w.ranges, w.range_sums, w.ext, few < w.num_ranges);
         PCX_LAUNCH_CHECK();
         launch_after(grid_order_kernel, nb, 256, 0, stream, w.keys_b, w.vals_b, N, w.ranges, w.range_sums, w.ext, w.num_ranges, w.keys_a, w.vals_a);
         PCX_LAUNCH_CHECK();
@@ -764,6 +799,10 @@ int count_cells(const float *d_points, const int32_t *d_sample, int wide, int64_
         if (int rc = wait_for_hand_over(host, stream)) return rc;
         const int32_t *h = reinterpret_cast<const int32_t *>(host.words);
         if (!crowded(h, N)) {
+            if (last & MORE_RANGES) {
+                const uint64_t unneeded = too_full(h + EXT_FEW_FULLEST, h + EXT_FEW_PAIRS, N, 4) ? MORE_RANGES : last + ONE_UNNEEDED;
+                if (unneeded != last) hint.store((uint64_t)cell_bits << 32 | (unneeded >= MORE_RANGES + UNNEEDED ? 0 : unneeded));
+            }
             h_info[0] = host.words[EXT_WORDS / 2], h_info[1] = h[3], h_info[2] = h[7];
             return PCX_OK;
         }
