@@ -295,6 +295,19 @@ int pcx_vvor(const void *d_a, const int32_t *d_a_idx, const void *d_b,
              int64_t n_b, int64_t n_o, int G, int Ma, int Cb, int dtype,
              int engine, void *d_ws, size_t ws_bytes, void *stream);
 
+/* The same for a caller that knows how many triplets the fullest o has (negative:
+ * not known).  With at most pcx_vvor_store_limit of them (0: never) the tensor
+ * engine's blocks take whole o's and store what they have summed; where it is not
+ * known, twice the average is taken for it, or the rows of a and b (twice the fewer)
+ * where these are more.  Results differ by the order of the fp32 sums. */
+int64_t pcx_vvor_store_limit(int64_t n_o, int G, int Ma, int Cb);
+int pcx_vvor_known(const void *d_a, const int32_t *d_a_idx, const void *d_b,
+                   const int32_t *d_b_idx, const int64_t *d_seg_offs,
+                   const int32_t *d_o_idx, void *d_out, int64_t T, int64_t n_a,
+                   int64_t n_b, int64_t n_o, int G, int Ma, int Cb, int dtype,
+                   int engine, int64_t fullest, void *d_ws, size_t ws_bytes,
+                   void *stream);
+
 /* ------------------------------------------------------------------------
  * VVOR without a workspace.  No counterpart in the reference.
  *
@@ -522,10 +535,12 @@ int pcx_radius_fill(const float *d_points, const float *d_queries, int64_t P,
  *   it stood at this hand-over (not cleared).
  *   `distance_type` 0 (ball) or 1 (Chebyshev); with PCX_RADIUS_WIDE_POINT_IDS or
  *   PCX_RADIUS_WIDE_QUERY_IDS OR-ed in, those sample ids are int64, of which the
- *   low words count (little endian).
+ *   low words count (little endian).  With PCX_RADIUS_FULLEST_TAP h_total of
+ *   pcx_radius_taps_fill points at FOUR: [3] the pairs of the fullest tap.
  *   pcx_radius_taps_supported  1 when kernel_size is served by this path. */
 #define PCX_RADIUS_WIDE_POINT_IDS 0x100
 #define PCX_RADIUS_WIDE_QUERY_IDS 0x200
+#define PCX_RADIUS_FULLEST_TAP 0x400
 int pcx_radius_taps_supported(int kernel_size);
 size_t pcx_radius_taps_workspace_bytes(int64_t P, int64_t Q, int kernel_size);
 int pcx_radius_taps_count(const float *d_points, const float *d_queries,

@@ -74,6 +74,8 @@ SIGNATURES = {
     "pcx_debug_wait_runs_out": (c_int, [ctypes.c_ulonglong, c_void_p]),
     "pcx_vvor_workspace_bytes": (c_size_t, [c_int64, c_int, c_int, c_int, c_int]),
     "pcx_vvor": (c_int, [c_void_p] * 7 + [c_int64] * 4 + [c_int] * 5 + [c_void_p, c_size_t, c_void_p]),
+    "pcx_vvor_store_limit": (c_int64, [c_int64, c_int, c_int, c_int]),
+    "pcx_vvor_known": (c_int, [c_void_p] * 7 + [c_int64] * 4 + [c_int] * 5 + [c_int64, c_void_p, c_size_t, c_void_p]),
     "pcx_vvor_static_scratch_max_elements": (c_size_t, []),
     "pcx_vvor_static_scratch": (c_int, [c_void_p] * 6 + [c_int64] * 4 + [c_int] * 4 + [c_void_p]),
     "pcx_segment_reduce_workspace_bytes": (c_size_t, [c_int64, c_int]),
@@ -163,7 +165,7 @@ def host():
         except ImportError as exc:
             raise RuntimeError("pointelligence_b200/lib/_pcx_host.so is missing or does not load: build it with "
                                f"`python -m pointelligence_b200.build` ({exc})") from exc
-        _pcx_host.set_hooks(_plan_hook, is_symmetric, _rows_ascend, _differentiable_backward)
+        _pcx_host.set_hooks(_plan_hook, is_symmetric, _rows_ascend, fullest_tap, _differentiable_backward)
         from .sparse_engines._dispatch_override import current_engine
 
         _pcx_host.set_engine(current_engine())
@@ -570,21 +572,21 @@ def _stamp(*tensors):
         return None
 
 
-def mark_built(i, j, seg_offs, K, symmetric):
+def mark_built(i, j, seg_offs, K, symmetric, fullest=None):
     """Record that ``(i, j)`` cut into ``K`` taps by ``seg_offs`` come from the geometry path: i ascends inside every
     tap.  ``symmetric``: the rulebook is its own mirror image: with ``(i, j, k)`` it holds ``(j, i, K - 1 - k)``.
     True for a self-search (queries are the points): the distance is symmetric and the tap of the opposite offset is
     the mirrored tap.  The input gradient of such a layer is then a forward pass over the SAME rulebook with the taps
-    of the weight reversed, so it needs no plan of its own (``tig_grad_input``).  Remembered by tensor identity, like
-    the plans."""
+    of the weight reversed, so it needs no plan of its own (``tig_grad_input``).  ``fullest``: triplets of the fullest
+    tap, where they were counted.  Remembered by tensor identity, like the plans."""
     import weakref
 
-    for key in [key for key, (refs, _, _, _) in _BUILT.items() if any(r() is None for r in refs)]:
+    for key in [key for key, (refs, *_) in _BUILT.items() if any(r() is None for r in refs)]:
         _BUILT.pop(key, None)
     stamp = _stamp(i, j, seg_offs)
     if stamp is not None:
         _BUILT[(i.data_ptr(), j.data_ptr(), i.numel())] = (tuple(weakref.ref(t) for t in (i, j, seg_offs)), stamp,
-                                                           int(K), bool(symmetric))
+                                                           int(K), bool(symmetric), fullest)
 
 
 def _built(i, j):
@@ -601,6 +603,15 @@ def _rows_ascend(i, j, seg_offs, K):
     merged, rows fall at the seams."""
     hit = _built(i, j)
     return hit is not None and hit[0][2]() is seg_offs and hit[1][2:] == _stamp(seg_offs) and hit[2] == int(K)
+
+
+def fullest_tap(i, j, seg_offs, K):
+    """Triplets of the fullest tap of a rulebook, or of the mirrored one of an up-sampling layer; None where nobody counted."""
+    for a, b in ((i, j), (j, i)):
+        hit = _built(a, b)
+        if hit is not None and hit[0][2]() is seg_offs and hit[1][2:] == _stamp(seg_offs) and hit[2] == int(K):
+            return hit[4]
+    return None
 
 
 def is_symmetric(i, j, K=None):
@@ -997,7 +1008,7 @@ def radius_taps(points, queries, radius, ps, qs, distance_type, kernel_size, ker
     estimate turns out too small) and returned as views of the first ``total`` entries."""
     ratio_key = (kernel_size, distance_type, float(radius))
     ratio = _TAPS_RATIO.get(ratio_key)
-    i, j, k, seg, num_neighbors, n, lonely, status = host().radius_taps(
+    i, j, k, seg, num_neighbors, n, lonely, status, fullest = host().radius_taps(
         points, queries, float(radius), ps, qs, distance_type, kernel_size, float(kernel_grid_size), want_k,
         -1.0 if ratio is None else ratio)
     if status:                 # the hand-over of the fill pass brought the status word along
@@ -1005,7 +1016,7 @@ def radius_taps(points, queries, radius, ps, qs, distance_type, kernel_size, ker
     if len(_TAPS_RATIO) > 256:
         _TAPS_RATIO.clear()
     _TAPS_RATIO[ratio_key] = max(ratio or 0.0, n / queries.shape[0])
-    num_neighbors.pcx_queries_without_neighbor = lonely   # spares the caller a pass over the counts
+    num_neighbors.pcx_counted = lonely, fullest   # queries without neighbour, pairs of the fullest tap: spares the caller passes over the pairs
     return i, j, k, seg, num_neighbors
 
 

@@ -27,6 +27,7 @@ namespace {
 PyObject *g_plan_hook = nullptr;       // (scatter, gather, seg, K, n_out, out_width, in_width, forced, split, capturing) -> None | plan tuple
 PyObject *g_symmetric_hook = nullptr;  // (i, j, K) -> bool
 PyObject *g_ascending_hook = nullptr;  // (scatter, gather, seg, K) -> bool: rows are known to ascend inside every tap
+PyObject *g_fullest_hook = nullptr;    // (index, index, seg, K) -> triplets of the fullest tap, or None
 PyObject *g_double_backward = nullptr; // differentiable backward of the convolution (create_graph)
 
 [[noreturn]] void raise(PyObject *type, const std::string &msg) {
@@ -309,6 +310,15 @@ Tensor mvmr(const Tensor &weight, const Tensor &feat, const Tensor &gather, cons
 }
 
 // --------------------------------------------------------------------- VVOR ----
+// Triplets of the fullest tap where that decides the kernel and a search has counted them, else -1.
+int64_t fullest_tap(const Tensor &a_idx, const Tensor &b_idx, const Tensor &seg, int64_t n_o, int64_t G, int64_t Ma, int64_t Cb) {
+    const int64_t T = a_idx.numel(), limit = pcx_vvor_store_limit(n_o, (int)G, (int)Ma, (int)Cb);
+    if (T <= limit || n_o <= 0 || T / n_o > limit) return -1;   // (stored, or summed, whatever it is)
+    py::gil_scoped_acquire gil;
+    py::object n = py::reinterpret_borrow<py::object>(g_fullest_hook)(a_idx, b_idx, seg, n_o);
+    return n.is_none() ? -1 : py::cast<int64_t>(n);
+}
+
 Tensor vvor(Tensor a, const Tensor &a_idx_, Tensor b, const Tensor &b_idx_, const OptTensor &seg_, const OptTensor &o_idx_,
             int64_t n_o, int64_t engine) {
     require_cuda(a), require_cuda(b), require_cuda(a_idx_), require_cuda(b_idx_), require_cuda(seg_), require_cuda(o_idx_);
@@ -328,9 +338,10 @@ Tensor vvor(Tensor a, const Tensor &a_idx_, Tensor b, const Tensor &b_idx_, cons
                  seg = seg_ ? as_i64(*seg_) : Tensor();
     Tensor out = at::empty({n_o, G, Ma, Cb}, a.options());
     Tensor ws = workspace(pcx_vvor_workspace_bytes(n_o, (int)G, (int)Ma, (int)Cb, code), a);
-    check(pcx_vvor(ptr(a), ptr_as<int32_t>(a_idx), ptr(b), ptr_as<int32_t>(b_idx), ptr_as<int64_t>(seg), ptr_as<int32_t>(o_idx),
-                   ptr(out), a_idx.numel(), a.size(0), b.size(0), n_o, (int)G, (int)Ma, (int)Cb, code, (int)engine, ptr(ws),
-                   ws.numel(), stream()));
+    const int64_t fullest = engine != 1 && is_half(a.scalar_type()) && seg_ ? fullest_tap(a_idx_, b_idx_, *seg_, n_o, G, Ma, Cb) : -1;
+    check(pcx_vvor_known(ptr(a), ptr_as<int32_t>(a_idx), ptr(b), ptr_as<int32_t>(b_idx), ptr_as<int64_t>(seg), ptr_as<int32_t>(o_idx),
+                         ptr(out), a_idx.numel(), a.size(0), b.size(0), n_o, (int)G, (int)Ma, (int)Cb, code, (int)engine, fullest, ptr(ws),
+                         ws.numel(), stream()));
     return out;
 }
 
@@ -555,8 +566,8 @@ Tensor ids(const Tensor &t) { return t.scalar_type() == at::kLong ? t.contiguous
 
 // Tap-segmented search: enqueue, fill into buffers sized from `ratio` (pairs per query of earlier searches
 // of this kind; negative: count first) and one hand-over.  Returns
-// (i, j, k | undefined, seg, num_neighbors, total, queries without neighbour, device status).
-std::tuple<Tensor, Tensor, OptTensor, Tensor, Tensor, int64_t, int64_t, int64_t> radius_taps(
+// (i, j, k | undefined, seg, num_neighbors, total, queries without neighbour, device status, pairs of the fullest tap).
+std::tuple<Tensor, Tensor, OptTensor, Tensor, Tensor, int64_t, int64_t, int64_t, int64_t> radius_taps(
     const Tensor &points_, const Tensor &queries_, double radius, const OptTensor &ps_, const OptTensor &qs_, int64_t distance_type,
     int64_t kernel_size, double grid, bool want_k, double ratio) {
     require_cuda(points_), require_cuda(queries_), require_cuda(ps_), require_cuda(qs_);
@@ -574,7 +585,7 @@ std::tuple<Tensor, Tensor, OptTensor, Tensor, Tensor, int64_t, int64_t, int64_t>
     check(pcx_radius_taps_count(ptr_as<float>(points), ptr_as<float>(queries), ptr_as<int32_t>(ps), ptr_as<int32_t>(qs), P, Q, radius,
                                 (int)distance_type, (int)kernel_size, grid, ptr_as<int64_t>(num_neighbors), ptr_as<int64_t>(seg),
                                 ptr(ws), ws.numel(), stream()));
-    int64_t total[3] = {0, 0, 0}, capacity;
+    int64_t total[4] = {0, 0, 0, 0}, capacity;
     if (ratio < 0) {
         check(pcx_radius_taps_total(P, Q, (int)kernel_size, total, ptr(ws), ws.numel(), stream()));
         capacity = total[0];
@@ -586,7 +597,7 @@ std::tuple<Tensor, Tensor, OptTensor, Tensor, Tensor, int64_t, int64_t, int64_t>
         i = at::empty({capacity}, i32), j = at::empty({capacity}, i32);
         if (want_k) k = at::empty({capacity}, i32);
         const int rc = pcx_radius_taps_fill(ptr_as<float>(queries), ptr_as<int32_t>(ps), ptr_as<int32_t>(qs), P, Q, radius,
-                                            (int)distance_type, (int)kernel_size, grid, capacity, ptr_as<int32_t>(i),
+                                            (int)distance_type | PCX_RADIUS_FULLEST_TAP, (int)kernel_size, grid, capacity, ptr_as<int32_t>(i),
                                             ptr_as<int32_t>(j), ptr_as<int32_t>(k), total, ptr(ws), ws.numel(), stream());
         if (rc == PCX_E_CAPACITY && attempt == 0 && total[0] > capacity) {
             capacity = total[0];   // the estimate was too small: exact size, fill pass only
@@ -597,7 +608,7 @@ std::tuple<Tensor, Tensor, OptTensor, Tensor, Tensor, int64_t, int64_t, int64_t>
     }
     const int64_t n = total[0];
     return {i.narrow(0, 0, n), j.narrow(0, 0, n), want_k ? OptTensor(k.narrow(0, 0, n)) : std::nullopt, seg, num_neighbors, n, total[1],
-            total[2]};
+            total[2], total[3]};
 }
 
 // (indices, points, sample | undefined, mapping | undefined, points per sample | undefined) of the centre-nearest
@@ -697,10 +708,11 @@ void record_streams(const std::vector<Tensor> &tensors) {
         if (t.is_cuda()) t.record_stream(c10::cuda::getCurrentCUDAStream(t.device().index()).unwrap());
 }
 
-void set_hooks(py::object plan, py::object symmetric, py::object ascending, py::object double_backward) {
+void set_hooks(py::object plan, py::object symmetric, py::object ascending, py::object fullest, py::object double_backward) {
     g_plan_hook = plan.release().ptr();
     g_symmetric_hook = symmetric.release().ptr();
     g_ascending_hook = ascending.release().ptr();
+    g_fullest_hook = fullest.release().ptr();
     g_double_backward = double_backward.release().ptr();
 }
 

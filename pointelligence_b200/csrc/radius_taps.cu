@@ -47,7 +47,7 @@ constexpr int THREADS = QPB * 8;  // one lane per (query, candidate cell)
 constexpr int MAX_K3 = 128;       // taps this path handles (kernel_size 3 and 5)
 constexpr int FOURS = 64;         // fours of candidates that a warp lists at a time
 constexpr int SCAN_THREADS = 1024, SCAN_ITEMS = 4;
-constexpr int DISTANCE = ~(PCX_RADIUS_WIDE_POINT_IDS | PCX_RADIUS_WIDE_QUERY_IDS);
+constexpr int DISTANCE = ~(PCX_RADIUS_WIDE_POINT_IDS | PCX_RADIUS_WIDE_QUERY_IDS | PCX_RADIUS_FULLEST_TAP);
 constexpr int BIN_THREADS = 256;
 constexpr int CROWDED = 1024;     // points of a bucket that are put in order by counting the lower ones
 
@@ -66,7 +66,8 @@ struct TapsWs {
     unsigned long long *tap_total;  // k3
     int64_t *seg;           // k3 + 1
     int64_t *ctrl;          // [0] total pairs, [1] a tap's count does not fit 31 bits, [2] taps scanned,
-                            // [3] queries without a neighbour, [4] points given room, [5] crowded buckets
+                            // [3] queries without a neighbour, [4] points given room, [5] crowded buckets,
+                            // [6] pairs of the fullest tap
     int bits;
     int64_t buckets, nblocks;
 };
@@ -447,11 +448,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) taps_colscan_kernel(uint32_t *bl
         unsigned long long v[4], sum = 0;
 #pragma unroll
         for (int u = 0; u < 4; ++u) v[u] = t0 + u < k3 ? __ldcg(tap_total + t0 + u) : 0ULL, sum += v[u];
-        unsigned long long incl = sum;
+        unsigned long long incl = sum, fullest = max(max(v[0], v[1]), max(v[2], v[3]));
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const unsigned long long up = __shfl_up_sync(0xffffffffu, incl, o);
             if ((int)threadIdx.x >= o) incl += up;
+            fullest = max(fullest, __shfl_xor_sync(0xffffffffu, fullest, o));
         }
         unsigned long long run = incl - sum;
 #pragma unroll
@@ -459,7 +461,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) taps_colscan_kernel(uint32_t *bl
             if (t0 + u <= k3) seg[t0 + u] = (int64_t)run, seg_out[t0 + u] = (int64_t)run;
             run += v[u];
         }
-        if (threadIdx.x == 31) ctrl[0] = (int64_t)incl, seg[k3] = (int64_t)incl, seg_out[k3] = (int64_t)incl;
+        if (threadIdx.x == 31) ctrl[0] = (int64_t)incl, ctrl[6] = (int64_t)fullest, seg[k3] = (int64_t)incl, seg_out[k3] = (int64_t)incl;
     }
 }
 
@@ -494,6 +496,7 @@ __global__ void __launch_bounds__(THREADS, REC_MAX > 1024 ? 4 : 5) taps_fill_ker
     if (blockIdx.x == 0 && threadIdx.x == 0 && a.host.words) {   // all there is to hand over is known before this pass
         for (int n = 0; n < 4; ++n) a.host.put(n, a.ctrl[n]);
         a.host.put(4, *(const volatile unsigned int *)a.status);
+        a.host.put(5, a.ctrl[6]);
         a.host.done();
     }
     const bool fits = a.ctrl[0] <= a.capacity && !a.ctrl[1];
@@ -665,13 +668,16 @@ TapArgs make_args(const TapsWs &w, const float *queries, const int32_t *point_sa
 bool fused(const TapArgs &a) { return a.use_s_max && a.variant == 1; }
 
 // ctrl[0 .. 3] and the device status word, in one wait
+// Words 0 to 3 and 6 of ctrl and the device status word, as the fill pass stores them.
 int read_ctrl(const TapsWs &w, int64_t *h, cudaStream_t stream) {
     unsigned int *d_status = nullptr;
     if (int rc = device_status_address(&d_status)) return rc;
     h[4] = 0;
-    PCX_CUDA(cudaMemcpyAsync(h, w.ctrl, 4 * sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
+    PCX_CUDA(cudaMemcpyAsync(h + 6, w.ctrl, 7 * sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
     PCX_CUDA(cudaMemcpyAsync(h + 4, d_status, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
     PCX_CUDA(cudaStreamSynchronize(stream));
+    std::copy(h + 6, h + 10, h);
+    h[5] = h[12];
     return PCX_OK;
 }
 
@@ -774,6 +780,7 @@ int pcx_radius_taps_fill(const float *d_queries, const int32_t *d_point_sample, 
     }
     if (int rc = a.host.words ? wait_for_hand_over(a.host, stream) : read_ctrl(w, h, stream)) return rc;
     h_total[0] = h[0], h_total[1] = h[3], h_total[2] = h[4];
+    if (distance_type & PCX_RADIUS_FULLEST_TAP) h_total[3] = h[5];
     if (h[1] || h[0] > INT32_MAX) PCX_FAIL(PCX_E_UNSUPPORTED, "prepared kernel-segment output currently requires fewer than 2^31 edges; got %lld", (long long)h[0]);
     if (h[0] > capacity) PCX_FAIL(PCX_E_CAPACITY, "pcx_radius_taps_fill: %lld pairs do not fit the capacity of %lld; nothing was written", (long long)h[0], (long long)capacity);
     return PCX_OK;

@@ -183,7 +183,20 @@ size_t pcx_vvor_workspace_bytes(int64_t n_o, int G, int Ma, int Cb, int dtype) {
 int pcx_vvor(const void *d_a, const int32_t *d_a_idx, const void *d_b, const int32_t *d_b_idx,
              const int64_t *d_seg_offs, const int32_t *d_o_idx, void *d_out, int64_t T, int64_t n_a,
              int64_t n_b, int64_t n_o, int G, int Ma, int Cb, int dtype, int engine, void *d_ws,
-             size_t ws_bytes, void *stream_) {
+             size_t ws_bytes, void *stream) {
+    return pcx_vvor_known(d_a, d_a_idx, d_b, d_b_idx, d_seg_offs, d_o_idx, d_out, T, n_a, n_b, n_o, G, Ma, Cb, dtype, engine, -1, d_ws, ws_bytes, stream);
+}
+
+int64_t pcx_vvor_store_limit(int64_t n_o, int G, int Ma, int Cb) {
+    uint64_t checked = 0;
+    if (n_o <= 0 || G <= 0 || Ma <= 0 || Cb <= 0 || !product_within((uint64_t)1 << 46, &checked, n_o, G, Ma, Cb)) return 0;
+    return vvor_store_limit(n_o, G, Ma, Cb);
+}
+
+int pcx_vvor_known(const void *d_a, const int32_t *d_a_idx, const void *d_b, const int32_t *d_b_idx,
+                   const int64_t *d_seg_offs, const int32_t *d_o_idx, void *d_out, int64_t T, int64_t n_a,
+                   int64_t n_b, int64_t n_o, int G, int Ma, int Cb, int dtype, int engine, int64_t fullest, void *d_ws,
+                   size_t ws_bytes, void *stream_) {
     cudaStream_t stream = (cudaStream_t)stream_;
     if (T < 0 || n_a < 0 || n_b < 0 || n_o < 0 || G <= 0 || Ma <= 0 || Cb <= 0)
         PCX_FAIL(PCX_E_ARG, "pcx_vvor: negative or zero size");
@@ -207,7 +220,7 @@ int pcx_vvor(const void *d_a, const int32_t *d_a_idx, const void *d_b, const int
     a.a = d_a, a.a_idx = d_a_idx, a.b = d_b, a.b_idx = d_b_idx, a.seg_offs = d_seg_offs, a.o_idx = d_o_idx;
     a.acc = dtype == PCX_F32 ? (float *)d_out : w.acc;
     a.chunk_table = w.chunk_table;
-    a.T = T, a.n_a = n_a, a.n_b = n_b, a.n_o = n_o, a.G = G, a.Ma = Ma, a.Cb = Cb, a.dtype = dtype;
+    a.T = T, a.n_a = n_a, a.n_b = n_b, a.n_o = n_o, a.fullest = fullest, a.G = G, a.Ma = Ma, a.Cb = Cb, a.dtype = dtype;
     if (force_engine()) engine = force_engine();
     const bool tensor_ok = T > 0 && vvor_tensor_supported(a);
     if (engine != PCX_ENGINE_CUDA_CORE && tensor_ok && vvor_stores(a)) {

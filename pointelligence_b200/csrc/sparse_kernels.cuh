@@ -31,7 +31,7 @@ struct VvorArgs {
     float *acc;              // (n_o, G, Ma, Cb) fp32, zeroed by the caller
     void *out;               // tensor engine: the output itself, where every tap is completed by one block (acc unused); else null
     int32_t *chunk_table;    // (n_o+1) scratch
-    int64_t T, n_a, n_b, n_o;
+    int64_t T, n_a, n_b, n_o, fullest;   // triplets of the fullest o; negative: not known
     int G, Ma, Cb, dtype;
 };
 
@@ -119,6 +119,7 @@ inline bool splits_evenly(int width) { return width >= 16 && width % (16 * parts
 
 bool mvmr_tensor_supported(const MvmrArgs &a);
 bool vvor_tensor_supported(const VvorArgs &a);
+int64_t vvor_store_limit(int64_t n_o, int G, int Ma, int Cb);
 bool vvor_stores(const VvorArgs &a);   // whether the tensor engine should store rows itself
 int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream);
 int vvor_tensor(const VvorArgs &a, cudaStream_t stream);

@@ -352,14 +352,22 @@ void store_parts(const VvorArgs &a, int *a_parts, int *b_parts) {
 
 }  // namespace
 
-// Whether CTAs take whole taps.  The fullest tap decides how long that takes, 10 ns a triplet of 256 x 256 channels and 7 of
-// 64 x 64 or 128 x 128; a rulebook of a cloud on itself has a triplet of every point in its centre tap, so that it holds the
-// average or the points, whichever is more.  The fp32 sums cost a microsecond a megabyte.  27 taps, fullest tap 950 / 3056 / 5150,
+// Up to how many triplets of the fullest tap CTAs take whole taps.  The fullest tap decides how long that takes, 10 ns a triplet of
+// 256 x 256 channels and 7 of 64 x 64 or 128 x 128; the fp32 sums cost a microsecond a megabyte.  27 taps, fullest tap 950 / 3056 / 5150,
 // sums and stored, us: 512 x 512 (28 MB) 44 / 54 / 57 and 29 / 51 / 74, 256 x 256 (7 MB) 28 / 30 / 40 and 18 / 33 / 47,
 // 128 x 128 (2 MB) 18 / 20 / 22 and 16 / 31 / 43, 64 x 64 15 / 15 / 17 and 16 / 31 / 43; 125 taps, 5050: 512 x 512 (131 MB) 143 and 96.
+int64_t vvor_store_limit(int64_t n_o, int G, int Ma, int Cb) {
+    const int64_t sums = n_o * G * Ma * Cb * 4;
+    return sums >= (1 << 20) ? 300 + sums / 10000 : 0;
+}
+
+// Searches hand the pairs of their fullest tap to the host.  Of other rulebooks nothing but the sizes is known here.  A room on itself
+// has a triplet of every point, or 1.1, in its centre tap; strided ones 1.1 to 2.1 for a row of the fewer (2.7 with 125 taps), sweeps
+// 1.2 to 1.7; where every tap is dense the fullest has 1.1 to 1.9 times the average.  All in one tap, 512 x 512 channels: 18 000
+// triplets 200 us stored and 90 summed, 72 000 736 and 129.
 bool vvor_stores(const VvorArgs &a) {
-    const int64_t fullest = std::max(a.T / a.n_o, std::min(a.n_a, a.n_b)), sums = a.n_o * a.G * a.Ma * a.Cb * 4;
-    return sums >= (1 << 20) && fullest <= 300 + sums / 10000;
+    const int64_t rows = std::min(a.n_a, a.n_b), guess = std::min(a.T, std::max(2 * a.T / a.n_o, a.n_a == a.n_b ? rows : 2 * rows));
+    return (a.fullest >= 0 ? a.fullest : guess) <= vvor_store_limit(a.n_o, a.G, a.Ma, a.Cb);
 }
 
 int vvor_tensor(const VvorArgs &a, cudaStream_t stream) {

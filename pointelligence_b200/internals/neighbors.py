@@ -134,8 +134,8 @@ def radius_search_sorted_grid8_segments(points, queries, radius, kernel_size, ke
                                                query_sample_inds, code, kernel_size=kernel_size,
                                                kernel_grid_size=float(kernel_grid_size), want_k=return_k)
     cast = counts.to(dtype_num_neighbors)
-    if hasattr(counts, "pcx_queries_without_neighbor"):
-        cast.pcx_queries_without_neighbor = counts.pcx_queries_without_neighbor
+    if hasattr(counts, "pcx_counted"):
+        cast.pcx_counted = counts.pcx_counted
     out = (i, j, seg, cast)
     return out + (k,) if return_k else out
 

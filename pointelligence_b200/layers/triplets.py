@@ -129,12 +129,12 @@ def _segmented(points, sample_inds, sample_sizes, neighbor_radius, kernel_size, 
                 return hit
         i, j, seg_offs, num_neighbors, k = _searched(points, query_points, sample_inds, query_sample_inds, neighbor_radius, ks,
                                                      kernel_grid_size, tap_stripes)
-        lonely = getattr(num_neighbors, "pcx_queries_without_neighbor", None)   # counted by the search itself
+        lonely, fullest = getattr(num_neighbors, "pcx_counted", (None, None))   # counted by the search itself
         if lonely is None:
             lonely = int((num_neighbors == 0).sum().item()) if num_neighbors.numel() else 0
         if lonely:
             raise AssertionError(_NO_NEIGHBOR_MSG)
-        _cabi.mark_built(i, j, seg_offs, ks ** 3, symmetric=query_points is points)   # a self-search is its own mirror image
+        _cabi.mark_built(i, j, seg_offs, ks ** 3, symmetric=query_points is points, fullest=fullest)   # a self-search is its own mirror image
         out = (i, j, k, seg_offs, (num_neighbors if return_num_neighbors else None))
         cache_put(key, out, points)
         return out
