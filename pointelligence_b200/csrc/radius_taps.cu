@@ -50,10 +50,11 @@ constexpr int SCAN_THREADS = 1024, SCAN_ITEMS = 4;
 constexpr int DISTANCE = ~(PCX_RADIUS_WIDE_POINT_IDS | PCX_RADIUS_WIDE_QUERY_IDS | PCX_RADIUS_FULLEST_TAP);
 constexpr int BIN_THREADS = 256;
 constexpr int CROWDED = 1024;     // points of a bucket that are put in order by counting the lower ones
+constexpr int MERGED = 32;        // ... by merging, where a bucket holds up to the MERGED-th part of all
 
 struct TapsWs {
     uint32_t *keys;         // bucket of a point
-    int32_t *arrival;       // ... and how many of the bucket's points were counted before it
+    int32_t *arrival;       // ... and how many of the bucket's points were counted before it; points of crowded buckets in order
     int32_t *order;         // the points, bucket by bucket, as they arrived
     int32_t *crowded;       // buckets with more than CROWDED points
     float4 *sorted_pts;     // xyz + original index (bit pattern), bucket by bucket, ascending inside a bucket
@@ -165,10 +166,61 @@ __global__ void __launch_bounds__(BIN_THREADS) taps_order_kernel(const uint32_t 
     if (p < P) order[table[keys[p]].x + arrival[p]] = (int32_t)p;
 }
 
+// `n` different numbers in ascending order, by a block: tiles of BIN_THREADS, then pairs of sorted runs, every number by a search in
+// the other run of its pair.  From `from` to `to`, with `other` as scratch (n each).
+__device__ __forceinline__ void merge_sort(const int32_t *from, int32_t *to, int32_t *other, int n) {
+    static_assert(BIN_THREADS == 256, "tiles of four numbers for 64 loads");
+    __shared__ int4 s_tile[BIN_THREADS / 4];
+    int passes = 0;
+    while ((BIN_THREADS << passes) < n) ++passes;
+    int32_t *src = passes & 1 ? other : to, *dst = passes & 1 ? to : other;
+    for (int first = 0; first < n; first += BIN_THREADS) {
+        const int at = first + (int)threadIdx.x;
+        const int32_t mine = at < n ? from[at] : INT_MAX;
+        reinterpret_cast<int32_t *>(s_tile)[threadIdx.x] = mine;
+        __syncthreads();
+        int lower = 0;
+#pragma unroll 8
+        for (int q = 0; q < BIN_THREADS / 4; ++q) {
+            const int4 v = s_tile[q];
+            lower += (v.x < mine) + (v.y < mine) + (v.z < mine) + (v.w < mine);
+        }
+        if (at < n) src[first + lower] = mine;
+        __syncthreads();
+    }
+    for (int width = BIN_THREADS; width < n; width *= 2) {
+        for (int first = 0; first < n; first += 4 * BIN_THREADS) {
+            int32_t mine[4];
+            int other_run[4], len[4], lower[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int at = first + u * BIN_THREADS + (int)threadIdx.x;
+                mine[u] = at < n ? src[at] : INT_MAX;
+                other_run[u] = (at / width ^ 1) * width;
+                len[u] = at < n ? max(0, min(width, n - other_run[u])) : 0;
+                lower[u] = 0;
+            }
+            for (int step = width; step > 0; step >>= 1)   // four searches at a time
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    if (lower[u] + step <= len[u] && src[other_run[u] + lower[u] + step - 1] < mine[u]) lower[u] += step;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int at = first + u * BIN_THREADS + (int)threadIdx.x;
+                if (at < n) dst[at / (2 * width) * (2 * width) + at % width + lower[u]] = mine[u];
+            }
+        }
+        __syncthreads();
+        int32_t *t = src;
+        src = dst, dst = t;
+    }
+}
+
 __global__ void __launch_bounds__(BIN_THREADS) taps_place_kernel(const float *__restrict__ pts, const int32_t *__restrict__ sample, int wide,
                                                                  const uint32_t *__restrict__ keys, const int32_t *__restrict__ order, int64_t P,
                                                                  const int2 *__restrict__ table, const int32_t *__restrict__ crowded,
-                                                                 const int64_t *__restrict__ ctrl, float4 *sorted_pts, int32_t *sorted_sample) {
+                                                                 const int64_t *__restrict__ ctrl, int32_t *arrival, float4 *sorted_pts,
+                                                                 int32_t *sorted_sample) {
     start_after_previous();
     auto put = [&](int32_t p, int32_t at) {
         sorted_pts[at] = make_float4(pts[3 * (int64_t)p], pts[3 * (int64_t)p + 1], pts[3 * (int64_t)p + 2], __int_as_float(p));
@@ -185,14 +237,23 @@ __global__ void __launch_bounds__(BIN_THREADS) taps_place_kernel(const float *__
             put(p, run.x + lower);
         }
     }
-    // Crowded buckets, a block each: all points are gone through in order.  There are at most P / CROWDED of them; a
-    // million points in buckets of 1500 take 1 ms.
+    // Crowded buckets, a block each, at most P / CROWDED of them.  Their points are merged; where a bucket has so many that that takes a
+    // block longer, all points are gone through in order (at most MERGED such).  The bucket's part of `arrival`, of no use by
+    // now, takes the result, its records the scratch.  This kernel, four million points in cells of 1100: 0.29 ms, and 16.4 where every
+    // crowded bucket went through all points; a million in cells of 20 000: 0.72 and 1.06.
     const int64_t n = ctrl[5];
     for (int64_t x = blockIdx.x; x < n; x += gridDim.x) {
         using Scan = cub::BlockScan<int32_t, BIN_THREADS>;
         __shared__ typename Scan::TempStorage tmp;
         const uint32_t key = (uint32_t)crowded[x];
-        int32_t at = table[key].x;
+        const int2 run = table[key];
+        if ((int64_t)run.y * MERGED <= P) {
+            merge_sort(order + run.x, arrival + run.x, reinterpret_cast<int32_t *>(sorted_pts + run.x), run.y);
+            for (int q = threadIdx.x; q < run.y; q += BIN_THREADS) put(arrival[run.x + q], run.x + q);
+            __syncthreads();
+            continue;
+        }
+        int32_t at = run.x;
         for (int64_t first = 0; first < P; first += 4 * BIN_THREADS) {
             const int64_t p = first + 4 * (int64_t)threadIdx.x;
             int32_t mine[4], before, all;
@@ -725,7 +786,7 @@ int pcx_radius_taps_count(const float *d_points, const float *d_queries, const i
     launch_after(taps_order_kernel, pblocks, BIN_THREADS, 0, stream, w.keys, w.arrival, P, w.table, w.order);
     PCX_LAUNCH_CHECK();
     launch_after(taps_place_kernel, pblocks, BIN_THREADS, 0, stream, d_points, d_point_sample, wide, w.keys, w.order, P, w.table, w.crowded, w.ctrl,
-                 w.sorted_pts, w.sorted_sample);
+                 w.arrival, w.sorted_pts, w.sorted_sample);
     PCX_LAUNCH_CHECK();
     TapArgs a = make_args(w, d_queries, d_point_sample, d_query_sample, Q, radius, distance_type, kernel_size, kernel_grid_size);
     a.num_neighbors = d_num_neighbors;

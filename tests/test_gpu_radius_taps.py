@@ -294,3 +294,51 @@ def test_crowded_cells_keep_their_points_in_order(crowd):
         _assert_same(*_both(pts, qry, None, None, 0.1, 3, 0.08))
     smp = torch.arange(pts.shape[0], device=dev) // ((pts.shape[0] + 2) // 3)
     _assert_same(*_both(pts, qry, smp, smp[::17].contiguous(), 0.1, 3, 0.08))
+
+
+@pytest.mark.parametrize("crowd", [(1025,), (1024 + 256, 5000), (2048, 2049), (70000, 40000, 1100), (33000, 16385, 2500)])
+@pytest.mark.parametrize("filler", [0, 90000, 1200000])
+@pytest.mark.parametrize("in_order", [False, True])
+def test_crowded_cells_of_any_size_keep_their_points_in_order(crowd, filler, in_order):
+    """More than 1024 points of a bucket are merged from tiles of 256, or, where that is more work, found by going through
+    all points."""
+    from pointelligence_b200 import _cabi
+
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(sum(crowd) + filler)
+    pts = torch.cat([torch.rand(n, 3, device=dev, generator=g) * 0.19 + 0.005 + 0.6 * c for c, n in enumerate(crowd)])
+    pts = torch.cat([pts, torch.rand(filler, 3, device=dev, generator=g) * 40.0 - 41.0])
+    if not in_order:
+        pts = pts[torch.randperm(pts.shape[0], device=dev, generator=g)].contiguous()
+    qry = pts[:: pts.shape[0] // 40].contiguous()
+    for smp in (None, torch.arange(pts.shape[0], device=dev) // ((pts.shape[0] + 2) // 3)):
+        _cabi._TAPS_RATIO.clear()
+        ref, got = _both(pts, qry, smp, None if smp is None else smp[:: pts.shape[0] // 40].contiguous(), 0.1, 3, 0.08)
+        _assert_same(ref, got)
+
+
+def test_many_crowded_cells_and_few_queries():
+    """Four million points, 1100 in every cell: putting them in order takes no longer than a few sorts of as many keys."""
+    from pointelligence_b200 import _cabi
+
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(0)
+    n = 4_000_000
+    side = (n / 1100) ** (1 / 3) * 0.2
+    pts = torch.rand(n, 3, device=dev, generator=g) * side
+    qry = pts[:32] + 1000.0      # near none of them: what is left is the order
+    keys = torch.randint(0, 1 << 40, (n,), device=dev, generator=g)
+
+    def best(call):
+        times = []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            call()
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        return min(times)
+
+    search = best(lambda: _cabi.radius_search(pts, qry, 0.1, None, None, 0, kernel_size=3, kernel_grid_size=0.08))
+    assert search < 5 * best(lambda: torch.sort(keys)), search
