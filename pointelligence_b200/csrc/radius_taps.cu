@@ -555,9 +555,10 @@ __global__ void __launch_bounds__(THREADS, REC_MAX > 1024 ? 4 : 5) taps_fill_ker
     __shared__ uint32_t s_base[MAX_K3];                     // next write position of each tap for this block
     __shared__ uint32_t s_start[MAX_K3], s_total[MAX_K3];   // first place of each tap among the sorted, its pairs in this round
     if (blockIdx.x == 0 && threadIdx.x == 0 && a.host.words) {   // all there is to hand over is known before this pass
-        for (int n = 0; n < 4; ++n) a.host.put(n, a.ctrl[n]);
-        a.host.put(4, *(const volatile unsigned int *)a.status);
-        a.host.put(5, a.ctrl[6]);
+        const int64_t words[4] = {a.ctrl[0], a.ctrl[1], a.ctrl[2], a.ctrl[3]}, fullest = a.ctrl[6];   // (loads before stores: one latency)
+        const unsigned int status = *(const volatile unsigned int *)a.status;
+        for (int n = 0; n < 4; ++n) a.host.put(n, words[n]);
+        a.host.put(4, status), a.host.put(5, fullest);
         a.host.done();
     }
     const bool fits = a.ctrl[0] <= a.capacity && !a.ctrl[1];
