@@ -72,6 +72,11 @@ __device__ __forceinline__ void start_after_previous() {
     wait_for_previous();
     let_next_be_set_up();
 }
+// Allows a kernel all the shared memory that a block of the device can have, once per device (a bit each in `done`).  Asked for as
+// much as a launch needs, a thread could take back what another had just asked for and was about to launch with.
+// `prefer`: multiprocessors are to be set up for as much shared memory as they have, too.
+int allow_shared_memory(const void *kernel, std::atomic<uint64_t> *done, bool prefer = false);
+
 template <typename... Params, typename... Args>
 void launch_after(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args &&...args) {
     cudaLaunchAttribute early = {};

@@ -1426,14 +1426,8 @@ int pcx::mvmr_planned(const void *d_weight, const void *d_feat, void *d_plan, si
     const size_t smem = 1024 + (size_t)p.nslots * p.slot_bytes + AHEAD * pack * ENTRY_BYTES;
     auto kernel = split_sums ? (pack == 4 ? mvmr_os_kernel<4, true> : pack == 2 ? mvmr_os_kernel<2, true> : mvmr_os_kernel<1, true>)
                              : (pack == 4 ? mvmr_os_kernel<4, false> : pack == 2 ? mvmr_os_kernel<2, false> : mvmr_os_kernel<1, false>);
-    static int granted[6][64] = {};
-    int dev = 0;
-    PCX_CUDA(cudaGetDevice(&dev));
-    int &most = granted[(pack >> 1) + (split_sums ? 3 : 0)][dev & 63];
-    if ((int)smem > most) {
-        PCX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        most = (int)smem;
-    }
+    static std::atomic<uint64_t> allowed[6];
+    if (int rc = allow_shared_memory((const void *)kernel, &allowed[(pack >> 1) + (split_sums ? 3 : 0)])) return rc;
     const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(pv.ngroups * p.nsplit * nparts, num_sms()));
     if (multi_buckets > 0 || odd) {   // (with no sums it looks at the weights alone)
         prof_begin("bucket_sum_kernel", stream);

@@ -590,13 +590,8 @@ int launch_thin(const PrepParams &prep, ThinParams p, const Shape &s, cudaStream
     launch_after(thin_table_kernel, (unsigned)((prep.T + 4 * PREP_THREADS - 1) / (4 * PREP_THREADS)), PREP_THREADS, 0, stream, prep);
     PCX_LAUNCH_CHECK();
     const size_t smem = std::max((size_t)1024 + SLOTS * p.slot_bytes, (size_t)ROWS * (p.N + 1) * 4);
-    static int granted[64] = {};   // per device
-    int dev = 0;
-    PCX_CUDA(cudaGetDevice(&dev));
-    if ((int)smem > granted[dev & 63]) {
-        PCX_CUDA(cudaFuncSetAttribute(mvmr_thin_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        granted[dev & 63] = (int)smem;
-    }
+    static std::atomic<uint64_t> allowed;
+    if (int rc = allow_shared_memory((const void *)mvmr_thin_kernel, &allowed)) return rc;
     const dim3 grid((unsigned)std::min<int64_t>(s.nblocks, std::max(1, CTAS * num_sms() / s.parts)), (unsigned)s.parts);
     prof_begin("mvmr_thin_kernel", stream);
     launch_after(mvmr_thin_kernel, grid, THREADS, smem, stream, p);

@@ -420,12 +420,14 @@ int ctas_per_sm(size_t smem, uint32_t ncols, int regs_per_thread, int threads = 
 // Registers per thread of a kernel (asked once per kernel; the persistent grids
 // must not exceed what is resident at once, or the surplus CTAs run as a second wave).
 template <typename Kernel>
-int kernel_registers(Kernel kernel, int *cached) {
-    if (*cached == 0) {
+int kernel_registers(Kernel kernel, std::atomic<int> *cached) {
+    int n = cached->load(std::memory_order_relaxed);
+    if (n == 0) {
         cudaFuncAttributes attr;
-        *cached = cudaFuncGetAttributes(&attr, kernel) == cudaSuccess ? attr.numRegs : 128;
+        n = cudaFuncGetAttributes(&attr, kernel) == cudaSuccess ? attr.numRegs : 128;
+        cached->store(n, std::memory_order_relaxed);
     }
-    return *cached;
+    return n;
 }
 
 // Dynamic shared memory padded so that at most 512 / ncols CTAs share an SM
@@ -434,17 +436,6 @@ size_t pad_for_tmem(size_t smem, uint32_t ncols) {
     size_t max_ctas = 512 / ncols;
     size_t floor_bytes = (size_t)232448 / (max_ctas + 1) + 1024;
     return smem > floor_bytes ? smem : floor_bytes;
-}
-
-// cudaFuncSetAttribute is a host-side round trip; raise the opt-in shared-memory
-// limit of a kernel only when a launch needs more than any launch before it.
-template <typename Kernel>
-int ensure_dynamic_smem(Kernel kernel, size_t smem, int *granted) {
-    if ((int)smem <= *granted) return PCX_OK;
-    PCX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PCX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    *granted = (int)smem;
-    return PCX_OK;
 }
 
 bool aligned16(const void *p) { return ((uintptr_t)p & 15) == 0; }
@@ -526,7 +517,8 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
     if (smem + static_smem > 232448 - 1024) PCX_FAIL(PCX_E_UNSUPPORTED, "mvmr tensor kernel does not fit (smem %zu)", smem);
     // (rows are never stored in a call that may do one again)
     const int mode = (store ? 2 : bulk ? 1 : p.chain > 1 ? 4 : more ? 3 : 0) + (a.only_if.words ? 5 : 0), threads = more ? 256 : 128;
-    static int granted_mvmr[10][64] = {}, regs_mvmr[10] = {};   // per kernel (and device)
+    static std::atomic<uint64_t> allowed[10];   // per kernel
+    static std::atomic<int> regs_mvmr[10];
     decltype(&mvmr_tc_kernel<0, 128, false, false>) const kernels[10] = {
         mvmr_tc_kernel<0, 128, false, false>, mvmr_tc_kernel<1, 128, false, false>, mvmr_tc_kernel<2, 128, false, false>,
         mvmr_tc_kernel<0, 256, false, false>, mvmr_tc_kernel<0, 256, true, false>,  mvmr_tc_kernel<0, 128, false, true>,
@@ -534,9 +526,7 @@ int mvmr_tensor(const MvmrArgs &a, cudaStream_t stream) {
         mvmr_tc_kernel<0, 256, true, true>};
     const auto kernel = kernels[mode];
     if (!kernel) PCX_FAIL(PCX_E_ARG, "mvmr tensor kernel: no such variant");
-    int dev = 0;
-    PCX_CUDA(cudaGetDevice(&dev));
-    if (int rc = ensure_dynamic_smem(kernel, smem, &granted_mvmr[mode][dev & 63])) return rc;
+    if (int rc = allow_shared_memory((const void *)kernel, &allowed[mode], true)) return rc;
     const int regs = kernel_registers(kernel, &regs_mvmr[mode]);
     const int occ = ctas_per_sm(smem + static_smem, p.ncols, regs, threads);
     const dim3 grid((unsigned)std::min<int64_t>(upper, std::max<int64_t>(1, (int64_t)occ * num_sms() / parts)), (unsigned)parts);

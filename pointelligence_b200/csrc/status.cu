@@ -69,6 +69,20 @@ int wait_for_hand_over(const HandOver &h, cudaStream_t stream) {
     }
 }
 
+int allow_shared_memory(const void *kernel, std::atomic<uint64_t> *done, bool prefer) {
+    int dev = 0, most = 0;
+    PCX_CUDA(cudaGetDevice(&dev));
+    const uint64_t bit = 1ull << (dev & 63);
+    if (done->load(std::memory_order_acquire) & bit) return PCX_OK;
+    cudaFuncAttributes own;
+    PCX_CUDA(cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+    PCX_CUDA(cudaFuncGetAttributes(&own, kernel));
+    PCX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)own.sharedSizeBytes));
+    if (prefer) PCX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    done->fetch_or(bit, std::memory_order_release);
+    return PCX_OK;
+}
+
 struct ProfRecord {
     const char *name;
     cudaEvent_t start, stop;

@@ -309,13 +309,8 @@ int launch_vvor(VvorTcParams &p, int parts, int64_t T, size_t block_rows, cudaSt
     if (p.nslots < 2) PCX_FAIL(PCX_E_UNSUPPORTED, "vvor tensor kernel does not fit (Ma=%d Cb=%d)", p.Ma, p.Cb);
     p.teams = std::min(TEAMS, p.nslots);   // a wait names its turn by parity: no team may be a whole ring ahead of another
     const size_t smem = rest + p.nslots * slot;
-    static int granted[64] = {};   // per device
-    int dev = 0;
-    PCX_CUDA(cudaGetDevice(&dev));
-    if ((int)smem > granted[dev & 63]) {
-        PCX_CUDA(cudaFuncSetAttribute(vvor_tc_kernel<CHR, STORE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        granted[dev & 63] = (int)smem;
-    }
+    static std::atomic<uint64_t> allowed;
+    if (int rc = allow_shared_memory((const void *)vvor_tc_kernel<CHR, STORE>, &allowed)) return rc;
     const dim3 grid((unsigned)std::min<int64_t>(STORE ? p.n_o : T / CHR + p.n_o + 1, std::max(1, num_sms() / parts)), (unsigned)parts);
     prof_begin("vvor_tc_kernel", stream);
     launch_after(vvor_tc_kernel<CHR, STORE>, grid, THREADS, smem, stream, p);
