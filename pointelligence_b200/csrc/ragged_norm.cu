@@ -965,6 +965,8 @@ int few_blocks(Kernel kernel, int64_t N, int C, int dtype, bool vec, int *cached
     return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)std::min(*cached, FEW_CTAS) * num_sms(), N / (2 * lanes)));
 }
 
+constexpr int NOT_TOGETHER = 1;   // the stream has a part of the chip (a green context): its blocks are not resident at once
+
 template <typename... Params, typename... Args>
 int launch_together(void (*kernel)(Params...), int blocks, cudaStream_t stream, Args &&...args) {
     cudaLaunchAttribute together = {};
@@ -973,7 +975,12 @@ int launch_together(void (*kernel)(Params...), int blocks, cudaStream_t stream, 
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((unsigned)blocks), config.blockDim = dim3(LN_THREADS), config.stream = stream;
     config.attrs = &together, config.numAttrs = 1;
-    PCX_CUDA(cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...));
+    const cudaError_t e = cudaLaunchKernelEx(&config, kernel, std::forward<Args>(args)...);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+        (void)cudaGetLastError();
+        return NOT_TOGETHER;
+    }
+    PCX_CUDA(e);
     PCX_LAUNCH_CHECK();
     return PCX_OK;
 }
@@ -1011,7 +1018,7 @@ int pcx_ragged_layer_norm(const void *d_x, const int64_t *d_lengths, const float
     prof_begin("layer_norm(fwd)", stream);   // all of its kernels
     if (S <= FEW && N > 0 && N * C * (int64_t)elem_size(dtype) <= FEW_BYTES) {
         const bool wide = vec_ok(C, dtype, {d_x, d_y, d_residual});
-        int blocks = 0, rc = PCX_OK;
+        int blocks = 0, rc = NOT_TOGETHER;
         PCX_LN_DISPATCH(dtype, wide, {
             static int resident = 0;
             blocks = std::min(FEW_BLOCKS, few_blocks(ln_few_kernel<T, VN>, N, C, dtype, wide, &resident));
@@ -1019,8 +1026,10 @@ int pcx_ragged_layer_norm(const void *d_x, const int64_t *d_lengths, const float
                 rc = launch_together(ln_few_kernel<T, VN>, blocks, stream, (const T *)d_x, d_lengths, d_weight, d_bias, (const T *)d_residual, (T *)d_y, d_mean,
                                      d_rstd, w.rec, N, (int)S, C, (float)eps, relu);
         });
-        prof_end(stream);
-        if (blocks > 0) return rc;
+        if (rc != NOT_TOGETHER) {
+            prof_end(stream);
+            return rc;
+        }
     }
     if (int rc = ln_offsets(d_lengths, S, N, w, stream)) return rc;
     const bool vec = vec_ok(C, dtype, {d_x, d_y, d_residual});
@@ -1059,7 +1068,7 @@ int pcx_ragged_layer_norm_backward(const void *d_grad_y, const void *d_x, const 
     const bool one_pass = C / (vec_ok(C, dtype, {d_grad_y, d_x, d_y, d_grad_x, d_grad_residual}) ? 16 / (int)elem_size(dtype) : 1) <= LN_THREADS;
     if (S <= FEW && N > 0 && one_pass && N * C * (int64_t)elem_size(dtype) <= FEW_BYTES) {
         const bool wide = vec_ok(C, dtype, {d_grad_y, d_x, d_y, d_grad_x, d_grad_residual});
-        int blocks = 0, rc = PCX_OK;
+        int blocks = 0, rc = NOT_TOGETHER;
         PCX_LN_DISPATCH(dtype, wide, {
             static int resident = 0;
             blocks = std::min(FEW_BLOCKS, few_blocks(ln_few_bwd_kernel<T, VN>, N, C, dtype, wide, &resident));
@@ -1067,8 +1076,10 @@ int pcx_ragged_layer_norm_backward(const void *d_grad_y, const void *d_x, const 
                 rc = launch_together(ln_few_bwd_kernel<T, VN>, blocks, stream, (const T *)d_grad_y, (const T *)d_x, (const T *)d_y, d_lengths, d_mean, d_rstd,
                                      d_weight, (float2 *)w.rec, d_grad_weight, d_grad_bias, (T *)d_grad_residual, (T *)d_grad_x, N, (int)S, C, relu);
         });
-        prof_end(stream);
-        if (blocks > 0) return rc;
+        if (rc != NOT_TOGETHER) {
+            prof_end(stream);
+            return rc;
+        }
     }
     if (int rc = ln_offsets(d_lengths, S, N, w, stream, true, d_grad_weight, d_grad_bias, C)) return rc;
     if (N == 0) return PCX_OK;

@@ -45,3 +45,36 @@ def test_against_fp64(lengths, C, dtype, tail):
     want = torch.autograd.grad(inner, [leaves[0], leaves[1], leaves[2]] + ([leaves[3]] if tail else []), go.double() * mask)
     for a, r in zip(got, want):
         assert float((a.double() - r).norm()) <= 4 * unit * float(r.norm()) + 1e-4 * float(go.double().norm()) * (1 if N * C < 64 else 1e-2)
+
+
+PART_OF_THE_CHIP = """
+import torch
+from pointelligence_b200.layers.norm import fused_layer_norm
+
+part = torch.cuda.GreenContext.create(num_sms=16, device_id=0)
+stream = part.Stream()
+g = torch.Generator(device="cuda").manual_seed(0)
+x = (torch.randn(20000, 64, device="cuda", generator=g) * 2 + 3).bfloat16().requires_grad_()
+go = torch.randn(20000, 64, device="cuda", generator=g).bfloat16()
+w, b = torch.ones(64, device="cuda").requires_grad_(), torch.zeros(64, device="cuda").requires_grad_()
+lengths = torch.tensor([15000, 5000], device="cuda")
+whole = torch.autograd.grad(fused_layer_norm(x, lengths, w, b, 1e-5), (x, w, b), go)
+torch.cuda.synchronize()
+with torch.cuda.stream(stream):
+    got = torch.autograd.grad(fused_layer_norm(x, lengths, w, b, 1e-5), (x, w, b), go)
+stream.synchronize()
+assert all(float((a.double() - r.double()).norm() / r.double().norm()) < 1e-3 for a, r in zip(got, whole))
+"""
+
+
+def test_on_a_part_of_the_chip():
+    """A stream that has fewer multiprocessors than the blocks of one launch would take together."""
+    import os
+    import subprocess
+    import sys
+
+    if not hasattr(torch.cuda, "GreenContext"):
+        pytest.skip("no green contexts")
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", PART_OF_THE_CHIP], cwd=root, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
