@@ -78,8 +78,8 @@ enum { CTRL_LOOKED = 16, CTRL_NEAR = 17 };
 // Order of the buckets.  bucket_sum_kernel is bound by what it gathers, most of which neighbouring rows gather as well, so where
 // the rows of a cloud lie next to each other in memory (what down-sampling emits: one triplet in 32 x 256 is asked whether
 // its feature row is close to that of the one before) buckets are numbered by bins of BIN_ROWS rows, else as their tiles come, by tap
-// signature: 1 M x 96 327 -> 245 us, 200 000 x 256 255 -> 180, x 96 113 -> 99, while mvmr_os_kernel, whose tiles then find their sums
-// further apart, takes 2 % more (459 -> 470, 348 -> 356, 125 -> 128).  A cloud in random order loses by it (200 000 x 96 117 -> 134).
+// signature: rooms with 8 to 10 triplets a row in the order of their cells, 1 M x 96 215 -> 173 us, 200 000 x 256 64 -> 58, x 96 33 -> 32,
+// while mvmr_os_kernel, whose tiles then find their sums further apart, takes up to 2 % more (401 -> 404, 260 -> 263, 107 -> 105).  A cloud in random order loses by it (200 000 x 96 117 -> 134).
 constexpr int BIN_ROWS = 64, BINS = 16384;   // rows of a bin, at least; bins, at most
 constexpr int NEAR = 2048;
 constexpr int64_t BINNED_ROWS = 65536;   // clouds from this size on: 40 000 x 96 takes 21 us either way

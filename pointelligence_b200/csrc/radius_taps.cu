@@ -69,7 +69,6 @@ struct TapsWs {
     int64_t *ctrl;          // [0] total pairs, [1] a tap's count does not fit 31 bits, [2] taps scanned,
                             // [3] queries without a neighbour, [4] points given room, [5] crowded buckets,
                             // [6] pairs of the fullest tap
-    int bits;
     int64_t buckets, nblocks;
 };
 
@@ -89,8 +88,7 @@ int bucket_bits(int64_t P) {
 size_t carve_taps(void *ws, int64_t P, int64_t Q, int k3, TapsWs *out) {
     Carver c(ws);
     TapsWs w;
-    w.bits = bucket_bits(P);
-    w.buckets = (int64_t)1 << w.bits;
+    w.buckets = (int64_t)1 << bucket_bits(P);
     w.nblocks = (Q + QPB - 1) / QPB;
     w.ctrl = c.take<int64_t>(8);
     w.tap_total = c.take<unsigned long long>(k3);
@@ -271,7 +269,7 @@ __global__ void __launch_bounds__(BIN_THREADS) taps_place_kernel(const float *__
 
 struct TapArgs {
     const float *queries;
-    const int32_t *query_sample, *point_sample;   // every second word of wide ids (1 << query_wide words apart)
+    const int32_t *query_sample;   // words of the queries' ids, 1 << query_wide apart (the points' are in sorted_sample)
     int query_wide;
     const float4 *sorted_pts;
     const int2 *table;
@@ -704,7 +702,7 @@ int check_common(int64_t P, int64_t Q, double radius, int distance_type, int ker
 TapArgs make_args(const TapsWs &w, const float *queries, const int32_t *point_sample, const int32_t *query_sample,
                   int64_t Q, double radius, int distance_type, int kernel_size, double grid) {
     TapArgs a = {};
-    a.queries = queries, a.query_sample = query_sample, a.point_sample = point_sample, a.query_wide = distance_type & PCX_RADIUS_WIDE_QUERY_IDS ? 1 : 0;
+    a.queries = queries, a.query_sample = query_sample, a.query_wide = distance_type & PCX_RADIUS_WIDE_QUERY_IDS ? 1 : 0;
     distance_type &= DISTANCE;
     a.sorted_pts = w.sorted_pts, a.table = w.table, a.kept_point = w.kept_point, a.kept_tap = w.kept_tap;
     a.sorted_sample = point_sample ? w.sorted_sample : nullptr, a.kept = kept_per_query(kernel_size * kernel_size * kernel_size);

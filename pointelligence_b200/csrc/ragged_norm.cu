@@ -109,6 +109,55 @@ __device__ __forceinline__ void merge(Moments &a, float n, float mean, float m2)
 
 constexpr int MOM_R = 4;
 
+// Moments of rows [lo, hi) of a block; valid in thread 0.
+template <typename T, int VN>
+__device__ __forceinline__ Moments moments_of(const T *__restrict__ x, const RowLayout &L, int64_t lo, int64_t hi, int C, Moments *scratch) {
+    Moments m{0.f, 0.f, 0.f, 0.f};
+    for (int cp = 0; cp * L.vcb < L.vc_total; ++cp) {
+        const int vcol = cp * L.vcb + L.vc;
+        if (vcol >= L.vc_total || L.lane >= L.lanes) continue;
+        const T *col = x + (int64_t)vcol * VN;
+        int64_t r = lo + L.lane;
+        for (; r + (MOM_R - 1) * L.lanes < hi; r += (int64_t)MOM_R * L.lanes) {
+            float v[MOM_R][VN], sum = 0.f, sq = 0.f;
+#pragma unroll
+            for (int k = 0; k < MOM_R; ++k) load_vec<T, VN>(col + (r + (int64_t)k * L.lanes) * C, v[k]);
+#pragma unroll
+            for (int k = 0; k < MOM_R; ++k)
+#pragma unroll
+                for (int i = 0; i < VN; ++i) sum += v[k][i];
+            const float mu = sum * (1.f / (MOM_R * VN));
+#pragma unroll
+            for (int k = 0; k < MOM_R; ++k)
+#pragma unroll
+                for (int i = 0; i < VN; ++i) sq += (v[k][i] - mu) * (v[k][i] - mu);
+            merge(m, (float)(MOM_R * VN), mu, sq);
+        }
+        for (; r < hi; r += L.lanes) {
+            float v[VN], sum = 0.f, sq = 0.f;
+            load_vec<T, VN>(col + r * C, v);
+#pragma unroll
+            for (int i = 0; i < VN; ++i) sum += v[i];
+            const float mu = sum * (1.f / VN);
+#pragma unroll
+            for (int i = 0; i < VN; ++i) sq += (v[i] - mu) * (v[i] - mu);
+            merge(m, (float)VN, mu, sq);
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float n = __shfl_xor_sync(0xffffffffu, m.n, o), mean = __shfl_xor_sync(0xffffffffu, m.mean, o),
+                    m2 = __shfl_xor_sync(0xffffffffu, m.m2, o);
+        merge(m, n, mean, m2);
+    }
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < LN_THREADS / 32; ++w) merge(m, scratch[w].n, scratch[w].mean, scratch[w].m2);
+    return m;
+}
+
 template <typename T, int VN>
 __global__ void __launch_bounds__(LN_THREADS, 4) ln_moments_kernel(const T *__restrict__ x, const int64_t *__restrict__ offsets, Moments *rec,
                                                                    int64_t N, int64_t S, int C, int rows) {
@@ -119,51 +168,8 @@ __global__ void __launch_bounds__(LN_THREADS, 4) ln_moments_kernel(const T *__re
     for (int64_t s = B.s_first; s <= B.s_last; ++s) {
         const int64_t lo = max(B.row0, offsets[s]), hi = min(B.row1, offsets[s + 1]);
         if (hi <= lo) continue;   // an empty sample inside the block (same decision in every thread)
-        Moments m{0.f, 0.f, 0.f, 0.f};
-        for (int cp = 0; cp * L.vcb < L.vc_total; ++cp) {
-            const int vcol = cp * L.vcb + L.vc;
-            if (vcol >= L.vc_total || L.lane >= L.lanes) continue;
-            const T *col = x + (int64_t)vcol * VN;
-            int64_t r = lo + L.lane;
-            for (; r + (MOM_R - 1) * L.lanes < hi; r += (int64_t)MOM_R * L.lanes) {
-                float v[MOM_R][VN], sum = 0.f, sq = 0.f;
-#pragma unroll
-                for (int k = 0; k < MOM_R; ++k) load_vec<T, VN>(col + (r + (int64_t)k * L.lanes) * C, v[k]);
-#pragma unroll
-                for (int k = 0; k < MOM_R; ++k)
-#pragma unroll
-                    for (int i = 0; i < VN; ++i) sum += v[k][i];
-                const float mu = sum * (1.f / (MOM_R * VN));
-#pragma unroll
-                for (int k = 0; k < MOM_R; ++k)
-#pragma unroll
-                    for (int i = 0; i < VN; ++i) sq += (v[k][i] - mu) * (v[k][i] - mu);
-                merge(m, (float)(MOM_R * VN), mu, sq);
-            }
-            for (; r < hi; r += L.lanes) {
-                float v[VN], sum = 0.f, sq = 0.f;
-                load_vec<T, VN>(col + r * C, v);
-#pragma unroll
-                for (int i = 0; i < VN; ++i) sum += v[i];
-                const float mu = sum * (1.f / VN);
-#pragma unroll
-                for (int i = 0; i < VN; ++i) sq += (v[i] - mu) * (v[i] - mu);
-                merge(m, (float)VN, mu, sq);
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float n = __shfl_xor_sync(0xffffffffu, m.n, o), mean = __shfl_xor_sync(0xffffffffu, m.mean, o),
-                        m2 = __shfl_xor_sync(0xffffffffu, m.m2, o);
-            merge(m, n, mean, m2);
-        }
-        __syncthreads();
-        if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = m;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            for (int w = 1; w < LN_THREADS / 32; ++w) merge(m, scratch[w].n, scratch[w].mean, scratch[w].m2);
-            rec[blockIdx.x + s] = m;
-        }
+        const Moments m = moments_of<T, VN>(x, L, lo, hi, C, scratch);
+        if (threadIdx.x == 0) rec[blockIdx.x + s] = m;
     }
 }
 
@@ -403,8 +409,8 @@ __global__ void __launch_bounds__(LN_THREADS, 4) ln_bwd_apply_kernel(const T *__
 // ---------------------------------------------------------------- small batches ----
 // Rows of up to 8 MB in up to 32 samples go through one kernel forward and one backward whose blocks are all resident (a
 // cooperative launch): sums of a block's rows, a barrier of the grid, the same rows again.  Such norms are bound by launches, of
-// which the kernels above take four and three: 2000 rows of 64 channels forward 26 -> 14 us, 5000 of 256 25 -> 19, 40 000 of 96
-// 18 -> 16; the 40 norms of a network on 40 000 points 0.34 ms less.  Beyond that the blocks of one launch see too few rows
+// which the kernels above take four and three: 2000 rows of 64 channels forward 25 -> 13 us, 5000 of 256 24 -> 13, 40 000 of 96
+// 23 -> 15; the 40 norms of a network on 40 000 points 0.34 ms less.  Beyond that the blocks of one launch see too few rows
 // in flight (300 000 x 64 29 and 44); larger batches sample by sample, so that the second look at a row is out of the L2,
 // lost as well (1.1 M x 64 in eight samples 84 and 120 forward, 130 and 184 backward): a sample a barrier is too little work for
 // the latency of its loads and folds.
@@ -432,55 +438,6 @@ struct FewSamples {
         __syncthreads();
     }
 };
-
-// Moments of rows [lo, hi) of a block; valid in thread 0.
-template <typename T, int VN>
-__device__ __forceinline__ Moments moments_of(const T *__restrict__ x, const RowLayout &L, int64_t lo, int64_t hi, int C, Moments *scratch) {
-    Moments m{0.f, 0.f, 0.f, 0.f};
-    for (int cp = 0; cp * L.vcb < L.vc_total; ++cp) {
-        const int vcol = cp * L.vcb + L.vc;
-        if (vcol >= L.vc_total || L.lane >= L.lanes) continue;
-        const T *col = x + (int64_t)vcol * VN;
-        int64_t r = lo + L.lane;
-        for (; r + (MOM_R - 1) * L.lanes < hi; r += (int64_t)MOM_R * L.lanes) {
-            float v[MOM_R][VN], sum = 0.f, sq = 0.f;
-#pragma unroll
-            for (int k = 0; k < MOM_R; ++k) load_vec<T, VN>(col + (r + (int64_t)k * L.lanes) * C, v[k]);
-#pragma unroll
-            for (int k = 0; k < MOM_R; ++k)
-#pragma unroll
-                for (int i = 0; i < VN; ++i) sum += v[k][i];
-            const float mu = sum * (1.f / (MOM_R * VN));
-#pragma unroll
-            for (int k = 0; k < MOM_R; ++k)
-#pragma unroll
-                for (int i = 0; i < VN; ++i) sq += (v[k][i] - mu) * (v[k][i] - mu);
-            merge(m, (float)(MOM_R * VN), mu, sq);
-        }
-        for (; r < hi; r += L.lanes) {
-            float v[VN], sum = 0.f, sq = 0.f;
-            load_vec<T, VN>(col + r * C, v);
-#pragma unroll
-            for (int i = 0; i < VN; ++i) sum += v[i];
-            const float mu = sum * (1.f / VN);
-#pragma unroll
-            for (int i = 0; i < VN; ++i) sq += (v[i] - mu) * (v[i] - mu);
-            merge(m, (float)VN, mu, sq);
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float n = __shfl_xor_sync(0xffffffffu, m.n, o), mean = __shfl_xor_sync(0xffffffffu, m.mean, o),
-                    m2 = __shfl_xor_sync(0xffffffffu, m.m2, o);
-        merge(m, n, mean, m2);
-    }
-    __syncthreads();
-    if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = m;
-    __syncthreads();
-    if (threadIdx.x == 0)
-        for (int w = 1; w < LN_THREADS / 32; ++w) merge(m, scratch[w].n, scratch[w].mean, scratch[w].m2);
-    return m;
-}
 
 template <typename T, int VN>
 __global__ void __launch_bounds__(LN_THREADS, FEW_CTAS) ln_few_kernel(const T *__restrict__ x, const int64_t *__restrict__ lengths, const float *__restrict__ weight,

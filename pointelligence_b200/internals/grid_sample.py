@@ -2,7 +2,8 @@
 
 ``center_nearest`` -- the reduction the convolution path uses -- runs entirely
 in the CUDA library: binning (Python-style floor division), 64-bit cell keys,
-radix sort, segment heads and the per-cell arg-min with the reference's fp32
+points put in the order of their cells by counting (by a radix sort where they
+crowd), segment heads and the per-cell arg-min with the reference's fp32
 arithmetic and lowest-index tie break.  The other reductions reuse its cell
 assignment and finish with a handful of torch calls.
 """

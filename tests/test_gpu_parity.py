@@ -656,7 +656,8 @@ def test_triplet_cache_scope_reuses_rulebooks():
                                            (60000, 0.001, 4e2)])
 @pytest.mark.parametrize("outlier", [False, True])
 def test_down_sampling_in_any_spread(n, cell, spread, outlier):
-    """Cells in order by counting, and by a sort where points crowd in few ranges of keys or the key space is too wide."""
+    """Cells in order by counting, and by a sort where points crowd in few ranges of keys (key spaces of up to 2^58 cells; wider ones, and
+    clouds one after the other at the same cell size, are in test_gpu_cell_order.py)."""
     from pointelligence_b200 import _cabi
 
     rng = np.random.default_rng(n)
