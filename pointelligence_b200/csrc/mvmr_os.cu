@@ -72,19 +72,6 @@ constexpr unsigned PLAN_MAGIC = 0x70637832u;
 
 // control words at the head of a plan
 enum { CTRL_MAGIC = 2, CTRL_GROUP = 3, CTRL_NMULTI = PCX_PLAN_MULTI_WORD, CTRL_UNSORTED = CTRL_NMULTI + 1, CTRL_WORDS = 64 };
-// ... of use while the plan is built: triplets looked at, those close to the one before
-enum { CTRL_LOOKED = 16, CTRL_NEAR = 17 };
-
-// Order of the buckets.  bucket_sum_kernel is bound by what it gathers, most of which neighbouring rows gather as well, so where
-// the rows of a cloud lie next to each other in memory (what down-sampling emits: one triplet in 32 x 256 is asked whether
-// its feature row is close to that of the one before) buckets are numbered by bins of BIN_ROWS rows, else as their tiles come, by tap
-// signature: rooms with 8 to 10 triplets a row in the order of their cells, 1 M x 96 215 -> 173 us, 200 000 x 256 64 -> 58, x 96 33 -> 32,
-// while mvmr_os_kernel, whose tiles then find their sums further apart, takes up to 2 % more (401 -> 404, 260 -> 263, 107 -> 105).  A cloud in random order loses by it (200 000 x 96 117 -> 134).
-constexpr int BIN_ROWS = 64, BINS = 16384;   // rows of a bin, at least; bins, at most
-constexpr int NEAR = 2048;
-constexpr int64_t BINNED_ROWS = 65536;   // clouds from this size on: 40 000 x 96 takes 21 us either way
-__host__ __device__ inline int64_t bin_rows(int64_t n_out) { return n_out <= (int64_t)BIN_ROWS * BINS ? BIN_ROWS : (n_out + BINS - 1) / BINS; }
-__device__ __forceinline__ bool rows_lie_together(const uint32_t *ctrl) { return 2 * ctrl[CTRL_NEAR] > ctrl[CTRL_LOOKED]; }
 
 struct PlanView {
     uint32_t *ctrl;        // CTRL_WORDS
@@ -198,19 +185,12 @@ __global__ void plan_init_kernel(int64_t n_out, uint32_t *sig, int32_t *row, int
 // Tap signature of every output row.  With more than 32 taps the taps are folded onto 32
 // bits (tap mod 32): rows that share a signature then share a superset of taps.  Notes rulebooks
 // whose rows do not ascend inside a tap.
-__global__ void plan_sig_kernel(const int32_t *__restrict__ scatter, const int32_t *__restrict__ gather, const int64_t *__restrict__ seg, int64_t T,
-                                int K, uint32_t *sig, uint32_t *ctrl) {
+__global__ void plan_sig_kernel(const int32_t *__restrict__ scatter, const int64_t *__restrict__ seg, int64_t T, int K,
+                                uint32_t *sig, uint32_t *ctrl) {
     start_after_previous();
     __shared__ int64_t s_seg[MAX_TAPS + 1];
     copy_seg(seg, K, s_seg);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (gather && blockIdx.x % 32 == 0) {
-        const int near = __syncthreads_count(t > 0 && t < T && abs(gather[t] - gather[t - 1]) <= NEAR);
-        if (threadIdx.x == 0) {
-            atomicAdd(&ctrl[CTRL_LOOKED], (uint32_t)min((int64_t)blockDim.x, T - t));
-            atomicAdd(&ctrl[CTRL_NEAR], (uint32_t)near);
-        }
-    }
     if (t >= T) return;
     const int k = tap_of(s_seg, K, t);
     const int32_t r = scatter[t];
@@ -240,11 +220,10 @@ __global__ void plan_order_kernel(const uint32_t *__restrict__ sig, int64_t n_ou
 }
 
 __global__ void plan_rank_kernel(const int32_t *__restrict__ row_sorted, int64_t n_out, int64_t n_pad, int32_t *rank,
-                                 int32_t *perm, uint32_t *bins, int nbins) {
+                                 int32_t *perm) {
     start_after_previous();
     const int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (x >= n_pad) return;
-    if (x < nbins) bins[x] = 0u;
     if (x < n_out) {
         const int32_t r = row_sorted[x];
         rank[r] = (int32_t)x;
@@ -258,65 +237,32 @@ __global__ void plan_rank_kernel(const int32_t *__restrict__ row_sorted, int64_t
 // consecutive triplets, so everything is placed by counting and no triplet is sorted.  Of any other rulebook these two kernels
 // touch nothing: placed in vain and cleared again, the strided rulebooks of a training step on 1.04 M points, taken backwards, cost 1.1 ms.
 
-// tile_rows[tile * 128 + slot] = first triplet of the bucket; triplets per tile; where rows lie together, buckets of several
-// triplets per bin
+// tile_rows[tile * 128 + slot] = first triplet of the bucket; triplets per tile
 __global__ void plan_heads_kernel(const int32_t *__restrict__ scatter, const int64_t *__restrict__ seg, const int32_t *__restrict__ rank,
-                                  int64_t T, int K, const uint32_t *__restrict__ ctrl, int32_t *tile_rows, int32_t *tile_cnt, uint32_t *bins,
-                                  int rows_of_bin) {
+                                  int64_t T, int K, const uint32_t *__restrict__ ctrl, int32_t *tile_rows, int32_t *tile_cnt) {
     start_after_previous();
     if (ctrl[CTRL_UNSORTED]) return;
     __shared__ int64_t s_seg[MAX_TAPS + 1];
     copy_seg(seg, K, s_seg);
-    const bool together = bins && rows_lie_together(ctrl);
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int bin = -1;
-    if (t < T) {
-        const int k = tap_of(s_seg, K, t);
-        const int32_t row = scatter[t];
-        if (t == s_seg[k] || scatter[t - 1] != row) {
-            int len = 1;
-            while (t + len < s_seg[k + 1] && scatter[t + len] == row) ++len;
-            const uint32_t r = (uint32_t)rank[row], tile = (r >> 7) * (uint32_t)K + (uint32_t)k;
-            tile_rows[((int64_t)tile << 7) | (r & 127u)] = (int32_t)t;
-            atomicAdd(&tile_cnt[tile], len);
-            if (len > 1) bin = row / rows_of_bin;
-        }
-    }
-    if (!together) return;
-    const unsigned same = __match_any_sync(0xffffffffu, bin);
-    if (bin >= 0 && (int)(threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&bins[bin], (uint32_t)__popc(same));
+    if (t >= T) return;
+    const int k = tap_of(s_seg, K, t);
+    const int32_t row = scatter[t];
+    if (t > s_seg[k] && scatter[t - 1] == row) return;
+    int len = 1;
+    while (t + len < s_seg[k + 1] && scatter[t + len] == row) ++len;
+    const uint32_t r = (uint32_t)rank[row], tile = (r >> 7) * (uint32_t)K + (uint32_t)k;
+    tile_rows[((int64_t)tile << 7) | (r & 127u)] = (int32_t)t;
+    atomicAdd(&tile_cnt[tile], len);
 }
 
-// The counts of the bins' buckets become the first bucket of each bin: one block, BINS / 1024 bins a thread.
-__global__ void __launch_bounds__(1024) plan_bins_kernel(uint32_t *bins, int nbins, const uint32_t *__restrict__ ctrl) {
-    start_after_previous();
-    if (ctrl[CTRL_UNSORTED] || !rows_lie_together(ctrl)) return;
-    __shared__ uint32_t s_sums[32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, b0 = (int)threadIdx.x * (BINS / 1024);
-    uint32_t n[BINS / 1024], sum = 0;
-#pragma unroll
-    for (int b = 0; b < BINS / 1024; ++b) n[b] = b0 + b < nbins ? bins[b0 + b] : 0u, sum += n[b];
-    uint32_t upto = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t up = __shfl_up_sync(0xffffffffu, upto, o);
-        if (lane >= o) upto += up;
-    }
-    if (lane == 31) s_sums[warp] = upto;
-    __syncthreads();
-    uint32_t at = upto - sum;
-    for (int w = 0; w < warp; ++w) at += s_sums[w];
-#pragma unroll
-    for (int b = 0; b < BINS / 1024; ++b) {
-        if (b0 + b < nbins) bins[b0 + b] = at;
-        at += n[b];
-    }
-}
-
-// One warp per (block, tap) tile: entries in slot order, the tile's source rows, its multi-triplet buckets.
+// One warp per (block, tap) tile: entries in slot order, the tile's source rows, its multi-triplet buckets, numbered as the tiles come.
+// (Numbered by output rows where the rows of a cloud lie together in memory, bucket_sum_kernel alone gains, 1 M x 96 215 -> 173 us, but
+// mvmr_os_kernel finds the sums of a tile further apart and buckets of many triplets follow each other: passes of 64 channels took 2 to
+// 35 % more, sweeps and clumped clouds the most, of 256 channels -8 to 17 %, a training step of 1.04 M points 0.4 % less.)
 __global__ void plan_tiles_kernel(const int32_t *__restrict__ scatter, const int32_t *__restrict__ gather, const int64_t *__restrict__ seg,
                                   int K, int64_t n_tiles, const int32_t *__restrict__ tile_offs, uint2 *entries, int32_t *tile_rows,
-                                  uint2 *buckets, uint32_t *ctrl, uint32_t *bins, int rows_of_bin) {
+                                  uint2 *buckets, uint32_t *ctrl) {
     start_after_previous();
     const int64_t tile = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int lane = threadIdx.x & 31;
@@ -327,14 +273,12 @@ __global__ void plan_tiles_kernel(const int32_t *__restrict__ scatter, const int
     int4 *slots = reinterpret_cast<int4 *>(tile_rows + (tile << 7)) + lane;
     const int4 h = *slots;
     const int32_t head[4] = {h.x, h.y, h.z, h.w};
-    const bool together = bins && rows_lie_together(ctrl);
-    int len[4], bin[4], sum = 0, multi = 0;
+    int len[4], sum = 0, multi = 0;
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
         len[s] = 0;
         if (head[s] >= 0) {
             const int32_t row = scatter[head[s]];
-            bin[s] = row / rows_of_bin;
             len[s] = 1;
             while (head[s] + len[s] < end && scatter[head[s] + len[s]] == row) ++len[s];
         }
@@ -361,9 +305,8 @@ __global__ void plan_tiles_kernel(const int32_t *__restrict__ scatter, const int
             if (len[s] == 1) source[s] = j;
         }
         if (len[s] > 1) {
-            const uint32_t id = together ? atomicAdd(&bins[bin[s]], 1u) : base++;
-            buckets[id] = make_uint2(entry, (uint32_t)len[s]);
-            source[s] = -2 - (int32_t)id;
+            buckets[base] = make_uint2(entry, (uint32_t)len[s]);
+            source[s] = -2 - (int32_t)base++;
         }
         entry += (uint32_t)len[s];
     }
@@ -1238,7 +1181,7 @@ int pcx_mvmr_plan_build_counted(const int32_t *d_scatter, const int32_t *d_gathe
     PCX_LAUNCH_CHECK();
     size_t bytes = w.cub_bytes;
     if (T > 0) {
-        launch_after(plan_sig_kernel, blocks(T), TPB, 0, stream, d_scatter, n_out >= BINNED_ROWS ? d_gather : nullptr, d_seg_offs, T, K, w.sig, pv.ctrl);
+        launch_after(plan_sig_kernel, blocks(T), TPB, 0, stream, d_scatter, d_seg_offs, T, K, w.sig, pv.ctrl);
         PCX_LAUNCH_CHECK();
     }
     // rows by (planes, signature), stable: rows of equal keys keep their order
@@ -1249,23 +1192,17 @@ int pcx_mvmr_plan_build_counted(const int32_t *d_scatter, const int32_t *d_gathe
     PCX_LAUNCH_CHECK();
     PCX_CUDA(cub::DeviceRadixSort::SortPairs(w.cub_tmp, bytes, w.order, w.order_sorted, w.row, w.row_sorted, (int)n_out, 0,
                                              std::min(K, 32) + 3 * ks, stream));
-    uint32_t *const bins = n_out >= BINNED_ROWS ? reinterpret_cast<uint32_t *>(w.order) : nullptr;   // (sorted by now)
-    const int rows_of_bin = (int)bin_rows(n_out), nbins = bins ? (int)((n_out + rows_of_bin - 1) / rows_of_bin) : 0;
-    launch_after(plan_rank_kernel, blocks(n_pad), TPB, 0, stream, w.row_sorted, n_out, n_pad, w.rank, pv.perm, bins, nbins);
+    launch_after(plan_rank_kernel, blocks(n_pad), TPB, 0, stream, w.row_sorted, n_out, n_pad, w.rank, pv.perm);
     PCX_LAUNCH_CHECK();
     if (T > 0) {
-        launch_after(plan_heads_kernel, blocks(T), TPB, 0, stream, d_scatter, d_seg_offs, w.rank, T, K, pv.ctrl, pv.tile_rows, w.tile_cnt, bins, rows_of_bin);
+        launch_after(plan_heads_kernel, blocks(T), TPB, 0, stream, d_scatter, d_seg_offs, w.rank, T, K, pv.ctrl, pv.tile_rows, w.tile_cnt);
         PCX_LAUNCH_CHECK();
-        if (bins) {
-            launch_after(plan_bins_kernel, 1, 1024, 0, stream, bins, nbins, pv.ctrl);
-            PCX_LAUNCH_CHECK();
-        }
     }
     bytes = w.cub_bytes;
     PCX_CUDA(cub::DeviceScan::ExclusiveSum(w.cub_tmp, bytes, w.tile_cnt, pv.tile_offs, (int)(n_tiles + 1), stream));
     if (T > 0) {
         launch_after(plan_tiles_kernel, blocks(n_tiles * 32), TPB, 0, stream, d_scatter, d_gather, d_seg_offs, K, n_tiles, pv.tile_offs, pv.entries,
-                                                                   pv.tile_rows, pv.buckets, pv.ctrl, bins, rows_of_bin);
+                                                                   pv.tile_rows, pv.buckets, pv.ctrl);
         PCX_LAUNCH_CHECK();
     }
     if (int rc = order_groups(pv, w, K, G, stream)) return rc;

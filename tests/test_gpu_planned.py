@@ -376,11 +376,11 @@ def test_small_clouds_split_by_taps_and_columns(n, G, C, M):
     assert _cabi.device_status() == 0
 
 
-@pytest.mark.parametrize("n", [65535, 65536, 65599, 150001, 1050000])   # below the clouds that are binned, the smallest, a last bin of a row, wider bins
+@pytest.mark.parametrize("n", [65535, 65536, 65599, 150001, 1050000])
 @pytest.mark.parametrize("shuffled", [False, True])                      # rows that lie together, and rows that do not
 def test_buckets_are_numbered_once_each(n, shuffled):
-    """Whatever order the buckets are numbered in: every number from 0 on is used by one slot of a tile, and its entries are those of
-    the slot's row, in the order of the rulebook."""
+    """Every number from 0 on is used by one slot of a tile, and its entries are those of the slot's row, in the order of the
+    rulebook."""
     from pointelligence_b200 import _cabi
 
     g = torch.Generator(device=DEV).manual_seed(n)
@@ -395,8 +395,6 @@ def test_buckets_are_numbered_once_each(n, shuffled):
     v, T = plan.views(), i.numel()
     m = rows.numel() * K
     assert plan.multi_buckets == m
-    looked, near_ = int(v["ctrl"][16]), int(v["ctrl"][17])
-    assert (2 * near_ > looked) == (n >= 65536 and not shuffled)
     where = (v["tile_rows"] < -1).nonzero()
     ids = (-2 - v["tile_rows"][where[:, 0], where[:, 1]]).long()
     assert torch.equal(torch.sort(ids).values, torch.arange(m, device=DEV))
