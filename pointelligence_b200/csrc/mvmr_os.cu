@@ -257,9 +257,10 @@ __global__ void plan_heads_kernel(const int32_t *__restrict__ scatter, const int
 }
 
 // One warp per (block, tap) tile: entries in slot order, the tile's source rows, its multi-triplet buckets, numbered as the tiles come.
-// (Numbered by output rows where the rows of a cloud lie together in memory, bucket_sum_kernel alone gains, 1 M x 96 215 -> 173 us, but
-// mvmr_os_kernel finds the sums of a tile further apart and buckets of many triplets follow each other: passes of 64 channels took 2 to
-// 35 % more, sweeps and clumped clouds the most, of 256 channels -8 to 17 %, a training step of 1.04 M points 0.4 % less.)
+// (Numbered by bins of output rows where the rows of a cloud lie together in memory, bucket_sum_kernel alone gains, 1 M x 96 215 -> 173
+// us, but mvmr_os_kernel finds the sums of a tile further apart, and buckets of many triplets follow each other.  A pass then took 0 to 13 %
+// more at 32 and 64 channels of a million rows, 2 to 35 % more at 64 of 100 000 to 600 000, sweeps and clumped clouds the most, and 0 to 10 %
+// less at 96 and 128 of a million; a training step of 1.04 M points 0.4 % less.  The plan does not know the channels.)
 __global__ void plan_tiles_kernel(const int32_t *__restrict__ scatter, const int32_t *__restrict__ gather, const int64_t *__restrict__ seg,
                                   int K, int64_t n_tiles, const int32_t *__restrict__ tile_offs, uint2 *entries, int32_t *tile_rows,
                                   uint2 *buckets, uint32_t *ctrl) {
