@@ -190,23 +190,33 @@ Tensor mvmr_split(const Tensor &weight, const Tensor &feat, const Tensor &gather
 }
 
 // Layers of up to 8 channels of the contraction on rulebooks of the geometry path (pcx_mvmr_thin: rows known to ascend
-// inside every tap).  That kernel's time goes with the (128 rows x 8 taps x 64 output channels) it multiplies, 8 to 16 ns each,
-// the scatter kernel's with the fp32 sums it adds, 2.2 to 3.3 TB/s: taken from 26 000 bytes of sums for each.  Measured, scatter
-// (with its padded copies) / this, us, and the bytes:
+// inside every tap).  That kernel takes its steps one after the other, a microsecond each, in up to 444 blocks at once: for every tile
+// of 128 rows x 64 output channels and every eight taps as many as the fullest (row, tap) has triplets, up to eight, of which only the
+// average over all is known here.  The scatter kernel adds fp32 sums at a steady rate, the faster one for rows of 64 channels.  The two
+// lines below are fitted to 760 calls (rooms, sweeps, uniform clouds of 300 to 400 000 points, 2 to 250 triplets a row, 27 and
+// 125 taps, 16 to 256 output channels): the choice is 2.4 % slower than the better of the two (geometric mean), 18 % faster than the
+// scatter kernel alone, and more than 10 % slower than that in 14 of them (sweeps, whose points crowd: at worst 198 us for 122).
+// Until there was a term for steps and for blocks that are too few, it was 25 % slower than the better one.  us, scatter / this:
 //
-//   27 taps    20 000 rows, 1.7 a row    -> 32  18 / 27 (7 000)     -> 64  21 / 29 (14 000)    -> 256  35 / 42 (14 000)
-//             150 000, 6.4                      70 / 61 (26 000)           90 / 70 (53 000)           437 / 192 (53 000)
-//              40 000, 16.4                     49 / 47 (67 000)           59 / 51 (134 000)          252 / 99 (134 000)
-//             600 000, 22.6                    649 / 319 (93 000)         871 / 356 (185 000)
-//   125 taps   80 000, 11.2                     63 / 99 (11 500)           76 / 106 (23 000)          336 / 286 (23 000)
-//              80 000, 23.4                    104 / 128 (24 000)         131 / 136 (48 000)          652 / 381 (48 000)
-//             150 000, 20.0                    154 / 176 (21 000)         195 / 188 (41 000)         1088 / 611 (41 000)
-bool thin_pays(at::ScalarType dtype, int64_t T, int64_t n_in, int64_t n_out, int64_t K, int64_t G, int64_t inw, int64_t outw) {
+//   27 taps    1000 points, 40 a row     -> 64   21 / 37    10 000, 40  -> 64   38 / 65     60 000, 15  -> 64   68 / 55
+//             100 000, 40                -> 32  199 / 100   200 000, 6  -> 128  225 / 110
+//   125 taps   30 000, 80                -> 32  121 / 75    100 000, 30 -> 32  144 / 114    200 000, 5   -> 32   63 / 129
+//
+// A layer that may round sums (`or_planned`) would get a plan of a dense rulebook instead of the scatter kernel: that takes 150 us and
+// more, for a rulebook that is mostly used once.  Only where most (row, tap) hold several triplets is it left to the plan, which adds
+// them up beforehand (32 000 points of a sweep with 124 triplets a row, 8 -> 256 channels: 49 us a pass on a plan, 240 here).
+bool thin_pays(at::ScalarType dtype, int64_t T, int64_t n_in, int64_t n_out, int64_t K, int64_t G, int64_t inw, int64_t outw, bool or_planned) {
     if (!is_half(dtype) || G != 1 || K <= 1 || K > 512 || inw <= 0 || inw > 8 || outw <= 0 || outw > 1024 || T <= 0 || T >= (int64_t(1) << 27) - 1 ||
         n_in <= 0 || n_out <= 0)
         return false;
-    const int64_t products = ((n_out + 127) / 128) * ((K + 7) / 8) * ((outw + 63) / 64);
-    return products < (int64_t(1) << 31) && T * outw * 4 >= 26000 * products;
+    const int64_t tiles = (n_out + 127) / 128, parts = (outw + 63) / 64, eights = (K + 7) / 8, width = (outw + 15) / 16 * 16;
+    if (tiles * eights * parts >= int64_t(1) << 31) return false;
+    const double triplets = 1e-6 * (double)T, a_cell = (double)T / ((double)n_out * (double)K);
+    if (or_planned && T >= 12 * n_out && a_cell >= 0.18) return a_cell < 1.;
+    const double thin = 30. + 17.3 * triplets + 0.14 * 512e-6 * (double)(tiles * K) +
+                        1.06 * std::max(1., (double)(tiles * parts) / 444.) * (double)eights * std::min(8., 1.3 + 2.05 * a_cell);
+    const double a_triplet = width == 64 ? 53. : width <= 32 ? 2.6 + 1.3 * (double)width : 1.35 * (double)width - 4.;
+    return thin < 17. + a_triplet * triplets + (width > 32 ? 1e-6 * (double)(n_out * width) : 0.);
 }
 bool rows_ascend(const Tensor &scatter, const Tensor &gather, const Tensor &seg, int64_t K) {
     py::gil_scoped_acquire gil;
@@ -252,7 +262,7 @@ Tensor mvmr_impl(Tensor weight, Tensor feat, const Tensor &gather_, const Tensor
     c10::cuda::CUDAGuard guard(feat.device());
     const bool plan_padded = engine & PLAN_PADDED && padded(C) == (C + 15) / 16 * 16 && padded(M) == (M + 15) / 16 * 16;
     engine &= ~PLAN_PADDED;
-    if (engine == 0 && seg_ && thin_pays(feat.scalar_type(), T, feat.size(0), n_out, K, G, inw, outw) &&
+    if (engine == 0 && seg_ && thin_pays(feat.scalar_type(), T, feat.size(0), n_out, K, G, inw, outw, plan_padded) &&
         // (a captured pass is replayed on whatever the index tensors hold then: on the kernels that take any order)
         c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None && rows_ascend(scatter_, gather_, *seg_, K)) {
         const Tensor y = mvmr_thin(weight, feat, gather_, scatter_, *seg_, n_out, flags, bias);

@@ -155,31 +155,33 @@ def _kernels(call):
     return out, names
 
 
-@pytest.mark.parametrize("C,M", [(24, 40), (40, 24), (3, 24), (24, 6), (40, 40)])
-def test_padded_widths_choose_their_kernels_like_others(C, M):
-    """A dense rulebook (about 17 triplets a row of 27 taps): the output-stationary kernel, which a layer of the next
-    multiples of 16 takes in both directions; three input channels forward, and six output channels backward, take the
-    kernel of thin layers instead."""
+@pytest.mark.parametrize("C,M,n,grid,per_row,thin", [
+    (24, 40, 6000, 0.0362, (13, 26), False), (40, 24, 6000, 0.0362, (13, 26), False), (40, 40, 6000, 0.0362, (13, 26), False),
+    (3, 24, 6000, 0.0362, (13, 26), True), (24, 6, 6000, 0.0362, (13, 26), True), (3, 64, 60000, 0.0165, (13, 26), True),
+    (64, 6, 60000, 0.0165, (13, 26), True), (3, 64, 60000, 0.023, (28, 60), False)])
+def test_padded_widths_choose_their_kernels_like_others(C, M, n, grid, per_row, thin):
+    """Dense rulebooks of 27 taps: the output-stationary kernel, which a layer of the next multiples of 16 takes in both
+    directions; contractions of up to eight channels take the kernel of thin layers on fewer than a triplet for a row and a tap."""
     from pointelligence_b200.backbone import Bf16PointConv3d
     from pointelligence_b200.layers import MetaData, PointConv3d
     from pointelligence_b200.layers.triplets import handle_stride_and_build_triplets
 
     g = torch.Generator(device="cuda").manual_seed(C + M)
-    pts = torch.rand(6000, 3, device="cuda", generator=g)
-    m = MetaData(points=pts, sample_inds=torch.zeros(6000, dtype=torch.int64, device="cuda"),
-                 sample_sizes=torch.tensor([6000], device="cuda"), grid_size=0.0362)
+    pts = torch.rand(n, 3, device="cuda", generator=g)
+    m = MetaData(points=pts, sample_inds=torch.zeros(n, dtype=torch.int64, device="cuda"),
+                 sample_sizes=torch.tensor([n], device="cuda"), grid_size=grid)
     m = handle_stride_and_build_triplets(m, 1.0, (3, 3, 3), 2.5)
-    assert 13 < m.i.numel() / 6000 < 30
+    assert per_row[0] < m.i.numel() / n < per_row[1]
     conv = Bf16PointConv3d(C, M, 3, device="cuda")
-    x = torch.randn(6000, C, device="cuda", generator=g).bfloat16().requires_grad_()
-    go = torch.randn(6000, M, device="cuda", generator=g).bfloat16()
-    y, forward = _kernels(lambda: conv(x, m.i, m.j, m.k, 6000, contract=m.contract, seg_offs=m.seg_offs))
+    x = torch.randn(n, C, device="cuda", generator=g).bfloat16().requires_grad_()
+    go = torch.randn(n, M, device="cuda", generator=g).bfloat16()
+    y, forward = _kernels(lambda: conv(x, m.i, m.j, m.k, n, contract=m.contract, seg_offs=m.seg_offs))
     (gx, gw), backward = _kernels(lambda: torch.autograd.grad(y, (x, conv.weight), go))
     convolutions = lambda names: [n.split("(")[0] for n in names if n.startswith(("bucket_sum", "mvmr_"))]
-    assert convolutions(forward) == (["mvmr_thin_kernel"] if C <= 8 else ["bucket_sum_kernel", "mvmr_os_kernel"])
-    assert convolutions(backward) == (["mvmr_thin_kernel"] if M <= 8 else ["bucket_sum_kernel", "mvmr_os_kernel"])
+    assert convolutions(forward) == (["mvmr_thin_kernel"] if thin and C <= 8 else ["bucket_sum_kernel", "mvmr_os_kernel"])
+    assert convolutions(backward) == (["mvmr_thin_kernel"] if thin and M <= 8 else ["bucket_sum_kernel", "mvmr_os_kernel"])
     w64, x64 = conv.weight.detach().bfloat16().double()[:, 0], x.detach().double()
-    ref, gref, wref = torch.zeros(6000, M, device="cuda").double(), torch.zeros(6000, C, device="cuda").double(), torch.zeros_like(w64)
+    ref, gref, wref = torch.zeros(n, M, device="cuda").double(), torch.zeros(n, C, device="cuda").double(), torch.zeros_like(w64)
     for t in range(27):
         s = slice(int(m.seg_offs[t]), int(m.seg_offs[t + 1]))
         ref.index_add_(0, m.i[s].long(), x64[m.j[s].long()] @ w64[t])
@@ -190,7 +192,7 @@ def test_padded_widths_choose_their_kernels_like_others(C, M):
         assert a.shape == r.shape and float((a.double() - r).norm() / r.norm()) < 1.5 * 2.0 ** -8
     # other layers of such widths keep exact operands
     plain = PointConv3d(C, M, 3, device="cuda", dtype=torch.bfloat16)
-    _, names = _kernels(lambda: plain(x, m.i, m.j, m.k, 6000, contract=m.contract, seg_offs=m.seg_offs))
+    _, names = _kernels(lambda: plain(x, m.i, m.j, m.k, n, contract=m.contract, seg_offs=m.seg_offs))
     assert "mvmr_os_kernel" not in convolutions(names)
 
 
