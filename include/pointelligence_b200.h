@@ -523,8 +523,8 @@ int pcx_radius_fill(const float *d_points, const float *d_queries, int64_t P,
  *       (one synchronisation) for a caller that has no capacity estimate.
  *   pcx_radius_taps_fill   writes d_out_i / d_out_j (/ d_out_k when not NULL),
  *       buffers of `capacity` int32 each, waits once, for the count, and returns
- *       the number of pairs in *h_total; the buffers are filled in the order of
- *       the stream, possibly after the call has returned.  When the pairs do not fit it writes
+ *       the number of pairs in *h_total; the buffers are filled, and the queries and
+ *       ids read, in the order of the stream, possibly after the call has returned.  When the pairs do not fit it writes
  *       nothing and returns PCX_E_CAPACITY with *h_total set: call it again
  *       with buffers of that size (the state is kept in d_ws, which must stay
  *       untouched between the calls).
