@@ -206,6 +206,31 @@ def test_sums_that_leave_the_range_or_are_no_numbers(dtype):
     assert _rel(got[ok], ref[ok].double()) <= 2 * BOUND[dtype]
 
 
+@pytest.mark.parametrize("room", [0, 1, 30, 100000])   # sums that the workspace holds
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_sums_that_find_no_room(room, dtype):
+    """Triplets of those are taken one by one, in the same eight taps as sums that found room."""
+    from pointelligence_b200 import _cabi
+
+    n, K, C, M, members = 1500, 27, 5, 40, 50
+    g = torch.Generator(device="cuda").manual_seed(room)
+    i, j, k, seg = _clumped(n, members, K, C, 5.0, 3, 4)
+    w = (torch.randn(K, C, M, device="cuda", generator=g) / C ** 0.5).to(dtype)
+    x = torch.randn(n, C, device="cuda", generator=g).to(dtype)
+    L, ptr = _cabi.lib(), _cabi.ptr
+    bare = L.pcx_mvmr_thin_workspace_bytes(n, n, K, C, M, 0) - 48 * n      # (with room for a sum a row)
+    ws = torch.empty(bare + 48 * room + 256, dtype=torch.uint8, device="cuda")
+    out = torch.full((n, M), float("nan"), device="cuda", dtype=dtype)
+    code = _cabi.dtype_code(dtype)
+    call = lambda size: L.pcx_mvmr_thin(ptr(w), ptr(x), ptr(j), ptr(i), ptr(seg), None, ptr(out), i.numel(), n, n, K, C, M, 0, code, ptr(ws), size,
+                                        _cabi.stream_ptr())
+    _cabi.check(call(bare + 48 * room + 256))
+    assert _rel(out, _exact(w, x, i, j, k, n)) <= BOUND[dtype]
+    most = int(_steps(ws, n, K).max())
+    assert most <= 8 if room == 100000 else most >= members
+    assert call(bare - 512) == -4      # PCX_E_CAPACITY
+
+
 def test_too_little_memory_for_the_table():
     """A call that the scatter kernels have room for is no error where the table of this one does not fit."""
     from pointelligence_b200 import _cabi
