@@ -156,14 +156,16 @@ __global__ void radius_key_kernel(const float *__restrict__ pts, const int32_t *
 }
 
 // Cell table: key -> [start, end) of the cell's points in the sorted order.  Heads of
-// runs insert (key, start); tails look their slot up and add the end.  Keys are >= 0.
+// runs insert (key, start); tails look their slot up and add the end.  Samples may be numbered below zero, and the cell
+// beyond the last one of sample -1, which queries look at and no point lies in, has the key of an empty slot: an empty
+// slot is looked for first and belongs to no cell.
 constexpr int64_t CELL_EMPTY = -1;
 __global__ void cell_table_heads_kernel(const int64_t *__restrict__ keys, int64_t P, int64_t *tkeys, int2 *tranges,
                                         uint64_t mask) {
     int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (p >= P) return;
     const int64_t key = keys[p];
-    if (p > 0 && keys[p - 1] == key) return;
+    if (key == CELL_EMPTY || (p > 0 && keys[p - 1] == key)) return;
     uint64_t slot = mix64((uint64_t)key) & mask;
     for (;;) {   // the table is at most half full: an empty slot always turns up
         const long long prev = (long long)atomicCAS((unsigned long long *)&tkeys[slot], (unsigned long long)CELL_EMPTY,
@@ -177,8 +179,8 @@ __device__ __forceinline__ int64_t cell_slot(const int64_t *__restrict__ tkeys, 
     uint64_t slot = mix64((uint64_t)key) & mask;
     for (;;) {
         const int64_t k = tkeys[slot];
-        if (k == key) return (int64_t)slot;
         if (k == CELL_EMPTY) return -1;
+        if (k == key) return (int64_t)slot;
         slot = (slot + 1) & mask;
     }
 }

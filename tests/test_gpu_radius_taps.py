@@ -342,3 +342,22 @@ def test_many_crowded_cells_and_few_queries():
 
     search = best(lambda: _cabi.radius_search(pts, qry, 0.1, None, None, 0, kernel_size=3, kernel_grid_size=0.08))
     assert search < 5 * best(lambda: torch.sort(keys)), search
+
+
+@pytest.mark.parametrize("lowest", [-1, -2, -7, -2**31])
+@pytest.mark.parametrize("samples", [1, 3])
+def test_samples_numbered_below_zero(lowest, samples):
+    """A query in the last cell of sample -1 along every axis looks at a cell whose key is that of an empty slot."""
+    from pointelligence_b200 import _cabi
+
+    dev = torch.device("cuda:0")
+    g = torch.Generator(device=dev).manual_seed(samples)
+    pts = torch.cat([torch.rand(400, 3, device=dev, generator=g), torch.full((20, 3), 1.15, device=dev)] * samples)
+    ids = torch.arange(samples, device=dev).repeat_interleave(420)
+    ref, got = _both(pts, pts, ids + lowest, ids + lowest, 0.1, 3, 0.08)
+    _assert_same(ref, got)
+    _assert_same(_both(pts, pts, ids, ids, 0.1, 3, 0.08)[0], ref)
+    below = _cabi.radius_search(pts, pts, 0.1, ids + lowest, ids + lowest, 0, return_distances=True)
+    above = _cabi.radius_search(pts, pts, 0.1, ids, ids, 0, return_distances=True)
+    for a, b in zip(below, above):
+        assert torch.equal(a, b)
